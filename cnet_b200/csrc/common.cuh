@@ -89,7 +89,7 @@ int skinny_bwd_x(cnb_ctx* ctx, const float* gr, const float* gi, const float* wr
 int skinny_bwd_w(cnb_ctx* ctx, const float* gr, const float* gi, const float* xr, const float* xi, float* dr,
                  float* di, int B, int in, int out, int accumulate, cudaStream_t st);
 
-// Shared-memory FFT (N = 256, 1024, 4096); inverse = conjugate direction.
+// Shared-memory FFT (fft_pipe.cu at N = 1024, fft_mixed.cu elsewhere); inverse = conjugate direction.
 bool fft_supported(int N);
 int fft_run(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, int B, int N, int inverse,
             int accumulate, cudaStream_t st);

@@ -1,0 +1,402 @@
+// FourierTrans at any length that fits shared memory: a mixed-radix Stockham transform, rows in shared memory.
+//
+// N is factored into radices of at most 16 (2..16; primes up to 13), as few passes as that takes: 784 = 14 x 14 x 4,
+// 1500 = 10 x 15 x 10, 4096 = 16 x 16 x 16.  A thread takes one butterfly of R points at a time in registers; pass p
+// with L = the product of the radices before it reads x[j + q N/R], multiplies by e^{-2 pi i (j % L) q / (L R)},
+// transforms over q and writes (j / L) L R + j % L + q L, so the last pass comes out in natural order.  The first
+// pass reads the planes and the last one writes them (consecutive threads, consecutive elements); the passes between
+// go through shared memory, whose elements are spread by one in every 16 against bank conflicts.
+//
+// Lengths with a prime factor above 13 use the chirp form (Bluestein): X[k] = c[k] sum_n (x[n] c[n]) conj(c[k-n]),
+// c[n] = e^{-pi i n^2 / N}, the convolution as two transforms of a length M >= 2N-1 that factors well, in the same
+// launch and the same shared memory.
+//
+// The conjugate transform is the forward one with the planes swapped on both sides.  HBM traffic: one read and one
+// write of the tensor; a product with the N x N twiddle matrix (the only other form for these lengths) costs 8 N
+// flops an element and the matrix.
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+#include <vector>
+
+#include "common.cuh"
+#include "fft_mixed.cuh"
+#include "fft_regs.cuh"
+
+namespace {
+
+using namespace cnb_mixed;
+using cnb_fft::FftEpilogue;
+
+constexpr int MAX_PASSES = 6, MAX_THREADS = 256;
+constexpr size_t MAX_SMEM = 224 * 1024;
+
+struct Pass {
+    int radix, L, nb;                 // nb = length / radix butterflies per row
+    unsigned mag_nb, mag_L;           // reciprocals for the two divisions of an index (0: the divisor is 1)
+    int tw;                           // first entry of the pass's twiddles: [q - 1][k], q = 1..radix-1, k < L
+};
+
+struct MixedPlan {
+    int n, m;                         // row length; transform length (m > n: chirp form)
+    int passes, rows, threads, stride; // rows per CTA; float2 per row of a buffer
+    int buffers;
+    Pass p[MAX_PASSES];
+    float scale;
+};
+
+__host__ __device__ __forceinline__ int pad_of(int i) { return i + (i >> 4); }
+
+__device__ __forceinline__ int div_by(int i, unsigned mag) { return mag ? (int) __umulhi((unsigned) i, mag) : i; }
+
+struct Io {
+    const float *xr, *xi;             // planes of this CTA's first row
+    float *yr, *yi;
+    const float2 *tw, *chirp, *spectrum;
+    const float2* src;                // shared-memory buffers, NULL: the planes
+    float2* dst;
+    int rows, accumulate;
+    bool spectral;                    // chirp form: this pass opens the inverse transform
+    size_t row0;
+};
+
+template <int R, bool EPI, bool CHIRP>
+__device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, const Io& io, const FftEpilogue& ep) {
+    const int items = io.rows * d.nb;
+    for (int i = threadIdx.x; i < items; i += blockDim.x) {
+        const int row = div_by(i, d.mag_nb), j = i - row * d.nb;
+        float2 v[R];
+        if (io.src) {
+            const float2* s = io.src + row * pl.stride;
+#pragma unroll
+            for (int q = 0; q < R; ++q) v[q] = s[pad_of(j + q * d.nb)];
+            if (CHIRP && io.spectral) {
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    const float2 t = cmul(v[q], __ldg(io.spectrum + j + q * d.nb));
+                    v[q] = make_float2(t.y, t.x);          // swapped: the inverse transform
+                }
+            }
+        } else {
+            const float* pr = io.xr + (size_t) row * pl.n + j;
+            const float* pi = io.xi + (size_t) row * pl.n + j;
+            if (CHIRP) {
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    const int e = j + q * d.nb;
+                    v[q] = make_float2(0.f, 0.f);
+                    if (e < pl.n) v[q] = cmul(make_float2(pr[q * d.nb], pi[q * d.nb]), __ldg(io.chirp + e));
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < R; ++q) v[q] = make_float2(pr[q * d.nb], pi[q * d.nb]);
+            }
+        }
+        const int k = j - div_by(j, d.mag_L) * d.L;
+        if (d.L > 1) {
+            const float2* w = io.tw + d.tw + k;
+#pragma unroll
+            for (int q = 1; q < R; ++q) v[q] = cmul(v[q], __ldg(w + (q - 1) * d.L));
+        }
+        dft<R>(v);
+        const int o = (j - k) * R + k;
+        if (io.dst) {
+            float2* t = io.dst + row * pl.stride;
+#pragma unroll
+            for (int q = 0; q < R; ++q) t[pad_of(o + q * d.L)] = v[q];
+        } else {
+            const size_t base = (size_t) row * pl.n + o;
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                const int e = o + q * d.L;
+                if (CHIRP && e >= pl.n) break;
+                const size_t g = base + (size_t) q * d.L;
+                float2 u = v[q];
+                if (CHIRP) u = cmul(make_float2(u.y, u.x), __ldg(io.chirp + e));
+                u.x *= pl.scale; u.y *= pl.scale;
+                if (!EPI && io.accumulate) { u.x += io.yr[g]; u.y += io.yi[g]; }
+                io.yr[g] = u.x;
+                io.yi[g] = u.y;
+                if (EPI) {
+                    const float hr = __ldg(ep.hr + e), hi = __ldg(ep.hi + e);
+                    const float gr = cnb_gelu(u.x * hr - u.y * hi), gi = cnb_gelu(u.x * hi + u.y * hr);
+                    const size_t at = (io.row0 + row) * (size_t) pl.n + e;
+                    if (ep.gr) { ep.gr[at] = gr; ep.gi[at] = gi; }
+                    if (ep.sp) {
+                        const size_t so = (io.row0 + row) * (size_t) ep.pitch + e;
+                        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 0), so, gr);
+                        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 1), so, gi);
+                    }
+                }
+            }
+        }
+    }
+}
+
+template <bool EPI, bool CHIRP>
+__global__ void __launch_bounds__(MAX_THREADS, 2)
+fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* yr, float* yi,
+            const float2* __restrict__ tw, const float2* __restrict__ chirp, const float2* __restrict__ spectrum, int B,
+            int accumulate, const FftEpilogue ep, const __grid_constant__ MixedPlan pl) {
+    cnb_pdl_enter();
+    extern __shared__ __align__(16) float2 bufs[];
+    Io io;
+    io.row0 = (size_t) blockIdx.x * pl.rows;
+    io.rows = min(pl.rows, B - (int) io.row0);
+    io.xr = xr + io.row0 * pl.n; io.xi = xi + io.row0 * pl.n;
+    io.yr = yr + io.row0 * pl.n; io.yi = yi + io.row0 * pl.n;
+    io.tw = tw; io.chirp = chirp; io.spectrum = spectrum;
+    io.accumulate = accumulate;
+    const int total = CHIRP ? 2 * pl.passes : pl.passes;
+    for (int s = 0; s < total; ++s) {
+        const Pass& d = pl.p[CHIRP && s >= pl.passes ? s - pl.passes : s];
+        io.src = s == 0 ? nullptr : bufs + (s & 1 ? 0 : pl.rows * pl.stride);
+        io.dst = s == total - 1 ? nullptr : bufs + (s & 1 ? pl.rows * pl.stride : 0);
+        io.spectral = CHIRP && s == pl.passes;
+        switch (d.radix) {
+#define CNB_RADIX(R) case R: run_pass<R, EPI, CHIRP>(pl, d, io, ep); break
+            CNB_RADIX(2); CNB_RADIX(3); CNB_RADIX(4); CNB_RADIX(5); CNB_RADIX(6); CNB_RADIX(7); CNB_RADIX(8); CNB_RADIX(9);
+            CNB_RADIX(10); CNB_RADIX(11); CNB_RADIX(12); CNB_RADIX(13); CNB_RADIX(14); CNB_RADIX(15); CNB_RADIX(16);
+#undef CNB_RADIX
+        }
+        if (s < total - 1) __syncthreads();
+    }
+}
+
+// twiddles of every pass, packed as Pass::tw says, in double
+__global__ void mixed_twiddle_k(float2* __restrict__ tw, const __grid_constant__ MixedPlan pl) {
+    for (int p = 0; p < pl.passes; ++p) {
+        const Pass d = pl.p[p];
+        if (d.L == 1) continue;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (d.radix - 1) * d.L; i += gridDim.x * blockDim.x) {
+            const int q = i / d.L + 1, k = i % d.L;
+            double s, c;
+            sincospi(-2.0 * (double) (k * q) / ((double) d.L * d.radix), &s, &c);
+            tw[d.tw + i] = make_float2((float) c, (float) s);
+        }
+    }
+}
+
+// chirp[n] = e^{-pi i n^2 / N}; spectrum = DFT_M of b, b[n] = b[M - n] = conj(chirp[n]) for n < N, 0 between, over M
+__global__ void mixed_chirp_k(float2* __restrict__ chirp, float2* __restrict__ spectrum, int N, int M) {
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+        double s, c;
+        sincospi((double) ((long) i * i % (2L * N)) / N, &s, &c);
+        chirp[i] = make_float2((float) c, (float) -s);
+    }
+    for (int k = warp; k < M; k += warps) {
+        double re = 0.0, im = 0.0;
+        for (int n = 1 + lane; n < N; n += 32) {           // b is even: 2 sum b[n] cos(2 pi n k / M)
+            double s, c;
+            sincospi((double) ((long) n * n % (2L * N)) / N, &s, &c);
+            const double t = 2.0 * cospi(2.0 * (double) ((long) n * k % M) / M);
+            re += c * t; im += s * t;
+        }
+        for (int o = 16; o > 0; o >>= 1) { re += __shfl_xor_sync(0xffffffffu, re, o); im += __shfl_xor_sync(0xffffffffu, im, o); }
+        if (lane == 0) spectrum[k] = make_float2((float) ((re + 1.0) / M), (float) (im / M));
+    }
+}
+
+// ------------------------------------------------------------------------------------------------------- plans
+unsigned reciprocal(int d) { return d == 1 ? 0u : (unsigned) ((1ull << 32) / (unsigned) d + 1); }
+
+// Work of a butterfly of R points in the units of an element's trip through shared memory: primes cost their
+// square, and every butterfly some index arithmetic.
+double butterfly_cost(int r) {
+    const int p = r % 13 == 0 ? 13 : r % 11 == 0 ? 11 : r % 7 == 0 ? 7 : r % 5 == 0 ? 5 : 2;
+    return 4.0 + r * (1.0 + 0.04 * p);
+}
+
+// every factorisation of m into exactly `left` radices, non-increasing
+void factorisations(int m, int left, int most, std::vector<int>& cur, std::vector<std::vector<int> >& out) {
+    if (left == 0) { if (m == 1) out.push_back(cur); return; }
+    for (int r = std::min(most, 16); r >= 2; --r) {
+        if (m % r) continue;
+        cur.push_back(r);
+        factorisations(m / r, left - 1, r, cur, out);
+        cur.pop_back();
+    }
+}
+
+// The radices of a transform of length m, or false when a prime factor exceeds 13.  Of the factorisations with the
+// fewest passes the one of least work; the largest radix goes into the middle, where consecutive threads need not
+// touch consecutive elements of the planes (narrow first and last passes keep those runs long).
+bool choose_radices(int m, std::vector<int>* radices, double* cost) {
+    for (int n = 1; n <= MAX_PASSES; ++n) {
+        std::vector<int> cur;
+        std::vector<std::vector<int> > all;
+        factorisations(m, n, 16, cur, all);
+        if (all.empty()) continue;
+        double best = 1e30;
+        for (auto& f : all) {
+            double c = 0;
+            for (int r : f) c += butterfly_cost(r) / r;
+            if (c < best) { best = c; *radices = f; }
+        }
+        if (radices->size() > 2) std::swap((*radices)[0], (*radices)[1]);
+        *cost = best * m;
+        return true;
+    }
+    return false;
+}
+
+size_t smem_bytes(int m, int rows, int buffers) { return (size_t) buffers * rows * (pad_of(m) + 1) * sizeof(float2); }
+
+int buffers_for(int passes, bool chirp) {
+    const int hops = (chirp ? 2 * passes : passes) - 1;     // passes that write shared memory
+    return hops > 1 ? 2 : hops;
+}
+
+// The length-dependent part of a plan; false: this length has no kernel here.
+bool plan_length(int N, MixedPlan* out) {
+    if (N < 2) return false;
+    std::vector<int> radices, r;
+    double cost = 0, c;
+    int m = N;
+    if (!choose_radices(N, &radices, &cost)) {
+        // chirp: of the lengths up to a fifth above the least one, the cheapest
+        cost = 1e30;
+        const int least = 2 * N - 1;
+        for (int t = least; t <= least + std::max(8, least / 5); ++t)
+            if (choose_radices(t, &r, &c) && c < cost) { cost = c; m = t; radices = r; }
+        if (radices.empty()) return false;
+    }
+    MixedPlan pl = {};
+    pl.n = N; pl.m = m;
+    pl.passes = (int) radices.size();
+    pl.stride = pad_of(m) + 1;
+    pl.buffers = buffers_for(pl.passes, m > N);
+    if (smem_bytes(m, 1, pl.buffers) > MAX_SMEM) return false;
+    int L = 1, tw = 0;
+    for (int p = 0; p < pl.passes; ++p) {
+        Pass& d = pl.p[p];
+        d.radix = radices[p]; d.L = L; d.nb = m / radices[p];
+        d.mag_nb = reciprocal(d.nb); d.mag_L = reciprocal(d.L);
+        d.tw = tw;
+        if (L > 1) tw += (d.radix - 1) * L;
+        L *= d.radix;
+    }
+    pl.scale = (float) (1.0 / std::sqrt((double) N));
+    *out = pl;
+    return true;
+}
+
+bool cached_plan(int N, MixedPlan* out) {
+    static std::mutex mu;
+    static std::map<int, MixedPlan> plans;                  // at most one entry per length; n = 0: no kernel
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = plans.find(N);
+    if (it == plans.end()) {
+        MixedPlan pl = {};
+        if (!plan_length(N, &pl)) pl.n = 0;
+        it = plans.emplace(N, pl).first;
+    }
+    *out = it->second;
+    return out->n != 0;
+}
+
+// Rows per CTA and threads: about four CTAs to an SM (up to 52 KB of shared memory each), so that some load or store
+// while others transform; rows are spread over the SMs first when the batch is small; of the thread counts the one
+// that wastes the fewest lanes over the passes.
+void plan_batch(MixedPlan* pl, int B, int sms) {
+    const size_t budget = 52 * 1024;
+    int rows = 1;
+    while (rows < 64 && smem_bytes(pl->m, rows + 1, std::max(1, pl->buffers)) <= budget && (long) (rows + 1) * pl->m <= 4096) ++rows;
+    rows = std::max(1, std::min(rows, (B + 2 * sms - 1) / (2 * sms)));
+    double best = 1e30;
+    for (int t = 64; t <= MAX_THREADS; t += 32) {
+        double c = 0;
+        for (int p = 0; p < pl->passes; ++p) {
+            const int items = rows * pl->p[p].nb;
+            c += (double) ((items + t - 1) / t) * butterfly_cost(pl->p[p].radix);
+        }
+        c *= t + 32;                                        // lanes held, and a little for every CTA
+        if (c < best * 0.999) { best = c; pl->threads = t; }
+    }
+    pl->rows = rows;
+}
+
+size_t table_entries(const MixedPlan& pl) {
+    size_t n = 0;
+    for (int p = 0; p < pl.passes; ++p) if (pl.p[p].L > 1) n += (size_t) (pl.p[p].radix - 1) * pl.p[p].L;
+    if (pl.m > pl.n) n += (size_t) pl.n + pl.m;
+    return std::max<size_t>(n, 1);
+}
+
+}  // namespace
+
+namespace cnb {
+
+bool fft_mixed_supported(int N) {
+    MixedPlan pl;
+    return cached_plan(N, &pl);
+}
+
+int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, int B, int N, int inverse,
+              int accumulate, const FftEpilogue& ep, cudaStream_t st) {
+    MixedPlan pl;
+    if (!cached_plan(N, &pl)) return set_error(CNB_ERR_UNSUPPORTED, "fft: N=%d", N);
+    plan_batch(&pl, B, usable_sms(ctx));
+    const bool chirp = pl.m > pl.n;
+    // the tables live in the arena; the map key -N keeps them apart from DFT matrices
+    cnb_twiddle t;
+    auto it = ctx->twiddles.find(-N);
+    const size_t entries = table_entries(pl), tw_entries = entries - (chirp ? (size_t) pl.n + pl.m : 0);
+    if (it == ctx->twiddles.end()) {
+        void* p = nullptr;
+        int rc = cnb_alloc(ctx, entries * sizeof(float2), &p);
+        if (rc != CNB_OK) return rc;
+        t.re = static_cast<float*>(p);
+        float2* tab = static_cast<float2*>(p);
+        mixed_twiddle_k<<<16, 256, 0, st>>>(tab, pl);
+        CNB_LAUNCH_CHECK("mixed_twiddle");
+        if (chirp) {
+            mixed_chirp_k<<<ctx->sm_count * 4, 256, 0, st>>>(tab + tw_entries, tab + tw_entries + pl.n, pl.n, pl.m);
+            CNB_LAUNCH_CHECK("mixed_chirp");
+        }
+        ctx->twiddles[-N] = t;
+    } else {
+        t = it->second;
+    }
+    const float2* tw = reinterpret_cast<const float2*>(t.re);
+    const float2* ch = tw + tw_entries;
+    const float2* spec = ch + pl.n;
+    if (inverse) { std::swap(xr, xi); std::swap(yr, yi); }
+    const size_t smem = smem_bytes(pl.m, pl.rows, pl.buffers);
+    const int form = (ep.hr ? 2 : 0) + (chirp ? 1 : 0);
+    static bool attr_done[64] = {};                         // the attribute is per device
+    if (!attr_done[ctx->device & 63]) {
+        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));
+        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));
+        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));
+        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));
+        attr_done[ctx->device & 63] = true;
+    }
+    const dim3 grid((unsigned) ((B + pl.rows - 1) / pl.rows)), block((unsigned) pl.threads);
+#define CNB_MIXED(E, C) CNB_CUDA(cnb::launch(fft_mixed_k<E, C>, grid, block, smem, st, 1, xr, xi, yr, yi, tw, ch, spec, B, accumulate, ep, pl))
+    switch (form) {
+        case 0: CNB_MIXED(false, false); break;
+        case 1: CNB_MIXED(false, true); break;
+        case 2: CNB_MIXED(true, false); break;
+        default: CNB_MIXED(true, true); break;
+    }
+#undef CNB_MIXED
+    CNB_LAUNCH_CHECK("fft_mixed");
+    return CNB_OK;
+}
+
+}  // namespace cnb
+
+extern "C" int cnb_fft_plan(int N, int B, int sm_count, int* out, int capacity) {
+    MixedPlan pl;
+    if (!out || capacity < 6 + MAX_PASSES || N < 1 || B < 1 || sm_count < 1)
+        return cnb::set_error(CNB_ERR_ARG, "cnb_fft_plan: N=%d B=%d", N, B);
+    if (!cached_plan(N, &pl)) return 0;
+    plan_batch(&pl, B, sm_count);
+    out[0] = pl.m; out[1] = pl.rows; out[2] = pl.threads; out[3] = pl.buffers; out[4] = pl.stride;
+    out[5] = (int) smem_bytes(pl.m, pl.rows, pl.buffers);
+    for (int p = 0; p < pl.passes; ++p) out[6 + p] = pl.p[p].radix;
+    return pl.passes;
+}

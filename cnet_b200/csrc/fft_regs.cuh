@@ -50,6 +50,7 @@ struct FftEpilogue {
     float* gi = nullptr;
     float* sp = nullptr;            // operand split of that (a split buffer with plane pitch np) or NULL
     size_t np = 0;
+    size_t pitch = 0;               // elements from one row of the split to the next
 };
 
 }  // namespace cnb_fft
@@ -60,4 +61,8 @@ namespace cnb {
 // predecessor, so that one launch must be fully serialised)
 int fft1024_pipe(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, const float2* tw, int B,
                  int inverse, int accumulate, const cnb_fft::FftEpilogue& ep, cudaStream_t st, bool fresh_table);
+// any length with a plan: mixed radices or the chirp form; planes of any alignment
+bool fft_mixed_supported(int N);
+int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, int B, int N, int inverse,
+              int accumulate, const cnb_fft::FftEpilogue& ep, cudaStream_t st);
 }  // namespace cnb

@@ -30,6 +30,8 @@ __global__ void tri_mask_k(float* __restrict__ fr, float* __restrict__ fi, int N
         if ((int) (i % N) > (int) (i / N)) { fr[i] = 0.f; fi[i] = 0.f; }
 }
 
+int fft_engine(int N) { return N == 256 || N == 1024 || N == 4096 ? 3 : 5; }
+
 const int kTriKey = 1 << 28;    // twiddle-cache key offset of the triangular matrices
 
 int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) {
@@ -148,7 +150,7 @@ int cnb_dft_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im, float* y_re,
     CNB_CHECK_ARG(ctx && x_re && x_im && y_re && y_im, "cnb_dft_fwd: null pointer");
     CNB_CHECK_ARG(B > 0 && N > 0 && N <= 16384, "cnb_dft_fwd: B=%d N=%d (N <= 16384)", B, N);
     if (cnb::fft_supported(N) && !ctx->force_dft_gemm) {
-        cnb::g_last_engine = 3;
+        cnb::g_last_engine = fft_engine(N);
         return cnb::fft_run(ctx, x_re, x_im, y_re, y_im, B, N, 0, 0, cnb::S(stream));
     }
     cnb_twiddle t;
@@ -163,7 +165,7 @@ int cnb_dft_bwd(cnb_ctx* ctx, const float* g_re, const float* g_im, float* dx_re
     CNB_CHECK_ARG(B > 0 && N > 0 && N <= 16384, "cnb_dft_bwd: B=%d N=%d (N <= 16384)", B, N);
     cudaStream_t st = cnb::S(stream);
     if (cnb::fft_supported(N) && !ctx->force_dft_gemm) {
-        cnb::g_last_engine = 3;
+        cnb::g_last_engine = fft_engine(N);
         return cnb::fft_run(ctx, g_re, g_im, dx_re, dx_im, B, N, 1, accumulate, st);
     }
     cnb_twiddle t;
@@ -245,7 +247,7 @@ int cnb_dft_hadamard_gelu_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im
     CNB_CHECK_ARG((y_re == nullptr) == (y_im == nullptr) && (y_re || y_split),
                   "cnb_dft_hadamard_gelu_fwd: y planes must be a pair, and may only be left out when y_split is given");
     CNB_CHECK_ARG(B > 0 && cnb::fft_supported(N), "cnb_dft_hadamard_gelu_fwd: B=%d, N=%d is not an FFT-kernel length", B, N);
-    cnb::g_last_engine = 3;
+    cnb::g_last_engine = fft_engine(N);
     return cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, y_split, B, N, cnb::S(stream));
 }
 

@@ -63,6 +63,7 @@ SIGNATURES = {
     "cnb_l2out_fwd_bwd": (C.c_int, [_vp] + [_P] * 5 + [C.c_int] * 2 + [_vp]),
     "cnb_adam_update": (C.c_int, [_vp, _P, _P, _P, _sz, C.c_float, C.c_float, C.c_int, _vp]),
     "cnb_set_dft_engine": (C.c_int, [_vp, C.c_int]),
+    "cnb_fft_plan": (C.c_int, [C.c_int] * 3 + [C.POINTER(C.c_int), C.c_int]),
     "cnb_hadamard_fwd": (C.c_int, [_vp] + [_P] * 4 + [C.c_int] + [_P] * 2 + [C.c_int] * 2 + [_vp]),
     "cnb_hadamard_bwd": (C.c_int, [_vp] + [_P] * 6 + [C.c_int] + [_P] * 2 + [C.c_int] + [_P] * 2 + [C.c_int] * 3 + [_vp]),
     "cnb_hadamard_bwd_static": (C.c_int, [_P] * 8 + [C.c_int] + [_P] * 2 + [C.c_int] * 3 + [_vp]),

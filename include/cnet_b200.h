@@ -145,9 +145,9 @@ int cnb_dft_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im,
  * CPU: impl/ft.h:57-80. */
 int cnb_dft_bwd(cnb_ctx* ctx, const float* g_re, const float* g_im,
                 float* dx_re, float* dx_im, int B, int N, int accumulate, void* stream);
-/* FourierTrans -> Hadamard(shared h) -> CGelu in one pass over the row (N = 256, 1024, 4096, see
+/* FourierTrans -> Hadamard(shared h) -> CGelu in one pass over the row (the N that have an FFT kernel, see
  * cnb_dft_fused_ok): u = DFT(x) is kept for the backward, y = gelu(u o h), optionally with the
- * operand split of y for the Linear that follows; y_re = y_im = NULL is allowed when y_split
+ * operand split of y for the Linear that follows (rows at a pitch of N rounded up to 64); y_re = y_im = NULL is allowed when y_split
  * is given (hi + l16 of the split is y to 2^-19, all the product sees of it, so a caller that only feeds the
  * Linear need not store y twice).
  * The Hadamard product a = u o h is not stored: cnb_hadamard_gelu_bwd recomputes it when a_re == NULL.  Same reference kernels as
@@ -165,10 +165,16 @@ int cnb_tdft_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im,
                  float* y_re, float* y_im, int B, int N, void* stream);
 int cnb_tdft_bwd(cnb_ctx* ctx, const float* g_re, const float* g_im,
                  float* dx_re, float* dx_im, int B, int N, int accumulate, void* stream);
-/* N = 256, 1024, 4096 run as a shared-memory FFT (one read + one write of the tensor); any other
- * N, or every N after cnb_set_dft_engine(ctx, 1), as a complex GEMM against the twiddle matrix.
- * cnb_last_gemm_engine() reports 3 after an FFT-kernel call. */
+/* Every N whose rows fit shared memory runs as a shared-memory FFT (one read + one write of the tensor): all up to
+ * 6000 or so, longer ones without a prime factor above 13; the rest, or every N after cnb_set_dft_engine(ctx, 1), as
+ * a complex GEMM against the twiddle matrix.  cnb_last_gemm_engine() reports 3 after an FFT-kernel call with
+ * N = 256, 1024 or 4096 and 5 with another N. */
 int cnb_set_dft_engine(cnb_ctx* ctx, int force_gemm);
+/* How the mixed-radix kernel would take B rows of length N on a device of sm_count SMs (host arithmetic only, no
+ * reference counterpart; for tests and tuning).  Returns the number of passes, 0 when N has no such kernel, and
+ * out = {transform length (> N: the chirp form), rows per CTA, threads, shared-memory buffers, elements per row of a
+ * buffer, shared-memory bytes, radix of every pass}; capacity >= 12. */
+int cnb_fft_plan(int N, int B, int sm_count, int* out, int capacity);
 
 /* --------------------------------------------------------- element-wise layers
  * Hadamard y = u o v; v is one vector [N] shared by the batch (v_batched = 0) or [B,N].
