@@ -338,6 +338,31 @@ __device__ __forceinline__ float4 ld_global_now(const float* p) {
     return v;
 }
 
+__device__ __forceinline__ float ld_global_now1(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+// Four consecutive floats of a row of which `left` (>= 1) remain: one 16-byte access, or (VEC = false: rows at any
+// 4-byte alignment, ragged ends) up to four single ones.
+template <bool VEC> __device__ __forceinline__ float4 ld_global_part(const float* p, int left) {
+    if constexpr (VEC) return ld_global_now(p);
+    float4 v = make_float4(ld_global_now1(p), 0.f, 0.f, 0.f);
+    if (left > 1) v.y = ld_global_now1(p + 1);
+    if (left > 2) v.z = ld_global_now1(p + 2);
+    if (left > 3) v.w = ld_global_now1(p + 3);
+    return v;
+}
+
+template <bool VEC> __device__ __forceinline__ void st_global_part(float* p, int left, float4 v) {
+    if constexpr (VEC) { *reinterpret_cast<float4*>(p) = v; return; }
+    p[0] = v.x;
+    if (left > 1) p[1] = v.y;
+    if (left > 2) p[2] = v.z;
+    if (left > 3) p[3] = v.w;
+}
+
 // all threads of all CTAs of the cluster; orders shared-memory writes before the peers' reads
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -359,9 +384,9 @@ __device__ __forceinline__ float4 ld_peer(uint32_t local_addr, uint32_t rank) {
 // residual, old D) is issued before the first sum, so a round costs one round trip.  Fixed summation order.
 // The CL partial tiles sit in the CTAs of cluster rank peer0 + c * peer_step (one CTA per tile: 0 and 1; CTA pairs:
 // this CTA's rank in its pair and 2: the peers are the CTAs that hold the same 128 rows).
-template <int CL>
+template <int CL, bool VEC>
 __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_base, uint32_t crank, int m0, int n0,
-                                               int et, bool vec_ok, uint32_t peer0, uint32_t peer_step) {
+                                               int et, uint32_t peer0, uint32_t peer_step) {
     constexpr int ROWS = BM / CL;
     constexpr int U = CL <= 4 ? 2 : 1;                   // chunks per thread and round
     for (int base = et; base < ROWS * 32; base += 128 * U) {
@@ -385,13 +410,11 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
                 const uint32_t peer = peer0 + (uint32_t) c * peer_step;
                 xr[u][c] = ld_peer(local, peer); xi[u][c] = ld_peer(local + PART_PLANE_BYTES, peer);
             }
-            if (vec_ok) {
-                if (p.r_re) { vr[u] = ld_global_now(p.r_re + o[u]); vi[u] = ld_global_now(p.r_im + o[u]); }
-                if (p.accumulate) {
-                    const float4 dr = ld_global_now(p.d_re + o[u]), di = ld_global_now(p.d_im + o[u]);
-                    vr[u].x += dr.x; vr[u].y += dr.y; vr[u].z += dr.z; vr[u].w += dr.w;
-                    vi[u].x += di.x; vi[u].y += di.y; vi[u].z += di.z; vi[u].w += di.w;
-                }
+            if (p.r_re) { vr[u] = ld_global_part<VEC>(p.r_re + o[u], p.N - gn[u]); vi[u] = ld_global_part<VEC>(p.r_im + o[u], p.N - gn[u]); }
+            if (p.accumulate) {
+                const float4 dr = ld_global_part<VEC>(p.d_re + o[u], p.N - gn[u]), di = ld_global_part<VEC>(p.d_im + o[u], p.N - gn[u]);
+                vr[u].x += dr.x; vr[u].y += dr.y; vr[u].z += dr.z; vr[u].w += dr.w;
+                vi[u].x += di.x; vi[u].y += di.y; vi[u].z += di.z; vi[u].w += di.w;
             }
         }
 #pragma unroll
@@ -403,20 +426,10 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
                 sr.x += xr[u][c].x; sr.y += xr[u][c].y; sr.z += xr[u][c].z; sr.w += xr[u][c].w;
                 si.x += xi[u][c].x; si.y += xi[u][c].y; si.z += xi[u][c].z; si.w += xi[u][c].w;
             }
-            if (vec_ok) {
-                vr[u].x += sr.x; vr[u].y += sr.y; vr[u].z += sr.z; vr[u].w += sr.w;
-                vi[u].x += si.x; vi[u].y += si.y; vi[u].z += si.z; vi[u].w += si.w;
-                *reinterpret_cast<float4*>(p.d_re + o[u]) = vr[u];
-                *reinterpret_cast<float4*>(p.d_im + o[u]) = vi[u];
-            } else {
-                const float wr[4] = {sr.x, sr.y, sr.z, sr.w}, wi[4] = {si.x, si.y, si.z, si.w};
-                for (int k = 0; k < 4 && gn[u] + k < p.N; ++k) {
-                    float ar = wr[k], ai = wi[k];
-                    if (p.r_re) { ar += p.r_re[o[u] + k]; ai += p.r_im[o[u] + k]; }
-                    if (p.accumulate) { ar += p.d_re[o[u] + k]; ai += p.d_im[o[u] + k]; }
-                    p.d_re[o[u] + k] = ar; p.d_im[o[u] + k] = ai;
-                }
-            }
+            vr[u].x += sr.x; vr[u].y += sr.y; vr[u].z += sr.z; vr[u].w += sr.w;
+            vi[u].x += si.x; vi[u].y += si.y; vi[u].z += si.z; vi[u].w += si.w;
+            st_global_part<VEC>(p.d_re + o[u], p.N - gn[u], vr[u]);
+            st_global_part<VEC>(p.d_im + o[u], p.N - gn[u], vi[u]);
         }
     }
 }
@@ -429,7 +442,9 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 #define CNB_GSTAMP(k, cond) do { } while (0)
 #endif
 
-template <bool PAIR>
+// VEC: rows of D and R are 16-byte aligned (N % 4 == 0); the form without it writes 32 consecutive floats of a row per
+// warp instruction instead of four 16-byte pieces of four rows.
+template <bool PAIR, bool VEC>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ CUtensorMap a_hi_im,
            const __grid_constant__ CUtensorMap a_h16, const __grid_constant__ CUtensorMap a_l16,
@@ -692,9 +707,6 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
         const int et = (warp - 2) * 32 + lane;       // 0..127 within the epilogue group
         const uint32_t tl = tmem_base + ((uint32_t) (q * 32) << 16);
         const float sgn = p.conjB ? 1.f : -1.f;
-        const bool vec_ok = (p.N % 4 == 0) &&
-            ((reinterpret_cast<uintptr_t>(p.d_re) | reinterpret_cast<uintptr_t>(p.d_im) |
-              reinterpret_cast<uintptr_t>(p.r_re) | reinterpret_cast<uintptr_t>(p.r_im)) & 15) == 0;
         int seg = 0;
         if (split_cluster) {
             // the whole k-slice is one segment; its partial sums go to shared memory for the cluster reduction
@@ -752,7 +764,7 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
             if (*abort_flag) { live = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool need_old = !partial && p.accumulate;
-            const bool pre = vec_ok && (add_res || need_old);
+            const bool pre = VEC && (add_res || need_old);
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 // What the write-out of this round adds from global memory (residual, old D) is requested
@@ -814,17 +826,17 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
                     if constexpr (PAIR) mbar_arrive_cluster(map_to_rank(acc_empty, lead_rank));   // the first CTA's MMA thread waits for both
                     else mbar_arrive(acc_empty);
                 }
-                // coalesced write-out: each warp instruction covers 4 rows x 128 contiguous bytes
+                if constexpr (VEC) {
+                    // coalesced write-out: each warp instruction covers 4 rows x 128 contiguous bytes
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    int idx = et + 128 * j;
-                    int r = idx >> 3, ch = idx & 7;
-                    int gm = m0 + r, gn = n0 + c0 + ch * 4;
-                    if (gm >= p.M || gn >= p.N) continue;
-                    float4 vr = *reinterpret_cast<const float4*>(stage_re + stage_off(r, ch));
-                    float4 vi = *reinterpret_cast<const float4*>(stage_im + stage_off(r, ch));
-                    size_t o = (size_t) gm * p.N + gn;
-                    if (vec_ok) {
+                    for (int j = 0; j < 8; ++j) {
+                        int idx = et + 128 * j;
+                        int r = idx >> 3, ch = idx & 7;
+                        int gm = m0 + r, gn = n0 + c0 + ch * 4;
+                        if (gm >= p.M || gn >= p.N) continue;
+                        float4 vr = *reinterpret_cast<const float4*>(stage_re + stage_off(r, ch));
+                        float4 vi = *reinterpret_cast<const float4*>(stage_im + stage_off(r, ch));
+                        size_t o = (size_t) gm * p.N + gn;
                         if (pre) {
                             vr.x += gr[j].x; vr.y += gr[j].y; vr.z += gr[j].z; vr.w += gr[j].w;
                             vi.x += gi[j].x; vi.y += gi[j].y; vi.z += gi[j].z; vi.w += gi[j].w;
@@ -841,16 +853,32 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
                             *reinterpret_cast<float4*>(p.d_re + o) = vr;
                             *reinterpret_cast<float4*>(p.d_im + o) = vi;
                         }
-                    } else {
-                        float wr[4] = {vr.x, vr.y, vr.z, vr.w}, wi[4] = {vi.x, vi.y, vi.z, vi.w};
-                        for (int k = 0; k < 4 && gn + k < p.N; ++k) {
-                            float xr = wr[k], xi = wi[k];
-                            if (add_res) { xr += p.r_re[o + k]; xi += p.r_im[o + k]; }
-                            if (partial) { atomicAdd(p.d_re + o + k, xr); atomicAdd(p.d_im + o + k, xi); }
-                            else {
-                                if (p.accumulate) { xr += p.d_re[o + k]; xi += p.d_im[o + k]; }
-                                p.d_re[o + k] = xr; p.d_im[o + k] = xi;
-                            }
+                    }
+                } else {
+                    // a warp takes 32 rows, one row's 32 floats per instruction; what is added to eight rows is
+                    // requested before the first of them is stored
+                    const int gn = n0 + c0 + lane;
+#pragma unroll 1
+                    for (int r0 = q * 32; r0 < q * 32 + 32; r0 += 8) {
+                        float ar[8], ai[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int gm = m0 + r0 + j;
+                            const size_t o = (size_t) gm * p.N + gn;
+                            const bool on = gm < p.M && gn < p.N;
+                            ar[j] = ai[j] = 0.f;
+                            if (on && add_res) { ar[j] = ld_global_now1(p.r_re + o); ai[j] = ld_global_now1(p.r_im + o); }
+                            if (on && need_old) { ar[j] += ld_global_now1(p.d_re + o); ai[j] += ld_global_now1(p.d_im + o); }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int gm = m0 + r0 + j;
+                            if (gm >= p.M || gn >= p.N) continue;
+                            const size_t o = (size_t) gm * p.N + gn;
+                            const int at = stage_off(r0 + j, lane >> 2) + (lane & 3);
+                            const float vr = stage_re[at] + ar[j], vi = stage_im[at] + ai[j];
+                            if (partial) { atomicAdd(p.d_re + o, vr); atomicAdd(p.d_im + o, vi); }
+                            else { p.d_re[o] = vr; p.d_im[o] = vi; }
                         }
                     }
                 }
@@ -876,13 +904,10 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
             const int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
             const int et = (warp - 2) * 32 + lane;
             const uint32_t peer0 = PAIR ? prank : 0u, peer_step = PAIR ? 2u : 1u;
-            const bool vec_ok = (p.N % 4 == 0) &&
-                ((reinterpret_cast<uintptr_t>(p.d_re) | reinterpret_cast<uintptr_t>(p.d_im) |
-                  reinterpret_cast<uintptr_t>(p.r_re) | reinterpret_cast<uintptr_t>(p.r_im)) & 15) == 0;
             switch (p.cluster) {
-                case 2: cluster_reduce<2>(p, smem_base, crank, m0, n0, et, vec_ok, peer0, peer_step); break;
-                case 4: cluster_reduce<4>(p, smem_base, crank, m0, n0, et, vec_ok, peer0, peer_step); break;
-                default: cluster_reduce<8>(p, smem_base, crank, m0, n0, et, vec_ok, peer0, peer_step); break;
+                case 2: cluster_reduce<2, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+                case 4: cluster_reduce<4, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+                default: cluster_reduce<8, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
             }
         }
         CNB_GSTAMP(7, threadIdx.x == 64);
@@ -913,26 +938,27 @@ __global__ void split_k(const float* __restrict__ s0, const float* __restrict__ 
     }
 }
 
-// the same, transposed while it is split ([R,C] -> [C,R])
-__global__ void split_transpose_k(const float* __restrict__ s0, const float* __restrict__ s1,
-                                  float* __restrict__ sp, size_t np, int R, int C) {
+// The same, from rows of `cols` floats at any 4-byte alignment to rows at `pitch` (a multiple of 4): a thread takes four
+// columns of a row, loads what there is of them and stores 16 and 8 bytes (the row's last group past `cols` too).
+__global__ void split_rows_k(const float* __restrict__ s0, const float* __restrict__ s1, float* __restrict__ sp, size_t np,
+                             int rows, int cols, int pitch) {
     cnb_pdl_enter();
-    __shared__ float t0[32][33], t1[32][33];
     const cnb_split_dst d0 = cnb_split_component(sp, np, 0), d1 = cnb_split_component(sp, np, 1);
-    int c = blockIdx.x * 32 + threadIdx.x;
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        int r = blockIdx.y * 32 + k;
-        if (r < R && c < C) { t0[k][threadIdx.x] = s0[(size_t) r * C + c]; t1[k][threadIdx.x] = s1[(size_t) r * C + c]; }
-    }
-    __syncthreads();
-    int r = blockIdx.y * 32 + threadIdx.x;
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        int cc = blockIdx.x * 32 + k;
-        if (r < R && cc < C) {
-            size_t o = (size_t) cc * R + r;
-            cnb_split_store1(d0, o, t0[threadIdx.x][k]);
-            cnb_split_store1(d1, o, t1[threadIdx.x][k]);
+    const int groups = (cols + 3) / 4;
+    const size_t total = (size_t) rows * groups;
+    for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t) gridDim.x * blockDim.x) {
+        const int row = (int) (i / groups), c = (int) (i - (size_t) row * groups) * 4;
+        const float* p = s0 + (size_t) row * cols + c;
+        const float* r = s1 + (size_t) row * cols + c;
+        float x[4], y[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool on = c + k < cols;
+            x[k] = on ? p[k] : 0.f; y[k] = on ? r[k] : 0.f;
         }
+        const size_t o = (size_t) row * pitch + c;
+        cnb_split_store4(d0, o, x[0], x[1], x[2], x[3]);
+        cnb_split_store4(d1, o, y[0], y[1], y[2], y[3]);
     }
 }
 
@@ -954,12 +980,16 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
+// In every map `pitch` is the distance in elements between two stored rows (a multiple of 8: TMA wants a 16-byte row
+// pitch, of 64 for the MN-major forms) and may exceed their length; what lies between them is never used: a K-major
+// box beyond K is zero-filled, and operand rows beyond the last one only reach output columns or rows that do not exist.
+
 // [rows, K] fp32 row-major plane; box = BK x 128 rows; 64-byte swizzle; zero fill outside.
-int make_map(CUtensorMap* m, const float* base, int rows, int K) {
+int make_map(CUtensorMap* m, const float* base, int rows, int K, int pitch) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[2] = {(cuuint64_t) K, (cuuint64_t) rows};
-    cuuint64_t strides[1] = {(cuuint64_t) K * sizeof(float)};
+    cuuint64_t strides[1] = {(cuuint64_t) pitch * sizeof(float)};
     cuuint32_t box[2] = {(cuuint32_t) BK, 128u};
     cuuint32_t estr[2] = {1u, 1u};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr,
@@ -969,31 +999,31 @@ int make_map(CUtensorMap* m, const float* base, int rows, int K) {
     return CNB_OK;
 }
 
-// MN-major plane stored [K, rows] (rows contiguous, rows % 32 == 0), seen as [rows/32][K][32]:
+// MN-major plane stored [K, rows] (rows contiguous, pitch % 32 == 0), seen as [pitch/32][K][32]:
 // one box {32, BK, 4} brings four 32-row slabs of 16 k-lines, slab after slab (128-byte swizzle,
 // 32-byte atomicity).
-int make_map_mn(CUtensorMap* m, const float* base, int rows, int K) {
+int make_map_mn(CUtensorMap* m, const float* base, int K, int pitch) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[3] = {32u, (cuuint64_t) K, (cuuint64_t) (rows / 32)};
-    cuuint64_t strides[2] = {(cuuint64_t) rows * sizeof(float), 32u * sizeof(float)};
+    cuuint64_t dims[3] = {32u, (cuuint64_t) K, (cuuint64_t) (pitch / 32)};
+    cuuint64_t strides[2] = {(cuuint64_t) pitch * sizeof(float), 32u * sizeof(float)};
     cuuint32_t box[3] = {32u, (cuuint32_t) BK, 4u};
     cuuint32_t estr[3] = {1u, 1u, 1u};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for an MN-major [%d,%d] plane", (int) r, K, rows);
+    if (r != CUDA_SUCCESS) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for an MN-major [%d,%d] plane", (int) r, K, pitch);
     return CNB_OK;
 }
 
 // A pair of bf16 planes (real, imaginary; np elements apart), each [rows, K] row-major, seen as [2][rows][K]: one
 // box {BK, 128, 2} brings the 128 rows of both planes, real then imaginary (planes_per_box = 1: of one plane);
 // 32-byte swizzle.
-int make_map16(CUtensorMap* m, const void* base, int rows, int K, size_t np, unsigned planes_per_box) {
+int make_map16(CUtensorMap* m, const void* base, int rows, int K, int pitch, size_t np, unsigned planes_per_box) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[3] = {(cuuint64_t) K, (cuuint64_t) rows, 2u};
-    cuuint64_t strides[2] = {(cuuint64_t) K * 2u, (cuuint64_t) np * 2u};
+    cuuint64_t strides[2] = {(cuuint64_t) pitch * 2u, (cuuint64_t) np * 2u};
     cuuint32_t box[3] = {(cuuint32_t) BK, 128u, planes_per_box};
     cuuint32_t estr[3] = {1u, 1u, 1u};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
@@ -1003,19 +1033,19 @@ int make_map16(CUtensorMap* m, const void* base, int rows, int K, size_t np, uns
     return CNB_OK;
 }
 
-// The same pair stored [K, rows] (rows contiguous, rows % 64 == 0), seen as [2][rows/64][K][64]: one box
+// The same pair stored [K, rows] (rows contiguous, pitch % 64 == 0), seen as [2][pitch/64][K][64]: one box
 // {64, BK, 2, 2} brings two 64-row slabs of 16 k-lines of both planes, slab after slab (128-byte swizzle).
-int make_map16_mn(CUtensorMap* m, const void* base, int rows, int K, size_t np, unsigned planes_per_box) {
+int make_map16_mn(CUtensorMap* m, const void* base, int K, int pitch, size_t np, unsigned planes_per_box) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[4] = {64u, (cuuint64_t) K, (cuuint64_t) (rows / 64), 2u};
-    cuuint64_t strides[3] = {(cuuint64_t) rows * 2u, 128u, (cuuint64_t) np * 2u};
+    cuuint64_t dims[4] = {64u, (cuuint64_t) K, (cuuint64_t) (pitch / 64), 2u};
+    cuuint64_t strides[3] = {(cuuint64_t) pitch * 2u, 128u, (cuuint64_t) np * 2u};
     cuuint32_t box[4] = {64u, (cuuint32_t) BK, 2u, planes_per_box};
     cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for an MN-major bf16 [%d,%d] plane pair", (int) r, K, rows);
+    if (r != CUDA_SUCCESS) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for an MN-major bf16 [%d,%d] plane pair", (int) r, K, pitch);
     return CNB_OK;
 }
 
@@ -1109,6 +1139,10 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
             // against 0.025 at 512 x 1024 x 1024)
             for (int c = pair ? 2 : 8; c >= 2; c >>= 1)
                 if ((long) tiles * c <= sms && k_blocks / c >= 4) { q.cluster = c; break; }
+            // Long K over few tiles leaves the cluster form most of the device idle: 83 x 102 x 13688, one tile, ran
+            // 107 k-blocks on each of 8 CTAs (126 us) where stream-K runs are 8 k-blocks long.  The atomics and the
+            // cleared output of that form cost about as much as 16 k-blocks.
+            if (q.cluster > 1 && k_blocks / q.cluster > 2 * upc + 16) q.cluster = 1;
         }
         if (q.cluster > 1) { ctas = (long) tiles * q.cluster; upc = 0; }
         q.splits_tiles = q.cluster == 1 && (lead_whole ? upc > 0 : (q.segments > 0 || (upc % k_blocks) != 0));
@@ -1142,37 +1176,58 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
 namespace cnb {
 
 bool cgemm_tc_shape_ok(int M, int N, int K) {
-    // TMA needs a 16-byte row pitch (8 bf16); small or skinny problems are faster on the SIMT tiles
-    return (K % 8 == 0) && K >= 32 && M >= 64 && N >= 64;
+    if (K % 8 == 0 && K >= 32 && M >= 64 && N >= 64) return true;
+    // Other sizes pay a split pass to padded rows and a 128 x 128 tile that may be part empty: from about two million
+    // complex multiplications on that is less than what the fp32 SIMT tiles take (777 x 1001 x 1333: 330 against
+    // 45 us), below it the SIMT tiles win.
+    return K >= 48 && (double) M * N * K >= (double) (1 << 21);
+}
+
+static size_t padded(int n, int to) { return ((size_t) n + to - 1) / to * to; }
+
+// elements of an operand of `rows` x K as cgemm_tc_run stores it: K-major rows at a pitch of K rounded up to 8 (16 bytes
+// of bf16), or, from a source stored [K, rows], MN-major lines at a pitch of rows rounded up to 64
+static size_t operand_elems(int rows, int K, int trans) {
+    const size_t n = trans ? (size_t) K * padded(rows, 64) : (size_t) rows * padded(K, 8);
+    return (n + 63) & ~size_t(63);
 }
 
 size_t cgemm_tc_workspace_bytes(int M, int N, int K) {
-    return 4 * ((size_t) M * K + (size_t) N * K) * sizeof(float) + 4096;
+    const size_t a = std::max(operand_elems(M, K, 0), operand_elems(M, K, 1)), b = std::max(operand_elems(N, K, 0), operand_elems(N, K, 1));
+    return 4 * (a + b) * sizeof(float) + 4096;
 }
 
-void split_launch(cnb_ctx* ctx, const float* s0, const float* s1, float* sp, size_t np, size_t n, cudaStream_t st) {
-    size_t blocks = (n / 4 + 255) / 256 + 1, cap = (size_t) ctx->sm_count * 16;
-    cnb::launch(split_k, dim3((unsigned) (blocks < cap ? blocks : cap)), dim3(256), 0, st, 1, s0, s1, sp, np, n);
+static void split_launch(cnb_ctx* ctx, const float* s0, const float* s1, float* sp, size_t np, int rows, int cols, int pitch,
+                         cudaStream_t st) {
+    const bool aligned = ((reinterpret_cast<uintptr_t>(s0) | reinterpret_cast<uintptr_t>(s1)) & 15) == 0;
+    const size_t cap = (size_t) ctx->sm_count * 16;
+    if (aligned && pitch == cols) {                      // one run of rows * cols floats
+        const size_t n = (size_t) rows * cols, blocks = (n / 4 + 255) / 256 + 1;
+        cnb::launch(split_k, dim3((unsigned) std::min(blocks, cap)), dim3(256), 0, st, 1, s0, s1, sp, np, n);
+    } else {
+        const size_t blocks = ((size_t) rows * ((cols + 3) / 4) + 255) / 256;
+        cnb::launch(split_rows_k, dim3((unsigned) std::min(blocks, cap)), dim3(256), 0, st, 1, s0, s1, sp, np, rows, cols, pitch);
+    }
 }
 
-// The GEMM proper on operands that are already split: a[4] / b[4] = the four slots of a split buffer (hi_re,
-// hi_im, [h16_re ; h16_im], [l16_re ; l16_im]; slot q+1 follows slot q at the plane pitch), elements stored
-// [rows, K] (major = 0) or [K, rows] (major = 1, needs rows % 64 == 0).
-int cgemm_tc_presplit(cnb_ctx* ctx, const float* const a[4], int a_mn, const float* const b[4], int b_mn, int conjB,
+// The GEMM proper on operands that are already split: the four slots of a split buffer (hi_re, hi_im,
+// [h16_re ; h16_im], [l16_re ; l16_im]) lie plane_pitch floats apart, elements are stored [rows, K] (mn = 0) or
+// [K, rows] (mn = 1) with stored rows at `pitch`.
+int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b, int conjB,
                       const float* r_re, const float* r_im, float* d_re, float* d_im, int M, int N, int K,
                       int accumulate, cudaStream_t st) {
     static bool attr_set[64] = {};                       // the attribute is per device
     if (!attr_set[ctx->device & 63]) {
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         attr_set[ctx->device & 63] = true;
     }
     if ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im)) & 3)
         return set_error(CNB_ERR_ARG, "cgemm_tc: misaligned output");
-    if ((a_mn && M % 64) || (b_mn && N % 64))
-        return set_error(CNB_ERR_ARG, "cgemm_tc: an MN-major operand needs a multiple of 64 rows");
-    if ((!a_mn && K % 8) || (!b_mn && K % 8))
-        return set_error(CNB_ERR_ARG, "cgemm_tc: a K-major operand needs K %% 8 == 0");
+    if (a.pitch % (a.mn ? 64 : 8) || b.pitch % (b.mn ? 64 : 8))
+        return set_error(CNB_ERR_ARG, "cgemm_tc: operand pitches %d and %d", a.pitch, b.pitch);
     const Schedule q = choose_schedule(M, N, K, accumulate, ctx->sm_count, ctx->gemm_cta_limit);
     const bool pair = q.pair;
     const long ctas = q.ctas, upc = q.upc;
@@ -1180,18 +1235,16 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const float* const a[4], int a_mn, const flo
 
     int rc;
     alignas(64) CUtensorMap maps[8];
-    const size_t npa = (size_t) (a[3] - a[2]), npb = (size_t) (b[3] - b[2]);     // plane pitch, elements
     const unsigned b_planes = pair ? 1u : 2u;            // pair: a CTA loads the real or the imaginary plane of B
-    for (int k = 0; k < 4; ++k) {
-        if (k < 2) {
-            rc = a_mn ? make_map_mn(&maps[k], a[k], M, K) : make_map(&maps[k], a[k], M, K);
-            if (rc != CNB_OK) return rc;
-            rc = b_mn ? make_map_mn(&maps[4 + k], b[k], N, K) : make_map(&maps[4 + k], b[k], N, K);
-            if (rc != CNB_OK) return rc;
-        } else {
-            rc = a_mn ? make_map16_mn(&maps[k], a[k], M, K, npa, 2u) : make_map16(&maps[k], a[k], M, K, npa, 2u);
-            if (rc != CNB_OK) return rc;
-            rc = b_mn ? make_map16_mn(&maps[4 + k], b[k], N, K, npb, b_planes) : make_map16(&maps[4 + k], b[k], N, K, npb, b_planes);
+    for (int side = 0; side < 2; ++side) {
+        const SplitOperand& o = side ? b : a;
+        const int rows = side ? N : M;
+        for (int k = 0; k < 4; ++k) {
+            CUtensorMap* m = &maps[4 * side + k];
+            const float* base = o.base + k * o.plane_pitch;
+            const unsigned planes = side ? b_planes : 2u;
+            if (k < 2) rc = o.mn ? make_map_mn(m, base, K, o.pitch) : make_map(m, base, rows, K, o.pitch);
+            else rc = o.mn ? make_map16_mn(m, base, K, o.pitch, o.plane_pitch, planes) : make_map16(m, base, rows, K, o.pitch, o.plane_pitch, planes);
             if (rc != CNB_OK) return rc;
         }
     }
@@ -1208,69 +1261,68 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const float* const a[4], int a_mn, const flo
     p.d_re = d_re; p.d_im = d_im; p.r_re = r_re; p.r_im = r_im;
     p.M = M; p.N = N; p.K = K; p.conjB = conjB; p.accumulate = accumulate;
     p.units_per_cta = (int) upc;
-    p.a_mn = a_mn; p.b_mn = b_mn;
+    p.a_mn = a.mn; p.b_mn = b.mn;
     p.cluster = cluster;
     p.whole_per_cta = whole_per_cta;
     p.segments = segments;
     p.status = ctx->d_status;
-    if (pair)
-        CNB_CUDA(cnb::launch(cgemm_tc_k<true>, dim3((unsigned) (2 * ctas)), dim3(NUM_THREADS), SMEM_BYTES, st, 2 * cluster, maps[0], maps[1],
-                             maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], p));
-    else
-        CNB_CUDA(cnb::launch(cgemm_tc_k<false>, dim3((unsigned) ctas), dim3(NUM_THREADS), SMEM_BYTES, st, cluster, maps[0], maps[1],
-                             maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], p));
+    const bool vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im) |
+                                     reinterpret_cast<uintptr_t>(r_re) | reinterpret_cast<uintptr_t>(r_im)) & 15) == 0;
+    auto go = [&](auto kernel, long grid, int cl) {
+        return cnb::launch(kernel, dim3((unsigned) grid), dim3(NUM_THREADS), SMEM_BYTES, st, cl, maps[0], maps[1], maps[2], maps[3],
+                           maps[4], maps[5], maps[6], maps[7], p);
+    };
+    if (pair) CNB_CUDA(vec ? go(cgemm_tc_k<true, true>, 2 * ctas, 2 * cluster) : go(cgemm_tc_k<true, false>, 2 * ctas, 2 * cluster));
+    else CNB_CUDA(vec ? go(cgemm_tc_k<false, true>, ctas, cluster) : go(cgemm_tc_k<false, false>, ctas, cluster));
     CNB_LAUNCH_CHECK("cgemm_tc");
     return CNB_OK;
 }
 
 // fp32 operands: split them into scratch first.  a_trans / b_trans say the source is stored
-// [K, rows]; it is then consumed MN-major in place (rows % 64 == 0) or transposed while it is split.
+// [K, rows]; it is then consumed MN-major.
 int cgemm_tc_run(cnb_ctx* ctx, const float* a_re, const float* a_im, int a_trans, const float* b_re,
                  const float* b_im, int b_trans, int conjB, const float* r_re, const float* r_im, float* d_re,
                  float* d_im, int M, int N, int K, int accumulate, cudaStream_t st, const float* b_split) {
     float* ws = nullptr;
-    int rc = ensure_scratch(ctx, cgemm_tc_workspace_bytes(M, N, K), &ws);
+    const size_t na = operand_elems(M, K, a_trans), nb = operand_elems(N, K, b_trans);
+    int rc = ensure_scratch(ctx, 4 * (na + (b_split ? 0 : nb)) * sizeof(float), &ws);
     if (rc != CNB_OK) return rc;
-    size_t na = ((size_t) M * K + 63) & ~size_t(63), nb = ((size_t) N * K + 63) & ~size_t(63);
-    float* ap[4] = {ws, ws + na, ws + 2 * na, ws + 3 * na};          // the four slots of a split buffer
-    float* bp[4] = {ws + 4 * na, ws + 4 * na + nb, ws + 4 * na + 2 * nb, ws + 4 * na + 3 * nb};
-    int a_mn = 0, b_mn = 0;
-    auto split = [&](const float* s0, const float* s1, float** dst, int rows, int trans, int* mn) -> int {
-        bool al = ((reinterpret_cast<uintptr_t>(s0) | reinterpret_cast<uintptr_t>(s1)) & 15) == 0;
-        const size_t np = (size_t) (dst[1] - dst[0]);
-        if (trans && !(rows % 64 == 0 && al)) {   // source is [K, rows] with ragged rows: transpose while splitting
-            dim3 grid((rows + 31) / 32, (K + 31) / 32), block(32, 8);
-            cnb::launch(split_transpose_k, grid, block, 0, st, 1, s0, s1, dst[0], np, K, rows);
-        } else {
-            if (!al) return set_error(CNB_ERR_ARG, "cgemm_tc: operand planes must be 16-byte aligned");
-            *mn = trans;
-            split_launch(ctx, s0, s1, dst[0], np, (size_t) rows * K, st);
-        }
-        CNB_LAUNCH_CHECK("split");
-        return CNB_OK;
-    };
-    if ((rc = split(a_re, a_im, ap, M, a_trans, &a_mn)) != CNB_OK) return rc;
+    SplitOperand a = {ws, na, (int) (a_trans ? padded(M, 64) : padded(K, 8)), a_trans};
+    SplitOperand b = {ws + 4 * na, nb, (int) (b_trans ? padded(N, 64) : padded(K, 8)), b_trans};
+    split_launch(ctx, a_re, a_im, ws, na, a_trans ? K : M, a_trans ? M : K, a.pitch, st);
+    CNB_LAUNCH_CHECK("split");
     if (b_split) {                                 // a constant B operand split once by its owner, [N, K]
-        for (int q = 0; q < 4; ++q) bp[q] = const_cast<float*>(b_split) + q * nb;
-    } else if ((rc = split(b_re, b_im, bp, N, b_trans, &b_mn)) != CNB_OK) {
-        return rc;
+        b.base = b_split;
+    } else {
+        split_launch(ctx, b_re, b_im, ws + 4 * na, nb, b_trans ? K : N, b_trans ? N : K, b.pitch, st);
+        CNB_LAUNCH_CHECK("split");
     }
-    return cgemm_tc_presplit(ctx, ap, a_mn, bp, b_mn, conjB, r_re, r_im, d_re, d_im, M, N, K, accumulate, st);
+    return cgemm_tc_presplit(ctx, a, b, conjB, r_re, r_im, d_re, d_im, M, N, K, accumulate, st);
+}
+
+// the split of a constant B operand [N, K] as cgemm_tc_run takes it
+size_t cgemm_tc_operand_bytes(int N, int K) { return 4 * operand_elems(N, K, 0) * sizeof(float); }
+
+int cgemm_tc_split_operand(cnb_ctx* ctx, const float* re, const float* im, int N, int K, float* split, cudaStream_t st) {
+    split_launch(ctx, re, im, split, operand_elems(N, K, 0), N, K, (int) padded(K, 8), st);
+    CNB_LAUNCH_CHECK("split");
+    return CNB_OK;
+}
+
+int split_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, int pitch, float* split, cudaStream_t st) {
+    if ((reinterpret_cast<uintptr_t>(split) & 15) != 0) return set_error(CNB_ERR_ARG, "split: the buffer must be 16-byte aligned");
+    split_launch(ctx, re, im, split, (size_t) rows * pitch, rows, cols, pitch, st);
+    CNB_LAUNCH_CHECK("split");
+    return CNB_OK;
 }
 
 int split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, cudaStream_t st) {
     if (((reinterpret_cast<uintptr_t>(re) | reinterpret_cast<uintptr_t>(im) | reinterpret_cast<uintptr_t>(split)) & 15) != 0)
         return set_error(CNB_ERR_ARG, "split: planes must be 16-byte aligned");
-    size_t np = (n + 63) & ~size_t(63);
-    split_launch(ctx, re, im, split, np, n, st);
+    const size_t np = (n + 63) & ~size_t(63), blocks = (n / 4 + 255) / 256 + 1, cap = (size_t) ctx->sm_count * 16;
+    cnb::launch(split_k, dim3((unsigned) std::min(blocks, cap)), dim3(256), 0, st, 1, re, im, split, np, n);
     CNB_LAUNCH_CHECK("split");
     return CNB_OK;
-}
-
-int cgemm_tc_nt(cnb_ctx* ctx, const float* a_re, const float* a_im, const float* b_re, const float* b_im, int conjB,
-                const float* r_re, const float* r_im, float* d_re, float* d_im, int M, int N, int K, int accumulate,
-                cudaStream_t st) {
-    return cgemm_tc_run(ctx, a_re, a_im, 0, b_re, b_im, 0, conjB, r_re, r_im, d_re, d_im, M, N, K, accumulate, st);
 }
 
 }  // namespace cnb

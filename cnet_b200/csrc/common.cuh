@@ -57,27 +57,32 @@ int cgemm_simt(cnb_ctx* ctx, const float* a_re, const float* a_im, long sam, lon
                const float* r_re, const float* r_im, float* d_re, float* d_im,
                int M, int N, int K, int accumulate, cudaStream_t st);
 
-// tcgen05 complex GEMM on split operands, K-major operands only:
-//   D[m,n] (+)= sum_k A[m,k] * (conjB ? conj(B[n,k]) : B[n,k]) (+ R[m,n]); A [M,K], B [N,K] row-major.
-// Returns CNB_ERR_UNSUPPORTED when the shape does not fit its tiles.
-int cgemm_tc_nt(cnb_ctx* ctx, const float* a_re, const float* a_im,
-                const float* b_re, const float* b_im, int conjB,
-                const float* r_re, const float* r_im, float* d_re, float* d_im,
-                int M, int N, int K, int accumulate, cudaStream_t st);
+// tcgen05 complex GEMM on split operands:
+//   D[m,n] (+)= sum_k A[m,k] * (conjB ? conj(B[n,k]) : B[n,k]) (+ R[m,n]); A [M,K], B [N,K].
+// The sizes for which it beats the SIMT tiles:
 bool cgemm_tc_shape_ok(int M, int N, int K);
-// General form: a_trans / b_trans = the source planes are stored [K, rows] (transposed while splitting).
+// fp32 operands, split into scratch first: a_trans / b_trans = the source planes are stored [K, rows].
 int cgemm_tc_run(cnb_ctx* ctx, const float* a_re, const float* a_im, int a_trans, const float* b_re,
                  const float* b_im, int b_trans, int conjB, const float* r_re, const float* r_im, float* d_re,
                  float* d_im, int M, int N, int K, int accumulate, cudaStream_t st,
                  const float* b_split = nullptr);
 size_t cgemm_tc_workspace_bytes(int M, int N, int K);
-// Operands already split: a[q] / b[q] = slot q of the split buffer (see cnb_split_component below); major 0 =
-// [rows, K], 1 = [K, rows].
-int cgemm_tc_presplit(cnb_ctx* ctx, const float* const a[4], int a_mn, const float* const b[4], int b_mn, int conjB,
+size_t cgemm_tc_operand_bytes(int N, int K);
+int cgemm_tc_split_operand(cnb_ctx* ctx, const float* re, const float* im, int N, int K, float* split, cudaStream_t st);
+// An operand that is already split (see cnb_split_component below): slots plane_pitch floats apart, stored rows
+// [rows, K] (mn = 0) or [K, rows] (mn = 1) at `pitch` elements.
+struct SplitOperand {
+    const float* base;
+    size_t plane_pitch;
+    int pitch, mn;
+};
+int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b, int conjB,
                       const float* r_re, const float* r_im, float* d_re, float* d_im, int M, int N, int K,
                       int accumulate, cudaStream_t st);
 // split = 4 consecutive slots of pad64(n) floats (see cnb_split_component below)
 int split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, cudaStream_t st);
+// the same of a matrix, its rows at `pitch` in the split
+int split_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, int pitch, float* split, cudaStream_t st);
 
 // Skinny Linear (out <= 16): HBM-bound fp32 kernels.
 bool skinny_ok(int B, int in, int out);

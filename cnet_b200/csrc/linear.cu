@@ -55,10 +55,10 @@ int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) {
     if (cnb::cgemm_tc_shape_ok(64, N, N) && (!cnb::fft_supported(N) || (key & kTriKey))) {
         // the matrix is a constant: where the GEMM is the transform's engine, its operand split is
         // made here, not by every product
-        rc = cnb_alloc(ctx, cnb_split_floats((size_t) N * N) * sizeof(float), &p);
+        rc = cnb_alloc(ctx, cnb::cgemm_tc_operand_bytes(N, N), &p);
         if (rc != CNB_OK) return rc;
         t.split = static_cast<float*>(p);
-        rc = cnb::split_planes(ctx, t.re, t.im, (size_t) N * N, t.split, st);
+        rc = cnb::cgemm_tc_split_operand(ctx, t.re, t.im, N, N, t.split, st);
         if (rc != CNB_OK) return rc;
     }
     ctx->twiddles[key] = t;
@@ -70,9 +70,10 @@ int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) {
 int twiddle_product(cnb_ctx* ctx, const cnb_twiddle& t, const float* x_re, const float* x_im, float* y_re, float* y_im,
                     int B, int N, int conj, int accumulate, cudaStream_t st) {
     if (cnb::cgemm_tc_shape_ok(B, N, N)) {
+        const int rc = cnb::cgemm_tc_run(ctx, x_re, x_im, 0, t.re, t.im, 0, conj, nullptr, nullptr, y_re, y_im, B, N, N,
+                                         accumulate, st, t.split);
         cnb::g_last_engine = 1;
-        return cnb::cgemm_tc_run(ctx, x_re, x_im, 0, t.re, t.im, 0, conj, nullptr, nullptr, y_re, y_im, B, N, N,
-                                 accumulate, st, t.split);
+        if (rc != CNB_ERR_ARENA) return rc;
     }
     cnb::g_last_engine = 2;
     return cnb::cgemm_simt(ctx, x_re, x_im, N, 1, t.re, t.im, N, 1, conj, nullptr, nullptr, y_re, y_im, B, N, N,
@@ -94,9 +95,10 @@ int cnb_linear_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im, const flo
         cnb::g_last_engine = 4;
         return cnb::skinny_fwd(ctx, x_re, x_im, w_re, w_im, y_re, y_im, B, in, out, st);
     }
-    if (cnb::cgemm_tc_shape_ok(B, out, in)) {
+    if (cnb::cgemm_tc_shape_ok(B, out, in)) {            // where the arena has no room for the split operands: the SIMT tiles
+        const int rc = cnb::cgemm_tc_run(ctx, x_re, x_im, 0, w_re, w_im, 0, 0, res_re, res_im, y_re, y_im, B, out, in, 0, st);
         cnb::g_last_engine = 1;
-        return cnb::cgemm_tc_nt(ctx, x_re, x_im, w_re, w_im, 0, res_re, res_im, y_re, y_im, B, out, in, 0, st);
+        if (rc != CNB_ERR_ARENA) return rc;
     }
     cnb::g_last_engine = 2;
     return cnb::cgemm_simt(ctx, x_re, x_im, in, 1, w_re, w_im, in, 1, 0, res_re, res_im, y_re, y_im, B, out, in,
@@ -114,10 +116,11 @@ int cnb_linear_bwd_x(cnb_ctx* ctx, const float* g_re, const float* g_im, const f
         return cnb::skinny_bwd_x(ctx, g_re, g_im, w_re, w_im, dx_re, dx_im, B, in, out, accumulate, st);
     }
     if (cnb::cgemm_tc_shape_ok(B, in, out)) {
-        // the B operand (n = i, k = o) is W stored [K = out, N = in]: transposed while it is split
+        // the B operand (n = i, k = o) is W stored [K = out, N = in]
+        const int rc = cnb::cgemm_tc_run(ctx, g_re, g_im, 0, w_re, w_im, 1, 1, nullptr, nullptr, dx_re, dx_im, B, in, out,
+                                         accumulate, st);
         cnb::g_last_engine = 1;
-        return cnb::cgemm_tc_run(ctx, g_re, g_im, 0, w_re, w_im, 1, 1, nullptr, nullptr, dx_re, dx_im, B, in, out,
-                                 accumulate, st);
+        if (rc != CNB_ERR_ARENA) return rc;
     }
     cnb::g_last_engine = 2;
     return cnb::cgemm_simt(ctx, g_re, g_im, out, 1, w_re, w_im, 1, in, 1, nullptr, nullptr, dx_re, dx_im, B, in,
@@ -135,10 +138,11 @@ int cnb_linear_bwd_w(cnb_ctx* ctx, const float* g_re, const float* g_im, const f
         return cnb::skinny_bwd_w(ctx, g_re, g_im, x_re, x_im, dw_re, dw_im, B, in, out, accumulate, st);
     }
     if (cnb::cgemm_tc_shape_ok(out, in, B)) {
-        // both operands are stored [K = B, rows]: transposed while they are split
+        // both operands are stored [K = B, rows]
+        const int rc = cnb::cgemm_tc_run(ctx, g_re, g_im, 1, x_re, x_im, 1, 1, nullptr, nullptr, dw_re, dw_im, out, in, B,
+                                         accumulate, st);
         cnb::g_last_engine = 1;
-        return cnb::cgemm_tc_run(ctx, g_re, g_im, 1, x_re, x_im, 1, 1, nullptr, nullptr, dw_re, dw_im, out, in, B,
-                                 accumulate, st);
+        if (rc != CNB_ERR_ARENA) return rc;
     }
     cnb::g_last_engine = 2;
     return cnb::cgemm_simt(ctx, g_re, g_im, 1, out, x_re, x_im, 1, in, 1, nullptr, nullptr, dw_re, dw_im, out, in,
@@ -197,45 +201,51 @@ int cnb_linear_split_ok(int B, int in, int out) {
 }
 
 namespace {
-inline void planes_of(const float* split, size_t n, const float* p[4]) {
-    size_t np = (n + 63) & ~size_t(63);
-    for (int q = 0; q < 4; ++q) p[q] = split + q * np;
+inline int pitch_of(int cols) { return (cols + 63) & ~63; }
+
+inline cnb::SplitOperand matrix_of(const float* split, int rows, int cols, int mn) {
+    return {split, (size_t) rows * pitch_of(cols), pitch_of(cols), mn};
 }
 }  // namespace
+
+int cnb_linear_matrix_ok(int B, int in, int out) {
+    if (cnb_linear_split_ok(B, in, out)) return 1;
+    // the line of cgemm_tc_shape_ok, for all three products of a layer together (a batch of 16 rows is K of dW*)
+    return (B >= 16 && in >= 48 && out >= 17 && (double) B * in * out >= (double) (1 << 21)) ? 1 : 0;
+}
+
+size_t cnb_split_matrix_floats(int rows, int cols) { return 4 * (size_t) rows * pitch_of(cols); }
+
+int cnb_split_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, float* split, void* stream) {
+    CNB_CHECK_ARG(ctx && re && im && split && rows > 0 && cols > 0, "cnb_split_matrix: bad argument");
+    return cnb::split_matrix(ctx, re, im, rows, cols, pitch_of(cols), split, cnb::S(stream));
+}
 
 int cnb_linear_fwd_split(cnb_ctx* ctx, const float* x_split, const float* w_split, const float* res_re,
                          const float* res_im, float* y_re, float* y_im, int B, int in, int out, void* stream) {
     CNB_CHECK_ARG(ctx && x_split && w_split && y_re && y_im, "cnb_linear_fwd_split: null pointer");
-    CNB_CHECK_ARG(cnb_linear_split_ok(B, in, out), "cnb_linear_fwd_split: B=%d in=%d out=%d not eligible", B, in, out);
-    const float *a[4], *b[4];
-    planes_of(x_split, (size_t) B * in, a);
-    planes_of(w_split, (size_t) out * in, b);
+    CNB_CHECK_ARG(cnb_linear_matrix_ok(B, in, out), "cnb_linear_fwd_split: B=%d in=%d out=%d not eligible", B, in, out);
     cnb::g_last_engine = 1;
-    return cnb::cgemm_tc_presplit(ctx, a, 0, b, 0, 0, res_re, res_im, y_re, y_im, B, out, in, 0, cnb::S(stream));
+    return cnb::cgemm_tc_presplit(ctx, matrix_of(x_split, B, in, 0), matrix_of(w_split, out, in, 0), 0, res_re, res_im, y_re,
+                                  y_im, B, out, in, 0, cnb::S(stream));
 }
 
 int cnb_linear_bwd_x_split(cnb_ctx* ctx, const float* g_split, const float* w_split, float* dx_re, float* dx_im,
                            int B, int in, int out, int accumulate, void* stream) {
     CNB_CHECK_ARG(ctx && g_split && w_split && dx_re && dx_im, "cnb_linear_bwd_x_split: null pointer");
-    CNB_CHECK_ARG(cnb_linear_split_ok(B, in, out), "cnb_linear_bwd_x_split: B=%d in=%d out=%d not eligible", B, in, out);
-    const float *a[4], *b[4];
-    planes_of(g_split, (size_t) B * out, a);
-    planes_of(w_split, (size_t) out * in, b);      // W [out, in] = [K, N]: MN-major B operand
-    cnb::g_last_engine = 1;
-    return cnb::cgemm_tc_presplit(ctx, a, 0, b, 1, 1, nullptr, nullptr, dx_re, dx_im, B, in, out, accumulate,
-                                  cnb::S(stream));
+    CNB_CHECK_ARG(cnb_linear_matrix_ok(B, in, out), "cnb_linear_bwd_x_split: B=%d in=%d out=%d not eligible", B, in, out);
+    cnb::g_last_engine = 1;                        // W [out, in] = [K, N]: MN-major B operand
+    return cnb::cgemm_tc_presplit(ctx, matrix_of(g_split, B, out, 0), matrix_of(w_split, out, in, 1), 1, nullptr, nullptr, dx_re,
+                                  dx_im, B, in, out, accumulate, cnb::S(stream));
 }
 
 int cnb_linear_bwd_w_split(cnb_ctx* ctx, const float* g_split, const float* x_split, float* dw_re, float* dw_im,
                            int B, int in, int out, int accumulate, void* stream) {
     CNB_CHECK_ARG(ctx && g_split && x_split && dw_re && dw_im, "cnb_linear_bwd_w_split: null pointer");
-    CNB_CHECK_ARG(cnb_linear_split_ok(B, in, out), "cnb_linear_bwd_w_split: B=%d in=%d out=%d not eligible", B, in, out);
-    const float *a[4], *b[4];
-    planes_of(g_split, (size_t) B * out, a);       // G [B, out] = [K, M]: MN-major A operand
-    planes_of(x_split, (size_t) B * in, b);        // X [B, in]  = [K, N]: MN-major B operand
-    cnb::g_last_engine = 1;
-    return cnb::cgemm_tc_presplit(ctx, a, 1, b, 1, 1, nullptr, nullptr, dw_re, dw_im, out, in, B, accumulate,
-                                  cnb::S(stream));
+    CNB_CHECK_ARG(cnb_linear_matrix_ok(B, in, out), "cnb_linear_bwd_w_split: B=%d in=%d out=%d not eligible", B, in, out);
+    cnb::g_last_engine = 1;                        // G [B, out] = [K, M] and X [B, in] = [K, N]: both MN-major
+    return cnb::cgemm_tc_presplit(ctx, matrix_of(g_split, B, out, 1), matrix_of(x_split, B, in, 1), 1, nullptr, nullptr, dw_re,
+                                  dw_im, out, in, B, accumulate, cnb::S(stream));
 }
 
 int cnb_dft_fused_ok(int N) { return cnb::fft_supported(N) ? 1 : 0; }

@@ -172,7 +172,7 @@ float* Hadamard::consumerSplit() {
 	if (!fused_gelu_ || fused_gelu_->no_outputs() != 1) return nullptr;
 	Linear* l = dynamic_cast<Linear*>(fused_gelu_->next(0));
 	if (l && l->use_split_ && l->previous(0) == fused_gelu_ &&
-			cnb_linear_split_ok(batch(), l->firstInputLength(), l->outSize())) {
+			cnb_linear_matrix_ok(batch(), l->firstInputLength(), l->outSize())) {
 		l->x_presplit_ = true;
 		return l->x_split_;
 	}
@@ -185,7 +185,7 @@ void Hadamard::forward() {
 	const Vars& v = in(1);
 	if (fused_gelu_) {
 		Vars& y = fused_gelu_->out_;
-		float* ysplit = consumerSplit();
+		float* ysplit = out_size_ % 64 == 0 ? consumerSplit() : nullptr;   // it writes one run, not rows at a pitch
 		check(cnb_hadamard_gelu_fwd_split(ctx(), u.real_, u.imag_, v.real_, v.imag_, out_.real_, out_.imag_, y.real_,
 				y.imag_, ysplit, batch(), out_size_, stream()));
 		return;
@@ -233,20 +233,20 @@ Linear::Linear(InSize in1, InSize in2)
 	  in2_len(in2.value()) {}
 
 size_t Linear::extraBytes(int batch) const {
-	if (!cnb_linear_split_ok(batch, in1_len, out_size_)) return 0;
-	return (cnb_split_floats((size_t) batch * in1_len) + cnb_split_floats((size_t) in2_len)) * sizeof(float);
+	if (!cnb_linear_matrix_ok(batch, in1_len, out_size_)) return 0;
+	return (cnb_split_matrix_floats(batch, in1_len) + cnb_split_matrix_floats(out_size_, in1_len)) * sizeof(float);
 }
 
 void Linear::bindExtra(char* mem, int batch) {
 	use_split_ = true;
 	x_split_ = reinterpret_cast<float*>(mem);
-	w_split_ = x_split_ + cnb_split_floats((size_t) batch * in1_len);
+	w_split_ = x_split_ + cnb_split_matrix_floats(batch, in1_len);
 }
 
 void Linear::splitWeights() {
 	if (!use_split_) return;
 	const Vars& w = in(1);
-	check(cnb_split_planes(ctx(), w.real_, w.imag_, (size_t) in2_len, w_split_, stream()));
+	check(cnb_split_matrix(ctx(), w.real_, w.imag_, out_size_, in1_len, w_split_, stream()));
 	w_split_version_ = net_->weights_version_;
 }
 
@@ -258,10 +258,10 @@ void Linear::forward() {
 		const Vars& r = fused_residual_->previous(residual_operand_)->output();
 		rr = r.real_; ri = r.imag_;
 	}
-	if (use_split_ && cnb_linear_split_ok(batch(), in1_len, out_size_)) {
+	if (use_split_ && cnb_linear_matrix_ok(batch(), in1_len, out_size_)) {
 		if (w_split_version_ != net_->weights_version_) splitWeights();
 		if (!x_presplit_)
-			check(cnb_split_planes(ctx(), x.real_, x.imag_, (size_t) batch() * in1_len, x_split_, stream()));
+			check(cnb_split_matrix(ctx(), x.real_, x.imag_, batch(), in1_len, x_split_, stream()));
 		x_presplit_ = false;
 		check(cnb_linear_fwd_split(ctx(), x_split_, w_split_, rr, ri, out_.real_, out_.imag_, batch(), in1_len,
 				out_size_, stream()));
@@ -275,9 +275,9 @@ void Linear::backward() {
 	CFunc* px = prev_func_[0];
 	CFunc* pw = prev_func_[1];
 	int acc_x = accumulate_into(px), acc_w = accumulate_into(pw);
-	if (use_split_ && cnb_linear_split_ok(batch(), in1_len, out_size_)) {
+	if (use_split_ && cnb_linear_matrix_ok(batch(), in1_len, out_size_)) {
 		float* gs = net_->g_split_;
-		check(cnb_split_planes(ctx(), out_.dz_star_real_, out_.dz_star_imag_, (size_t) batch() * out_size_, gs, stream()));
+		check(cnb_split_matrix(ctx(), out_.dz_star_real_, out_.dz_star_imag_, batch(), out_size_, gs, stream()));
 		// Small problems give each of the 148 persistent CTAs only a few k-blocks, so prologue and
 		// epilogue dominate: run the two independent products side by side on half the SMs each.
 		const bool side_by_side = net_->side_stream_ != nullptr &&
@@ -598,14 +598,14 @@ size_t CNet::requiredArenaBytes(int B) const {
 		else floats += 4 * pad64((size_t) B * f->out_size_);
 		if (CEmbedding* e = dynamic_cast<CEmbedding*>(f)) floats += 4 * pad64((size_t) e->inSize());
 		if ((dynamic_cast<FourierTrans*>(f) && !cnb_dft_fused_ok((int) f->in_size_)) || dynamic_cast<TriangFourier*>(f))     // twiddle planes + their split
-			dft += (size_t) 2 * f->in_size_ * f->in_size_ * 4 + cnb_split_floats((size_t) f->in_size_ * f->in_size_) * 4 + 1024;
+			dft += (size_t) 2 * f->in_size_ * f->in_size_ * 4 + cnb_split_matrix_floats(f->in_size_, f->in_size_) * 4 + 1024;
 		extra += f->extraBytes(B) + 256;
 	}
 	size_t gs = 0;
 	for (auto f : func_list_)
 		if (Linear* l = dynamic_cast<Linear*>(f))
-			if (cnb_linear_split_ok(B, l->firstInputLength(), l->outSize()))
-				gs = std::max(gs, cnb_split_floats((size_t) B * l->outSize()) * sizeof(float));
+			if (cnb_linear_matrix_ok(B, l->firstInputLength(), l->outSize()))
+				gs = std::max(gs, cnb_split_matrix_floats(B, l->outSize()) * sizeof(float));
 	size_t staging = 0;                                // input pipeline: one staged batch + labels
 	if (!func_list_.empty()) {
 		CFunc* f0 = func_list_.front();
@@ -806,7 +806,7 @@ bool CNet::allocateOnGpu(int B) {
 		size_t gs = 0;
 		for (auto f : func_list_)
 			if (Linear* l = dynamic_cast<Linear*>(f))
-				if (l->use_split_) gs = std::max(gs, cnb_split_floats((size_t) B * l->outSize()) * sizeof(float));
+				if (l->use_split_) gs = std::max(gs, cnb_split_matrix_floats(B, l->outSize()) * sizeof(float));
 		if (gs) {
 			if ((rc = cnb_alloc(ctx_, gs, &p)) != CNB_OK) { fail(rc, "gradient split planes"); return false; }
 			g_split_ = static_cast<float*>(p);
@@ -1211,8 +1211,8 @@ void CNet::updateInputs(float lr) {
 		Linear* l = dynamic_cast<Linear*>(f);
 		if (!l || !l->use_split_ || spans.size() + 2 > CNB_MAX_SPLIT_SPANS || wgrad_count_ % 4) continue;
 		const Vars& w = l->prev_func_[1]->out_;
-		const size_t np = cnb_split_floats((size_t) l->in2_len) / 4;
-		if (l->in2_len % 4 || w.real_ < weight_base_ || w.imag_ + l->in2_len > weight_base_ + wgrad_count_) continue;
+		const size_t np = cnb_split_matrix_floats(l->out_size_, l->in1_len) / 4;
+		if (l->in1_len % 64 || w.real_ < weight_base_ || w.imag_ + l->in2_len > weight_base_ + wgrad_count_) continue;
 		// slots of the split buffer: hi_re, hi_im (fp32), then [h16_re ; h16_im] and [l16_re ; l16_im] as bf16
 		uint16_t* h16 = reinterpret_cast<uint16_t*>(l->w_split_ + 2 * np);
 		uint16_t* l16 = reinterpret_cast<uint16_t*>(l->w_split_ + 3 * np);
@@ -1323,20 +1323,23 @@ bool CNet::readOutput(int uid, int what, float* re, float* im) {
 	if (what == 0 && f->value_split_) {
 		// Only the operand split of the value was stored: hi (the value cut to TF32) plus the bf16 rounding of
 		// the remainder gives it back to 2^-19 relative, which is what the consuming product saw of it.
-		const size_t np = cnb_split_floats((size_t) cur_batch_ * f->out_size_) / 4;   // plane pitch of the batch in flight
-		std::vector<uint16_t> lo(n);
+		const size_t np = cnb_split_matrix_floats(cur_batch_, f->out_size_) / 4;   // plane pitch of the batch in flight
+		const size_t pitch = np / cur_batch_;
+		std::vector<float> hi(np);
+		std::vector<uint16_t> lo(np);
 		const uint16_t* l16 = reinterpret_cast<const uint16_t*>(f->value_split_ + 3 * np);
 		for (int q = 0; q < 2; ++q) {
 			float* dst = q ? im : re;
-			int rc = cnb_d2h(ctx_, dst, f->value_split_ + q * np, n * sizeof(float), stream_);
-			if (rc == CNB_OK) rc = cnb_d2h(ctx_, lo.data(), l16 + q * np, n * sizeof(uint16_t), stream_);
+			int rc = cnb_d2h(ctx_, hi.data(), f->value_split_ + q * np, np * sizeof(float), stream_);
+			if (rc == CNB_OK) rc = cnb_d2h(ctx_, lo.data(), l16 + q * np, np * sizeof(uint16_t), stream_);
 			if (rc == CNB_OK) rc = cnb_sync(ctx_, stream_);
 			if (rc != CNB_OK) { fail(rc, "readOutput"); return false; }
 			for (size_t k = 0; k < n; ++k) {
-				const uint32_t bits = (uint32_t) lo[k] << 16;
+				const size_t at = k / f->out_size_ * pitch + k % f->out_size_;
+				const uint32_t bits = (uint32_t) lo[at] << 16;
 				float v;
 				std::memcpy(&v, &bits, sizeof v);
-				dst[k] += v;
+				dst[k] = hi[at] + v;
 			}
 		}
 		return true;

@@ -118,6 +118,13 @@ int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_
 size_t cnb_split_floats(size_t n);
 int cnb_split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, void* stream);
 int cnb_linear_split_ok(int B, int in, int out);
+/* The same for a layer of any sizes large enough to be worth it (cnb_linear_matrix_ok; every cnb_linear_split_ok one
+ * is): the split of a matrix keeps its rows at a pitch of `cols` rounded up to 64 elements, so np = rows * pitch above
+ * and the buffer holds cnb_split_matrix_floats(rows, cols) floats; with cols a multiple of 64 it is
+ * cnb_split_planes' own.  The three _split products below take X [B, in], W [out, in] and G [B, out] so. */
+int cnb_linear_matrix_ok(int B, int in, int out);
+size_t cnb_split_matrix_floats(int rows, int cols);
+int cnb_split_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, float* split, void* stream);
 int cnb_linear_fwd_split(cnb_ctx* ctx, const float* x_split, const float* w_split,
                          const float* res_re, const float* res_im,
                          float* y_re, float* y_im, int B, int in, int out, void* stream);

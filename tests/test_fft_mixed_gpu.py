@@ -26,17 +26,12 @@ def test_mixed_radix_lengths(ctx, B, N):  # noqa: F811
     assert ctx.last_gemm_engine() in (3, 5)
     assert util.relerr(_host(ctx.dft_bwd(_dev(x))), _pair(b)) < TOL
     assert util.relerr(_host(ctx.dft_bwd(_dev(x), out=_dev(x))), _pair(b + _c(x))) < TOL
-    u, split = ctx.dft_hadamard_gelu_fwd(_dev(x), _dev(h), split=_padded_split(ctx, B, N))
+    u, split = ctx.dft_hadamard_gelu_fwd(_dev(x), _dev(h))
     assert util.relerr(_host(u), _pair(f)) < TOL
     a = f * _c(h)
     want = co._gelu(a.real), co._gelu(a.imag)
     # the split keeps the value to 2^-18 beside the transform's own error
     assert util.relerr(_unsplit(split, B, N), want) < TOL + 2.0 ** -18
-
-
-def _padded_split(ctx, B, N):  # noqa: F811
-    import torch
-    return torch.zeros(ctx.lib.cnb_split_floats(B * ((N + 63) // 64 * 64)), dtype=torch.float32, device="cuda")
 
 
 def _unsplit(split, B, N):
