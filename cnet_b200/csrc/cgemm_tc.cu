@@ -52,8 +52,18 @@
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 16;
-constexpr int PLANE_BYTES = BM * BK * 4;             // 8 KB: one operand slot of one stage
+constexpr int BM = 128, BN = 128;
+constexpr int PLANE_BYTES = 8192;                    // one operand slot of one stage: 128 rows of 64 bytes
+
+// Operand forms.  SPLIT: fp32 hi, bf16 of hi and lo, k-blocks of 16 (the split buffers of the C ABI).  PACKED: two fp16
+// parts of the scaled value, k-blocks of 32 in the same bytes.
+enum Form { SPLIT = 0, PACKED = 1 };
+template <int FORM> struct FormCfg {
+    static constexpr int BK = FORM == PACKED ? 32 : 16;
+    static constexpr int MAPS = FORM == PACKED ? 4 : 8;
+};
+// tensor maps of A, then of B.  SPLIT: hi_re, hi_im, h16, l16 each; PACKED: high parts, low parts (both planes a map).
+template <int FORM> struct OperandMaps { CUtensorMap m[FormCfg<FORM>::MAPS]; };
 // One CTA per tile: 8 slots (A: 4, B: 4) = 64 KB per stage, 3 stages.  A pair of CTAs per 256-row tile
 // (cta_group::2): each CTA stages its own 128 rows of A (4 slots) and one of the two halves of the stacked B
 // operand (B_re rows in the first CTA, B_im rows in the second: 2 slots) = 48 KB per stage, 4 stages.
@@ -79,6 +89,8 @@ struct TcParams {
     int cluster;              // > 1: that many CTAs of one cluster share a tile, each a slice of K
     int whole_per_cta;        // > 0: every CTA first takes that many whole tiles, then its run of the remaining units
     int segments;             // > 0: CTA r takes k-segment r / tiles of tile r % tiles (units_per_cta k-blocks each)
+    const int* a_exp;         // PACKED: the powers of two that A and B were scaled by
+    const int* b_exp;
     int* status;
     // The pair form (cgemm_tc_k<true>): cluster = K slices per tile, each slice a CTA pair (cluster of 2 * cluster CTAs).
 };
@@ -227,6 +239,20 @@ __device__ __forceinline__ uint64_t smem_desc_mn128_b16(uint32_t addr) {
     d |= (uint64_t) 2 << 61;                          // layout type: 128-byte swizzle
     return d;
 }
+
+// fp16 MN-major operand tile with 32 k-lines a slab: as above, slabs 4 KB apart.
+__device__ __forceinline__ uint64_t smem_desc_mn128_h(uint32_t addr) {
+    uint64_t d = 0;
+    d |= (uint64_t) ((addr >> 4) & 0x3FFF);
+    d |= (uint64_t) (4096 >> 4) << 16;
+    d |= (uint64_t) (1024 >> 4) << 32;
+    d |= (uint64_t) 1 << 46;
+    d |= (uint64_t) 2 << 61;                          // layout type: 128-byte swizzle
+    return d;
+}
+
+// kind::f16 with fp16 operands, fp32 accumulate, M = 128, N = 256
+constexpr uint32_t kInstrDescH = (1u << 4) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
 
 // kind::f16 with bf16 operands, fp32 accumulate, M = 128, N = 256
 constexpr uint32_t kInstrDesc16 = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
@@ -444,14 +470,11 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 
 // VEC: rows of D and R are 16-byte aligned (N % 4 == 0); the form without it writes 32 consecutive floats of a row per
 // warp instruction instead of four 16-byte pieces of four rows.
-template <bool PAIR, bool VEC>
+template <bool PAIR, bool VEC, int FORM>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ CUtensorMap a_hi_im,
-           const __grid_constant__ CUtensorMap a_h16, const __grid_constant__ CUtensorMap a_l16,
-           const __grid_constant__ CUtensorMap b_hi_re, const __grid_constant__ CUtensorMap b_hi_im,
-           const __grid_constant__ CUtensorMap b_h16, const __grid_constant__ CUtensorMap b_l16,
-           const TcParams p) {
+cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
     extern __shared__ uint8_t smem_raw[];
+    constexpr int BK = FormCfg<FORM>::BK;
     CNB_GSTAMP(0, threadIdx.x == 0);
     // operand stages need the alignment of their swizzle pattern; 1024 B covers every mode
     constexpr int STAGES = Cfg<PAIR>::STAGES, STAGE_BYTES = Cfg<PAIR>::STAGE_BYTES, TILE_M = Cfg<PAIR>::TILE_M;
@@ -533,10 +556,8 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
     }
-    if (warp == 0 && lane < 8) {   // descriptor fetch of the 8 operand maps, off the first TMA's critical path
-        const CUtensorMap* maps[8] = {&a_hi_re, &a_hi_im, &a_h16, &a_l16, &b_hi_re, &b_hi_im, &b_h16, &b_l16};
-        asm volatile("prefetch.tensormap [%0];" ::"l"(maps[lane]) : "memory");
-    }
+    if (warp == 0 && lane < FormCfg<FORM>::MAPS)   // descriptor fetch of the operand maps, off the first TMA's critical path
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&om.m[lane]) : "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if constexpr (PAIR) cluster_sync();                  // the peer's barriers exist before anything signals them
@@ -552,7 +573,6 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
-            const CUtensorMap* maps[8] = {&a_hi_re, &a_hi_im, &a_h16, &a_l16, &b_hi_re, &b_hi_im, &b_h16, &b_l16};
             long it = 0;
             bool live = true;
             for (int pass = 0; pass < 2 && live; ++pass)
@@ -563,6 +583,26 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
                 uint32_t phase = (uint32_t) (it / STAGES) & 1;
                 if (!mbar_wait(empty_bar(s), phase ^ 1, abort_flag, p.status, 1)) { live = false; break; }
                 uint32_t dst = smem_base + s * STAGE_BYTES;
+                if constexpr (FORM == PACKED) {
+                    // slots 0..3: A high re, im, low re, im; then B: all four, or (pair) this CTA's plane of high and low
+                    const uint32_t bar = PAIR ? map_to_rank(full_bar(s), lead_rank) : full_bar(s);
+                    if (prank == 0) mbar_expect_tx(full_bar(s), (PAIR ? 2 : 1) * STAGE_BYTES);
+                    auto load = [&](uint32_t to, const CUtensorMap* m, bool mn, int r0, int plane) {
+                        if (mn) {
+                            if constexpr (PAIR) tma2_load_4d(to, m, bar, 0, kb * BK, r0 / 64, plane);
+                            else tma_load_4d(to, m, bar, 0, kb * BK, r0 / 64, plane);
+                        } else {
+                            if constexpr (PAIR) tma2_load_3d(to, m, bar, kb * BK, r0, plane);
+                            else tma_load_3d(to, m, bar, kb * BK, r0, plane);
+                        }
+                    };
+                    load(dst, &om.m[0], p.a_mn, m0, 0);
+                    load(dst + 2 * PLANE_BYTES, &om.m[1], p.a_mn, m0, 0);
+                    load(dst + 4 * PLANE_BYTES, &om.m[2], p.b_mn, n0, PAIR ? (int) prank : 0);
+                    load(dst + (PAIR ? 5 : 6) * PLANE_BYTES, &om.m[3], p.b_mn, n0, PAIR ? (int) prank : 0);
+                    continue;
+                } else {
+                const CUtensorMap* maps = om.m;
                 if constexpr (PAIR) {
                     // Both CTAs fill their own stage; all completion bytes go to the full barrier of the pair's
                     // first CTA, which expects the bytes of both.
@@ -571,22 +611,22 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {        // this CTA's 128 rows of A: hi_re, hi_im, h16 pair, l16 pair
                         if (q < 2) {
-                            if (p.a_mn) tma2_load_3d(dst + q * PLANE_BYTES, maps[q], bar, 0, kb * BK, m0 / 32);
-                            else tma2_load_2d(dst + q * PLANE_BYTES, maps[q], bar, kb * BK, m0);
+                            if (p.a_mn) tma2_load_3d(dst + q * PLANE_BYTES, maps + q, bar, 0, kb * BK, m0 / 32);
+                            else tma2_load_2d(dst + q * PLANE_BYTES, maps + q, bar, kb * BK, m0);
                         } else {
-                            if (p.a_mn) tma2_load_4d(dst + q * PLANE_BYTES, maps[q], bar, 0, kb * BK, m0 / 64, 0);
-                            else tma2_load_3d(dst + q * PLANE_BYTES, maps[q], bar, kb * BK, m0, 0);
+                            if (p.a_mn) tma2_load_4d(dst + q * PLANE_BYTES, maps + q, bar, 0, kb * BK, m0 / 64, 0);
+                            else tma2_load_3d(dst + q * PLANE_BYTES, maps + q, bar, kb * BK, m0, 0);
                         }
                     }
                     // this CTA's half of the stacked B operand: the real planes (first CTA) or the imaginary ones
                     const int c = (int) prank;
                     uint32_t db = dst + 4 * PLANE_BYTES;
-                    if (p.b_mn) tma2_load_3d(db, maps[4 + c], bar, 0, kb * BK, n0 / 32);
-                    else tma2_load_2d(db, maps[4 + c], bar, kb * BK, n0);
+                    if (p.b_mn) tma2_load_3d(db, maps + 4 + c, bar, 0, kb * BK, n0 / 32);
+                    else tma2_load_2d(db, maps + 4 + c, bar, kb * BK, n0);
                     db += PLANE_BYTES;
                     for (int q = 6; q < 8; ++q, db += PLANE_BYTES / 2) {      // h16, l16: boxes of one plane
-                        if (p.b_mn) tma2_load_4d(db, maps[q], bar, 0, kb * BK, n0 / 64, c);
-                        else tma2_load_3d(db, maps[q], bar, kb * BK, n0, c);
+                        if (p.b_mn) tma2_load_4d(db, maps + q, bar, 0, kb * BK, n0 / 64, c);
+                        else tma2_load_3d(db, maps + q, bar, kb * BK, n0, c);
                     }
                     continue;
                 }
@@ -596,12 +636,13 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
                     const int r0 = q < 4 ? m0 : n0;
                     const bool mn = q < 4 ? p.a_mn : p.b_mn;
                     if ((q & 3) < 2) {                   // an fp32 hi plane
-                        if (mn) tma_load_3d(dst + q * PLANE_BYTES, maps[q], full_bar(s), 0, kb * BK, r0 / 32);
-                        else tma_load_2d(dst + q * PLANE_BYTES, maps[q], full_bar(s), kb * BK, r0);
+                        if (mn) tma_load_3d(dst + q * PLANE_BYTES, maps + q, full_bar(s), 0, kb * BK, r0 / 32);
+                        else tma_load_2d(dst + q * PLANE_BYTES, maps + q, full_bar(s), kb * BK, r0);
                     } else {                             // a pair of bf16 planes [re ; im]
-                        if (mn) tma_load_4d(dst + q * PLANE_BYTES, maps[q], full_bar(s), 0, kb * BK, r0 / 64, 0);
-                        else tma_load_3d(dst + q * PLANE_BYTES, maps[q], full_bar(s), kb * BK, r0, 0);
+                        if (mn) tma_load_4d(dst + q * PLANE_BYTES, maps + q, full_bar(s), 0, kb * BK, r0 / 64, 0);
+                        else tma_load_3d(dst + q * PLANE_BYTES, maps + q, full_bar(s), kb * BK, r0, 0);
                     }
+                }
                 }
             }
         }
@@ -633,6 +674,36 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     uint32_t st = smem_base + s * STAGE_BYTES;
                     const uint32_t first = kb == kb0 ? 0u : 1u;
+                    if constexpr (FORM == PACKED) {
+                        // high.low + low.high first, then high.high, a k-step of 16 at a time
+                        const uint32_t idesch = (kInstrDescH | mn_bits) + m_bits;
+                        constexpr int b_low = PAIR ? 5 : 6;
+#pragma unroll
+                        for (int j = 0; j < BK / 16; ++j) {
+                            const uint32_t ka = p.a_mn ? j * 2048 : j * 32, kbo = p.b_mn ? j * 2048 : j * 32;
+                            auto adesc = [&](int slot) {
+                                const uint32_t a = st + slot * PLANE_BYTES + ka;
+                                return p.a_mn ? smem_desc_mn128_h(a) : smem_desc_sw64(a);
+                            };
+                            auto bdesc = [&](int slot) {
+                                const uint32_t b = st + slot * PLANE_BYTES + kbo;
+                                return p.b_mn ? smem_desc_mn128_h(b) : smem_desc_sw64(b);
+                            };
+                            auto mma = [&](uint32_t acc, uint64_t a, uint64_t b, uint32_t add) {
+                                if constexpr (PAIR) umma2_bf16(acc, a, b, idesch, add); else umma_bf16(acc, a, b, idesch, add);
+                            };
+                            const uint64_t bh = bdesc(4), bl = bdesc(b_low);
+                            const uint32_t add = j == 0 ? first : 1u;
+                            mma(tmem_base, adesc(2), bh, add);
+                            mma(tmem_base, adesc(0), bl, 1u);
+                            mma(tmem_base, adesc(0), bh, 1u);
+                            mma(tmem_base + 256, adesc(3), bh, add);
+                            mma(tmem_base + 256, adesc(1), bl, 1u);
+                            mma(tmem_base + 256, adesc(1), bh, 1u);
+                        }
+                        if constexpr (PAIR) umma2_commit_both(empty_bar(s), lead_rank); else umma_commit(empty_bar(s));
+                        continue;
+                    } else {
                     if constexpr (PAIR) {
                         // slots: 0 / 1 A hi_re / hi_im, 2 / 3 A h16 / l16 [re ; im], 4 B hi, 5 B h16 then l16
                         auto a16 = [&](int slot, int im) {
@@ -694,6 +765,7 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
                         umma_tf32(tmem_base + 256, adesc(1), b_h, idesc, 1u);        // hi(A_im) . hi(B)
                     }
                     umma_commit(empty_bar(s));       // the stage is free once these MMAs have read it
+                    }
                 }
                 if (ok) { if constexpr (PAIR) umma2_commit_both(acc_full, lead_rank); else umma_commit(acc_full); }
                 CNB_GSTAMP(3, true);
@@ -707,6 +779,14 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
         const int et = (warp - 2) * 32 + lane;       // 0..127 within the epilogue group
         const uint32_t tl = tmem_base + ((uint32_t) (q * 32) << 16);
         const float sgn = p.conjB ? 1.f : -1.f;
+        // PACKED: the scales of both operands are taken out again, in two factors so that neither leaves fp32's range
+        float u0 = 1.f, u1 = 1.f;
+        if constexpr (FORM == PACKED) {
+            const int e = -(*p.a_exp + *p.b_exp), h = e >> 1;
+            u0 = __uint_as_float((uint32_t) (h + 127) << 23);
+            u1 = __uint_as_float((uint32_t) (e - h + 127) << 23);
+        }
+        auto out = [&](float v) { return FORM == PACKED ? v * u0 * u1 : v; };
         int seg = 0;
         if (split_cluster) {
             // the whole k-slice is one segment; its partial sums go to shared memory for the cluster reduction
@@ -737,11 +817,11 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
                     for (int i = 0; i < 16; i += 4) {
                         const int o = part_off(row, (c0 + i) >> 2);
                         *reinterpret_cast<float4*>(part_re + o) =
-                            make_float4(a[i] + sgn * f[i], a[i + 1] + sgn * f[i + 1], a[i + 2] + sgn * f[i + 2],
-                                        a[i + 3] + sgn * f[i + 3]);
+                            make_float4(out(a[i] + sgn * f[i]), out(a[i + 1] + sgn * f[i + 1]), out(a[i + 2] + sgn * f[i + 2]),
+                                        out(a[i + 3] + sgn * f[i + 3]));
                         *reinterpret_cast<float4*>(part_im + o) =
-                            make_float4(e[i] - sgn * b[i], e[i + 1] - sgn * b[i + 1], e[i + 2] - sgn * b[i + 2],
-                                        e[i + 3] - sgn * b[i + 3]);
+                            make_float4(out(e[i] - sgn * b[i]), out(e[i + 1] - sgn * b[i + 1]), out(e[i + 2] - sgn * b[i + 2]),
+                                        out(e[i + 3] - sgn * b[i + 3]));
                     }
                 }
             }
@@ -799,8 +879,8 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
 #pragma unroll
                         for (int i = 0; i < 16; i += 4)
                             *reinterpret_cast<float4*>(stage_re + stage_off(row, 4 * h + i / 4)) =
-                                make_float4(a[i] + sgn * f[i], a[i + 1] + sgn * f[i + 1], a[i + 2] + sgn * f[i + 2],
-                                            a[i + 3] + sgn * f[i + 3]);
+                                make_float4(out(a[i] + sgn * f[i]), out(a[i + 1] + sgn * f[i + 1]), out(a[i + 2] + sgn * f[i + 2]),
+                                            out(a[i + 3] + sgn * f[i + 3]));
                     }
                 }
                 {
@@ -813,8 +893,8 @@ cgemm_tc_k(const __grid_constant__ CUtensorMap a_hi_re, const __grid_constant__ 
 #pragma unroll
                         for (int i = 0; i < 16; i += 4)
                             *reinterpret_cast<float4*>(stage_im + stage_off(row, 4 * h + i / 4)) =
-                                make_float4(e[i] - sgn * b[i], e[i + 1] - sgn * b[i + 1], e[i + 2] - sgn * b[i + 2],
-                                            e[i + 3] - sgn * b[i + 3]);
+                                make_float4(out(e[i] - sgn * b[i]), out(e[i + 1] - sgn * b[i + 1]), out(e[i + 2] - sgn * b[i + 2]),
+                                            out(e[i + 3] - sgn * b[i + 3]));
                     }
                 }
                 if (c0 + 32 == BN) {
@@ -938,27 +1018,103 @@ __global__ void split_k(const float* __restrict__ s0, const float* __restrict__ 
     }
 }
 
-// The same, from rows of `cols` floats at any 4-byte alignment to rows at `pitch` (a multiple of 4): a thread takes four
-// columns of a row, loads what there is of them and stores 16 and 8 bytes (the row's last group past `cols` too).
-__global__ void split_rows_k(const float* __restrict__ s0, const float* __restrict__ s1, float* __restrict__ sp, size_t np,
-                             int rows, int cols, int pitch) {
+// Packed operands.  x = 2^-e (high + low), high = fp16(x 2^e), low = fp16(x 2^e - high), with one e for the whole
+// matrix that brings its largest component into [2^14, 2^15): 22 bits of every component down to 2^-18 of the largest
+// (2^-14, fp16's least normal, is 2^-29 of it, and low starts 11 bits lower), fewer below, an absolute error of 2^-40
+// of the largest at most.  A first pass finds the largest component, the second packs.
+struct PackJob {
+    const float* re; const float* im;
+    __half* dst;                       // four planes of rows * pitch: high re, high im, low re, low im
+    cnb_pack_head* head;               // max_bits and ticket are zero between uses
+    int rows, cols, pitch, blocks;
+};
+template <int N> struct PackJobs { PackJob j[N]; };
+
+__device__ __forceinline__ int pack_exponent(unsigned max_bits) {
+    const int e = 14 + 127 - (int) (max_bits >> 23);     // all zero: 2^126 of nothing
+    return e > 126 ? 126 : e;
+}
+
+template <int N>
+__global__ void __launch_bounds__(256) pack_max_k(const __grid_constant__ PackJobs<N> jobs) {
     cnb_pdl_enter();
-    const cnb_split_dst d0 = cnb_split_component(sp, np, 0), d1 = cnb_split_component(sp, np, 1);
-    const int groups = (cols + 3) / 4;
-    const size_t total = (size_t) rows * groups;
-    for (size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t) gridDim.x * blockDim.x) {
-        const int row = (int) (i / groups), c = (int) (i - (size_t) row * groups) * 4;
-        const float* p = s0 + (size_t) row * cols + c;
-        const float* r = s1 + (size_t) row * cols + c;
-        float x[4], y[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const bool on = c + k < cols;
-            x[k] = on ? p[k] : 0.f; y[k] = on ? r[k] : 0.f;
+    const PackJob& job = jobs.j[blockIdx.y];
+    if ((int) blockIdx.x >= job.blocks) return;
+    const size_t n = (size_t) job.rows * job.cols, step = (size_t) job.blocks * 256;
+    unsigned m = 0;
+    size_t done = 0;
+    if (((reinterpret_cast<uintptr_t>(job.re) | reinterpret_cast<uintptr_t>(job.im)) & 15) == 0) {
+        const size_t n4 = n / 4;
+        for (size_t i = (size_t) blockIdx.x * 256 + threadIdx.x; i < n4; i += step) {
+            const float4 a = reinterpret_cast<const float4*>(job.re)[i], b = reinterpret_cast<const float4*>(job.im)[i];
+            m = max(m, max(max(cnb_abs_bits(a.x), cnb_abs_bits(a.y)), max(cnb_abs_bits(a.z), cnb_abs_bits(a.w))));
+            m = max(m, max(max(cnb_abs_bits(b.x), cnb_abs_bits(b.y)), max(cnb_abs_bits(b.z), cnb_abs_bits(b.w))));
         }
-        const size_t o = (size_t) row * pitch + c;
-        cnb_split_store4(d0, o, x[0], x[1], x[2], x[3]);
-        cnb_split_store4(d1, o, y[0], y[1], y[2], y[3]);
+        done = n4 * 4;
+    }
+    for (size_t i = done + (size_t) blockIdx.x * 256 + threadIdx.x; i < n; i += step) m = max(m, max(cnb_abs_bits(job.re[i]), cnb_abs_bits(job.im[i])));
+    cnb_pack_max_block(job.head, m);
+}
+
+template <int N>
+__global__ void __launch_bounds__(256) pack_k(const __grid_constant__ PackJobs<N> jobs) {
+    cnb_pdl_enter();
+    const PackJob& job = jobs.j[blockIdx.y];
+    if ((int) blockIdx.x >= job.blocks) return;
+    __shared__ int s_exp;
+    if (threadIdx.x == 0) {
+        const int e = pack_exponent(__ldcg(&job.head->max_bits));
+        s_exp = e;
+        if (blockIdx.x == 0) job.head->exponent = e;
+        __threadfence();
+        if (atomicAdd(&job.head->ticket, 1u) == (unsigned) job.blocks - 1) {      // every block has read it: ready for the next use
+            job.head->max_bits = 0;
+            job.head->ticket = 0;
+        }
+    }
+    __syncthreads();
+    const float scale = __uint_as_float((unsigned) (s_exp + 127) << 23);
+    // Consecutive threads take consecutive columns: four each where the rows allow 16-byte loads (8-byte stores), else
+    // two (4-byte accesses), so that every access of a warp is one run.
+    const bool vec = job.cols % 4 == 0 && ((reinterpret_cast<uintptr_t>(job.re) | reinterpret_cast<uintptr_t>(job.im)) & 15) == 0;
+    const size_t np = (size_t) job.rows * job.pitch;
+    const int groups = vec ? job.cols / 4 : (job.cols + 1) / 2;
+    const size_t total = (size_t) job.rows * groups;
+    auto part = [&](float a, float b, __half2* hi, __half2* lo) {
+        a *= scale; b *= scale;
+        *hi = __floats2half2_rn(a, b);
+        const float2 f = __half22float2(*hi);
+        *lo = __floats2half2_rn(a - f.x, b - f.y);
+    };
+    for (size_t i = (size_t) blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t) job.blocks * 256) {
+        // rows without padding are one run; else a 32-bit division where it does (a 64-bit one was half the kernel's time)
+        const bool flat = vec && job.pitch == job.cols;
+        const int row = flat ? 0 : total >> 32 ? (int) (i / groups) : (int) ((unsigned) i / (unsigned) groups);
+        const int g = (int) (i - (size_t) row * groups);
+        if (vec) {
+            const size_t src = flat ? 4 * i : (size_t) row * job.cols + 4 * g, dst = flat ? 4 * i : (size_t) row * job.pitch + 4 * g;
+            const float4 x = *reinterpret_cast<const float4*>(job.re + src), y = *reinterpret_cast<const float4*>(job.im + src);
+            __align__(8) __half2 hi[2], lo[2];
+            part(x.x, x.y, &hi[0], &lo[0]); part(x.z, x.w, &hi[1], &lo[1]);
+            *reinterpret_cast<uint2*>(job.dst + dst) = *reinterpret_cast<uint2*>(hi);
+            *reinterpret_cast<uint2*>(job.dst + 2 * np + dst) = *reinterpret_cast<uint2*>(lo);
+            part(y.x, y.y, &hi[0], &lo[0]); part(y.z, y.w, &hi[1], &lo[1]);
+            *reinterpret_cast<uint2*>(job.dst + np + dst) = *reinterpret_cast<uint2*>(hi);
+            *reinterpret_cast<uint2*>(job.dst + 3 * np + dst) = *reinterpret_cast<uint2*>(lo);
+        } else {
+            const int c = 2 * g;
+            const bool two = c + 1 < job.cols;
+            const size_t src = (size_t) row * job.cols + c, dst = (size_t) row * job.pitch + c;
+            const float x0 = job.re[src], y0 = job.im[src];
+            const float x1 = two ? job.re[src + 1] : 0.f, y1 = two ? job.im[src + 1] : 0.f;
+            __half2 hi, lo;
+            part(x0, x1, &hi, &lo);
+            *reinterpret_cast<__half2*>(job.dst + dst) = hi;
+            *reinterpret_cast<__half2*>(job.dst + 2 * np + dst) = lo;
+            part(y0, y1, &hi, &lo);
+            *reinterpret_cast<__half2*>(job.dst + np + dst) = hi;
+            *reinterpret_cast<__half2*>(job.dst + 3 * np + dst) = lo;
+        }
     }
 }
 
@@ -986,6 +1142,7 @@ EncodeTiledFn encode_fn() {
 
 // [rows, K] fp32 row-major plane; box = BK x 128 rows; 64-byte swizzle; zero fill outside.
 int make_map(CUtensorMap* m, const float* base, int rows, int K, int pitch) {
+    constexpr int BK = FormCfg<SPLIT>::BK;
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[2] = {(cuuint64_t) K, (cuuint64_t) rows};
@@ -1003,6 +1160,7 @@ int make_map(CUtensorMap* m, const float* base, int rows, int K, int pitch) {
 // one box {32, BK, 4} brings four 32-row slabs of 16 k-lines, slab after slab (128-byte swizzle,
 // 32-byte atomicity).
 int make_map_mn(CUtensorMap* m, const float* base, int K, int pitch) {
+    constexpr int BK = FormCfg<SPLIT>::BK;
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[3] = {32u, (cuuint64_t) K, (cuuint64_t) (pitch / 32)};
@@ -1016,36 +1174,38 @@ int make_map_mn(CUtensorMap* m, const float* base, int K, int pitch) {
     return CNB_OK;
 }
 
-// A pair of bf16 planes (real, imaginary; np elements apart), each [rows, K] row-major, seen as [2][rows][K]: one
+// A pair of 16-bit planes (real, imaginary; np elements apart), each [rows, K] row-major, seen as [2][rows][K]: one
 // box {BK, 128, 2} brings the 128 rows of both planes, real then imaginary (planes_per_box = 1: of one plane);
-// 32-byte swizzle.
-int make_map16(CUtensorMap* m, const void* base, int rows, int K, int pitch, size_t np, unsigned planes_per_box) {
+// the swizzle is the box's row of 2 BK bytes.
+int make_map16(CUtensorMap* m, const void* base, int rows, int K, int pitch, size_t np, unsigned planes_per_box, int BK,
+               CUtensorMapDataType type) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[3] = {(cuuint64_t) K, (cuuint64_t) rows, 2u};
     cuuint64_t strides[2] = {(cuuint64_t) pitch * 2u, (cuuint64_t) np * 2u};
     cuuint32_t box[3] = {(cuuint32_t) BK, 128u, planes_per_box};
     cuuint32_t estr[3] = {1u, 1u, 1u};
-    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    CUresult r = fn(m, type, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, BK == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for a bf16 [%d,%d] plane pair", (int) r, rows, K);
+    if (r != CUDA_SUCCESS) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for a 16-bit [%d,%d] plane pair", (int) r, rows, K);
     return CNB_OK;
 }
 
 // The same pair stored [K, rows] (rows contiguous, pitch % 64 == 0), seen as [2][pitch/64][K][64]: one box
 // {64, BK, 2, 2} brings two 64-row slabs of 16 k-lines of both planes, slab after slab (128-byte swizzle).
-int make_map16_mn(CUtensorMap* m, const void* base, int K, int pitch, size_t np, unsigned planes_per_box) {
+int make_map16_mn(CUtensorMap* m, const void* base, int K, int pitch, size_t np, unsigned planes_per_box, int BK,
+                  CUtensorMapDataType type) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[4] = {64u, (cuuint64_t) K, (cuuint64_t) (pitch / 64), 2u};
     cuuint64_t strides[3] = {(cuuint64_t) pitch * 2u, 128u, (cuuint64_t) np * 2u};
     cuuint32_t box[4] = {64u, (cuuint32_t) BK, 2u, planes_per_box};
     cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
-    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
+    CUresult r = fn(m, type, 4, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for an MN-major bf16 [%d,%d] plane pair", (int) r, K, pitch);
+    if (r != CUDA_SUCCESS) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for an MN-major 16-bit [%d,%d] plane pair", (int) r, K, pitch);
     return CNB_OK;
 }
 
@@ -1071,7 +1231,8 @@ __global__ void zero_pair_k(float* __restrict__ a, float* __restrict__ b, size_t
 // units are dealt.  Host arithmetic only (also reachable as cnb_gemm_schedule, for tests that need no GPU).
 struct Schedule { bool pair; long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles; };
 
-Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit) {
+// Depths below are counted in blocks of 16 and scaled to the form's own (bk = 16 or 32).
+Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int bk) {
     // Schedule, by tile count ("CTA" = one CTA, or the CTA pair of a 256-row tile; sms = how many of them this launch
     // may fill: leaving a few SMs free (gemm_cta_limit) lets a concurrent collective's kernels run beside the GEMM):
     //  * tiles >= 4 x SMs, or one nearly full wave of one-tile CTAs when D is not read: whole tiles, grid =
@@ -1082,13 +1243,14 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
     //  * few tiles and short runs: a cluster per tile (below); otherwise plain stream-K.
     // K > 4096 keeps to stream-K runs: one fp32 accumulation chain in tensor memory that long costs accuracy.
     struct Plan { long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles; };
-    const int k_blocks = (K + BK - 1) / BK;
+    const int k_blocks = (K + bk - 1) / bk;
+    auto blocks = [&](int of16) { return (long) std::max(1, of16 * 16 / bk); };
     auto plan = [&](bool pair) {
         Plan q = {};
         const int tile_m = pair ? 2 * BM : BM;
         const int tiles = ((M + tile_m - 1) / tile_m) * ((N + BN - 1) / BN);
         const long total = (long) tiles * k_blocks;
-        const long min_units = 8;                            // do not split below 8 k-blocks per CTA
+        const long min_units = blocks(8);                    // do not split below 8 k-blocks per CTA
         const int all = pair ? sm_count / 2 : sm_count;
         // Pairs under an SM limit (a few SMs set aside for a collective's kernel): a pair needs both SMs of a TPC and
         // each SM set aside may cost a pair its partner, so they are counted twice (6 set aside: 68 pairs).
@@ -1099,9 +1261,9 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
         const int pairs_left = halved ? sm_limit / 2 - 4 : (sm_limit - set_aside) / 2;
         const int sms = sm_limit > 0
             ? std::min(pair ? std::max(1, pairs_left) : sm_limit, all) : all;
-        const bool full_wave = !accumulate && tiles <= sms && (long) tiles * 100 >= (long) sms * 85 && k_blocks <= 256;
-        const bool whole_tiles = (tiles >= all * 4 && sm_limit <= 0 && k_blocks <= 256) || full_wave;
-        const bool lead_whole = !whole_tiles && tiles > sms && k_blocks <= 256;
+        const bool full_wave = !accumulate && tiles <= sms && (long) tiles * 100 >= (long) sms * 85 && k_blocks <= blocks(256);
+        const bool whole_tiles = (tiles >= all * 4 && sm_limit <= 0 && k_blocks <= blocks(256)) || full_wave;
+        const bool lead_whole = !whole_tiles && tiles > sms && k_blocks <= blocks(256);
         long ctas = std::min<long>(sms, std::max<long>(1, total / min_units));
         if (whole_tiles) ctas = tiles;                        // many tiles: whole tiles, no atomics
         long upc = (total + ctas - 1) / ctas;
@@ -1113,8 +1275,8 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
         // outside, in fp32 round-to-nearest): several equal waves of CTAs instead of one persistent wave.
         // Only K > 4096 gets here with longer runs; a whole tile of K <= 4096 is at most 256 k-blocks.  Each tile is
         // cut into equal segments and the CTAs are numbered segment-major (see the kernel).
-        constexpr long kMaxChain = 64;
-        if (!whole_tiles && upc > kMaxChain && k_blocks > 256) {
+        const long kMaxChain = blocks(64);
+        if (!whole_tiles && upc > kMaxChain && k_blocks > blocks(256)) {
             q.segments = (int) ((k_blocks + kMaxChain - 1) / kMaxChain);     // per tile, each at most kMaxChain k-blocks
             upc = (k_blocks + q.segments - 1) / q.segments;
             ctas = (long) tiles * q.segments;
@@ -1134,15 +1296,15 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
         // Worth it while a stream-K run would be short (<= 48 k-blocks): with long runs the atomics are
         // amortised and using every SM wins over the clusters' rounded-down CTA count.
         q.cluster = 1;
-        if (!whole_tiles && !lead_whole && upc <= 48) {
+        if (!whole_tiles && !lead_whole && upc <= blocks(48)) {
             // pairs: two slices at most (clusters of 8 CTAs do not all fit a GPC side by side: measured 0.043 ms
             // against 0.025 at 512 x 1024 x 1024)
             for (int c = pair ? 2 : 8; c >= 2; c >>= 1)
-                if ((long) tiles * c <= sms && k_blocks / c >= 4) { q.cluster = c; break; }
+                if ((long) tiles * c <= sms && k_blocks / c >= blocks(4)) { q.cluster = c; break; }
             // Long K over few tiles leaves the cluster form most of the device idle: 83 x 102 x 13688, one tile, ran
             // 107 k-blocks on each of 8 CTAs (126 us) where stream-K runs are 8 k-blocks long.  The atomics and the
             // cleared output of that form cost about as much as 16 k-blocks.
-            if (q.cluster > 1 && k_blocks / q.cluster > 2 * upc + 16) q.cluster = 1;
+            if (q.cluster > 1 && k_blocks / q.cluster > 2 * upc + blocks(16)) q.cluster = 1;
         }
         if (q.cluster > 1) { ctas = (long) tiles * q.cluster; upc = 0; }
         q.splits_tiles = q.cluster == 1 && (lead_whole ? upc > 0 : (q.segments > 0 || (upc % k_blocks) != 0));
@@ -1177,37 +1339,22 @@ namespace cnb {
 
 bool cgemm_tc_shape_ok(int M, int N, int K) {
     if (K % 8 == 0 && K >= 32 && M >= 64 && N >= 64) return true;
-    // Other sizes pay a split pass to padded rows and a 128 x 128 tile that may be part empty: from about two million
-    // complex multiplications on that is less than what the fp32 SIMT tiles take (777 x 1001 x 1333: 330 against
-    // 45 us), below it the SIMT tiles win.
+    // Other sizes leave more of the 128 x 128 tiles empty: from about two million complex multiplications on packing
+    // and tiles together take less than the fp32 SIMT tiles (777 x 1001 x 1333: 330 against 45 us), below it they do not.
     return K >= 48 && (double) M * N * K >= (double) (1 << 21);
 }
 
 static size_t padded(int n, int to) { return ((size_t) n + to - 1) / to * to; }
 
-// elements of an operand of `rows` x K as cgemm_tc_run stores it: K-major rows at a pitch of K rounded up to 8 (16 bytes
-// of bf16), or, from a source stored [K, rows], MN-major lines at a pitch of rows rounded up to 64
-static size_t operand_elems(int rows, int K, int trans) {
-    const size_t n = trans ? (size_t) K * padded(rows, 64) : (size_t) rows * padded(K, 8);
-    return (n + 63) & ~size_t(63);
+// An operand of `rows` x K as cgemm_tc_run stores it: K-major rows at a pitch of K rounded up to 8 (TMA's 16 bytes), or,
+// from a source stored [K, rows], MN-major lines at a pitch of rows rounded up to 64.
+static int operand_pitch(int rows, int K, int trans) { return (int) (trans ? padded(rows, 64) : padded(K, 8)); }
+static size_t operand_bytes(int rows, int K, int trans) {
+    return (8 * (size_t) (trans ? K : rows) * operand_pitch(rows, K, trans) + 255) & ~size_t(255);
 }
 
 size_t cgemm_tc_workspace_bytes(int M, int N, int K) {
-    const size_t a = std::max(operand_elems(M, K, 0), operand_elems(M, K, 1)), b = std::max(operand_elems(N, K, 0), operand_elems(N, K, 1));
-    return 4 * (a + b) * sizeof(float) + 4096;
-}
-
-static void split_launch(cnb_ctx* ctx, const float* s0, const float* s1, float* sp, size_t np, int rows, int cols, int pitch,
-                         cudaStream_t st) {
-    const bool aligned = ((reinterpret_cast<uintptr_t>(s0) | reinterpret_cast<uintptr_t>(s1)) & 15) == 0;
-    const size_t cap = (size_t) ctx->sm_count * 16;
-    if (aligned && pitch == cols) {                      // one run of rows * cols floats
-        const size_t n = (size_t) rows * cols, blocks = (n / 4 + 255) / 256 + 1;
-        cnb::launch(split_k, dim3((unsigned) std::min(blocks, cap)), dim3(256), 0, st, 1, s0, s1, sp, np, n);
-    } else {
-        const size_t blocks = ((size_t) rows * ((cols + 3) / 4) + 255) / 256;
-        cnb::launch(split_rows_k, dim3((unsigned) std::min(blocks, cap)), dim3(256), 0, st, 1, s0, s1, sp, np, rows, cols, pitch);
-    }
+    return std::max(operand_bytes(M, K, 0), operand_bytes(M, K, 1)) + std::max(operand_bytes(N, K, 0), operand_bytes(N, K, 1)) + 4096;
 }
 
 // The GEMM proper on operands that are already split: the four slots of a split buffer (hi_re, hi_im,
@@ -1218,39 +1365,53 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
                       int accumulate, cudaStream_t st) {
     static bool attr_set[64] = {};                       // the attribute is per device
     if (!attr_set[ctx->device & 63]) {
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+#define CNB_TC_ATTR(P, V, F) CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<P, V, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES))
+        CNB_TC_ATTR(false, false, SPLIT); CNB_TC_ATTR(true, false, SPLIT); CNB_TC_ATTR(false, true, SPLIT); CNB_TC_ATTR(true, true, SPLIT);
+        CNB_TC_ATTR(false, false, PACKED); CNB_TC_ATTR(true, false, PACKED); CNB_TC_ATTR(false, true, PACKED); CNB_TC_ATTR(true, true, PACKED);
+#undef CNB_TC_ATTR
         attr_set[ctx->device & 63] = true;
     }
     if ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im)) & 3)
         return set_error(CNB_ERR_ARG, "cgemm_tc: misaligned output");
     if (a.pitch % (a.mn ? 64 : 8) || b.pitch % (b.mn ? 64 : 8))
         return set_error(CNB_ERR_ARG, "cgemm_tc: operand pitches %d and %d", a.pitch, b.pitch);
-    const Schedule q = choose_schedule(M, N, K, accumulate, ctx->sm_count, ctx->gemm_cta_limit);
+    const bool packed = a.exponent != nullptr;
+    const int bk = packed ? FormCfg<PACKED>::BK : FormCfg<SPLIT>::BK;
+    const Schedule q = choose_schedule(M, N, K, accumulate, ctx->sm_count, ctx->gemm_cta_limit, bk);
     const bool pair = q.pair;
-    const long ctas = q.ctas, upc = q.upc;
-    const int whole_per_cta = q.whole_per_cta, clear_from_row = q.clear_from_row, cluster = q.cluster, segments = q.segments;
+    const long ctas = q.ctas;
+    const int cluster = q.cluster;
 
     int rc;
-    alignas(64) CUtensorMap maps[8];
+    OperandMaps<SPLIT> maps_s;
+    OperandMaps<PACKED> maps_p;
     const unsigned b_planes = pair ? 1u : 2u;            // pair: a CTA loads the real or the imaginary plane of B
     for (int side = 0; side < 2; ++side) {
         const SplitOperand& o = side ? b : a;
         const int rows = side ? N : M;
+        const unsigned planes = side ? b_planes : 2u;
+        if (packed) {
+            for (int k = 0; k < 2; ++k) {                // high parts, low parts
+                CUtensorMap* m = &maps_p.m[2 * side + k];
+                const __half* base = reinterpret_cast<const __half*>(o.base) + 2 * k * o.plane_pitch;
+                rc = o.mn ? make_map16_mn(m, base, K, o.pitch, o.plane_pitch, planes, bk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16)
+                          : make_map16(m, base, rows, K, o.pitch, o.plane_pitch, planes, bk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
+                if (rc != CNB_OK) return rc;
+            }
+            continue;
+        }
         for (int k = 0; k < 4; ++k) {
-            CUtensorMap* m = &maps[4 * side + k];
+            CUtensorMap* m = &maps_s.m[4 * side + k];
             const float* base = o.base + k * o.plane_pitch;
-            const unsigned planes = side ? b_planes : 2u;
             if (k < 2) rc = o.mn ? make_map_mn(m, base, K, o.pitch) : make_map(m, base, rows, K, o.pitch);
-            else rc = o.mn ? make_map16_mn(m, base, K, o.pitch, o.plane_pitch, planes) : make_map16(m, base, rows, K, o.pitch, o.plane_pitch, planes);
+            else rc = o.mn ? make_map16_mn(m, base, K, o.pitch, o.plane_pitch, planes, bk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)
+                           : make_map16(m, base, rows, K, o.pitch, o.plane_pitch, planes, bk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
             if (rc != CNB_OK) return rc;
         }
     }
     if (q.splits_tiles && !accumulate) {
         // one launch clears both planes (they need not be adjacent or in one allocation)
-        const size_t first = (size_t) clear_from_row * N;
+        const size_t first = (size_t) q.clear_from_row * N;
         const size_t plane = (size_t) M * N - first;
         const size_t vec = plane / 4 + 1;
         const int blocks = (int) std::min<size_t>((vec + 255) / 256, (size_t) ctx->sm_count * 8);
@@ -1260,67 +1421,97 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     TcParams p;
     p.d_re = d_re; p.d_im = d_im; p.r_re = r_re; p.r_im = r_im;
     p.M = M; p.N = N; p.K = K; p.conjB = conjB; p.accumulate = accumulate;
-    p.units_per_cta = (int) upc;
+    p.units_per_cta = (int) q.upc;
     p.a_mn = a.mn; p.b_mn = b.mn;
+    p.a_exp = a.exponent; p.b_exp = b.exponent;
     p.cluster = cluster;
-    p.whole_per_cta = whole_per_cta;
-    p.segments = segments;
+    p.whole_per_cta = q.whole_per_cta;
+    p.segments = q.segments;
     p.status = ctx->d_status;
     const bool vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im) |
                                      reinterpret_cast<uintptr_t>(r_re) | reinterpret_cast<uintptr_t>(r_im)) & 15) == 0;
-    auto go = [&](auto kernel, long grid, int cl) {
-        return cnb::launch(kernel, dim3((unsigned) grid), dim3(NUM_THREADS), SMEM_BYTES, st, cl, maps[0], maps[1], maps[2], maps[3],
-                           maps[4], maps[5], maps[6], maps[7], p);
+    auto go = [&](auto kernel, const auto& maps) {
+        return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(NUM_THREADS), SMEM_BYTES, st, pair ? 2 * cluster : cluster, maps, p);
     };
-    if (pair) CNB_CUDA(vec ? go(cgemm_tc_k<true, true>, 2 * ctas, 2 * cluster) : go(cgemm_tc_k<true, false>, 2 * ctas, 2 * cluster));
-    else CNB_CUDA(vec ? go(cgemm_tc_k<false, true>, ctas, cluster) : go(cgemm_tc_k<false, false>, ctas, cluster));
+    cudaError_t e;
+    if (packed) {
+        if (pair) e = vec ? go(cgemm_tc_k<true, true, PACKED>, maps_p) : go(cgemm_tc_k<true, false, PACKED>, maps_p);
+        else e = vec ? go(cgemm_tc_k<false, true, PACKED>, maps_p) : go(cgemm_tc_k<false, false, PACKED>, maps_p);
+    } else {
+        if (pair) e = vec ? go(cgemm_tc_k<true, true, SPLIT>, maps_s) : go(cgemm_tc_k<true, false, SPLIT>, maps_s);
+        else e = vec ? go(cgemm_tc_k<false, true, SPLIT>, maps_s) : go(cgemm_tc_k<false, false, SPLIT>, maps_s);
+    }
+    CNB_CUDA(e);
     CNB_LAUNCH_CHECK("cgemm_tc");
     return CNB_OK;
 }
 
-// fp32 operands: split them into scratch first.  a_trans / b_trans say the source is stored
-// [K, rows]; it is then consumed MN-major.
+// ------------------------------------------------------------------------------------------------ packed operands
+SplitOperand packed_operand(const PackRequest& r, int mn) {
+    return {static_cast<const float*>(r.planes), (size_t) r.rows * r.pitch, r.pitch, mn, &r.head->exponent};
+}
+
+// Jobs in pairs of launches of at most 32; have_max: the heads already hold the largest components.
+template <int N> static int pack_some(cnb_ctx* ctx, const PackRequest* r, int n, bool have_max, cudaStream_t st) {
+    PackJobs<N> jobs;
+    int blocks = 0;
+    // enough blocks in all to fill the device twice over, whatever the number of jobs
+    const size_t cap = std::max<size_t>(16, (size_t) ctx->sm_count * 16 / n);
+    for (int k = 0; k < n; ++k) {
+        if (reinterpret_cast<uintptr_t>(r[k].planes) & 127 || r[k].pitch % 8)
+            return set_error(CNB_ERR_ARG, "pack: planes must be 128-byte aligned, pitch %d a multiple of 8", r[k].pitch);
+        const size_t items = (size_t) r[k].rows * ((r[k].cols + 3) / 4);
+        jobs.j[k] = {r[k].re, r[k].im, static_cast<__half*>(r[k].planes), r[k].head, r[k].rows, r[k].cols, r[k].pitch,
+                     (int) std::min((items + 255) / 256, cap)};
+        blocks = std::max(blocks, jobs.j[k].blocks);
+    }
+    if (!have_max) {
+        cnb::launch(pack_max_k<N>, dim3(blocks, n), dim3(256), 0, st, 1, jobs);
+        CNB_LAUNCH_CHECK("pack_max");
+    }
+    cnb::launch(pack_k<N>, dim3(blocks, n), dim3(256), 0, st, 1, jobs);
+    CNB_LAUNCH_CHECK("pack");
+    return CNB_OK;
+}
+
+int pack(cnb_ctx* ctx, const PackRequest* r, int n, bool have_max, cudaStream_t st) {
+    if (n <= 2) return pack_some<2>(ctx, r, n, have_max, st);
+    for (int k = 0; k < n; k += 32) {
+        const int rc = pack_some<32>(ctx, r + k, std::min(32, n - k), have_max, st);
+        if (rc != CNB_OK) return rc;
+    }
+    return CNB_OK;
+}
+
+// fp32 operands, packed into scratch first.  a_trans / b_trans say the source is stored [K, rows]; it is then consumed
+// MN-major.  The heads sit in the context's status block, which starts at zero.
 int cgemm_tc_run(cnb_ctx* ctx, const float* a_re, const float* a_im, int a_trans, const float* b_re,
                  const float* b_im, int b_trans, int conjB, const float* r_re, const float* r_im, float* d_re,
-                 float* d_im, int M, int N, int K, int accumulate, cudaStream_t st, const float* b_split) {
+                 float* d_im, int M, int N, int K, int accumulate, cudaStream_t st, const PackRequest* b_packed) {
     float* ws = nullptr;
-    const size_t na = operand_elems(M, K, a_trans), nb = operand_elems(N, K, b_trans);
-    int rc = ensure_scratch(ctx, 4 * (na + (b_split ? 0 : nb)) * sizeof(float), &ws);
+    const size_t na = operand_bytes(M, K, a_trans), nb = b_packed ? 0 : operand_bytes(N, K, b_trans);
+    int rc = ensure_scratch(ctx, na + nb, &ws);
     if (rc != CNB_OK) return rc;
-    SplitOperand a = {ws, na, (int) (a_trans ? padded(M, 64) : padded(K, 8)), a_trans};
-    SplitOperand b = {ws + 4 * na, nb, (int) (b_trans ? padded(N, 64) : padded(K, 8)), b_trans};
-    split_launch(ctx, a_re, a_im, ws, na, a_trans ? K : M, a_trans ? M : K, a.pitch, st);
-    CNB_LAUNCH_CHECK("split");
-    if (b_split) {                                 // a constant B operand split once by its owner, [N, K]
-        b.base = b_split;
-    } else {
-        split_launch(ctx, b_re, b_im, ws + 4 * na, nb, b_trans ? K : N, b_trans ? N : K, b.pitch, st);
-        CNB_LAUNCH_CHECK("split");
-    }
-    return cgemm_tc_presplit(ctx, a, b, conjB, r_re, r_im, d_re, d_im, M, N, K, accumulate, st);
+    cnb_pack_head* heads = reinterpret_cast<cnb_pack_head*>(ctx->d_status + 768);
+    PackRequest r[2];
+    r[0] = {a_re, a_im, a_trans ? K : M, a_trans ? M : K, operand_pitch(M, K, a_trans), ws, heads};
+    if (b_packed) r[1] = *b_packed;
+    else r[1] = {b_re, b_im, b_trans ? K : N, b_trans ? N : K, operand_pitch(N, K, b_trans), reinterpret_cast<char*>(ws) + na, heads + 1};
+    rc = pack(ctx, r, b_packed ? 1 : 2, false, st);
+    if (rc != CNB_OK) return rc;
+    return cgemm_tc_presplit(ctx, packed_operand(r[0], a_trans), packed_operand(r[1], b_trans), conjB, r_re, r_im, d_re, d_im, M, N,
+                             K, accumulate, st);
 }
 
-// the split of a constant B operand [N, K] as cgemm_tc_run takes it
-size_t cgemm_tc_operand_bytes(int N, int K) { return 4 * operand_elems(N, K, 0) * sizeof(float); }
-
-int cgemm_tc_split_operand(cnb_ctx* ctx, const float* re, const float* im, int N, int K, float* split, cudaStream_t st) {
-    split_launch(ctx, re, im, split, operand_elems(N, K, 0), N, K, (int) padded(K, 8), st);
-    CNB_LAUNCH_CHECK("split");
-    return CNB_OK;
-}
-
-int split_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, int pitch, float* split, cudaStream_t st) {
-    if ((reinterpret_cast<uintptr_t>(split) & 15) != 0) return set_error(CNB_ERR_ARG, "split: the buffer must be 16-byte aligned");
-    split_launch(ctx, re, im, split, (size_t) rows * pitch, rows, cols, pitch, st);
-    CNB_LAUNCH_CHECK("split");
-    return CNB_OK;
+static void split_launch(cnb_ctx* ctx, const float* s0, const float* s1, float* sp, size_t np, size_t n, cudaStream_t st) {
+    const size_t blocks = (n / 4 + 255) / 256 + 1, cap = (size_t) ctx->sm_count * 16;
+    cnb::launch(split_k, dim3((unsigned) std::min(blocks, cap)), dim3(256), 0, st, 1, s0, s1, sp, np, n);
 }
 
 int split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, cudaStream_t st) {
     if (((reinterpret_cast<uintptr_t>(re) | reinterpret_cast<uintptr_t>(im) | reinterpret_cast<uintptr_t>(split)) & 15) != 0)
         return set_error(CNB_ERR_ARG, "split: planes must be 16-byte aligned");
-    const size_t np = (n + 63) & ~size_t(63), blocks = (n / 4 + 255) / 256 + 1, cap = (size_t) ctx->sm_count * 16;
-    cnb::launch(split_k, dim3((unsigned) std::min(blocks, cap)), dim3(256), 0, st, 1, re, im, split, np, n);
+    split_launch(ctx, re, im, split, (n + 63) & ~size_t(63), n, st);
     CNB_LAUNCH_CHECK("split");
     return CNB_OK;
 }
@@ -1330,7 +1521,7 @@ int split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float
 extern "C" int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8) {
     if (!out8 || M <= 0 || N <= 0 || K <= 0 || sm_count <= 0)
         return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_schedule: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
-    const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit);
+    const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<SPLIT>::BK);
     out8[0] = q.pair ? 1 : 0;
     out8[1] = (int) (q.pair ? 2 * q.ctas : q.ctas);      // CTAs of the launch
     out8[2] = q.cluster * (q.pair ? 2 : 1);              // CTAs per cluster (1: no cluster)

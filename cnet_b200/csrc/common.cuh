@@ -1,6 +1,7 @@
 // Shared declarations of the device library: context, error plumbing, launch helpers.
 #pragma once
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -13,8 +14,12 @@
 struct cnb_twiddle {
     float* re = nullptr;   // [N, N] planes, F[p,q] = N^-1/2 e^{-2 pi i pq/N}
     float* im = nullptr;
-    float* split = nullptr;   // split buffer of the matrix (made once), or null when the tiles cannot take it
+    void* pack = nullptr;  // the matrix packed (made once; head, then planes), or null when the tiles cannot take it
 };
+
+// Head of a packed operand: the scale's exponent, the largest component (the bits of its magnitude) on its way to
+// becoming that, and how many blocks of the packing launch have read it.
+struct cnb_pack_head { int exponent; unsigned max_bits, ticket, unused; };
 
 struct cnb_ctx {
     int device = 0;
@@ -61,28 +66,36 @@ int cgemm_simt(cnb_ctx* ctx, const float* a_re, const float* a_im, long sam, lon
 //   D[m,n] (+)= sum_k A[m,k] * (conjB ? conj(B[n,k]) : B[n,k]) (+ R[m,n]); A [M,K], B [N,K].
 // The sizes for which it beats the SIMT tiles:
 bool cgemm_tc_shape_ok(int M, int N, int K);
-// fp32 operands, split into scratch first: a_trans / b_trans = the source planes are stored [K, rows].
+// A packed operand: fp16 high and low parts of a matrix scaled by one power of two (cgemm_tc.cu), the form that
+// everything but the C ABI's split buffers goes through.
+struct PackRequest {
+    const float* re; const float* im;  // [rows, cols]
+    int rows, cols, pitch;             // pitch of the packed rows: a multiple of 8, of 64 where they are read MN-major
+    void* planes;                      // 8 * rows * pitch bytes, 128-byte aligned
+    cnb_pack_head* head;               // zeroed before the first use
+};
+int pack(cnb_ctx* ctx, const PackRequest* r, int n, bool have_max, cudaStream_t st);
+// fp32 operands, packed into scratch first: a_trans / b_trans = the source planes are stored [K, rows]; b_packed: a
+// constant B that its owner has packed.
 int cgemm_tc_run(cnb_ctx* ctx, const float* a_re, const float* a_im, int a_trans, const float* b_re,
                  const float* b_im, int b_trans, int conjB, const float* r_re, const float* r_im, float* d_re,
                  float* d_im, int M, int N, int K, int accumulate, cudaStream_t st,
-                 const float* b_split = nullptr);
+                 const PackRequest* b_packed = nullptr);
 size_t cgemm_tc_workspace_bytes(int M, int N, int K);
-size_t cgemm_tc_operand_bytes(int N, int K);
-int cgemm_tc_split_operand(cnb_ctx* ctx, const float* re, const float* im, int N, int K, float* split, cudaStream_t st);
 // An operand that is already split (see cnb_split_component below): slots plane_pitch floats apart, stored rows
 // [rows, K] (mn = 0) or [K, rows] (mn = 1) at `pitch` elements.
 struct SplitOperand {
     const float* base;
     size_t plane_pitch;
     int pitch, mn;
+    const int* exponent;               // not NULL: a packed operand (fp16 high and low parts, cgemm_tc.cu), base its first plane
 };
 int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b, int conjB,
                       const float* r_re, const float* r_im, float* d_re, float* d_im, int M, int N, int K,
                       int accumulate, cudaStream_t st);
+SplitOperand packed_operand(const PackRequest& r, int mn);
 // split = 4 consecutive slots of pad64(n) floats (see cnb_split_component below)
 int split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, cudaStream_t st);
-// the same of a matrix, its rows at `pitch` in the split
-int split_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, int pitch, float* split, cudaStream_t st);
 
 // Skinny Linear (out <= 16): HBM-bound fp32 kernels.
 bool skinny_ok(int B, int in, int out);
@@ -99,9 +112,14 @@ bool fft_supported(int N);
 int fft_run(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, int B, int N, int inverse,
             int accumulate, cudaStream_t st);
 // Forward FFT whose epilogue also applies Hadamard(h) -> CGelu: u = FFT(x) -> (ur, ui); y = gelu(u o h) ->
-// (yr, yi) and, when sp != NULL, the operand split of y.
+// (yr, yi) and, when sp != NULL, the operand split of y; when head != NULL the largest component of y goes there.
 int fft_hadamard_gelu(cnb_ctx* ctx, const float* xr, const float* xi, const float* hr, const float* hi, float* ur,
-                      float* ui, float* yr, float* yi, float* sp, int B, int N, cudaStream_t st);
+                      float* ui, float* yr, float* yi, float* sp, cnb_pack_head* head, int B, int N, cudaStream_t st);
+
+// w -= lr g over the arena; where *have_max comes back true the heads of the matrices have received their largest new
+// components.
+int sgd_update_max(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zero_grad, const PackRequest* r, int nr,
+                   bool* have_max, cudaStream_t st);
 
 }  // namespace cnb
 
@@ -166,6 +184,20 @@ __device__ __forceinline__ void cnb_split_store4(const cnb_split_dst& d, size_t 
     b.y = (uint32_t) cnb_bf16_bits(x2 - h2) | ((uint32_t) cnb_bf16_bits(x3 - h3) << 16);
     *reinterpret_cast<uint2*>(d.h16 + i) = a;
     *reinterpret_cast<uint2*>(d.l16 + i) = b;
+}
+
+__device__ __forceinline__ unsigned cnb_abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+
+// the largest of all threads' m into a pack head; every thread of the block (at most 1024) calls it
+__device__ __forceinline__ void cnb_pack_max_block(cnb_pack_head* head, unsigned m) {
+    __shared__ unsigned warp_max[32];
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int) (blockDim.x >> 5); ++w) m = max(m, warp_max[w]);
+        atomicMax(&head->max_bits, m);
+    }
 }
 
 // Programmatic dependent launch.  Every kernel of the step is launched with the "programmatic stream

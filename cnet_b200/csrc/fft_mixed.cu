@@ -56,12 +56,13 @@ struct Io {
     const float2* src;                // shared-memory buffers, NULL: the planes
     float2* dst;
     int rows, accumulate;
+    unsigned largest;                 // of the tail's components, this thread's (bits of the magnitude)
     bool spectral;                    // chirp form: this pass opens the inverse transform
     size_t row0;
 };
 
 template <int R, bool EPI, bool CHIRP>
-__device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, const Io& io, const FftEpilogue& ep) {
+__device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io& io, const FftEpilogue& ep) {
     const int items = io.rows * d.nb;
     for (int i = threadIdx.x; i < items; i += blockDim.x) {
         const int row = div_by(i, d.mag_nb), j = i - row * d.nb;
@@ -123,10 +124,10 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, con
                     const size_t at = (io.row0 + row) * (size_t) pl.n + e;
                     if (ep.gr) { ep.gr[at] = gr; ep.gi[at] = gi; }
                     if (ep.sp) {
-                        const size_t so = (io.row0 + row) * (size_t) ep.pitch + e;
-                        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 0), so, gr);
-                        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 1), so, gi);
+                        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 0), at, gr);
+                        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 1), at, gi);
                     }
+                    io.largest = max(io.largest, max(cnb_abs_bits(gr), cnb_abs_bits(gi)));
                 }
             }
         }
@@ -147,6 +148,7 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
     io.yr = yr + io.row0 * pl.n; io.yi = yi + io.row0 * pl.n;
     io.tw = tw; io.chirp = chirp; io.spectrum = spectrum;
     io.accumulate = accumulate;
+    io.largest = 0;
     const int total = CHIRP ? 2 * pl.passes : pl.passes;
     for (int s = 0; s < total; ++s) {
         const Pass& d = pl.p[CHIRP && s >= pl.passes ? s - pl.passes : s];
@@ -161,6 +163,7 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
         }
         if (s < total - 1) __syncthreads();
     }
+    if (EPI && ep.head) cnb_pack_max_block(ep.head, io.largest);
 }
 
 // twiddles of every pass, packed as Pass::tw says, in double

@@ -50,7 +50,7 @@ struct FftEpilogue {
     float* gi = nullptr;
     float* sp = nullptr;            // operand split of that (a split buffer with plane pitch np) or NULL
     size_t np = 0;
-    size_t pitch = 0;               // elements from one row of the split to the next
+    cnb_pack_head* head = nullptr;  // receives the largest component of the values, or NULL
 };
 
 }  // namespace cnb_fft

@@ -34,6 +34,10 @@ int fft_engine(int N) { return N == 256 || N == 1024 || N == 4096 ? 3 : 5; }
 
 const int kTriKey = 1 << 28;    // twiddle-cache key offset of the triangular matrices
 
+cnb::PackRequest twiddle_pack(const cnb_twiddle& t, int N) {
+    return {t.re, t.im, N, N, (N + 7) & ~7, static_cast<char*>(t.pack) + 256, static_cast<cnb_pack_head*>(t.pack)};
+}
+
 int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) {
     const int N = key & (kTriKey - 1);
     auto it = ctx->twiddles.find(key);
@@ -53,12 +57,13 @@ int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) {
         CNB_LAUNCH_CHECK("tri_mask");
     }
     if (cnb::cgemm_tc_shape_ok(64, N, N) && (!cnb::fft_supported(N) || (key & kTriKey))) {
-        // the matrix is a constant: where the GEMM is the transform's engine, its operand split is
-        // made here, not by every product
-        rc = cnb_alloc(ctx, cnb::cgemm_tc_operand_bytes(N, N), &p);
+        // the matrix is a constant: where the GEMM is the transform's engine, it is packed here, not by every product
+        const int pitch = (N + 7) & ~7;
+        rc = cnb_alloc(ctx, 256 + 8 * (size_t) N * pitch, &t.pack);
         if (rc != CNB_OK) return rc;
-        t.split = static_cast<float*>(p);
-        rc = cnb::cgemm_tc_split_operand(ctx, t.re, t.im, N, N, t.split, st);
+        CNB_CUDA(cudaMemsetAsync(t.pack, 0, 256, st));
+        const cnb::PackRequest r = twiddle_pack(t, N);
+        rc = cnb::pack(ctx, &r, 1, false, st);
         if (rc != CNB_OK) return rc;
     }
     ctx->twiddles[key] = t;
@@ -70,8 +75,9 @@ int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) {
 int twiddle_product(cnb_ctx* ctx, const cnb_twiddle& t, const float* x_re, const float* x_im, float* y_re, float* y_im,
                     int B, int N, int conj, int accumulate, cudaStream_t st) {
     if (cnb::cgemm_tc_shape_ok(B, N, N)) {
+        const cnb::PackRequest r = twiddle_pack(t, N);
         const int rc = cnb::cgemm_tc_run(ctx, x_re, x_im, 0, t.re, t.im, 0, conj, nullptr, nullptr, y_re, y_im, B, N, N,
-                                         accumulate, st, t.split);
+                                         accumulate, st, t.pack ? &r : nullptr);
         cnb::g_last_engine = 1;
         if (rc != CNB_ERR_ARENA) return rc;
     }
@@ -201,51 +207,104 @@ int cnb_linear_split_ok(int B, int in, int out) {
 }
 
 namespace {
-inline int pitch_of(int cols) { return (cols + 63) & ~63; }
+// a split buffer of cnb_split_planes: one run of rows * cols elements, cols a multiple of 64
+inline cnb::SplitOperand split_of(const float* split, int rows, int cols, int mn) {
+    return {split, (size_t) rows * cols, cols, mn, nullptr};
+}
 
-inline cnb::SplitOperand matrix_of(const float* split, int rows, int cols, int mn) {
-    return {split, (size_t) rows * pitch_of(cols), pitch_of(cols), mn};
+// a pack of the C ABI: 256 bytes of head, then the planes with rows at a pitch of `cols` rounded up to 64, so that it
+// can be read K-major and MN-major
+inline cnb::PackRequest pack_of(const float* re, const float* im, const void* pack, int rows, int cols) {
+    char* p = static_cast<char*>(const_cast<void*>(pack));
+    return {re, im, rows, cols, (cols + 63) & ~63, p + 256, reinterpret_cast<cnb_pack_head*>(p)};
+}
+inline cnb::SplitOperand packed_of(const void* pack, int rows, int cols, int mn) {
+    return cnb::packed_operand(pack_of(nullptr, nullptr, pack, rows, cols), mn);
 }
 }  // namespace
-
-int cnb_linear_matrix_ok(int B, int in, int out) {
-    if (cnb_linear_split_ok(B, in, out)) return 1;
-    // the line of cgemm_tc_shape_ok, for all three products of a layer together (a batch of 16 rows is K of dW*)
-    return (B >= 16 && in >= 48 && out >= 17 && (double) B * in * out >= (double) (1 << 21)) ? 1 : 0;
-}
-
-size_t cnb_split_matrix_floats(int rows, int cols) { return 4 * (size_t) rows * pitch_of(cols); }
-
-int cnb_split_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, float* split, void* stream) {
-    CNB_CHECK_ARG(ctx && re && im && split && rows > 0 && cols > 0, "cnb_split_matrix: bad argument");
-    return cnb::split_matrix(ctx, re, im, rows, cols, pitch_of(cols), split, cnb::S(stream));
-}
 
 int cnb_linear_fwd_split(cnb_ctx* ctx, const float* x_split, const float* w_split, const float* res_re,
                          const float* res_im, float* y_re, float* y_im, int B, int in, int out, void* stream) {
     CNB_CHECK_ARG(ctx && x_split && w_split && y_re && y_im, "cnb_linear_fwd_split: null pointer");
-    CNB_CHECK_ARG(cnb_linear_matrix_ok(B, in, out), "cnb_linear_fwd_split: B=%d in=%d out=%d not eligible", B, in, out);
+    CNB_CHECK_ARG(cnb_linear_split_ok(B, in, out), "cnb_linear_fwd_split: B=%d in=%d out=%d not eligible", B, in, out);
     cnb::g_last_engine = 1;
-    return cnb::cgemm_tc_presplit(ctx, matrix_of(x_split, B, in, 0), matrix_of(w_split, out, in, 0), 0, res_re, res_im, y_re,
-                                  y_im, B, out, in, 0, cnb::S(stream));
+    return cnb::cgemm_tc_presplit(ctx, split_of(x_split, B, in, 0), split_of(w_split, out, in, 0), 0, res_re, res_im, y_re, y_im,
+                                  B, out, in, 0, cnb::S(stream));
 }
 
 int cnb_linear_bwd_x_split(cnb_ctx* ctx, const float* g_split, const float* w_split, float* dx_re, float* dx_im,
                            int B, int in, int out, int accumulate, void* stream) {
     CNB_CHECK_ARG(ctx && g_split && w_split && dx_re && dx_im, "cnb_linear_bwd_x_split: null pointer");
-    CNB_CHECK_ARG(cnb_linear_matrix_ok(B, in, out), "cnb_linear_bwd_x_split: B=%d in=%d out=%d not eligible", B, in, out);
+    CNB_CHECK_ARG(cnb_linear_split_ok(B, in, out), "cnb_linear_bwd_x_split: B=%d in=%d out=%d not eligible", B, in, out);
     cnb::g_last_engine = 1;                        // W [out, in] = [K, N]: MN-major B operand
-    return cnb::cgemm_tc_presplit(ctx, matrix_of(g_split, B, out, 0), matrix_of(w_split, out, in, 1), 1, nullptr, nullptr, dx_re,
+    return cnb::cgemm_tc_presplit(ctx, split_of(g_split, B, out, 0), split_of(w_split, out, in, 1), 1, nullptr, nullptr, dx_re,
                                   dx_im, B, in, out, accumulate, cnb::S(stream));
 }
 
 int cnb_linear_bwd_w_split(cnb_ctx* ctx, const float* g_split, const float* x_split, float* dw_re, float* dw_im,
                            int B, int in, int out, int accumulate, void* stream) {
     CNB_CHECK_ARG(ctx && g_split && x_split && dw_re && dw_im, "cnb_linear_bwd_w_split: null pointer");
-    CNB_CHECK_ARG(cnb_linear_matrix_ok(B, in, out), "cnb_linear_bwd_w_split: B=%d in=%d out=%d not eligible", B, in, out);
+    CNB_CHECK_ARG(cnb_linear_split_ok(B, in, out), "cnb_linear_bwd_w_split: B=%d in=%d out=%d not eligible", B, in, out);
     cnb::g_last_engine = 1;                        // G [B, out] = [K, M] and X [B, in] = [K, N]: both MN-major
-    return cnb::cgemm_tc_presplit(ctx, matrix_of(g_split, B, out, 1), matrix_of(x_split, B, in, 1), 1, nullptr, nullptr, dw_re,
+    return cnb::cgemm_tc_presplit(ctx, split_of(g_split, B, out, 1), split_of(x_split, B, in, 1), 1, nullptr, nullptr, dw_re,
                                   dw_im, out, in, B, accumulate, cnb::S(stream));
+}
+
+/* ---- packed operands ---- */
+size_t cnb_pack_bytes(int rows, int cols) { return 256 + 8 * (size_t) rows * ((cols + 63) & ~63); }
+
+int cnb_pack_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, void* pack, int have_max,
+                    void* stream) {
+    CNB_CHECK_ARG(ctx && re && im && pack && rows > 0 && cols > 0, "cnb_pack_matrix: bad argument");
+    const cnb::PackRequest r = pack_of(re, im, pack, rows, cols);
+    return cnb::pack(ctx, &r, 1, have_max != 0, cnb::S(stream));
+}
+
+int cnb_linear_pack_ok(int B, int in, int out) {
+    if (cnb_linear_split_ok(B, in, out)) return 1;
+    // the line of cgemm_tc_shape_ok, for all three products of a layer together (a batch of 16 rows is K of dW*)
+    return (B >= 16 && in >= 48 && out >= 17 && (double) B * in * out >= (double) (1 << 21)) ? 1 : 0;
+}
+
+int cnb_linear_fwd_packed(cnb_ctx* ctx, const void* x_pack, const void* w_pack, const float* res_re, const float* res_im,
+                          float* y_re, float* y_im, int B, int in, int out, void* stream) {
+    CNB_CHECK_ARG(ctx && x_pack && w_pack && y_re && y_im && B > 0 && in > 0 && out > 0, "cnb_linear_fwd_packed: bad argument");
+    cnb::g_last_engine = 1;
+    return cnb::cgemm_tc_presplit(ctx, packed_of(x_pack, B, in, 0), packed_of(w_pack, out, in, 0), 0, res_re, res_im, y_re, y_im,
+                                  B, out, in, 0, cnb::S(stream));
+}
+
+int cnb_linear_bwd_x_packed(cnb_ctx* ctx, const void* g_pack, const void* w_pack, float* dx_re, float* dx_im, int B, int in,
+                            int out, int accumulate, void* stream) {
+    CNB_CHECK_ARG(ctx && g_pack && w_pack && dx_re && dx_im && B > 0 && in > 0 && out > 0, "cnb_linear_bwd_x_packed: bad argument");
+    cnb::g_last_engine = 1;
+    return cnb::cgemm_tc_presplit(ctx, packed_of(g_pack, B, out, 0), packed_of(w_pack, out, in, 1), 1, nullptr, nullptr, dx_re,
+                                  dx_im, B, in, out, accumulate, cnb::S(stream));
+}
+
+int cnb_linear_bwd_w_packed(cnb_ctx* ctx, const void* g_pack, const void* x_pack, float* dw_re, float* dw_im, int B, int in,
+                            int out, int accumulate, void* stream) {
+    CNB_CHECK_ARG(ctx && g_pack && x_pack && dw_re && dw_im && B > 0 && in > 0 && out > 0, "cnb_linear_bwd_w_packed: bad argument");
+    cnb::g_last_engine = 1;
+    return cnb::cgemm_tc_presplit(ctx, packed_of(g_pack, B, out, 1), packed_of(x_pack, B, in, 1), 1, nullptr, nullptr, dw_re,
+                                  dw_im, out, in, B, accumulate, cnb::S(stream));
+}
+
+/* the update of a weight arena, then its packed matrices: the largest components are found while the new values pass by */
+int cnb_sgd_update_packed(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zero_grad, const cnb_pack_span* spans,
+                          int nspans, void* stream) {
+    CNB_CHECK_ARG(ctx && w && g && n > 0 && nspans >= 0 && (nspans == 0 || spans), "cnb_sgd_update_packed: bad argument");
+    std::vector<cnb::PackRequest> r;
+    for (int k = 0; k < nspans; ++k) {
+        const cnb_pack_span& s = spans[k];
+        CNB_CHECK_ARG(s.rows > 0 && s.cols > 0 && s.pack && s.re + (size_t) s.rows * s.cols <= n && s.im + (size_t) s.rows * s.cols <= n,
+                      "cnb_sgd_update_packed: matrix %d is not inside the arena", k);
+        r.push_back(pack_of(w + s.re, w + s.im, s.pack, s.rows, s.cols));
+    }
+    bool have_max = false;
+    int rc = cnb::sgd_update_max(ctx, w, g, n, lr, zero_grad, r.data(), nspans, &have_max, cnb::S(stream));
+    if (rc != CNB_OK || nspans == 0) return rc;
+    return cnb::pack(ctx, r.data(), nspans, have_max, cnb::S(stream));
 }
 
 int cnb_dft_fused_ok(int N) { return cnb::fft_supported(N) ? 1 : 0; }
@@ -258,7 +317,18 @@ int cnb_dft_hadamard_gelu_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im
                   "cnb_dft_hadamard_gelu_fwd: y planes must be a pair, and may only be left out when y_split is given");
     CNB_CHECK_ARG(B > 0 && cnb::fft_supported(N), "cnb_dft_hadamard_gelu_fwd: B=%d, N=%d is not an FFT-kernel length", B, N);
     cnb::g_last_engine = fft_engine(N);
-    return cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, y_split, B, N, cnb::S(stream));
+    return cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, y_split, nullptr, B, N, cnb::S(stream));
+}
+
+int cnb_dft_hadamard_gelu_fwd_packed(cnb_ctx* ctx, const float* x_re, const float* x_im, const float* h_re, const float* h_im,
+                                     float* u_re, float* u_im, float* y_re, float* y_im, void* y_pack, int B, int N, void* stream) {
+    CNB_CHECK_ARG(ctx && x_re && x_im && h_re && h_im && u_re && u_im && y_re && y_im && y_pack, "cnb_dft_hadamard_gelu_fwd_packed: null pointer");
+    CNB_CHECK_ARG(B > 0 && cnb::fft_supported(N), "cnb_dft_hadamard_gelu_fwd_packed: B=%d, N=%d is not an FFT-kernel length", B, N);
+    cnb::g_last_engine = fft_engine(N);
+    const cnb::PackRequest r = pack_of(y_re, y_im, y_pack, B, N);
+    const int rc = cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, nullptr, r.head, B, N, cnb::S(stream));
+    if (rc != CNB_OK) return rc;
+    return cnb::pack(ctx, &r, 1, true, cnb::S(stream));
 }
 
 int cnb_tdft_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im, float* y_re, float* y_im, int B, int N,

@@ -149,11 +149,12 @@ void FourierTrans::forward() {
 	if (fused_hg_) {
 		const Vars& h = fused_hg_->previous(1)->output();
 		Vars& y = fused_hg_->fused_gelu_->out_;
-		// the only reader of y is the Linear that takes the split planes: y itself is not stored a second time
-		float* ysplit = fused_hg_->consumerSplit();
-		fused_hg_->fused_gelu_->value_split_ = ysplit;
-		check(cnb_dft_hadamard_gelu_fwd(ctx(), x.real_, x.imag_, h.real_, h.imag_, out_.real_, out_.imag_,
-				ysplit ? nullptr : y.real_, ysplit ? nullptr : y.imag_, ysplit, batch(), in_size_, stream()));
+		if (void* pack = fused_hg_->consumerPack())
+			check(cnb_dft_hadamard_gelu_fwd_packed(ctx(), x.real_, x.imag_, h.real_, h.imag_, out_.real_, out_.imag_, y.real_,
+					y.imag_, pack, batch(), in_size_, stream()));
+		else
+			check(cnb_dft_hadamard_gelu_fwd(ctx(), x.real_, x.imag_, h.real_, h.imag_, out_.real_, out_.imag_, y.real_, y.imag_,
+					nullptr, batch(), in_size_, stream()));
 		return;
 	}
 	check(cnb_dft_fwd(ctx(), x.real_, x.imag_, out_.real_, out_.imag_, batch(), in_size_, stream()));
@@ -167,14 +168,13 @@ void FourierTrans::backward() {
 }
 
 // ----------------------------------------------------------------- Hadamard
-float* Hadamard::consumerSplit() {
-	// a Linear that is the only consumer of the GELU output gets its operand split planes from the producer
+void* Hadamard::consumerPack() {
+	// a Linear that is the only consumer of the GELU output gets its packed operand from the producer
 	if (!fused_gelu_ || fused_gelu_->no_outputs() != 1) return nullptr;
 	Linear* l = dynamic_cast<Linear*>(fused_gelu_->next(0));
-	if (l && l->use_split_ && l->previous(0) == fused_gelu_ &&
-			cnb_linear_matrix_ok(batch(), l->firstInputLength(), l->outSize())) {
-		l->x_presplit_ = true;
-		return l->x_split_;
+	if (l && l->packs() && l->previous(0) == fused_gelu_) {
+		l->x_is_packed_ = true;
+		return l->x_pack_;
 	}
 	return nullptr;
 }
@@ -185,9 +185,8 @@ void Hadamard::forward() {
 	const Vars& v = in(1);
 	if (fused_gelu_) {
 		Vars& y = fused_gelu_->out_;
-		float* ysplit = out_size_ % 64 == 0 ? consumerSplit() : nullptr;   // it writes one run, not rows at a pitch
-		check(cnb_hadamard_gelu_fwd_split(ctx(), u.real_, u.imag_, v.real_, v.imag_, out_.real_, out_.imag_, y.real_,
-				y.imag_, ysplit, batch(), out_size_, stream()));
+		check(cnb_hadamard_gelu_fwd(ctx(), u.real_, u.imag_, v.real_, v.imag_, out_.real_, out_.imag_, y.real_, y.imag_,
+				batch(), out_size_, stream()));
 		return;
 	}
 	check(cnb_hadamard_fwd(ctx(), u.real_, u.imag_, v.real_, v.imag_, prev_func_[1]->batched_ ? 1 : 0, out_.real_,
@@ -233,21 +232,24 @@ Linear::Linear(InSize in1, InSize in2)
 	  in2_len(in2.value()) {}
 
 size_t Linear::extraBytes(int batch) const {
-	if (!cnb_linear_matrix_ok(batch, in1_len, out_size_)) return 0;
-	return (cnb_split_matrix_floats(batch, in1_len) + cnb_split_matrix_floats(out_size_, in1_len)) * sizeof(float);
+	if (!cnb_linear_pack_ok(batch, in1_len, out_size_)) return 0;
+	return ((cnb_pack_bytes(batch, in1_len) + 255) & ~size_t(255)) + cnb_pack_bytes(out_size_, in1_len);
 }
 
 void Linear::bindExtra(char* mem, int batch) {
-	use_split_ = true;
-	x_split_ = reinterpret_cast<float*>(mem);
-	w_split_ = x_split_ + cnb_split_matrix_floats(batch, in1_len);
+	x_pack_ = mem;
+	w_pack_ = mem + ((cnb_pack_bytes(batch, in1_len) + 255) & ~size_t(255));
+	check(cnb_memset0(ctx(), x_pack_, 256, stream()));       // the heads start at zero
+	check(cnb_memset0(ctx(), w_pack_, 256, stream()));
 }
 
-void Linear::splitWeights() {
-	if (!use_split_) return;
+bool Linear::packs() const { return x_pack_ && cnb_linear_pack_ok(batch(), in1_len, out_size_); }
+
+void Linear::packWeights() {
+	if (!x_pack_) return;
 	const Vars& w = in(1);
-	check(cnb_split_matrix(ctx(), w.real_, w.imag_, out_size_, in1_len, w_split_, stream()));
-	w_split_version_ = net_->weights_version_;
+	check(cnb_pack_matrix(ctx(), w.real_, w.imag_, out_size_, in1_len, w_pack_, 0, stream()));
+	w_pack_version_ = net_->weights_version_;
 }
 
 void Linear::forward() {
@@ -258,13 +260,13 @@ void Linear::forward() {
 		const Vars& r = fused_residual_->previous(residual_operand_)->output();
 		rr = r.real_; ri = r.imag_;
 	}
-	if (use_split_ && cnb_linear_matrix_ok(batch(), in1_len, out_size_)) {
-		if (w_split_version_ != net_->weights_version_) splitWeights();
-		if (!x_presplit_)
-			check(cnb_split_matrix(ctx(), x.real_, x.imag_, batch(), in1_len, x_split_, stream()));
-		x_presplit_ = false;
-		check(cnb_linear_fwd_split(ctx(), x_split_, w_split_, rr, ri, out_.real_, out_.imag_, batch(), in1_len,
-				out_size_, stream()));
+	if (packs()) {
+		if (w_pack_version_ != net_->weights_version_) packWeights();
+		if (!x_is_packed_)
+			check(cnb_pack_matrix(ctx(), x.real_, x.imag_, batch(), in1_len, x_pack_, 0, stream()));
+		x_is_packed_ = false;
+		check(cnb_linear_fwd_packed(ctx(), x_pack_, w_pack_, rr, ri, out_.real_, out_.imag_, batch(), in1_len, out_size_,
+				stream()));
 		return;
 	}
 	check(cnb_linear_fwd(ctx(), x.real_, x.imag_, w.real_, w.imag_, rr, ri, out_.real_, out_.imag_, batch(), in1_len,
@@ -275,9 +277,9 @@ void Linear::backward() {
 	CFunc* px = prev_func_[0];
 	CFunc* pw = prev_func_[1];
 	int acc_x = accumulate_into(px), acc_w = accumulate_into(pw);
-	if (use_split_ && cnb_linear_matrix_ok(batch(), in1_len, out_size_)) {
-		float* gs = net_->g_split_;
-		check(cnb_split_matrix(ctx(), out_.dz_star_real_, out_.dz_star_imag_, batch(), out_size_, gs, stream()));
+	if (packs()) {
+		void* gp = net_->g_pack_;
+		check(cnb_pack_matrix(ctx(), out_.dz_star_real_, out_.dz_star_imag_, batch(), out_size_, gp, 0, stream()));
 		// Small problems give each of the 148 persistent CTAs only a few k-blocks, so prologue and
 		// epilogue dominate: run the two independent products side by side on half the SMs each.
 		const bool side_by_side = net_->side_stream_ != nullptr &&
@@ -288,18 +290,18 @@ void Linear::backward() {
 			cudaEventRecord((cudaEvent_t) net_->ev_side_fork_, ms);
 			cudaStreamWaitEvent(ss, (cudaEvent_t) net_->ev_side_fork_, 0);
 			cnb_set_gemm_sm_limit(ctx(), limit / 2);
-			check(cnb_linear_bwd_w_split(ctx(), gs, x_split_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
+			check(cnb_linear_bwd_w_packed(ctx(), gp, x_pack_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
 					in1_len, out_size_, acc_w, ss));
-			check(cnb_linear_bwd_x_split(ctx(), gs, w_split_, px->out_.dz_star_real_, px->out_.dz_star_imag_, batch(),
+			check(cnb_linear_bwd_x_packed(ctx(), gp, w_pack_, px->out_.dz_star_real_, px->out_.dz_star_imag_, batch(),
 					in1_len, out_size_, acc_x, ms));
 			cnb_set_gemm_sm_limit(ctx(), net_->dp_gemm_ctas_ > 0 ? net_->dp_gemm_ctas_ : 0);
 			cudaEventRecord((cudaEvent_t) net_->ev_side_join_, ss);
 			cudaStreamWaitEvent(ms, (cudaEvent_t) net_->ev_side_join_, 0);
 			return;
 		}
-		check(cnb_linear_bwd_w_split(ctx(), gs, x_split_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
+		check(cnb_linear_bwd_w_packed(ctx(), gp, x_pack_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
 				in1_len, out_size_, acc_w, stream()));
-		check(cnb_linear_bwd_x_split(ctx(), gs, w_split_, px->out_.dz_star_real_, px->out_.dz_star_imag_, batch(),
+		check(cnb_linear_bwd_x_packed(ctx(), gp, w_pack_, px->out_.dz_star_real_, px->out_.dz_star_imag_, batch(),
 				in1_len, out_size_, acc_x, stream()));
 		return;
 	}
@@ -597,15 +599,15 @@ size_t CNet::requiredArenaBytes(int B) const {
 		if (weight) floats += 4 * pad64(f->out_size_);
 		else floats += 4 * pad64((size_t) B * f->out_size_);
 		if (CEmbedding* e = dynamic_cast<CEmbedding*>(f)) floats += 4 * pad64((size_t) e->inSize());
-		if ((dynamic_cast<FourierTrans*>(f) && !cnb_dft_fused_ok((int) f->in_size_)) || dynamic_cast<TriangFourier*>(f))     // twiddle planes + their split
-			dft += (size_t) 2 * f->in_size_ * f->in_size_ * 4 + cnb_split_matrix_floats(f->in_size_, f->in_size_) * 4 + 1024;
+		if ((dynamic_cast<FourierTrans*>(f) && !cnb_dft_fused_ok((int) f->in_size_)) || dynamic_cast<TriangFourier*>(f))     // twiddle planes + their pack
+			dft += (size_t) 2 * f->in_size_ * f->in_size_ * 4 + cnb_pack_bytes(f->in_size_, f->in_size_) + 1024;
 		extra += f->extraBytes(B) + 256;
 	}
 	size_t gs = 0;
 	for (auto f : func_list_)
 		if (Linear* l = dynamic_cast<Linear*>(f))
-			if (cnb_linear_matrix_ok(B, l->firstInputLength(), l->outSize()))
-				gs = std::max(gs, cnb_split_matrix_floats(B, l->outSize()) * sizeof(float));
+			if (cnb_linear_pack_ok(B, l->firstInputLength(), l->outSize()))
+				gs = std::max(gs, cnb_pack_bytes(B, l->outSize()));
 	size_t staging = 0;                                // input pipeline: one staged batch + labels
 	if (!func_list_.empty()) {
 		CFunc* f0 = func_list_.front();
@@ -806,10 +808,11 @@ bool CNet::allocateOnGpu(int B) {
 		size_t gs = 0;
 		for (auto f : func_list_)
 			if (Linear* l = dynamic_cast<Linear*>(f))
-				if (l->use_split_) gs = std::max(gs, cnb_split_matrix_floats(B, l->outSize()) * sizeof(float));
+				if (l->x_pack_) gs = std::max(gs, cnb_pack_bytes(B, l->outSize()));
 		if (gs) {
-			if ((rc = cnb_alloc(ctx_, gs, &p)) != CNB_OK) { fail(rc, "gradient split planes"); return false; }
-			g_split_ = static_cast<float*>(p);
+			if ((rc = cnb_alloc(ctx_, gs, &p)) != CNB_OK) { fail(rc, "packed gradient"); return false; }
+			g_pack_ = p;
+			cnb_memset0(ctx_, g_pack_, 256, stream_);
 		}
 	}
 	// 3. upload the host copies of the weights
@@ -839,7 +842,7 @@ bool CNet::setInputValues(int uid, const float* re, const float* im, int len) {
 	if (rc == CNB_OK) rc = cnb_sync(ctx_, stream_);
 	if (rc != CNB_OK) { fail(rc, "setInputValues"); return false; }
 	++weights_version_;
-	// a captured step holds no launch that re-splits the Linear weights: it would multiply by the old ones
+	// a captured step holds no launch that re-packs the Linear weights: it would multiply by the old ones
 	if (graph_exec_) graph_stale_ = "weights were set from the host after the step was captured";
 	return true;
 }
@@ -1182,7 +1185,7 @@ bool CNet::endCapture() {
 
 bool CNet::launchGraph() {
 	if (!graph_exec_) { fail(CNB_ERR_ARG, "launchGraph: capture a step first"); return false; }
-	// grids, row counts and the "weights are already split" decision were frozen at capture time
+	// grids, row counts and the "weights are already packed" decision were frozen at capture time
 	if (cur_batch_ != graph_batch_) {
 		fail(CNB_ERR_ARG, "launchGraph: the batch in flight has " + std::to_string(cur_batch_) + " rows, the captured step was sized for " +
 				std::to_string(graph_batch_) + "; capture again");
@@ -1204,32 +1207,27 @@ void CNet::updateInputs(float lr) {
 	if (!ctx_ || !wgrad_count_) return;
 	if (dp_gemm_ctas_ > 0) cnb_set_gemm_sm_limit(ctx_, 0);
 	if (!joinCollectives()) return;
-	// the new Linear weights leave the update already split, once, for the next forward and dX* products
-	std::vector<cnb_split_span> spans;
+	// the new Linear weights leave the update already packed, once, for the next forward and dX* products
+	std::vector<cnb_pack_span> spans;
 	std::vector<Linear*> fused;
 	for (auto f : func_list_) {
 		Linear* l = dynamic_cast<Linear*>(f);
-		if (!l || !l->use_split_ || spans.size() + 2 > CNB_MAX_SPLIT_SPANS || wgrad_count_ % 4) continue;
+		if (!l || !l->x_pack_) continue;
 		const Vars& w = l->prev_func_[1]->out_;
-		const size_t np = cnb_split_matrix_floats(l->out_size_, l->in1_len) / 4;
-		if (l->in1_len % 64 || w.real_ < weight_base_ || w.imag_ + l->in2_len > weight_base_ + wgrad_count_) continue;
-		// slots of the split buffer: hi_re, hi_im (fp32), then [h16_re ; h16_im] and [l16_re ; l16_im] as bf16
-		uint16_t* h16 = reinterpret_cast<uint16_t*>(l->w_split_ + 2 * np);
-		uint16_t* l16 = reinterpret_cast<uint16_t*>(l->w_split_ + 3 * np);
-		spans.push_back({(size_t) (w.real_ - weight_base_), (size_t) l->in2_len, l->w_split_, h16, l16});
-		spans.push_back({(size_t) (w.imag_ - weight_base_), (size_t) l->in2_len, l->w_split_ + np, h16 + np, l16 + np});
+		if (w.real_ < weight_base_ || w.imag_ + l->in2_len > weight_base_ + wgrad_count_) continue;
+		spans.push_back({(size_t) (w.real_ - weight_base_), (size_t) (w.imag_ - weight_base_), l->out_size_, l->in1_len, l->w_pack_});
 		fused.push_back(l);
 	}
 	int rc = spans.empty()
 		? cnb_sgd_update(ctx_, weight_base_, wgrad_base_, wgrad_count_, lr, 1, stream_)
-		: cnb_sgd_update_split(ctx_, weight_base_, wgrad_base_, wgrad_count_, lr, 1, spans.data(), (int) spans.size(), stream_);
+		: cnb_sgd_update_packed(ctx_, weight_base_, wgrad_base_, wgrad_count_, lr, 1, spans.data(), (int) spans.size(), stream_);
 	if (rc != CNB_OK) { fail(rc, "updateInputs"); return; }
 	reduced_since_update_ = false;
 	++weights_version_;
-	for (auto l : fused) l->w_split_version_ = weights_version_;
+	for (auto l : fused) l->w_pack_version_ = weights_version_;
 	for (auto f : func_list_)
 		if (Linear* l = dynamic_cast<Linear*>(f))
-			if (l->w_split_version_ != weights_version_) l->splitWeights();
+			if (l->w_pack_version_ != weights_version_) l->packWeights();
 }
 
 void CNet::adamUpdate(float lr, float beta, int t) {
@@ -1253,7 +1251,7 @@ void CNet::adamUpdate(float lr, float beta, int t) {
 	reduced_since_update_ = false;
 	++weights_version_;
 	for (auto f : func_list_)
-		if (Linear* l = dynamic_cast<Linear*>(f)) l->splitWeights();
+		if (Linear* l = dynamic_cast<Linear*>(f)) l->packWeights();
 }
 
 void CNet::infer() {
@@ -1320,30 +1318,6 @@ bool CNet::readOutput(int uid, int what, float* re, float* im) {
 	if (what != 0 && f->grad_transient_) sr = nullptr;       // overwritten by the gradient of the Residual's operand
 	if (!sr) { fail(CNB_ERR_ARG, f->getName() + ": tensor not materialised (fused)"); return false; }
 	size_t n = (size_t) (f->batched_ ? cur_batch_ : 1) * f->out_size_;
-	if (what == 0 && f->value_split_) {
-		// Only the operand split of the value was stored: hi (the value cut to TF32) plus the bf16 rounding of
-		// the remainder gives it back to 2^-19 relative, which is what the consuming product saw of it.
-		const size_t np = cnb_split_matrix_floats(cur_batch_, f->out_size_) / 4;   // plane pitch of the batch in flight
-		const size_t pitch = np / cur_batch_;
-		std::vector<float> hi(np);
-		std::vector<uint16_t> lo(np);
-		const uint16_t* l16 = reinterpret_cast<const uint16_t*>(f->value_split_ + 3 * np);
-		for (int q = 0; q < 2; ++q) {
-			float* dst = q ? im : re;
-			int rc = cnb_d2h(ctx_, hi.data(), f->value_split_ + q * np, np * sizeof(float), stream_);
-			if (rc == CNB_OK) rc = cnb_d2h(ctx_, lo.data(), l16 + q * np, np * sizeof(uint16_t), stream_);
-			if (rc == CNB_OK) rc = cnb_sync(ctx_, stream_);
-			if (rc != CNB_OK) { fail(rc, "readOutput"); return false; }
-			for (size_t k = 0; k < n; ++k) {
-				const size_t at = k / f->out_size_ * pitch + k % f->out_size_;
-				const uint32_t bits = (uint32_t) lo[at] << 16;
-				float v;
-				std::memcpy(&v, &bits, sizeof v);
-				dst[k] = hi[at] + v;
-			}
-		}
-		return true;
-	}
 	int rc = cnb_d2h(ctx_, re, sr, n * sizeof(float), stream_);
 	if (rc == CNB_OK) rc = cnb_d2h(ctx_, im, si, n * sizeof(float), stream_);
 	if (rc != CNB_OK) { fail(rc, "readOutput"); return false; }

@@ -141,7 +141,6 @@ public:
 	Vars out_;
 	bool batched_ = true;        // false: one row shared by the batch (weights)
 	bool grad_written_ = false;  // has a consumer already written dL/dz* of out_ in this backward?
-	const float* value_split_ = nullptr; // value planes are not stored: out = hi + l16 of this split buffer (the value to 2^-19)
 	bool grad_transient_ = false; // dL/dz* planes are shared with a Residual operand and accumulated over in place
 	bool fused_away_ = false;    // a neighbour's fused kernel does this layer's work
 
@@ -241,7 +240,7 @@ class Hadamard : public CFunc {                     // impl/hadamard.h:11-107
 	friend class FourierTrans;
 	CFunc* fused_gelu_ = nullptr;                   // Hadamard(shared h) -> CGelu run as one kernel pair
 	bool in_fft_epilogue_ = false;                  // the producing FourierTrans computes this layer's forward
-	float* consumerSplit();                         // split planes of the Linear fed by the fused GELU, or NULL
+	void* consumerPack();                           // packed operand of the Linear fed by the fused GELU, or NULL
 public:
 	Hadamard(Uid uid, InSize a, InSize b) : CFunc(uid, InSize(a.value() + b.value()), OutSize(a.value())) {}
 	Hadamard(InSize a, InSize b) : CFunc(InSize(a.value() + b.value()), OutSize(a.value())) {}
@@ -267,16 +266,16 @@ class Linear : public CFunc {                       // impl/linear.h:11-156
 	int in1_len, in2_len;
 	CFunc* fused_residual_ = nullptr;               // Residual add done in the GEMM epilogue
 	int residual_operand_ = 0;                      // which Residual input is the other addend
-	// operand split buffers kept by the layer: x is split in forward() and reused by dW*, W is
-	// split when the weights change and reused by forward and dX*
-	float* x_split_ = nullptr;
-	float* w_split_ = nullptr;
-	bool use_split_ = false;
-	bool x_presplit_ = false;                       // the producer of x writes x_split_ itself
-	unsigned long long w_split_version_ = ~0ull;
+	// packed operands kept by the layer: x is packed in forward() and reused by dW*, W is packed when the weights
+	// change and reused by forward and dX*; NULL where the layer runs on raw planes
+	void* x_pack_ = nullptr;
+	void* w_pack_ = nullptr;
+	bool x_is_packed_ = false;                      // the producer of x has written x_pack_ itself
+	unsigned long long w_pack_version_ = ~0ull;
+	bool packs() const;                             // the batch in flight runs on packed operands
 	size_t extraBytes(int batch) const override;
 	void bindExtra(char* mem, int batch) override;
-	void splitWeights();
+	void packWeights();
 public:
 	Linear(Uid uid, InSize in1, InSize in2);
 	Linear(InSize in1, InSize in2);
@@ -409,7 +408,7 @@ class CNet {
 	void* hook_user_ = nullptr;
 	int dp_gemm_ctas_ = 0;                          // GEMM grid cap while all-reduces are in flight
 	unsigned long long weights_version_ = 0;        // bumped whenever weight values change
-	float* g_split_ = nullptr;                      // shared split planes of a Linear's output gradient
+	void* g_pack_ = nullptr;                        // shared packed operand: a Linear's output gradient
 	void* side_stream_ = nullptr;                   // second compute stream: dW* runs beside dX* at small batches
 	void* ev_side_fork_ = nullptr;
 	void* ev_side_join_ = nullptr;

@@ -45,12 +45,17 @@ SIGNATURES = {
     "cnb_split_floats": (_sz, [_sz]),
     "cnb_split_planes": (C.c_int, [_vp, _P, _P, _sz, _P, _vp]),
     "cnb_linear_split_ok": (C.c_int, [C.c_int, C.c_int, C.c_int]),
-    "cnb_linear_matrix_ok": (C.c_int, [C.c_int, C.c_int, C.c_int]),
-    "cnb_split_matrix_floats": (_sz, [C.c_int, C.c_int]),
-    "cnb_split_matrix": (C.c_int, [_vp, _P, _P, C.c_int, C.c_int, _P, _vp]),
     "cnb_linear_fwd_split": (C.c_int, [_vp] + [_P] * 6 + [C.c_int] * 3 + [_vp]),
     "cnb_linear_bwd_x_split": (C.c_int, [_vp] + [_P] * 4 + [C.c_int] * 4 + [_vp]),
     "cnb_linear_bwd_w_split": (C.c_int, [_vp] + [_P] * 4 + [C.c_int] * 4 + [_vp]),
+    "cnb_pack_bytes": (_sz, [C.c_int, C.c_int]),
+    "cnb_pack_matrix": (C.c_int, [_vp, _P, _P, C.c_int, C.c_int, _P, C.c_int, _vp]),
+    "cnb_linear_pack_ok": (C.c_int, [C.c_int, C.c_int, C.c_int]),
+    "cnb_linear_fwd_packed": (C.c_int, [_vp] + [_P] * 6 + [C.c_int] * 3 + [_vp]),
+    "cnb_linear_bwd_x_packed": (C.c_int, [_vp] + [_P] * 4 + [C.c_int] * 4 + [_vp]),
+    "cnb_linear_bwd_w_packed": (C.c_int, [_vp] + [_P] * 4 + [C.c_int] * 4 + [_vp]),
+    "cnb_dft_hadamard_gelu_fwd_packed": (C.c_int, [_vp] + [_P] * 9 + [C.c_int] * 2 + [_vp]),
+    "cnb_sgd_update_packed": (C.c_int, [_vp, _P, _P, _sz, C.c_float, C.c_int, _vp, C.c_int, _vp]),
     "cnb_set_gemm_sm_limit": (C.c_int, [_vp, C.c_int]),
     "cnb_last_gemm_engine": (C.c_int, []),
     "cnb_linear_workspace": (_sz, [C.c_int, C.c_int, C.c_int]),

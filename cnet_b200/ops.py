@@ -120,7 +120,7 @@ class Context:
         B, N = x[0].shape
         u = u if u is not None else self._new(B, N)
         if split is None:
-            split = self.torch.empty(self.lib.cnb_split_matrix_floats(B, N), dtype=self.torch.float32, device="cuda")
+            split = self.torch.empty(self.lib.cnb_split_floats(B * N), dtype=self.torch.float32, device="cuda")
         _lib.check(self.lib.cnb_dft_hadamard_gelu_fwd(self.h, _p(x[0]), _p(x[1]), _p(h[0]), _p(h[1]), _p(u[0]), _p(u[1]),
                                                       None, None, _p(split), B, N, self._stream()), "dft_hadamard_gelu_fwd")
         return u, split

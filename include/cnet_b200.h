@@ -118,13 +118,6 @@ int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_
 size_t cnb_split_floats(size_t n);
 int cnb_split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, void* stream);
 int cnb_linear_split_ok(int B, int in, int out);
-/* The same for a layer of any sizes large enough to be worth it (cnb_linear_matrix_ok; every cnb_linear_split_ok one
- * is): the split of a matrix keeps its rows at a pitch of `cols` rounded up to 64 elements, so np = rows * pitch above
- * and the buffer holds cnb_split_matrix_floats(rows, cols) floats; with cols a multiple of 64 it is
- * cnb_split_planes' own.  The three _split products below take X [B, in], W [out, in] and G [B, out] so. */
-int cnb_linear_matrix_ok(int B, int in, int out);
-size_t cnb_split_matrix_floats(int rows, int cols);
-int cnb_split_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, float* split, void* stream);
 int cnb_linear_fwd_split(cnb_ctx* ctx, const float* x_split, const float* w_split,
                          const float* res_re, const float* res_im,
                          float* y_re, float* y_im, int B, int in, int out, void* stream);
@@ -132,6 +125,26 @@ int cnb_linear_bwd_x_split(cnb_ctx* ctx, const float* g_split, const float* w_sp
                            float* dx_re, float* dx_im, int B, int in, int out, int accumulate, void* stream);
 int cnb_linear_bwd_w_split(cnb_ctx* ctx, const float* g_split, const float* x_split,
                            float* dw_re, float* dw_im, int B, int in, int out, int accumulate, void* stream);
+/* Packed operands: what the raw-plane products above and the host facade put through the tensor cores.  A matrix is
+ * scaled by one power of two that brings its largest component into [2^14, 2^15) and kept as two fp16 parts,
+ * high = fp16(x) and low = fp16(x - high): 22 bits of every component down to 2^-18 of the largest, then gradually
+ * fewer, an absolute error of 2^-40 of the largest at most.  A product is high.high + high.low + low.high on the
+ * FP16 pipe with fp32 accumulation and takes the scales out again.  A pack is cnb_pack_bytes(rows, cols) of 256-byte
+ * aligned memory, its first 256 bytes zeroed once before the first use: [0, 256) the head, then as fp16 the planes
+ * high re, high im, low re, low im, rows at a pitch of `cols` rounded up to 64.  Any sizes; cnb_linear_pack_ok says
+ * for which a layer gains by it.  have_max: a kernel before has left the largest component in the head
+ * (cnb_dft_hadamard_gelu_fwd_packed, cnb_sgd_update_packed do), otherwise a pass over the matrix finds it.  Same
+ * reference call sites as cnb_linear_fwd / _bwd_x / _bwd_w. */
+size_t cnb_pack_bytes(int rows, int cols);
+int cnb_pack_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, void* pack, int have_max,
+                    void* stream);
+int cnb_linear_pack_ok(int B, int in, int out);
+int cnb_linear_fwd_packed(cnb_ctx* ctx, const void* x_pack, const void* w_pack, const float* res_re, const float* res_im,
+                          float* y_re, float* y_im, int B, int in, int out, void* stream);
+int cnb_linear_bwd_x_packed(cnb_ctx* ctx, const void* g_pack, const void* w_pack, float* dx_re, float* dx_im, int B, int in,
+                            int out, int accumulate, void* stream);
+int cnb_linear_bwd_w_packed(cnb_ctx* ctx, const void* g_pack, const void* x_pack, float* dw_re, float* dw_im, int B, int in,
+                            int out, int accumulate, void* stream);
 /* The tensor-core GEMM is persistent (one CTA per SM, all shared memory).  max_ctas > 0 caps its
  * grid so that the remaining SMs stay free for kernels that must run beside it (the gradient
  * all-reduce of a data-parallel job); 0 restores the full grid.  No reference counterpart. */
@@ -154,7 +167,7 @@ int cnb_dft_bwd(cnb_ctx* ctx, const float* g_re, const float* g_im,
                 float* dx_re, float* dx_im, int B, int N, int accumulate, void* stream);
 /* FourierTrans -> Hadamard(shared h) -> CGelu in one pass over the row (the N that have an FFT kernel, see
  * cnb_dft_fused_ok): u = DFT(x) is kept for the backward, y = gelu(u o h), optionally with the
- * operand split of y for the Linear that follows (rows at a pitch of N rounded up to 64); y_re = y_im = NULL is allowed when y_split
+ * operand split of y for the Linear that follows; y_re = y_im = NULL is allowed when y_split
  * is given (hi + l16 of the split is y to 2^-19, all the product sees of it, so a caller that only feeds the
  * Linear need not store y twice).
  * The Hadamard product a = u o h is not stored: cnb_hadamard_gelu_bwd recomputes it when a_re == NULL.  Same reference kernels as
@@ -164,6 +177,9 @@ int cnb_dft_hadamard_gelu_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im
                               const float* h_re, const float* h_im,
                               float* u_re, float* u_im, float* y_re, float* y_im,
                               float* y_split, int B, int N, void* stream);
+/* The same with y stored and packed for the products of the Linear that follows (a pack of [B, N]). */
+int cnb_dft_hadamard_gelu_fwd_packed(cnb_ctx* ctx, const float* x_re, const float* x_im, const float* h_re, const float* h_im,
+                                     float* u_re, float* u_im, float* y_re, float* y_im, void* y_pack, int B, int N, void* stream);
 /* TriangFourier: Y[b,p] = N^-1/2 sum_{q <= p} X[b,q] e^{-2 pi i pq/N} and its backward
  * dX*[b,q] (+)= N^-1/2 sum_{p >= q} G*[b,p] e^{+2 pi i pq/N}: the complex GEMM against the
  * lower-triangular twiddle matrix.  Replaces TrianFourierGpu::gpu_T_fft_forward / _backward
@@ -321,6 +337,11 @@ int cnb_sgd_update(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zer
 typedef struct cnb_split_span { size_t begin; size_t count; float* hi; void* h16; void* l16; } cnb_split_span;
 int cnb_sgd_update_split(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zero_grad,
                          const cnb_split_span* spans, int nspans, void* stream);
+
+/* The same update, after which the given matrices of the arena (planes at w + re and w + im) lie packed in `pack`. */
+typedef struct cnb_pack_span { size_t re; size_t im; int rows; int cols; void* pack; } cnb_pack_span;
+int cnb_sgd_update_packed(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zero_grad,
+                          const cnb_pack_span* spans, int nspans, void* stream);
 
 /* The reference's momentum-only "Adam": m = beta m + (1 - beta) g; w -= lr m / (1 - beta^(t+1));
  * g = 0.  Replaces gpu_update_adam_input (gpu/kernels.h:77, gpu/kernels.cpp:494-525).

@@ -35,9 +35,8 @@ def test_mixed_radix_lengths(ctx, B, N):  # noqa: F811
 
 
 def _unsplit(split, B, N):
-    """hi + l16 of both planes of a split buffer whose rows lie at a pitch of N rounded up to 64."""
+    """hi + l16 of both planes of a split buffer."""
     import torch
-    pitch = (N + 63) // 64 * 64
-    n = B * pitch
-    lo = split[3 * n:4 * n].view(torch.bfloat16).float()
-    return tuple((split[q * n:(q + 1) * n] + lo[q * n:(q + 1) * n]).view(B, pitch)[:, :N].cpu().numpy() for q in range(2))
+    np_ = split.numel() // 4
+    lo = split[3 * np_:].view(torch.bfloat16).float()
+    return tuple((split[q * np_:(q + 1) * np_] + lo[q * np_:(q + 1) * np_])[:B * N].view(B, N).cpu().numpy() for q in range(2))
