@@ -1,7 +1,14 @@
-// Row reductions of the complex training step: L2 normalisation (the reference's
-// "SoftMax") forward/backward and the fused CrossEntropy forward + backward seed.
-// One CTA per sample row; warp-shuffle tree + one shared-memory hop.  Rows are read once
-// for the reduction and once (from L2/L1) for the element-wise pass.
+// Row reductions of the complex training step: L2 normalisation (the reference's "SoftMax") forward / backward, the
+// fused CrossEntropy forward + backward seed, and L2Out.
+//
+// All are HBM-bound: a row is read once and kept in registers between its reduction and the element-wise pass.  G
+// threads share a row and hold E elements of every plane each, so that a row of any usual length finds a form in which
+// most of them work and enough loads are in flight: 8 lanes (rows up to 32, four rows to a warp), a warp (up to 512), a
+// CTA of 128 (2048) or 512 threads (8192), a cluster of up to eight such CTAs (65536, partial sums through distributed
+// shared memory).  16-byte accesses where the row length and the planes allow them, else consecutive threads take
+// consecutive elements.  65536 x 20 through a CTA of one warp per row took 69 us a kernel, 300 x 27000 through two
+// passes over each row 60 to 82.
+#include <algorithm>
 #include <initializer_list>
 
 #include "common.cuh"
@@ -26,8 +33,171 @@ __device__ __forceinline__ float block_sum(float v, float* smem) {
     return r;
 }
 
-__global__ void softmax_fwd_k(const float* __restrict__ zr, const float* __restrict__ zi,
-                              float* __restrict__ yr, float* __restrict__ yi, float* __restrict__ inv_norm, int N) {
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Sum over the G threads of a row, or over the whole cluster when it has `parts` CTAs; valid in every thread.
+template <int G> __device__ __forceinline__ float row_sum(float v, int parts) {
+    if constexpr (G <= 32) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    } else {
+        __shared__ float sm[32], part;
+        v = block_sum(v, sm);
+        if (parts > 1) {
+            if (threadIdx.x == 0) part = v;
+            cluster_sync();
+            const uint32_t local = (uint32_t) __cvta_generic_to_shared(&part);
+            v = 0.f;
+            for (int c = 0; c < parts; ++c) {                // the same order in every CTA
+                uint32_t remote;
+                float x;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(c));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote) : "memory");
+                v += x;
+            }
+            cluster_sync();                                  // no CTA leaves while a peer still reads its part
+        }
+        return v;
+    }
+}
+
+// What a thread holds of a row: element k is at at(k).
+template <int G, int E, int VEC> struct Tile {
+    size_t base;                    // first element of the row
+    int t0, n;                      // this thread's place among the row's, row length
+    bool live;
+    int row;
+
+    __device__ __forceinline__ Tile(int rows, int n_, int parts) : n(n_) {
+        if constexpr (G <= 32) {
+            row = (int) ((blockIdx.x * (unsigned) blockDim.x + threadIdx.x) / G);
+            t0 = threadIdx.x % G;
+        } else {
+            row = (int) (blockIdx.x / (unsigned) parts);
+            t0 = threadIdx.x + (int) (blockIdx.x % (unsigned) parts) * G;
+        }
+        live = row < rows;
+        base = (size_t) row * n;
+        stride = (G <= 32 ? 1 : parts) * G;
+    }
+    int stride;                     // threads on the row, over all CTAs of its cluster
+    __device__ __forceinline__ int at(int k) const { return VEC == 4 ? 4 * (t0 + (k / 4) * stride) + k % 4 : t0 + k * stride; }
+    __device__ __forceinline__ void load(const float* p, float (&v)[E]) const {
+#pragma unroll
+        for (int k = 0; k < E; k += VEC) {
+            const bool on = live && at(k) < n;
+            if constexpr (VEC == 4) {
+                const float4 x = on ? *reinterpret_cast<const float4*>(p + base + at(k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[k] = x.x; v[k + 1] = x.y; v[k + 2] = x.z; v[k + 3] = x.w;
+            } else {
+                v[k] = on ? p[base + at(k)] : 0.f;
+            }
+        }
+    }
+    __device__ __forceinline__ void store(float* p, const float (&v)[E]) const {
+#pragma unroll
+        for (int k = 0; k < E; k += VEC) {
+            if (!live || at(k) >= n) continue;
+            if constexpr (VEC == 4) *reinterpret_cast<float4*>(p + base + at(k)) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+            else p[base + at(k)] = v[k];
+        }
+    }
+};
+
+constexpr int cta_threads(int g) { return g < 128 ? 256 : g; }
+
+template <int G, int E, int VEC>
+__global__ void __launch_bounds__(cta_threads(G))
+softmax_fwd_k(const float* __restrict__ zr, const float* __restrict__ zi, float* __restrict__ yr, float* __restrict__ yi,
+              float* __restrict__ inv_norm, int rows, int n, int parts) {
+    cnb_pdl_enter();
+    const Tile<G, E, VEC> t(rows, n, parts);
+    float a[E], b[E], s = 0.f;
+    t.load(zr, a); t.load(zi, b);
+#pragma unroll
+    for (int k = 0; k < E; ++k) s += a[k] * a[k] + b[k] * b[k];
+    s = row_sum<G>(s, parts);
+    const float inv = 1.0f / fmaxf(sqrtf(s), 1e-15f);
+    if (t.live && t.t0 == 0) inv_norm[t.row] = inv;
+#pragma unroll
+    for (int k = 0; k < E; ++k) { a[k] *= inv; b[k] *= inv; }
+    t.store(yr, a); t.store(yi, b);
+}
+
+template <int G, int E, int VEC>
+__global__ void __launch_bounds__(cta_threads(G))
+softmax_bwd_k(const float* __restrict__ gr, const float* __restrict__ gi, const float* __restrict__ zr,
+              const float* __restrict__ zi, const float* __restrict__ inv_norm, float* __restrict__ dr,
+              float* __restrict__ di, int rows, int n, int parts, int accumulate) {
+    cnb_pdl_enter();
+    const Tile<G, E, VEC> t(rows, n, parts);
+    float a[E], b[E], x[E], y[E], s = 0.f;
+    t.load(gr, a); t.load(gi, b); t.load(zr, x); t.load(zi, y);
+    const float inv = t.live ? inv_norm[t.row] : 0.f;
+#pragma unroll
+    for (int k = 0; k < E; ++k) s += a[k] * x[k] + b[k] * y[k];          // Re(g* conj(z))
+    s = row_sum<G>(s, parts);
+    const float c = s * inv * inv * inv;
+#pragma unroll
+    for (int k = 0; k < E; ++k) { a[k] = a[k] * inv - x[k] * c; b[k] = b[k] * inv - y[k] * c; }
+    if (accumulate) {
+        t.load(dr, x); t.load(di, y);
+#pragma unroll
+        for (int k = 0; k < E; ++k) { a[k] += x[k]; b[k] += y[k]; }
+    }
+    t.store(dr, a); t.store(di, b);
+}
+
+template <int G, int E, int VEC>
+__global__ void __launch_bounds__(cta_threads(G))
+crossent_k(const float* __restrict__ zr, const float* __restrict__ zi, const int32_t* __restrict__ labels,
+           float* __restrict__ loss, float* __restrict__ dr, float* __restrict__ di, int rows, int n, int parts) {
+    cnb_pdl_enter();
+    const Tile<G, E, VEC> t(rows, n, parts);
+    const int l = t.live ? min(max(labels[t.row], 0), n - 1) : 0;
+    float a[E], b[E], s = 0.f;
+    t.load(zr, a); t.load(zi, b);
+    // the label's element, asked for again (it is on its way to this SM) rather than passed between threads
+    const float lr = t.live ? zr[t.base + l] : 0.f, li = t.live ? zi[t.base + l] : 0.f;
+#pragma unroll
+    for (int k = 0; k < E; ++k) s += a[k] * a[k] + b[k] * b[k];
+    s = row_sum<G>(s, parts);
+    const float S = fmaxf(s, 1e-15f), m2 = lr * lr + li * li;
+    if (t.live && t.t0 == 0) loss[t.row] = -logf(fmaxf(m2 / S, 1e-15f));
+    if (dr == nullptr) return;
+    const float m = fmaxf(m2, 1e-15f);
+    const float cl = -(S - m) / (m * S), co = 1.0f / S;
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        const float c = t.at(k) == l ? cl : co;
+        a[k] *= c; b[k] *= c;
+    }
+    t.store(dr, a); t.store(di, b);
+}
+
+// L2Out: loss[b] = sum |z|^2; seed dz* = z
+template <int G, int E, int VEC>
+__global__ void __launch_bounds__(cta_threads(G))
+l2out_k(const float* __restrict__ zr, const float* __restrict__ zi, float* __restrict__ loss, float* __restrict__ dr,
+        float* __restrict__ di, int rows, int n, int parts) {
+    cnb_pdl_enter();
+    const Tile<G, E, VEC> t(rows, n, parts);
+    float a[E], b[E], s = 0.f;
+    t.load(zr, a); t.load(zi, b);
+#pragma unroll
+    for (int k = 0; k < E; ++k) s += a[k] * a[k] + b[k] * b[k];
+    if (dr) { t.store(dr, a); t.store(di, b); }
+    s = row_sum<G>(s, parts);
+    if (t.live && t.t0 == 0) loss[t.row] = s;
+}
+
+// Rows beyond the longest cluster: one CTA reads the row once to reduce and again for the element-wise pass.
+__global__ void softmax_fwd_long_k(const float* __restrict__ zr, const float* __restrict__ zi,
+                                   float* __restrict__ yr, float* __restrict__ yi, float* __restrict__ inv_norm, int N) {
     cnb_pdl_enter();
     __shared__ float sm[32];
     size_t base = (size_t) blockIdx.x * N;
@@ -46,10 +216,10 @@ __global__ void softmax_fwd_k(const float* __restrict__ zr, const float* __restr
     }
 }
 
-__global__ void softmax_bwd_k(const float* __restrict__ gr, const float* __restrict__ gi,
-                              const float* __restrict__ zr, const float* __restrict__ zi,
-                              const float* __restrict__ inv_norm, float* __restrict__ dr, float* __restrict__ di,
-                              int N, int accumulate) {
+__global__ void softmax_bwd_long_k(const float* __restrict__ gr, const float* __restrict__ gi,
+                                   const float* __restrict__ zr, const float* __restrict__ zi,
+                                   const float* __restrict__ inv_norm, float* __restrict__ dr, float* __restrict__ di,
+                                   int N, int accumulate) {
     cnb_pdl_enter();
     __shared__ float sm[32];
     size_t base = (size_t) blockIdx.x * N;
@@ -67,9 +237,9 @@ __global__ void softmax_bwd_k(const float* __restrict__ gr, const float* __restr
     }
 }
 
-__global__ void crossent_k(const float* __restrict__ zr, const float* __restrict__ zi,
-                           const int32_t* __restrict__ labels, float* __restrict__ loss,
-                           float* __restrict__ dr, float* __restrict__ di, int M) {
+__global__ void crossent_long_k(const float* __restrict__ zr, const float* __restrict__ zi,
+                                const int32_t* __restrict__ labels, float* __restrict__ loss,
+                                float* __restrict__ dr, float* __restrict__ di, int M) {
     cnb_pdl_enter();
     __shared__ float sm[32];
     size_t base = (size_t) blockIdx.x * M;
@@ -95,9 +265,8 @@ __global__ void crossent_k(const float* __restrict__ zr, const float* __restrict
     }
 }
 
-// L2Out: loss[b] = sum |z|^2; seed dz* = z
-__global__ void l2out_k(const float* __restrict__ zr, const float* __restrict__ zi, float* __restrict__ loss,
-                        float* __restrict__ dr, float* __restrict__ di, int N) {
+__global__ void l2out_long_k(const float* __restrict__ zr, const float* __restrict__ zi, float* __restrict__ loss,
+                             float* __restrict__ dr, float* __restrict__ di, int N) {
     cnb_pdl_enter();
     __shared__ float sm[32];
     size_t base = (size_t) blockIdx.x * N;
@@ -111,136 +280,36 @@ __global__ void l2out_k(const float* __restrict__ zr, const float* __restrict__ 
     if (threadIdx.x == 0) loss[blockIdx.x] = s;
 }
 
-// Register-cached forms for rows of up to 16-byte-aligned 4 * CACHE * blockDim floats: the row is read ONCE
-// with 16-byte loads, kept in registers across the reduction, and the element-wise pass works from the
-// registers (the two-pass kernels above read the row a second time; at 8192 columns that second read is
-// what kept them at ~0.55 of the copy bandwidth).
-constexpr int CACHE = 4;         // float4 per plane and thread
-
-__device__ __forceinline__ float4 ld4(const float* p, size_t i) { return *reinterpret_cast<const float4*>(p + i); }
-__device__ __forceinline__ void st4(float* p, size_t i, float4 v) { *reinterpret_cast<float4*>(p + i) = v; }
-__device__ __forceinline__ float4 scale4(float4 a, float s) { return make_float4(a.x * s, a.y * s, a.z * s, a.w * s); }
-__device__ __forceinline__ float dot4(float4 a, float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
-
-__global__ void __launch_bounds__(512) softmax_fwd_cached_k(const float* __restrict__ zr, const float* __restrict__ zi,
-                                                            float* __restrict__ yr, float* __restrict__ yi,
-                                                            float* __restrict__ inv_norm, int N) {
-    cnb_pdl_enter();
-    __shared__ float sm[32];
-    const size_t base = (size_t) blockIdx.x * N;
-    float4 a[CACHE], b[CACHE];
-    float s = 0.f;
-#pragma unroll
-    for (int v = 0; v < CACHE; ++v) {
-        const int i = 4 * (threadIdx.x + v * blockDim.x);
-        if (i < N) { a[v] = ld4(zr, base + i); b[v] = ld4(zi, base + i); s += dot4(a[v], a[v]) + dot4(b[v], b[v]); }
-    }
-    s = block_sum(s, sm);
-    const float inv = 1.0f / fmaxf(sqrtf(s), 1e-15f);
-    if (threadIdx.x == 0) inv_norm[blockIdx.x] = inv;
-#pragma unroll
-    for (int v = 0; v < CACHE; ++v) {
-        const int i = 4 * (threadIdx.x + v * blockDim.x);
-        if (i < N) { st4(yr, base + i, scale4(a[v], inv)); st4(yi, base + i, scale4(b[v], inv)); }
-    }
-}
-
-__global__ void __launch_bounds__(512) softmax_bwd_cached_k(const float* __restrict__ gr, const float* __restrict__ gi,
-                                                            const float* __restrict__ zr, const float* __restrict__ zi,
-                                                            const float* __restrict__ inv_norm, float* __restrict__ dr,
-                                                            float* __restrict__ di, int N, int accumulate) {
-    cnb_pdl_enter();
-    __shared__ float sm[32];
-    const size_t base = (size_t) blockIdx.x * N;
-    float4 a[CACHE], b[CACHE], x[CACHE], y[CACHE];
-    float s = 0.f;
-#pragma unroll
-    for (int v = 0; v < CACHE; ++v) {
-        const int i = 4 * (threadIdx.x + v * blockDim.x);
-        if (i < N) {
-            a[v] = ld4(gr, base + i); b[v] = ld4(gi, base + i); x[v] = ld4(zr, base + i); y[v] = ld4(zi, base + i);
-            s += dot4(a[v], x[v]) + dot4(b[v], y[v]);            // Re(g* conj(z))
-        }
-    }
-    s = block_sum(s, sm);
-    const float inv = inv_norm[blockIdx.x];
-    const float c = s * inv * inv * inv;
-#pragma unroll
-    for (int v = 0; v < CACHE; ++v) {
-        const int i = 4 * (threadIdx.x + v * blockDim.x);
-        if (i < N) {
-            float4 p = make_float4(a[v].x * inv - x[v].x * c, a[v].y * inv - x[v].y * c, a[v].z * inv - x[v].z * c, a[v].w * inv - x[v].w * c);
-            float4 q = make_float4(b[v].x * inv - y[v].x * c, b[v].y * inv - y[v].y * c, b[v].z * inv - y[v].z * c, b[v].w * inv - y[v].w * c);
-            if (accumulate) {
-                const float4 o = ld4(dr, base + i), w = ld4(di, base + i);
-                p.x += o.x; p.y += o.y; p.z += o.z; p.w += o.w;
-                q.x += w.x; q.y += w.y; q.z += w.z; q.w += w.w;
-            }
-            st4(dr, base + i, p); st4(di, base + i, q);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(512) crossent_cached_k(const float* __restrict__ zr, const float* __restrict__ zi,
-                                                         const int32_t* __restrict__ labels, float* __restrict__ loss,
-                                                         float* __restrict__ dr, float* __restrict__ di, int M) {
-    cnb_pdl_enter();
-    __shared__ float sm[32];
-    const size_t base = (size_t) blockIdx.x * M;
-    float4 a[CACHE], b[CACHE];
-    float s = 0.f;
-#pragma unroll
-    for (int v = 0; v < CACHE; ++v) {
-        const int i = 4 * (threadIdx.x + v * blockDim.x);
-        if (i < M) { a[v] = ld4(zr, base + i); b[v] = ld4(zi, base + i); s += dot4(a[v], a[v]) + dot4(b[v], b[v]); }
-    }
-    // the label's element is handed over by the thread that holds it (a global load after the reduction would
-    // put an L2 round trip on every row's critical path)
-    __shared__ float s_lab[2];
-    int l = labels[blockIdx.x];
-    l = min(max(l, 0), M - 1);
-#pragma unroll
-    for (int v = 0; v < CACHE; ++v) {
-        const int i = 4 * (threadIdx.x + v * blockDim.x);
-        if (i < M && l >= i && l < i + 4) {
-            const int k = l - i;
-            s_lab[0] = k == 0 ? a[v].x : k == 1 ? a[v].y : k == 2 ? a[v].z : a[v].w;
-            s_lab[1] = k == 0 ? b[v].x : k == 1 ? b[v].y : k == 2 ? b[v].z : b[v].w;
-        }
-    }
-    s = block_sum(s, sm);                                 // its barriers also publish s_lab
-    const float S = fmaxf(s, 1e-15f);
-    const float lr = s_lab[0], li = s_lab[1];
-    const float m2 = lr * lr + li * li;
-    if (threadIdx.x == 0) loss[blockIdx.x] = -logf(fmaxf(m2 / S, 1e-15f));
-    if (dr == nullptr) return;
-    const float m = fmaxf(m2, 1e-15f);
-    const float cl = -(S - m) / (m * S), co = 1.0f / S;
-#pragma unroll
-    for (int v = 0; v < CACHE; ++v) {
-        const int i = 4 * (threadIdx.x + v * blockDim.x);
-        if (i < M) {
-            // the label's own coefficient (selects, not an indexed component: that would put the row in local memory)
-            const float c0 = (i == l) ? cl : co, c1 = (i + 1 == l) ? cl : co, c2 = (i + 2 == l) ? cl : co, c3 = (i + 3 == l) ? cl : co;
-            st4(dr, base + i, make_float4(a[v].x * c0, a[v].y * c1, a[v].z * c2, a[v].w * c3));
-            st4(di, base + i, make_float4(b[v].x * c0, b[v].y * c1, b[v].z * c2, b[v].w * c3));
-        }
-    }
-}
-
-// rows the cached kernels take: 16-byte aligned planes, N % 4 == 0, and the row fits the CTA's registers
-inline bool cached_ok(int n, int threads, std::initializer_list<const void*> planes) {
-    if (n % 4 || n < 1024 || n / 4 > threads * CACHE) return false;
-    for (const void* p : planes) if (p && (reinterpret_cast<uintptr_t>(p) & 15)) return false;
+bool vec_ok(int n, std::initializer_list<const void*> planes) {
+    if (n % 4) return false;
+    for (const void* p : planes) if (reinterpret_cast<uintptr_t>(p) & 15) return false;
     return true;
 }
 
-inline int threads_for(int n) {
-    int t = 32;
-    while (t < n / 4 && t < 512) t <<= 1;
-    return t;
-}
+}  // namespace
 
+// The form for rows of n elements (the lines are where a thread's 4 or 16 elements are used up) and its launch; NAME is
+// the kernel, the argument list ends with rows, n, parts and what may follow them.
+#define CNB_ROWS_GO(NAME, G, E, V, CTAS, PARTS, ...)                                                                     \
+    cnb::launch(NAME<G, E, V>, dim3((unsigned) (CTAS)), dim3(cta_threads(G)), 0, st, PARTS, __VA_ARGS__)
+#define CNB_ROWS_V(NAME, V, rows, n, ...)                                                                                \
+    do {                                                                                                                 \
+        if ((n) <= 32) CNB_ROWS_GO(NAME, 8, 4, V, ((rows) + 31) / 32, 1, __VA_ARGS__);                                   \
+        else if ((n) <= 128) CNB_ROWS_GO(NAME, 32, 4, V, ((rows) + 7) / 8, 1, __VA_ARGS__);                              \
+        else if ((n) <= 512) CNB_ROWS_GO(NAME, 32, 16, V, ((rows) + 7) / 8, 1, __VA_ARGS__);                             \
+        else if ((n) <= 2048) CNB_ROWS_GO(NAME, 128, 16, V, rows, 1, __VA_ARGS__);                                       \
+        else CNB_ROWS_GO(NAME, 512, 16, V, (size_t) (rows) * parts, parts, __VA_ARGS__);                                 \
+    } while (0)
+#define CNB_ROWS(NAME, vec, rows, n, ...)                                                                                \
+    do {                                                                                                                 \
+        if (vec) CNB_ROWS_V(NAME, 4, rows, n, __VA_ARGS__);                                                              \
+        else CNB_ROWS_V(NAME, 1, rows, n, __VA_ARGS__);                                                                  \
+        CNB_LAUNCH_CHECK(#NAME);                                                                                         \
+    } while (0)
+
+namespace {
+constexpr int kLongest = 65536;
+int parts_for(int n) { return n <= 8192 ? 1 : n <= 16384 ? 2 : n <= 32768 ? 4 : 8; }
 }  // namespace
 
 extern "C" {
@@ -249,11 +318,14 @@ int cnb_softmax_fwd(cnb_ctx* ctx, const float* z_re, const float* z_im, float* y
                     float* inv_norm, int B, int N, void* stream) {
     CNB_CHECK_ARG(ctx && z_re && z_im && y_re && y_im && inv_norm, "cnb_softmax_fwd: null pointer");
     CNB_CHECK_ARG(B > 0 && N > 0, "cnb_softmax_fwd: B=%d N=%d", B, N);
-    if (cached_ok(N, threads_for(N), {z_re, z_im, y_re, y_im}))
-        cnb::launch(softmax_fwd_cached_k, dim3(B), dim3(threads_for(N)), 0, cnb::S(stream), 1, z_re, z_im, y_re, y_im, inv_norm, N);
-    else
-        cnb::launch(softmax_fwd_k, dim3(B), dim3(threads_for(N)), 0, cnb::S(stream), 1, z_re, z_im, y_re, y_im, inv_norm, N);
-    CNB_LAUNCH_CHECK("softmax_fwd");
+    cudaStream_t st = cnb::S(stream);
+    const int parts = parts_for(N);
+    if (N > kLongest) {
+        cnb::launch(softmax_fwd_long_k, dim3(B), dim3(512), 0, st, 1, z_re, z_im, y_re, y_im, inv_norm, N);
+        CNB_LAUNCH_CHECK("softmax_fwd");
+    } else {
+        CNB_ROWS(softmax_fwd_k, vec_ok(N, {z_re, z_im, y_re, y_im}), B, N, z_re, z_im, y_re, y_im, inv_norm, B, N, parts);
+    }
     return CNB_OK;
 }
 
@@ -263,11 +335,15 @@ int cnb_softmax_bwd(cnb_ctx* ctx, const float* g_re, const float* g_im, const fl
     CNB_CHECK_ARG(ctx && g_re && g_im && z_re && z_im && inv_norm && dz_re && dz_im,
                   "cnb_softmax_bwd: null pointer");
     CNB_CHECK_ARG(B > 0 && N > 0, "cnb_softmax_bwd: B=%d N=%d", B, N);
-    if (cached_ok(N, threads_for(N), {g_re, g_im, z_re, z_im, dz_re, dz_im}))
-        cnb::launch(softmax_bwd_cached_k, dim3(B), dim3(threads_for(N)), 0, cnb::S(stream), 1, g_re, g_im, z_re, z_im, inv_norm, dz_re, dz_im, N, accumulate);
-    else
-        cnb::launch(softmax_bwd_k, dim3(B), dim3(threads_for(N)), 0, cnb::S(stream), 1, g_re, g_im, z_re, z_im, inv_norm, dz_re, dz_im, N, accumulate);
-    CNB_LAUNCH_CHECK("softmax_bwd");
+    cudaStream_t st = cnb::S(stream);
+    const int parts = parts_for(N);
+    if (N > kLongest) {
+        cnb::launch(softmax_bwd_long_k, dim3(B), dim3(512), 0, st, 1, g_re, g_im, z_re, z_im, inv_norm, dz_re, dz_im, N, accumulate);
+        CNB_LAUNCH_CHECK("softmax_bwd");
+    } else {
+        CNB_ROWS(softmax_bwd_k, vec_ok(N, {g_re, g_im, z_re, z_im, dz_re, dz_im}), B, N, g_re, g_im, z_re, z_im, inv_norm, dz_re,
+                 dz_im, B, N, parts, accumulate);
+    }
     return CNB_OK;
 }
 
@@ -276,11 +352,14 @@ int cnb_crossent_fwd_bwd(cnb_ctx* ctx, const float* z_re, const float* z_im, con
     CNB_CHECK_ARG(ctx && z_re && z_im && labels && loss, "cnb_crossent_fwd_bwd: null pointer");
     CNB_CHECK_ARG((dz_re == nullptr) == (dz_im == nullptr), "cnb_crossent_fwd_bwd: dz planes must be a pair");
     CNB_CHECK_ARG(B > 0 && M > 0, "cnb_crossent_fwd_bwd: B=%d M=%d", B, M);
-    if (cached_ok(M, threads_for(M), {z_re, z_im, dz_re, dz_im}))
-        cnb::launch(crossent_cached_k, dim3(B), dim3(threads_for(M)), 0, cnb::S(stream), 1, z_re, z_im, labels, loss, dz_re, dz_im, M);
-    else
-        cnb::launch(crossent_k, dim3(B), dim3(threads_for(M)), 0, cnb::S(stream), 1, z_re, z_im, labels, loss, dz_re, dz_im, M);
-    CNB_LAUNCH_CHECK("crossent");
+    cudaStream_t st = cnb::S(stream);
+    const int parts = parts_for(M);
+    if (M > kLongest) {
+        cnb::launch(crossent_long_k, dim3(B), dim3(512), 0, st, 1, z_re, z_im, labels, loss, dz_re, dz_im, M);
+        CNB_LAUNCH_CHECK("crossent");
+    } else {
+        CNB_ROWS(crossent_k, vec_ok(M, {z_re, z_im, dz_re, dz_im}), B, M, z_re, z_im, labels, loss, dz_re, dz_im, B, M, parts);
+    }
     return CNB_OK;
 }
 
@@ -289,8 +368,14 @@ int cnb_l2out_fwd_bwd(cnb_ctx* ctx, const float* z_re, const float* z_im, float*
     CNB_CHECK_ARG(ctx && z_re && z_im && loss, "cnb_l2out_fwd_bwd: null pointer");
     CNB_CHECK_ARG((dz_re == nullptr) == (dz_im == nullptr), "cnb_l2out_fwd_bwd: dz planes must be a pair");
     CNB_CHECK_ARG(B > 0 && N > 0, "cnb_l2out_fwd_bwd: B=%d N=%d", B, N);
-    cnb::launch(l2out_k, dim3(B), dim3(threads_for(N)), 0, cnb::S(stream), 1, z_re, z_im, loss, dz_re, dz_im, N);
-    CNB_LAUNCH_CHECK("l2out");
+    cudaStream_t st = cnb::S(stream);
+    const int parts = parts_for(N);
+    if (N > kLongest) {
+        cnb::launch(l2out_long_k, dim3(B), dim3(512), 0, st, 1, z_re, z_im, loss, dz_re, dz_im, N);
+        CNB_LAUNCH_CHECK("l2out");
+    } else {
+        CNB_ROWS(l2out_k, vec_ok(N, {z_re, z_im, dz_re, dz_im}), B, N, z_re, z_im, loss, dz_re, dz_im, B, N, parts);
+    }
     return CNB_OK;
 }
 
