@@ -1047,12 +1047,12 @@ __global__ void __launch_bounds__(256) pack_max_k(const __grid_constant__ PackJo
         const size_t n4 = n / 4;
         for (size_t i = (size_t) blockIdx.x * 256 + threadIdx.x; i < n4; i += step) {
             const float4 a = reinterpret_cast<const float4*>(job.re)[i], b = reinterpret_cast<const float4*>(job.im)[i];
-            m = max(m, max(max(cnb_abs_bits(a.x), cnb_abs_bits(a.y)), max(cnb_abs_bits(a.z), cnb_abs_bits(a.w))));
-            m = max(m, max(max(cnb_abs_bits(b.x), cnb_abs_bits(b.y)), max(cnb_abs_bits(b.z), cnb_abs_bits(b.w))));
+            m = max(m, max(max(cnb_scale_bits(a.x), cnb_scale_bits(a.y)), max(cnb_scale_bits(a.z), cnb_scale_bits(a.w))));
+            m = max(m, max(max(cnb_scale_bits(b.x), cnb_scale_bits(b.y)), max(cnb_scale_bits(b.z), cnb_scale_bits(b.w))));
         }
         done = n4 * 4;
     }
-    for (size_t i = done + (size_t) blockIdx.x * 256 + threadIdx.x; i < n; i += step) m = max(m, max(cnb_abs_bits(job.re[i]), cnb_abs_bits(job.im[i])));
+    for (size_t i = done + (size_t) blockIdx.x * 256 + threadIdx.x; i < n; i += step) m = max(m, max(cnb_scale_bits(job.re[i]), cnb_scale_bits(job.im[i])));
     cnb_pack_max_block(job.head, m);
 }
 

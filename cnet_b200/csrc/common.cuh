@@ -186,7 +186,12 @@ __device__ __forceinline__ void cnb_split_store4(const cnb_split_dst& d, size_t 
     *reinterpret_cast<uint2*>(d.l16 + i) = b;
 }
 
-__device__ __forceinline__ unsigned cnb_abs_bits(float x) { return __float_as_uint(x) & 0x7fffffffu; }
+// The magnitude of a component as an ordered integer for the scale of a packed operand.  Infinities and NaN count as
+// zero: they stay what they are under any scale, and must not take the finite rows beside them out of range.
+__device__ __forceinline__ unsigned cnb_scale_bits(float x) {
+    const unsigned b = __float_as_uint(x) & 0x7fffffffu;
+    return b < 0x7f800000u ? b : 0u;
+}
 
 // the largest of all threads' m into a pack head; every thread of the block (at most 1024) calls it
 __device__ __forceinline__ void cnb_pack_max_block(cnb_pack_head* head, unsigned m) {

@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(256) sgd_max_k(float* __restrict__ w, float* _
     for (size_t i = ((size_t) blockIdx.x * 256 + threadIdx.x) * 4; i < count; i += (size_t) gridDim.x * 1024) {
         Pack<4> a = ld<4>(w, begin + i), b = ld<4>(g, begin + i);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) { a.v[k] -= lr * b.v[k]; b.v[k] = 0.f; m = max(m, cnb_abs_bits(a.v[k])); }
+        for (int k = 0; k < 4; ++k) { a.v[k] -= lr * b.v[k]; b.v[k] = 0.f; m = max(m, cnb_scale_bits(a.v[k])); }
         st<4>(w, begin + i, a);
         if (zero_grad) st<4>(g, begin + i, b);
     }

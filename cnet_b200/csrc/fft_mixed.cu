@@ -127,7 +127,7 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
                         cnb_split_store1(cnb_split_component(ep.sp, ep.np, 0), at, gr);
                         cnb_split_store1(cnb_split_component(ep.sp, ep.np, 1), at, gi);
                     }
-                    io.largest = max(io.largest, max(cnb_abs_bits(gr), cnb_abs_bits(gi)));
+                    io.largest = max(io.largest, max(cnb_scale_bits(gr), cnb_scale_bits(gi)));
                 }
             }
         }

@@ -216,7 +216,7 @@ fft1024_pipe_k(const float* __restrict__ xr, const float* __restrict__ xi, float
                 const float gr = cnb_gelu(re[p] * hr - im[p] * hi);
                 const float gi = cnb_gelu(re[p] * hi + im[p] * hr);
                 if (ep.gr) { ep.gr[o + e] = gr; ep.gi[o + e] = gi; }
-                largest = max(largest, max(cnb_abs_bits(gr), cnb_abs_bits(gi)));
+                largest = max(largest, max(cnb_scale_bits(gr), cnb_scale_bits(gi)));
                 if (ep.sp) {
                     cnb_split_store1(sp_re, o + e, gr);
                     cnb_split_store1(sp_im, o + e, gi);

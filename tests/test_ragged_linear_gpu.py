@@ -83,6 +83,19 @@ def test_packed_range(ctx, scale):  # noqa: F811
     assert err.max() < 2.0 ** -18, err.max()
 
 
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_packed_nonfinite_row(ctx, bad):  # noqa: F811
+    """A row with an infinity or a NaN makes its own results NaN and leaves every other row as it is without it."""
+    rng = np.random.default_rng(5)
+    x, w = _rand(rng, 200, 320), _rand(rng, 192, 320)
+    want = _pair(_c(x) @ _c(w).T)
+    x[0][7, 33] = bad
+    y = _host(ctx.linear_fwd(_dev(x), _dev(w)))
+    keep = np.arange(200) != 7
+    assert util.relerr(tuple(p[keep] for p in y), tuple(p[keep] for p in want)) < TOL
+    assert not np.isfinite(y[0][7]).any() and not np.isfinite(y[1][7]).any()
+
+
 def test_packed_zero_matrix(ctx):  # noqa: F811
     x, w = (np.zeros((128, 128), np.float32),) * 2, _rand(np.random.default_rng(4), 128, 128)
     y = _host(ctx.linear_fwd(_dev(x), _dev(w)))
