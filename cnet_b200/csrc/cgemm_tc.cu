@@ -38,9 +38,12 @@
 // k-range is shared by several CTAs is summed with fp32 atomics into a pre-zeroed output.
 //
 // Roles.  warp 0: TMA producer; warp 1: TMEM allocation + MMA issue (one elected thread);
-// warps 2..5: epilogue (tcgen05.ld, combine, stage through shared memory, coalesced 16-byte
-// stores / atomics with residual or accumulate); tensor memory is handed back to the MMA warp as
-// soon as it has been read, so the write-out overlaps the next run of MMAs.
+// warps 2..9: epilogue (tcgen05.ld, combine, stage through shared memory, coalesced 16-byte
+// stores / atomics with residual or accumulate), two groups of four warps with half of a tile's columns each;
+// tensor memory is handed back to the MMA warp as soon as it has been read, so the write-out overlaps the next
+// run of MMAs.  With one group a whole tile left in 4.6 us after its last MMA, 8.9 with a residual and 18.8 where
+// rows are not 16-byte aligned; 777 x 1333 x 1001 forward and both gradients 179 -> 157 us, 512 x 1024 x 1024 in a
+// cluster of four 17.4 -> 16.6 (what is left there: 3.9 us of reading the peers' partial tiles).
 // Every mbarrier wait is bounded (2 s); on expiry the kernel records an error word, skips to
 // the common exit, frees its tensor memory and returns.
 #include <cuda.h>
@@ -73,10 +76,10 @@ template <bool PAIR> struct Cfg {
     static constexpr int TILE_M = PAIR ? 2 * BM : BM;
 };
 constexpr int OPERAND_BYTES = 3 * 8 * PLANE_BYTES;   // 192 KB of operand stages in both forms
-constexpr int EPI_BYTES = 2 * 128 * 32 * 4;           // 32 KB: one epilogue round, re and im staging
+constexpr int EPI_GROUPS = 2, EPI_THREADS = 128 * EPI_GROUPS, NUM_THREADS = 64 + EPI_THREADS;
+constexpr int EPI_BYTES = EPI_GROUPS * 2 * 128 * 16 * 4;  // 32 KB: one epilogue round of both groups, re and im staging
 constexpr int SMEM_BYTES = OPERAND_BYTES + EPI_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 static_assert(Cfg<false>::STAGES * Cfg<false>::STAGE_BYTES == OPERAND_BYTES && Cfg<true>::STAGES * Cfg<true>::STAGE_BYTES == OPERAND_BYTES, "stages");
-constexpr int NUM_THREADS = 192;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 
@@ -321,11 +324,31 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// the four warps of one epilogue group
+__device__ __forceinline__ void epi_bar_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
 
-// Staging tile of one epilogue round: 128 rows x 32 floats per plane, 16-byte chunks XOR-swizzled
-// by the row so that both the row-per-thread writes and the row-segment reads are conflict-free.
-__device__ __forceinline__ int stage_off(int row, int chunk) { return row * 32 + ((chunk ^ (row & 7)) << 2); }
+// Shared memory by its 32-bit address: through a generic pointer the compiler keeps every load behind the global store
+// before it, which made a round trip of each 16 bytes written out.
+__device__ __forceinline__ void st_shared4(uint32_t a, float x, float y, float z, float w) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+__device__ __forceinline__ float4 ld_shared4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float ld_shared1(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+
+// Staging tile of one epilogue round: 128 rows x 16 floats per plane, 16-byte chunks XOR-swizzled by the row so that
+// both the row-per-thread writes and the row-segment reads are conflict-free.  In bytes.
+__device__ __forceinline__ uint32_t stage_off(int row, int chunk) {
+    return (uint32_t) (row * 64 + ((chunk ^ ((row >> 1) & 3)) << 4));
+}
+constexpr uint32_t STAGE_PLANE = 128 * 16 * 4;
 
 // Partial tile of one CTA in cluster mode: 128 rows x 128 floats per plane over the (then idle) operand
 // stages, 16-byte chunks XOR-swizzled by the row like the staging tile.
@@ -415,14 +438,14 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
                                                int et, uint32_t peer0, uint32_t peer_step) {
     constexpr int ROWS = BM / CL;
     constexpr int U = CL <= 4 ? 2 : 1;                   // chunks per thread and round
-    for (int base = et; base < ROWS * 32; base += 128 * U) {
+    for (int base = et; base < ROWS * 32; base += EPI_THREADS * U) {
         float4 xr[U][CL], xi[U][CL], vr[U], vi[U];
         size_t o[U];
         bool live[U];
         int gn[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int idx = base + 128 * u;
+            const int idx = base + EPI_THREADS * u;
             const int r = (int) crank * ROWS + (idx >> 5), ch = idx & 31;
             const int gm = m0 + r;
             gn[u] = n0 + ch * 4;
@@ -479,8 +502,6 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
     // operand stages need the alignment of their swizzle pattern; 1024 B covers every mode
     constexpr int STAGES = Cfg<PAIR>::STAGES, STAGE_BYTES = Cfg<PAIR>::STAGE_BYTES, TILE_M = Cfg<PAIR>::TILE_M;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    float* stage_re = reinterpret_cast<float*>(smem + OPERAND_BYTES);
-    float* stage_im = stage_re + 128 * 32;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OPERAND_BYTES + EPI_BYTES);
     // bars[0..S) full, bars[S..2S) empty, bars[2S] accumulators ready, bars[2S+1] accumulators drained
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2);
@@ -541,7 +562,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         mbar_init(acc_full, 1);
-        mbar_init(acc_empty, PAIR ? 2 : 1);              // pair: the epilogues of both CTAs hand the accumulators back
+        mbar_init(acc_empty, (PAIR ? 2 : 1) * EPI_GROUPS);   // every epilogue group (pair: of both CTAs) hands the accumulators back
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -776,7 +797,8 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
         // -------------------------------------------------------------------- epilogue
         const int q = warp & 3;                      // TMEM lane quarter this warp may read
         const int row = q * 32 + lane;
-        const int et = (warp - 2) * 32 + lane;       // 0..127 within the epilogue group
+        const int group = (warp - 2) >> 2;           // the half of the columns this warp takes
+        const int et = ((warp - 2) & 3) * 32 + lane; // 0..127 within the epilogue group
         const uint32_t tl = tmem_base + ((uint32_t) (q * 32) << 16);
         const float sgn = p.conjB ? 1.f : -1.f;
         // PACKED: the scales of both operands are taken out again, in two factors so that neither leaves fp32's range
@@ -787,26 +809,25 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
             u1 = __uint_as_float((uint32_t) (e - h + 127) << 23);
         }
         auto out = [&](float v) { return FORM == PACKED ? v * u0 * u1 : v; };
+        const uint32_t stage = smem_base + OPERAND_BYTES + (uint32_t) group * 2 * STAGE_PLANE;
         int seg = 0;
         if (split_cluster) {
             // the whole k-slice is one segment; its partial sums go to shared memory for the cluster reduction
             {
                 const int tile = blockIdx.x / cluster_ctas, rows_per = BM / p.cluster;
                 const int row = (tile / tiles_n) * TILE_M + row_off + (int) crank * rows_per + et, n0 = (tile % tiles_n) * BN;
-                if (et < rows_per) {                     // the band of rows this CTA will write out
+                if (group == 0 && et < rows_per) {       // the band of rows this CTA will write out
                     if (p.r_re) prefetch_tile_rows(p, p.r_re, p.r_im, row, n0);
                     if (p.accumulate) prefetch_tile_rows(p, p.d_re, p.d_im, row, n0);
                 }
             }
             mbar_wait(acc_full, 0u, abort_flag, p.status, 3);
             CNB_GSTAMP(4, et == 0);
-            epi_bar_sync();
+            epi_bar_sync(group);
             if (!*abort_flag) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                float* part_re = reinterpret_cast<float*>(smem);
-                float* part_im = part_re + 128 * 128;
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 16) {
+                for (int c0 = group * 64; c0 < group * 64 + 64; c0 += 16) {
                     float a[16], f[16], b[16], e[16];
                     tmem_ld16(tl + c0, a);                   // A_re.B_re
                     tmem_ld16(tl + 384 + c0, f);             // A_im.B_im
@@ -815,13 +836,11 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int i = 0; i < 16; i += 4) {
-                        const int o = part_off(row, (c0 + i) >> 2);
-                        *reinterpret_cast<float4*>(part_re + o) =
-                            make_float4(out(a[i] + sgn * f[i]), out(a[i + 1] + sgn * f[i + 1]), out(a[i + 2] + sgn * f[i + 2]),
-                                        out(a[i + 3] + sgn * f[i + 3]));
-                        *reinterpret_cast<float4*>(part_im + o) =
-                            make_float4(out(e[i] - sgn * b[i]), out(e[i + 1] - sgn * b[i + 1]), out(e[i + 2] - sgn * b[i + 2]),
-                                        out(e[i + 3] - sgn * b[i + 3]));
+                        const uint32_t o = smem_base + 4u * (uint32_t) part_off(row, (c0 + i) >> 2);
+                        st_shared4(o, out(a[i] + sgn * f[i]), out(a[i + 1] + sgn * f[i + 1]), out(a[i + 2] + sgn * f[i + 2]),
+                                   out(a[i + 3] + sgn * f[i + 3]));
+                        st_shared4(o + PART_PLANE_BYTES, out(e[i] - sgn * b[i]), out(e[i + 1] - sgn * b[i + 1]),
+                                   out(e[i + 2] - sgn * b[i + 2]), out(e[i + 3] - sgn * b[i + 3]));
                     }
                 }
             }
@@ -836,114 +855,111 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
             int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
             const bool partial = !(kb0 == 0 && kb1 == k_blocks);   // split tiles are summed with atomics
             const bool add_res = p.r_re != nullptr && kb0 == 0;
-            // one row of the tile per epilogue thread, requested before the wait for the MMAs
-            if (add_res) prefetch_tile_rows(p, p.r_re, p.r_im, m0 + et, n0);
-            if (!partial && p.accumulate) prefetch_tile_rows(p, p.d_re, p.d_im, m0 + et, n0);
-            mbar_wait(acc_full, (uint32_t) seg & 1, abort_flag, p.status, 3);
-            epi_bar_sync();                          // everyone arrives, then agree on the outcome
-            if (*abort_flag) { live = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const bool need_old = !partial && p.accumulate;
             const bool pre = VEC && (add_res || need_old);
+            // one row of the tile per epilogue thread, requested before the wait for the MMAs
+            if (group == 0) {
+                if (add_res) prefetch_tile_rows(p, p.r_re, p.r_im, m0 + et, n0);
+                if (need_old) prefetch_tile_rows(p, p.d_re, p.d_im, m0 + et, n0);
+            }
+            // What a round adds from global memory (the residual if there is one, else old D) is requested a round
+            // ahead, the first one's under the MMAs: asked for in the round itself it doubled the round's time, and
+            // asked for between the stores each load would wait for the store before it.
+            float4 gr[4], gi[4];
+            auto request = [&](int c0) {
+                const float* sr = add_res ? p.r_re : p.d_re;
+                const float* si = add_res ? p.r_im : p.d_im;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int idx = et + 128 * j;
+                    const int gm = m0 + (idx >> 2), gn = n0 + c0 + (idx & 3) * 4;
+                    gr[j] = make_float4(0.f, 0.f, 0.f, 0.f); gi[j] = gr[j];
+                    if (gm >= p.M || gn >= p.N) continue;
+                    const size_t o = (size_t) gm * p.N + gn;
+                    gr[j] = ld_global_now(sr + o);
+                    gi[j] = ld_global_now(si + o);
+                }
+            };
+            const int c_first = group * 64, c_last = c_first + 48;
+            if (pre) request(c_first);
+            mbar_wait(acc_full, (uint32_t) seg & 1, abort_flag, p.status, 3);
+            epi_bar_sync(group);                     // everyone arrives, then agree on the outcome
+            if (*abort_flag) { live = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-                // What the write-out of this round adds from global memory (residual, old D) is requested
-                // now, so that it arrives while the accumulators are drained; asked for between the
-                // stores below, each load would wait for the store before it.
-                float4 gr[8], gi[8];
-                if (pre) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int idx = et + 128 * j;
-                        const int gm = m0 + (idx >> 3), gn = n0 + c0 + (idx & 7) * 4;
-                        gr[j] = make_float4(0.f, 0.f, 0.f, 0.f); gi[j] = gr[j];
-                        if (gm >= p.M || gn >= p.N) continue;
-                        const size_t o = (size_t) gm * p.N + gn;
-                        // the residual if there is one, else old D (both at once: old D is read at the store)
-                        if (add_res) {
-                            gr[j] = ld_global_now(p.r_re + o);
-                            gi[j] = ld_global_now(p.r_im + o);
-                        } else {
-                            gr[j] = ld_global_now(p.d_re + o);
-                            gi[j] = ld_global_now(p.d_im + o);
-                        }
-                    }
-                }
+            for (int c0 = c_first; c0 <= c_last; c0 += 16) {
                 {
-                    float a[16], f[16];
+                    float a[16], f[16], b[16], e[16];
+                    tmem_ld16(tl + c0, a);                   // A_re.B_re
+                    tmem_ld16(tl + 384 + c0, f);             // A_im.B_im
+                    tmem_ld16(tl + 128 + c0, b);             // A_re.B_im
+                    tmem_ld16(tl + 256 + c0, e);             // A_im.B_re
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        tmem_ld16(tl + c0 + 16 * h, a);            // A_re.B_re
-                        tmem_ld16(tl + 384 + c0 + 16 * h, f);      // A_im.B_im
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int i = 0; i < 16; i += 4)
-                            *reinterpret_cast<float4*>(stage_re + stage_off(row, 4 * h + i / 4)) =
-                                make_float4(out(a[i] + sgn * f[i]), out(a[i + 1] + sgn * f[i + 1]), out(a[i + 2] + sgn * f[i + 2]),
-                                            out(a[i + 3] + sgn * f[i + 3]));
+                    for (int i = 0; i < 16; i += 4) {
+                        const uint32_t o = stage + stage_off(row, i / 4);
+                        st_shared4(o, out(a[i] + sgn * f[i]), out(a[i + 1] + sgn * f[i + 1]), out(a[i + 2] + sgn * f[i + 2]),
+                                   out(a[i + 3] + sgn * f[i + 3]));
+                        st_shared4(o + STAGE_PLANE, out(e[i] - sgn * b[i]), out(e[i + 1] - sgn * b[i + 1]),
+                                   out(e[i + 2] - sgn * b[i + 2]), out(e[i + 3] - sgn * b[i + 3]));
                     }
                 }
-                {
-                    float b[16], e[16];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        tmem_ld16(tl + 128 + c0 + 16 * h, b);      // A_re.B_im
-                        tmem_ld16(tl + 256 + c0 + 16 * h, e);      // A_im.B_re
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int i = 0; i < 16; i += 4)
-                            *reinterpret_cast<float4*>(stage_im + stage_off(row, 4 * h + i / 4)) =
-                                make_float4(out(e[i] - sgn * b[i]), out(e[i + 1] - sgn * b[i + 1]), out(e[i + 2] - sgn * b[i + 2]),
-                                            out(e[i + 3] - sgn * b[i + 3]));
-                    }
-                }
-                if (c0 + 32 == BN) {
+                if (c0 == c_last) {
                     // last TMEM read of this segment done: hand the accumulators back to the MMA warp
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 }
-                epi_bar_sync();
-                if (c0 + 32 == BN && et == 0) {
+                epi_bar_sync(group);
+                if (c0 == c_last && et == 0) {
                     if constexpr (PAIR) mbar_arrive_cluster(map_to_rank(acc_empty, lead_rank));   // the first CTA's MMA thread waits for both
                     else mbar_arrive(acc_empty);
                 }
                 if constexpr (VEC) {
-                    // coalesced write-out: each warp instruction covers 4 rows x 128 contiguous bytes
+                    // coalesced write-out: each warp instruction covers 8 rows x 64 contiguous bytes
+                    float4 vr[4], vi[4];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        int idx = et + 128 * j;
-                        int r = idx >> 3, ch = idx & 7;
-                        int gm = m0 + r, gn = n0 + c0 + ch * 4;
-                        if (gm >= p.M || gn >= p.N) continue;
-                        float4 vr = *reinterpret_cast<const float4*>(stage_re + stage_off(r, ch));
-                        float4 vi = *reinterpret_cast<const float4*>(stage_im + stage_off(r, ch));
-                        size_t o = (size_t) gm * p.N + gn;
-                        if (pre) {
-                            vr.x += gr[j].x; vr.y += gr[j].y; vr.z += gr[j].z; vr.w += gr[j].w;
-                            vi.x += gi[j].x; vi.y += gi[j].y; vi.z += gi[j].z; vi.w += gi[j].w;
+                    for (int j = 0; j < 4; ++j) {
+                        const int idx = et + 128 * j;
+                        const uint32_t at = stage + stage_off(idx >> 2, idx & 3);
+                        vr[j] = ld_shared4(at);
+                        vi[j] = ld_shared4(at + STAGE_PLANE);
+                    }
+                    if (pre) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            vr[j].x += gr[j].x; vr[j].y += gr[j].y; vr[j].z += gr[j].z; vr[j].w += gr[j].w;
+                            vi[j].x += gi[j].x; vi[j].y += gi[j].y; vi[j].z += gi[j].z; vi[j].w += gi[j].w;
                         }
+                        if (c0 != c_last) request(c0 + 16);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int idx = et + 128 * j;
+                        const int gm = m0 + (idx >> 2), gn = n0 + c0 + (idx & 3) * 4;
+                        if (gm >= p.M || gn >= p.N) continue;
+                        const size_t o = (size_t) gm * p.N + gn;
                         if (add_res && need_old) {       // both at once: old D is read here
                             const float4 xr = *reinterpret_cast<const float4*>(p.d_re + o), xi = *reinterpret_cast<const float4*>(p.d_im + o);
-                            vr.x += xr.x; vr.y += xr.y; vr.z += xr.z; vr.w += xr.w;
-                            vi.x += xi.x; vi.y += xi.y; vi.z += xi.z; vi.w += xi.w;
+                            vr[j].x += xr.x; vr[j].y += xr.y; vr[j].z += xr.z; vr[j].w += xr.w;
+                            vi[j].x += xi.x; vi[j].y += xi.y; vi[j].z += xi.z; vi[j].w += xi.w;
                         }
                         if (partial) {
-                            atomicAdd(reinterpret_cast<float4*>(p.d_re + o), vr);
-                            atomicAdd(reinterpret_cast<float4*>(p.d_im + o), vi);
+                            atomicAdd(reinterpret_cast<float4*>(p.d_re + o), vr[j]);
+                            atomicAdd(reinterpret_cast<float4*>(p.d_im + o), vi[j]);
                         } else {
-                            *reinterpret_cast<float4*>(p.d_re + o) = vr;
-                            *reinterpret_cast<float4*>(p.d_im + o) = vi;
+                            *reinterpret_cast<float4*>(p.d_re + o) = vr[j];
+                            *reinterpret_cast<float4*>(p.d_im + o) = vi[j];
                         }
                     }
                 } else {
-                    // a warp takes 32 rows, one row's 32 floats per instruction; what is added to eight rows is
+                    // a warp takes 32 rows, 16 floats of two rows per instruction; what is added to sixteen rows is
                     // requested before the first of them is stored
-                    const int gn = n0 + c0 + lane;
+                    const int gn = n0 + c0 + (lane & 15), half = lane >> 4;
 #pragma unroll 1
-                    for (int r0 = q * 32; r0 < q * 32 + 32; r0 += 8) {
+                    for (int r0 = q * 32 + half; r0 < q * 32 + 32; r0 += 16) {
                         float ar[8], ai[8];
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            const int gm = m0 + r0 + j;
+                            const int gm = m0 + r0 + 2 * j;
                             const size_t o = (size_t) gm * p.N + gn;
                             const bool on = gm < p.M && gn < p.N;
                             ar[j] = ai[j] = 0.f;
@@ -952,17 +968,21 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                         }
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            const int gm = m0 + r0 + j;
+                            const uint32_t at = stage + stage_off(r0 + 2 * j, (lane & 15) >> 2) + 4u * (uint32_t) (lane & 3);
+                            ar[j] += ld_shared1(at);
+                            ai[j] += ld_shared1(at + STAGE_PLANE);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int gm = m0 + r0 + 2 * j;
                             if (gm >= p.M || gn >= p.N) continue;
                             const size_t o = (size_t) gm * p.N + gn;
-                            const int at = stage_off(r0 + j, lane >> 2) + (lane & 3);
-                            const float vr = stage_re[at] + ar[j], vi = stage_im[at] + ai[j];
-                            if (partial) { atomicAdd(p.d_re + o, vr); atomicAdd(p.d_im + o, vi); }
-                            else { p.d_re[o] = vr; p.d_im[o] = vi; }
+                            if (partial) { atomicAdd(p.d_re + o, ar[j]); atomicAdd(p.d_im + o, ai[j]); }
+                            else { p.d_re[o] = ar[j]; p.d_im[o] = ai[j]; }
                         }
                     }
                 }
-                epi_bar_sync();                      // staging is reused by the next round
+                epi_bar_sync(group);                 // staging is reused by the next round
             }
             u += kb1 - kb0;
         }
