@@ -55,13 +55,16 @@ struct Io {
     const float2 *tw, *chirp, *spectrum;
     const float2* src;                // shared-memory buffers, NULL: the planes
     float2* dst;
-    int rows, accumulate;
+    int rows;
     unsigned largest;                 // of the tail's components, this thread's (bits of the magnitude)
     bool spectral;                    // chirp form: this pass opens the inverse transform
     size_t row0;
 };
 
-template <int R, bool EPI, bool CHIRP>
+// What becomes of a finished row: stored, stored and taken through the tail, or added to what is there.
+enum Finish { STORE = 0, TAIL = 1, ADD = 2 };
+
+template <int R, int FINISH, bool CHIRP>
 __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io& io, const FftEpilogue& ep) {
     const int items = io.rows * d.nb;
     for (int i = threadIdx.x; i < items; i += blockDim.x) {
@@ -107,6 +110,17 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
             for (int q = 0; q < R; ++q) t[pad_of(o + q * d.L)] = v[q];
         } else {
             const size_t base = (size_t) row * pl.n + o;
+            // Old values are requested together, before the first store: between the stores each load waited for the
+            // store before it, R round trips one after another.  A form of its own, because the registers they sit
+            // in cost the plain transform a CTA per SM (1000 x 1500 both ways 26.5 -> 30.2 us).
+            float2 old[FINISH == ADD ? R : 1];
+            if (FINISH == ADD) {
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    const size_t g = (size_t) row * pl.n + (CHIRP ? min(o + q * d.L, pl.n - 1) : o + q * d.L);
+                    old[FINISH == ADD ? q : 0] = make_float2(io.yr[g], io.yi[g]);
+                }
+            }
 #pragma unroll
             for (int q = 0; q < R; ++q) {
                 const int e = o + q * d.L;
@@ -115,10 +129,10 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
                 float2 u = v[q];
                 if (CHIRP) u = cmul(make_float2(u.y, u.x), __ldg(io.chirp + e));
                 u.x *= pl.scale; u.y *= pl.scale;
-                if (!EPI && io.accumulate) { u.x += io.yr[g]; u.y += io.yi[g]; }
+                if (FINISH == ADD) { u.x += old[FINISH == ADD ? q : 0].x; u.y += old[FINISH == ADD ? q : 0].y; }
                 io.yr[g] = u.x;
                 io.yi[g] = u.y;
-                if (EPI) {
+                if (FINISH == TAIL) {
                     const float hr = __ldg(ep.hr + e), hi = __ldg(ep.hi + e);
                     const float gr = cnb_gelu(u.x * hr - u.y * hi), gi = cnb_gelu(u.x * hi + u.y * hr);
                     const size_t at = (io.row0 + row) * (size_t) pl.n + e;
@@ -134,11 +148,11 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
     }
 }
 
-template <bool EPI, bool CHIRP>
+template <int FINISH, bool CHIRP>
 __global__ void __launch_bounds__(MAX_THREADS, 2)
 fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* yr, float* yi,
             const float2* __restrict__ tw, const float2* __restrict__ chirp, const float2* __restrict__ spectrum, int B,
-            int accumulate, const FftEpilogue ep, const __grid_constant__ MixedPlan pl) {
+            const FftEpilogue ep, const __grid_constant__ MixedPlan pl) {
     cnb_pdl_enter();
     extern __shared__ __align__(16) float2 bufs[];
     Io io;
@@ -147,7 +161,6 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
     io.xr = xr + io.row0 * pl.n; io.xi = xi + io.row0 * pl.n;
     io.yr = yr + io.row0 * pl.n; io.yi = yi + io.row0 * pl.n;
     io.tw = tw; io.chirp = chirp; io.spectrum = spectrum;
-    io.accumulate = accumulate;
     io.largest = 0;
     const int total = CHIRP ? 2 * pl.passes : pl.passes;
     for (int s = 0; s < total; ++s) {
@@ -156,14 +169,14 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
         io.dst = s == total - 1 ? nullptr : bufs + (s & 1 ? pl.rows * pl.stride : 0);
         io.spectral = CHIRP && s == pl.passes;
         switch (d.radix) {
-#define CNB_RADIX(R) case R: run_pass<R, EPI, CHIRP>(pl, d, io, ep); break
+#define CNB_RADIX(R) case R: run_pass<R, FINISH, CHIRP>(pl, d, io, ep); break
             CNB_RADIX(2); CNB_RADIX(3); CNB_RADIX(4); CNB_RADIX(5); CNB_RADIX(6); CNB_RADIX(7); CNB_RADIX(8); CNB_RADIX(9);
             CNB_RADIX(10); CNB_RADIX(11); CNB_RADIX(12); CNB_RADIX(13); CNB_RADIX(14); CNB_RADIX(15); CNB_RADIX(16);
 #undef CNB_RADIX
         }
         if (s < total - 1) __syncthreads();
     }
-    if (EPI && ep.head) cnb_pack_max_block(ep.head, io.largest);
+    if (FINISH == TAIL && ep.head) cnb_pack_max_block(ep.head, io.largest);
 }
 
 // twiddles of every pass, packed as Pass::tw says, in double
@@ -368,23 +381,24 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
     const float2* spec = ch + pl.n;
     if (inverse) { std::swap(xr, xi); std::swap(yr, yi); }
     const size_t smem = smem_bytes(pl.m, pl.rows, pl.buffers);
-    const int form = (ep.hr ? 2 : 0) + (chirp ? 1 : 0);
+    const Finish finish = ep.hr ? TAIL : accumulate ? ADD : STORE;
     static bool attr_done[64] = {};                         // the attribute is per device
     if (!attr_done[ctx->device & 63]) {
-        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));
-        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));
-        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));
-        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));
+#define CNB_MIXED_ATTR(F, C) CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM))
+        CNB_MIXED_ATTR(STORE, false); CNB_MIXED_ATTR(TAIL, false); CNB_MIXED_ATTR(ADD, false);
+        CNB_MIXED_ATTR(STORE, true); CNB_MIXED_ATTR(TAIL, true); CNB_MIXED_ATTR(ADD, true);
+#undef CNB_MIXED_ATTR
         attr_done[ctx->device & 63] = true;
     }
     const dim3 grid((unsigned) ((B + pl.rows - 1) / pl.rows)), block((unsigned) pl.threads);
-#define CNB_MIXED(E, C) CNB_CUDA(cnb::launch(fft_mixed_k<E, C>, grid, block, smem, st, 1, xr, xi, yr, yi, tw, ch, spec, B, accumulate, ep, pl))
-    switch (form) {
-        case 0: CNB_MIXED(false, false); break;
-        case 1: CNB_MIXED(false, true); break;
-        case 2: CNB_MIXED(true, false); break;
-        default: CNB_MIXED(true, true); break;
-    }
+#define CNB_MIXED(F)                                                                                                          \
+    do {                                                                                                                      \
+        if (chirp) CNB_CUDA(cnb::launch(fft_mixed_k<F, true>, grid, block, smem, st, 1, xr, xi, yr, yi, tw, ch, spec, B, ep, pl)); \
+        else CNB_CUDA(cnb::launch(fft_mixed_k<F, false>, grid, block, smem, st, 1, xr, xi, yr, yi, tw, ch, spec, B, ep, pl));      \
+    } while (0)
+    if (finish == TAIL) CNB_MIXED(TAIL);
+    else if (finish == ADD) CNB_MIXED(ADD);
+    else CNB_MIXED(STORE);
 #undef CNB_MIXED
     CNB_LAUNCH_CHECK("fft_mixed");
     return CNB_OK;
