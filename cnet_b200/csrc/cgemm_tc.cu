@@ -49,6 +49,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -92,6 +93,7 @@ struct TcParams {
     int cluster;              // > 1: that many CTAs of one cluster share a tile, each a slice of K
     int whole_per_cta;        // > 0: every CTA first takes that many whole tiles, then its run of the remaining units
     int segments;             // > 0: CTA r takes k-segment r / tiles of tile r % tiles (units_per_cta k-blocks each)
+    int chain;                // DRAIN: k-blocks that are summed in tensor memory at most
     const int* a_exp;         // PACKED: the powers of two that A and B were scaled by
     const int* b_exp;
     int* status;
@@ -324,6 +326,34 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+    uint32_t r[8];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The accumulators of one chain (this thread's row, the 64 columns of its group from `tl` on) into the running sums,
+// rounded to nearest.
+__device__ __forceinline__ void drain_chain(uint32_t tl, float sgn, float (&sr)[64], float (&si)[64]) {
+#pragma unroll
+    for (int c = 0; c < 64; c += 8) {
+        float x[8], y[8];
+        tmem_ld8(tl + c, x);                             // A_re.B_re
+        tmem_ld8(tl + 384 + c, y);                       // A_im.B_im
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sr[c + i] += x[i] + sgn * y[i];
+        tmem_ld8(tl + 256 + c, x);                       // A_im.B_re
+        tmem_ld8(tl + 128 + c, y);                       // A_re.B_im
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 8; ++i) si[c + i] += x[i] - sgn * y[i];
+    }
+}
+
 // the four warps of one epilogue group
 __device__ __forceinline__ void epi_bar_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
 
@@ -493,7 +523,10 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 
 // VEC: rows of D and R are 16-byte aligned (N % 4 == 0); the form without it writes 32 consecutive floats of a row per
 // warp instruction instead of four 16-byte pieces of four rows.
-template <bool PAIR, bool VEC, int FORM>
+// DRAIN: a run of more than p.chain k-blocks is cut into chains of that many; after each the epilogue takes the
+// accumulators into running sums in registers (max_chain says why).  777 x 1333 -> 1001, three products: 158 -> 172 us,
+// forward off by 4.4e-7 of float64 instead of 2.4e-6 (fp32 FMAs: 6.6e-7).
+template <bool PAIR, bool VEC, int FORM, bool DRAIN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -682,6 +715,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
             for (long u = pass ? u2_begin : u_begin, ue = pass ? u2_end : u_end; u < ue && ok; ++seg) {
                 int kb0 = (int) (u % k_blocks);
                 int kb1 = (int) min((long) k_blocks, kb0 + (ue - u));
+                if constexpr (DRAIN) kb1 = min(kb1, kb0 + p.chain);      // every chain is a segment of its own here
                 // the epilogue must have drained the previous segment's accumulators
                 ok = mbar_wait(acc_empty, (uint32_t) (seg & 1) ^ 1, abort_flag, p.status, 4);
                 if (!ok) break;
@@ -696,11 +730,12 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                     uint32_t st = smem_base + s * STAGE_BYTES;
                     const uint32_t first = kb == kb0 ? 0u : 1u;
                     if constexpr (FORM == PACKED) {
-                        // high.low + low.high first, then high.high, a k-step of 16 at a time
+                        // high.low + low.high first, then high.high: a k-step of 16 at a time, or (DRAIN) the whole block
+                        // at a time, so that the small terms of a chain of one block meet a small accumulator (K = 50:
+                        // 1.5e-7 -> 1.1e-7 off float64, FMAs 1.3e-7)
                         const uint32_t idesch = (kInstrDescH | mn_bits) + m_bits;
                         constexpr int b_low = PAIR ? 5 : 6;
-#pragma unroll
-                        for (int j = 0; j < BK / 16; ++j) {
+                        auto step = [&](int j, bool low, bool high) {
                             const uint32_t ka = p.a_mn ? j * 2048 : j * 32, kbo = p.b_mn ? j * 2048 : j * 32;
                             auto adesc = [&](int slot) {
                                 const uint32_t a = st + slot * PLANE_BYTES + ka;
@@ -715,12 +750,16 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                             };
                             const uint64_t bh = bdesc(4), bl = bdesc(b_low);
                             const uint32_t add = j == 0 ? first : 1u;
-                            mma(tmem_base, adesc(2), bh, add);
-                            mma(tmem_base, adesc(0), bl, 1u);
-                            mma(tmem_base, adesc(0), bh, 1u);
-                            mma(tmem_base + 256, adesc(3), bh, add);
-                            mma(tmem_base + 256, adesc(1), bl, 1u);
-                            mma(tmem_base + 256, adesc(1), bh, 1u);
+                            if (low) { mma(tmem_base, adesc(2), bh, add); mma(tmem_base, adesc(0), bl, 1u); }
+                            if (high) mma(tmem_base, adesc(0), bh, 1u);
+                            if (low) { mma(tmem_base + 256, adesc(3), bh, add); mma(tmem_base + 256, adesc(1), bl, 1u); }
+                            if (high) mma(tmem_base + 256, adesc(1), bh, 1u);
+                        };
+#pragma unroll
+                        for (int j = 0; j < BK / 16; ++j) step(j, true, !DRAIN);
+                        if constexpr (DRAIN) {
+#pragma unroll
+                            for (int j = 0; j < BK / 16; ++j) step(j, false, true);
                         }
                         if constexpr (PAIR) umma2_commit_both(empty_bar(s), lead_rank); else umma_commit(empty_bar(s));
                         continue;
@@ -811,6 +850,28 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
         auto out = [&](float v) { return FORM == PACKED ? v * u0 * u1 : v; };
         const uint32_t stage = smem_base + OPERAND_BYTES + (uint32_t) group * 2 * STAGE_PLANE;
         int seg = 0;
+        // DRAIN: the chains of one segment of `blocks` k-blocks into the running sums; false after a wait gave up
+        float sr[DRAIN ? 64 : 1], si[DRAIN ? 64 : 1];
+        auto sum_chains = [&](int blocks) {
+            if constexpr (DRAIN) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i) sr[i] = si[i] = 0.f;
+                for (int done = 0; done < blocks; done += p.chain, ++seg) {
+                    mbar_wait(acc_full, (uint32_t) seg & 1, abort_flag, p.status, 3);
+                    epi_bar_sync(group);
+                    if (*abort_flag) return false;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    drain_chain(tl + group * 64, sgn, sr, si);
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    epi_bar_sync(group);
+                    if (et == 0) {
+                        if constexpr (PAIR) mbar_arrive_cluster(map_to_rank(acc_empty, lead_rank));
+                        else mbar_arrive(acc_empty);
+                    }
+                }
+            }
+            return true;
+        };
         if (split_cluster) {
             // the whole k-slice is one segment; its partial sums go to shared memory for the cluster reduction
             {
@@ -821,6 +882,16 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                     if (p.accumulate) prefetch_tile_rows(p, p.d_re, p.d_im, row, n0);
                 }
             }
+            if constexpr (DRAIN) {
+                if (sum_chains((int) (u_end - u_begin))) {           // after the last chain the stages are idle
+#pragma unroll
+                    for (int i = 0; i < 64; i += 4) {
+                        const uint32_t o = smem_base + 4u * (uint32_t) part_off(row, group * 16 + (i >> 2));
+                        st_shared4(o, out(sr[i]), out(sr[i + 1]), out(sr[i + 2]), out(sr[i + 3]));
+                        st_shared4(o + PART_PLANE_BYTES, out(si[i]), out(si[i + 1]), out(si[i + 2]), out(si[i + 3]));
+                    }
+                }
+            } else {
             mbar_wait(acc_full, 0u, abort_flag, p.status, 3);
             CNB_GSTAMP(4, et == 0);
             epi_bar_sync(group);
@@ -844,12 +915,13 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                     }
                 }
             }
+            }
             CNB_GSTAMP(5, et == 0);
             u_end = u_begin;                             // nothing left for the loop below
         }
         bool live = true;
         for (int pass = 0; pass < 2 && live; ++pass)
-        for (long u = pass ? u2_begin : u_begin, ue = pass ? u2_end : u_end; u < ue; ++seg) {
+        for (long u = pass ? u2_begin : u_begin, ue = pass ? u2_end : u_end; u < ue; seg += DRAIN ? 0 : 1) {
             int tile = (int) (u / k_blocks), kb0 = (int) (u % k_blocks);
             int kb1 = (int) min((long) k_blocks, kb0 + (ue - u));
             int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
@@ -864,31 +936,46 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
             }
             // What a round adds from global memory (the residual if there is one, else old D) is requested a round
             // ahead, the first one's under the MMAs: asked for in the round itself it doubled the round's time, and
-            // asked for between the stores each load would wait for the store before it.
-            float4 gr[4], gi[4];
-            auto request = [&](int c0) {
-                const float* sr = add_res ? p.r_re : p.d_re;
-                const float* si = add_res ? p.r_im : p.d_im;
+            // asked for between the stores each load would wait for the store before it.  (DRAIN: half a round at a time,
+            // and not ahead; the registers hold the running sums.)
+            constexpr int U = DRAIN ? 2 : 4;
+            float4 gr[U], gi[U];
+            auto request = [&](int c0, int h) {
+                const float* xr = add_res ? p.r_re : p.d_re;
+                const float* xi = add_res ? p.r_im : p.d_im;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int idx = et + 128 * j;
+                for (int j = 0; j < U; ++j) {
+                    const int idx = et + 128 * (h + j);
                     const int gm = m0 + (idx >> 2), gn = n0 + c0 + (idx & 3) * 4;
                     gr[j] = make_float4(0.f, 0.f, 0.f, 0.f); gi[j] = gr[j];
                     if (gm >= p.M || gn >= p.N) continue;
                     const size_t o = (size_t) gm * p.N + gn;
-                    gr[j] = ld_global_now(sr + o);
-                    gi[j] = ld_global_now(si + o);
+                    gr[j] = ld_global_now(xr + o);
+                    gi[j] = ld_global_now(xi + o);
                 }
             };
             const int c_first = group * 64, c_last = c_first + 48;
-            if (pre) request(c_first);
-            mbar_wait(acc_full, (uint32_t) seg & 1, abort_flag, p.status, 3);
-            epi_bar_sync(group);                     // everyone arrives, then agree on the outcome
-            if (*abort_flag) { live = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-            for (int c0 = c_first; c0 <= c_last; c0 += 16) {
-                {
+            if (!DRAIN && pre) request(c_first, 0);
+            if constexpr (DRAIN) {
+                if (!sum_chains(kb1 - kb0)) { live = false; break; }
+            } else {
+                mbar_wait(acc_full, (uint32_t) seg & 1, abort_flag, p.status, 3);
+                epi_bar_sync(group);                 // everyone arrives, then agree on the outcome
+                if (*abort_flag) { live = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+#pragma unroll(DRAIN ? 4 : 1)
+            for (int round = 0; round < 4; ++round) {
+                const int c0 = c_first + 16 * round;
+                if constexpr (DRAIN) {
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4) {
+                        const uint32_t o = stage + stage_off(row, i / 4);
+                        const int k = DRAIN ? 16 * round + i : 0;        // (the other form has one element)
+                        st_shared4(o, out(sr[k]), out(sr[k + 1]), out(sr[k + 2]), out(sr[k + 3]));
+                        st_shared4(o + STAGE_PLANE, out(si[k]), out(si[k + 1]), out(si[k + 2]), out(si[k + 3]));
+                    }
+                } else {
                     float a[16], f[16], b[16], e[16];
                     tmem_ld16(tl + c0, a);                   // A_re.B_re
                     tmem_ld16(tl + 384 + c0, f);             // A_im.B_im
@@ -904,50 +991,54 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                                    out(e[i + 2] - sgn * b[i + 2]), out(e[i + 3] - sgn * b[i + 3]));
                     }
                 }
-                if (c0 == c_last) {
+                if (!DRAIN && c0 == c_last) {
                     // last TMEM read of this segment done: hand the accumulators back to the MMA warp
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 }
                 epi_bar_sync(group);
-                if (c0 == c_last && et == 0) {
+                if (!DRAIN && c0 == c_last && et == 0) {
                     if constexpr (PAIR) mbar_arrive_cluster(map_to_rank(acc_empty, lead_rank));   // the first CTA's MMA thread waits for both
                     else mbar_arrive(acc_empty);
                 }
                 if constexpr (VEC) {
                     // coalesced write-out: each warp instruction covers 8 rows x 64 contiguous bytes
-                    float4 vr[4], vi[4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int idx = et + 128 * j;
-                        const uint32_t at = stage + stage_off(idx >> 2, idx & 3);
-                        vr[j] = ld_shared4(at);
-                        vi[j] = ld_shared4(at + STAGE_PLANE);
-                    }
-                    if (pre) {
+                    for (int h = 0; h < 4; h += U) {
+                        float4 vr[U], vi[U];
+                        if (DRAIN && pre) request(c0, h);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            vr[j].x += gr[j].x; vr[j].y += gr[j].y; vr[j].z += gr[j].z; vr[j].w += gr[j].w;
-                            vi[j].x += gi[j].x; vi[j].y += gi[j].y; vi[j].z += gi[j].z; vi[j].w += gi[j].w;
+                        for (int j = 0; j < U; ++j) {
+                            const int idx = et + 128 * (h + j);
+                            const uint32_t at = stage + stage_off(idx >> 2, idx & 3);
+                            vr[j] = ld_shared4(at);
+                            vi[j] = ld_shared4(at + STAGE_PLANE);
                         }
-                        if (c0 != c_last) request(c0 + 16);
-                    }
+                        if (pre) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int idx = et + 128 * j;
-                        const int gm = m0 + (idx >> 2), gn = n0 + c0 + (idx & 3) * 4;
-                        if (gm >= p.M || gn >= p.N) continue;
-                        const size_t o = (size_t) gm * p.N + gn;
-                        if (add_res && need_old) {       // both at once: old D is read here
-                            const float4 xr = *reinterpret_cast<const float4*>(p.d_re + o), xi = *reinterpret_cast<const float4*>(p.d_im + o);
-                            vr[j].x += xr.x; vr[j].y += xr.y; vr[j].z += xr.z; vr[j].w += xr.w;
-                            vi[j].x += xi.x; vi[j].y += xi.y; vi[j].z += xi.z; vi[j].w += xi.w;
+                            for (int j = 0; j < U; ++j) {
+                                vr[j].x += gr[j].x; vr[j].y += gr[j].y; vr[j].z += gr[j].z; vr[j].w += gr[j].w;
+                                vi[j].x += gi[j].x; vi[j].y += gi[j].y; vi[j].z += gi[j].z; vi[j].w += gi[j].w;
+                            }
+                            if (!DRAIN && c0 != c_last) request(c0 + 16, 0);
                         }
-                        if (partial) {
-                            atomicAdd(reinterpret_cast<float4*>(p.d_re + o), vr[j]);
-                            atomicAdd(reinterpret_cast<float4*>(p.d_im + o), vi[j]);
-                        } else {
-                            *reinterpret_cast<float4*>(p.d_re + o) = vr[j];
-                            *reinterpret_cast<float4*>(p.d_im + o) = vi[j];
+#pragma unroll
+                        for (int j = 0; j < U; ++j) {
+                            const int idx = et + 128 * (h + j);
+                            const int gm = m0 + (idx >> 2), gn = n0 + c0 + (idx & 3) * 4;
+                            if (gm >= p.M || gn >= p.N) continue;
+                            const size_t o = (size_t) gm * p.N + gn;
+                            if (add_res && need_old) {   // both at once: old D is read here
+                                const float4 xr = *reinterpret_cast<const float4*>(p.d_re + o), xi = *reinterpret_cast<const float4*>(p.d_im + o);
+                                vr[j].x += xr.x; vr[j].y += xr.y; vr[j].z += xr.z; vr[j].w += xr.w;
+                                vi[j].x += xi.x; vi[j].y += xi.y; vi[j].z += xi.z; vi[j].w += xi.w;
+                            }
+                            if (partial) {
+                                atomicAdd(reinterpret_cast<float4*>(p.d_re + o), vr[j]);
+                                atomicAdd(reinterpret_cast<float4*>(p.d_im + o), vi[j]);
+                            } else {
+                                *reinterpret_cast<float4*>(p.d_re + o) = vr[j];
+                                *reinterpret_cast<float4*>(p.d_im + o) = vi[j];
+                            }
                         }
                     }
                 } else {
@@ -1357,8 +1448,18 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
 
 namespace cnb {
 
+// Sizes whose products have always been split ones here, at 19 bits an operand: packed ones are nearer to float64 there
+// whatever the length of the chain (512 x 1024 x 1024: 1.9e-6 -> 0.9e-6, 4096 x 1024 x 1024: 4.5e-6 -> 3.1e-6).
+static bool split_sizes(int M, int N, int K) { return K % 8 == 0 && K >= 32 && M >= 64 && N >= 64; }
+
+// Every other size could run as fp32 FMAs (cgemm_simt.cu), and the tiles must not be less exact than those.  The tensor
+// core truncates as it accumulates: measured on balanced data one chain of C products is off by 4.2e-9 C of the result,
+// rounded FMAs over K products by 1.8e-8 sqrt(K), and a sum of chains rounded to nearest by what one chain is.  So a chain
+// may be 4.28 sqrt(K) long, in blocks of 32.
+static int max_chain(int K) { return std::max(1, (int) (4.28 * std::sqrt((double) K) / FormCfg<PACKED>::BK)); }
+
 bool cgemm_tc_shape_ok(int M, int N, int K) {
-    if (K % 8 == 0 && K >= 32 && M >= 64 && N >= 64) return true;
+    if (split_sizes(M, N, K)) return true;
     // Other sizes leave more of the 128 x 128 tiles empty: from about two million complex multiplications on packing
     // and tiles together take less than the fp32 SIMT tiles (777 x 1001 x 1333: 330 against 45 us), below it they do not.
     return K >= 48 && (double) M * N * K >= (double) (1 << 21);
@@ -1385,9 +1486,14 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
                       int accumulate, cudaStream_t st) {
     static bool attr_set[64] = {};                       // the attribute is per device
     if (!attr_set[ctx->device & 63]) {
-#define CNB_TC_ATTR(P, V, F) CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<P, V, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES))
-        CNB_TC_ATTR(false, false, SPLIT); CNB_TC_ATTR(true, false, SPLIT); CNB_TC_ATTR(false, true, SPLIT); CNB_TC_ATTR(true, true, SPLIT);
-        CNB_TC_ATTR(false, false, PACKED); CNB_TC_ATTR(true, false, PACKED); CNB_TC_ATTR(false, true, PACKED); CNB_TC_ATTR(true, true, PACKED);
+#define CNB_TC_ATTR(F, D)                                                                                                   \
+    do {                                                                                                                    \
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, false, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES)); \
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, true, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));  \
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, false, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));  \
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, true, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));   \
+    } while (0)
+        CNB_TC_ATTR(SPLIT, false); CNB_TC_ATTR(PACKED, false); CNB_TC_ATTR(PACKED, true);
 #undef CNB_TC_ATTR
         attr_set[ctx->device & 63] = true;
     }
@@ -1453,14 +1559,19 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     auto go = [&](auto kernel, const auto& maps) {
         return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(NUM_THREADS), SMEM_BYTES, st, pair ? 2 * cluster : cluster, maps, p);
     };
+    // the longest run of k-blocks that one CTA sums for a tile
+    const int k_blocks = (K + bk - 1) / bk;
+    const int run = cluster > 1 ? (k_blocks + cluster - 1) / cluster : q.whole_per_cta > 0 ? k_blocks : (int) std::min<long>(q.upc, k_blocks);
+    p.chain = max_chain(K);
+    const bool drain = packed && !split_sizes(M, N, K) && run > p.chain;
     cudaError_t e;
-    if (packed) {
-        if (pair) e = vec ? go(cgemm_tc_k<true, true, PACKED>, maps_p) : go(cgemm_tc_k<true, false, PACKED>, maps_p);
-        else e = vec ? go(cgemm_tc_k<false, true, PACKED>, maps_p) : go(cgemm_tc_k<false, false, PACKED>, maps_p);
-    } else {
-        if (pair) e = vec ? go(cgemm_tc_k<true, true, SPLIT>, maps_s) : go(cgemm_tc_k<true, false, SPLIT>, maps_s);
-        else e = vec ? go(cgemm_tc_k<false, true, SPLIT>, maps_s) : go(cgemm_tc_k<false, false, SPLIT>, maps_s);
-    }
+#define CNB_TC_GO(F, D, maps)                                                                                              \
+    (pair ? (vec ? go(cgemm_tc_k<true, true, F, D>, maps) : go(cgemm_tc_k<true, false, F, D>, maps))                       \
+          : (vec ? go(cgemm_tc_k<false, true, F, D>, maps) : go(cgemm_tc_k<false, false, F, D>, maps)))
+    if (drain) e = CNB_TC_GO(PACKED, true, maps_p);
+    else if (packed) e = CNB_TC_GO(PACKED, false, maps_p);
+    else e = CNB_TC_GO(SPLIT, false, maps_s);
+#undef CNB_TC_GO
     CNB_CUDA(e);
     CNB_LAUNCH_CHECK("cgemm_tc");
     return CNB_OK;
