@@ -14,7 +14,7 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3",
 
 def _sources():
     src = [os.path.join(HERE, "csrc", f) for f in CSRC] + [os.path.join(HERE, "host", f) for f in HOST]
-    deps = src + [os.path.join(HERE, "csrc", "common.cuh"), os.path.join(HERE, "csrc", "fft_regs.cuh"), os.path.join(HERE, "csrc", "fft_mixed.cuh"), os.path.join(HERE, "host", "cnet.h"), os.path.join(HERE, "host", "dp_nccl.h"), os.path.join(HERE, "host", "data_reader.h"),
+    deps = src + [os.path.join(HERE, "csrc", "common.cuh"), os.path.join(HERE, "csrc", "cgemm_fma.cuh"), os.path.join(HERE, "csrc", "fft_regs.cuh"), os.path.join(HERE, "csrc", "fft_mixed.cuh"), os.path.join(HERE, "host", "cnet.h"), os.path.join(HERE, "host", "dp_nccl.h"), os.path.join(HERE, "host", "data_reader.h"),
                   os.path.join(HERE, "..", "include", "cnet_b200.h"),
                   os.path.join(HERE, "..", "include", "cnet_b200_host.h")]
     return src, deps

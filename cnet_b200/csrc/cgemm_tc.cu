@@ -52,6 +52,7 @@
 #include <cmath>
 #include <cstdlib>
 
+#include "cgemm_fma.cuh"
 #include "common.cuh"
 
 namespace {
@@ -94,8 +95,11 @@ struct TcParams {
     int whole_per_cta;        // > 0: every CTA first takes that many whole tiles, then its run of the remaining units
     int segments;             // > 0: CTA r takes k-segment r / tiles of tile r % tiles (units_per_cta k-blocks each)
     int chain;                // DRAIN: k-blocks that are summed in tensor memory at most
-    const int* a_exp;         // PACKED: the powers of two that A and B were scaled by
+    const int* a_exp;         // PACKED: the powers of two that A and B were scaled by, or kPlain
     const int* b_exp;
+    const void* a_planes; const void* b_planes;       // PACKED: what the tensor maps describe, for the FMA form
+    size_t a_np, b_np;
+    int a_pitch, b_pitch;
     int* status;
     // The pair form (cgemm_tc_k<true>): cluster = K slices per tile, each slice a CTA pair (cluster of 2 * cluster CTAs).
 };
@@ -335,6 +339,40 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Packed operands: a matrix that is stored as fp32 planes instead of fp16 parts has this for its exponent.
+constexpr int kPlain = 1 << 20;
+
+struct PackedElement {
+    const void* planes;
+    size_t np;
+    int pitch, exponent;
+    bool k_fast;                             // stored [rows, K]
+    __device__ __forceinline__ float2 operator()(int row, int k) const {
+        const size_t o = k_fast ? (size_t) row * pitch + k : (size_t) k * pitch + row;
+        if (exponent == kPlain) {
+            const float* f = static_cast<const float*>(planes) + o;
+            return make_float2(f[0], f[np]);
+        }
+        const __half* h = static_cast<const __half*>(planes) + o;
+        const float unscale = __uint_as_float((unsigned) (127 - exponent) << 23);
+        return make_float2((__half2float(h[0]) + __half2float(h[2 * np])) * unscale, (__half2float(h[np]) + __half2float(h[3 * np])) * unscale);
+    }
+};
+
+// The product where an operand is plain: fp32 FMAs by the epilogue's threads, the CTAs of the launch taking 64 x 64 tiles
+// in turn whatever the schedule, after the tile product of the same bytes (which meant nothing) has run without a store.
+// Nothing waits for the exponents that way where no operand is plain.  1.7 ms at 4096 x 1024 x 1024
+// (80 us as a tile product), 0.24 ms at 512 rows (17 us).
+__device__ __noinline__ void fma_product(const TcParams& p, void* smem) {
+    const PackedElement a = {p.a_planes, p.a_np, p.a_pitch, *p.a_exp, !p.a_mn}, b = {p.b_planes, p.b_np, p.b_pitch, *p.b_exp, !p.b_mn};
+    const cnb_fma::Result r = {p.d_re, p.d_im, p.r_re, p.r_im, p.M, p.N, p.K, p.conjB, p.accumulate};
+    const int tiles_n = (p.N + cnb_fma::TN - 1) / cnb_fma::TN, tiles = (p.M + cnb_fma::TM - 1) / cnb_fma::TM * tiles_n;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x)
+        cnb_fma::tile(a, b, r, *static_cast<cnb_fma::Slabs*>(smem), t / tiles_n * cnb_fma::TM, t % tiles_n * cnb_fma::TN,
+                      (int) threadIdx.x - (NUM_THREADS - EPI_THREADS),
+                      [] { asm volatile("bar.sync %0, %1;" ::"n"(1 + EPI_GROUPS), "n"(EPI_THREADS) : "memory"); });
+}
+
 // The accumulators of one chain (this thread's row, the 64 columns of its group from `tl` on) into the running sums,
 // rounded to nearest.
 __device__ __forceinline__ void drain_chain(uint32_t tl, float sgn, float (&sr)[64], float (&si)[64]) {
@@ -528,7 +566,7 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 // forward off by 4.4e-7 of float64 instead of 2.4e-6 (fp32 FMAs: 6.6e-7).
 template <bool PAIR, bool VEC, int FORM, bool DRAIN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
+cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__ TcParams p) {
     extern __shared__ uint8_t smem_raw[];
     constexpr int BK = FormCfg<FORM>::BK;
     CNB_GSTAMP(0, threadIdx.x == 0);
@@ -623,6 +661,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
     cnb_pdl_trigger();
     cnb_pdl_wait();
     CNB_GSTAMP(1, threadIdx.x == 0);
+    bool plain = false;                                  // known to the epilogue's warps
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -843,11 +882,14 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
         // PACKED: the scales of both operands are taken out again, in two factors so that neither leaves fp32's range
         float u0 = 1.f, u1 = 1.f;
         if constexpr (FORM == PACKED) {
-            const int e = -(*p.a_exp + *p.b_exp), h = e >> 1;
+            const int ea = *p.a_exp, eb = *p.b_exp;
+            plain = ea == kPlain || eb == kPlain;
+            const int e = -(ea + eb), h = e >> 1;
             u0 = __uint_as_float((uint32_t) (h + 127) << 23);
             u1 = __uint_as_float((uint32_t) (e - h + 127) << 23);
         }
         auto out = [&](float v) { return FORM == PACKED ? v * u0 * u1 : v; };
+        const int rows = plain ? 0 : p.M;                // plain: nothing is read of D or R, or stored
         const uint32_t stage = smem_base + OPERAND_BYTES + (uint32_t) group * 2 * STAGE_PLANE;
         int seg = 0;
         // DRAIN: the chains of one segment of `blocks` k-blocks into the running sums; false after a wait gave up
@@ -948,7 +990,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                     const int idx = et + 128 * (h + j);
                     const int gm = m0 + (idx >> 2), gn = n0 + c0 + (idx & 3) * 4;
                     gr[j] = make_float4(0.f, 0.f, 0.f, 0.f); gi[j] = gr[j];
-                    if (gm >= p.M || gn >= p.N) continue;
+                    if (gm >= rows || gn >= p.N) continue;
                     const size_t o = (size_t) gm * p.N + gn;
                     gr[j] = ld_global_now(xr + o);
                     gi[j] = ld_global_now(xi + o);
@@ -1025,7 +1067,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                         for (int j = 0; j < U; ++j) {
                             const int idx = et + 128 * (h + j);
                             const int gm = m0 + (idx >> 2), gn = n0 + c0 + (idx & 3) * 4;
-                            if (gm >= p.M || gn >= p.N) continue;
+                            if (gm >= rows || gn >= p.N) continue;
                             const size_t o = (size_t) gm * p.N + gn;
                             if (add_res && need_old) {   // both at once: old D is read here
                                 const float4 xr = *reinterpret_cast<const float4*>(p.d_re + o), xi = *reinterpret_cast<const float4*>(p.d_im + o);
@@ -1052,7 +1094,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
                         for (int j = 0; j < 8; ++j) {
                             const int gm = m0 + r0 + 2 * j;
                             const size_t o = (size_t) gm * p.N + gn;
-                            const bool on = gm < p.M && gn < p.N;
+                            const bool on = gm < rows && gn < p.N;
                             ar[j] = ai[j] = 0.f;
                             if (on && add_res) { ar[j] = ld_global_now1(p.r_re + o); ai[j] = ld_global_now1(p.r_im + o); }
                             if (on && need_old) { ar[j] += ld_global_now1(p.d_re + o); ai[j] += ld_global_now1(p.d_im + o); }
@@ -1066,7 +1108,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
                             const int gm = m0 + r0 + 2 * j;
-                            if (gm >= p.M || gn >= p.N) continue;
+                            if (gm >= rows || gn >= p.N) continue;
                             const size_t o = (size_t) gm * p.N + gn;
                             if (partial) { atomicAdd(p.d_re + o, ar[j]); atomicAdd(p.d_im + o, ai[j]); }
                             else { p.d_re[o] = ar[j]; p.d_im[o] = ai[j]; }
@@ -1090,7 +1132,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
         // Every thread of every CTA of the cluster reaches both barriers, also after a bounded wait gave up.
         cluster_sync();                                  // all partial tiles are in shared memory
         CNB_GSTAMP(6, threadIdx.x == 64);
-        if (warp >= 2 && !*abort_flag) {
+        if (warp >= 2 && !plain && !*abort_flag) {
             const int tile = blockIdx.x / cluster_ctas;
             const int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
             const int et = (warp - 2) * 32 + lane;
@@ -1105,6 +1147,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const TcParams p) {
         cluster_sync();                                  // no CTA leaves while a peer still reads its shared memory
         CNB_GSTAMP(8, threadIdx.x == 64);
     }
+    if (FORM == PACKED && plain) fma_product(p, smem);   // shared memory is idle: every chain has been read out
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -1130,41 +1173,103 @@ __global__ void split_k(const float* __restrict__ s0, const float* __restrict__ 
 }
 
 // Packed operands.  x = 2^-e (high + low), high = fp16(x 2^e), low = fp16(x 2^e - high), with one e for the whole
-// matrix that brings its largest component into [2^14, 2^15): 22 bits of every component down to 2^-18 of the largest
-// (2^-14, fp16's least normal, is 2^-29 of it, and low starts 11 bits lower), fewer below, an absolute error of 2^-40
-// of the largest at most.  A first pass finds the largest component, the second packs.
+// matrix that brings its largest component into [2^14, 2^15): 22 bits of every component down to 2^-17 of the largest,
+// fewer below, an absolute error of 2^-39 of the largest at most (half of fp16's least subnormal, 2^-25, beside 2^14).
+//
+// That must not cost what fp32's exponent range gave: rows of another scale than their neighbours keep their own
+// relative precision in the forward product and dX*, columns in dW*.  So the first pass also finds the largest component
+// of every group of 1 x 128 and of 32 x 1 elements, and a matrix in which one of these (not all zero) lies below 2^-17 of
+// the largest is stored as it is, as fp32 planes in the same bytes, and multiplied in fp32 FMAs.
 struct PackJob {
     const float* re; const float* im;
-    __half* dst;                       // four planes of rows * pitch: high re, high im, low re, low im
-    cnb_pack_head* head;               // max_bits and ticket are zero between uses
-    int rows, cols, pitch, blocks;
+    __half* dst;                       // four planes of rows * pitch: high re, high im, low re, low im (or two of float)
+    cnb_pack_head* head;               // max_bits, low_bits and ticket are zero between uses
+    int rows, cols, pitch, blocks, max_blocks;
 };
 template <int N> struct PackJobs { PackJob j[N]; };
 
-__device__ __forceinline__ int pack_exponent(unsigned max_bits) {
-    const int e = 14 + 127 - (int) (max_bits >> 23);     // all zero: 2^126 of nothing
-    return e > 126 ? 126 : e;
+constexpr int GROUP_ROWS = 32, GROUP_COLS = 128;
+
+__device__ __forceinline__ bool pack_vec(const PackJob& job) {
+    return job.cols % 4 == 0 && ((reinterpret_cast<uintptr_t>(job.re) | reinterpret_cast<uintptr_t>(job.im)) & 15) == 0;
 }
 
+// kPlain: some group is too small beside the largest component, or that itself is so small that no scale of fp32 brings it to 2^14.
+__device__ __forceinline__ int pack_exponent(unsigned max_bits, unsigned low_bits) {
+    if (max_bits == 0) return 0;
+    const int e = 14 + 127 - (int) (max_bits >> 23);
+    const bool wide = low_bits != 0 && __uint_as_float(~low_bits) < __uint_as_float(max_bits) * 0x1p-17f;
+    return wide || e > 126 ? kPlain : e;
+}
+
+// Blocks take tiles of GROUP_ROWS x GROUP_COLS in turn, a warp four rows of a tile and a lane four elements of each.
 template <int N>
 __global__ void __launch_bounds__(256) pack_max_k(const __grid_constant__ PackJobs<N> jobs) {
     cnb_pdl_enter();
     const PackJob& job = jobs.j[blockIdx.y];
-    if ((int) blockIdx.x >= job.blocks) return;
-    const size_t n = (size_t) job.rows * job.cols, step = (size_t) job.blocks * 256;
-    unsigned m = 0;
-    size_t done = 0;
-    if (((reinterpret_cast<uintptr_t>(job.re) | reinterpret_cast<uintptr_t>(job.im)) & 15) == 0) {
-        const size_t n4 = n / 4;
-        for (size_t i = (size_t) blockIdx.x * 256 + threadIdx.x; i < n4; i += step) {
-            const float4 a = reinterpret_cast<const float4*>(job.re)[i], b = reinterpret_cast<const float4*>(job.im)[i];
-            m = max(m, max(max(cnb_scale_bits(a.x), cnb_scale_bits(a.y)), max(cnb_scale_bits(a.z), cnb_scale_bits(a.w))));
-            m = max(m, max(max(cnb_scale_bits(b.x), cnb_scale_bits(b.y)), max(cnb_scale_bits(b.z), cnb_scale_bits(b.w))));
+    if ((int) blockIdx.x >= job.max_blocks) return;
+    __shared__ unsigned col[8][GROUP_COLS], block_most[8], block_low[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool vec = pack_vec(job);
+    const int tiles_x = (job.cols + GROUP_COLS - 1) / GROUP_COLS;
+    const long tiles = (long) ((job.rows + GROUP_ROWS - 1) / GROUP_ROWS) * tiles_x;
+    unsigned most = 0, low = 0;        // low: ~ of the least group maximum, 0 while there is none
+    for (long t = blockIdx.x; t < tiles; t += job.max_blocks) {
+        const int r0 = (int) (t / tiles_x) * GROUP_ROWS + warp, c0 = (int) (t % tiles_x) * GROUP_COLS;
+        float re[4][4], im[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = r0 + 8 * i;
+            const size_t at = (size_t) row * job.cols + c0;
+            if (vec) {
+                const bool on = row < job.rows && c0 + 4 * lane < job.cols;
+                const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 x = on ? *reinterpret_cast<const float4*>(job.re + at + 4 * lane) : z;
+                const float4 y = on ? *reinterpret_cast<const float4*>(job.im + at + 4 * lane) : z;
+                re[i][0] = x.x; re[i][1] = x.y; re[i][2] = x.z; re[i][3] = x.w;
+                im[i][0] = y.x; im[i][1] = y.y; im[i][2] = y.z; im[i][3] = y.w;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const bool on = row < job.rows && c0 + lane + 32 * k < job.cols;
+                    re[i][k] = on ? job.re[at + lane + 32 * k] : 0.f;
+                    im[i][k] = on ? job.im[at + lane + 32 * k] : 0.f;
+                }
+            }
         }
-        done = n4 * 4;
+        unsigned c[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            unsigned g = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const unsigned m = max(cnb_scale_bits(re[i][k]), cnb_scale_bits(im[i][k]));
+                c[k] = max(c[k], m);
+                g = max(g, m);
+            }
+            g = __reduce_max_sync(0xffffffffu, g);
+            most = max(most, g);
+            if (g) low = max(low, ~g);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) col[warp][k * 32 + lane] = c[k];      // every column has a place of its own
+        __syncthreads();
+        if (threadIdx.x < GROUP_COLS) {
+            unsigned g = 0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) g = max(g, col[w][threadIdx.x]);
+            if (g) low = max(low, ~g);
+        }
+        __syncthreads();
     }
-    for (size_t i = done + (size_t) blockIdx.x * 256 + threadIdx.x; i < n; i += step) m = max(m, max(cnb_scale_bits(job.re[i]), cnb_scale_bits(job.im[i])));
-    cnb_pack_max_block(job.head, m);
+    low = __reduce_max_sync(0xffffffffu, low);
+    if (lane == 0) { block_most[warp] = most; block_low[warp] = low; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) { most = max(most, block_most[w]); low = max(low, block_low[w]); }
+        atomicMax(&job.head->max_bits, most);
+        atomicMax(&job.head->low_bits, low);
+    }
 }
 
 template <int N>
@@ -1174,20 +1279,23 @@ __global__ void __launch_bounds__(256) pack_k(const __grid_constant__ PackJobs<N
     if ((int) blockIdx.x >= job.blocks) return;
     __shared__ int s_exp;
     if (threadIdx.x == 0) {
-        const int e = pack_exponent(__ldcg(&job.head->max_bits));
+        const int e = pack_exponent(__ldcg(&job.head->max_bits), __ldcg(&job.head->low_bits));
         s_exp = e;
         if (blockIdx.x == 0) job.head->exponent = e;
         __threadfence();
         if (atomicAdd(&job.head->ticket, 1u) == (unsigned) job.blocks - 1) {      // every block has read it: ready for the next use
             job.head->max_bits = 0;
+            job.head->low_bits = 0;
             job.head->ticket = 0;
         }
     }
     __syncthreads();
-    const float scale = __uint_as_float((unsigned) (s_exp + 127) << 23);
+    const bool plain = s_exp == kPlain;
+    const float scale = plain ? 1.f : __uint_as_float((unsigned) (s_exp + 127) << 23);
+    float* const plain_dst = reinterpret_cast<float*>(job.dst);
     // Consecutive threads take consecutive columns: four each where the rows allow 16-byte loads (8-byte stores), else
     // two (4-byte accesses), so that every access of a warp is one run.
-    const bool vec = job.cols % 4 == 0 && ((reinterpret_cast<uintptr_t>(job.re) | reinterpret_cast<uintptr_t>(job.im)) & 15) == 0;
+    const bool vec = pack_vec(job);
     const size_t np = (size_t) job.rows * job.pitch;
     const int groups = vec ? job.cols / 4 : (job.cols + 1) / 2;
     const size_t total = (size_t) job.rows * groups;
@@ -1205,6 +1313,11 @@ __global__ void __launch_bounds__(256) pack_k(const __grid_constant__ PackJobs<N
         if (vec) {
             const size_t src = flat ? 4 * i : (size_t) row * job.cols + 4 * g, dst = flat ? 4 * i : (size_t) row * job.pitch + 4 * g;
             const float4 x = *reinterpret_cast<const float4*>(job.re + src), y = *reinterpret_cast<const float4*>(job.im + src);
+            if (plain) {
+                *reinterpret_cast<float4*>(plain_dst + dst) = x;
+                *reinterpret_cast<float4*>(plain_dst + np + dst) = y;
+                continue;
+            }
             __align__(8) __half2 hi[2], lo[2];
             part(x.x, x.y, &hi[0], &lo[0]); part(x.z, x.w, &hi[1], &lo[1]);
             *reinterpret_cast<uint2*>(job.dst + dst) = *reinterpret_cast<uint2*>(hi);
@@ -1218,6 +1331,11 @@ __global__ void __launch_bounds__(256) pack_k(const __grid_constant__ PackJobs<N
             const size_t src = (size_t) row * job.cols + c, dst = (size_t) row * job.pitch + c;
             const float x0 = job.re[src], y0 = job.im[src];
             const float x1 = two ? job.re[src + 1] : 0.f, y1 = two ? job.im[src + 1] : 0.f;
+            if (plain) {
+                *reinterpret_cast<float2*>(plain_dst + dst) = make_float2(x0, x1);
+                *reinterpret_cast<float2*>(plain_dst + np + dst) = make_float2(y0, y1);
+                continue;
+            }
             __half2 hi, lo;
             part(x0, x1, &hi, &lo);
             *reinterpret_cast<__half2*>(job.dst + dst) = hi;
@@ -1550,6 +1668,9 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     p.units_per_cta = (int) q.upc;
     p.a_mn = a.mn; p.b_mn = b.mn;
     p.a_exp = a.exponent; p.b_exp = b.exponent;
+    p.a_planes = a.base; p.b_planes = b.base;
+    p.a_np = a.plane_pitch; p.b_np = b.plane_pitch;
+    p.a_pitch = a.pitch; p.b_pitch = b.pitch;
     p.cluster = cluster;
     p.whole_per_cta = q.whole_per_cta;
     p.segments = q.segments;
@@ -1582,33 +1703,33 @@ SplitOperand packed_operand(const PackRequest& r, int mn) {
     return {static_cast<const float*>(r.planes), (size_t) r.rows * r.pitch, r.pitch, mn, &r.head->exponent};
 }
 
-// Jobs in pairs of launches of at most 32; have_max: the heads already hold the largest components.
-template <int N> static int pack_some(cnb_ctx* ctx, const PackRequest* r, int n, bool have_max, cudaStream_t st) {
+// Jobs in pairs of launches of at most 32.
+template <int N> static int pack_some(cnb_ctx* ctx, const PackRequest* r, int n, cudaStream_t st) {
     PackJobs<N> jobs;
-    int blocks = 0;
+    int blocks = 0, max_blocks = 0;
     // enough blocks in all to fill the device twice over, whatever the number of jobs
     const size_t cap = std::max<size_t>(16, (size_t) ctx->sm_count * 16 / n);
     for (int k = 0; k < n; ++k) {
         if (reinterpret_cast<uintptr_t>(r[k].planes) & 127 || r[k].pitch % 8)
             return set_error(CNB_ERR_ARG, "pack: planes must be 128-byte aligned, pitch %d a multiple of 8", r[k].pitch);
         const size_t items = (size_t) r[k].rows * ((r[k].cols + 3) / 4);
+        const size_t tiles = ((size_t) (r[k].rows + GROUP_ROWS - 1) / GROUP_ROWS) * ((r[k].cols + GROUP_COLS - 1) / GROUP_COLS);
         jobs.j[k] = {r[k].re, r[k].im, static_cast<__half*>(r[k].planes), r[k].head, r[k].rows, r[k].cols, r[k].pitch,
-                     (int) std::min((items + 255) / 256, cap)};
+                     (int) std::min((items + 255) / 256, cap), (int) std::min(tiles, cap)};
         blocks = std::max(blocks, jobs.j[k].blocks);
+        max_blocks = std::max(max_blocks, jobs.j[k].max_blocks);
     }
-    if (!have_max) {
-        cnb::launch(pack_max_k<N>, dim3(blocks, n), dim3(256), 0, st, 1, jobs);
-        CNB_LAUNCH_CHECK("pack_max");
-    }
+    cnb::launch(pack_max_k<N>, dim3(max_blocks, n), dim3(256), 0, st, 1, jobs);
+    CNB_LAUNCH_CHECK("pack_max");
     cnb::launch(pack_k<N>, dim3(blocks, n), dim3(256), 0, st, 1, jobs);
     CNB_LAUNCH_CHECK("pack");
     return CNB_OK;
 }
 
-int pack(cnb_ctx* ctx, const PackRequest* r, int n, bool have_max, cudaStream_t st) {
-    if (n <= 2) return pack_some<2>(ctx, r, n, have_max, st);
+int pack(cnb_ctx* ctx, const PackRequest* r, int n, cudaStream_t st) {
+    if (n <= 2) return pack_some<2>(ctx, r, n, st);
     for (int k = 0; k < n; k += 32) {
-        const int rc = pack_some<32>(ctx, r + k, std::min(32, n - k), have_max, st);
+        const int rc = pack_some<32>(ctx, r + k, std::min(32, n - k), st);
         if (rc != CNB_OK) return rc;
     }
     return CNB_OK;
@@ -1628,7 +1749,7 @@ int cgemm_tc_run(cnb_ctx* ctx, const float* a_re, const float* a_im, int a_trans
     r[0] = {a_re, a_im, a_trans ? K : M, a_trans ? M : K, operand_pitch(M, K, a_trans), ws, heads};
     if (b_packed) r[1] = *b_packed;
     else r[1] = {b_re, b_im, b_trans ? K : N, b_trans ? N : K, operand_pitch(N, K, b_trans), reinterpret_cast<char*>(ws) + na, heads + 1};
-    rc = pack(ctx, r, b_packed ? 1 : 2, false, st);
+    rc = pack(ctx, r, b_packed ? 1 : 2, st);
     if (rc != CNB_OK) return rc;
     return cgemm_tc_presplit(ctx, packed_operand(r[0], a_trans), packed_operand(r[1], b_trans), conjB, r_re, r_im, d_re, d_im, M, N,
                              K, accumulate, st);

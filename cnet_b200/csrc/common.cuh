@@ -17,9 +17,9 @@ struct cnb_twiddle {
     void* pack = nullptr;  // the matrix packed (made once; head, then planes), or null when the tiles cannot take it
 };
 
-// Head of a packed operand: the scale's exponent, the largest component (the bits of its magnitude) on its way to
-// becoming that, and how many blocks of the packing launch have read it.
-struct cnb_pack_head { int exponent; unsigned max_bits, ticket, unused; };
+// Head of a packed operand: the scale's exponent; on their way to becoming that, the largest component and the
+// complement of the least group maximum (as bits of magnitudes); how many blocks of the packing launch have read them.
+struct cnb_pack_head { int exponent; unsigned max_bits, ticket, low_bits; };
 
 struct cnb_ctx {
     int device = 0;
@@ -74,7 +74,7 @@ struct PackRequest {
     void* planes;                      // 8 * rows * pitch bytes, 128-byte aligned
     cnb_pack_head* head;               // zeroed before the first use
 };
-int pack(cnb_ctx* ctx, const PackRequest* r, int n, bool have_max, cudaStream_t st);
+int pack(cnb_ctx* ctx, const PackRequest* r, int n, cudaStream_t st);
 // fp32 operands, packed into scratch first: a_trans / b_trans = the source planes are stored [K, rows]; b_packed: a
 // constant B that its owner has packed.
 int cgemm_tc_run(cnb_ctx* ctx, const float* a_re, const float* a_im, int a_trans, const float* b_re,
@@ -112,14 +112,9 @@ bool fft_supported(int N);
 int fft_run(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, int B, int N, int inverse,
             int accumulate, cudaStream_t st);
 // Forward FFT whose epilogue also applies Hadamard(h) -> CGelu: u = FFT(x) -> (ur, ui); y = gelu(u o h) ->
-// (yr, yi) and, when sp != NULL, the operand split of y; when head != NULL the largest component of y goes there.
+// (yr, yi) and, when sp != NULL, the operand split of y.
 int fft_hadamard_gelu(cnb_ctx* ctx, const float* xr, const float* xi, const float* hr, const float* hi, float* ur,
-                      float* ui, float* yr, float* yi, float* sp, cnb_pack_head* head, int B, int N, cudaStream_t st);
-
-// w -= lr g over the arena; where *have_max comes back true the heads of the matrices have received their largest new
-// components.
-int sgd_update_max(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zero_grad, const PackRequest* r, int nr,
-                   bool* have_max, cudaStream_t st);
+                      float* ui, float* yr, float* yi, float* sp, int B, int N, cudaStream_t st);
 
 }  // namespace cnb
 
@@ -191,18 +186,6 @@ __device__ __forceinline__ void cnb_split_store4(const cnb_split_dst& d, size_t 
 __device__ __forceinline__ unsigned cnb_scale_bits(float x) {
     const unsigned b = __float_as_uint(x) & 0x7fffffffu;
     return b < 0x7f800000u ? b : 0u;
-}
-
-// the largest of all threads' m into a pack head; every thread of the block (at most 1024) calls it
-__device__ __forceinline__ void cnb_pack_max_block(cnb_pack_head* head, unsigned m) {
-    __shared__ unsigned warp_max[32];
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int) (blockDim.x >> 5); ++w) m = max(m, warp_max[w]);
-        atomicMax(&head->max_bits, m);
-    }
 }
 
 // Programmatic dependent launch.  Every kernel of the step is launched with the "programmatic stream

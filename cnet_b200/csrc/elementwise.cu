@@ -5,8 +5,6 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
-#include <utility>
-#include <vector>
 
 #include "common.cuh"
 
@@ -416,29 +414,6 @@ __global__ void sgd_split_k(float* __restrict__ w, float* __restrict__ g, size_t
     }
 }
 
-// The update of one arena in segments, each of them a plane of a packed matrix or what lies between two: the largest
-// new component of a plane goes to its matrix's head.  blockIdx.y picks the segment.
-constexpr int MAX_SEGMENTS = 129;
-struct SgdSegments {
-    size_t begin[MAX_SEGMENTS], count[MAX_SEGMENTS];
-    cnb_pack_head* head[MAX_SEGMENTS];
-};
-
-__global__ void __launch_bounds__(256) sgd_max_k(float* __restrict__ w, float* __restrict__ g, float lr, int zero_grad,
-                                                 const __grid_constant__ SgdSegments sg) {
-    cnb_pdl_enter();
-    const size_t begin = sg.begin[blockIdx.y], count = sg.count[blockIdx.y];
-    unsigned m = 0;
-    for (size_t i = ((size_t) blockIdx.x * 256 + threadIdx.x) * 4; i < count; i += (size_t) gridDim.x * 1024) {
-        Pack<4> a = ld<4>(w, begin + i), b = ld<4>(g, begin + i);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) { a.v[k] -= lr * b.v[k]; b.v[k] = 0.f; m = max(m, cnb_scale_bits(a.v[k])); }
-        st<4>(w, begin + i, a);
-        if (zero_grad) st<4>(g, begin + i, b);
-    }
-    if (sg.head[blockIdx.y]) cnb_pack_max_block(sg.head[blockIdx.y], m);
-}
-
 template <typename... P> bool all_aligned(P... p) { return (aligned16(p) && ...); }
 
 int colreduce_launch(cnb_ctx* ctx, int mode, const float* gr, const float* gi, const float* ar, const float* ai,
@@ -675,48 +650,6 @@ int cnb_sgd_update_split(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, i
 }
 
 }  // extern "C"
-
-namespace cnb {
-
-int sgd_update_max(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zero_grad, const PackRequest* r, int nr,
-                   bool* have_max, cudaStream_t st) {
-    // segments in arena order; ranges that are no multiples of 16 bytes, or too many of them, take the plain update
-    SgdSegments sg;
-    std::vector<std::pair<size_t, int> > planes;           // begin, matrix
-    bool fits = 2 * nr + 2 * nr + 1 <= MAX_SEGMENTS && n % 4 == 0 && all_aligned(w, g);
-    for (int k = 0; k < nr && fits; ++k) {
-        planes.push_back({(size_t) (r[k].re - w), k});
-        planes.push_back({(size_t) (r[k].im - w), k});
-    }
-    std::sort(planes.begin(), planes.end());
-    int segments = 0;
-    size_t at = 0, longest = 0;
-    auto add = [&](size_t begin, size_t count, cnb_pack_head* head) {
-        if (begin % 4 || count % 4) fits = false;
-        if (count == 0 || !fits) return;
-        sg.begin[segments] = begin; sg.count[segments] = count; sg.head[segments] = head;
-        longest = std::max(longest, count);
-        ++segments;
-    };
-    for (auto& p : planes) {
-        if (!fits || p.first < at) { fits = false; break; }
-        const size_t count = (size_t) r[p.second].rows * r[p.second].cols;
-        add(at, p.first - at, nullptr);
-        add(p.first, count, r[p.second].head);
-        at = p.first + count;
-    }
-    if (fits) add(at, n - at, nullptr);
-    *have_max = fits && nr > 0;
-    if (!*have_max) return cnb_sgd_update(ctx, w, g, n, lr, zero_grad, st);
-    // about 16 blocks per SM over all segments, none with less than 1024 floats
-    const size_t cap = std::max<size_t>(8, (size_t) ctx->sm_count * 16 / segments);
-    const unsigned blocks = (unsigned) std::min((longest + 1023) / 1024, cap);
-    cnb::launch(sgd_max_k, dim3(blocks, segments), dim3(256), 0, st, 1, w, g, lr, zero_grad, sg);
-    CNB_LAUNCH_CHECK("sgd_max");
-    return CNB_OK;
-}
-
-}  // namespace cnb
 
 // ---------------------------------------------------------------------------------------
 // Hadamard backward without any allocation.

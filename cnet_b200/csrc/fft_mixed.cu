@@ -56,7 +56,6 @@ struct Io {
     const float2* src;                // shared-memory buffers, NULL: the planes
     float2* dst;
     int rows;
-    unsigned largest;                 // of the tail's components, this thread's (bits of the magnitude)
     bool spectral;                    // chirp form: this pass opens the inverse transform
     size_t row0;
 };
@@ -141,7 +140,6 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
                         cnb_split_store1(cnb_split_component(ep.sp, ep.np, 0), at, gr);
                         cnb_split_store1(cnb_split_component(ep.sp, ep.np, 1), at, gi);
                     }
-                    io.largest = max(io.largest, max(cnb_scale_bits(gr), cnb_scale_bits(gi)));
                 }
             }
         }
@@ -161,7 +159,6 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
     io.xr = xr + io.row0 * pl.n; io.xi = xi + io.row0 * pl.n;
     io.yr = yr + io.row0 * pl.n; io.yi = yi + io.row0 * pl.n;
     io.tw = tw; io.chirp = chirp; io.spectrum = spectrum;
-    io.largest = 0;
     const int total = CHIRP ? 2 * pl.passes : pl.passes;
     for (int s = 0; s < total; ++s) {
         const Pass& d = pl.p[CHIRP && s >= pl.passes ? s - pl.passes : s];
@@ -176,7 +173,6 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
         }
         if (s < total - 1) __syncthreads();
     }
-    if (FINISH == TAIL && ep.head) cnb_pack_max_block(ep.head, io.largest);
 }
 
 // twiddles of every pass, packed as Pass::tw says, in double

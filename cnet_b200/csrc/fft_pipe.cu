@@ -128,7 +128,6 @@ fft1024_pipe_k(const float* __restrict__ xr, const float* __restrict__ xi, float
     __syncthreads();
 
     uint32_t phase = 0;
-    unsigned largest = 0;
     bool stored = false;
 #ifdef CNB_FFT_TIMING
     int stamp_row = 0;
@@ -216,7 +215,6 @@ fft1024_pipe_k(const float* __restrict__ xr, const float* __restrict__ xi, float
                 const float gr = cnb_gelu(re[p] * hr - im[p] * hi);
                 const float gi = cnb_gelu(re[p] * hi + im[p] * hr);
                 if (ep.gr) { ep.gr[o + e] = gr; ep.gi[o + e] = gi; }
-                largest = max(largest, max(cnb_scale_bits(gr), cnb_scale_bits(gi)));
                 if (ep.sp) {
                     cnb_split_store1(sp_re, o + e, gr);
                     cnb_split_store1(sp_im, o + e, gi);
@@ -227,10 +225,6 @@ fft1024_pipe_k(const float* __restrict__ xr, const float* __restrict__ xi, float
 #ifdef CNB_FFT_TIMING
         ++stamp_row;
 #endif
-    }
-    if (ep.head) {                                       // one atomic per warp: the warps of a CTA end at different rows
-        largest = __reduce_max_sync(0xffffffffu, largest);
-        if (t == 0) atomicMax(&ep.head->max_bits, largest);
     }
     // shared memory stays allocated until the engine has read the last row out of it
     if (t == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");

@@ -50,7 +50,6 @@ struct FftEpilogue {
     float* gi = nullptr;
     float* sp = nullptr;            // operand split of that (a split buffer with plane pitch np) or NULL
     size_t np = 0;
-    cnb_pack_head* head = nullptr;  // receives the largest component of the values, or NULL
 };
 
 }  // namespace cnb_fft

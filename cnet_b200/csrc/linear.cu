@@ -63,7 +63,7 @@ int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) {
         if (rc != CNB_OK) return rc;
         CNB_CUDA(cudaMemsetAsync(t.pack, 0, 256, st));
         const cnb::PackRequest r = twiddle_pack(t, N);
-        rc = cnb::pack(ctx, &r, 1, false, st);
+        rc = cnb::pack(ctx, &r, 1, st);
         if (rc != CNB_OK) return rc;
     }
     ctx->twiddles[key] = t;
@@ -257,7 +257,8 @@ int cnb_pack_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, in
                     void* stream) {
     CNB_CHECK_ARG(ctx && re && im && pack && rows > 0 && cols > 0, "cnb_pack_matrix: bad argument");
     const cnb::PackRequest r = pack_of(re, im, pack, rows, cols);
-    return cnb::pack(ctx, &r, 1, have_max != 0, cnb::S(stream));
+    (void) have_max;                               // the scale follows from more than the largest component
+    return cnb::pack(ctx, &r, 1, cnb::S(stream));
 }
 
 int cnb_linear_pack_ok(int B, int in, int out) {
@@ -290,7 +291,7 @@ int cnb_linear_bwd_w_packed(cnb_ctx* ctx, const void* g_pack, const void* x_pack
                                   dw_im, out, in, B, accumulate, cnb::S(stream));
 }
 
-/* the update of a weight arena, then its packed matrices: the largest components are found while the new values pass by */
+/* the update of a weight arena, then its packed matrices */
 int cnb_sgd_update_packed(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zero_grad, const cnb_pack_span* spans,
                           int nspans, void* stream) {
     CNB_CHECK_ARG(ctx && w && g && n > 0 && nspans >= 0 && (nspans == 0 || spans), "cnb_sgd_update_packed: bad argument");
@@ -301,10 +302,9 @@ int cnb_sgd_update_packed(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, 
                       "cnb_sgd_update_packed: matrix %d is not inside the arena", k);
         r.push_back(pack_of(w + s.re, w + s.im, s.pack, s.rows, s.cols));
     }
-    bool have_max = false;
-    int rc = cnb::sgd_update_max(ctx, w, g, n, lr, zero_grad, r.data(), nspans, &have_max, cnb::S(stream));
+    const int rc = cnb_sgd_update(ctx, w, g, n, lr, zero_grad, stream);
     if (rc != CNB_OK || nspans == 0) return rc;
-    return cnb::pack(ctx, r.data(), nspans, have_max, cnb::S(stream));
+    return cnb::pack(ctx, r.data(), nspans, cnb::S(stream));
 }
 
 int cnb_dft_fused_ok(int N) { return cnb::fft_supported(N) ? 1 : 0; }
@@ -317,7 +317,7 @@ int cnb_dft_hadamard_gelu_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im
                   "cnb_dft_hadamard_gelu_fwd: y planes must be a pair, and may only be left out when y_split is given");
     CNB_CHECK_ARG(B > 0 && cnb::fft_supported(N), "cnb_dft_hadamard_gelu_fwd: B=%d, N=%d is not an FFT-kernel length", B, N);
     cnb::g_last_engine = fft_engine(N);
-    return cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, y_split, nullptr, B, N, cnb::S(stream));
+    return cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, y_split, B, N, cnb::S(stream));
 }
 
 int cnb_dft_hadamard_gelu_fwd_packed(cnb_ctx* ctx, const float* x_re, const float* x_im, const float* h_re, const float* h_im,
@@ -326,9 +326,9 @@ int cnb_dft_hadamard_gelu_fwd_packed(cnb_ctx* ctx, const float* x_re, const floa
     CNB_CHECK_ARG(B > 0 && cnb::fft_supported(N), "cnb_dft_hadamard_gelu_fwd_packed: B=%d, N=%d is not an FFT-kernel length", B, N);
     cnb::g_last_engine = fft_engine(N);
     const cnb::PackRequest r = pack_of(y_re, y_im, y_pack, B, N);
-    const int rc = cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, nullptr, r.head, B, N, cnb::S(stream));
+    const int rc = cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, nullptr, B, N, cnb::S(stream));
     if (rc != CNB_OK) return rc;
-    return cnb::pack(ctx, &r, 1, true, cnb::S(stream));
+    return cnb::pack(ctx, &r, 1, cnb::S(stream));
 }
 
 int cnb_tdft_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im, float* y_re, float* y_im, int B, int N,

@@ -127,13 +127,15 @@ int cnb_linear_bwd_w_split(cnb_ctx* ctx, const float* g_split, const float* x_sp
                            float* dw_re, float* dw_im, int B, int in, int out, int accumulate, void* stream);
 /* Packed operands: what the raw-plane products above and the host facade put through the tensor cores.  A matrix is
  * scaled by one power of two that brings its largest component into [2^14, 2^15) and kept as two fp16 parts,
- * high = fp16(x) and low = fp16(x - high): 22 bits of every component down to 2^-18 of the largest, then gradually
- * fewer, an absolute error of 2^-40 of the largest at most.  A product is high.high + high.low + low.high on the
- * FP16 pipe with fp32 accumulation and takes the scales out again.  A pack is cnb_pack_bytes(rows, cols) of 256-byte
+ * high = fp16(x) and low = fp16(x - high): 22 bits of every component down to 2^-17 of the largest, then gradually
+ * fewer, an absolute error of 2^-39 of the largest at most.  A product is high.high + high.low + low.high on the
+ * FP16 pipe with fp32 accumulation and takes the scales out again.  A matrix in which the largest component of some
+ * 1 x 128 or 32 x 1 elements is less than 2^-17 of the whole's (and not zero) keeps its fp32 values in the pack, and its
+ * products run as fp32 FMAs.  A pack is cnb_pack_bytes(rows, cols) of 256-byte
  * aligned memory, its first 256 bytes zeroed once before the first use: [0, 256) the head, then as fp16 the planes
  * high re, high im, low re, low im, rows at a pitch of `cols` rounded up to 64.  Any sizes; cnb_linear_pack_ok says
- * for which a layer gains by it.  have_max: a kernel before has left the largest component in the head
- * (cnb_dft_hadamard_gelu_fwd_packed, cnb_sgd_update_packed do), otherwise a pass over the matrix finds it.  Same
+ * for which a layer gains by it.  have_max: accepted, and no longer
+ * of use: the pass over the matrix is always made.  Same
  * reference call sites as cnb_linear_fwd / _bwd_x / _bwd_w. */
 size_t cnb_pack_bytes(int rows, int cols);
 int cnb_pack_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, int cols, void* pack, int have_max,
