@@ -15,11 +15,13 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// Ordinary loads, here and below: the kernels before this one in the stream may still be writing what it reads until
+// cnb_pdl_enter returns, and a load through the read-only path (__ldg) is not held behind that.
 __device__ __forceinline__ void ldv(const float* p, float (&v)[4]) {
-    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 t = *reinterpret_cast<const float4*>(p);
     v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
 }
-__device__ __forceinline__ void ldv(const float* p, float (&v)[1]) { v[0] = __ldg(p); }
+__device__ __forceinline__ void ldv(const float* p, float (&v)[1]) { v[0] = *p; }
 
 // OT is a compile-time bound of `out` (4, 8, 10 or 16): the accumulators of the unused outputs cost
 // no registers.  W = 4: every lane works on 4 consecutive inputs with 16-byte accesses (in % 4 == 0).
@@ -30,8 +32,8 @@ __device__ __forceinline__ void ldv(const float* p, float (&v)[1]) { v[0] = __ld
 // shuffles.  X is read once.
 template <int OT, int W>
 __global__ void __launch_bounds__(512)
-skinny_fwd_k(const float* __restrict__ xr, const float* __restrict__ xi, const float* __restrict__ wr,
-             const float* __restrict__ wi, float* __restrict__ yr, float* __restrict__ yi, int B, int in, int out,
+skinny_fwd_k(const float* xr, const float* xi, const float* wr,
+             const float* wi, float* __restrict__ yr, float* __restrict__ yi, int B, int in, int out,
              int row_warps) {
     cnb_pdl_enter();
     extern __shared__ __align__(16) float sw[];          // [out][in] re, then [out][in] im
@@ -40,8 +42,8 @@ skinny_fwd_k(const float* __restrict__ xr, const float* __restrict__ xi, const f
     const int total = out * in;
     if constexpr (W == 4) {
         for (int e = threadIdx.x * 4; e < total; e += blockDim.x * 4) {
-            *reinterpret_cast<float4*>(swr + e) = __ldg(reinterpret_cast<const float4*>(wr + e));
-            *reinterpret_cast<float4*>(swi + e) = __ldg(reinterpret_cast<const float4*>(wi + e));
+            *reinterpret_cast<float4*>(swr + e) = *reinterpret_cast<const float4*>(wr + e);
+            *reinterpret_cast<float4*>(swi + e) = *reinterpret_cast<const float4*>(wi + e);
         }
     } else {
         for (int e = threadIdx.x; e < total; e += blockDim.x) { swr[e] = wr[e]; swi[e] = wi[e]; }
@@ -102,8 +104,8 @@ skinny_fwd_k(const float* __restrict__ xr, const float* __restrict__ xi, const f
 // round trips: 1 x 784 -> 10 took 13.3 us (cold) as that and 64 x 784 as much.
 template <int OT, int W, int RB>
 __global__ void __launch_bounds__(256)
-skinny_fwd_rows_k(const float* __restrict__ xr, const float* __restrict__ xi, const float* __restrict__ wr,
-                  const float* __restrict__ wi, float* __restrict__ yr, float* __restrict__ yi, int B, int in, int out) {
+skinny_fwd_rows_k(const float* xr, const float* xi, const float* wr,
+                  const float* wi, float* __restrict__ yr, float* __restrict__ yi, int B, int in, int out) {
     cnb_pdl_enter();
     __shared__ float part[8][RB * OT * 2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -160,8 +162,8 @@ skinny_fwd_rows_k(const float* __restrict__ xr, const float* __restrict__ xi, co
 // rows; G[b, :] is a broadcast read.  W is fetched once per (column group, row chunk).
 template <int OT, int W>
 __global__ void __launch_bounds__(256, (OT * W > 40 ? 1 : 2))
-skinny_bwd_x_k(const float* __restrict__ gr, const float* __restrict__ gi, const float* __restrict__ wr,
-               const float* __restrict__ wi, float* __restrict__ dr, float* __restrict__ di, int B, int in, int out,
+skinny_bwd_x_k(const float* gr, const float* gi, const float* wr,
+               const float* wi, float* __restrict__ dr, float* __restrict__ di, int B, int in, int out,
                int accumulate, int rows_per_chunk) {
     cnb_pdl_enter();
     const int i = (blockIdx.x * 256 + threadIdx.x) * W;
@@ -181,8 +183,8 @@ skinny_bwd_x_k(const float* __restrict__ gr, const float* __restrict__ gi, const
 #pragma unroll
     for (int o = 0; o < OT; ++o) {
         const bool on = o < out && r0 < r1;
-        ga[o] = on ? __ldg(gr + (size_t) r0 * out + o) : 0.f;
-        gc[o] = on ? __ldg(gi + (size_t) r0 * out + o) : 0.f;
+        ga[o] = on ? gr[(size_t) r0 * out + o] : 0.f;
+        gc[o] = on ? gi[(size_t) r0 * out + o] : 0.f;
     }
     for (int b = r0; b < r1; ++b) {
         float a_[OT], c_[OT];
@@ -191,7 +193,7 @@ skinny_bwd_x_k(const float* __restrict__ gr, const float* __restrict__ gi, const
         if (b + 1 < r1) {
 #pragma unroll
             for (int o = 0; o < OT; ++o)
-                if (o < out) { ga[o] = __ldg(gr + (size_t) (b + 1) * out + o); gc[o] = __ldg(gi + (size_t) (b + 1) * out + o); }
+                if (o < out) { ga[o] = gr[(size_t) (b + 1) * out + o]; gc[o] = gi[(size_t) (b + 1) * out + o]; }
         }
         float sr[W], si[W];
 #pragma unroll
@@ -228,8 +230,8 @@ skinny_bwd_x_k(const float* __restrict__ gr, const float* __restrict__ gi, const
 // block = 32 column groups of W columns x 8 row lanes (W = 4: 16-byte reads of X)
 template <int OT, int W>
 __global__ void __launch_bounds__(256, (OT * W > 40 ? 1 : 2))
-skinny_bwd_w_stage1_k(const float* __restrict__ gr, const float* __restrict__ gi, const float* __restrict__ xr,
-                      const float* __restrict__ xi, float* __restrict__ pr, float* __restrict__ pi, int B, int in,
+skinny_bwd_w_stage1_k(const float* gr, const float* gi, const float* xr,
+                      const float* xi, float* __restrict__ pr, float* __restrict__ pi, int B, int in,
                       int out, int rows_per_chunk) {
     cnb_pdl_enter();
     __shared__ float sr[8][32 * W + 1], si[8][32 * W + 1];
@@ -248,7 +250,7 @@ skinny_bwd_w_stage1_k(const float* __restrict__ gr, const float* __restrict__ gi
 #pragma unroll
             for (int o = 0; o < OT; ++o) {
                 if (o < out) {
-                    const float a = __ldg(gr + (size_t) b * out + o), c = __ldg(gi + (size_t) b * out + o);
+                    const float a = gr[(size_t) b * out + o], c = gi[(size_t) b * out + o];
 #pragma unroll
                     for (int k = 0; k < W; ++k) {
                         ar[o][k] += a * x[k] + c * y[k];       // (a + ic)(x - iy)
@@ -284,7 +286,7 @@ skinny_bwd_w_stage1_k(const float* __restrict__ gr, const float* __restrict__ gi
 }
 
 // stage 2: 32 outputs x 8 chunk lanes per block, fixed summation order
-__global__ void skinny_bwd_w_stage2_k(const float* __restrict__ pr, const float* __restrict__ pi, float* __restrict__ dr,
+__global__ void skinny_bwd_w_stage2_k(const float* pr, const float* pi, float* __restrict__ dr,
                                       float* __restrict__ di, int chunks, size_t n, int accumulate) {
     cnb_pdl_enter();
     __shared__ float sr[8][33], si[8][33];

@@ -99,11 +99,12 @@ def test_zero_lines_and_lone_elements(ctx):  # noqa: F811
     assert _err(tuple(p[keep] for p in y), want[keep], 1) < TOL
 
 
-@pytest.mark.parametrize("n_in,n_out", [(256, 128), (250, 37)])
-def test_net_with_rows_of_any_scale(n_in, n_out):
-    """Through Net, in a captured step: the form is chosen on the device, for each batch anew."""
+@pytest.mark.parametrize("B,n_in,n_out", [(480, 256, 128), (480, 250, 37),
+                                          (160, 250, 37), (160, 250, 10)])     # SIMT tiles, skinny kernels
+def test_net_with_rows_of_any_scale(B, n_in, n_out):
+    """Through Net, in a captured step: the form is chosen on the device, for each batch anew, and every kernel reads what
+    the kernel before it wrote for this batch."""
     import torch
-    B = 480
     dev, ora = Net(), co.OracleNet()
     sd, so = configs.build_linear(dev, n_in, n_out), configs.build_linear(ora, n_in, n_out)
     for uid, (re, im) in configs.init_weights(sd, 3).items():
