@@ -15,6 +15,8 @@ struct cnb_twiddle {
     float* re = nullptr;   // [N, N] planes, F[p,q] = N^-1/2 e^{-2 pi i pq/N}
     float* im = nullptr;
     void* pack = nullptr;  // the matrix packed (made once; head, then planes), or null when the tiles cannot take it
+    cudaEvent_t built = nullptr;           // recorded behind the kernels that make the table; null once they are known to be done
+    unsigned long long stream_id = 0;      // the stream they run on
 };
 
 // Head of a packed operand: the scale's exponent; on their way to becoming that, the largest component and the
@@ -44,6 +46,13 @@ int set_error(int code, const char* fmt, ...);
 void count_launch();
 int ensure_scratch(cnb_ctx* ctx, size_t bytes, float** out);
 extern thread_local int g_last_engine;
+
+// A table of constants from the context's cache, made by `make(stream, &table)` (arena memory and launches) at its first
+// use.  On return work on `st` may read it: its kernels ran on `st` before, or have completed.  While `st` is being
+// captured the table is made on a stream of its own, since what is captured does not run until the graph does.
+typedef int (*TableMake)(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* t);
+int table(cnb_ctx* ctx, int key, cudaStream_t st, TableMake make, cnb_twiddle* out);
+void drop_tables(cnb_ctx* ctx);
 
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 

@@ -40,6 +40,70 @@ int ensure_scratch(cnb_ctx* ctx, size_t bytes, float** out) {
     return CNB_OK;
 }
 
+// Calls on other streams than a captured one are allowed to this thread while it lives.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+static void settle(cnb_twiddle* t) {
+    if (t->built) cudaEventDestroy(t->built);
+    t->built = nullptr;
+}
+
+void drop_tables(cnb_ctx* ctx) {
+    for (auto& e : ctx->twiddles) settle(&e.second);
+    ctx->twiddles.clear();
+}
+
+int table(cnb_ctx* ctx, int key, cudaStream_t st, TableMake make, cnb_twiddle* out) {
+    auto it = ctx->twiddles.find(key);
+    if (it != ctx->twiddles.end() && !it->second.built) { *out = it->second; return CNB_OK; }
+    RelaxedCapture relaxed;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CNB_CUDA(cudaStreamIsCapturing(st, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (!captured) CNB_CUDA(cudaStreamGetId(st, &id));
+    if (it != ctx->twiddles.end()) {
+        cnb_twiddle& t = it->second;
+        const cudaError_t e = cudaEventQuery(t.built);
+        if (e == cudaErrorNotReady) {
+            cudaGetLastError();
+            // another stream, or a graph that may be launched on one: wait here, once in the table's life
+            if (captured || id != t.stream_id) {
+                CNB_CUDA(cudaEventSynchronize(t.built));
+                settle(&t);
+            }
+        } else {
+            CNB_CUDA(e);
+            settle(&t);
+        }
+        *out = t;
+        return CNB_OK;
+    }
+    cnb_twiddle t;
+    if (captured) {
+        cudaStream_t own;
+        CNB_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+        int rc = make(ctx, key, own, &t);
+        const cudaError_t e = cudaStreamSynchronize(own);
+        cudaStreamDestroy(own);
+        if (rc != CNB_OK) return rc;
+        CNB_CUDA(e);
+    } else {
+        const int rc = make(ctx, key, st, &t);
+        if (rc != CNB_OK) return rc;
+        CNB_CUDA(cudaEventCreateWithFlags(&t.built, cudaEventDisableTiming));
+        CNB_CUDA(cudaEventRecord(t.built, st));
+        t.stream_id = id;
+    }
+    ctx->twiddles[key] = t;
+    *out = t;
+    return CNB_OK;
+}
+
 }  // namespace cnb
 
 extern "C" {
@@ -95,6 +159,7 @@ int cnb_create_external(int device, void* arena, size_t arena_bytes, cnb_ctx** o
 
 int cnb_destroy(cnb_ctx* ctx) {
     if (!ctx) return CNB_OK;
+    cnb::drop_tables(ctx);
     if (ctx->owns && ctx->base) cudaFree(ctx->base);
     delete ctx;
     return CNB_OK;
@@ -116,7 +181,7 @@ int cnb_reset(cnb_ctx* ctx) {
     ctx->used = 4096;           // keep the status word and the counters
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
-    ctx->twiddles.clear();
+    cnb::drop_tables(ctx);
     return CNB_OK;
 }
 

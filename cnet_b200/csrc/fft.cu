@@ -20,6 +20,17 @@ __global__ void fft_twiddle_k(float2* __restrict__ tw, int R) {
     tw[i] = make_float2((float) c, (float) s);
 }
 
+int make_pipe_table(cnb_ctx* ctx, int, cudaStream_t st, cnb_twiddle* t) {
+    constexpr int R = 32;
+    void* p = nullptr;
+    const int rc = cnb_alloc(ctx, R * R * sizeof(float2), &p);
+    if (rc != CNB_OK) return rc;
+    t->re = static_cast<float*>(p);
+    fft_twiddle_k<<<(R * R + 255) / 256, 256, 0, st>>>(static_cast<float2*>(p), R);
+    CNB_LAUNCH_CHECK("fft_twiddle");
+    return CNB_OK;
+}
+
 bool aligned16(const void* a, const void* b, const void* c, const void* d) {
     return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
              reinterpret_cast<uintptr_t>(d)) & 15) == 0;
@@ -38,21 +49,9 @@ static int fft_dispatch(cnb_ctx* ctx, const float* xr, const float* xi, float* y
     // its inter-pass twiddle table lives in the arena; DFT matrices have positive map keys, fft_mixed's tables -N
     constexpr int key = -(1 << 20);
     cnb_twiddle t;
-    bool fresh = false;            // the table is being made by the launch just before this one
-    auto it = ctx->twiddles.find(key);
-    if (it == ctx->twiddles.end()) {
-        fresh = true;
-        void* p = nullptr;
-        int rc = cnb_alloc(ctx, (size_t) N * sizeof(float2), &p);
-        if (rc != CNB_OK) return rc;
-        t.re = static_cast<float*>(p);
-        fft_twiddle_k<<<(N + 255) / 256, 256, 0, st>>>(reinterpret_cast<float2*>(p), 32);
-        CNB_LAUNCH_CHECK("fft_twiddle");
-        ctx->twiddles[key] = t;
-    } else {
-        t = it->second;
-    }
-    return fft1024_pipe(ctx, xr, xi, yr, yi, reinterpret_cast<const float2*>(t.re), B, inverse, accumulate, ep, st, fresh);
+    const int rc = table(ctx, key, st, make_pipe_table, &t);
+    if (rc != CNB_OK) return rc;
+    return fft1024_pipe(ctx, xr, xi, yr, yi, reinterpret_cast<const float2*>(t.re), B, inverse, accumulate, ep, st);
 }
 
 int fft_run(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, int B, int N, int inverse,

@@ -330,11 +330,30 @@ void plan_batch(MixedPlan* pl, int B, int sms) {
     pl->rows = rows;
 }
 
-size_t table_entries(const MixedPlan& pl) {
+size_t twiddle_entries(const MixedPlan& pl) {
     size_t n = 0;
     for (int p = 0; p < pl.passes; ++p) if (pl.p[p].L > 1) n += (size_t) (pl.p[p].radix - 1) * pl.p[p].L;
-    if (pl.m > pl.n) n += (size_t) pl.n + pl.m;
-    return std::max<size_t>(n, 1);
+    return n;
+}
+
+// twiddles of the passes, then for the chirp form c[0..n) and the spectrum
+int make_mixed_tables(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* t) {
+    MixedPlan pl;
+    cached_plan(-key, &pl);
+    const size_t tw_entries = twiddle_entries(pl);
+    const bool chirp = pl.m > pl.n;
+    void* p = nullptr;
+    const int rc = cnb_alloc(ctx, std::max<size_t>(1, tw_entries + (chirp ? (size_t) pl.n + pl.m : 0)) * sizeof(float2), &p);
+    if (rc != CNB_OK) return rc;
+    t->re = static_cast<float*>(p);
+    float2* tab = static_cast<float2*>(p);
+    mixed_twiddle_k<<<16, 256, 0, st>>>(tab, pl);
+    CNB_LAUNCH_CHECK("mixed_twiddle");
+    if (chirp) {
+        mixed_chirp_k<<<ctx->sm_count * 4, 256, 0, st>>>(tab + tw_entries, tab + tw_entries + pl.n, pl.n, pl.m);
+        CNB_LAUNCH_CHECK("mixed_chirp");
+    }
+    return CNB_OK;
 }
 
 }  // namespace
@@ -354,24 +373,9 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
     const bool chirp = pl.m > pl.n;
     // the tables live in the arena; the map key -N keeps them apart from DFT matrices
     cnb_twiddle t;
-    auto it = ctx->twiddles.find(-N);
-    const size_t entries = table_entries(pl), tw_entries = entries - (chirp ? (size_t) pl.n + pl.m : 0);
-    if (it == ctx->twiddles.end()) {
-        void* p = nullptr;
-        int rc = cnb_alloc(ctx, entries * sizeof(float2), &p);
-        if (rc != CNB_OK) return rc;
-        t.re = static_cast<float*>(p);
-        float2* tab = static_cast<float2*>(p);
-        mixed_twiddle_k<<<16, 256, 0, st>>>(tab, pl);
-        CNB_LAUNCH_CHECK("mixed_twiddle");
-        if (chirp) {
-            mixed_chirp_k<<<ctx->sm_count * 4, 256, 0, st>>>(tab + tw_entries, tab + tw_entries + pl.n, pl.n, pl.m);
-            CNB_LAUNCH_CHECK("mixed_chirp");
-        }
-        ctx->twiddles[-N] = t;
-    } else {
-        t = it->second;
-    }
+    const int rc = table(ctx, -N, st, make_mixed_tables, &t);
+    if (rc != CNB_OK) return rc;
+    const size_t tw_entries = twiddle_entries(pl);
     const float2* tw = reinterpret_cast<const float2*>(t.re);
     const float2* ch = tw + tw_entries;
     const float2* spec = ch + pl.n;

@@ -235,7 +235,7 @@ fft1024_pipe_k(const float* __restrict__ xr, const float* __restrict__ xi, float
 namespace cnb {
 
 int fft1024_pipe(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, const float2* tw, int B,
-                 int inverse, int accumulate, const cnb_fft::FftEpilogue& ep, cudaStream_t st, bool /*fresh_table*/) {
+                 int inverse, int accumulate, const cnb_fft::FftEpilogue& ep, cudaStream_t st) {
     static bool attr_done[64] = {};                      // the attribute is per device
     if (!attr_done[ctx->device & 63]) {
         CNB_CUDA(cudaFuncSetAttribute(fft1024_pipe_k<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));

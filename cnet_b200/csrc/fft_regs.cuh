@@ -59,7 +59,7 @@ namespace cnb {
 // fresh_table: `tw` is written by the launch just before this one (the kernel reads it before it waits for its
 // predecessor, so that one launch must be fully serialised)
 int fft1024_pipe(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, const float2* tw, int B,
-                 int inverse, int accumulate, const cnb_fft::FftEpilogue& ep, cudaStream_t st, bool fresh_table);
+                 int inverse, int accumulate, const cnb_fft::FftEpilogue& ep, cudaStream_t st);
 // any length with a plan: mixed radices or the chirp form; planes of any alignment
 bool fft_mixed_supported(int N);
 int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, int B, int N, int inverse,

@@ -38,38 +38,34 @@ cnb::PackRequest twiddle_pack(const cnb_twiddle& t, int N) {
     return {t.re, t.im, N, N, (N + 7) & ~7, static_cast<char*>(t.pack) + 256, static_cast<cnb_pack_head*>(t.pack)};
 }
 
-int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) {
+int make_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* t) {
     const int N = key & (kTriKey - 1);
-    auto it = ctx->twiddles.find(key);
-    if (it != ctx->twiddles.end()) { *out = it->second; return CNB_OK; }
-    cnb_twiddle t;
     void* p = nullptr;
     int rc = cnb_alloc(ctx, (size_t) N * N * sizeof(float), &p);
     if (rc != CNB_OK) return rc;
-    t.re = static_cast<float*>(p);
+    t->re = static_cast<float*>(p);
     rc = cnb_alloc(ctx, (size_t) N * N * sizeof(float), &p);
     if (rc != CNB_OK) return rc;
-    t.im = static_cast<float*>(p);
-    twiddle_k<<<ctx->sm_count * 4, 256, 0, st>>>(t.re, t.im, N);
+    t->im = static_cast<float*>(p);
+    twiddle_k<<<ctx->sm_count * 4, 256, 0, st>>>(t->re, t->im, N);
     CNB_LAUNCH_CHECK("twiddle");
     if (key & kTriKey) {
-        tri_mask_k<<<ctx->sm_count * 4, 256, 0, st>>>(t.re, t.im, N);
+        tri_mask_k<<<ctx->sm_count * 4, 256, 0, st>>>(t->re, t->im, N);
         CNB_LAUNCH_CHECK("tri_mask");
     }
     if (cnb::cgemm_tc_shape_ok(64, N, N) && (!cnb::fft_supported(N) || (key & kTriKey))) {
         // the matrix is a constant: where the GEMM is the transform's engine, it is packed here, not by every product
         const int pitch = (N + 7) & ~7;
-        rc = cnb_alloc(ctx, 256 + 8 * (size_t) N * pitch, &t.pack);
+        rc = cnb_alloc(ctx, 256 + 8 * (size_t) N * pitch, &t->pack);
         if (rc != CNB_OK) return rc;
-        CNB_CUDA(cudaMemsetAsync(t.pack, 0, 256, st));
-        const cnb::PackRequest r = twiddle_pack(t, N);
-        rc = cnb::pack(ctx, &r, 1, st);
-        if (rc != CNB_OK) return rc;
+        CNB_CUDA(cudaMemsetAsync(t->pack, 0, 256, st));
+        const cnb::PackRequest r = twiddle_pack(*t, N);
+        return cnb::pack(ctx, &r, 1, st);
     }
-    ctx->twiddles[key] = t;
-    *out = t;
     return CNB_OK;
 }
+
+int get_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* out) { return cnb::table(ctx, key, st, make_twiddle, out); }
 
 // X F^T (conj = 0) or G conj(F) (conj = 1) with F symmetric, so F itself is the K-major operand
 int twiddle_product(cnb_ctx* ctx, const cnb_twiddle& t, const float* x_re, const float* x_im, float* y_re, float* y_im,
