@@ -223,6 +223,7 @@ int cnb_linear_fwd_split(cnb_ctx* ctx, const float* x_split, const float* w_spli
                          const float* res_im, float* y_re, float* y_im, int B, int in, int out, void* stream) {
     CNB_CHECK_ARG(ctx && x_split && w_split && y_re && y_im, "cnb_linear_fwd_split: null pointer");
     CNB_CHECK_ARG(cnb_linear_split_ok(B, in, out), "cnb_linear_fwd_split: B=%d in=%d out=%d not eligible", B, in, out);
+    CNB_CHECK_ARG((res_re == nullptr) == (res_im == nullptr), "cnb_linear_fwd_split: residual planes must be a pair");
     cnb::g_last_engine = 1;
     return cnb::cgemm_tc_presplit(ctx, split_of(x_split, B, in, 0), split_of(w_split, out, in, 0), 0, res_re, res_im, y_re, y_im,
                                   B, out, in, 0, cnb::S(stream));
@@ -266,6 +267,7 @@ int cnb_linear_pack_ok(int B, int in, int out) {
 int cnb_linear_fwd_packed(cnb_ctx* ctx, const void* x_pack, const void* w_pack, const float* res_re, const float* res_im,
                           float* y_re, float* y_im, int B, int in, int out, void* stream) {
     CNB_CHECK_ARG(ctx && x_pack && w_pack && y_re && y_im && B > 0 && in > 0 && out > 0, "cnb_linear_fwd_packed: bad argument");
+    CNB_CHECK_ARG((res_re == nullptr) == (res_im == nullptr), "cnb_linear_fwd_packed: residual planes must be a pair");
     cnb::g_last_engine = 1;
     return cnb::cgemm_tc_presplit(ctx, packed_of(x_pack, B, in, 0), packed_of(w_pack, out, in, 0), 0, res_re, res_im, y_re, y_im,
                                   B, out, in, 0, cnb::S(stream));
@@ -294,7 +296,8 @@ int cnb_sgd_update_packed(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, 
     std::vector<cnb::PackRequest> r;
     for (int k = 0; k < nspans; ++k) {
         const cnb_pack_span& s = spans[k];
-        CNB_CHECK_ARG(s.rows > 0 && s.cols > 0 && s.pack && s.re + (size_t) s.rows * s.cols <= n && s.im + (size_t) s.rows * s.cols <= n,
+        const size_t count = s.rows > 0 && s.cols > 0 ? (size_t) s.rows * s.cols : 0;
+        CNB_CHECK_ARG(count > 0 && count <= n && s.pack && s.re <= n - count && s.im <= n - count,
                       "cnb_sgd_update_packed: matrix %d is not inside the arena", k);
         r.push_back(pack_of(w + s.re, w + s.im, s.pack, s.rows, s.cols));
     }
