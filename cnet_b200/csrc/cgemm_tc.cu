@@ -1742,7 +1742,7 @@ int cgemm_tc_run(cnb_ctx* ctx, const float* a_re, const float* a_im, int a_trans
                  float* d_im, int M, int N, int K, int accumulate, cudaStream_t st, const PackRequest* b_packed) {
     float* ws = nullptr;
     const size_t na = operand_bytes(M, K, a_trans), nb = b_packed ? 0 : operand_bytes(N, K, b_trans);
-    int rc = ensure_scratch(ctx, na + nb, &ws);
+    int rc = ensure_scratch(ctx, na + nb, false, st, &ws);
     if (rc != CNB_OK) return rc;
     cnb_pack_head* heads = reinterpret_cast<cnb_pack_head*>(ctx->d_status + 768);
     PackRequest r[2];

@@ -410,7 +410,7 @@ int skinny_bwd_w(cnb_ctx* ctx, const float* gr, const float* gi, const float* xr
     chunks = (B + rows - 1) / rows;
     float* ws = nullptr;
     size_t n = (size_t) out * in;
-    int rc = ensure_scratch(ctx, (size_t) chunks * n * 2 * sizeof(float), &ws);
+    int rc = ensure_scratch(ctx, (size_t) chunks * n * 2 * sizeof(float), true, nullptr, &ws);
     if (rc != CNB_OK) return rc;
     float* pr = ws;
     float* pi = ws + (size_t) chunks * n;

@@ -33,8 +33,11 @@ struct cnb_ctx {
     int* d_status = nullptr;          // device error word (bounded waits report here)
     int* d_counters = nullptr;        // 8 sets of 64 "CTAs done" counters, zero between launches
     unsigned counter_set = 0;
-    float* scratch = nullptr;         // column-reduction partials and GEMM operand staging
+    // Column-reduction partials and packed operands of raw products: the last bytes of the arena, so that growing it
+    // takes in what it had.
+    float* scratch = nullptr;
     size_t scratch_bytes = 0;
+    size_t scratch_kept = 0;          // of them, what no allocation may take back
     std::map<int, cnb_twiddle> twiddles;
     int gemm_cta_limit = 0;           // > 0: the tensor-core GEMM uses at most this many CTAs (SMs)
     bool force_dft_gemm = false;      // FourierTrans as a GEMM even where the FFT kernel applies
@@ -44,7 +47,9 @@ namespace cnb {
 
 int set_error(int code, const char* fmt, ...);
 void count_launch();
-int ensure_scratch(cnb_ctx* ctx, size_t bytes, float** out);
+// keep: the caller has no way of doing without.  What packed operands alone asked for is given back to an allocation that
+// finds no other room; their products have the SIMT tiles.
+int ensure_scratch(cnb_ctx* ctx, size_t bytes, bool keep, cudaStream_t st, float** out);
 extern thread_local int g_last_engine;
 
 // A table of constants from the context's cache, made by `make(stream, &table)` (arena memory and launches) at its first

@@ -1,4 +1,5 @@
 // Context, device arena, copies and error reporting of the C ABI.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -27,14 +28,27 @@ bool pdl_enabled() {
     return on;
 }
 
-int ensure_scratch(cnb_ctx* ctx, size_t bytes, float** out) {
+static size_t arena_end(const cnb_ctx* ctx) { return ctx->size & ~size_t(255); }
+
+static int scratch_size(cnb_ctx* ctx, size_t bytes) {
+    if (ctx->used + bytes > arena_end(ctx))
+        return set_error(CNB_ERR_ARENA, "arena exhausted: %zu used + %zu of scratch > %zu", ctx->used, bytes, ctx->size);
+    ctx->scratch_bytes = bytes;
+    ctx->scratch = reinterpret_cast<float*>(ctx->base + arena_end(ctx) - bytes);
+    return CNB_OK;
+}
+
+int ensure_scratch(cnb_ctx* ctx, size_t bytes, bool keep, cudaStream_t st, float** out) {
+    bytes = (std::max(bytes, size_t(8) << 20) + 255) & ~size_t(255);
     if (bytes > ctx->scratch_bytes) {
-        size_t want = bytes < (8u << 20) ? (8u << 20) : bytes;
-        void* p = nullptr;
-        int rc = cnb_alloc(ctx, want, &p);
+        const int rc = scratch_size(ctx, bytes);
         if (rc != CNB_OK) return rc;
-        ctx->scratch = static_cast<float*>(p);
-        ctx->scratch_bytes = want;
+    }
+    if (bytes > ctx->scratch_kept) {
+        // a captured launch comes back to the scratch whenever its graph runs
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (!keep && cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+        if (keep || capture != cudaStreamCaptureStatusNone) ctx->scratch_kept = bytes;
     }
     *out = ctx->scratch;
     return CNB_OK;
@@ -168,9 +182,15 @@ int cnb_destroy(cnb_ctx* ctx) {
 int cnb_alloc(cnb_ctx* ctx, size_t bytes, void** out) {
     CNB_CHECK_ARG(ctx && out, "cnb_alloc: null argument");
     size_t need = (bytes + 255) & ~size_t(255);
-    if (ctx->used + need > ctx->size)
-        return cnb::set_error(CNB_ERR_ARENA, "arena exhausted: %zu used + %zu requested > %zu", ctx->used, need,
-                              ctx->size);
+    const size_t end = cnb::arena_end(ctx);
+    if (ctx->used + need > end - ctx->scratch_bytes && ctx->used + need <= end - ctx->scratch_kept) {
+        // The scratch gives way, once no kernel works on it any more.  (Not while a stream is captured: that cannot wait.)
+        if (cudaDeviceSynchronize() == cudaSuccess) cnb::scratch_size(ctx, ctx->scratch_kept);
+        else cudaGetLastError();
+    }
+    if (ctx->used + need > end - ctx->scratch_bytes)
+        return cnb::set_error(CNB_ERR_ARENA, "arena exhausted: %zu used + %zu requested > %zu", ctx->used + ctx->scratch_bytes,
+                              need, ctx->size);
     *out = ctx->base + ctx->used;
     ctx->used += need;
     return CNB_OK;
@@ -180,12 +200,12 @@ int cnb_reset(cnb_ctx* ctx) {
     CNB_CHECK_ARG(ctx, "cnb_reset: null context");
     ctx->used = 4096;           // keep the status word and the counters
     ctx->scratch = nullptr;
-    ctx->scratch_bytes = 0;
+    ctx->scratch_bytes = ctx->scratch_kept = 0;
     cnb::drop_tables(ctx);
     return CNB_OK;
 }
 
-size_t cnb_arena_used(const cnb_ctx* ctx) { return ctx ? ctx->used : 0; }
+size_t cnb_arena_used(const cnb_ctx* ctx) { return ctx ? ctx->used + ctx->scratch_bytes : 0; }
 size_t cnb_arena_size(const cnb_ctx* ctx) { return ctx ? ctx->size : 0; }
 
 int cnb_device_info(int device, int* sm_count, int* cc_major, int* cc_minor, size_t* total_mem) {

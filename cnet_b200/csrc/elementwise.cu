@@ -443,7 +443,7 @@ int colreduce_launch(cnb_ctx* ctx, int mode, const float* gr, const float* gi, c
     int rows = (B + chunks - 1) / chunks;
     chunks = (B + rows - 1) / rows;
     float* part = nullptr;
-    int rc = cnb::ensure_scratch(ctx, (size_t) chunks * N * 2 * sizeof(float), &part);
+    int rc = cnb::ensure_scratch(ctx, (size_t) chunks * N * 2 * sizeof(float), true, nullptr, &part);
     if (rc != CNB_OK) return rc;
     float* pr = part;
     float* pi = part + (size_t) chunks * N;

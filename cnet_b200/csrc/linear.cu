@@ -366,7 +366,7 @@ int cnb_set_dft_engine(cnb_ctx* ctx, int force_gemm) {
 int cnb_reserve_scratch(cnb_ctx* ctx, size_t bytes) {
     CNB_CHECK_ARG(ctx, "cnb_reserve_scratch: null context");
     float* p = nullptr;
-    return cnb::ensure_scratch(ctx, bytes, &p);
+    return cnb::ensure_scratch(ctx, bytes, true, nullptr, &p);
 }
 
 }  // extern "C"

@@ -580,12 +580,14 @@ bool CNet::planFusion() {
 	return true;
 }
 
-size_t CNet::scratchBytes(int B) const {
+// products: with room for the packed operands of raw products, which can do without (they run as fp32 FMAs then)
+size_t CNet::scratchBytes(int B, bool products) const {
 	size_t scratch = 8u << 20;
 	for (auto f : func_list_) {
 		if (Linear* l = dynamic_cast<Linear*>(f))
-			scratch = std::max(scratch, cnb_linear_workspace(B, l->firstInputLength(), l->outSize()));
-		if (dynamic_cast<FourierTrans*>(f) || dynamic_cast<TriangFourier*>(f))
+			if (products || l->outSize() <= 16)
+				scratch = std::max(scratch, cnb_linear_workspace(B, l->firstInputLength(), l->outSize()));
+		if (products && (dynamic_cast<FourierTrans*>(f) || dynamic_cast<TriangFourier*>(f)))
 			scratch = std::max(scratch, cnb_linear_workspace(B, f->in_size_, f->in_size_));
 		if (f->type_ == isHadamard) scratch = std::max(scratch, (size_t) 128 * f->out_size_ * 2 * sizeof(float));
 	}
@@ -593,14 +595,12 @@ size_t CNet::scratchBytes(int B) const {
 }
 
 size_t CNet::requiredArenaBytes(int B) const {
-	size_t floats = 0, extra = 0, dft = 0;
+	size_t floats = 0, extra = 0;
 	for (auto f : func_list_) {
 		bool weight = dynamic_cast<CInput*>(f) && f != func_list_.front();
 		if (weight) floats += 4 * pad64(f->out_size_);
 		else floats += 4 * pad64((size_t) B * f->out_size_);
 		if (CEmbedding* e = dynamic_cast<CEmbedding*>(f)) floats += 4 * pad64((size_t) e->inSize());
-		if ((dynamic_cast<FourierTrans*>(f) && !cnb_dft_fused_ok((int) f->in_size_)) || dynamic_cast<TriangFourier*>(f))     // twiddle planes + their pack
-			dft += (size_t) 2 * f->in_size_ * f->in_size_ * 4 + cnb_pack_bytes(f->in_size_, f->in_size_) + 1024;
 		extra += f->extraBytes(B) + 256;
 	}
 	size_t gs = 0;
@@ -608,20 +608,28 @@ size_t CNet::requiredArenaBytes(int B) const {
 		if (Linear* l = dynamic_cast<Linear*>(f))
 			if (cnb_linear_pack_ok(B, l->firstInputLength(), l->outSize()))
 				gs = std::max(gs, cnb_pack_bytes(B, l->outSize()));
-	size_t staging = 0;                                // input pipeline: one staged batch + labels
+	return floats * sizeof(float) + extra + gs + laterBytes(B) + scratchBytes(B) + (16u << 20);
+}
+
+// What is taken from the arena after allocateOnGpu: the Adam momentum planes on the first adamUpdate, the matrices of
+// transforms that run as products at their first use, the input pipeline's staged batch.
+size_t CNet::laterBytes(int B) const {
+	size_t later = 0;
+	for (auto f : func_list_) {
+		bool weight = dynamic_cast<CInput*>(f) && f != func_list_.front();
+		if (weight) later += 2 * pad64(f->out_size_) * sizeof(float);
+		if (CEmbedding* e = dynamic_cast<CEmbedding*>(f)) later += 2 * pad64((size_t) e->inSize()) * sizeof(float);
+		if ((dynamic_cast<FourierTrans*>(f) && !cnb_dft_fused_ok((int) f->in_size_)) || dynamic_cast<TriangFourier*>(f))     // twiddle planes + their pack
+			later += (size_t) 2 * f->in_size_ * f->in_size_ * 4 + cnb_pack_bytes(f->in_size_, f->in_size_) + 1024;
+	}
+	size_t staging = 0;                                // one staged batch + labels
 	if (!func_list_.empty()) {
 		CFunc* f0 = func_list_.front();
 		if (CEmbedding* em = dynamic_cast<CEmbedding*>(f0)) staging = (size_t) B * em->noOutTokens() * 4;
 		else staging = 2 * (size_t) B * f0->out_size_ * 4;
 		staging += (size_t) B * 4 + 1024;
 	}
-	size_t momentum = 0;                               // Adam momentum planes (allocated on first adamUpdate)
-	for (auto f : func_list_) {
-		bool weight = dynamic_cast<CInput*>(f) && f != func_list_.front();
-		if (weight) momentum += 2 * pad64(f->out_size_) * sizeof(float);
-		if (CEmbedding* e = dynamic_cast<CEmbedding*>(f)) momentum += 2 * pad64((size_t) e->inSize()) * sizeof(float);
-	}
-	return floats * sizeof(float) + extra + dft + gs + staging + momentum + scratchBytes(B) + (16u << 20);
+	return later + staging;
 }
 
 bool CNet::allocateOnGpu(int B) {
@@ -687,7 +695,7 @@ bool CNet::allocateOnGpu(int B) {
 			side_stream_ = st; ev_side_fork_ = e0; ev_side_join_ = e1;
 		}
 	}
-	if ((rc = cnb_reserve_scratch(ctx_, scratchBytes(B))) != CNB_OK) { fail(rc, "scratch"); return false; }
+	if ((rc = cnb_reserve_scratch(ctx_, scratchBytes(B, false))) != CNB_OK) { fail(rc, "scratch"); return false; }
 
 	// 1. weights: one block of value planes and one block of dz* planes with the same layout,
 	//    in backward order (reverse insertion), so gradient buckets complete front to back.
@@ -790,6 +798,12 @@ bool CNet::allocateOnGpu(int B) {
 			}
 		}
 	}
+	// An arena that was sized by hand may have no room for packed operands beside what is taken later: the layer then
+	// runs on its raw planes.
+	auto room = [&] {
+		const size_t taken = cnb_arena_used(ctx_) + laterBytes(B) + (1u << 20);
+		return cnb_arena_size(ctx_) > taken ? cnb_arena_size(ctx_) - taken : 0;
+	};
 	for (auto f : func_list_) {
 		if (Linear* l = dynamic_cast<Linear*>(f)) {
 			if (l->fused_residual_) {
@@ -799,6 +813,12 @@ bool CNet::allocateOnGpu(int B) {
 			}
 		}
 		size_t eb = f->extraBytes(B);
+		if (Linear* l = dynamic_cast<Linear*>(f)) {
+			size_t gs = 0;                              // the packed gradient is one for all layers, as large as the largest
+			for (auto q : func_list_)
+				if (Linear* o = dynamic_cast<Linear*>(q)) if (o == l || o->x_pack_) gs = std::max(gs, cnb_pack_bytes(B, o->outSize()));
+			if (eb && eb + gs + 512 > room()) eb = 0;
+		}
 		if (eb) {
 			if ((rc = cnb_alloc(ctx_, eb, &p)) != CNB_OK) { fail(rc, f->getName()); return false; }
 			f->bindExtra(static_cast<char*>(p), B);
@@ -815,6 +835,7 @@ bool CNet::allocateOnGpu(int B) {
 			cnb_memset0(ctx_, g_pack_, 256, stream_);
 		}
 	}
+	if (scratchBytes(B) <= room() + scratchBytes(B, false)) cnb_reserve_scratch(ctx_, scratchBytes(B));
 	// 3. upload the host copies of the weights
 	for (auto f : inputs_) {
 		if (f == main_in_ && !dynamic_cast<CEmbedding*>(f)) continue;
