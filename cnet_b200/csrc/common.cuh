@@ -126,9 +126,9 @@ bool fft_supported(int N);
 int fft_run(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, int B, int N, int inverse,
             int accumulate, cudaStream_t st);
 // Forward FFT whose epilogue also applies Hadamard(h) -> CGelu: u = FFT(x) -> (ur, ui); y = gelu(u o h) ->
-// (yr, yi) and, when sp != NULL, the operand split of y.
+// (yr, yi) and, when sp != NULL, the operand split of y; u o h -> (ar, ai) where these are given (not at N = 1024).
 int fft_hadamard_gelu(cnb_ctx* ctx, const float* xr, const float* xi, const float* hr, const float* hi, float* ur,
-                      float* ui, float* yr, float* yi, float* sp, int B, int N, cudaStream_t st);
+                      float* ui, float* ar, float* ai, float* yr, float* yi, float* sp, int B, int N, cudaStream_t st);
 
 }  // namespace cnb
 

@@ -60,8 +60,9 @@ int fft_run(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi
 }
 
 int fft_hadamard_gelu(cnb_ctx* ctx, const float* xr, const float* xi, const float* hr, const float* hi, float* ur,
-                      float* ui, float* yr, float* yi, float* sp, int B, int N, cudaStream_t st) {
+                      float* ui, float* ar, float* ai, float* yr, float* yi, float* sp, int B, int N, cudaStream_t st) {
     FftEpilogue ep;
+    ep.ar = ar; ep.ai = ai;
     ep.hr = hr; ep.hi = hi; ep.gr = yr; ep.gi = yi; ep.sp = sp;
     ep.np = ((size_t) B * N + 63) & ~size_t(63);
     return fft_dispatch(ctx, xr, xi, ur, ui, B, N, 0, 0, ep, st);

@@ -133,8 +133,10 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
                 io.yi[g] = u.y;
                 if (FINISH == TAIL) {
                     const float hr = __ldg(ep.hr + e), hi = __ldg(ep.hi + e);
-                    const float gr = cnb_gelu(u.x * hr - u.y * hi), gi = cnb_gelu(u.x * hi + u.y * hr);
+                    const float ar = u.x * hr - u.y * hi, ai = u.x * hi + u.y * hr;
+                    const float gr = cnb_gelu(ar), gi = cnb_gelu(ai);
                     const size_t at = (io.row0 + row) * (size_t) pl.n + e;
+                    if (ep.ar) { ep.ar[at] = ar; ep.ai[at] = ai; }
                     if (ep.gr) { ep.gr[at] = gr; ep.gi[at] = gi; }
                     if (ep.sp) {
                         cnb_split_store1(cnb_split_component(ep.sp, ep.np, 0), at, gr);

@@ -50,14 +50,14 @@ struct FftEpilogue {
     float* gi = nullptr;
     float* sp = nullptr;            // operand split of that (a split buffer with plane pitch np) or NULL
     size_t np = 0;
+    float* ar = nullptr;            // u o h planes [B, N], or NULL (fft1024_pipe does not store them)
+    float* ai = nullptr;
 };
 
 }  // namespace cnb_fft
 
 namespace cnb {
 // N = 1024: persistent kernel fed and drained by bulk copies
-// fresh_table: `tw` is written by the launch just before this one (the kernel reads it before it waits for its
-// predecessor, so that one launch must be fully serialised)
 int fft1024_pipe(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* yi, const float2* tw, int B,
                  int inverse, int accumulate, const cnb_fft::FftEpilogue& ep, cudaStream_t st);
 // any length with a plan: mixed radices or the chirp form; planes of any alignment

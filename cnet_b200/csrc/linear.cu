@@ -316,17 +316,28 @@ int cnb_dft_hadamard_gelu_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im
                   "cnb_dft_hadamard_gelu_fwd: y planes must be a pair, and may only be left out when y_split is given");
     CNB_CHECK_ARG(B > 0 && cnb::fft_supported(N), "cnb_dft_hadamard_gelu_fwd: B=%d, N=%d is not an FFT-kernel length", B, N);
     cnb::g_last_engine = fft_engine(N);
-    return cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, y_split, B, N, cnb::S(stream));
+    return cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, nullptr, nullptr, y_re, y_im, y_split, B, N, cnb::S(stream));
 }
 
 int cnb_dft_hadamard_gelu_fwd_packed(cnb_ctx* ctx, const float* x_re, const float* x_im, const float* h_re, const float* h_im,
                                      float* u_re, float* u_im, float* y_re, float* y_im, void* y_pack, int B, int N, void* stream) {
-    CNB_CHECK_ARG(ctx && x_re && x_im && h_re && h_im && u_re && u_im && y_re && y_im && y_pack, "cnb_dft_hadamard_gelu_fwd_packed: null pointer");
-    CNB_CHECK_ARG(B > 0 && cnb::fft_supported(N), "cnb_dft_hadamard_gelu_fwd_packed: B=%d, N=%d is not an FFT-kernel length", B, N);
+    CNB_CHECK_ARG(y_pack, "cnb_dft_hadamard_gelu_fwd_packed: null pointer");
+    return cnb_dft_hadamard_gelu_fwd_keep(ctx, x_re, x_im, h_re, h_im, u_re, u_im, nullptr, nullptr, y_re, y_im, y_pack, B, N, stream);
+}
+
+int cnb_dft_keeps_product(int N) { return N != 1024 && cnb::fft_supported(N) ? 1 : 0; }
+
+int cnb_dft_hadamard_gelu_fwd_keep(cnb_ctx* ctx, const float* x_re, const float* x_im, const float* h_re, const float* h_im,
+                                   float* u_re, float* u_im, float* a_re, float* a_im, float* y_re, float* y_im, void* y_pack, int B,
+                                   int N, void* stream) {
+    CNB_CHECK_ARG(ctx && x_re && x_im && h_re && h_im && u_re && u_im && y_re && y_im, "cnb_dft_hadamard_gelu_fwd_keep: null pointer");
+    CNB_CHECK_ARG((a_re == nullptr) == (a_im == nullptr), "cnb_dft_hadamard_gelu_fwd_keep: product planes must be a pair");
+    CNB_CHECK_ARG(B > 0 && cnb::fft_supported(N), "cnb_dft_hadamard_gelu_fwd_keep: B=%d, N=%d is not an FFT-kernel length", B, N);
+    CNB_CHECK_ARG(!a_re || cnb_dft_keeps_product(N), "cnb_dft_hadamard_gelu_fwd_keep: the kernel of N=%d does not store the product", N);
     cnb::g_last_engine = fft_engine(N);
+    const int rc = cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, a_re, a_im, y_re, y_im, nullptr, B, N, cnb::S(stream));
+    if (rc != CNB_OK || !y_pack) return rc;
     const cnb::PackRequest r = pack_of(y_re, y_im, y_pack, B, N);
-    const int rc = cnb::fft_hadamard_gelu(ctx, x_re, x_im, h_re, h_im, u_re, u_im, y_re, y_im, nullptr, B, N, cnb::S(stream));
-    if (rc != CNB_OK) return rc;
     return cnb::pack(ctx, &r, 1, cnb::S(stream));
 }
 

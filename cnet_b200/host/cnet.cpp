@@ -149,12 +149,9 @@ void FourierTrans::forward() {
 	if (fused_hg_) {
 		const Vars& h = fused_hg_->previous(1)->output();
 		Vars& y = fused_hg_->fused_gelu_->out_;
-		if (void* pack = fused_hg_->consumerPack())
-			check(cnb_dft_hadamard_gelu_fwd_packed(ctx(), x.real_, x.imag_, h.real_, h.imag_, out_.real_, out_.imag_, y.real_,
-					y.imag_, pack, batch(), in_size_, stream()));
-		else
-			check(cnb_dft_hadamard_gelu_fwd(ctx(), x.real_, x.imag_, h.real_, h.imag_, out_.real_, out_.imag_, y.real_, y.imag_,
-					nullptr, batch(), in_size_, stream()));
+		Vars& a = fused_hg_->out_;                  // no planes where the product is not stored
+		check(cnb_dft_hadamard_gelu_fwd_keep(ctx(), x.real_, x.imag_, h.real_, h.imag_, out_.real_, out_.imag_, a.real_, a.imag_,
+				y.real_, y.imag_, fused_hg_->consumerPack(), batch(), in_size_, stream()));
 		return;
 	}
 	check(cnb_dft_fwd(ctx(), x.real_, x.imag_, out_.real_, out_.imag_, batch(), in_size_, stream()));
@@ -199,7 +196,8 @@ void Hadamard::backward() {
 	int acc_u = accumulate_into(pu), acc_v = accumulate_into(pv);
 	if (fused_gelu_) {
 		const Vars& g = fused_gelu_->out_;
-		check(cnb_hadamard_gelu_bwd(ctx(), g.dz_star_real_, g.dz_star_imag_, out_.real_, out_.imag_, pu->out_.real_,
+		check(cnb_hadamard_gelu_bwd(ctx(), g.dz_star_real_, g.dz_star_imag_, in_fft_epilogue_ ? nullptr : out_.real_,
+				in_fft_epilogue_ ? nullptr : out_.imag_, pu->out_.real_,
 				pu->out_.imag_, pv->out_.real_, pv->out_.imag_, pu->out_.dz_star_real_, pu->out_.dz_star_imag_, acc_u,
 				pv->out_.dz_star_real_, pv->out_.dz_star_imag_, acc_v, batch(), out_size_, stream()));
 		return;
@@ -761,8 +759,10 @@ bool CNet::allocateOnGpu(int B) {
 		bool alias = false;
 		if (Linear* l = dynamic_cast<Linear*>(f)) alias = l->fused_residual_ != nullptr;
 		if (alias) continue;                    // bound to the Residual's tensors below
+		// Inside a FourierTrans, a = u o h is recomputed in the backward; it is stored for those who read it back, except
+		// by the kernel of 1024 points and at 256 and 4096, where it has never been.
 		if (Hadamard* hd = dynamic_cast<Hadamard*>(f))
-			if (hd->in_fft_epilogue_) continue;         // a = u o h is never stored (recomputed in the backward)
+			if (hd->in_fft_epilogue_ && (!cnb_dft_keeps_product(f->out_size_) || f->out_size_ == 256 || f->out_size_ == 4096)) continue;
 		bool need_grad = !(dynamic_cast<Hadamard*>(f) && static_cast<Hadamard*>(f)->fused_gelu_);
 		size_t planes = need_grad ? 4 : 2;
 		if ((rc = cnb_alloc(ctx_, planes * n * sizeof(float), &p)) != CNB_OK) { fail(rc, f->getName()); return false; }

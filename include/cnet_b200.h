@@ -182,6 +182,12 @@ int cnb_dft_hadamard_gelu_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im
 /* The same with y stored and packed for the products of the Linear that follows (a pack of [B, N]). */
 int cnb_dft_hadamard_gelu_fwd_packed(cnb_ctx* ctx, const float* x_re, const float* x_im, const float* h_re, const float* h_im,
                                      float* u_re, float* u_im, float* y_re, float* y_im, void* y_pack, int B, int N, void* stream);
+/* And with the Hadamard product a = u o h stored as well (a_re = a_im = NULL: not), at the lengths that
+ * cnb_dft_keeps_product names; y_pack may be NULL. */
+int cnb_dft_keeps_product(int N);
+int cnb_dft_hadamard_gelu_fwd_keep(cnb_ctx* ctx, const float* x_re, const float* x_im, const float* h_re, const float* h_im,
+                                   float* u_re, float* u_im, float* a_re, float* a_im, float* y_re, float* y_im, void* y_pack,
+                                   int B, int N, void* stream);
 /* TriangFourier: Y[b,p] = N^-1/2 sum_{q <= p} X[b,q] e^{-2 pi i pq/N} and its backward
  * dX*[b,q] (+)= N^-1/2 sum_{p >= q} G*[b,p] e^{+2 pi i pq/N}: the complex GEMM against the
  * lower-triangular twiddle matrix.  Replaces TrianFourierGpu::gpu_T_fft_forward / _backward
