@@ -74,7 +74,7 @@ template <int G, int E, int VEC> struct Tile {
 
     __device__ __forceinline__ Tile(int rows, int n_, int parts) : n(n_) {
         if constexpr (G <= 32) {
-            row = (int) ((blockIdx.x * (unsigned) blockDim.x + threadIdx.x) / G);
+            row = (int) (blockIdx.x * (blockDim.x / G) + threadIdx.x / G);       // not of a product that passes 2^32
             t0 = threadIdx.x % G;
         } else {
             row = (int) (blockIdx.x / (unsigned) parts);
@@ -294,9 +294,9 @@ bool vec_ok(int n, std::initializer_list<const void*> planes) {
     cnb::launch(NAME<G, E, V>, dim3((unsigned) (CTAS)), dim3(cta_threads(G)), 0, st, PARTS, __VA_ARGS__)
 #define CNB_ROWS_V(NAME, V, rows, n, ...)                                                                                \
     do {                                                                                                                 \
-        if ((n) <= 32) CNB_ROWS_GO(NAME, 8, 4, V, ((rows) + 31) / 32, 1, __VA_ARGS__);                                   \
-        else if ((n) <= 128) CNB_ROWS_GO(NAME, 32, 4, V, ((rows) + 7) / 8, 1, __VA_ARGS__);                              \
-        else if ((n) <= 512) CNB_ROWS_GO(NAME, 32, 16, V, ((rows) + 7) / 8, 1, __VA_ARGS__);                             \
+        if ((n) <= 32) CNB_ROWS_GO(NAME, 8, 4, V, ((size_t) (rows) + 31) / 32, 1, __VA_ARGS__);                          \
+        else if ((n) <= 128) CNB_ROWS_GO(NAME, 32, 4, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                     \
+        else if ((n) <= 512) CNB_ROWS_GO(NAME, 32, 16, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                    \
         else if ((n) <= 2048) CNB_ROWS_GO(NAME, 128, 16, V, rows, 1, __VA_ARGS__);                                       \
         else CNB_ROWS_GO(NAME, 512, 16, V, (size_t) (rows) * parts, parts, __VA_ARGS__);                                 \
     } while (0)
