@@ -44,9 +44,11 @@ class Context:
         return self.torch.cuda.current_stream().cuda_stream
 
     def _like(self, x):
-        """A fresh pair of planes of the shape of x's (cheaper than naming the shape)."""
-        like = self.torch.empty_like
-        return like(x[0]), like(x[1])
+        """A fresh pair of planes of the shape of x's, contiguous float32 as the kernels write them, whatever the strides
+        and type of x (cheaper than naming the shape)."""
+        like, t = self.torch.empty_like, self.torch
+        return (like(x[0], dtype=t.float32, memory_format=t.contiguous_format),
+                like(x[0], dtype=t.float32, memory_format=t.contiguous_format))
 
     def _new(self, *shape):
         return (self.torch.empty(*shape, dtype=self.torch.float32, device="cuda"),
