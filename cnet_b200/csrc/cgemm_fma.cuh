@@ -1,4 +1,4 @@
-// One 64 x 64 tile of a complex product in fp32 FMAs: 256 threads with a 4 x 4 block of complex accumulators each, k-slabs
+// One 64 x 64 tile of a complex product of packed operands in fp32 FMAs (cgemm_tc.cu): 256 threads with a 4 x 4 block of complex accumulators each, k-slabs
 // of 16 in shared memory, the next slab on its way while one is worked on.  The terms of an element are added in the
 // order of k.
 #pragma once

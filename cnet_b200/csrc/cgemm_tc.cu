@@ -1493,7 +1493,9 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
         const bool full_wave = !accumulate && tiles <= sms && (long) tiles * 100 >= (long) sms * 85 && k_blocks <= blocks(256);
         const bool whole_tiles = (tiles >= all * 4 && sm_limit <= 0 && k_blocks <= blocks(256)) || full_wave;
         const bool lead_whole = !whole_tiles && tiles > sms && k_blocks <= blocks(256);
-        long ctas = std::min<long>(sms, std::max<long>(1, total / min_units));
+        // min_units is about splitting tiles: whole ones are dealt to as many CTAs as there are.  (With a short K
+        // total / min_units alone put 16 tiles of 2 blocks on 8 CTAs: 2000 x 50 x 50 36 -> 23 us, 777 x 1001 x 60 36 -> 23.)
+        long ctas = std::min<long>(sms, std::max<long>(tiles, total / min_units));
         if (whole_tiles) ctas = tiles;                        // many tiles: whole tiles, no atomics
         long upc = (total + ctas - 1) / ctas;
         if (whole_tiles) upc = k_blocks;
@@ -1580,6 +1582,9 @@ bool cgemm_tc_shape_ok(int M, int N, int K) {
     if (split_sizes(M, N, K)) return true;
     // Other sizes leave more of the 128 x 128 tiles empty: from about two million complex multiplications on packing
     // and tiles together take less than the fp32 SIMT tiles (777 x 1001 x 1333: 330 against 45 us), below it they do not.
+    // A short K leaves little to gain on either: 2000 x 50 takes 13 us in FMAs and 23 in tiles at K = 60, 20 and 18 at
+    // K = 100; with more 64 x 64 tiles than SMs the FMAs need another wave (1000 x 1000 x 60: 23 and 20).
+    if (K < 96 && (long) ((M + 63) / 64) * ((N + 63) / 64) <= 148) return false;
     return K >= 48 && (double) M * N * K >= (double) (1 << 21);
 }
 
@@ -1770,10 +1775,10 @@ int split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float
 
 }  // namespace cnb
 
-extern "C" int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8) {
+static int schedule_of(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int bk, int* out8) {
     if (!out8 || M <= 0 || N <= 0 || K <= 0 || sm_count <= 0)
         return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_schedule: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
-    const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<SPLIT>::BK);
+    const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, bk);
     out8[0] = q.pair ? 1 : 0;
     out8[1] = (int) (q.pair ? 2 * q.ctas : q.ctas);      // CTAs of the launch
     out8[2] = q.cluster * (q.pair ? 2 : 1);              // CTAs per cluster (1: no cluster)
@@ -1783,4 +1788,12 @@ extern "C" int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_cou
     out8[6] = q.splits_tiles ? 1 : 0;
     out8[7] = q.clear_from_row;
     return CNB_OK;
+}
+
+extern "C" int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8) {
+    return schedule_of(M, N, K, accumulate, sm_count, sm_limit, FormCfg<SPLIT>::BK, out8);
+}
+
+extern "C" int cnb_gemm_schedule_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8) {
+    return schedule_of(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK, out8);
 }
