@@ -1178,13 +1178,16 @@ __global__ void split_k(const float* __restrict__ s0, const float* __restrict__ 
 //
 // That must not cost what fp32's exponent range gave: rows of another scale than their neighbours keep their own
 // relative precision in the forward product and dX*, columns in dW*.  So the first pass also finds the largest component
-// of every group of 1 x 128 and of 32 x 1 elements, and a matrix in which one of these (not all zero) lies below 2^-17 of
-// the largest is stored as it is, as fp32 planes in the same bytes, and multiplied in fp32 FMAs.
+// of every group of 1 x 128 and of 32 x 1 elements (down to about half of that where the sizes are no multiples: a remainder of
+// a few elements would be small by chance, which the values of a CGelu often are), and a matrix in which one of these (not
+// all zero) lies below 2^-17 of the largest is stored as it is, as fp32 planes in the same bytes, and multiplied in fp32
+// FMAs.
 struct PackJob {
     const float* re; const float* im;
     __half* dst;                       // four planes of rows * pitch: high re, high im, low re, low im (or two of float)
     cnb_pack_head* head;               // max_bits, low_bits and ticket are zero between uses
     int rows, cols, pitch, blocks, max_blocks;
+    int tiles_x, tiles_y;              // groups of the first pass; the first rows % tiles_y of them have a row more, likewise columns
 };
 template <int N> struct PackJobs { PackJob j[N]; };
 
@@ -1202,7 +1205,7 @@ __device__ __forceinline__ int pack_exponent(unsigned max_bits, unsigned low_bit
     return wide || e > 126 ? kPlain : e;
 }
 
-// Blocks take tiles of GROUP_ROWS x GROUP_COLS in turn, a warp four rows of a tile and a lane four elements of each.
+// Blocks take tiles of up to GROUP_ROWS x GROUP_COLS in turn, a warp four rows of a tile and a lane four elements of each.
 template <int N>
 __global__ void __launch_bounds__(256) pack_max_k(const __grid_constant__ PackJobs<N> jobs) {
     cnb_pdl_enter();
@@ -1211,18 +1214,20 @@ __global__ void __launch_bounds__(256) pack_max_k(const __grid_constant__ PackJo
     __shared__ unsigned col[8][GROUP_COLS], block_most[8], block_low[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool vec = pack_vec(job);
-    const int tiles_x = (job.cols + GROUP_COLS - 1) / GROUP_COLS;
-    const long tiles = (long) ((job.rows + GROUP_ROWS - 1) / GROUP_ROWS) * tiles_x;
+    const int unit = vec ? 4 : 1, units = job.cols / unit, tiles = job.tiles_x * job.tiles_y;
+    const int width = units / job.tiles_x, wider = units % job.tiles_x, height = job.rows / job.tiles_y, higher = job.rows % job.tiles_y;
     unsigned most = 0, low = 0;        // low: ~ of the least group maximum, 0 while there is none
-    for (long t = blockIdx.x; t < tiles; t += job.max_blocks) {
-        const int r0 = (int) (t / tiles_x) * GROUP_ROWS + warp, c0 = (int) (t % tiles_x) * GROUP_COLS;
+    for (int t = blockIdx.x; t < tiles; t += job.max_blocks) {
+        const int y = t / job.tiles_x, x = t % job.tiles_x;
+        const int top = y * height + min(y, higher), r0 = top + warp, r1 = top + height + (y < higher);
+        const int c0 = (x * width + min(x, wider)) * unit, c1 = c0 + (width + (x < wider)) * unit;
         float re[4][4], im[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int row = r0 + 8 * i;
             const size_t at = (size_t) row * job.cols + c0;
             if (vec) {
-                const bool on = row < job.rows && c0 + 4 * lane < job.cols;
+                const bool on = row < r1 && c0 + 4 * lane < c1;
                 const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
                 const float4 x = on ? *reinterpret_cast<const float4*>(job.re + at + 4 * lane) : z;
                 const float4 y = on ? *reinterpret_cast<const float4*>(job.im + at + 4 * lane) : z;
@@ -1231,7 +1236,7 @@ __global__ void __launch_bounds__(256) pack_max_k(const __grid_constant__ PackJo
             } else {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const bool on = row < job.rows && c0 + lane + 32 * k < job.cols;
+                    const bool on = row < r1 && c0 + lane + 32 * k < c1;
                     re[i][k] = on ? job.re[at + lane + 32 * k] : 0.f;
                     im[i][k] = on ? job.im[at + lane + 32 * k] : 0.f;
                 }
@@ -1718,9 +1723,10 @@ template <int N> static int pack_some(cnb_ctx* ctx, const PackRequest* r, int n,
         if (reinterpret_cast<uintptr_t>(r[k].planes) & 127 || r[k].pitch % 8)
             return set_error(CNB_ERR_ARG, "pack: planes must be 128-byte aligned, pitch %d a multiple of 8", r[k].pitch);
         const size_t items = (size_t) r[k].rows * ((r[k].cols + 3) / 4);
-        const size_t tiles = ((size_t) (r[k].rows + GROUP_ROWS - 1) / GROUP_ROWS) * ((r[k].cols + GROUP_COLS - 1) / GROUP_COLS);
+        const int tiles_x = (r[k].cols - 1) / GROUP_COLS + 1, tiles_y = (r[k].rows - 1) / GROUP_ROWS + 1;
+        const size_t tiles = (size_t) tiles_x * tiles_y;
         jobs.j[k] = {r[k].re, r[k].im, static_cast<__half*>(r[k].planes), r[k].head, r[k].rows, r[k].cols, r[k].pitch,
-                     (int) std::min((items + 255) / 256, cap), (int) std::min(tiles, cap)};
+                     (int) std::min((items + 255) / 256, cap), (int) std::min(tiles, cap), tiles_x, tiles_y};
         blocks = std::max(blocks, jobs.j[k].blocks);
         max_blocks = std::max(max_blocks, jobs.j[k].max_blocks);
     }

@@ -132,7 +132,7 @@ int cnb_linear_bwd_w_split(cnb_ctx* ctx, const float* g_split, const float* x_sp
  * high = fp16(x) and low = fp16(x - high): 22 bits of every component down to 2^-17 of the largest, then gradually
  * fewer, an absolute error of 2^-39 of the largest at most.  A product is high.high + high.low + low.high on the
  * FP16 pipe with fp32 accumulation and takes the scales out again.  A matrix in which the largest component of some
- * 1 x 128 or 32 x 1 elements is less than 2^-17 of the whole's (and not zero) keeps its fp32 values in the pack, and its
+ * 1 x 128 or 32 x 1 elements (at odd sizes down to half of that) is less than 2^-17 of the whole's (and not zero) keeps its fp32 values in the pack, and its
  * products run as fp32 FMAs.  A pack is cnb_pack_bytes(rows, cols) of 256-byte
  * aligned memory, its first 256 bytes zeroed once before the first use: [0, 256) the head, then as fp16 the planes
  * high re, high im, low re, low im, rows at a pitch of `cols` rounded up to 64.  Any sizes; cnb_linear_pack_ok says

@@ -143,3 +143,17 @@ def test_net_with_rows_of_any_scale(B, n_in, n_out):
         err = np.linalg.norm(got[0] + 1j * got[1].astype(np.float64) - dx, axis=1) / np.linalg.norm(dx, axis=1)
         assert (err < TOL * np.maximum(1, spread)).all(), err.max()
     assert util.relerr(dev.get_values(sd.layers["w"]), ora.get_values(so.layers["w"])) == 0
+
+
+@pytest.mark.parametrize("rows,cols", [(33, 900), (65, 129), (97, 257), (4097, 130), (32, 128), (500, 1025)])
+def test_remainders_are_not_mistaken_for_small_lines(ctx, rows, cols):  # noqa: F811
+    """Values of a CGelu of heavy-tailed products, of which many lone ones are tiny: at sizes one beyond a group the
+    matrix is still packed, not kept plain."""
+    import torch
+    rng = np.random.default_rng(rows + cols)
+    a = _c(_rand(rng, rows, cols)) * _c(_rand(rng, rows, cols)) * 2
+    y = tuple(co._gelu(p).astype(np.float32) for p in (a.real, a.imag))
+    pack = torch.zeros(ctx.lib.cnb_pack_bytes(rows, cols) // 4, device="cuda")
+    d = _dev(y)
+    assert ctx.lib.cnb_pack_matrix(ctx.h, d[0].data_ptr(), d[1].data_ptr(), rows, cols, pack.data_ptr(), 0, ctx._stream()) == 0
+    assert pack[:1].view(torch.int32).item() < 1 << 20
