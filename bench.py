@@ -196,58 +196,28 @@ def cpu_baseline(workload, seconds=15.0):
                       "(oracle/_ref), %.1f s" % (k, gbatch, dt)}
 
 
-# DRAM traffic of one launch of the dominant kernel from the ncu capture summarised under profiles/
-# (dram__bytes_read.sum + dram__bytes_write.sum), keyed by (M, N, K); None where not captured.
-NCU_TRAFFIC_BYTES = {(4096, 1024, 1024): 126.3e6}
+def _pack(ctx, t):
+    """A matrix packed for the tensor-core products, as the layers of a Net keep their operands."""
+    import torch
+    rows, cols = t[0].shape
+    p = torch.zeros(ctx.lib.cnb_pack_bytes(rows, cols), dtype=torch.uint8, device="cuda")
+    return _repack(ctx, t, p)
 
-_TF32 = {}
+
+def _repack(ctx, t, p):
+    from cnet_b200 import lib as cl
+    rows, cols = t[0].shape
+    cl.check(ctx.lib.cnb_pack_matrix(ctx.h, t[0].data_ptr(), t[1].data_ptr(), rows, cols, p.data_ptr(), 0, ctx._stream()), "pack")
+    return p
 
 
-def _tf32_peak(torch, gpu_index):
-    """Dense TF32 throughput of this GPU, measured the way MEASURED_PEAKS.json's bf16 figure was: torch.matmul
-    (cuBLAS, fp32 operands with TF32 allowed) at 8192^3, best of 10 launches (burst) and back to back for ~2 s
-    (sustained), clocks sampled during the sustained loop.  A measuring stick only: no kernel of the path uses it."""
-    if _TF32:
-        return _TF32
-    n = 8192
-    old = torch.backends.cuda.matmul.allow_tf32
-    torch.backends.cuda.matmul.allow_tf32 = True
-    try:
-        a = torch.randn(n, n, device="cuda")
-        b = torch.randn(n, n, device="cuda")
-        c = torch.empty(n, n, device="cuda")
-        for _ in range(3):
-            torch.matmul(a, b, out=c)
-        best = 1e30
-        for _ in range(10):
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            torch.matmul(a, b, out=c)
-            e1.record()
-            torch.cuda.synchronize()
-            best = min(best, e0.elapsed_time(e1))
-        clocks = _Clocks(gpu_index, interval_ms=50)
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        count = 0
-        t0 = time.perf_counter()
-        e0.record()
-        while time.perf_counter() - t0 < 2.0:
-            for _ in range(25):
-                torch.matmul(a, b, out=c)
-            count += 25
-            torch.cuda.synchronize()
-        e1.record()
-        torch.cuda.synchronize()
-        clk = clocks.stop()
-        flops = 2.0 * n ** 3
-        _TF32.update({"tf32_tflops": flops / (best * 1e-3) / 1e12,
-                      "tf32_tflops_sustained": flops * count / (e0.elapsed_time(e1) * 1e-3) / 1e12,
-                      "sm_mhz_sustained": clk.get("sm_mhz"), "reasons_sustained": clk.get("reasons"),
-                      "how": "torch.matmul fp32 with TF32 allowed, 8192^3: best of 10 (burst), back to back for 2 s (sustained)"})
-    finally:
-        torch.backends.cuda.matmul.allow_tf32 = old
-    del a, b, c
-    return _TF32
+def _packed_product(ctx, kind, a, b, out, B, n_in, n_out):
+    """cnb_linear_fwd_packed / _bwd_x_packed / _bwd_w_packed into `out`."""
+    from cnet_b200 import lib as cl
+    fn = getattr(ctx.lib, "cnb_linear_%s_packed" % kind)
+    extra = (None, None) if kind == "fwd" else ()
+    tail = (B, n_in, n_out) if kind == "fwd" else (B, n_in, n_out, 0)
+    cl.check(fn(ctx.h, a.data_ptr(), b.data_ptr(), *extra, out[0].data_ptr(), out[1].data_ptr(), *tail, ctx._stream()), kind)
 
 
 def _time_launches(torch, fn, reps=20, clocks_for=None):
@@ -320,30 +290,19 @@ def _hbm_entry(torch, peaks, name, fns, nbytes):
             "operand_sets": len(fns)}
 
 
-def _tensor_roof(torch, peaks, dur, mhz, B, n_out, n_in, gpu_index):
-    """Roofline of the split complex GEMM.  Every real product of the 8*M*N*K algorithmic flops passes the tensor
-    cores three times: hi.hi on the TF32 pipe and the two cross terms on the BF16 pipe, so the time per
-    algorithmic flop at peak is 1/TF32 + 2/BF16 (TF32 measured in this run, BF16 from the peaks file).
-    frac_3xtf32 = the same launch against the all-TF32 form's roofline (TF32 / 3), for comparison."""
+def _tensor_roof(torch, peaks, dur, mhz, B, n_out, n_in):
+    """Roofline of the complex GEMM on packed operands.  Every real product of the 8*M*N*K algorithmic flops passes the
+    tensor cores three times at the 16-bit rate (high.high, high.low, low.high), so the roof is a third of the measured
+    dense bf16 throughput."""
     flops = 8.0 * B * n_in * n_out
     achieved = flops / (dur * 1e-3) / 1e12
-    tf = _tf32_peak(torch, gpu_index)
-    peak = 1.0 / (1.0 / tf["tf32_tflops"] + 2.0 / peaks["bf16"])
-    sustained = 1.0 / (1.0 / tf["tf32_tflops_sustained"] + 2.0 / (peaks["bf16_sustained"] or peaks["bf16"]))
-    derived = 1.0 / (2.0 / peaks["bf16"] + 2.0 / peaks["bf16"])      # what the peaks file alone gives: TF32 = bf16 / 2
+    peak, sustained = peaks["bf16"] / 3.0, (peaks["bf16_sustained"] or peaks["bf16"]) / 3.0
     return {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-            "frac_derived": achieved / derived, "peak_derived": derived,
-            "frac_sustained": achieved / sustained,
-            "frac_3xtf32": achieved / (tf["tf32_tflops"] / 3.0), "peak_3xtf32": tf["tf32_tflops"] / 3.0,
-            "traffic": NCU_TRAFFIC_BYTES.get((B, n_out, n_in)),
-            "kernel": "cgemm_tc_k (tcgen05: TF32 hi.hi + BF16 cross terms)",
+            "frac_sustained": achieved / sustained, "traffic": None,
+            "kernel": "cgemm_tc_k (tcgen05, packed fp16 operands: high.high + high.low + low.high)",
             "shape": [B, n_out, n_in], "ms_per_launch": dur, "sm_mhz_during": mhz,
-            "ms_x_mhz": (dur * mhz) if mhz else None, "tf32_peak": tf,
-            "peak_note": "1 / (1/TF32 + 2/BF16): dense TF32 measured in this run (cuBLAS 8192^3 burst %.1f TFLOP/s, sustained "
-                         "%.1f at %s MHz), BF16 burst %.1f of %s; frac_derived = with TF32 taken as BF16 / 2; "
-                         "frac_3xtf32 = against TF32 / 3"
-                         % (tf["tf32_tflops"], tf["tf32_tflops_sustained"], tf["sm_mhz_sustained"], peaks["bf16"],
-                            peaks["source"])}
+            "ms_x_mhz": (dur * mhz) if mhz else None,
+            "peak_note": "BF16 / 3: three 16-bit passes a real product, BF16 burst %.1f of %s" % (peaks["bf16"], peaks["source"])}
 
 
 def _roofline(workload, kw, B, gbatch, step_ms, device, hbm_kernels=True):
@@ -364,15 +323,15 @@ def _roofline(workload, kw, B, gbatch, step_ms, device, hbm_kernels=True):
     w = tuple(torch.randn(n_out, n_in, device="cuda") * n_in ** -0.5 for _ in range(2))
     hbm = []
     if ctx.lib.cnb_linear_split_ok(B, n_in, n_out):
-        # operands pre-split; every launch of the timed run has activations and output of its own (the weights
+        # operands packed beforehand; every launch of the timed run has activations and output of its own (the weights
         # are shared, as a layer's are), so no launch finds its operands in L2
-        SG = _nsets(24.0 * B * n_in + 8.0 * B * n_out, hi=12)
-        ws = ctx.split(w)
-        xs = [ctx.split(tuple(torch.randn(B, n_in, device="cuda") for _ in range(2))) for _ in range(SG)]
+        SG = _nsets(8.0 * B * n_in + 8.0 * B * n_out, hi=12)
+        ws = _pack(ctx, w)
+        xs = [_pack(ctx, tuple(torch.randn(B, n_in, device="cuda") for _ in range(2))) for _ in range(SG)]
         ys = [ctx._new(B, n_out) for _ in range(SG)]
-        fns = [lambda k=k: ctx.linear_fwd_split(xs[k], ws, B, n_in, n_out, out=ys[k]) for k in range(SG)]
+        fns = [lambda k=k: _packed_product(ctx, "fwd", xs[k], ws, ys[k], B, n_in, n_out) for k in range(SG)]
         dur, mhz = _time_stream(torch, fns, launches=200, clocks_for=device)
-        roof = _tensor_roof(torch, peaks, dur, mhz, B, n_out, n_in, device)
+        roof = _tensor_roof(torch, peaks, dur, mhz, B, n_out, n_in)
         roof["ms_single"] = _time_launches(torch, fns[0], reps=20)
         roof["timing"] = ("ms_per_launch: average of 200 launches back to back on the stream over %d operand sets (larger than L2 "
                           "together); ms_single: one launch between two events after an L2 flush" % SG)
@@ -445,11 +404,10 @@ def _roofline(workload, kw, B, gbatch, step_ms, device, hbm_kernels=True):
         # the second product of the net at its shape (K = hidden)
         x2 = tuple(torch.randn(B, H, device="cuda") for _ in range(2))
         w2 = tuple(torch.randn(V, H, device="cuda") * H ** -0.5 for _ in range(2))
-        xs2, ws2 = ctx.split(x2), ctx.split(w2)
-        d2 = _time_stream(torch, [lambda k=k: ctx.linear_fwd_split(xs2, ws2, B, H, V, out=yv[k]) for k in range(S)], launches=20)
+        xs2, ws2 = _pack(ctx, x2), _pack(ctx, w2)
+        d2 = _time_stream(torch, [lambda k=k: _packed_product(ctx, "fwd", xs2, ws2, yv[k], B, H, V) for k in range(S)], launches=20)
         roof["second_gemm"] = {"shape": [B, V, H], "ms_per_launch": d2,
-                               "frac": 8.0 * B * H * V / (d2 * 1e-3) / 1e12 / roof["peak"],
-                               "frac_3xtf32": 8.0 * B * H * V / (d2 * 1e-3) / 1e12 / roof["peak_3xtf32"]}
+                               "frac": 8.0 * B * H * V / (d2 * 1e-3) / 1e12 / roof["peak"]}
     elif hbm_kernels:
         N = n_in
         S = _nsets(16.0 * B * N)
@@ -473,12 +431,14 @@ def _roofline(workload, kw, B, gbatch, step_ms, device, hbm_kernels=True):
                   [lambda k=k: L.cnb_dft_fwd(H_, P(u[k][0]), P(u[k][1]), P(o[k][0]), P(o[k][1]), B, N, st) for k in range(S)],
                   16.0 * B * N)]
         if L.cnb_dft_fused_ok(N):
-            # the forms that run inside the step: forward with the Hadamard + CGelu + operand split tail (reads x; writes
-            # u and four split planes), backward accumulating into the gradient (reads g, read-modify-writes dx)
-            sp = [torch.empty(L.cnb_split_floats(B * N), dtype=torch.float32, device="cuda") for _ in range(S)]
-            cases.append(("fft1024_pipe_k<-1> + Hadamard + CGelu + split tail (as in the step)" if N == 1024 else "FourierTrans forward + tail",
-                          [lambda k=k: L.cnb_dft_hadamard_gelu_fwd(H_, P(u[k][0]), P(u[k][1]), P(h[0]), P(h[1]), P(o[k][0]), P(o[k][1]), None, None, P(sp[k]), B, N, st) for k in range(S)],
-                          32.0 * B * N))
+            # the forms that run inside the step: forward with the Hadamard + CGelu tail (reads x; writes u and y), the
+            # packing of y (reads it twice, writes the pack), backward accumulating into the gradient (reads g,
+            # read-modify-writes dx)
+            cases.append(("fft1024_pipe_k<-1> + Hadamard + CGelu tail (as in the step)" if N == 1024 else "FourierTrans forward + tail",
+                          [lambda k=k: L.cnb_dft_hadamard_gelu_fwd(H_, P(u[k][0]), P(u[k][1]), P(h[0]), P(h[1]), P(o[k][0]), P(o[k][1]), P(a[k][0]), P(a[k][1]), None, B, N, st) for k in range(S)],
+                          24.0 * B * N))
+            packs = [_pack(ctx, g[k]) for k in range(S)]
+            cases.append(("pack_max_k + pack_k", [lambda k=k: _repack(ctx, g[k], packs[k]) for k in range(S)], 24.0 * B * N))
             cases.append(("fft1024_pipe_k<+1> backward, reduce-add into the gradient (as in the step)" if N == 1024 else "FourierTrans backward + accumulate",
                           [lambda k=k: L.cnb_dft_bwd(H_, P(g[k][0]), P(g[k][1]), P(o[k][0]), P(o[k][1]), B, N, 1, st) for k in range(S)],
                           24.0 * B * N))
@@ -505,7 +465,7 @@ def _median(v):
 
 def run_linear(args, steps=None, repeats=None, quiet=False):
     """Config 2: one complex Linear layer, forward plus both backward products, through the C-ABI
-    operators (operands split once per step, three tensor-core GEMMs).  Single GPU."""
+    operators (operands packed once per step, three tensor-core GEMMs).  Single GPU."""
     import torch
     from cnet_b200 import lib as cl
     from cnet_b200.ops import Context
@@ -533,10 +493,11 @@ def run_linear(args, steps=None, repeats=None, quiet=False):
             d.copy_(h, non_blocking=True)
 
     def step():
-        xs, ws, gs = ctx.split(x), ctx.split(w), ctx.split(g)
-        ctx.linear_fwd_split(xs, ws, B, n_in, n_out, out=y)
-        ctx.linear_bwd_x_split(gs, ws, B, n_in, n_out, out=dx)
-        ctx.linear_bwd_w_split(gs, xs, B, n_in, n_out, out=dw)
+        for t, p in ((x, px), (w, pw), (g, pg)):
+            _repack(ctx, t, p)
+        _packed_product(ctx, "fwd", px, pw, y, B, n_in, n_out)
+        _packed_product(ctx, "bwd_x", pg, pw, dx, B, n_in, n_out)
+        _packed_product(ctx, "bwd_w", pg, px, dw, B, n_in, n_out)
 
     def e2e_step():
         upload()
@@ -562,6 +523,7 @@ def run_linear(args, steps=None, repeats=None, quiet=False):
         return 1e3 * (time.perf_counter() - t0)
 
     upload()
+    px, pw, pg = _pack(ctx, x), _pack(ctx, w), _pack(ctx, g)
     for _ in range(max(3, args.warmup)):
         step()
     clocks = _Clocks(0)
@@ -578,9 +540,8 @@ def run_linear(args, steps=None, repeats=None, quiet=False):
     peaks = _peaks()
     per_step = ms / steps
     tflops = 3 * 8.0 * B * n_in * n_out / (per_step * 1e-3) / 1e12
-    xs_, ws_ = ctx.split(x), ctx.split(w)
-    dur, mhz = _time_launches(torch, lambda: ctx.linear_fwd_split(xs_, ws_, B, n_in, n_out, out=y), reps=40, clocks_for=0)
-    roof = _tensor_roof(torch, peaks, dur, mhz, B, n_out, n_in, 0)
+    dur, mhz = _time_launches(torch, lambda: _packed_product(ctx, "fwd", px, pw, y, B, n_in, n_out), reps=40, clocks_for=0)
+    roof = _tensor_roof(torch, peaks, dur, mhz, B, n_out, n_in)
     roof["step_gemm_tflops"] = tflops
     line = {
         "metric": "train samples/sec (fwd+bwd+update)", "value": B / (per_step * 1e-3), "unit": "samples/s",
