@@ -1,18 +1,20 @@
-// tcgen05 complex GEMM with an error-compensated operand split, for sm_100a.
+// tcgen05 complex GEMM on error-compensated operands, for sm_100a.
 //
 //   D[m,n] (+)= sum_k A[m,k] * (conjB ? conj(B[n,k]) : B[n,k]) (+ R[m,n])
-//   A [M,K], B [N,K] complex, K-major (row-major) or MN-major ([K, rows]) split planes.
+//   A [M,K], B [N,K] complex, K-major (row-major) or MN-major ([K, rows]).
 //
-// Numerics.  Every fp32 operand x is split once, before the GEMM, into hi = x with the 13 low
-// mantissa bits cleared (exactly a TF32 value) and lo = x - hi (exact in fp32).  Each real
-// product is three tensor-core MMAs with fp32 accumulation in tensor memory:
+// Numerics.  Two operand forms, each three tensor-core MMAs per real product with fp32 accumulation in tensor memory.
+// PACKED, what everything but the C ABI's split buffers runs on: two fp16 parts, high and low, of the matrix scaled by one
+// power of two (22 bits; see pack_k below, also for matrices whose range is too wide for that and which run as fp32
+// FMAs); high.low + low.high + high.high on the FP16 pipe, 1.5 TF32-equivalents, 4 operand bytes per real element.  Sizes
+// whose alternative are fp32 FMAs are summed in chains short enough not to be less exact than those (max_chain).
+// SPLIT, the split buffers: hi = x with the 13 low mantissa bits cleared (exactly a TF32 value) and lo = x - hi (exact in
+// fp32);
 //     hi*hi                on the TF32 pipe (exact products), and
 //     hi*lo + lo*hi        on the BF16 pipe, from hi and lo rounded to bf16 (h16, l16).
-// The cross terms are 2^-10 of the product, so their bf16 rounding (2^-9 each factor) costs 2^-18 of the
+// Its cross terms are 2^-10 of the product, so their bf16 rounding (2^-9 each factor) costs 2^-18 of the
 // product per cross term at worst (2^-19.5 rms for both), next to the 2^-20 of the dropped lo*lo term; fp32's
-// exponent range is kept (no scaling).
-// A BF16 MMA of depth 16 takes the time of a TF32 MMA of depth 8, so a real product costs two TF32-equivalents
-// instead of the three of the all-TF32 form, for the same operand bytes (8 per real element).
+// exponent range is kept (no scaling).  Two TF32-equivalents a real product, 8 operand bytes per real element.
 //
 // Tiling.  One CTA computes a 128 x 128 complex tile.  The B tile is staged as ONE 256-row
 // operand [B_re rows ; B_im rows], so every MMA is 128 x 256 and the complex structure
@@ -20,7 +22,9 @@
 //     acc1 = A_re * [B_re ; B_im]^T      (TMEM columns   0..255)
 //     acc2 = A_im * [B_re ; B_im]^T      (TMEM columns 256..511)
 //     D_re = acc1[:, :128] -/+ acc2[:, 128:],   D_im = acc1[:, 128:] +/- acc2[:, :128]   (epilogue)
-// Per 16-deep k-block a stage holds 8 operand slots of 8 KB = 64 KB; 3 stages:
+// A stage holds 8 operand slots of 8 KB = 64 KB; 3 stages.  PACKED, a k-block of 32:
+//     A high re, high im, low re, low im, then the same of B (fp16, 64-byte swizzle);
+// per k-block and accumulator: 6 FP16 MMAs (k-steps of 16).  SPLIT, a k-block of 16:
 //     A hi_re, A hi_im (fp32, 64-byte swizzle),  A h16 [re ; im], A l16 [re ; im] (bf16, 32-byte swizzle),
 //     B hi_re, B hi_im,                          B h16 [re ; im], B l16 [re ; im];
 // per k-block and accumulator: 2 TF32 MMAs (k-steps of 8) + 2 BF16 MMAs (one k-step of 16).

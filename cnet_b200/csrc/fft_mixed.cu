@@ -1,6 +1,6 @@
 // FourierTrans at any length that fits shared memory: a mixed-radix Stockham transform, rows in shared memory.
 //
-// N is factored into radices of at most 16 (2..16; primes up to 13), as few passes as that takes: 784 = 14 x 14 x 4,
+// N is factored into radices of at most 16 (2..16; primes up to 13), as few passes as that takes: 784 = 8 x 14 x 7,
 // 1500 = 10 x 15 x 10, 4096 = 16 x 16 x 16.  A thread takes one butterfly of R points at a time in registers; pass p
 // with L = the product of the radices before it reads x[j + q N/R], multiplies by e^{-2 pi i (j % L) q / (L R)},
 // transforms over q and writes (j / L) L R + j % L + q L, so the last pass comes out in natural order.  The first

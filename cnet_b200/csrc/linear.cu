@@ -1,5 +1,5 @@
 // Complex Linear (forward, dX*, dW*) and FourierTrans as a complex GEMM against a
-// twiddle matrix: shape dispatch between the tcgen05 tiles (split operands) and the fp32 SIMT tiles.
+// twiddle matrix: shape dispatch between the tcgen05 tiles (packed operands) and the fp32 SIMT tiles.
 #include <algorithm>
 #include <cmath>
 #include <vector>

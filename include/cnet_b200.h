@@ -93,9 +93,10 @@ int cnb_linear_bwd_w(cnb_ctx* ctx, const float* g_re, const float* g_im,
                      const float* x_re, const float* x_im,
                      float* dw_re, float* dw_im, int B, int in, int out,
                      int accumulate, void* stream);
-/* Scratch bytes the three products of a Linear(B, in, out) may take from the arena (operand
- * split buffers of the tensor-core GEMM), and a way to reserve the step's maximum up front
- * so that no call on the step path grows the scratch region.  Replace the per-call cudaMalloc of
+/* Scratch bytes the three products of a Linear(B, in, out) may take from the arena (packed
+ * operands of the tensor-core GEMM), and a way to reserve the step's maximum up front
+ * so that no call on the step path grows the scratch region.  What raw products take without such a reservation is
+ * given back to a cnb_alloc or a table that finds no other room (unless a captured graph uses it).  Replace the per-call cudaMalloc of
  * gpu/reduce.cpp:594-598 and gpu/reducegrad.cpp:309-322. */
 size_t cnb_linear_workspace(int B, int in, int out);
 int cnb_reserve_scratch(cnb_ctx* ctx, size_t bytes);
@@ -154,8 +155,8 @@ int cnb_linear_bwd_w_packed(cnb_ctx* ctx, const void* g_pack, const void* x_pack
  * all-reduce of a data-parallel job); 0 restores the full grid.  No reference counterpart. */
 int cnb_set_gemm_sm_limit(cnb_ctx* ctx, int max_ctas);
 /* Which GEMM engine the last cnb_linear_* call on this thread used:
- * 1 = tcgen05 tensor-core tiles (split operands: TF32 hi.hi + BF16 cross terms), 2 = fp32 SIMT tiles (ragged shapes),
- * 4 = skinny fp32 kernels (out <= 16, HBM-bound). */
+ * 1 = tcgen05 tensor-core tiles (packed or split operands; a packed matrix of wide range is multiplied in fp32 FMAs
+ * there), 2 = fp32 SIMT tiles (small products, a short K, no room for packed operands), 4 = skinny fp32 kernels (out <= 16, HBM-bound). */
 int cnb_last_gemm_engine(void);
 
 /* ---------------------------------------------------------------- FourierTrans
