@@ -212,6 +212,14 @@ __device__ __forceinline__ void cnb_pdl_trigger() { asm volatile("griddepcontrol
 __device__ __forceinline__ void cnb_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void cnb_pdl_enter() { cnb_pdl_trigger(); cnb_pdl_wait(); }
 
+// A value that kernels before this one may have written, read among this kernel's own stores: not through __ldg, which is not
+// held behind cnb_pdl_wait, and without the order that a plain load has against the stores before it.
+__device__ __forceinline__ float cnb_ld_behind_wait(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
 namespace cnb {
 
 bool pdl_enabled();                // CNB_PDL=0 in the environment launches every kernel fully serialised

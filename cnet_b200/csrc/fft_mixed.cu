@@ -132,7 +132,9 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
                 io.yr[g] = u.x;
                 io.yi[g] = u.y;
                 if (FINISH == TAIL) {
-                    const float hr = __ldg(ep.hr + e), hi = __ldg(ep.hi + e);
+                    // the kernels before may have written h: the read-only path only behind a barrier of this one
+                    const bool lone = pl.passes == 1;
+                    const float hr = lone ? cnb_ld_behind_wait(ep.hr + e) : __ldg(ep.hr + e), hi = lone ? cnb_ld_behind_wait(ep.hi + e) : __ldg(ep.hi + e);
                     const float ar = u.x * hr - u.y * hi, ai = u.x * hi + u.y * hr;
                     const float gr = cnb_gelu(ar), gi = cnb_gelu(ai);
                     const size_t at = (io.row0 + row) * (size_t) pl.n + e;
