@@ -42,7 +42,7 @@
 // k-range is shared by several CTAs is summed with fp32 atomics into a pre-zeroed output.
 //
 // Roles.  warp 0: TMA producer; warp 1: TMEM allocation + MMA issue (one elected thread);
-// warps 2..9: epilogue (tcgen05.ld, combine, stage through shared memory, coalesced 16-byte
+// the last eight warps: epilogue (tcgen05.ld, combine, stage through shared memory, coalesced 16-byte
 // stores / atomics with residual or accumulate), two groups of four warps with half of a tile's columns each;
 // tensor memory is handed back to the MMA warp as soon as it has been read, so the write-out overlaps the next
 // run of MMAs.  With one group a whole tile left in 4.6 us after its last MMA, 8.9 with a residual and 18.8 where
@@ -55,6 +55,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 
 #include "cgemm_fma.cuh"
 #include "common.cuh"
@@ -82,7 +83,12 @@ template <bool PAIR> struct Cfg {
     static constexpr int TILE_M = PAIR ? 2 * BM : BM;
 };
 constexpr int OPERAND_BYTES = 3 * 8 * PLANE_BYTES;   // 192 KB of operand stages in both forms
-constexpr int EPI_GROUPS = 2, EPI_THREADS = 128 * EPI_GROUPS, NUM_THREADS = 64 + EPI_THREADS;
+constexpr int EPI_GROUPS = 2, EPI_THREADS = 128 * EPI_GROUPS;
+// Threads: DRAIN, three warpgroups (two warps of the first have nothing to do), with this many registers a thread of the first
+// and of the epilogue's two out of what all are launched with; else the two warps and the epilogue.
+template <bool DRAIN> struct Threads { static constexpr int FIRST_EPI = DRAIN ? 128 : 64, ALL = FIRST_EPI + EPI_THREADS; };
+constexpr int LAUNCH_REGS = 168, ISSUE_REGS = 56, EPI_REGS = 224;
+static_assert(128 * ISSUE_REGS + EPI_THREADS * EPI_REGS <= Threads<true>::ALL * LAUNCH_REGS, "registers");
 constexpr int EPI_BYTES = EPI_GROUPS * 2 * 128 * 16 * 4;  // 32 KB: one epilogue round of both groups, re and im staging
 constexpr int SMEM_BYTES = OPERAND_BYTES + EPI_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 static_assert(Cfg<false>::STAGES * Cfg<false>::STAGE_BYTES == OPERAND_BYTES && Cfg<true>::STAGES * Cfg<true>::STAGE_BYTES == OPERAND_BYTES, "stages");
@@ -98,7 +104,7 @@ struct TcParams {
     int cluster;              // > 1: that many CTAs of one cluster share a tile, each a slice of K
     int whole_per_cta;        // > 0: every CTA first takes that many whole tiles, then its run of the remaining units
     int segments;             // > 0: CTA r takes k-segment r / tiles of tile r % tiles (units_per_cta k-blocks each)
-    int chain;                // DRAIN: k-blocks that are summed in tensor memory at most
+    int chain, small_first;   // PACKED: k-blocks that are summed in tensor memory at most; whether runs are longer than that
     const int* a_exp;         // PACKED: the powers of two that A and B were scaled by, or kPlain
     const int* b_exp;
     const void* a_planes; const void* b_planes;       // PACKED: what the tensor maps describe, for the FMA form
@@ -200,8 +206,11 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t local_addr, uint32_t ra
     return remote;
 }
 
+// Hands a CTA's accumulators back to the pair's first CTA.  What the arrival orders are tensor-memory loads, which the
+// tcgen05 fence in front of it has ordered; release at cluster scope would also wait for every store of the thread before
+// it (1.4 us of idle MMAs after each chain and each tile).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 // MN-major operand tile (source stored [K, rows]): slabs of 32 rows-of-the-operand, each slab
@@ -334,15 +343,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-    uint32_t r[8];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 // Packed operands: a matrix that is stored as fp32 planes instead of fp16 parts has this for its exponent.
 constexpr int kPlain = 1 << 20;
 
@@ -373,26 +373,24 @@ __device__ __noinline__ void fma_product(const TcParams& p, void* smem) {
     const int tiles_n = (p.N + cnb_fma::TN - 1) / cnb_fma::TN, tiles = (p.M + cnb_fma::TM - 1) / cnb_fma::TM * tiles_n;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x)
         cnb_fma::tile(a, b, r, *static_cast<cnb_fma::Slabs*>(smem), t / tiles_n * cnb_fma::TM, t % tiles_n * cnb_fma::TN,
-                      (int) threadIdx.x - (NUM_THREADS - EPI_THREADS),
+                      (int) threadIdx.x - ((int) blockDim.x - EPI_THREADS),
                       [] { asm volatile("bar.sync %0, %1;" ::"n"(1 + EPI_GROUPS), "n"(EPI_THREADS) : "memory"); });
 }
 
-// The accumulators of one chain (this thread's row, the 64 columns of its group from `tl` on) into the running sums,
-// rounded to nearest.
-__device__ __forceinline__ void drain_chain(uint32_t tl, float sgn, float (&sr)[64], float (&si)[64]) {
+// One accumulator of a chain (this thread's row, the 64 columns of its group from `tl` on) into the running sums, rounded
+// to nearest: acc1 holds A_re.[B_re ; B_im], acc2 A_im.[B_re ; B_im].  The last load has completed on return.
+template <int ACC> __device__ __forceinline__ void drain_chain(uint32_t tl, float sgn, float (&sr)[64], float (&si)[64]) {
 #pragma unroll
-    for (int c = 0; c < 64; c += 8) {
-        float x[8], y[8];
-        tmem_ld8(tl + c, x);                             // A_re.B_re
-        tmem_ld8(tl + 384 + c, y);                       // A_im.B_im
+    for (int c = 0; c < 64; c += 16) {
+        float x[16], y[16];
+        tmem_ld16(tl + ACC * 256 + c, x);                // . B_re
+        tmem_ld16(tl + ACC * 256 + 128 + c, y);          // . B_im
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int i = 0; i < 8; ++i) sr[c + i] += x[i] + sgn * y[i];
-        tmem_ld8(tl + 256 + c, x);                       // A_im.B_re
-        tmem_ld8(tl + 128 + c, y);                       // A_re.B_im
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int i = 0; i < 8; ++i) si[c + i] += x[i] - sgn * y[i];
+        for (int i = 0; i < 16; ++i) {
+            if (ACC == 0) { sr[c + i] += x[i]; si[c + i] -= sgn * y[i]; }
+            else { si[c + i] += x[i]; sr[c + i] += sgn * y[i]; }
+        }
     }
 }
 
@@ -566,10 +564,14 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 // VEC: rows of D and R are 16-byte aligned (N % 4 == 0); the form without it writes 32 consecutive floats of a row per
 // warp instruction instead of four 16-byte pieces of four rows.
 // DRAIN: a run of more than p.chain k-blocks is cut into chains of that many; after each the epilogue takes the
-// accumulators into running sums in registers (max_chain says why).  777 x 1333 -> 1001, three products: 158 -> 172 us,
-// forward off by 4.4e-7 of float64 instead of 2.4e-6 (fp32 FMAs: 6.6e-7).
+// accumulators into running sums in registers (max_chain says why), one while the other is still multiplied, so that the
+// MMAs hardly wait: 777 x 1333 -> 1001 forward, six chains, 40.3 -> 33.7 us beside one accumulator barrier and the epilogue
+// on its share of 168 registers.  The same form runs where a CTA goes through several tiles: a tile leaves tensor memory in
+// 0.3 us and is written out under the next one's MMAs (4096 x 1024 x 1024 76 -> 70 us).  Launches of one chain and one tile
+// a CTA take the form without: they leave registers of the SM to the kernels around them, and their set-up runs under the
+// tail of the kernel before (512-row training step 772 -> 743 us).
 template <bool PAIR, bool VEC, int FORM, bool DRAIN>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(Threads<DRAIN>::ALL, 1)
 cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__ TcParams p) {
     extern __shared__ uint8_t smem_raw[];
     constexpr int BK = FormCfg<FORM>::BK;
@@ -578,8 +580,9 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
     constexpr int STAGES = Cfg<PAIR>::STAGES, STAGE_BYTES = Cfg<PAIR>::STAGE_BYTES, TILE_M = Cfg<PAIR>::TILE_M;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OPERAND_BYTES + EPI_BYTES);
-    // bars[0..S) full, bars[S..2S) empty, bars[2S] accumulators ready, bars[2S+1] accumulators drained
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2);
+    // bars[0..S) full, bars[S..2S) empty, bars[2S] accumulators ready, bars[2S+1] accumulators drained; DRAIN: these two of
+    // acc1, bars[2S+2] and bars[2S+3] of acc2
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -597,18 +600,11 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
     const long cta_idx = PAIR ? (long) (blockIdx.x >> 1) : (long) blockIdx.x;
     const long cta_cnt = PAIR ? (long) (gridDim.x >> 1) : (long) gridDim.x;
     const int row_off = PAIR ? (int) prank * BM : 0;
-    // up to two consecutive runs of (tile, k-block) units per CTA
-    long u_begin = cta_idx * p.units_per_cta;
+    // Whole tiles first, every cta_cnt-th (so that the CTAs work on neighbours at any time), then one run of (tile, k-block)
+    // units of those that are left.
+    const long left = (long) p.whole_per_cta * cta_cnt * k_blocks;
+    long u_begin = min(total_units, left + cta_idx * p.units_per_cta);
     long u_end = min(total_units, u_begin + p.units_per_cta);
-    long u2_begin = 0, u2_end = 0;
-    if (p.whole_per_cta > 0) {
-        const long lead = (long) p.whole_per_cta * k_blocks;             // whole tiles first ...
-        const long rest0 = lead * cta_cnt;                                // ... then a share of what is left
-        u2_begin = min(total_units, rest0 + cta_idx * p.units_per_cta);
-        u2_end = min(total_units, u2_begin + p.units_per_cta);
-        u_begin = lead * cta_idx;
-        u_end = u_begin + lead;
-    }
     if (p.segments > 0) {
         // Capped chains (K > 4096): consecutive CTAs take the SAME k-segment of consecutive tiles, so the CTAs that
         // run together read the same columns of A and B and share them through L2 (tile-major runs had every CTA
@@ -627,17 +623,24 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
         u_begin = tile * k_blocks + (long) k_blocks * crank / p.cluster;
         u_end = tile * k_blocks + (long) k_blocks * (crank + 1) / p.cluster;
     }
+    auto run_begin = [&](int r) { return r < p.whole_per_cta ? min(total_units, (cta_idx + r * cta_cnt) * k_blocks) : u_begin; };
+    auto run_end = [&](int r) { return r < p.whole_per_cta ? min(total_units, (cta_idx + r * cta_cnt + 1) * k_blocks) : u_end; };
     const uint32_t smem_base = smem_u32(smem);
     const uint32_t bar_base = smem_u32(bars);
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
     const uint32_t acc_full = bar_base + 8u * (2 * STAGES);
     const uint32_t acc_empty = bar_base + 8u * (2 * STAGES + 1);
+    const uint32_t acc2_full = bar_base + 8u * (2 * STAGES + 2), acc2_empty = bar_base + 8u * (2 * STAGES + 3);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         mbar_init(acc_full, 1);
-        mbar_init(acc_empty, (PAIR ? 2 : 1) * EPI_GROUPS);   // every epilogue group (pair: of both CTAs) hands the accumulators back
+        mbar_init(acc2_full, 1);
+        // every epilogue group, or (DRAIN) every one of their warps, hands the accumulators back; pair: of both CTAs
+        const uint32_t hands = (PAIR ? 2 : 1) * (DRAIN ? EPI_THREADS / 32 : EPI_GROUPS);
+        mbar_init(acc_empty, hands);
+        mbar_init(acc2_empty, hands);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -665,15 +668,28 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
     cnb_pdl_trigger();
     cnb_pdl_wait();
     CNB_GSTAMP(1, threadIdx.x == 0);
-    bool plain = false;                                  // known to the epilogue's warps
+    // Where the roles end, each in its own branch: behind a common end the registers of the smaller share would hold for
+    // both.  Every thread of every CTA reaches these barriers, also after a bounded wait gave up.  A pair's CTA neither
+    // leaves nor frees tensor memory while the other may still signal its barriers, read its shared memory (the first CTA's
+    // MMAs read the peer's operand stages) or write its tensor memory; with a K split all partial tiles are in shared memory.
+    auto finish = [&] {
+        __syncwarp();
+        asm volatile("barrier.cta.sync.aligned 0;" ::: "memory");
+        if (PAIR || split_cluster) cluster_sync();
+    };
 
+    // DRAIN: the epilogue's running sums want more registers than an equal share.  The shares change once: a group that took
+    // its own back could do so before the others have theirs.
+    constexpr int EPI_WARP = Threads<DRAIN>::FIRST_EPI / 32;
+    if (warp < EPI_WARP) {
+    if (DRAIN) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ISSUE_REGS));
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
             long it = 0;
             bool live = true;
-            for (int pass = 0; pass < 2 && live; ++pass)
-            for (long u = pass ? u2_begin : u_begin, ue = pass ? u2_end : u_end; u < ue; ++u, ++it) {
+            for (int r = 0; r <= p.whole_per_cta && live; ++r)
+            for (long u = run_begin(r), ue = run_end(r); u < ue; ++u, ++it) {
                 int tile = (int) (u / k_blocks), kb = (int) (u % k_blocks);
                 int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
                 int s = (int) (it % STAGES);
@@ -754,15 +770,22 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             // pair: M = 256 over the two CTAs
             const uint32_t m_bits = PAIR ? ((256u >> 4) << 24) - ((128u >> 4) << 24) : 0u;
             const uint32_t idesc = (kInstrDesc | mn_bits) + m_bits, idesc16 = (kInstrDesc16 | mn_bits) + m_bits;
-            for (int pass = 0; pass < 2; ++pass)
-            for (long u = pass ? u2_begin : u_begin, ue = pass ? u2_end : u_end; u < ue && ok; ++seg) {
+            // PACKED: one thread issues an MMA every 140 cycles; a descriptor is one addition to what is known here
+            const uint32_t idesch = (kInstrDescH | mn_bits) + m_bits;
+            const uint64_t a_desc = p.a_mn ? smem_desc_mn128_h(0) : smem_desc_sw64(0), b_desc = p.b_mn ? smem_desc_mn128_h(0) : smem_desc_sw64(0);
+            const uint32_t a_step = (p.a_mn ? 2048 : 32) >> 4, b_step = (p.b_mn ? 2048 : 32) >> 4;
+            for (int r = 0; r <= p.whole_per_cta; ++r)
+            for (long u = run_begin(r), ue = run_end(r); u < ue && ok; ++seg) {
                 int kb0 = (int) (u % k_blocks);
                 int kb1 = (int) min((long) k_blocks, kb0 + (ue - u));
                 if constexpr (DRAIN) kb1 = min(kb1, kb0 + p.chain);      // every chain is a segment of its own here
                 // the epilogue must have drained the previous segment's accumulators
-                ok = mbar_wait(acc_empty, (uint32_t) (seg & 1) ^ 1, abort_flag, p.status, 4);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                auto drained = [&](uint32_t bar) {
+                    const bool done = mbar_wait(bar, (uint32_t) (seg & 1) ^ 1, abort_flag, p.status, 4);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    return done;
+                };
+                if constexpr (!DRAIN) { ok = drained(acc_empty); if (!ok) break; }
                 for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
                     int s = (int) (it % STAGES);
                     uint32_t phase = (uint32_t) (it / STAGES) & 1;
@@ -773,38 +796,47 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                     uint32_t st = smem_base + s * STAGE_BYTES;
                     const uint32_t first = kb == kb0 ? 0u : 1u;
                     if constexpr (FORM == PACKED) {
-                        // high.low + low.high first, then high.high: a k-step of 16 at a time, or (DRAIN) the whole block
-                        // at a time, so that the small terms of a chain of one block meet a small accumulator (K = 50:
-                        // 1.5e-7 -> 1.1e-7 off float64, FMAs 1.3e-7)
-                        const uint32_t idesch = (kInstrDescH | mn_bits) + m_bits;
                         constexpr int b_low = PAIR ? 5 : 6;
-                        auto step = [&](int j, bool low, bool high) {
-                            const uint32_t ka = p.a_mn ? j * 2048 : j * 32, kbo = p.b_mn ? j * 2048 : j * 32;
-                            auto adesc = [&](int slot) {
-                                const uint32_t a = st + slot * PLANE_BYTES + ka;
-                                return p.a_mn ? smem_desc_mn128_h(a) : smem_desc_sw64(a);
-                            };
-                            auto bdesc = [&](int slot) {
-                                const uint32_t b = st + slot * PLANE_BYTES + kbo;
-                                return p.b_mn ? smem_desc_mn128_h(b) : smem_desc_sw64(b);
-                            };
-                            auto mma = [&](uint32_t acc, uint64_t a, uint64_t b, uint32_t add) {
-                                if constexpr (PAIR) umma2_bf16(acc, a, b, idesch, add); else umma_bf16(acc, a, b, idesch, add);
-                            };
-                            const uint64_t bh = bdesc(4), bl = bdesc(b_low);
-                            const uint32_t add = j == 0 ? first : 1u;
-                            if (low) { mma(tmem_base, adesc(2), bh, add); mma(tmem_base, adesc(0), bl, 1u); }
-                            if (high) mma(tmem_base, adesc(0), bh, 1u);
-                            if (low) { mma(tmem_base + 256, adesc(3), bh, add); mma(tmem_base + 256, adesc(1), bl, 1u); }
-                            if (high) mma(tmem_base + 256, adesc(1), bh, 1u);
+                        const uint32_t at = (st >> 4) & 0x3FFF;      // (in a cluster the CTA's rank stands above the offset)
+                        // term 0: low.high, 1: high.low, 2: high.high
+                        auto mma = [&](int j, int acc, int term) {
+                            const uint64_t ad = a_desc + (at + (term == 0 ? 2 + acc : acc) * (PLANE_BYTES >> 4) + j * a_step);
+                            const uint64_t bd = b_desc + (at + (term == 1 ? b_low : 4) * (PLANE_BYTES >> 4) + j * b_step);
+                            const uint32_t add = j == 0 && term == 0 ? first : 1u;
+                            if constexpr (PAIR) umma2_bf16(tmem_base + 256 * acc, ad, bd, idesch, add);
+                            else umma_bf16(tmem_base + 256 * acc, ad, bd, idesch, add);
                         };
+                        // DRAIN: at a chain's ends the accumulators take turns by the block: acc1 is summed up while acc2 of the
+                        // chain's last block is multiplied, acc2 while acc1 of the next chain's first block is.  Where runs
+                        // are cut the small terms of a block come first there, so that in a chain of one block they meet a
+                        // small accumulator (K = 50: 1.5e-7 -> 1.1e-7 off float64, FMAs 1.3e-7).
+                        const bool last = kb + 1 == kb1;
+                        if (DRAIN && (kb == kb0 || last)) {
 #pragma unroll
-                        for (int j = 0; j < BK / 16; ++j) step(j, true, !DRAIN);
-                        if constexpr (DRAIN) {
+                            for (int acc = 0; acc < 2; ++acc) {
+                                if (kb == kb0 && !drained(acc ? acc2_empty : acc_empty)) { ok = false; break; }
 #pragma unroll
-                            for (int j = 0; j < BK / 16; ++j) step(j, false, true);
+                                for (int j = 0; j < BK / 16; ++j) {
+                                    mma(j, acc, 0); mma(j, acc, 1);
+                                    if (!p.small_first) mma(j, acc, 2);
+                                }
+                                if (p.small_first) {
+#pragma unroll
+                                    for (int j = 0; j < BK / 16; ++j) mma(j, acc, 2);
+                                }
+                                if (acc == 1) { if constexpr (PAIR) umma2_commit_both(empty_bar(s), lead_rank); else umma_commit(empty_bar(s)); }
+                                if (last) {
+                                    const uint32_t bar = acc ? acc2_full : acc_full;
+                                    if constexpr (PAIR) umma2_commit_both(bar, lead_rank); else umma_commit(bar);
+                                }
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < BK / 16; ++j)
+#pragma unroll
+                                for (int acc = 0; acc < 2; ++acc) { mma(j, acc, 0); mma(j, acc, 1); mma(j, acc, 2); }
+                            if constexpr (PAIR) umma2_commit_both(empty_bar(s), lead_rank); else umma_commit(empty_bar(s));
                         }
-                        if constexpr (PAIR) umma2_commit_both(empty_bar(s), lead_rank); else umma_commit(empty_bar(s));
                         continue;
                     } else {
                     if constexpr (PAIR) {
@@ -870,17 +902,27 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                     umma_commit(empty_bar(s));       // the stage is free once these MMAs have read it
                     }
                 }
-                if (ok) { if constexpr (PAIR) umma2_commit_both(acc_full, lead_rank); else umma_commit(acc_full); }
+                if (ok && !DRAIN) { if constexpr (PAIR) umma2_commit_both(acc_full, lead_rank); else umma_commit(acc_full); }
                 CNB_GSTAMP(3, true);
                 u += kb1 - kb0;
             }
         }
+    }
+    finish();
+    if (split_cluster) cluster_sync();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    }
     } else {
         // -------------------------------------------------------------------- epilogue
+        bool plain = false;
+        if (DRAIN) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EPI_REGS));
         const int q = warp & 3;                      // TMEM lane quarter this warp may read
         const int row = q * 32 + lane;
-        const int group = (warp - 2) >> 2;           // the half of the columns this warp takes
-        const int et = ((warp - 2) & 3) * 32 + lane; // 0..127 within the epilogue group
+        const int group = (warp - EPI_WARP) >> 2;           // the half of the columns this warp takes
+        const int et = ((warp - EPI_WARP) & 3) * 32 + lane; // 0..127 within the epilogue group
         const uint32_t tl = tmem_base + ((uint32_t) (q * 32) << 16);
         const float sgn = p.conjB ? 1.f : -1.f;
         // PACKED: the scales of both operands are taken out again, in two factors so that neither leaves fp32's range
@@ -903,18 +945,24 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
 #pragma unroll
                 for (int i = 0; i < 64; ++i) sr[i] = si[i] = 0.f;
                 for (int done = 0; done < blocks; done += p.chain, ++seg) {
-                    mbar_wait(acc_full, (uint32_t) seg & 1, abort_flag, p.status, 3);
-                    epi_bar_sync(group);
-                    if (*abort_flag) return false;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    drain_chain(tl + group * 64, sgn, sr, si);
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    epi_bar_sync(group);
-                    if (et == 0) {
-                        if constexpr (PAIR) mbar_arrive_cluster(map_to_rank(acc_empty, lead_rank));
-                        else mbar_arrive(acc_empty);
-                    }
+                    // every warp by itself; after a wait gave up the others end at once
+                    auto sum = [&](auto acc, uint32_t full, uint32_t empty) {
+                        mbar_wait(full, (uint32_t) seg & 1, abort_flag, p.status, 3);
+                        __syncwarp();
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        drain_chain<decltype(acc)::value>(tl + group * 64, sgn, sr, si);
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) {
+                            if constexpr (PAIR) mbar_arrive_cluster(map_to_rank(empty, lead_rank));
+                            else mbar_arrive(empty);
+                        }
+                    };
+                    sum(std::integral_constant<int, 0>(), acc_full, acc_empty);
+                    sum(std::integral_constant<int, 1>(), acc2_full, acc2_empty);
                 }
+                epi_bar_sync(group);                 // everyone arrives, then agree on the outcome
+                if (*abort_flag) return false;
             }
             return true;
         };
@@ -966,8 +1014,8 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             u_end = u_begin;                             // nothing left for the loop below
         }
         bool live = true;
-        for (int pass = 0; pass < 2 && live; ++pass)
-        for (long u = pass ? u2_begin : u_begin, ue = pass ? u2_end : u_end; u < ue; seg += DRAIN ? 0 : 1) {
+        for (int r = 0; r <= p.whole_per_cta && live; ++r)
+        for (long u = run_begin(r), ue = run_end(r); u < ue; seg += DRAIN ? 0 : 1) {
             int tile = (int) (u / k_blocks), kb0 = (int) (u % k_blocks);
             int kb1 = (int) min((long) k_blocks, kb0 + (ue - u));
             int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
@@ -982,9 +1030,8 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             }
             // What a round adds from global memory (the residual if there is one, else old D) is requested a round
             // ahead, the first one's under the MMAs: asked for in the round itself it doubled the round's time, and
-            // asked for between the stores each load would wait for the store before it.  (DRAIN: half a round at a time,
-            // and not ahead; the registers hold the running sums.)
-            constexpr int U = DRAIN ? 2 : 4;
+            // asked for between the stores each load would wait for the store before it.
+            constexpr int U = 4;
             float4 gr[U], gi[U];
             auto request = [&](int c0, int h) {
                 const float* xr = add_res ? p.r_re : p.d_re;
@@ -1001,7 +1048,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                 }
             };
             const int c_first = group * 64, c_last = c_first + 48;
-            if (!DRAIN && pre) request(c_first, 0);
+            if (pre) request(c_first, 0);
             if constexpr (DRAIN) {
                 if (!sum_chains(kb1 - kb0)) { live = false; break; }
             } else {
@@ -1051,7 +1098,6 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
 #pragma unroll
                     for (int h = 0; h < 4; h += U) {
                         float4 vr[U], vi[U];
-                        if (DRAIN && pre) request(c0, h);
 #pragma unroll
                         for (int j = 0; j < U; ++j) {
                             const int idx = et + 128 * (h + j);
@@ -1065,7 +1111,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                                 vr[j].x += gr[j].x; vr[j].y += gr[j].y; vr[j].z += gr[j].z; vr[j].w += gr[j].w;
                                 vi[j].x += gi[j].x; vi[j].y += gi[j].y; vi[j].z += gi[j].z; vi[j].w += gi[j].w;
                             }
-                            if (!DRAIN && c0 != c_last) request(c0 + 16, 0);
+                            if (c0 != c_last) request(c0 + 16, 0);
                         }
 #pragma unroll
                         for (int j = 0; j < U; ++j) {
@@ -1124,38 +1170,25 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             u += kb1 - kb0;
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    }
-    __syncthreads();
-    if (PAIR && !split_cluster) {
-        // No CTA of the pair leaves (or frees tensor memory) while the other may still signal its barriers, read its
-        // shared memory (the first CTA's MMAs read the peer's operand stages) or write its tensor memory.  Every thread
-        // reaches this barrier, also after a bounded wait gave up.  (With a K split the two barriers below do that.)
-        cluster_sync();
-    }
-    if (split_cluster) {
-        // Every thread of every CTA of the cluster reaches both barriers, also after a bounded wait gave up.
-        cluster_sync();                                  // all partial tiles are in shared memory
-        CNB_GSTAMP(6, threadIdx.x == 64);
-        if (warp >= 2 && !plain && !*abort_flag) {
-            const int tile = blockIdx.x / cluster_ctas;
-            const int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
-            const int et = (warp - 2) * 32 + lane;
-            const uint32_t peer0 = PAIR ? prank : 0u, peer_step = PAIR ? 2u : 1u;
-            switch (p.cluster) {
-                case 2: cluster_reduce<2, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
-                case 4: cluster_reduce<4, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
-                default: cluster_reduce<8, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+        finish();
+        if (split_cluster) {
+            CNB_GSTAMP(6, threadIdx.x == Threads<DRAIN>::FIRST_EPI);
+            if (!plain && !*abort_flag) {
+                const int tile = blockIdx.x / cluster_ctas;
+                const int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
+                const int et = (warp - EPI_WARP) * 32 + lane;
+                const uint32_t peer0 = PAIR ? prank : 0u, peer_step = PAIR ? 2u : 1u;
+                switch (p.cluster) {
+                    case 2: cluster_reduce<2, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+                    case 4: cluster_reduce<4, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+                    default: cluster_reduce<8, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+                }
             }
+            CNB_GSTAMP(7, threadIdx.x == Threads<DRAIN>::FIRST_EPI);
+            cluster_sync();                              // no CTA leaves while a peer still reads its shared memory
+            CNB_GSTAMP(8, threadIdx.x == Threads<DRAIN>::FIRST_EPI);
         }
-        CNB_GSTAMP(7, threadIdx.x == 64);
-        cluster_sync();                                  // no CTA leaves while a peer still reads its shared memory
-        CNB_GSTAMP(8, threadIdx.x == 64);
-    }
-    if (FORM == PACKED && plain) fma_product(p, smem);   // shared memory is idle: every chain has been read out
-    if (warp == 1) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
-        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+        if (FORM == PACKED && plain) fma_product(p, smem);   // shared memory is idle: every chain has been read out
     }
 }
 
@@ -1467,7 +1500,10 @@ __global__ void zero_pair_k(float* __restrict__ a, float* __restrict__ b, size_t
 
 // The schedule of one product: which form (one CTA per tile or CTA pairs), how many CTAs, how the (tile, k-block)
 // units are dealt.  Host arithmetic only (also reachable as cnb_gemm_schedule, for tests that need no GPU).
-struct Schedule { bool pair; long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles; };
+struct Schedule { bool pair; long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles, joined; };
+
+// The longest chain of a product with K > 4096, in k-blocks of 16 (see choose_schedule).
+constexpr int kMaxChain16 = 64;
 
 // Depths below are counted in blocks of 16 and scaled to the form's own (bk = 16 or 32).
 Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int bk) {
@@ -1480,8 +1516,9 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
     //    and only the remainder needs atomics and a cleared output;
     //  * few tiles and short runs: a cluster per tile (below); otherwise plain stream-K.
     // K > 4096 keeps to stream-K runs: one fp32 accumulation chain in tensor memory that long costs accuracy.
-    struct Plan { long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles; };
+    struct Plan { long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles, joined; };
     const int k_blocks = (K + bk - 1) / bk;
+    const bool packed = bk == FormCfg<PACKED>::BK;
     auto blocks = [&](int of16) { return (long) std::max(1, of16 * 16 / bk); };
     auto plan = [&](bool pair) {
         Plan q = {};
@@ -1515,15 +1552,40 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
         // outside, in fp32 round-to-nearest): several equal waves of CTAs instead of one persistent wave.
         // Only K > 4096 gets here with longer runs; a whole tile of K <= 4096 is at most 256 k-blocks.  Each tile is
         // cut into equal segments and the CTAs are numbered segment-major (see the kernel).
-        const long kMaxChain = blocks(64);
-        if (!whole_tiles && upc > kMaxChain && k_blocks > blocks(256)) {
+        // (packed operands: the running sums in registers cut the chains, whatever the run)
+        const long kMaxChain = blocks(kMaxChain16);
+        if (packed && !whole_tiles && upc > kMaxChain && k_blocks > blocks(256)) {
+            // As few segments as cost least: waves of runs, and what a run costs beside its k-blocks (start, write-out) as
+            // about 9 of them, the cleared output and the atomics as another 5.
+            long best = 0;
+            for (int c = 1; (c - 1) * kMaxChain < k_blocks; ++c) {
+                const long cost = ((long) tiles * c + sms - 1) / sms * ((k_blocks + c - 1) / c + 9) + (c > 1 ? 5 : 0);
+                if (best == 0 || cost < best) { best = cost; q.segments = c; }
+            }
+            upc = (k_blocks + q.segments - 1) / q.segments;
+            ctas = (long) tiles * q.segments;
+            if (q.segments == 1) {
+                q.segments = 0;
+                upc = 0;
+                ctas = std::min<long>(tiles, sms);
+                q.whole_per_cta = (int) ((tiles + ctas - 1) / ctas);
+            }
+        } else if (!whole_tiles && upc > kMaxChain && k_blocks > blocks(256)) {
             q.segments = (int) ((k_blocks + kMaxChain - 1) / kMaxChain);     // per tile, each at most kMaxChain k-blocks
             upc = (k_blocks + q.segments - 1) / q.segments;
             ctas = (long) tiles * q.segments;
         } else {
             ctas = (total + upc - 1) / upc;
         }
-        if (lead_whole) {
+        if (packed && tiles > sms && (whole_tiles || (lead_whole && tiles % sms * 10 >= sms * 7))) {
+            // Whole tiles by CTAs that stay: the write-out of one runs under the MMAs of the next.  Also where a remainder
+            // of tiles, nearly a wave of them, would be shared: no cleared output and no atomics (4096 x 1024 x 1024, 128
+            // tiles on 74 pairs: 76 -> 71 us; step of the 4096-row stack 3000 -> 2920).
+            ctas = sms;
+            upc = 0;
+            q.whole_per_cta = (tiles + sms - 1) / sms;
+            q.joined = lead_whole;
+        } else if (lead_whole) {
             ctas = sms;
             q.whole_per_cta = tiles / sms;
             const long rest = (long) (tiles - q.whole_per_cta * sms) * k_blocks;
@@ -1536,7 +1598,7 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
         // Worth it while a stream-K run would be short (<= 48 k-blocks): with long runs the atomics are
         // amortised and using every SM wins over the clusters' rounded-down CTA count.
         q.cluster = 1;
-        if (!whole_tiles && !lead_whole && upc <= blocks(48)) {
+        if (!whole_tiles && q.whole_per_cta == 0 && upc <= blocks(48)) {
             // pairs: two slices at most (clusters of 8 CTAs do not all fit a GPC side by side: measured 0.043 ms
             // against 0.025 at 512 x 1024 x 1024)
             for (int c = pair ? 2 : 8; c >= 2; c >>= 1)
@@ -1547,7 +1609,7 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
             if (q.cluster > 1 && k_blocks / q.cluster > 2 * upc + blocks(16)) q.cluster = 1;
         }
         if (q.cluster > 1) { ctas = (long) tiles * q.cluster; upc = 0; }
-        q.splits_tiles = q.cluster == 1 && (lead_whole ? upc > 0 : (q.segments > 0 || (upc % k_blocks) != 0));
+        q.splits_tiles = q.cluster == 1 && (q.whole_per_cta > 0 ? upc > 0 : (q.segments > 0 || (upc % k_blocks) != 0));
         q.ctas = ctas; q.upc = upc;
         return q;
     };
@@ -1569,7 +1631,7 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
     }
     Schedule r;
     r.pair = pair; r.ctas = q.ctas; r.upc = q.upc; r.whole_per_cta = q.whole_per_cta; r.clear_from_row = q.clear_from_row;
-    r.cluster = q.cluster; r.segments = q.segments; r.splits_tiles = q.splits_tiles;
+    r.cluster = q.cluster; r.segments = q.segments; r.splits_tiles = q.splits_tiles; r.joined = q.joined;
     return r;
 }
 
@@ -1586,6 +1648,18 @@ static bool split_sizes(int M, int N, int K) { return K % 8 == 0 && K >= 32 && M
 // rounded FMAs over K products by 1.8e-8 sqrt(K), and a sum of chains rounded to nearest by what one chain is.  So a chain
 // may be 4.28 sqrt(K) long, in blocks of 32.
 static int max_chain(int K) { return std::max(1, (int) (4.28 * std::sqrt((double) K) / FormCfg<PACKED>::BK)); }
+
+// The chain of a packed product in k-blocks of 32.  At sizes that were split products, whole tiles of K <= 4096 are one
+// chain; a longer K is cut at choose_schedule's cap, and whole tiles that used to be shared runs (`joined`) at 24, shorter
+// than those were (4096 x 1024 x 1024, two chains of 16: 1.8e-6 off float64, was 3.1e-6; a chain costs a 4096-row training
+// step 1 %).
+static int chain_blocks(int M, int N, int K, bool joined) {
+    if (!split_sizes(M, N, K)) return max_chain(K);
+    const int k_blocks = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK;
+    const int most = K > 4096 ? kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK : joined ? 24 : k_blocks;
+    const int chains = (k_blocks + most - 1) / most;
+    return (k_blocks + chains - 1) / chains;
+}
 
 bool cgemm_tc_shape_ok(int M, int N, int K) {
     if (split_sizes(M, N, K)) return true;
@@ -1627,6 +1701,13 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     } while (0)
         CNB_TC_ATTR(SPLIT, false); CNB_TC_ATTR(PACKED, false); CNB_TC_ATTR(PACKED, true);
 #undef CNB_TC_ATTR
+        cudaFuncAttributes fa[4];                        // the shares of a DRAIN launch must add up to what it starts with
+        CNB_CUDA(cudaFuncGetAttributes(&fa[0], cgemm_tc_k<false, false, PACKED, true>));
+        CNB_CUDA(cudaFuncGetAttributes(&fa[1], cgemm_tc_k<false, true, PACKED, true>));
+        CNB_CUDA(cudaFuncGetAttributes(&fa[2], cgemm_tc_k<true, false, PACKED, true>));
+        CNB_CUDA(cudaFuncGetAttributes(&fa[3], cgemm_tc_k<true, true, PACKED, true>));
+        for (const cudaFuncAttributes& f : fa)
+            if (f.numRegs < LAUNCH_REGS) return set_error(CNB_ERR_CUDA, "cgemm_tc: built with %d registers a thread, not %d", f.numRegs, LAUNCH_REGS);
         attr_set[ctx->device & 63] = true;
     }
     if ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im)) & 3)
@@ -1691,14 +1772,17 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     p.status = ctx->d_status;
     const bool vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im) |
                                      reinterpret_cast<uintptr_t>(r_re) | reinterpret_cast<uintptr_t>(r_im)) & 15) == 0;
-    auto go = [&](auto kernel, const auto& maps) {
-        return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(NUM_THREADS), SMEM_BYTES, st, pair ? 2 * cluster : cluster, maps, p);
-    };
     // the longest run of k-blocks that one CTA sums for a tile
     const int k_blocks = (K + bk - 1) / bk;
     const int run = cluster > 1 ? (k_blocks + cluster - 1) / cluster : q.whole_per_cta > 0 ? k_blocks : (int) std::min<long>(q.upc, k_blocks);
-    p.chain = max_chain(K);
-    const bool drain = packed && !split_sizes(M, N, K) && run > p.chain;
+    p.chain = chain_blocks(M, N, K, q.joined);
+    p.small_first = run > p.chain;
+    const bool several = cluster == 1 && q.segments == 0 && (q.whole_per_cta > 0 || q.upc != k_blocks);     // tiles a CTA
+    const bool drain = packed && (run > p.chain || several);
+    auto go = [&](auto kernel, const auto& maps) {
+        return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(drain ? Threads<true>::ALL : Threads<false>::ALL), SMEM_BYTES, st,
+                           pair ? 2 * cluster : cluster, maps, p);
+    };
     cudaError_t e;
 #define CNB_TC_GO(F, D, maps)                                                                                              \
     (pair ? (vec ? go(cgemm_tc_k<true, true, F, D>, maps) : go(cgemm_tc_k<true, false, F, D>, maps))                       \
@@ -1792,9 +1876,11 @@ static int schedule_of(int M, int N, int K, int accumulate, int sm_count, int sm
     out8[0] = q.pair ? 1 : 0;
     out8[1] = (int) (q.pair ? 2 * q.ctas : q.ctas);      // CTAs of the launch
     out8[2] = q.cluster * (q.pair ? 2 : 1);              // CTAs per cluster (1: no cluster)
-    out8[3] = (int) q.upc;
+    const int chain = kMaxChain16 * FormCfg<SPLIT>::BK / bk;
+    const bool cut = q.segments > 0 && q.upc > chain;        // packed: a segment is several chains
+    out8[3] = (int) (cut ? chain : q.upc);
     out8[4] = q.whole_per_cta;
-    out8[5] = q.segments;
+    out8[5] = cut ? q.segments * (int) ((q.upc + chain - 1) / chain) : q.segments;
     out8[6] = q.splits_tiles ? 1 : 0;
     out8[7] = q.clear_from_row;
     return CNB_OK;
