@@ -1314,47 +1314,67 @@ __global__ void __launch_bounds__(256) pack_max_k(const __grid_constant__ PackJo
     }
 }
 
+// Small matrices (those of a 512-row batch, 4 MB) are a chain of round trips: the head, then the data.  What a thread converts
+// first is requested before the head is read, and the head is given back at the end.
 template <int N>
 __global__ void __launch_bounds__(256) pack_k(const __grid_constant__ PackJobs<N> jobs) {
     cnb_pdl_enter();
     const PackJob& job = jobs.j[blockIdx.y];
     if ((int) blockIdx.x >= job.blocks) return;
-    __shared__ int s_exp;
-    if (threadIdx.x == 0) {
-        const int e = pack_exponent(__ldcg(&job.head->max_bits), __ldcg(&job.head->low_bits));
-        s_exp = e;
-        if (blockIdx.x == 0) job.head->exponent = e;
-        __threadfence();
-        if (atomicAdd(&job.head->ticket, 1u) == (unsigned) job.blocks - 1) {      // every block has read it: ready for the next use
-            job.head->max_bits = 0;
-            job.head->low_bits = 0;
-            job.head->ticket = 0;
-        }
-    }
-    __syncthreads();
-    const bool plain = s_exp == kPlain;
-    const float scale = plain ? 1.f : __uint_as_float((unsigned) (s_exp + 127) << 23);
-    float* const plain_dst = reinterpret_cast<float*>(job.dst);
     // Consecutive threads take consecutive columns: four each where the rows allow 16-byte loads (8-byte stores), else
     // two (4-byte accesses), so that every access of a warp is one run.
     const bool vec = pack_vec(job);
     const size_t np = (size_t) job.rows * job.pitch;
     const int groups = vec ? job.cols / 4 : (job.cols + 1) / 2;
     const size_t total = (size_t) job.rows * groups;
+    // rows without padding are one run; else a 32-bit division where it does (a 64-bit one was half the kernel's time)
+    const bool flat = vec && job.pitch == job.cols;
+    struct Item { float4 x, y; size_t dst; };
+    auto fetch = [&](size_t i) {
+        Item v;
+        const int row = flat ? 0 : total >> 32 ? (int) (i / groups) : (int) ((unsigned) i / (unsigned) groups);
+        const int g = (int) (i - (size_t) row * groups);
+        if (vec) {
+            const size_t src = flat ? 4 * i : (size_t) row * job.cols + 4 * g;
+            v.dst = flat ? 4 * i : (size_t) row * job.pitch + 4 * g;
+            v.x = *reinterpret_cast<const float4*>(job.re + src);
+            v.y = *reinterpret_cast<const float4*>(job.im + src);
+        } else {
+            const int c = 2 * g;
+            const bool two = c + 1 < job.cols;
+            const size_t src = (size_t) row * job.cols + c;
+            v.dst = (size_t) row * job.pitch + c;
+            v.x = make_float4(job.re[src], two ? job.re[src + 1] : 0.f, 0.f, 0.f);
+            v.y = make_float4(job.im[src], two ? job.im[src + 1] : 0.f, 0.f, 0.f);
+        }
+        return v;
+    };
+    const size_t stride = (size_t) job.blocks * 256;
+    size_t i = (size_t) blockIdx.x * 256 + threadIdx.x;
+    Item item = {};
+    if (i < total) item = fetch(i);
+    __shared__ int s_exp;
+    if (threadIdx.x == 0) {
+        const int e = pack_exponent(__ldcg(&job.head->max_bits), __ldcg(&job.head->low_bits));
+        s_exp = e;
+        if (blockIdx.x == 0) job.head->exponent = e;
+    }
+    __syncthreads();
+    const bool plain = s_exp == kPlain;
+    const float scale = plain ? 1.f : __uint_as_float((unsigned) (s_exp + 127) << 23);
+    float* const plain_dst = reinterpret_cast<float*>(job.dst);
     auto part = [&](float a, float b, __half2* hi, __half2* lo) {
         a *= scale; b *= scale;
         *hi = __floats2half2_rn(a, b);
         const float2 f = __half22float2(*hi);
         *lo = __floats2half2_rn(a - f.x, b - f.y);
     };
-    for (size_t i = (size_t) blockIdx.x * 256 + threadIdx.x; i < total; i += (size_t) job.blocks * 256) {
-        // rows without padding are one run; else a 32-bit division where it does (a 64-bit one was half the kernel's time)
-        const bool flat = vec && job.pitch == job.cols;
-        const int row = flat ? 0 : total >> 32 ? (int) (i / groups) : (int) ((unsigned) i / (unsigned) groups);
-        const int g = (int) (i - (size_t) row * groups);
+    while (i < total) {
+        const float4 x = item.x, y = item.y;
+        const size_t dst = item.dst;
+        i += stride;
+        if (i < total) item = fetch(i);                  // the next one, before this one's stores
         if (vec) {
-            const size_t src = flat ? 4 * i : (size_t) row * job.cols + 4 * g, dst = flat ? 4 * i : (size_t) row * job.pitch + 4 * g;
-            const float4 x = *reinterpret_cast<const float4*>(job.re + src), y = *reinterpret_cast<const float4*>(job.im + src);
             if (plain) {
                 *reinterpret_cast<float4*>(plain_dst + dst) = x;
                 *reinterpret_cast<float4*>(plain_dst + np + dst) = y;
@@ -1368,24 +1388,25 @@ __global__ void __launch_bounds__(256) pack_k(const __grid_constant__ PackJobs<N
             *reinterpret_cast<uint2*>(job.dst + np + dst) = *reinterpret_cast<uint2*>(hi);
             *reinterpret_cast<uint2*>(job.dst + 3 * np + dst) = *reinterpret_cast<uint2*>(lo);
         } else {
-            const int c = 2 * g;
-            const bool two = c + 1 < job.cols;
-            const size_t src = (size_t) row * job.cols + c, dst = (size_t) row * job.pitch + c;
-            const float x0 = job.re[src], y0 = job.im[src];
-            const float x1 = two ? job.re[src + 1] : 0.f, y1 = two ? job.im[src + 1] : 0.f;
             if (plain) {
-                *reinterpret_cast<float2*>(plain_dst + dst) = make_float2(x0, x1);
-                *reinterpret_cast<float2*>(plain_dst + np + dst) = make_float2(y0, y1);
+                *reinterpret_cast<float2*>(plain_dst + dst) = make_float2(x.x, x.y);
+                *reinterpret_cast<float2*>(plain_dst + np + dst) = make_float2(y.x, y.y);
                 continue;
             }
             __half2 hi, lo;
-            part(x0, x1, &hi, &lo);
+            part(x.x, x.y, &hi, &lo);
             *reinterpret_cast<__half2*>(job.dst + dst) = hi;
             *reinterpret_cast<__half2*>(job.dst + 2 * np + dst) = lo;
-            part(y0, y1, &hi, &lo);
+            part(y.x, y.y, &hi, &lo);
             *reinterpret_cast<__half2*>(job.dst + np + dst) = hi;
             *reinterpret_cast<__half2*>(job.dst + 3 * np + dst) = lo;
         }
+    }
+    // every block has read the head (this one's thread 0 before the barrier above): the last one makes it ready for the next use
+    if (threadIdx.x == 0 && atomicAdd(&job.head->ticket, 1u) == (unsigned) job.blocks - 1) {
+        job.head->max_bits = 0;
+        job.head->low_bits = 0;
+        job.head->ticket = 0;
     }
 }
 

@@ -290,18 +290,32 @@ int cnb_linear_bwd_w_packed(cnb_ctx* ctx, const void* g_pack, const void* x_pack
 }
 
 /* the update of a weight arena, then its packed matrices */
+static int span_requests(const float* w, size_t n, const cnb_pack_span* spans, int nspans, const char* who, std::vector<cnb::PackRequest>* r) {
+    for (int k = 0; k < nspans; ++k) {
+        const cnb_pack_span& s = spans[k];
+        const size_t count = s.rows > 0 && s.cols > 0 ? (size_t) s.rows * s.cols : 0;
+        CNB_CHECK_ARG(count > 0 && count <= n && s.pack && s.re <= n - count && s.im <= n - count, "%s: matrix %d is not inside the arena", who, k);
+        r->push_back(pack_of(w + s.re, w + s.im, s.pack, s.rows, s.cols));
+    }
+    return CNB_OK;
+}
+
 int cnb_sgd_update_packed(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, int zero_grad, const cnb_pack_span* spans,
                           int nspans, void* stream) {
     CNB_CHECK_ARG(ctx && w && g && n > 0 && nspans >= 0 && (nspans == 0 || spans), "cnb_sgd_update_packed: bad argument");
     std::vector<cnb::PackRequest> r;
-    for (int k = 0; k < nspans; ++k) {
-        const cnb_pack_span& s = spans[k];
-        const size_t count = s.rows > 0 && s.cols > 0 ? (size_t) s.rows * s.cols : 0;
-        CNB_CHECK_ARG(count > 0 && count <= n && s.pack && s.re <= n - count && s.im <= n - count,
-                      "cnb_sgd_update_packed: matrix %d is not inside the arena", k);
-        r.push_back(pack_of(w + s.re, w + s.im, s.pack, s.rows, s.cols));
-    }
-    const int rc = cnb_sgd_update(ctx, w, g, n, lr, zero_grad, stream);
+    int rc = span_requests(w, n, spans, nspans, "cnb_sgd_update_packed", &r);
+    if (rc == CNB_OK) rc = cnb_sgd_update(ctx, w, g, n, lr, zero_grad, stream);
+    if (rc != CNB_OK || nspans == 0) return rc;
+    return cnb::pack(ctx, r.data(), nspans, cnb::S(stream));
+}
+
+int cnb_adam_update_packed(cnb_ctx* ctx, float* w, float* m, float* g, size_t n, float lr, float beta, int t,
+                           const cnb_pack_span* spans, int nspans, void* stream) {
+    CNB_CHECK_ARG(ctx && w && m && g && n > 0 && nspans >= 0 && (nspans == 0 || spans), "cnb_adam_update_packed: bad argument");
+    std::vector<cnb::PackRequest> r;
+    int rc = span_requests(w, n, spans, nspans, "cnb_adam_update_packed", &r);
+    if (rc == CNB_OK) rc = cnb_adam_update(ctx, w, m, g, n, lr, beta, t, stream);
     if (rc != CNB_OK || nspans == 0) return rc;
     return cnb::pack(ctx, r.data(), nspans, cnb::S(stream));
 }

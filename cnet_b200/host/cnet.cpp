@@ -1228,24 +1228,32 @@ void CNet::updateInputs(float lr) {
 	if (!ctx_ || !wgrad_count_) return;
 	if (dp_gemm_ctas_ > 0) cnb_set_gemm_sm_limit(ctx_, 0);
 	if (!joinCollectives()) return;
-	// the new Linear weights leave the update already packed, once, for the next forward and dX* products
+	std::vector<Linear*> packed;
+	const std::vector<cnb_pack_span> spans = packSpans(&packed);
+	const int rc = cnb_sgd_update_packed(ctx_, weight_base_, wgrad_base_, wgrad_count_, lr, 1, spans.data(), (int) spans.size(), stream_);
+	if (rc != CNB_OK) { fail(rc, "updateInputs"); return; }
+	weightsUpdated(packed);
+}
+
+// The Linear weights leave an update already packed, once, for the next forward and dX* products: all that lie in the weight
+// arena by the update's own launches.
+std::vector<cnb_pack_span> CNet::packSpans(std::vector<Linear*>* packed) const {
 	std::vector<cnb_pack_span> spans;
-	std::vector<Linear*> fused;
 	for (auto f : func_list_) {
 		Linear* l = dynamic_cast<Linear*>(f);
 		if (!l || !l->x_pack_) continue;
 		const Vars& w = l->prev_func_[1]->out_;
 		if (w.real_ < weight_base_ || w.imag_ + l->in2_len > weight_base_ + wgrad_count_) continue;
 		spans.push_back({(size_t) (w.real_ - weight_base_), (size_t) (w.imag_ - weight_base_), l->out_size_, l->in1_len, l->w_pack_});
-		fused.push_back(l);
+		packed->push_back(l);
 	}
-	int rc = spans.empty()
-		? cnb_sgd_update(ctx_, weight_base_, wgrad_base_, wgrad_count_, lr, 1, stream_)
-		: cnb_sgd_update_packed(ctx_, weight_base_, wgrad_base_, wgrad_count_, lr, 1, spans.data(), (int) spans.size(), stream_);
-	if (rc != CNB_OK) { fail(rc, "updateInputs"); return; }
+	return spans;
+}
+
+void CNet::weightsUpdated(const std::vector<Linear*>& packed) {
 	reduced_since_update_ = false;
 	++weights_version_;
-	for (auto l : fused) l->w_pack_version_ = weights_version_;
+	for (auto l : packed) l->w_pack_version_ = weights_version_;
 	for (auto f : func_list_)
 		if (Linear* l = dynamic_cast<Linear*>(f))
 			if (l->w_pack_version_ != weights_version_) l->packWeights();
@@ -1267,12 +1275,11 @@ void CNet::adamUpdate(float lr, float beta, int t) {
 		momentum_base_ = static_cast<float*>(p);
 		cnb_memset0(ctx_, momentum_base_, wgrad_count_ * sizeof(float), stream_);
 	}
-	int rc = cnb_adam_update(ctx_, weight_base_, momentum_base_, wgrad_base_, wgrad_count_, lr, beta, t, stream_);
+	std::vector<Linear*> packed;
+	const std::vector<cnb_pack_span> spans = packSpans(&packed);
+	const int rc = cnb_adam_update_packed(ctx_, weight_base_, momentum_base_, wgrad_base_, wgrad_count_, lr, beta, t, spans.data(), (int) spans.size(), stream_);
 	if (rc != CNB_OK) { fail(rc, "adamUpdate"); return; }
-	reduced_since_update_ = false;
-	++weights_version_;
-	for (auto f : func_list_)
-		if (Linear* l = dynamic_cast<Linear*>(f)) l->packWeights();
+	weightsUpdated(packed);
 }
 
 void CNet::infer() {

@@ -421,6 +421,8 @@ class CNet {
 	void* ev_sym_fork_ = nullptr;
 	void* ev_sym_join_ = nullptr;
 	bool joinCollectives();                         // the compute stream waits for every collective in flight
+	std::vector<cnb_pack_span> packSpans(std::vector<Linear*>* packed) const;
+	void weightsUpdated(const std::vector<Linear*>& packed);
 	void* graph_exec_ = nullptr;                    // cudaGraphExec_t of a captured step
 	bool capturing_ = false;
 	unsigned long long graph_launches_ = 0;         // kernels inside the captured step

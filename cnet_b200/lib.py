@@ -57,6 +57,7 @@ SIGNATURES = {
     "cnb_dft_hadamard_gelu_fwd_packed": (C.c_int, [_vp] + [_P] * 9 + [C.c_int] * 2 + [_vp]),
     "cnb_dft_keeps_product": (C.c_int, [C.c_int]),
     "cnb_dft_hadamard_gelu_fwd_keep": (C.c_int, [_vp] + [_P] * 11 + [C.c_int] * 2 + [_vp]),
+    "cnb_adam_update_packed": (C.c_int, [_vp, _P, _P, _P, _sz, C.c_float, C.c_float, C.c_int, _vp, C.c_int, _vp]),
     "cnb_sgd_update_packed": (C.c_int, [_vp, _P, _P, _sz, C.c_float, C.c_int, _vp, C.c_int, _vp]),
     "cnb_set_gemm_sm_limit": (C.c_int, [_vp, C.c_int]),
     "cnb_last_gemm_engine": (C.c_int, []),

@@ -359,6 +359,9 @@ int cnb_sgd_update_packed(cnb_ctx* ctx, float* w, float* g, size_t n, float lr, 
  * CPU: impl/cfunc.h:273-287 + impl/cnet.h:423-431. */
 int cnb_adam_update(cnb_ctx* ctx, float* w, float* m, float* g, size_t n, float lr, float beta, int t,
                     void* stream);
+/* The same, after which the given matrices lie packed, as cnb_sgd_update_packed leaves them. */
+int cnb_adam_update_packed(cnb_ctx* ctx, float* w, float* m, float* g, size_t n, float lr, float beta, int t,
+                           const cnb_pack_span* spans, int nspans, void* stream);
 
 /* ------------------------------------------------------------- data parallelism
  * Sum of `count` floats at `local` over the ranks of one NVSwitch domain, in place, by this library's own kernel
