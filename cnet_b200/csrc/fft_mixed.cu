@@ -5,7 +5,7 @@
 // with L = the product of the radices before it reads x[j + q N/R], multiplies by e^{-2 pi i (j % L) q / (L R)},
 // transforms over q and writes (j / L) L R + j % L + q L, so the last pass comes out in natural order.  The first
 // pass reads the planes and the last one writes them (consecutive threads, consecutive elements); the passes between
-// go through shared memory, whose elements are spread by one in every 16 against bank conflicts.
+// go through shared memory, whose elements are spread by one in every 16 against bank conflicts where that helps (choose_spread).
 //
 // Lengths with a prime factor above 13 use the chirp form (Bluestein): X[k] = c[k] sum_n (x[n] c[n]) conj(c[k-n]),
 // c[n] = e^{-pi i n^2 / N}, the convolution as two transforms of a length M >= 2N-1 that factors well, in the same
@@ -40,12 +40,15 @@ struct Pass {
 struct MixedPlan {
     int n, m;                         // row length; transform length (m > n: chirp form)
     int passes, rows, threads, stride; // rows per CTA; float2 per row of a buffer
-    int buffers;
+    int buffers, shift;               // shift: spread of the buffers' rows, 4 or NO_SPREAD
     Pass p[MAX_PASSES];
     float scale;
 };
 
-__host__ __device__ __forceinline__ int pad_of(int i) { return i + (i >> 4); }
+// Where element i of a row lies in a buffer: every 16th set one further (shift 4), or as it is.  Constants of the kernel: a
+// shift read from the plan cost every length 1 to 3 %.
+constexpr int SPREAD = 4, NO_SPREAD = 31;
+template <int SHIFT> __host__ __device__ __forceinline__ int pad_of(int i) { return i + (SHIFT == NO_SPREAD ? 0 : i >> SHIFT); }
 
 __device__ __forceinline__ int div_by(int i, unsigned mag) { return mag ? (int) __umulhi((unsigned) i, mag) : i; }
 
@@ -63,7 +66,7 @@ struct Io {
 // What becomes of a finished row: stored, stored and taken through the tail, or added to what is there.
 enum Finish { STORE = 0, TAIL = 1, ADD = 2 };
 
-template <int R, int FINISH, bool CHIRP>
+template <int R, int FINISH, bool CHIRP, int SHIFT>
 __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io& io, const FftEpilogue& ep) {
     const int items = io.rows * d.nb;
     for (int i = threadIdx.x; i < items; i += blockDim.x) {
@@ -72,7 +75,7 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
         if (io.src) {
             const float2* s = io.src + row * pl.stride;
 #pragma unroll
-            for (int q = 0; q < R; ++q) v[q] = s[pad_of(j + q * d.nb)];
+            for (int q = 0; q < R; ++q) v[q] = s[pad_of<SHIFT>(j + q * d.nb)];
             if (CHIRP && io.spectral) {
 #pragma unroll
                 for (int q = 0; q < R; ++q) {
@@ -106,7 +109,7 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
         if (io.dst) {
             float2* t = io.dst + row * pl.stride;
 #pragma unroll
-            for (int q = 0; q < R; ++q) t[pad_of(o + q * d.L)] = v[q];
+            for (int q = 0; q < R; ++q) t[pad_of<SHIFT>(o + q * d.L)] = v[q];
         } else {
             const size_t base = (size_t) row * pl.n + o;
             // Old values are requested together, before the first store: between the stores each load waited for the
@@ -150,7 +153,7 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
     }
 }
 
-template <int FINISH, bool CHIRP>
+template <int FINISH, bool CHIRP, int SHIFT>
 __global__ void __launch_bounds__(MAX_THREADS, 2)
 fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* yr, float* yi,
             const float2* __restrict__ tw, const float2* __restrict__ chirp, const float2* __restrict__ spectrum, int B,
@@ -170,7 +173,7 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
         io.dst = s == total - 1 ? nullptr : bufs + (s & 1 ? pl.rows * pl.stride : 0);
         io.spectral = CHIRP && s == pl.passes;
         switch (d.radix) {
-#define CNB_RADIX(R) case R: run_pass<R, FINISH, CHIRP>(pl, d, io, ep); break
+#define CNB_RADIX(R) case R: run_pass<R, FINISH, CHIRP, SHIFT>(pl, d, io, ep); break
             CNB_RADIX(2); CNB_RADIX(3); CNB_RADIX(4); CNB_RADIX(5); CNB_RADIX(6); CNB_RADIX(7); CNB_RADIX(8); CNB_RADIX(9);
             CNB_RADIX(10); CNB_RADIX(11); CNB_RADIX(12); CNB_RADIX(13); CNB_RADIX(14); CNB_RADIX(15); CNB_RADIX(16);
 #undef CNB_RADIX
@@ -258,7 +261,45 @@ bool choose_radices(int m, std::vector<int>* radices, double* cost) {
     return false;
 }
 
-size_t smem_bytes(int m, int rows, int buffers) { return (size_t) buffers * rows * (pad_of(m) + 1) * sizeof(float2); }
+int row_stride(int m) { return pad_of<SPREAD>(m) + 1; }
+size_t smem_bytes(int m, int rows, int buffers) { return (size_t) buffers * rows * row_stride(m) * sizeof(float2); }
+
+// Wavefronts of the 8-byte accesses of up to 32 lanes: 16 at a time, a word pair per bank pair.
+int wavefronts(const int (&at)[32], int lanes) {
+    int sum = 0;
+    for (int h = 0; h < lanes; h += 16) {
+        int most = 0, count[16] = {};
+        for (int l = h; l < std::min(lanes, h + 16); ++l) most = std::max(most, ++count[at[l] & 15]);
+        sum += most;
+    }
+    return sum;
+}
+
+// The spread of fewest wavefronts over the first warps' butterflies of every pass, weighed by the butterflies they stand for.
+// Radix 16 wants every 16th element set apart; runs 10 apart get into each other's way by it: 1500 = 10 x 15 x 10 had 4.8
+// wavefronts too many a store (1000 rows 12.9 -> 11.0 us; 10000 x 100 8.8 -> 7.9, 1000 x 1000 11.4 -> 9.7).
+int choose_spread(const MixedPlan& pl) {
+    double cost[2] = {0, 0};
+    for (int v = 0; v < 2; ++v)
+        for (int p = 0; p < pl.passes; ++p) {
+            const Pass& d = pl.p[p];
+            const int warps = std::min(4, (d.nb + 31) / 32);
+            int sum = 0;
+            for (int w = 0; w < warps; ++w)
+                for (int q = 0; q < d.radix; ++q) {
+                    int to[32], from[32], n = 0;
+                    for (int i = 32 * w; i < std::min(32 * w + 32, d.nb); ++i, ++n) {
+                        const int o = (i - i % d.L) * d.radix + i % d.L + q * d.L, s = i + q * d.nb;
+                        to[n] = v ? pad_of<SPREAD>(o) : o;
+                        from[n] = v ? pad_of<SPREAD>(s) : s;
+                    }
+                    sum += (p + 1 < pl.passes ? wavefronts(to, n) : 0) + (p > 0 ? wavefronts(from, n) : 0);
+                }
+            cost[v] += (double) sum * d.nb / std::min(32 * warps, d.nb);
+        }
+    return cost[0] < 0.95 * cost[1] ? NO_SPREAD : SPREAD;
+}
+
 
 int buffers_for(int passes, bool chirp) {
     const int hops = (chirp ? 2 * passes : passes) - 1;     // passes that write shared memory
@@ -282,7 +323,7 @@ bool plan_length(int N, MixedPlan* out) {
     MixedPlan pl = {};
     pl.n = N; pl.m = m;
     pl.passes = (int) radices.size();
-    pl.stride = pad_of(m) + 1;
+    pl.stride = row_stride(m);
     pl.buffers = buffers_for(pl.passes, m > N);
     if (smem_bytes(m, 1, pl.buffers) > MAX_SMEM) return false;
     int L = 1, tw = 0;
@@ -294,6 +335,7 @@ bool plan_length(int N, MixedPlan* out) {
         if (L > 1) tw += (d.radix - 1) * L;
         L *= d.radix;
     }
+    pl.shift = m > N ? SPREAD : choose_spread(pl);
     pl.scale = (float) (1.0 / std::sqrt((double) N));
     *out = pl;
     return true;
@@ -315,12 +357,14 @@ bool cached_plan(int N, MixedPlan* out) {
 
 // Rows per CTA and threads: about four CTAs to an SM (up to 52 KB of shared memory each), so that some load or store
 // while others transform; rows are spread over the SMs first when the batch is small; of the thread counts the one
-// that wastes the fewest lanes over the passes.
+// that wastes the fewest lanes over the passes, or, with no more than a CTA to an SM, the one with the fewest butterflies
+// one after another (64 x 784, 128 threads instead of 64: 5.7 -> 5.1 us, with the tail 8.3 -> 6.4).
 void plan_batch(MixedPlan* pl, int B, int sms) {
     const size_t budget = 52 * 1024;
     int rows = 1;
     while (rows < 64 && smem_bytes(pl->m, rows + 1, std::max(1, pl->buffers)) <= budget && (long) (rows + 1) * pl->m <= 4096) ++rows;
     rows = std::max(1, std::min(rows, (B + 2 * sms - 1) / (2 * sms)));
+    const bool alone = (B + rows - 1) / rows <= sms;
     double best = 1e30;
     for (int t = 64; t <= MAX_THREADS; t += 32) {
         double c = 0;
@@ -328,7 +372,7 @@ void plan_batch(MixedPlan* pl, int B, int sms) {
             const int items = rows * pl->p[p].nb;
             c += (double) ((items + t - 1) / t) * butterfly_cost(pl->p[p].radix);
         }
-        c *= t + 32;                                        // lanes held, and a little for every CTA
+        if (!alone) c *= t + 32;                            // lanes held, and a little for every CTA
         if (c < best * 0.999) { best = c; pl->threads = t; }
     }
     pl->rows = rows;
@@ -388,18 +432,20 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
     const Finish finish = ep.hr ? TAIL : accumulate ? ADD : STORE;
     static bool attr_done[64] = {};                         // the attribute is per device
     if (!attr_done[ctx->device & 63]) {
-#define CNB_MIXED_ATTR(F, C) CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM))
-        CNB_MIXED_ATTR(STORE, false); CNB_MIXED_ATTR(TAIL, false); CNB_MIXED_ATTR(ADD, false);
-        CNB_MIXED_ATTR(STORE, true); CNB_MIXED_ATTR(TAIL, true); CNB_MIXED_ATTR(ADD, true);
+#define CNB_MIXED_ATTR(F)                                                                                                          \
+    do {                                                                                                                           \
+        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, false, SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM)); \
+        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, false, NO_SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM)); \
+        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, true, SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));  \
+    } while (0)
+        CNB_MIXED_ATTR(STORE); CNB_MIXED_ATTR(TAIL); CNB_MIXED_ATTR(ADD);
 #undef CNB_MIXED_ATTR
         attr_done[ctx->device & 63] = true;
     }
     const dim3 grid((unsigned) ((B + pl.rows - 1) / pl.rows)), block((unsigned) pl.threads);
-#define CNB_MIXED(F)                                                                                                          \
-    do {                                                                                                                      \
-        if (chirp) CNB_CUDA(cnb::launch(fft_mixed_k<F, true>, grid, block, smem, st, 1, xr, xi, yr, yi, tw, ch, spec, B, ep, pl)); \
-        else CNB_CUDA(cnb::launch(fft_mixed_k<F, false>, grid, block, smem, st, 1, xr, xi, yr, yi, tw, ch, spec, B, ep, pl));      \
-    } while (0)
+    auto go = [&](auto kernel) { return cnb::launch(kernel, grid, block, smem, st, 1, xr, xi, yr, yi, tw, ch, spec, B, ep, pl); };
+#define CNB_MIXED(F) \
+    CNB_CUDA(chirp ? go(fft_mixed_k<F, true, SPREAD>) : pl.shift == SPREAD ? go(fft_mixed_k<F, false, SPREAD>) : go(fft_mixed_k<F, false, NO_SPREAD>))
     if (finish == TAIL) CNB_MIXED(TAIL);
     else if (finish == ADD) CNB_MIXED(ADD);
     else CNB_MIXED(STORE);
