@@ -1,11 +1,14 @@
 """Builds libcnet_b200.so in-tree: the sm_100a kernels + C ABI (csrc/) and the C++ host
-facade (host/).  ``python -m cnet_b200.build`` or ``build(force=True)``."""
+facade (host/), and ops_native.so, the operators' calls from Python (host/ops_native.cpp).
+``python -m cnet_b200.build`` or ``build(force=True)``."""
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "libcnet_b200.so")
+OPS = os.path.join(HERE, "ops_native.so")
 CSRC = ["context.cu", "elementwise.cu", "rowreduce.cu", "embed.cu", "cgemm_simt.cu", "cgemm_tc.cu", "linear.cu", "fft.cu", "fft_pipe.cu", "fft_mixed.cu", "cgemv_skinny.cu", "dp_allreduce.cu"]
 HOST = ["cnet.cpp", "capi.cpp", "dp_nccl.cpp", "model_saver.cpp", "data_reader.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "-lineinfo",
@@ -27,7 +30,34 @@ def up_to_date():
     return all(os.path.getmtime(d) <= t for d in _sources()[1] if os.path.exists(d))
 
 
+def _build_ops(env):
+    """The CPython module, against this interpreter's and torch's headers; the library beside it is found by $ORIGIN."""
+    import torch
+    root = os.path.dirname(torch.__file__)
+    src = os.path.join(HERE, "host", "ops_native.cpp")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+           "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I", sysconfig.get_paths()["include"], "-isystem", "/usr/local/cuda/include", src, "-o", OPS,
+           "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda",
+           "-L", HERE, "-l:libcnet_b200.so", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, env=env)
+    if r.returncode != 0:
+        raise RuntimeError("ops_native failed:\n" + r.stdout.decode())
+
+
+def _ops_up_to_date():
+    deps = [os.path.join(HERE, "host", "ops_native.cpp"), os.path.join(HERE, "..", "include", "cnet_b200.h"), __file__]
+    return os.path.exists(OPS) and all(os.path.getmtime(d) <= os.path.getmtime(OPS) for d in deps)
+
+
 def build(force=False, verbose=False):
+    lib = _build_lib(force, verbose)
+    if force or not _ops_up_to_date():
+        _build_ops({k: v for k, v in os.environ.items() if k not in ("CXX", "CC")})
+    return lib
+
+
+def _build_lib(force, verbose):
     if not force and up_to_date():
         return LIB
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

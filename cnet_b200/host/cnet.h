@@ -423,6 +423,8 @@ class CNet {
 	bool joinCollectives();                         // the compute stream waits for every collective in flight
 	std::vector<cnb_pack_span> packSpans(std::vector<Linear*>* packed) const;
 	void weightsUpdated(const std::vector<Linear*>& packed);
+	static constexpr size_t kBounceBytes = 64 << 10;
+	void* bounce_ = nullptr;                        // pinned memory for small read-backs
 	void* graph_exec_ = nullptr;                    // cudaGraphExec_t of a captured step
 	bool capturing_ = false;
 	unsigned long long graph_launches_ = 0;         // kernels inside the captured step

@@ -1,15 +1,39 @@
 """Direct calls of the C-ABI operators (include/cnet_b200.h) on torch CUDA tensors.
 
 torch only owns the memory and the stream; every operator below is one call into
-libcnet_b200.so.  Complex tensors are (re, im) pairs of contiguous float32 tensors.
+libcnet_b200.so, of Linear, FourierTrans, SoftMax and CrossEntropy by way of ops_native.so (host/ops_native.cpp), which
+makes the results too.  Complex tensors are (re, im) pairs of contiguous float32 tensors.
 """
 import ctypes as C
+import importlib.machinery
+import importlib.util
+import os
 
 from . import lib as _lib
 
 
 def _p(t):
     return None if t is None else t.data_ptr()
+
+
+_native = None
+
+
+def _load_native():
+    """The module ops_native.so beside the library (once)."""
+    global _native
+    if _native is None:
+        path = os.path.join(_lib.HERE, "ops_native.so")
+        if not os.path.exists(path):
+            raise _lib.CnetError("ops_native.so is not built (run `python -m cnet_b200.build`)")
+        import torch  # noqa: F401                       # the module finds torch's libraries loaded,
+        _lib.load()                                      # and this one
+        loader = importlib.machinery.ExtensionFileLoader("ops_native", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ops_native", path, loader=loader))
+        loader.exec_module(mod)
+        mod.set_error_class(_lib.CnetError)
+        _native = mod
+    return _native
 
 
 class Context:
@@ -21,6 +45,7 @@ class Context:
             raise _lib.CnetError("no CUDA device: the path has no CPU fallback")
         self.lib = _lib.load()
         self.torch = torch
+        self.native = _load_native()
         self.h = C.c_void_p()
         _lib.check(self.lib.cnb_create(device, arena_bytes, C.byref(self.h)), "cnb_create")
         # The raw handle of the current stream costs 0.15 us where torch exposes it and 3.2 us as a Stream object: a
@@ -56,31 +81,13 @@ class Context:
 
     # ------------------------------------------------------------------ Linear
     def linear_fwd(self, x, w, res=None):
-        B, n_in = x[0].shape
-        n_out = w[0].shape[0]
-        y = self._new(B, n_out)
-        _lib.check(self.lib.cnb_linear_fwd(self.h, _p(x[0]), _p(x[1]), _p(w[0]), _p(w[1]),
-                                           _p(res[0]) if res else None, _p(res[1]) if res else None,
-                                           _p(y[0]), _p(y[1]), B, n_in, n_out, self._stream()), "linear_fwd")
-        return y
+        return self.native.linear_fwd(self.h.value if self.h else None, x, w, res)
 
     def linear_bwd_x(self, g, w, out=None):
-        B, n_out = g[0].shape
-        n_in = w[0].shape[1]
-        acc = 1 if out is not None else 0
-        dx = out if out is not None else self._new(B, n_in)
-        _lib.check(self.lib.cnb_linear_bwd_x(self.h, _p(g[0]), _p(g[1]), _p(w[0]), _p(w[1]), _p(dx[0]), _p(dx[1]),
-                                             B, n_in, n_out, acc, self._stream()), "linear_bwd_x")
-        return dx
+        return self.native.linear_bwd_x(self.h.value if self.h else None, g, w, out)
 
     def linear_bwd_w(self, g, x, out=None):
-        B, n_out = g[0].shape
-        n_in = x[0].shape[1]
-        acc = 1 if out is not None else 0
-        dw = out if out is not None else self._new(n_out, n_in)
-        _lib.check(self.lib.cnb_linear_bwd_w(self.h, _p(g[0]), _p(g[1]), _p(x[0]), _p(x[1]), _p(dw[0]), _p(dw[1]),
-                                             B, n_in, n_out, acc, self._stream()), "linear_bwd_w")
-        return dw
+        return self.native.linear_bwd_w(self.h.value if self.h else None, g, x, out)
 
     # operands split once (fp32 hi, bf16 hi and lo) and reused by several products
     def split(self, x):
@@ -113,18 +120,10 @@ class Context:
 
     # ------------------------------------------------------------ FourierTrans
     def dft_fwd(self, x):
-        B, N = x[0].shape
-        y = self._like(x)
-        _lib.check(self.lib.cnb_dft_fwd(self.h, _p(x[0]), _p(x[1]), _p(y[0]), _p(y[1]), B, N, self._stream()), "dft_fwd")
-        return y
+        return self.native.dft_fwd(self.h.value if self.h else None, x)
 
     def dft_bwd(self, g, out=None):
-        B, N = g[0].shape
-        acc = 1 if out is not None else 0
-        dx = out if out is not None else self._like(g)
-        _lib.check(self.lib.cnb_dft_bwd(self.h, _p(g[0]), _p(g[1]), _p(dx[0]), _p(dx[1]), B, N, acc, self._stream()),
-                   "dft_bwd")
-        return dx
+        return self.native.dft_bwd(self.h.value if self.h else None, g, out)
 
     def dft_hadamard_gelu_fwd(self, x, h, u=None, split=None):
         """FourierTrans forward with the Hadamard(h) -> CGelu tail in the same kernel: u = FFT(x) and the operand
@@ -194,27 +193,13 @@ class Context:
 
     # ---------------------------------------------------------- row reductions
     def softmax_fwd(self, z):
-        B, N = z[0].shape
-        y = self._like(z)
-        inv = self.torch.empty(B, dtype=self.torch.float32, device="cuda")
-        _lib.check(self.lib.cnb_softmax_fwd(self.h, _p(z[0]), _p(z[1]), _p(y[0]), _p(y[1]), _p(inv), B, N,
-                                            self._stream()), "softmax_fwd")
-        return y, inv
+        return self.native.softmax_fwd(self.h.value if self.h else None, z)
 
     def softmax_bwd(self, g, z, inv):
-        B, N = z[0].shape
-        d = self._like(z)
-        _lib.check(self.lib.cnb_softmax_bwd(self.h, _p(g[0]), _p(g[1]), _p(z[0]), _p(z[1]), _p(inv), _p(d[0]), _p(d[1]),
-                                            B, N, 0, self._stream()), "softmax_bwd")
-        return d
+        return self.native.softmax_bwd(self.h.value if self.h else None, g, z, inv)
 
     def crossent(self, z, labels, backward=True):
-        B, M = z[0].shape
-        loss = self.torch.empty(B, dtype=self.torch.float32, device="cuda")
-        d = self._like(z) if backward else (None, None)
-        _lib.check(self.lib.cnb_crossent_fwd_bwd(self.h, _p(z[0]), _p(z[1]), _p(labels), _p(loss), _p(d[0]), _p(d[1]),
-                                                 B, M, self._stream()), "crossent")
-        return loss, d
+        return self.native.crossent(self.h.value if self.h else None, z, labels, backward)
 
     # --------------------------------------------------------------- embedding
     def embed_fwd(self, table, tokens):

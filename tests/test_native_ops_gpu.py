@@ -1,0 +1,74 @@
+"""The operators that go through ops_native.so: the values and errors of the C ABI calls that they make, results in place,
+planes that are no tensors, another stream."""
+import pytest
+
+from cnet_b200.lib import CnetError
+from cnet_b200.ops import Context
+
+pytestmark = pytest.mark.gpu
+
+
+class Plane:
+    """Something with a shape and an address."""
+
+    def __init__(self, t):
+        self.t, self.shape = t, tuple(t.shape)
+
+    def data_ptr(self):
+        return self.t.data_ptr()
+
+
+@pytest.mark.parametrize("wrap", [tuple, list, lambda p: (Plane(p[0]), Plane(p[1]))])
+def test_the_same_as_the_c_calls(wrap):
+    import torch
+    ctx = Context(arena_bytes=32 << 20)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1)
+    pair = lambda *s: (torch.randn(*s, generator=gen, device="cuda"), torch.randn(*s, generator=gen, device="cuda"))
+    x, w, g, r = pair(7, 20), pair(5, 20), pair(7, 5), pair(7, 5)
+    p, st = lambda t: t.data_ptr(), torch.cuda.current_stream().cuda_stream
+    like = lambda a: (torch.empty_like(a[0]), torch.empty_like(a[0]))
+    same = lambda a, b: torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    lib = ctx.lib
+    y = like(g)
+    assert lib.cnb_linear_fwd(ctx.h, p(x[0]), p(x[1]), p(w[0]), p(w[1]), p(r[0]), p(r[1]), p(y[0]), p(y[1]), 7, 20, 5, st) == 0
+    assert same(ctx.linear_fwd(wrap(x), wrap(w), res=wrap(r)), y)
+    dx = like(x)
+    assert lib.cnb_linear_bwd_x(ctx.h, p(g[0]), p(g[1]), p(w[0]), p(w[1]), p(dx[0]), p(dx[1]), 7, 20, 5, 0, st) == 0
+    assert same(ctx.linear_bwd_x(wrap(g), wrap(w)), dx)
+    out = (torch.ones_like(dx[0]), torch.ones_like(dx[0]))
+    assert ctx.linear_bwd_x(wrap(g), wrap(w), out=out) is out and torch.equal(out[0], dx[0] + 1)
+    dw = like(w)
+    assert lib.cnb_linear_bwd_w(ctx.h, p(g[0]), p(g[1]), p(x[0]), p(x[1]), p(dw[0]), p(dw[1]), 7, 20, 5, 0, st) == 0
+    assert same(ctx.linear_bwd_w(wrap(g), wrap(x)), dw)
+    f = like(x)
+    assert lib.cnb_dft_fwd(ctx.h, p(x[0]), p(x[1]), p(f[0]), p(f[1]), 7, 20, st) == 0
+    assert same(ctx.dft_fwd(wrap(x)), f)
+    back = (x[0].clone(), x[1].clone())
+    assert ctx.dft_bwd(wrap(f), out=back) is back and torch.allclose(back[0], 2 * x[0], atol=1e-5)
+    s, inv = ctx.softmax_fwd(wrap(g))
+    assert s[0].shape == (7, 5) and inv.shape == (7,)
+    labels = torch.arange(7, device="cuda", dtype=torch.int32) % 5
+    loss, d = ctx.crossent(wrap(s), labels)
+    only, none = ctx.crossent(wrap(s), labels, backward=False)
+    assert torch.equal(loss, only) and none == (None, None)
+    assert ctx.softmax_bwd(wrap(d), wrap(g), inv)[0].shape == (7, 5)
+
+
+def test_errors_and_streams():
+    import torch
+    ctx = Context(arena_bytes=32 << 20)
+    x = (torch.randn(64, 100, device="cuda"), torch.randn(64, 100, device="cuda"))
+    want = ctx.dft_fwd(x)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        got = ctx.dft_fwd(x)
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], want[0])
+    with pytest.raises(ValueError):
+        ctx.dft_fwd((x[0][0], x[1][0]))
+    with pytest.raises(CnetError, match="dft_fwd failed"):
+        ctx.dft_fwd((torch.empty(0, 100, device="cuda"),) * 2)
+    ctx.close()
+    with pytest.raises(CnetError, match="null"):
+        ctx.dft_fwd(x)
