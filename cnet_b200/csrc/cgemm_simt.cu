@@ -1,78 +1,85 @@
 // fp32 SIMT complex GEMM on generic strides: the products that are too small, too narrow or too short for the tensor-core
 // tiles, and all of them where the arena has no room for packed operands; every operand orientation of the Linear backward
-// without staging copies.  64x64 output tile, 16-deep k-slab in shared memory, 256 threads each owning a 4x4 block of
-// complex accumulators.  (cgemm_fma.cuh has the same tile for packed operands, the next slab on its way while one is
-// worked on; with that the products here took 3 us more at K = 17..26, 9.3 -> 13.2 at 500 x 900 x 26.)
+// without staging copies.
+//
+// Tiles of T x T outputs (16 or 32), one or four of them a thread, k-slabs of 32 in two shared-memory buffers, the next slab
+// on its way while one is worked on.  What bounds them is the chain of a CTA's slabs, each a round trip to L2, and few CTAs:
+// with tiles of 64 x 64 and slabs of 16, fetched and then worked on, 64 x 64 -> 32 took 12 us and 128 x 128, K = 128 23 us
+// (now 2.8 and 5.2), 2000 x 50 -> 50 13 (6.0), 500 x 900, K = 26 9.1 (6.8), 2000 x 2000, K = 18 54 (32).  The terms of an
+// output are added one by one in the order of k whatever the tile.
 #include "common.cuh"
 
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
-
+// What the kernels before this one may still be writing is read by ordinary loads behind cnb_pdl_enter.
+template <int T>
 __global__ void __launch_bounds__(256)
-cgemm_simt_k(const float* __restrict__ a_re, const float* __restrict__ a_im, long sam, long sak,
-             const float* __restrict__ b_re, const float* __restrict__ b_im, long sbn, long sbk, int conjB,
-             const float* __restrict__ r_re, const float* __restrict__ r_im,
-             float* __restrict__ d_re, float* __restrict__ d_im, int M, int N, int K, int accumulate) {
+cgemm_simt_k(const float* a_re, const float* a_im, long sam, long sak, const float* b_re, const float* b_im, long sbn, long sbk,
+             int conjB, const float* r_re, const float* r_im, float* d_re, float* d_im, int M, int N, int K, int accumulate) {
     cnb_pdl_enter();
-    __shared__ float As_r[TK][TM + 4], As_i[TK][TM + 4], Bs_r[TK][TN + 4], Bs_i[TK][TN + 4];
-    int tid = threadIdx.x;
-    int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    int tx = tid & 15, ty = tid >> 4;          // 16 x 16 threads, 4x4 micro-tile each
-    float cr[4][4] = {}, ci[4][4] = {};
-    // loader mapping: pick the index that is contiguous in memory as the fast one
-    bool a_kfast = (sak == 1), b_kfast = (sbk == 1);
-    for (int k0 = 0; k0 < K; k0 += TK) {
+    constexpr int SLAB = 32, U = T / 16, LOADS = T * SLAB / 256;
+    __shared__ float2 As[2][SLAB][T + 1], Bs[2][SLAB][T + 1];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int tiles_n = (N + T - 1) / T, m0 = (int) (blockIdx.x / (unsigned) tiles_n) * T, n0 = (int) (blockIdx.x % (unsigned) tiles_n) * T;
+    // loader mapping: the index that is contiguous in memory is the fast one
+    const bool a_kfast = sak == 1, b_kfast = sbk == 1;
+    float2 na[LOADS], nb[LOADS];
+    auto fetch = [&](int k0) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int e = tid + j * 256;             // 0..1023 = TM*TK
-            int mm = a_kfast ? e / TK : e % TM;
-            int kk = a_kfast ? e % TK : e / TM;
-            int gm = m0 + mm, gk = k0 + kk;
-            float vr = 0.f, vi = 0.f;
-            if (gm < M && gk < K) { size_t o = (size_t) gm * sam + (size_t) gk * sak; vr = a_re[o]; vi = a_im[o]; }
-            As_r[kk][mm] = vr; As_i[kk][mm] = vi;
-            int nn = b_kfast ? e / TK : e % TN;
-            kk = b_kfast ? e % TK : e / TN;
-            int gn = n0 + nn; gk = k0 + kk;
-            vr = 0.f; vi = 0.f;
-            if (gn < N && gk < K) { size_t o = (size_t) gn * sbn + (size_t) gk * sbk; vr = b_re[o]; vi = b_im[o]; }
-            Bs_r[kk][nn] = vr; Bs_i[kk][nn] = conjB ? -vi : vi;
+        for (int j = 0; j < LOADS; ++j) {
+            const int e = tid + j * 256;
+            const int gm = m0 + (a_kfast ? e / SLAB : e % T), ka = k0 + (a_kfast ? e % SLAB : e / T);
+            const int gn = n0 + (b_kfast ? e / SLAB : e % T), kb = k0 + (b_kfast ? e % SLAB : e / T);
+            na[j] = nb[j] = make_float2(0.f, 0.f);
+            if (gm < M && ka < K) { const size_t o = (size_t) gm * sam + (size_t) ka * sak; na[j] = make_float2(a_re[o], a_im[o]); }
+            if (gn < N && kb < K) { const size_t o = (size_t) gn * sbn + (size_t) kb * sbk; nb[j] = make_float2(b_re[o], b_im[o]); }
         }
-        __syncthreads();
+    };
+    float cr[U][U] = {}, ci[U][U] = {};
+    fetch(0);
+    for (int k0 = 0, s = 0; k0 < K; k0 += SLAB, s ^= 1) {
 #pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            float ar[4], ai[4], br[4], bi[4];
+        for (int j = 0; j < LOADS; ++j) {
+            const int e = tid + j * 256;
+            As[s][a_kfast ? e % SLAB : e / T][a_kfast ? e / SLAB : e % T] = na[j];
+            Bs[s][b_kfast ? e % SLAB : e / T][b_kfast ? e / SLAB : e % T] = make_float2(nb[j].x, conjB ? -nb[j].y : nb[j].y);
+        }
+        __syncthreads();                                 // the other buffer was last read before the barrier of the slab before
+        if (k0 + SLAB < K) fetch(k0 + SLAB);
+        const float2* as = &As[s][0][ty];
+        const float2* bs = &Bs[s][0][tx];
+        auto step = [&](int kk) {
+            float2 a[U], b[U];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                ar[i] = As_r[kk][ty * 4 + i]; ai[i] = As_i[kk][ty * 4 + i];
-                br[i] = Bs_r[kk][tx * 4 + i]; bi[i] = Bs_i[kk][tx * 4 + i];
-            }
+            for (int i = 0; i < U; ++i) { a[i] = as[kk * (T + 1) + 16 * i]; b[i] = bs[kk * (T + 1) + 16 * i]; }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < U; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    cr[i][j] += ar[i] * br[j] - ai[i] * bi[j];
-                    ci[i][j] += ar[i] * bi[j] + ai[i] * br[j];
+                for (int j = 0; j < U; ++j) {
+                    cr[i][j] += a[i].x * b[j].x - a[i].y * b[j].y;
+                    ci[i][j] += a[i].x * b[j].y + a[i].y * b[j].x;
                 }
+        };
+        if (K - k0 >= SLAB) {
+#pragma unroll
+            for (int kk = 0; kk < SLAB; ++kk) step(kk);
+        } else {
+#pragma unroll 4
+            for (int kk = 0; kk < K - k0; ++kk) step(kk);
         }
-        __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
+    for (int i = 0; i < U; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int gn = n0 + tx * 4 + j;
-            if (gn >= N) continue;
-            size_t o = (size_t) gm * N + gn;
+        for (int j = 0; j < U; ++j) {
+            const int gm = m0 + ty + 16 * i, gn = n0 + tx + 16 * j;
+            if (gm >= M || gn >= N) continue;
+            const size_t o = (size_t) gm * N + gn;
             float vr = cr[i][j], vi = ci[i][j];
             if (r_re) { vr += r_re[o]; vi += r_im[o]; }
             if (accumulate) { vr += d_re[o]; vi += d_im[o]; }
             d_re[o] = vr; d_im[o] = vi;
         }
-    }
 }
 
 }  // namespace
@@ -82,10 +89,15 @@ namespace cnb {
 int cgemm_simt(cnb_ctx* ctx, const float* a_re, const float* a_im, long sam, long sak, const float* b_re,
                const float* b_im, long sbn, long sbk, int conjB, const float* r_re, const float* r_im,
                float* d_re, float* d_im, int M, int N, int K, int accumulate, cudaStream_t st) {
-    (void) ctx;
-    dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
-    cnb::launch(cgemm_simt_k, dim3(grid), dim3(256), 0, st, 1, a_re, a_im, sam, sak, b_re, b_im, sbn, sbk, conjB, r_re, r_im, d_re, d_im,
-                                       M, N, K, accumulate);
+    auto go = [&](auto kernel, long tiles) {
+        return cnb::launch(kernel, dim3((unsigned) tiles), dim3(256), 0, st, 1, a_re, a_im, sam, sak, b_re, b_im, sbn, sbk, conjB, r_re, r_im,
+                           d_re, d_im, M, N, K, accumulate);
+    };
+    // Small tiles while they hardly fill the device, where twice the loads for an output cost nothing: one to an SM whatever
+    // K (30 x 20, K = 3000: 156 us with the others, 85), up to six of a short K (4096 x 16, K = 100: 14.6 and 9.8; 1000 x
+    // 60, K = 1000, two to an SM: 77 and 81).
+    const long small = (long) ((M + 15) / 16) * ((N + 15) / 16), large = (long) ((M + 31) / 32) * ((N + 31) / 32);
+    CNB_CUDA(small <= ctx->sm_count || (K <= 256 && small <= 6L * ctx->sm_count) ? go(cgemm_simt_k<16>, small) : go(cgemm_simt_k<32>, large));
     CNB_LAUNCH_CHECK("cgemm_simt");
     return CNB_OK;
 }

@@ -1683,11 +1683,15 @@ static int chain_blocks(int M, int N, int K, bool joined) {
 }
 
 bool cgemm_tc_shape_ok(int M, int N, int K) {
+    // Small products are done by the SIMT tiles before the operands would be packed: 128 x 128, K = 128 takes 5.3 us there
+    // and 13.6 here, K = 256 8.9 and 14.5, 200 x 100, K = 200 9.9 and 16.7, 200 x 200, K = 200 17.0 and 17.8; 1000 x 100,
+    // K = 200 19 and 16, 300 x 100, K = 300 22 and 17.
+    if (K <= 256 && (double) M * N * K <= 8e6) return false;
     if (split_sizes(M, N, K)) return true;
     // Other sizes leave more of the 128 x 128 tiles empty: from about two million complex multiplications on packing
-    // and tiles together take less than the fp32 SIMT tiles (777 x 1001 x 1333: 330 against 45 us), below it they do not.
-    // A short K leaves little to gain on either: 2000 x 50 takes 13 us in FMAs and 23 in tiles at K = 60, 20 and 18 at
-    // K = 100; with more 64 x 64 tiles than SMs the FMAs need another wave (1000 x 1000 x 60: 23 and 20).
+    // and tiles together take less than the fp32 SIMT tiles (64 x 64, K = 512: 15.5 against 12.3 us), below it they do not.
+    // A short K leaves little to gain on either: 2000 x 50 takes 6 us in FMAs and 23 in tiles at K = 50; with more 64 x 64
+    // blocks than SMs the FMAs take several waves (1000 x 1000 x 60: 21 and 20).
     if (K < 96 && (long) ((M + 63) / 64) * ((N + 63) / 64) <= 148) return false;
     return K >= 48 && (double) M * N * K >= (double) (1 << 21);
 }
