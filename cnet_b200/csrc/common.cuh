@@ -35,7 +35,6 @@ struct cnb_ctx {
     unsigned counter_set = 0;
     // Column-reduction partials and packed operands of raw products: the last bytes of the arena, so that growing it
     // takes in what it had.
-    float* scratch = nullptr;
     size_t scratch_bytes = 0;
     size_t scratch_kept = 0;          // of them, what no allocation may take back
     std::map<int, cnb_twiddle> twiddles;

@@ -34,7 +34,6 @@ static int scratch_size(cnb_ctx* ctx, size_t bytes) {
     if (ctx->used + bytes > arena_end(ctx))
         return set_error(CNB_ERR_ARENA, "arena exhausted: %zu used + %zu of scratch > %zu", ctx->used, bytes, ctx->size);
     ctx->scratch_bytes = bytes;
-    ctx->scratch = reinterpret_cast<float*>(ctx->base + arena_end(ctx) - bytes);
     return CNB_OK;
 }
 
@@ -50,7 +49,9 @@ int ensure_scratch(cnb_ctx* ctx, size_t bytes, bool keep, cudaStream_t st, float
         if (!keep && cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
         if (keep || capture != cudaStreamCaptureStatusNone) ctx->scratch_kept = bytes;
     }
-    *out = ctx->scratch;
+    // The last bytes, of which scratch_kept counts too: the front of a larger scratch may be given back while a captured launch
+    // still works on it.
+    *out = reinterpret_cast<float*>(ctx->base + arena_end(ctx) - bytes);
     return CNB_OK;
 }
 
@@ -199,7 +200,6 @@ int cnb_alloc(cnb_ctx* ctx, size_t bytes, void** out) {
 int cnb_reset(cnb_ctx* ctx) {
     CNB_CHECK_ARG(ctx, "cnb_reset: null context");
     ctx->used = 4096;           // keep the status word and the counters
-    ctx->scratch = nullptr;
     ctx->scratch_bytes = ctx->scratch_kept = 0;
     cnb::drop_tables(ctx);
     return CNB_OK;
