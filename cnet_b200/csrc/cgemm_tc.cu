@@ -396,6 +396,9 @@ template <int ACC> __device__ __forceinline__ void drain_chain(uint32_t tl, floa
 
 // the four warps of one epilogue group
 __device__ __forceinline__ void epi_bar_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+// One decision for the group.  The flag may be set at any time by the producer, the MMA thread or the other group, so threads
+// that each looked at it after the barrier could part ways, some to the role's end and some to the group's next barrier.
+__device__ __forceinline__ bool epi_gave_up(int group, volatile int* abort_flag) { return cnb_group_any(1 + group, 128, *abort_flag != 0); }
 
 // Shared memory by its 32-bit address: through a generic pointer the compiler keeps every load behind the global store
 // before it, which made a round trip of each 16 bytes written out.
@@ -961,8 +964,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                     sum(std::integral_constant<int, 0>(), acc_full, acc_empty);
                     sum(std::integral_constant<int, 1>(), acc2_full, acc2_empty);
                 }
-                epi_bar_sync(group);                 // everyone arrives, then agree on the outcome
-                if (*abort_flag) return false;
+                if (epi_gave_up(group, abort_flag)) return false;
             }
             return true;
         };
@@ -988,8 +990,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             } else {
             mbar_wait(acc_full, 0u, abort_flag, p.status, 3);
             CNB_GSTAMP(4, et == 0);
-            epi_bar_sync(group);
-            if (!*abort_flag) {
+            if (!epi_gave_up(group, abort_flag)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
                 for (int c0 = group * 64; c0 < group * 64 + 64; c0 += 16) {
@@ -1053,8 +1054,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                 if (!sum_chains(kb1 - kb0)) { live = false; break; }
             } else {
                 mbar_wait(acc_full, (uint32_t) seg & 1, abort_flag, p.status, 3);
-                epi_bar_sync(group);                 // everyone arrives, then agree on the outcome
-                if (*abort_flag) { live = false; break; }
+                if (epi_gave_up(group, abort_flag)) { live = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
 #pragma unroll(DRAIN ? 4 : 1)

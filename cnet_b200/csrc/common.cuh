@@ -219,6 +219,19 @@ __device__ __forceinline__ float cnb_ld_behind_wait(const float* p) {
     return v;
 }
 
+// Whether `mine` holds for any of the `threads` threads (whole warps) that meet at the CTA's barrier `barrier`: the same
+// answer for all of them.
+__device__ __forceinline__ bool cnb_group_any(int barrier, int threads, bool mine) {
+    unsigned any;
+    asm volatile(
+        "{\n\t.reg .pred m, a;\n\t"
+        "setp.ne.u32 m, %1, 0;\n\t"
+        "barrier.cta.red.or.pred a, %2, %3, m;\n\t"
+        "selp.u32 %0, 1, 0, a;\n\t}"
+        : "=r"(any) : "r"((unsigned) mine), "r"(barrier), "r"(threads) : "memory");
+    return any != 0;
+}
+
 namespace cnb {
 
 bool pdl_enabled();                // CNB_PDL=0 in the environment launches every kernel fully serialised
