@@ -52,13 +52,21 @@ void shape2(PyObject* o, int64_t* rows, int64_t* cols) {
 	if (PyErr_Occurred()) throw Raised();
 }
 
-// The two planes of a pair, as references of their own.
+// The two planes of a pair, as references of their own.  A pair is whatever o[0] and o[1] work for in Python: a tensor of two
+// planes is no sequence to C.
 struct Pair {
 	PyObject *re = nullptr, *im = nullptr;
 	explicit Pair(PyObject* o) {
-		re = PySequence_GetItem(o, 0);
-		im = re ? PySequence_GetItem(o, 1) : nullptr;
+		re = item(o, 0);
+		im = re ? item(o, 1) : nullptr;
 		if (!im) { Py_XDECREF(re); throw Raised(); }
+	}
+	static PyObject* item(PyObject* o, Py_ssize_t k) {
+		if (PyTuple_Check(o) || PyList_Check(o)) return PySequence_GetItem(o, k);
+		PyObject* key = PyLong_FromSsize_t(k);
+		PyObject* v = key ? PyObject_GetItem(o, key) : nullptr;
+		Py_XDECREF(key);
+		return v;
 	}
 	Pair(const Pair&) = delete;
 	~Pair() { Py_DECREF(re); Py_DECREF(im); }

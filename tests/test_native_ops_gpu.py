@@ -72,3 +72,27 @@ def test_errors_and_streams():
     ctx.close()
     with pytest.raises(CnetError, match="null"):
         ctx.dft_fwd(x)
+
+
+def test_a_tensor_of_two_planes_is_a_pair():
+    import torch
+    ctx = Context(arena_bytes=32 << 20)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(2)
+    pair = lambda *s: (torch.randn(*s, generator=gen, device="cuda"), torch.randn(*s, generator=gen, device="cuda"))
+    same = lambda a, b: torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    x, w, g = pair(7, 20), pair(5, 20), pair(7, 5)
+    sx, sw, sg = torch.stack(x), torch.stack(w), torch.stack(g)
+    assert same(ctx.linear_fwd(sx, sw), ctx.linear_fwd(x, w))
+    assert same(ctx.linear_bwd_x(sg, sw), ctx.linear_bwd_x(g, w))
+    assert same(ctx.linear_bwd_w(sg, sx), ctx.linear_bwd_w(g, x))
+    assert same(ctx.dft_fwd(sx), ctx.dft_fwd(x))
+    y, inv = ctx.softmax_fwd(g)
+    assert same(ctx.softmax_fwd(sg)[0], y) and same(ctx.softmax_bwd(sx[:, :, :5].contiguous(), sg, inv), ctx.softmax_bwd((x[0][:, :5].contiguous(), x[1][:, :5].contiguous()), g, inv))
+    labels = torch.arange(7, device="cuda", dtype=torch.int32) % 5
+    assert torch.equal(ctx.crossent(torch.stack(y), labels)[0], ctx.crossent(y, labels)[0])
+    for f, like in ((lambda out: ctx.linear_bwd_x(g, w, out=out), x), (lambda out: ctx.linear_bwd_w(g, x, out=out), w), (lambda out: ctx.dft_bwd(x, out=out), x)):
+        planes, stacked = (torch.ones_like(like[0]), torch.ones_like(like[0])), torch.ones_like(torch.stack(like))
+        assert f(stacked) is stacked and same(stacked, f(planes))
+    with pytest.raises(IndexError):
+        ctx.dft_fwd(sx[:1])
