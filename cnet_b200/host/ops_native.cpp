@@ -20,7 +20,9 @@ PyObject* g_error = nullptr;                     // cnet_b200.lib.CnetError
 // a Python error is set
 struct Raised {};
 
+// Nothing (None) is the null pointer, which the C ABI refuses where it needs a plane.
 float* address(PyObject* o) {
+	if (o == Py_None) return nullptr;
 	if (THPVariable_Check(o)) return static_cast<float*>(THPVariable_Unpack(o).data_ptr());
 	PyObject* v = PyObject_CallMethod(o, "data_ptr", nullptr);
 	if (!v) throw Raised();
@@ -260,7 +262,7 @@ PyObject* crossent(PyObject*, PyObject* const* a, Py_ssize_t n) {
 		at::Tensor loss = fresh({B}, at::Device(at::kCUDA));
 		float* pl = static_cast<float*>(loss.data_ptr());
 		const float *zr = z.r(), *zi = z.i();
-		const int32_t* labels = reinterpret_cast<const int32_t*>(a[2] == Py_None ? nullptr : address(a[2]));
+		const int32_t* labels = reinterpret_cast<const int32_t*>(address(a[2]));
 		void* st = stream();
 		PyObject* second;
 		if (backward) {

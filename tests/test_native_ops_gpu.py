@@ -96,3 +96,19 @@ def test_a_tensor_of_two_planes_is_a_pair():
         assert f(stacked) is stacked and same(stacked, f(planes))
     with pytest.raises(IndexError):
         ctx.dft_fwd(sx[:1])
+
+
+def test_a_missing_plane_is_the_c_calls_error():
+    import torch
+    ctx = Context(arena_bytes=32 << 20)
+    x = (torch.randn(4, 6, device="cuda"), torch.randn(4, 6, device="cuda"))
+    half = (x[0], None)
+    inv, labels = torch.ones(4, device="cuda"), torch.zeros(4, device="cuda", dtype=torch.int32)
+    for f in (lambda: ctx.linear_fwd(half, x), lambda: ctx.linear_fwd(x, half), lambda: ctx.linear_bwd_x(x, half), lambda: ctx.linear_bwd_w(half, x),
+              lambda: ctx.dft_fwd(half), lambda: ctx.dft_bwd(x, out=half), lambda: ctx.dft_bwd(x, out=(None, None)), lambda: ctx.softmax_fwd(half),
+              lambda: ctx.softmax_bwd(half, x, inv), lambda: ctx.softmax_bwd(x, x, None), lambda: ctx.crossent(half, labels),
+              lambda: ctx.crossent(x, None)):
+        with pytest.raises(CnetError, match="null"):
+            f()
+    with pytest.raises(CnetError, match="pair"):
+        ctx.linear_fwd(x, x, res=(torch.zeros(4, 4, device="cuda"), None))
