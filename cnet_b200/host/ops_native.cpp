@@ -54,6 +54,27 @@ void shape2(PyObject* o, int64_t* rows, int64_t* cols) {
 	if (PyErr_Occurred()) throw Raised();
 }
 
+// One extent of a plane that may have more dimensions than two: of a weight [out, 28, 28] only what the product cannot take
+// from the other operand is asked for.
+int64_t extent(PyObject* o, int axis) {
+	if (THPVariable_Check(o)) {
+		const at::Tensor& t = THPVariable_Unpack(o);
+		if (t.dim() <= axis) {
+			PyErr_SetString(PyExc_IndexError, "a plane of too few dimensions");
+			throw Raised();
+		}
+		return t.size(axis);
+	}
+	PyObject* s = PyObject_GetAttrString(o, "shape");
+	PyObject* v = s ? PySequence_GetItem(s, axis) : nullptr;
+	Py_XDECREF(s);
+	if (!v) throw Raised();
+	const int64_t n = PyLong_AsLongLong(v);
+	Py_DECREF(v);
+	if (PyErr_Occurred()) throw Raised();
+	return n;
+}
+
 // The two planes of a pair, as references of their own.  A pair is whatever o[0] and o[1] work for in Python: a tensor of two
 // planes is no sequence to C.
 struct Pair {
@@ -143,8 +164,9 @@ PyObject* linear_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
 	return guarded(n, 4, [&]() -> PyObject* {
 		cnb_ctx* ctx = context(a[0]);
 		const Pair x(a[1]), w(a[2]);
-		int64_t B, in, out, k;
-		shape2(x.re, &B, &in); shape2(w.re, &out, &k);
+		int64_t B, in;
+		shape2(x.re, &B, &in);
+		const int64_t out = extent(w.re, 0);
 		float *rr = nullptr, *ri = nullptr;
 		const int has = PyObject_IsTrue(a[3]);
 		if (has < 0) throw Raised();
@@ -162,8 +184,9 @@ PyObject* linear_bwd_x(PyObject*, PyObject* const* a, Py_ssize_t n) {
 	return guarded(n, 4, [&]() -> PyObject* {
 		cnb_ctx* ctx = context(a[0]);
 		const Pair g(a[1]), w(a[2]);
-		int64_t B, out, k, in;
-		shape2(g.re, &B, &out); shape2(w.re, &k, &in);
+		int64_t B, out;
+		shape2(g.re, &B, &out);
+		const int64_t in = extent(w.re, 1);
 		Result dx(a[3], B, in, at::Device(at::kCUDA));
 		const float *gr = g.r(), *gi = g.i(), *wr = w.r(), *wi = w.i();
 		void* st = stream();
@@ -177,8 +200,9 @@ PyObject* linear_bwd_w(PyObject*, PyObject* const* a, Py_ssize_t n) {
 	return guarded(n, 4, [&]() -> PyObject* {
 		cnb_ctx* ctx = context(a[0]);
 		const Pair g(a[1]), x(a[2]);
-		int64_t B, out, k, in;
-		shape2(g.re, &B, &out); shape2(x.re, &k, &in);
+		int64_t B, out;
+		shape2(g.re, &B, &out);
+		const int64_t in = extent(x.re, 1);
 		Result dw(a[3], out, in, at::Device(at::kCUDA));
 		const float *gr = g.r(), *gi = g.i(), *xr = x.r(), *xi = x.i();
 		void* st = stream();

@@ -112,3 +112,17 @@ def test_a_missing_plane_is_the_c_calls_error():
             f()
     with pytest.raises(CnetError, match="pair"):
         ctx.linear_fwd(x, x, res=(torch.zeros(4, 4, device="cuda"), None))
+
+
+def test_the_other_operand_may_have_more_dimensions():
+    import torch
+    ctx = Context(arena_bytes=32 << 20)
+    pair = lambda *s: (torch.randn(*s, device="cuda"), torch.randn(*s, device="cuda"))
+    same = lambda a, b: a[0].shape == b[0].shape and torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    view = lambda a, *s: (a[0].view(*s), a[1].view(*s))
+    x, w, g = pair(7, 20), pair(5, 20), pair(7, 5)
+    assert same(ctx.linear_fwd(x, view(w, 5, 4, 5)), ctx.linear_fwd(x, w))
+    assert same(ctx.linear_bwd_x(g, view(w, 5, 20, 1)), ctx.linear_bwd_x(g, w))
+    assert same(ctx.linear_bwd_w(g, view(x, 7, 20, 1)), ctx.linear_bwd_w(g, x))
+    with pytest.raises(IndexError):
+        ctx.linear_bwd_x(g, view(w, 100))
