@@ -30,16 +30,20 @@ def up_to_date():
     return all(os.path.getmtime(d) <= t for d in _sources()[1] if os.path.exists(d))
 
 
-def _build_ops(env):
-    """The CPython module, against this interpreter's and torch's headers; the library beside it is found by $ORIGIN."""
+def ops_command(src, out):
+    """The compiler's call that makes a CPython module of host/ops_native.cpp, against this interpreter's and torch's headers."""
     import torch
     root = os.path.dirname(torch.__file__)
-    src = os.path.join(HERE, "host", "ops_native.cpp")
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
-           "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
-           "-I", sysconfig.get_paths()["include"], "-isystem", "/usr/local/cuda/include", src, "-o", OPS,
-           "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda",
-           "-L", HERE, "-l:libcnet_b200.so", "-Wl,-rpath,$ORIGIN"]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI,
+            "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            "-I", sysconfig.get_paths()["include"], "-isystem", "/usr/local/cuda/include", src, "-o", out,
+            "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda",
+            "-L", HERE, "-l:libcnet_b200.so", "-Wl,-rpath,$ORIGIN"]
+
+
+def _build_ops(env):
+    """The module; the library beside it is found by $ORIGIN."""
+    cmd = ops_command(os.path.join(HERE, "host", "ops_native.cpp"), OPS)
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, env=env)
     if r.returncode != 0:
         raise RuntimeError("ops_native failed:\n" + r.stdout.decode())

@@ -140,11 +140,14 @@ cnb_ctx* context(PyObject* o) {
 
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
+// Other threads may run Python meanwhile; the interpreter is this thread's again however that ends, also by an exception.
+struct Unlocked {
+	PyThreadState* state = PyEval_SaveThread();
+	~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 template <class F> void call(const char* what, F f) {
-	int rc;
-	Py_BEGIN_ALLOW_THREADS
-	rc = f();
-	Py_END_ALLOW_THREADS
+	const int rc = [&] { const Unlocked unlocked; return f(); }();
 	if (rc < 0) {
 		PyErr_Format(g_error ? g_error : PyExc_RuntimeError, "%s failed (%d): %s", what, rc, cnb_last_error());
 		throw Raised();
