@@ -1338,6 +1338,7 @@ bool CNet::sync() {
 bool CNet::readOutput(int uid, int what, float* re, float* im) {
 	auto it = map_.find(uid);
 	if (it == map_.end() || !ctx_) { fail(CNB_ERR_ARG, "readOutput: bad uid / not allocated"); return false; }
+	if (!re || !im) { fail(CNB_ERR_ARG, "readOutput: null plane"); return false; }
 	CFunc* f = it->second;
 	const Vars& v = f->out_;
 	const float* sr = what == 0 ? v.real_ : v.dz_star_real_;
