@@ -4,6 +4,7 @@
 #include "cnet.h"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1350,13 +1351,23 @@ bool CNet::readOutput(int uid, int what, float* re, float* im) {
 	if (!sr) { fail(CNB_ERR_ARG, f->getName() + ": tensor not materialised (fused)"); return false; }
 	size_t n = (size_t) (f->batched_ ? cur_batch_ : 1) * f->out_size_;
 	const size_t bytes = n * sizeof(float);
-	if (bounce_ && 2 * bytes <= kBounceBytes && si >= sr + n) {
-		// both planes as the two rows of one copy, one wait: a copy to pageable memory and its wait take 12 us each
-		cudaError_t e = cudaMemcpy2DAsync(bounce_, bytes, sr, (size_t) (si - sr) * sizeof(float), bytes, 2, cudaMemcpyDeviceToHost, (cudaStream_t) stream_);
-		if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t) stream_);
+	if (bounce_ && 2 * bytes <= kBounceBytes) {
+		// One wait: a copy to pageable memory and its wait take 12 us each.  Both planes are the two rows of one copy, whose pitch
+		// may be 2^31 - 1 bytes at most: planes lie as far apart as the allocated batch makes them, of which this may be one row.
+		cudaStream_t st = (cudaStream_t) stream_;
+		char* const second = static_cast<char*>(bounce_) + bytes;
+		const size_t apart = si >= sr + n ? (size_t) (si - sr) * sizeof(float) : 0;
+		cudaError_t e;
+		if (apart > 0 && apart <= (size_t) INT_MAX) {
+			e = cudaMemcpy2DAsync(bounce_, bytes, sr, apart, bytes, 2, cudaMemcpyDeviceToHost, st);
+		} else {
+			e = cudaMemcpyAsync(bounce_, sr, bytes, cudaMemcpyDeviceToHost, st);
+			if (e == cudaSuccess) e = cudaMemcpyAsync(second, si, bytes, cudaMemcpyDeviceToHost, st);
+		}
+		if (e == cudaSuccess) e = cudaStreamSynchronize(st);
 		if (e != cudaSuccess) { fail(CNB_ERR_CUDA, std::string("readOutput: ") + cudaGetErrorString(e)); return false; }
 		std::memcpy(re, bounce_, bytes);
-		std::memcpy(im, static_cast<char*>(bounce_) + bytes, bytes);
+		std::memcpy(im, second, bytes);
 		return true;
 	}
 	int rc = cnb_d2h(ctx_, re, sr, bytes, stream_);

@@ -29,3 +29,21 @@ def test_a_null_plane_is_refused():
         net.lib.cnh_clear_error(net.h)
     got = net.get_record(spec.main, 0)
     assert np.array_equal(got[0], x[0]) and np.array_equal(got[1], x[1])
+
+
+@pytest.mark.parametrize("allocated,rows", [(64, 64), (64, 3), (4096, 1)])
+def test_part_of_the_allocated_batch(allocated, rows):
+    net, spec, x = _net(100, 10, allocated, rows)
+    got = net.get_record(spec.main, 0)
+    assert np.array_equal(got[0], x[0]) and np.array_equal(got[1], x[1])
+
+
+def test_planes_further_apart_than_a_copy_may_stride():
+    """Planes of 65536 x 8192 floats lie 2^31 bytes apart, one more than the pitch of a 2D copy can be."""
+    net = Net()
+    spec = configs.build_linear(net, n_in=8192, n_out=2)
+    net.allocate(65536)
+    x = tuple(np.random.default_rng(1).standard_normal((1, 8192), dtype=np.float32) for _ in range(2))
+    net.upload(x=x, labels=np.zeros(1, np.int32))
+    got = net.get_record(spec.main, 0)
+    assert np.array_equal(got[0], x[0]) and np.array_equal(got[1], x[1])
