@@ -1903,11 +1903,9 @@ static int schedule_of(int M, int N, int K, int accumulate, int sm_count, int sm
     out8[0] = q.pair ? 1 : 0;
     out8[1] = (int) (q.pair ? 2 * q.ctas : q.ctas);      // CTAs of the launch
     out8[2] = q.cluster * (q.pair ? 2 : 1);              // CTAs per cluster (1: no cluster)
-    const int chain = kMaxChain16 * FormCfg<SPLIT>::BK / bk;
-    const bool cut = q.segments > 0 && q.upc > chain;        // packed: a segment is several chains
-    out8[3] = (int) (cut ? chain : q.upc);
+    out8[3] = (int) q.upc;
     out8[4] = q.whole_per_cta;
-    out8[5] = cut ? q.segments * (int) ((q.upc + chain - 1) / chain) : q.segments;
+    out8[5] = q.segments;
     out8[6] = q.splits_tiles ? 1 : 0;
     out8[7] = q.clear_from_row;
     return CNB_OK;
@@ -1919,4 +1917,11 @@ extern "C" int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_cou
 
 extern "C" int cnb_gemm_schedule_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8) {
     return schedule_of(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK, out8);
+}
+
+extern "C" int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit) {
+    if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0)
+        return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_chain_packed: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
+    const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK);
+    return cnb::chain_blocks(M, N, K, q.joined);
 }

@@ -114,10 +114,13 @@ int cnb_reserve_scratch(cnb_ctx* ctx, size_t bytes);
  * of sm_count SMs of which the launch may fill sm_limit (0: all): host arithmetic only, no device needed (no
  * reference counterpart; for tests and tuning).  out8 = {CTA pairs (cta_group::2) or not, CTAs of the launch,
  * CTAs per cluster, k-blocks per run, whole tiles per CTA before the shared remainder, k-segments per tile
- * (capped chains), tiles summed with atomics or not, first row of the output that atomics touch}. */
+ * (K > 4096), tiles summed with atomics or not, first row of the output that atomics touch}. */
 int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8);
 /* The same for packed operands (k-blocks of 32), which all other tensor-core products run on. */
 int cnb_gemm_schedule_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8);
+/* k-blocks of 32 that such a launch sums in tensor memory at most: a longer run is cut into chains of that many, which are
+ * added up in registers.  (An error code, below zero, for sizes that are none.) */
+int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit);
 size_t cnb_split_floats(size_t n);
 int cnb_split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, void* stream);
 int cnb_linear_split_ok(int B, int in, int out);

@@ -28,7 +28,61 @@ def test_products_fill_the_sms_they_may_use(M, N, K, acc, limit):
     if s["pair"]:
         assert s["ctas"] % 2 == 0 and s["cluster_ctas"] in (2, 4) and M >= 256
     if s["segments"]:
-        assert k_blocks > 128 and s["run"] <= 32 and s["run"] * s["segments"] >= k_blocks     # capped accumulation chains
+        _check_segments(s, M, N, K)
+
+
+def _check_segments(s, M, N, K):
+    """The segments of a tile cover its k-blocks, none of them empty, one CTA (or pair) each."""
+    tiles = -(-M // (256 if s["pair"] else 128)) * -(-N // 128)
+    k_blocks = -(-K // 32)
+    assert s["ctas"] == tiles * s["segments"] * (2 if s["pair"] else 1), s
+    assert k_blocks > 128 and (s["segments"] - 1) * s["run"] < k_blocks <= s["segments"] * s["run"], s
+
+
+@pytest.mark.parametrize("limit", LIMITS)
+@pytest.mark.parametrize("M,N,K", [(2000, 2000, 60000), (130, 1030, 9000), (700, 515, 8200), (1024, 8192, 16384), (100, 2048, 16384), (64, 64, 100000),
+                                   (1000, 2050, 4104), (4096, 4096, 8192)])
+def test_a_long_k_is_cut_into_chains(M, N, K, limit):
+    """Whatever the form of the launch (segments, whole tiles, short runs), no more than 1024 products are summed in tensor
+    memory at sizes of multiples of 8, and 4.28 sqrt(K) at others; a chain is no shorter than an equal cut at that length makes it."""
+    s = _schedule(M, N, K, 0, limit)
+    chain = L.load().cnb_gemm_chain_packed(M, N, K, 0, SMS, limit)
+    k_blocks = -(-K // 32)
+    if K % 8 == 0:
+        assert chain == -(-k_blocks // -(-k_blocks // 32)), (chain, s)
+    else:
+        assert chain == int(4.28 * K ** 0.5 / 32), chain
+    if s["segments"]:
+        _check_segments(s, M, N, K)
+    elif s["whole_per_cta"] and not s["atomics"]:
+        tiles = -(-M // (256 if s["pair"] else 128)) * -(-N // 128)
+        assert s["ctas"] // (2 if s["pair"] else 1) * s["whole_per_cta"] >= tiles
+
+
+def test_segments_of_known_launches():
+    assert {(2000, 2000, 60000): 4, (130, 1030, 9000): 8} == {k: _schedule(*k, 0, 0)["segments"] for k in ((2000, 2000, 60000), (130, 1030, 9000))}
+
+
+@pytest.mark.parametrize("M,N,K,chain", [
+    (4096, 1024, 1024, 16),        # 128 tiles on 74 pairs, whole: two chains of 16 where one of 32 would pass 24
+    (4096, 1024, 512, 16),         # the same tiles, short of the cap
+    (512, 1024, 1024, 32),         # clusters along K: one chain
+    (4096, 4096, 4096, 128),       # whole tiles of K <= 4096: one chain
+    (777, 1001, 1333, 4),          # K of no multiple of 8: 4.28 sqrt(1333) = 156 products
+    (50, 70, 50, 1),
+])
+def test_chains(M, N, K, chain):
+    assert L.load().cnb_gemm_chain_packed(M, N, K, 0, SMS, 0) == chain
+
+
+def test_chain_refusals():
+    for bad in ((0, 8, 8), (8, 0, 8), (8, 8, 0)):
+        assert L.load().cnb_gemm_chain_packed(*bad, 0, SMS, 0) < 0
+
+
+def test_whole_tiles_of_a_long_k():
+    s = _schedule(1000, 2050, 4104, 0, 0)
+    assert s["whole_per_cta"] > 0 and s["segments"] == 0 and not s["atomics"]
 
 
 @pytest.mark.parametrize("limit", LIMITS)
