@@ -1,6 +1,8 @@
 """Builds libcnet_b200.so in-tree: the sm_100a kernels + C ABI (csrc/) and the C++ host
-facade (host/), and ops_native.so, the operators' calls from Python (host/ops_native.cpp).
+facade (host/), and ops_native.so, the operators' calls from Python (host/ops_native.cpp), for which torch and its headers
+have to be there; the library needs neither.
 ``python -m cnet_b200.build`` or ``build(force=True)``."""
+import importlib.util
 import os
 import subprocess
 import sys
@@ -56,6 +58,9 @@ def _ops_up_to_date():
 
 def build(force=False, verbose=False):
     lib = _build_lib(force, verbose)
+    if importlib.util.find_spec("torch") is None:
+        print("torch is not installed: without ops_native.so, which cnet_b200.ops needs", file=sys.stderr)
+        return lib
     if force or not _ops_up_to_date():
         _build_ops({k: v for k, v in os.environ.items() if k not in ("CXX", "CC")})
     return lib
