@@ -11,6 +11,7 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "libcnet_b200.so")
 OPS = os.path.join(HERE, "ops_native.so")
+OPS_KEY = os.path.join(HERE, "build", "ops_native.key")
 CSRC = ["context.cu", "elementwise.cu", "rowreduce.cu", "embed.cu", "cgemm_simt.cu", "cgemm_tc.cu", "linear.cu", "fft.cu", "fft_pipe.cu", "fft_mixed.cu", "cgemv_skinny.cu", "dp_allreduce.cu"]
 HOST = ["cnet.cpp", "capi.cpp", "dp_nccl.cpp", "model_saver.cpp", "data_reader.cpp"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O3", "-lineinfo",
@@ -43,17 +44,33 @@ def ops_command(src, out):
             "-L", HERE, "-l:libcnet_b200.so", "-Wl,-rpath,$ORIGIN"]
 
 
+def ops_key():
+    """What a build of the module depends on beside its sources: the interpreter and the torch whose headers it saw."""
+    import torch
+    return "%s, torch %s, C++11 ABI %d" % (sysconfig.get_config_var("EXT_SUFFIX"), torch.__version__, torch._C._GLIBCXX_USE_CXX11_ABI)
+
+
 def _build_ops(env):
-    """The module; the library beside it is found by $ORIGIN."""
-    cmd = ops_command(os.path.join(HERE, "host", "ops_native.cpp"), OPS)
+    """The module; the library beside it is found by $ORIGIN.  It appears whole: another process may be loading the one before."""
+    key = ops_key()
+    part = "%s.%d.tmp" % (OPS, os.getpid())
+    cmd = ops_command(os.path.join(HERE, "host", "ops_native.cpp"), part) + ['-DCNET_BUILT_FOR="%s"' % key]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, env=env)
     if r.returncode != 0:
+        if os.path.exists(part):
+            os.remove(part)
         raise RuntimeError("ops_native failed:\n" + r.stdout.decode())
+    os.replace(part, OPS)
+    os.makedirs(os.path.dirname(OPS_KEY), exist_ok=True)
+    with open(OPS_KEY, "w") as f:
+        f.write(key)
 
 
 def _ops_up_to_date():
     deps = [os.path.join(HERE, "host", "ops_native.cpp"), os.path.join(HERE, "..", "include", "cnet_b200.h"), __file__]
-    return os.path.exists(OPS) and all(os.path.getmtime(d) <= os.path.getmtime(OPS) for d in deps)
+    if not os.path.exists(OPS) or not os.path.exists(OPS_KEY) or open(OPS_KEY).read() != ops_key():
+        return False
+    return all(os.path.getmtime(d) <= os.path.getmtime(OPS) for d in deps)
 
 
 def build(force=False, verbose=False):

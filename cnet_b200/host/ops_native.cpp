@@ -321,4 +321,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "ops_native", nullptr, -1, methods,
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit_ops_native() { return PyModule_Create(&module); }
+#ifndef CNET_BUILT_FOR
+#define CNET_BUILT_FOR ""
+#endif
+
+PyMODINIT_FUNC PyInit_ops_native() {
+	PyObject* m = PyModule_Create(&module);
+	if (m && PyModule_AddStringConstant(m, "built_for", CNET_BUILT_FOR) < 0) { Py_DECREF(m); return nullptr; }
+	return m;
+}

@@ -9,6 +9,7 @@ import importlib.machinery
 import importlib.util
 import os
 
+from . import build as _build
 from . import lib as _lib
 
 
@@ -29,8 +30,15 @@ def _load_native():
         import torch  # noqa: F401                       # the module finds torch's libraries loaded,
         _lib.load()                                      # and this one
         loader = importlib.machinery.ExtensionFileLoader("ops_native", path)
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ops_native", path, loader=loader))
-        loader.exec_module(mod)
+        try:
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("ops_native", path, loader=loader))
+            loader.exec_module(mod)
+            made_for = mod.built_for
+        except ImportError as e:                         # symbols that this torch or interpreter does not have
+            made_for = str(e)
+        if made_for != _build.ops_key():                 # layouts of tensors and Python objects are compiled into it
+            raise _lib.CnetError("ops_native.so is built for another torch or Python (%s; this is %s): run `python -m cnet_b200.build`"
+                                 % (made_for, _build.ops_key()))
         mod.set_error_class(_lib.CnetError)
         _native = mod
     return _native
