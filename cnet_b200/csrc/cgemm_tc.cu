@@ -1682,11 +1682,7 @@ static int chain_blocks(int M, int N, int K, bool joined) {
     return (k_blocks + chains - 1) / chains;
 }
 
-bool cgemm_tc_shape_ok(int M, int N, int K) {
-    // Small products are done by the SIMT tiles before the operands would be packed: 128 x 128, K = 128 takes 5.3 us there
-    // and 13.6 here, K = 256 8.9 and 14.5, 200 x 100, K = 200 9.9 and 16.7, 200 x 200, K = 200 17.0 and 17.8; 1000 x 100,
-    // K = 200 19 and 16, 300 x 100, K = 300 22 and 17.
-    if (K <= 256 && (double) M * N * K <= 8e6) return false;
+bool cgemm_tc_fits(int M, int N, int K) {
     if (split_sizes(M, N, K)) return true;
     // Other sizes leave more of the 128 x 128 tiles empty: from about two million complex multiplications on packing
     // and tiles together take less than the fp32 SIMT tiles (64 x 64, K = 512: 15.5 against 12.3 us), below it they do not.
@@ -1694,6 +1690,14 @@ bool cgemm_tc_shape_ok(int M, int N, int K) {
     // blocks than SMs the FMAs take several waves (1000 x 1000 x 60: 21 and 20).
     if (K < 96 && (long) ((M + 63) / 64) * ((N + 63) / 64) <= 148) return false;
     return K >= 48 && (double) M * N * K >= (double) (1 << 21);
+}
+
+bool cgemm_tc_shape_ok(int M, int N, int K) {
+    // Small products are done by the SIMT tiles before the operands would be packed: 128 x 128, K = 128 takes 5.3 us there
+    // and 13.6 here, K = 256 8.9 and 14.5, 200 x 100, K = 200 9.9 and 16.7, 200 x 200, K = 200 17.0 and 17.8; 1000 x 100,
+    // K = 200 19 and 16, 300 x 100, K = 300 22 and 17.
+    if (K <= 256 && (double) M * N * K <= 8e6) return false;
+    return cgemm_tc_fits(M, N, K);
 }
 
 static size_t padded(int n, int to) { return ((size_t) n + to - 1) / to * to; }

@@ -77,7 +77,8 @@ int cgemm_simt(cnb_ctx* ctx, const float* a_re, const float* a_im, long sam, lon
 
 // tcgen05 complex GEMM on split operands:
 //   D[m,n] (+)= sum_k A[m,k] * (conjB ? conj(B[n,k]) : B[n,k]) (+ R[m,n]); A [M,K], B [N,K].
-// The sizes for which it beats the SIMT tiles:
+// The sizes that its tiles are made for, and those of them for which it beats the SIMT tiles with the operands still to be packed:
+bool cgemm_tc_fits(int M, int N, int K);
 bool cgemm_tc_shape_ok(int M, int N, int K);
 // A packed operand: fp16 high and low parts of a matrix scaled by one power of two (cgemm_tc.cu), the form that
 // everything but the C ABI's split buffers goes through.

@@ -53,8 +53,10 @@ int make_twiddle(cnb_ctx* ctx, int key, cudaStream_t st, cnb_twiddle* t) {
         tri_mask_k<<<ctx->sm_count * 4, 256, 0, st>>>(t->re, t->im, N);
         CNB_LAUNCH_CHECK("tri_mask");
     }
-    if (cnb::cgemm_tc_shape_ok(64, N, N) && (!cnb::fft_supported(N) || (key & kTriKey))) {
-        // the matrix is a constant: where the GEMM is the transform's engine, it is packed here, not by every product
+    if (cnb::cgemm_tc_fits(64, N, N) && (!cnb::fft_supported(N) || (key & kTriKey))) {
+        // The matrix is a constant: where the GEMM is the transform's engine, it is packed here, not by every product.  Small
+        // batches may be left to FMAs (up to 122 rows of 256 points); which batch comes first says nothing about later ones.
+        // Packed with every product it took 1 us of 20 at 4000 rows.
         const int pitch = (N + 7) & ~7;
         rc = cnb_alloc(ctx, 256 + 8 * (size_t) N * pitch, &t->pack);
         if (rc != CNB_OK) return rc;
