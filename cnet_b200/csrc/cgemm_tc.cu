@@ -84,9 +84,12 @@ template <bool PAIR> struct Cfg {
 };
 constexpr int OPERAND_BYTES = 3 * 8 * PLANE_BYTES;   // 192 KB of operand stages in both forms
 constexpr int EPI_GROUPS = 2, EPI_THREADS = 128 * EPI_GROUPS;
-// Threads: DRAIN, three warpgroups (two warps of the first have nothing to do), with this many registers a thread of the first
-// and of the epilogue's two out of what all are launched with; else the two warps and the epilogue.
-template <bool DRAIN> struct Threads { static constexpr int FIRST_EPI = DRAIN ? 128 : 64, ALL = FIRST_EPI + EPI_THREADS; };
+// What becomes of the accumulators: written out (NONE), or taken into running sums in registers, each while the other is still
+// multiplied (OVERLAP) or both together (EXACT).
+enum Drain { NONE = 0, OVERLAP = 1, EXACT = 2 };
+// Threads: running sums, three warpgroups (two warps of the first have nothing to do), with this many registers a thread of the
+// first and of the epilogue's two out of what all are launched with; else the two warps and the epilogue.
+template <int DRAIN> struct Threads { static constexpr int FIRST_EPI = DRAIN ? 128 : 64, ALL = FIRST_EPI + EPI_THREADS; };
 constexpr int LAUNCH_REGS = 168, ISSUE_REGS = 56, EPI_REGS = 224;
 static_assert(128 * ISSUE_REGS + EPI_THREADS * EPI_REGS <= Threads<true>::ALL * LAUNCH_REGS, "registers");
 constexpr int EPI_BYTES = EPI_GROUPS * 2 * 128 * 16 * 4;  // 32 KB: one epilogue round of both groups, re and im staging
@@ -104,7 +107,7 @@ struct TcParams {
     int cluster;              // > 1: that many CTAs of one cluster share a tile, each a slice of K
     int whole_per_cta;        // > 0: every CTA first takes that many whole tiles, then its run of the remaining units
     int segments;             // > 0: CTA r takes k-segment r / tiles of tile r % tiles (units_per_cta k-blocks each)
-    int chain, small_first;   // PACKED: k-blocks that are summed in tensor memory at most; whether runs are longer than that
+    int chain;                // PACKED: k-blocks that are summed in tensor memory at most
     const int* a_exp;         // PACKED: the powers of two that A and B were scaled by, or kPlain
     const int* b_exp;
     const void* a_planes; const void* b_planes;       // PACKED: what the tensor maps describe, for the FMA form
@@ -343,6 +346,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+    uint32_t r[8];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 // Packed operands: a matrix that is stored as fp32 planes instead of fp16 parts has this for its exponent.
 constexpr int kPlain = 1 << 20;
 
@@ -390,6 +402,24 @@ template <int ACC> __device__ __forceinline__ void drain_chain(uint32_t tl, floa
         for (int i = 0; i < 16; ++i) {
             if (ACC == 0) { sr[c + i] += x[i]; si[c + i] -= sgn * y[i]; }
             else { si[c + i] += x[i]; sr[c + i] += sgn * y[i]; }
+        }
+    }
+}
+
+// Both accumulators together: their difference is rounded at the chain's magnitude, and only the sum at the running sums'.
+__device__ __forceinline__ void drain_exact(uint32_t tl, float sgn, float (&sr)[64], float (&si)[64]) {
+#pragma unroll
+    for (int c = 0; c < 64; c += 8) {
+        float a[8], f[8], b[8], e[8];
+        tmem_ld8(tl + c, a);                             // A_re.B_re
+        tmem_ld8(tl + 384 + c, f);                       // A_im.B_im
+        tmem_ld8(tl + 128 + c, b);                       // A_re.B_im
+        tmem_ld8(tl + 256 + c, e);                       // A_im.B_re
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            sr[c + i] += a[i] + sgn * f[i];
+            si[c + i] += e[i] - sgn * b[i];
         }
     }
 }
@@ -567,13 +597,16 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 // VEC: rows of D and R are 16-byte aligned (N % 4 == 0); the form without it writes 32 consecutive floats of a row per
 // warp instruction instead of four 16-byte pieces of four rows.
 // DRAIN: a run of more than p.chain k-blocks is cut into chains of that many; after each the epilogue takes the
-// accumulators into running sums in registers (max_chain says why), one while the other is still multiplied, so that the
-// MMAs hardly wait: 777 x 1333 -> 1001 forward, six chains, 40.3 -> 33.7 us beside one accumulator barrier and the epilogue
-// on its share of 168 registers.  The same form runs where a CTA goes through several tiles: a tile leaves tensor memory in
-// 0.3 us and is written out under the next one's MMAs (4096 x 1024 x 1024 76 -> 70 us).  Launches of one chain and one tile
-// a CTA take the form without: they leave registers of the SM to the kernels around them, and their set-up runs under the
-// tail of the kernel before (512-row training step 772 -> 743 us).
-template <bool PAIR, bool VEC, int FORM, bool DRAIN>
+// accumulators into running sums in registers (max_chain says why).
+// OVERLAP: one while the other is still multiplied, so that the MMAs hardly wait.  Where a CTA goes through several tiles, and
+// for the chains of sizes that were split products: a tile leaves tensor memory in 0.3 us and is written out under the next
+// one's MMAs (4096 x 1024 x 1024 75 -> 70 us).
+// EXACT: both together, so that a chain costs one rounding at the magnitude of the running sums and not two.  For the short chains
+// of the other sizes, which are to be no further off than fp32 FMAs: 777 x 1333 -> 1001 forward, eleven chains, 4.44e-7 off
+// float64 and 48.2 us with the packing, 4.61e-7 and 46.8 as OVERLAP.
+// Launches of one chain and one tile a CTA (NONE) leave registers of the SM to the kernels around them, and their set-up
+// runs under the tail of the kernel before (512-row training step 772 -> 743 us).
+template <bool PAIR, bool VEC, int FORM, int DRAIN>
 __global__ void __launch_bounds__(Threads<DRAIN>::ALL, 1)
 cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__ TcParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -583,8 +616,8 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
     constexpr int STAGES = Cfg<PAIR>::STAGES, STAGE_BYTES = Cfg<PAIR>::STAGE_BYTES, TILE_M = Cfg<PAIR>::TILE_M;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OPERAND_BYTES + EPI_BYTES);
-    // bars[0..S) full, bars[S..2S) empty, bars[2S] accumulators ready, bars[2S+1] accumulators drained; DRAIN: these two of
-    // acc1, bars[2S+2] and bars[2S+3] of acc2
+    // bars[0..S) full, bars[S..2S) empty, bars[2S] accumulators ready, bars[2S+1] accumulators drained; OVERLAP: these two
+    // of acc1, bars[2S+2] and bars[2S+3] of acc2
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -788,7 +821,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     return done;
                 };
-                if constexpr (!DRAIN) { ok = drained(acc_empty); if (!ok) break; }
+                if constexpr (DRAIN != OVERLAP) { ok = drained(acc_empty); if (!ok) break; }
                 for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
                     int s = (int) (it % STAGES);
                     uint32_t phase = (uint32_t) (it / STAGES) & 1;
@@ -809,24 +842,17 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                             if constexpr (PAIR) umma2_bf16(tmem_base + 256 * acc, ad, bd, idesch, add);
                             else umma_bf16(tmem_base + 256 * acc, ad, bd, idesch, add);
                         };
-                        // DRAIN: at a chain's ends the accumulators take turns by the block: acc1 is summed up while acc2 of the
-                        // chain's last block is multiplied, acc2 while acc1 of the next chain's first block is.  Where runs
-                        // are cut the small terms of a block come first there, so that in a chain of one block they meet a
-                        // small accumulator (K = 50: 1.5e-7 -> 1.1e-7 off float64, FMAs 1.3e-7).
+                        // OVERLAP: at a chain's ends the accumulators take turns by the block: acc1 is summed up while acc2 of
+                        // the chain's last block is multiplied, acc2 while acc1 of the next chain's first block is.
+                        // EXACT: the small terms of a block come first, so that in a chain of one block they meet a small
+                        // accumulator (K = 50: 1.5e-7 -> 1.1e-7 off float64, FMAs 1.3e-7).
                         const bool last = kb + 1 == kb1;
-                        if (DRAIN && (kb == kb0 || last)) {
+                        if (DRAIN == OVERLAP && (kb == kb0 || last)) {
 #pragma unroll
                             for (int acc = 0; acc < 2; ++acc) {
                                 if (kb == kb0 && !drained(acc ? acc2_empty : acc_empty)) { ok = false; break; }
 #pragma unroll
-                                for (int j = 0; j < BK / 16; ++j) {
-                                    mma(j, acc, 0); mma(j, acc, 1);
-                                    if (!p.small_first) mma(j, acc, 2);
-                                }
-                                if (p.small_first) {
-#pragma unroll
-                                    for (int j = 0; j < BK / 16; ++j) mma(j, acc, 2);
-                                }
+                                for (int j = 0; j < BK / 16; ++j) { mma(j, acc, 0); mma(j, acc, 1); mma(j, acc, 2); }
                                 if (acc == 1) { if constexpr (PAIR) umma2_commit_both(empty_bar(s), lead_rank); else umma_commit(empty_bar(s)); }
                                 if (last) {
                                     const uint32_t bar = acc ? acc2_full : acc_full;
@@ -837,7 +863,14 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
 #pragma unroll
                             for (int j = 0; j < BK / 16; ++j)
 #pragma unroll
-                                for (int acc = 0; acc < 2; ++acc) { mma(j, acc, 0); mma(j, acc, 1); mma(j, acc, 2); }
+                                for (int acc = 0; acc < 2; ++acc) {
+                                    mma(j, acc, 0); mma(j, acc, 1);
+                                    if (DRAIN != EXACT) mma(j, acc, 2);
+                                }
+                            if (DRAIN == EXACT) {
+#pragma unroll
+                                for (int j = 0; j < BK / 16; ++j) { mma(j, 0, 2); mma(j, 1, 2); }
+                            }
                             if constexpr (PAIR) umma2_commit_both(empty_bar(s), lead_rank); else umma_commit(empty_bar(s));
                         }
                         continue;
@@ -905,7 +938,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                     umma_commit(empty_bar(s));       // the stage is free once these MMAs have read it
                     }
                 }
-                if (ok && !DRAIN) { if constexpr (PAIR) umma2_commit_both(acc_full, lead_rank); else umma_commit(acc_full); }
+                if (ok && DRAIN != OVERLAP) { if constexpr (PAIR) umma2_commit_both(acc_full, lead_rank); else umma_commit(acc_full); }
                 CNB_GSTAMP(3, true);
                 u += kb1 - kb0;
             }
@@ -953,7 +986,8 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                         mbar_wait(full, (uint32_t) seg & 1, abort_flag, p.status, 3);
                         __syncwarp();
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        drain_chain<decltype(acc)::value>(tl + group * 64, sgn, sr, si);
+                        if constexpr (DRAIN == EXACT) drain_exact(tl + group * 64, sgn, sr, si);
+                        else drain_chain<decltype(acc)::value>(tl + group * 64, sgn, sr, si);
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
                         if (lane == 0) {
@@ -962,7 +996,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                         }
                     };
                     sum(std::integral_constant<int, 0>(), acc_full, acc_empty);
-                    sum(std::integral_constant<int, 1>(), acc2_full, acc2_empty);
+                    if constexpr (DRAIN == OVERLAP) sum(std::integral_constant<int, 1>(), acc2_full, acc2_empty);
                 }
                 if (epi_gave_up(group, abort_flag)) return false;
             }
@@ -1728,15 +1762,18 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
         CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, false, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));  \
         CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, true, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));   \
     } while (0)
-        CNB_TC_ATTR(SPLIT, false); CNB_TC_ATTR(PACKED, false); CNB_TC_ATTR(PACKED, true);
+        CNB_TC_ATTR(SPLIT, NONE); CNB_TC_ATTR(PACKED, NONE); CNB_TC_ATTR(PACKED, OVERLAP); CNB_TC_ATTR(PACKED, EXACT);
 #undef CNB_TC_ATTR
-        cudaFuncAttributes fa[4];                        // the shares of a DRAIN launch must add up to what it starts with
-        CNB_CUDA(cudaFuncGetAttributes(&fa[0], cgemm_tc_k<false, false, PACKED, true>));
-        CNB_CUDA(cudaFuncGetAttributes(&fa[1], cgemm_tc_k<false, true, PACKED, true>));
-        CNB_CUDA(cudaFuncGetAttributes(&fa[2], cgemm_tc_k<true, false, PACKED, true>));
-        CNB_CUDA(cudaFuncGetAttributes(&fa[3], cgemm_tc_k<true, true, PACKED, true>));
-        for (const cudaFuncAttributes& f : fa)
-            if (f.numRegs < LAUNCH_REGS) return set_error(CNB_ERR_CUDA, "cgemm_tc: built with %d registers a thread, not %d", f.numRegs, LAUNCH_REGS);
+        // the shares of a launch with running sums must add up to what it starts with
+#define CNB_TC_REGS(P, V, D)                                                                                                \
+    do {                                                                                                                    \
+        cudaFuncAttributes f;                                                                                               \
+        CNB_CUDA(cudaFuncGetAttributes(&f, cgemm_tc_k<P, V, PACKED, D>));                                                   \
+        if (f.numRegs < LAUNCH_REGS) return set_error(CNB_ERR_CUDA, "cgemm_tc: built with %d registers a thread, not %d", f.numRegs, LAUNCH_REGS); \
+    } while (0)
+        CNB_TC_REGS(false, false, OVERLAP); CNB_TC_REGS(false, true, OVERLAP); CNB_TC_REGS(true, false, OVERLAP); CNB_TC_REGS(true, true, OVERLAP);
+        CNB_TC_REGS(false, false, EXACT); CNB_TC_REGS(false, true, EXACT); CNB_TC_REGS(true, false, EXACT); CNB_TC_REGS(true, true, EXACT);
+#undef CNB_TC_REGS
         attr_set[ctx->device & 63] = true;
     }
     if ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im)) & 3)
@@ -1805,22 +1842,22 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     const int k_blocks = (K + bk - 1) / bk;
     const int run = cluster > 1 ? (k_blocks + cluster - 1) / cluster : q.whole_per_cta > 0 ? k_blocks : (int) std::min<long>(q.upc, k_blocks);
     p.chain = chain_blocks(M, N, K, q.joined);
-    p.small_first = run > p.chain;
     // several tiles a CTA (a single tile's runs are not: 83 x 102, K = 13688 took 1.4 us more in that form)
     const int tiles = (M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM) * ((N + BN - 1) / BN);
     const bool several = cluster == 1 && q.segments == 0 && tiles > 1 && (q.whole_per_cta > 0 || q.upc != k_blocks);
-    const bool drain = packed && (run > p.chain || several);
+    const Drain drain = !packed || (run <= p.chain && !several) ? NONE : run > p.chain && !split_sizes(M, N, K) ? EXACT : OVERLAP;
     auto go = [&](auto kernel, const auto& maps) {
-        return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(drain ? Threads<true>::ALL : Threads<false>::ALL), SMEM_BYTES, st,
+        return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(drain == NONE ? Threads<NONE>::ALL : Threads<OVERLAP>::ALL), SMEM_BYTES, st,
                            pair ? 2 * cluster : cluster, maps, p);
     };
     cudaError_t e;
 #define CNB_TC_GO(F, D, maps)                                                                                              \
     (pair ? (vec ? go(cgemm_tc_k<true, true, F, D>, maps) : go(cgemm_tc_k<true, false, F, D>, maps))                       \
           : (vec ? go(cgemm_tc_k<false, true, F, D>, maps) : go(cgemm_tc_k<false, false, F, D>, maps)))
-    if (drain) e = CNB_TC_GO(PACKED, true, maps_p);
-    else if (packed) e = CNB_TC_GO(PACKED, false, maps_p);
-    else e = CNB_TC_GO(SPLIT, false, maps_s);
+    if (!packed) e = CNB_TC_GO(SPLIT, NONE, maps_s);
+    else if (drain == EXACT) e = CNB_TC_GO(PACKED, EXACT, maps_p);
+    else if (drain == OVERLAP) e = CNB_TC_GO(PACKED, OVERLAP, maps_p);
+    else e = CNB_TC_GO(PACKED, NONE, maps_p);
 #undef CNB_TC_GO
     CNB_CUDA(e);
     CNB_LAUNCH_CHECK("cgemm_tc");
