@@ -1705,13 +1705,14 @@ static bool split_sizes(int M, int N, int K) { return K % 8 == 0 && K >= 32 && M
 static int max_chain(int K) { return std::max(1, (int) (4.28 * std::sqrt((double) K) / FormCfg<PACKED>::BK)); }
 
 // The chain of a packed product in k-blocks of 32.  At sizes that were split products, whole tiles of K <= 4096 are one
-// chain; a longer K is cut at choose_schedule's cap, and whole tiles that used to be shared runs (`joined`) at 24, shorter
-// than those were (4096 x 1024 x 1024, two chains of 16: 1.8e-6 off float64, was 3.1e-6; a chain costs a 4096-row training
-// step 1 %).
+// chain, and a longer K is cut at choose_schedule's cap.  Whole tiles that used to be shared runs (`joined`) take two chains
+// at least, of 24 at most: what was shared had shorter chains than a whole tile (4096 x 1024, K = 512: 1.57e-6 off float64,
+// 1.83e-6 as one chain, 0.93e-6 as two; K = 1024 3.11e-6, and 1.83e-6 as two).  A second chain takes up to 2.5 us (K = 256:
+// 34.8 us as shared runs, 23.7 as one chain, 26.2 as two; K = 512 47.1, 37.8, 38.0).
 static int chain_blocks(int M, int N, int K, bool joined) {
     if (!split_sizes(M, N, K)) return max_chain(K);
     const int k_blocks = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK;
-    const int most = K > 4096 ? kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK : joined ? 24 : k_blocks;
+    const int most = K > 4096 ? kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK : joined ? std::max(2, std::min(24, (k_blocks + 1) / 2)) : k_blocks;
     const int chains = (k_blocks + most - 1) / most;
     return (k_blocks + chains - 1) / chains;
 }

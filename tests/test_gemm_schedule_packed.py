@@ -65,7 +65,9 @@ def test_segments_of_known_launches():
 
 @pytest.mark.parametrize("M,N,K,chain", [
     (4096, 1024, 1024, 16),        # 128 tiles on 74 pairs, whole: two chains of 16 where one of 32 would pass 24
-    (4096, 1024, 512, 16),         # the same tiles, short of the cap
+    (4096, 1024, 512, 8),          # the same tiles, short of the cap: two chains all the same
+    (4096, 1024, 96, 2),
+    (4096, 1024, 64, 2),           # two blocks: one chain
     (512, 1024, 1024, 32),         # clusters along K: one chain
     (4096, 4096, 4096, 128),       # whole tiles of K <= 4096: one chain
     (777, 1001, 1333, 4),          # K of no multiple of 8: 4.28 sqrt(1333) = 156 products

@@ -54,3 +54,19 @@ def test_products_of_several_tiles_and_chains(M, N, K, kind):
     first = ctx.linear_fwd(x, w)
     if not s["atomics"]:
         assert torch.equal(again[0], first[0]) and torch.equal(again[1], first[1])
+
+
+@pytest.mark.parametrize("M,N,K", [(4096, 1024, 128), (4096, 1024, 512), (3840, 1152, 256), (4096, 1024, 768)])
+def test_whole_tiles_that_used_to_be_shared_are_no_further_off(M, N, K):
+    """Two chains: 4.2e-9 (cgemm_tc.cu) of half the products, and the operands' 22 bits.  As one chain K = 512 was 1.83e-6 off."""
+    import torch
+    s = _schedule(M, N, K)
+    assert s["whole_per_cta"] == 2 and not s["atomics"], s
+    ctx = Context(arena_bytes=(64 << 20) + 24 * (M * K + N * K + 64 * (M + N + K)))
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(K)
+    planes = lambda *n: (torch.randn(*n, generator=gen, device="cuda"), torch.randn(*n, generator=gen, device="cuda"))
+    full = lambda a: torch.complex(a[0].double(), a[1].double())
+    x, w = planes(M, K), planes(N, K)
+    y, want = full(ctx.linear_fwd(x, w)), full(x) @ full(w).T
+    assert float(torch.linalg.vector_norm(y - want) / torch.linalg.vector_norm(want)) < 4.2e-9 * K / 2 + 2.0 ** -23
