@@ -1704,17 +1704,26 @@ static bool split_sizes(int M, int N, int K) { return K % 8 == 0 && K >= 32 && M
 // may be 4.28 sqrt(K) long, in blocks of 32.
 static int max_chain(int K) { return std::max(1, (int) (4.28 * std::sqrt((double) K) / FormCfg<PACKED>::BK)); }
 
-// The chain of a packed product in k-blocks of 32.  At sizes that were split products, whole tiles of K <= 4096 are one
-// chain, and a longer K is cut at choose_schedule's cap.  Whole tiles that used to be shared runs (`joined`) take two chains
-// at least, of 24 at most: what was shared had shorter chains than a whole tile (4096 x 1024, K = 512: 1.57e-6 off float64,
-// 1.83e-6 as one chain, 0.93e-6 as two; K = 1024 3.11e-6, and 1.83e-6 as two).  A second chain takes up to 2.5 us (K = 256:
-// 34.8 us as shared runs, 23.7 as one chain, 26.2 as two; K = 512 47.1, 37.8, 38.0).
-static int chain_blocks(int M, int N, int K, bool joined) {
-    if (!split_sizes(M, N, K)) return max_chain(K);
-    const int k_blocks = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK;
-    const int most = K > 4096 ? kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK : joined ? std::max(2, std::min(24, (k_blocks + 1) / 2)) : k_blocks;
-    const int chains = (k_blocks + most - 1) / most;
-    return (k_blocks + chains - 1) / chains;
+// The longest run of k-blocks that one CTA sums for a tile.
+static int longest_run(const Schedule& q, int k_blocks) {
+    return q.cluster > 1 ? (k_blocks + q.cluster - 1) / q.cluster : q.whole_per_cta > 0 ? k_blocks : (int) std::min<long>(q.upc, k_blocks);
+}
+
+// The chain of a packed product in k-blocks of 32.
+//
+// At sizes that were split products, whole tiles of K <= 4096 are one chain, and a longer K is cut at choose_schedule's cap.  Whole
+// tiles that used to be shared runs (`joined`) take two chains at least, of 24 at most: what was shared had shorter chains than a
+// whole tile (4096 x 1024, K = 512: 1.57e-6 off float64, 1.83e-6 as one chain, 0.93e-6 as two; K = 1024 3.11e-6, and 1.83e-6 as
+// two).  A second chain takes up to 2.5 us (K = 256: 34.8 us as shared runs, 23.7 as one chain, 26.2 as two; K = 512 47.1,
+// 37.8, 38.0).
+//
+// At others max_chain is the line.  A run of K > 4096 that is longer than the cap is cut as evenly as runs of that length were:
+// 1500 x 1500, K = 4100 in chains of 8, 8, 8 and 2 a run 8.7e-7 off, in chains of 8 throughout 9.3e-7, of 7 7.8e-7.
+static int chain_blocks(int M, int N, int K, const Schedule& q) {
+    const int n = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK, cap = kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK;
+    auto evenly = [](int blocks, int most) { const int chains = (blocks + most - 1) / most; return (blocks + chains - 1) / chains; };
+    if (split_sizes(M, N, K)) return evenly(n, K > 4096 ? cap : q.joined ? std::max(2, std::min(24, (n + 1) / 2)) : n);
+    return K > 4096 && longest_run(q, n) > cap ? evenly(evenly(n, cap), max_chain(K)) : max_chain(K);
 }
 
 bool cgemm_tc_fits(int M, int N, int K) {
@@ -1839,10 +1848,8 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     p.status = ctx->d_status;
     const bool vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im) |
                                      reinterpret_cast<uintptr_t>(r_re) | reinterpret_cast<uintptr_t>(r_im)) & 15) == 0;
-    // the longest run of k-blocks that one CTA sums for a tile
-    const int k_blocks = (K + bk - 1) / bk;
-    const int run = cluster > 1 ? (k_blocks + cluster - 1) / cluster : q.whole_per_cta > 0 ? k_blocks : (int) std::min<long>(q.upc, k_blocks);
-    p.chain = chain_blocks(M, N, K, q.joined);
+    const int k_blocks = (K + bk - 1) / bk, run = longest_run(q, k_blocks);
+    p.chain = chain_blocks(M, N, K, q);
     // several tiles a CTA (a single tile's runs are not: 83 x 102, K = 13688 took 1.4 us more in that form)
     const int tiles = (M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM) * ((N + BN - 1) / BN);
     const bool several = cluster == 1 && q.segments == 0 && tiles > 1 && (q.whole_per_cta > 0 || q.upc != k_blocks);
@@ -1965,5 +1972,5 @@ extern "C" int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm
     if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0)
         return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_chain_packed: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
     const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK);
-    return cnb::chain_blocks(M, N, K, q.joined);
+    return cnb::chain_blocks(M, N, K, q);
 }

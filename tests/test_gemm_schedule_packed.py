@@ -41,17 +41,22 @@ def _check_segments(s, M, N, K):
 
 @pytest.mark.parametrize("limit", LIMITS)
 @pytest.mark.parametrize("M,N,K", [(2000, 2000, 60000), (130, 1030, 9000), (700, 515, 8200), (1024, 8192, 16384), (100, 2048, 16384), (64, 64, 100000),
-                                   (1000, 2050, 4104), (4096, 4096, 8192)])
+                                   (1000, 2050, 4104), (4096, 4096, 8192), (1500, 1500, 4100), (700, 1301, 9001), (1069, 38, 4215)])
 def test_a_long_k_is_cut_into_chains(M, N, K, limit):
     """Whatever the form of the launch (segments, whole tiles, short runs), no more than 1024 products are summed in tensor
-    memory at sizes of multiples of 8, and 4.28 sqrt(K) at others; a chain is no shorter than an equal cut at that length makes it."""
+    memory at sizes of multiples of 8, and 4.28 sqrt(K) at others; a chain is no shorter than an equal cut at that length makes
+    it, of K or (others, where a run is longer than 1024 products) of the runs that K was once cut into."""
     s = _schedule(M, N, K, 0, limit)
     chain = L.load().cnb_gemm_chain_packed(M, N, K, 0, SMS, limit)
     k_blocks = -(-K // 32)
     if K % 8 == 0:
         assert chain == -(-k_blocks // -(-k_blocks // 32)), (chain, s)
     else:
-        assert chain == int(4.28 * K ** 0.5 / 32), chain
+        most = int(4.28 * K ** 0.5 / 32)
+        former = -(-k_blocks // -(-k_blocks // 32))
+        cluster = s["cluster_ctas"] // (2 if s["pair"] else 1)
+        run = -(-k_blocks // cluster) if cluster > 1 else k_blocks if s["whole_per_cta"] else min(s["run"], k_blocks)
+        assert chain == (-(-former // -(-former // most)) if run > 32 else most), (chain, s)
     if s["segments"]:
         _check_segments(s, M, N, K)
     elif s["whole_per_cta"] and not s["atomics"]:
@@ -72,6 +77,9 @@ def test_segments_of_known_launches():
     (4096, 4096, 4096, 128),       # whole tiles of K <= 4096: one chain
     (777, 1001, 1333, 4),          # K of no multiple of 8: 4.28 sqrt(1333) = 156 products
     (50, 70, 50, 1),
+    (1500, 1500, 4100, 7),         # 129 blocks in one run, cut as the 26 of a fifth were: four chains
+    (700, 1301, 9001, 11),         # as 32 blocks in three chains
+    (1069, 38, 4215, 8),           # short runs: 4.28 sqrt(4215) = 277 products
 ])
 def test_chains(M, N, K, chain):
     assert L.load().cnb_gemm_chain_packed(M, N, K, 0, SMS, 0) == chain
