@@ -107,7 +107,7 @@ struct TcParams {
     int cluster;              // > 1: that many CTAs of one cluster share a tile, each a slice of K
     int whole_per_cta;        // > 0: every CTA first takes that many whole tiles, then its run of the remaining units
     int segments;             // > 0: CTA r takes k-segment r / tiles of tile r % tiles (units_per_cta k-blocks each)
-    int chain;                // PACKED: k-blocks that are summed in tensor memory at most
+    int chain, first;         // PACKED: k-blocks that are summed in tensor memory at most; the same of a tile's first ones
     const int* a_exp;         // PACKED: the powers of two that A and B were scaled by, or kPlain
     const int* b_exp;
     const void* a_planes; const void* b_planes;       // PACKED: what the tensor maps describe, for the FMA form
@@ -814,7 +814,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             for (long u = run_begin(r), ue = run_end(r); u < ue && ok; ++seg) {
                 int kb0 = (int) (u % k_blocks);
                 int kb1 = (int) min((long) k_blocks, kb0 + (ue - u));
-                if constexpr (DRAIN) kb1 = min(kb1, kb0 + p.chain);      // every chain is a segment of its own here
+                if constexpr (DRAIN) kb1 = min(kb1, kb0 + (kb0 == 0 ? p.first : p.chain));    // every chain is a segment of its own here
                 // the epilogue must have drained the previous segment's accumulators
                 auto drained = [&](uint32_t bar) {
                     const bool done = mbar_wait(bar, (uint32_t) (seg & 1) ^ 1, abort_flag, p.status, 4);
@@ -974,13 +974,13 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
         const int rows = plain ? 0 : p.M;                // plain: nothing is read of D or R, or stored
         const uint32_t stage = smem_base + OPERAND_BYTES + (uint32_t) group * 2 * STAGE_PLANE;
         int seg = 0;
-        // DRAIN: the chains of one segment of `blocks` k-blocks into the running sums; false after a wait gave up
+        // DRAIN: the chains of the k-blocks from `kb` to `end` of a tile into the running sums; false after a wait gave up
         float sr[DRAIN ? 64 : 1], si[DRAIN ? 64 : 1];
-        auto sum_chains = [&](int blocks) {
+        auto sum_chains = [&](int kb, int end) {
             if constexpr (DRAIN) {
 #pragma unroll
                 for (int i = 0; i < 64; ++i) sr[i] = si[i] = 0.f;
-                for (int done = 0; done < blocks; done += p.chain, ++seg) {
+                for (; kb < end; kb += kb == 0 ? p.first : p.chain, ++seg) {
                     // every warp by itself; after a wait gave up the others end at once
                     auto sum = [&](auto acc, uint32_t full, uint32_t empty) {
                         mbar_wait(full, (uint32_t) seg & 1, abort_flag, p.status, 3);
@@ -1013,7 +1013,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                 }
             }
             if constexpr (DRAIN) {
-                if (sum_chains((int) (u_end - u_begin))) {           // after the last chain the stages are idle
+                if (sum_chains((int) (u_begin % k_blocks), (int) (u_begin % k_blocks) + (int) (u_end - u_begin))) {           // after the last chain the stages are idle
 #pragma unroll
                     for (int i = 0; i < 64; i += 4) {
                         const uint32_t o = smem_base + 4u * (uint32_t) part_off(row, group * 16 + (i >> 2));
@@ -1085,7 +1085,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             const int c_first = group * 64, c_last = c_first + 48;
             if (pre) request(c_first, 0);
             if constexpr (DRAIN) {
-                if (!sum_chains(kb1 - kb0)) { live = false; break; }
+                if (!sum_chains(kb0, kb1)) { live = false; break; }
             } else {
                 mbar_wait(acc_full, (uint32_t) seg & 1, abort_flag, p.status, 3);
                 if (epi_gave_up(group, abort_flag)) { live = false; break; }
@@ -1709,7 +1709,7 @@ static int longest_run(const Schedule& q, int k_blocks) {
     return q.cluster > 1 ? (k_blocks + q.cluster - 1) / q.cluster : q.whole_per_cta > 0 ? k_blocks : (int) std::min<long>(q.upc, k_blocks);
 }
 
-// The chain of a packed product in k-blocks of 32.
+// The chains of a packed product in k-blocks of 32: a tile's first ones, and those of all others.
 //
 // At sizes that were split products, whole tiles of K <= 4096 are one chain, and a longer K is cut at choose_schedule's cap.  Whole
 // tiles that used to be shared runs (`joined`) take two chains at least, of 24 at most: what was shared had shorter chains than a
@@ -1719,11 +1719,19 @@ static int longest_run(const Schedule& q, int k_blocks) {
 //
 // At others max_chain is the line.  A run of K > 4096 that is longer than the cap is cut as evenly as runs of that length were:
 // 1500 x 1500, K = 4100 in chains of 8, 8, 8 and 2 a run 8.7e-7 off, in chains of 8 throughout 9.3e-7, of 7 7.8e-7.
-static int chain_blocks(int M, int N, int K, const Schedule& q) {
+// `joined` there: what whole chains leave of K, or one of them, goes to both ends (4089 x 1019, K = 777, 25 blocks: 3.36e-7 off
+// as shared runs, 3.39e-7 as 8 x 3 + 1, 3.27e-7 as 2 + 7 x 3 + 2; 3321 x 1275, K = 250, 8 blocks: 2.22e-7, 2.27e-7 as 4 x 2, 2.06e-7
+// as 1 + 3 x 2 + 1).
+struct Chains { int first, rest; };
+static Chains chain_blocks(int M, int N, int K, const Schedule& q) {
     const int n = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK, cap = kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK;
     auto evenly = [](int blocks, int most) { const int chains = (blocks + most - 1) / most; return (blocks + chains - 1) / chains; };
-    if (split_sizes(M, N, K)) return evenly(n, K > 4096 ? cap : q.joined ? std::max(2, std::min(24, (n + 1) / 2)) : n);
-    return K > 4096 && longest_run(q, n) > cap ? evenly(evenly(n, cap), max_chain(K)) : max_chain(K);
+    if (split_sizes(M, N, K)) {
+        const int c = evenly(n, K > 4096 ? cap : q.joined ? std::max(2, std::min(24, (n + 1) / 2)) : n);
+        return {c, c};
+    }
+    const int c = K > 4096 && longest_run(q, n) > cap ? evenly(evenly(n, cap), max_chain(K)) : max_chain(K);
+    return {q.joined && n > c ? (n % c + c + 1) / 2 : c, c};
 }
 
 bool cgemm_tc_fits(int M, int N, int K) {
@@ -1849,7 +1857,9 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     const bool vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im) |
                                      reinterpret_cast<uintptr_t>(r_re) | reinterpret_cast<uintptr_t>(r_im)) & 15) == 0;
     const int k_blocks = (K + bk - 1) / bk, run = longest_run(q, k_blocks);
-    p.chain = chain_blocks(M, N, K, q);
+    const Chains chains = chain_blocks(M, N, K, q);
+    p.chain = chains.rest;
+    p.first = chains.first;
     // several tiles a CTA (a single tile's runs are not: 83 x 102, K = 13688 took 1.4 us more in that form)
     const int tiles = (M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM) * ((N + BN - 1) / BN);
     const bool several = cluster == 1 && q.segments == 0 && tiles > 1 && (q.whole_per_cta > 0 || q.upc != k_blocks);
@@ -1972,5 +1982,5 @@ extern "C" int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm
     if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0)
         return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_chain_packed: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
     const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK);
-    return cnb::chain_blocks(M, N, K, q);
+    return cnb::chain_blocks(M, N, K, q).rest;
 }
