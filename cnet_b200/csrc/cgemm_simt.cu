@@ -6,18 +6,19 @@
 // on its way while one is worked on.  What bounds them is the chain of a CTA's slabs, each a round trip to L2, and few CTAs:
 // with tiles of 64 x 64 and slabs of 16, fetched and then worked on, 64 x 64 -> 32 took 12 us and 128 x 128, K = 128 23 us
 // (now 2.8 and 5.2), 2000 x 50 -> 50 13 (6.0), 500 x 900, K = 26 9.1 (6.8), 2000 x 2000, K = 18 54 (32).  The terms of an
-// output are added one by one in the order of k whatever the tile.
+// output are added one by one in the order of k whatever the tile, but for the products that cgemm_fma_in_chains names.
 #include "common.cuh"
 
 namespace {
 
 // What the kernels before this one may still be writing is read by ordinary loads behind cnb_pdl_enter.
-template <int T>
+// CHAINS: the terms of an output are added up in sixteens, and the sums of these in turn.
+template <int T, bool CHAINS>
 __global__ void __launch_bounds__(256)
 cgemm_simt_k(const float* a_re, const float* a_im, long sam, long sak, const float* b_re, const float* b_im, long sbn, long sbk,
              int conjB, const float* r_re, const float* r_im, float* d_re, float* d_im, int M, int N, int K, int accumulate) {
     cnb_pdl_enter();
-    constexpr int SLAB = 32, U = T / 16, LOADS = T * SLAB / 256;
+    constexpr int SLAB = 32, U = T / 16, LOADS = T * SLAB / 256, CHAIN = 16;
     __shared__ float2 As[2][SLAB][T + 1], Bs[2][SLAB][T + 1];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int tiles_n = (N + T - 1) / T, m0 = (int) (blockIdx.x / (unsigned) tiles_n) * T, n0 = (int) (blockIdx.x % (unsigned) tiles_n) * T;
@@ -35,7 +36,13 @@ cgemm_simt_k(const float* a_re, const float* a_im, long sam, long sak, const flo
             if (gn < N && kb < K) { const size_t o = (size_t) gn * sbn + (size_t) kb * sbk; nb[j] = make_float2(b_re[o], b_im[o]); }
         }
     };
-    float cr[U][U] = {}, ci[U][U] = {};
+    float cr[U][U] = {}, ci[U][U] = {}, sr[U][U] = {}, si[U][U] = {};
+    auto end_chain = [&] {
+#pragma unroll
+        for (int i = 0; i < U; ++i)
+#pragma unroll
+            for (int j = 0; j < U; ++j) { sr[i][j] += cr[i][j]; si[i][j] += ci[i][j]; cr[i][j] = ci[i][j] = 0.f; }
+    };
     fetch(0);
     for (int k0 = 0, s = 0; k0 < K; k0 += SLAB, s ^= 1) {
 #pragma unroll
@@ -62,10 +69,16 @@ cgemm_simt_k(const float* a_re, const float* a_im, long sam, long sak, const flo
         };
         if (K - k0 >= SLAB) {
 #pragma unroll
-            for (int kk = 0; kk < SLAB; ++kk) step(kk);
+            for (int kk = 0; kk < SLAB; ++kk) {
+                step(kk);
+                if (CHAINS && kk % CHAIN == CHAIN - 1) end_chain();
+            }
         } else {
 #pragma unroll 4
-            for (int kk = 0; kk < K - k0; ++kk) step(kk);
+            for (int kk = 0; kk < K - k0; ++kk) {
+                step(kk);
+                if (CHAINS && (kk % CHAIN == CHAIN - 1 || kk + 1 == K - k0)) end_chain();
+            }
         }
     }
 #pragma unroll
@@ -75,7 +88,7 @@ cgemm_simt_k(const float* a_re, const float* a_im, long sam, long sak, const flo
             const int gm = m0 + ty + 16 * i, gn = n0 + tx + 16 * j;
             if (gm >= M || gn >= N) continue;
             const size_t o = (size_t) gm * N + gn;
-            float vr = cr[i][j], vi = ci[i][j];
+            float vr = CHAINS ? sr[i][j] : cr[i][j], vi = CHAINS ? si[i][j] : ci[i][j];
             if (r_re) { vr += r_re[o]; vi += r_im[o]; }
             if (accumulate) { vr += d_re[o]; vi += d_im[o]; }
             d_re[o] = vr; d_im[o] = vi;
@@ -97,7 +110,9 @@ int cgemm_simt(cnb_ctx* ctx, const float* a_re, const float* a_im, long sam, lon
     // K (30 x 20, K = 3000: 156 us with the others, 85), up to six of a short K (4096 x 16, K = 100: 14.6 and 9.8; 1000 x
     // 60, K = 1000, two to an SM: 77 and 81).
     const long small = (long) ((M + 15) / 16) * ((N + 15) / 16), large = (long) ((M + 31) / 32) * ((N + 31) / 32);
-    CNB_CUDA(small <= ctx->sm_count || (K <= 256 && small <= 6L * ctx->sm_count) ? go(cgemm_simt_k<16>, small) : go(cgemm_simt_k<32>, large));
+    const bool tile16 = small <= ctx->sm_count || (K <= 256 && small <= 6L * ctx->sm_count);
+    if (cgemm_fma_in_chains(M, N, K)) CNB_CUDA(tile16 ? go(cgemm_simt_k<16, true>, small) : go(cgemm_simt_k<32, true>, large));
+    else CNB_CUDA(tile16 ? go(cgemm_simt_k<16, false>, small) : go(cgemm_simt_k<32, false>, large));
     CNB_LAUNCH_CHECK("cgemm_simt");
     return CNB_OK;
 }

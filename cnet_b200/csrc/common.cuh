@@ -80,6 +80,9 @@ int cgemm_simt(cnb_ctx* ctx, const float* a_re, const float* a_im, long sam, lon
 // The sizes that its tiles are made for, and those of them for which it beats the SIMT tiles with the operands still to be packed:
 bool cgemm_tc_fits(int M, int N, int K);
 bool cgemm_tc_shape_ok(int M, int N, int K);
+// Products left to the SIMT tiles by that line whose chains in tensor memory would be shorter than K: summed one by one they
+// would be less exact.
+bool cgemm_fma_in_chains(int M, int N, int K);
 // A packed operand: fp16 high and low parts of a matrix scaled by one power of two (cgemm_tc.cu), the form that
 // everything but the C ABI's split buffers goes through.
 struct PackRequest {
