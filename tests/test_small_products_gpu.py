@@ -58,3 +58,29 @@ def test_small_products_of_ragged_sizes_are_as_exact_as_in_chains(M, N, K):
                     (ctx.linear_bwd_w(g, xt), full(g).T @ full(xt).conj())):
         assert off(y, want) < 1.16e-7
     assert ctx.last_gemm_engine() == 2
+
+
+@pytest.mark.parametrize("M,N,K", [(1000, 500, 64), (1000, 500, 63), (1031, 1001, 65), (777, 1333, 95), (2000, 641, 80), (64, 9000, 128), (7103, 65, 79)])
+def test_large_products_without_room(M, N, K):
+    """Tiles of 64 x 64 (and K = 63, just below them), every operand orientation, on top of a residual or of what is there; the
+    same bits as in smaller tiles, which take some of the rows alone."""
+    import torch
+    ctx = Context(arena_bytes=1 << 20)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(M + N + K)
+    planes = lambda *s: (torch.randn(*s, generator=gen, device="cuda"), torch.randn(*s, generator=gen, device="cuda"))
+    full = lambda a: torch.complex(a[0].double(), a[1].double())
+    tol = 2 * 1.8e-8 * K ** 0.5 + 2.0 ** -23
+    off = lambda y, want: float(torch.linalg.vector_norm(full(y) - want) / torch.linalg.vector_norm(want))
+    x, w, r = planes(M, K), planes(N, K), planes(M, N)
+    wt, g, xt = planes(K, N), planes(K, M), planes(K, N)
+    copy = lambda: (r[0].clone(), r[1].clone())
+    part = lambda a, k: (a[0][:k].contiguous(), a[1][:k].contiguous())
+    few = min(M, 40)
+    y = ctx.linear_fwd(x, w)
+    assert ctx.last_gemm_engine() == 2 and off(y, full(x) @ full(w).T) < tol
+    z = ctx.linear_fwd(part(x, few), w)
+    assert torch.equal(y[0][:few], z[0]) and torch.equal(y[1][:few], z[1])
+    assert off(ctx.linear_fwd(x, w, res=r), full(x) @ full(w).T + full(r)) < tol
+    assert off(ctx.linear_bwd_x(x, wt, out=copy()), full(r) + full(x) @ full(wt).conj()) < tol
+    assert off(ctx.linear_bwd_w(g, xt, out=copy()), full(r) + full(g).T @ full(xt).conj()) < tol
