@@ -600,7 +600,7 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 // accumulators into running sums in registers (max_chain says why).
 // OVERLAP: one while the other is still multiplied, so that the MMAs hardly wait.  Where a CTA goes through several tiles, and
 // for the chains of sizes that were split products: a tile leaves tensor memory in 0.3 us and is written out under the next
-// one's MMAs (4096 x 1024 x 1024 75 -> 70 us).
+// one's MMAs (4096 x 1024 x 1024 74.4 -> 69.8 us).
 // EXACT: both together, so that a chain costs one rounding at the magnitude of the running sums and not two.  For the short chains
 // of the other sizes, which are to be no further off than fp32 FMAs: 777 x 1333 -> 1001 forward, eleven chains, 4.44e-7 off
 // float64 and 48.2 us with the packing, 4.61e-7 and 46.8 as OVERLAP.
@@ -1568,13 +1568,15 @@ constexpr int kMaxChain16 = 64;
 Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int bk) {
     // Schedule, by tile count ("CTA" = one CTA, or the CTA pair of a 256-row tile; sms = how many of them this launch
     // may fill: leaving a few SMs free (gemm_cta_limit) lets a concurrent collective's kernels run beside the GEMM):
-    //  * tiles >= 4 x SMs, or one nearly full wave of one-tile CTAs when D is not read: whole tiles, grid =
-    //    tiles, plain stores, fixed summation order;
+    //  * tiles >= 4 x SMs, or one nearly full wave of one-tile CTAs when D is not read: whole tiles, plain stores, fixed
+    //    summation order; grid = tiles, or (packed operands) one CTA per SM that stays and takes every n-th tile;
     //  * more tiles than SMs: persistent CTAs, one per SM; each takes tiles / SMs whole tiles and then an
     //    equal run of the remaining tiles' k-blocks (summed with atomics), so every SM finishes together
-    //    and only the remainder needs atomics and a cleared output;
+    //    and only the remainder needs atomics and a cleared output.  Packed operands: a remainder that is nearly a wave is
+    //    taken as whole tiles too (below);
     //  * few tiles and short runs: a cluster per tile (below); otherwise plain stream-K.
-    // K > 4096 keeps to stream-K runs: one fp32 accumulation chain in tensor memory that long costs accuracy.
+    // K > 4096: one fp32 accumulation chain in tensor memory that long costs accuracy.  Split operands keep to runs of kMaxChain16
+    // at most; packed ones cut their runs into chains (chain_blocks), and a tile into as few segments as cost least, or none.
     struct Plan { long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles, joined; };
     const int k_blocks = (K + bk - 1) / bk;
     const bool packed = bk == FormCfg<PACKED>::BK;
@@ -1615,7 +1617,9 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
         const long kMaxChain = blocks(kMaxChain16);
         if (packed && !whole_tiles && upc > kMaxChain && k_blocks > blocks(256)) {
             // As few segments as cost least: waves of runs, and what a run costs beside its k-blocks (start, write-out) as
-            // about 9 of them, the cleared output and the atomics as another 5.
+            // about 9 of them, the cleared output and the atomics as another 5.  At 15 sizes, K from 4100 to 65536, the choice took
+            // at most 6.4 % more than the best of one to five (300 x 1024, K = 8192 71.6 us, 67.3 in four; 1024 x 2048, K = 16384
+            // 544, 525 in one), at twelve of them at most 2.1 %.
             long best = 0;
             for (int c = 1; (c - 1) * kMaxChain < k_blocks; ++c) {
                 const long cost = ((long) tiles * c + sms - 1) / sms * ((k_blocks + c - 1) / c + 9) + (c > 1 ? 5 : 0);
@@ -1637,9 +1641,12 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
             ctas = (total + upc - 1) / upc;
         }
         if (packed && tiles > sms && (whole_tiles || (lead_whole && tiles % sms * 10 >= sms * 7))) {
-            // Whole tiles by CTAs that stay: the write-out of one runs under the MMAs of the next.  Also where a remainder
-            // of tiles, nearly a wave of them, would be shared: no cleared output and no atomics (4096 x 1024 x 1024, 128
-            // tiles on 74 pairs: 76 -> 71 us; step of the 4096-row stack 3000 -> 2920).
+            // Whole tiles by CTAs that stay: the write-out of one runs under the MMAs of the next.  Also where a remainder of
+            // tiles, seven tenths of a wave or more, would be shared: no cleared output and no atomics.  Shared and whole on 74 pairs,
+            // us: 0.95 of a wave left (4096 x 1152) K = 512 42.0 and 39.5, K = 1024 80.5 and 74.4, K = 2048 150 and 144; 0.73 (4096 x 1024)
+            // 41.4 and 38.0, 69.7 and 69.8, 134 and 136; 0.62 (2560 x 1536) 40.5 and 36.8, 65.9 and 66.9, 123 and 132.  On top of
+            // what is there, K = 1024: 0.95 79.1 and 76.7, 0.73 67.9 and 71.5, 0.84 of a third wave 111 and 119.  (The line is one for
+            // all K: a long one, and an accumulating product, would have it nearer to a whole wave, a short one at a third.)
             ctas = sms;
             upc = 0;
             q.whole_per_cta = (tiles + sms - 1) / sms;

@@ -262,7 +262,9 @@ int cnb_pack_matrix(cnb_ctx* ctx, const float* re, const float* im, int rows, in
 
 int cnb_linear_pack_ok(int B, int in, int out) {
     if (cnb_linear_split_ok(B, in, out)) return 1;
-    // the line of cgemm_tc_shape_ok, for all three products of a layer together (a batch of 16 rows is K of dW*)
+    // The line of cgemm_tc_fits, for all three products of a layer together (a batch of 16 rows is K of dW*).  Not that of
+    // cgemm_tc_shape_ok, which leaves small products to FMAs because they would have to pack both operands first: a layer packs
+    // X and G once for two products each, and W with the update.
     return (B >= 16 && in >= 48 && out >= 17 && (double) B * in * out >= (double) (1 << 21)) ? 1 : 0;
 }
 
