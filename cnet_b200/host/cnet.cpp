@@ -1353,7 +1353,7 @@ bool CNet::readOutput(int uid, int what, float* re, float* im) {
 	const size_t bytes = n * sizeof(float);
 	if (bounce_ && 2 * bytes <= kBounceBytes) {
 		// One wait: a copy to pageable memory and its wait take 12 us each.  Both planes are the two rows of one copy, whose pitch
-		// may be 2^31 - 1 bytes at most: planes lie as far apart as the allocated batch makes them, of which this may be one row.
+		// is documented up to 2^31 - 1 bytes: planes lie as far apart as the allocated batch makes them, of which this may be a row.
 		cudaStream_t st = (cudaStream_t) stream_;
 		char* const second = static_cast<char*>(bounce_) + bytes;
 		const size_t apart = si >= sr + n ? (size_t) (si - sr) * sizeof(float) : 0;

@@ -39,7 +39,8 @@ def test_part_of_the_allocated_batch(allocated, rows):
 
 
 def test_planes_further_apart_than_a_copy_may_stride():
-    """Planes of 65536 x 8192 floats lie 2^31 bytes apart, one more than the pitch of a 2D copy can be."""
+    """Planes of 65536 x 8192 floats lie 2^31 bytes apart, one more than the documented limit of a 2D copy's pitch
+    (cudaDevAttrMaxPitch; the driver that this was written on takes it all the same)."""
     net = Net()
     spec = configs.build_linear(net, n_in=8192, n_out=2)
     net.allocate(65536)
