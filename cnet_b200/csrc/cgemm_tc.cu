@@ -1349,39 +1349,49 @@ __global__ void __launch_bounds__(256) pack_max_k(const __grid_constant__ PackJo
     }
 }
 
-// Small matrices (those of a 512-row batch, 4 MB) are a chain of round trips: the head, then the data.  Four columns at a time,
-// what a thread converts first is requested before the head is read, each further piece before the stores of the one before,
-// and the head is given back at the end (4096 x 4096 65.9 -> 63.7 us, 300 x 500 5.0 -> 4.5).  Two at a time that is no gain: it
-// takes registers, six CTAs to an SM instead of eight, from loads of 4 bytes that want many in flight (5306 x 3317 82.8
-// us, as plain loops of loads and stores 77.9).  VEC: all matrices go four columns at a time.
-template <int N, bool VEC>
-__global__ void __launch_bounds__(256, VEC ? 6 : 0) pack_k(const __grid_constant__ PackJobs<N> jobs) {
+// Small matrices (those of a 512-row batch, 4 MB) are a chain of round trips: the head, then the data.  AHEAD: what a thread
+// converts first is requested before the head is read, each further piece before the stores of the one before, and the head is
+// given back at the end (4096 x 4096 65.9 -> 63.7 us, 300 x 500 5.0 -> 4.5, 1000 x 1001 9.8 -> 8.4).  Two columns at a time that
+// is no gain where there are more blocks than are resident: it takes registers, six CTAs to an SM instead of eight, from loads of
+// 4 bytes that want many in flight (5306 x 3317 82.8 us, as plain loops of loads and stores 77.9; 1001 x 1333, nine blocks to an
+// SM, 10.2 and 9.5; 777 x 1333, seven, 8.6 and 9.1).
+template <int N, bool AHEAD>
+__global__ void __launch_bounds__(256) pack_k(const __grid_constant__ PackJobs<N> jobs) {
     cnb_pdl_enter();
     const PackJob& job = jobs.j[blockIdx.y];
     if ((int) blockIdx.x >= job.blocks) return;
     // Consecutive threads take consecutive columns: four each where the rows allow 16-byte loads (8-byte stores), else
     // two (4-byte accesses), so that every access of a warp is one run.
-    const bool vec = VEC || pack_vec(job);
+    const bool vec = pack_vec(job);
     const size_t np = (size_t) job.rows * job.pitch;
     const int groups = vec ? job.cols / 4 : (job.cols + 1) / 2;
     const size_t total = (size_t) job.rows * groups;
     // rows without padding are one run; else a 32-bit division where it does (a 64-bit one was half the kernel's time)
     const bool flat = vec && job.pitch == job.cols;
-    auto row_of = [&](size_t i) { return flat ? 0 : total >> 32 ? (int) (i / groups) : (int) ((unsigned) i / (unsigned) groups); };
     struct Item { float4 x, y; size_t dst; };
     auto fetch = [&](size_t i) {
         Item v;
-        const int row = row_of(i), g = (int) (i - (size_t) row * groups);
-        const size_t src = flat ? 4 * i : (size_t) row * job.cols + 4 * g;
-        v.dst = flat ? 4 * i : (size_t) row * job.pitch + 4 * g;
-        v.x = *reinterpret_cast<const float4*>(job.re + src);
-        v.y = *reinterpret_cast<const float4*>(job.im + src);
+        const int row = flat ? 0 : total >> 32 ? (int) (i / groups) : (int) ((unsigned) i / (unsigned) groups);
+        const int g = (int) (i - (size_t) row * groups);
+        if (!AHEAD || vec) {
+            const size_t src = flat ? 4 * i : (size_t) row * job.cols + 4 * g;
+            v.dst = flat ? 4 * i : (size_t) row * job.pitch + 4 * g;
+            v.x = *reinterpret_cast<const float4*>(job.re + src);
+            v.y = *reinterpret_cast<const float4*>(job.im + src);
+        } else {
+            const int c = 2 * g;
+            const bool two = c + 1 < job.cols;
+            const size_t src = (size_t) row * job.cols + c;
+            v.dst = (size_t) row * job.pitch + c;
+            v.x = make_float4(job.re[src], two ? job.re[src + 1] : 0.f, 0.f, 0.f);
+            v.y = make_float4(job.im[src], two ? job.im[src + 1] : 0.f, 0.f, 0.f);
+        }
         return v;
     };
     const size_t stride = (size_t) job.blocks * 256;
     size_t i = (size_t) blockIdx.x * 256 + threadIdx.x;
     Item item = {};
-    if (vec && i < total) item = fetch(i);
+    if ((AHEAD || vec) && i < total) item = fetch(i);
     __shared__ int s_exp;
     if (threadIdx.x == 0) {
         const int e = pack_exponent(__ldcg(&job.head->max_bits), __ldcg(&job.head->low_bits));
@@ -1398,28 +1408,30 @@ __global__ void __launch_bounds__(256, VEC ? 6 : 0) pack_k(const __grid_constant
         const float2 f = __half22float2(*hi);
         *lo = __floats2half2_rn(a - f.x, b - f.y);
     };
-    if (!vec) {
+    auto put2 = [&](float x0, float x1, float y0, float y1, size_t dst) {
+        if (plain) {
+            *reinterpret_cast<float2*>(plain_dst + dst) = make_float2(x0, x1);
+            *reinterpret_cast<float2*>(plain_dst + np + dst) = make_float2(y0, y1);
+            return;
+        }
+        __half2 hi, lo;
+        part(x0, x1, &hi, &lo);
+        *reinterpret_cast<__half2*>(job.dst + dst) = hi;
+        *reinterpret_cast<__half2*>(job.dst + 2 * np + dst) = lo;
+        part(y0, y1, &hi, &lo);
+        *reinterpret_cast<__half2*>(job.dst + np + dst) = hi;
+        *reinterpret_cast<__half2*>(job.dst + 3 * np + dst) = lo;
+    };
+    if (!AHEAD && !vec) {
         // (the planes of a pack are nobody else's, so that the loads of several rounds may go before the stores)
         const float* __restrict__ re = job.re;
         const float* __restrict__ im = job.im;
         for (; i < total; i += stride) {
-            const int row = row_of(i), c = 2 * (int) (i - (size_t) row * groups);
+            const int row = total >> 32 ? (int) (i / groups) : (int) ((unsigned) i / (unsigned) groups), c = 2 * (int) (i - (size_t) row * groups);
             const bool two = c + 1 < job.cols;
-            const size_t src = (size_t) row * job.cols + c, dst = (size_t) row * job.pitch + c;
+            const size_t src = (size_t) row * job.cols + c;
             const float x0 = re[src], y0 = im[src];
-            const float x1 = two ? re[src + 1] : 0.f, y1 = two ? im[src + 1] : 0.f;
-            if (plain) {
-                *reinterpret_cast<float2*>(plain_dst + dst) = make_float2(x0, x1);
-                *reinterpret_cast<float2*>(plain_dst + np + dst) = make_float2(y0, y1);
-                continue;
-            }
-            __half2 hi, lo;
-            part(x0, x1, &hi, &lo);
-            *reinterpret_cast<__half2*>(job.dst + dst) = hi;
-            *reinterpret_cast<__half2*>(job.dst + 2 * np + dst) = lo;
-            part(y0, y1, &hi, &lo);
-            *reinterpret_cast<__half2*>(job.dst + np + dst) = hi;
-            *reinterpret_cast<__half2*>(job.dst + 3 * np + dst) = lo;
+            put2(x0, two ? re[src + 1] : 0.f, y0, two ? im[src + 1] : 0.f, (size_t) row * job.pitch + c);
         }
     }
     while (i < total) {
@@ -1427,6 +1439,10 @@ __global__ void __launch_bounds__(256, VEC ? 6 : 0) pack_k(const __grid_constant
         const size_t dst = item.dst;
         i += stride;
         if (i < total) item = fetch(i);                  // the next one, before this one's stores
+        if (AHEAD && !vec) {
+            put2(x.x, x.y, y.x, y.y, dst);
+            continue;
+        }
         if (plain) {
             *reinterpret_cast<float4*>(plain_dst + dst) = x;
             *reinterpret_cast<float4*>(plain_dst + np + dst) = y;
@@ -1909,8 +1925,10 @@ template <int N> static int pack_some(cnb_ctx* ctx, const PackRequest* r, int n,
     bool vec = true;
     for (int k = 0; k < n; ++k) vec = vec && pack_vec(r[k].re, r[k].im, r[k].cols);
     // Enough blocks in all to fill the device a few times over, whatever the number of jobs.  Of two operands the large one's
-    // blocks are to be one wave, six (VEC) or eight CTAs to an SM: 829 x 4812 -> 13 dW* 37.5 us at eight of VEC, 35.9 at six.
+    // blocks are to be one wave, of six CTAs to an SM or (in plain loops) eight: 829 x 4812 -> 13 dW*, all in fours, 37.5 us with
+    // eight blocks to an SM for each of its operands, 35.9 with six.
     const size_t cap = std::max<size_t>(16, (size_t) ctx->sm_count * (vec && n > 1 ? 12 : 16) / n);
+    size_t all = 0;
     for (int k = 0; k < n; ++k) {
         if (reinterpret_cast<uintptr_t>(r[k].planes) & 127 || r[k].pitch % 8)
             return set_error(CNB_ERR_ARG, "pack: planes must be 128-byte aligned, pitch %d a multiple of 8", r[k].pitch);
@@ -1920,11 +1938,12 @@ template <int N> static int pack_some(cnb_ctx* ctx, const PackRequest* r, int n,
         jobs.j[k] = {r[k].re, r[k].im, static_cast<__half*>(r[k].planes), r[k].head, r[k].rows, r[k].cols, r[k].pitch,
                      (int) std::min((items + 255) / 256, cap), (int) std::min(tiles, cap), tiles_x, tiles_y};
         blocks = std::max(blocks, jobs.j[k].blocks);
+        all += jobs.j[k].blocks;
         max_blocks = std::max(max_blocks, jobs.j[k].max_blocks);
     }
     cnb::launch(pack_max_k<N>, dim3(max_blocks, n), dim3(256), 0, st, 1, jobs);
     CNB_LAUNCH_CHECK("pack_max");
-    if (vec) cnb::launch(pack_k<N, true>, dim3(blocks, n), dim3(256), 0, st, 1, jobs);
+    if (vec || all <= 7 * (size_t) ctx->sm_count) cnb::launch(pack_k<N, true>, dim3(blocks, n), dim3(256), 0, st, 1, jobs);
     else cnb::launch(pack_k<N, false>, dim3(blocks, n), dim3(256), 0, st, 1, jobs);
     CNB_LAUNCH_CHECK("pack");
     return CNB_OK;
