@@ -598,12 +598,12 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 // warp instruction instead of four 16-byte pieces of four rows.
 // DRAIN: a run of more than p.chain k-blocks is cut into chains of that many; after each the epilogue takes the
 // accumulators into running sums in registers (max_chain says why).
-// OVERLAP: one while the other is still multiplied, so that the MMAs hardly wait.  Where a CTA goes through several tiles, and
-// for the chains of sizes that were split products: a tile leaves tensor memory in 0.3 us and is written out under the next
-// one's MMAs (4096 x 1024 x 1024 74.4 -> 69.8 us).
-// EXACT: both together, so that a chain costs one rounding at the magnitude of the running sums and not two.  For the short chains
-// of the other sizes, which are to be no further off than fp32 FMAs: 777 x 1333 -> 1001 forward, eleven chains, 4.44e-7 off
-// float64 and 48.2 us with the packing, 4.61e-7 and 46.8 as OVERLAP.
+// OVERLAP: one while the other is still multiplied, so that the MMAs hardly wait.  Where a CTA goes through several tiles (one
+// leaves tensor memory in 0.3 us and is written out under the next one's MMAs: 4096 x 1024 x 1024 74.4 -> 69.8 us), and where
+// chains are long or many (chain_blocks).
+// EXACT: both together, so that a chain costs one rounding at the magnitude of the running sums and not two.  For the few or short
+// chains of sizes that are to be no further off than fp32 FMAs: 466 x 2805, K = 97, four chains of one block, 1.14e-7 off
+// float64 and 1.19e-7 as OVERLAP.
 // Launches of one chain and one tile a CTA (NONE) leave registers of the SM to the kernels around them, and their set-up
 // runs under the tail of the kernel before (512-row training step 772 -> 743 us).
 template <bool PAIR, bool VEC, int FORM, int DRAIN>
@@ -1749,16 +1749,22 @@ static int longest_run(const Schedule& q, int k_blocks) {
 // `joined` there: what whole chains leave of K, or one of them, goes to both ends (4089 x 1019, K = 777, 25 blocks: 3.36e-7 off
 // as shared runs, 3.39e-7 as 8 x 3 + 1, 3.27e-7 as 2 + 7 x 3 + 2; 3321 x 1275, K = 250, 8 blocks: 2.22e-7, 2.27e-7 as 4 x 2, 2.06e-7
 // as 1 + 3 x 2 + 1).
-struct Chains { int first, rest; };
+//
+// Runs by CTA pairs that make five chains or more of at least three blocks take the accumulators out one after the other, and a
+// block less a chain for it: the MMAs wait less, and the second rounding weighs less than the block (4089 x 1019, K = 1001 4.47e-7
+// off as shared runs, 91 us as EXACT, 81 and 3.72e-7 so; 777 x 1001, K = 1333 47.6 -> 45.0 us, 4.44e-7 -> 3.75e-7; a mean of
+// 0.95 over 28 sizes).  In fewer chains, or by single CTAs, that is no gain (1.00 to 1.04 over 85).
+struct Chains { int first, rest; bool exact; };
 static Chains chain_blocks(int M, int N, int K, const Schedule& q) {
     const int n = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK, cap = kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK;
     auto evenly = [](int blocks, int most) { const int chains = (blocks + most - 1) / most; return (blocks + chains - 1) / chains; };
     if (split_sizes(M, N, K)) {
         const int c = evenly(n, K > 4096 ? cap : q.joined ? std::max(2, std::min(24, (n + 1) / 2)) : n);
-        return {c, c};
+        return {c, c, false};
     }
-    const int c = K > 4096 && longest_run(q, n) > cap ? evenly(evenly(n, cap), max_chain(K)) : max_chain(K);
-    return {q.joined && n > c ? (n % c + c + 1) / 2 : c, c};
+    const int run = longest_run(q, n), c = K > 4096 && run > cap ? evenly(evenly(n, cap), max_chain(K)) : max_chain(K);
+    if (q.pair && max_chain(K) >= 3 && run > 4 * c) return {c - 1, c - 1, false};
+    return {q.joined && n > c ? (n % c + c + 1) / 2 : c, c, true};
 }
 
 bool cgemm_tc_fits(int M, int N, int K) {
@@ -1772,9 +1778,11 @@ bool cgemm_tc_fits(int M, int N, int K) {
 }
 
 bool cgemm_tc_shape_ok(int M, int N, int K) {
-    // Small products are done by the SIMT tiles before the operands would be packed: 128 x 128, K = 128 takes 5.3 us there
-    // and 13.6 here, K = 256 8.9 and 14.5, 200 x 100, K = 200 9.9 and 16.7, 200 x 200, K = 200 17.0 and 17.8; 1000 x 100,
-    // K = 200 19 and 16, 300 x 100, K = 300 22 and 17.
+    // Small products are done by the SIMT tiles before the operands would be packed.  FMAs, packing and tiles, us: 128 x 128,
+    // K = 128 4.9 and 13.6, K = 256 8.6 and 14.3, 200 x 100, K = 200 9.9 and 16.7, 200 x 200, K = 200 17.0 and 17.8; 300 x 256,
+    // K = 200, 15 million, 17.9 and 16.7; 300 x 256, K = 256 21.9 and 14.5.  The line is on the safe side: FMAs are ahead to
+    // K = 400 or so where outputs are few (128 x 128, K = 300 9.9 and 17.0, K = 400 12.7 and 16.1, K = 512 15.7 and 14.7), and
+    // beyond 8 million where K is short (1000 x 256, K = 64 9.9 and 12.6; 4000 x 64, K = 100 15.6 and 15.9).
     if (K <= 256 && (double) M * N * K <= 8e6) return false;
     return cgemm_tc_fits(M, N, K);
 }
@@ -1894,7 +1902,7 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     // several tiles a CTA (a single tile's runs are not: 83 x 102, K = 13688 took 1.4 us more in that form)
     const int tiles = (M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM) * ((N + BN - 1) / BN);
     const bool several = cluster == 1 && q.segments == 0 && tiles > 1 && (q.whole_per_cta > 0 || q.upc != k_blocks);
-    const Drain drain = !packed || (run <= p.chain && !several) ? NONE : run > p.chain && !split_sizes(M, N, K) ? EXACT : OVERLAP;
+    const Drain drain = !packed || (run <= p.chain && !several) ? NONE : run > p.chain && chains.exact ? EXACT : OVERLAP;
     auto go = [&](auto kernel, const auto& maps) {
         return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(drain == NONE ? Threads<NONE>::ALL : Threads<OVERLAP>::ALL), SMEM_BYTES, st,
                            pair ? 2 * cluster : cluster, maps, p);

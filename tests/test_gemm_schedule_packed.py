@@ -45,7 +45,8 @@ def _check_segments(s, M, N, K):
 def test_a_long_k_is_cut_into_chains(M, N, K, limit):
     """Whatever the form of the launch (segments, whole tiles, short runs), no more than 1024 products are summed in tensor
     memory at sizes of multiples of 8, and 4.28 sqrt(K) at others; a chain is no shorter than an equal cut at that length makes
-    it, of K or (others, where a run is longer than 1024 products) of the runs that K was once cut into."""
+    it, of K or (others, where a run is longer than 1024 products) of the runs that K was once cut into; a block less where pairs
+    sum five chains or more."""
     s = _schedule(M, N, K, 0, limit)
     chain = L.load().cnb_gemm_chain_packed(M, N, K, 0, SMS, limit)
     k_blocks = -(-K // 32)
@@ -56,7 +57,8 @@ def test_a_long_k_is_cut_into_chains(M, N, K, limit):
         former = -(-k_blocks // -(-k_blocks // 32))
         cluster = s["cluster_ctas"] // (2 if s["pair"] else 1)
         run = -(-k_blocks // cluster) if cluster > 1 else k_blocks if s["whole_per_cta"] else min(s["run"], k_blocks)
-        assert chain == (-(-former // -(-former // most)) if run > 32 else most), (chain, s)
+        c = -(-former // -(-former // most)) if run > 32 else most
+        assert chain == (c - 1 if s["pair"] and most >= 3 and run > 4 * c else c), (chain, s)
     if s["segments"]:
         _check_segments(s, M, N, K)
     elif s["whole_per_cta"] and not s["atomics"]:
@@ -75,10 +77,12 @@ def test_segments_of_known_launches():
     (4096, 1024, 64, 2),           # two blocks: one chain
     (512, 1024, 1024, 32),         # clusters along K: one chain
     (4096, 4096, 4096, 128),       # whole tiles of K <= 4096: one chain
-    (777, 1001, 1333, 4),          # K of no multiple of 8: 4.28 sqrt(1333) = 156 products
+    (777, 1001, 1333, 3),          # K of no multiple of 8: 4.28 sqrt(1333) = 156 products, and a block less for six chains by pairs
+    (77, 1001, 1333, 4),           # single CTAs
+    (777, 1001, 500, 2),           # two blocks at most
     (50, 70, 50, 1),
-    (1500, 1500, 4100, 7),         # 129 blocks in one run, cut as the 26 of a fifth were: four chains
-    (700, 1301, 9001, 11),         # as 32 blocks in three chains
+    (1500, 1500, 4100, 6),         # 129 blocks in one run, cut as the 26 of a fifth were: four chains, and a block less
+    (700, 1301, 9001, 10),         # as 32 blocks in three chains, and a block less
     (1069, 38, 4215, 8),           # short runs: 4.28 sqrt(4215) = 277 products
 ])
 def test_chains(M, N, K, chain):
