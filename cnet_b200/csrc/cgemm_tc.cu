@@ -1746,9 +1746,8 @@ static int longest_run(const Schedule& q, int k_blocks) {
 //
 // At others max_chain is the line.  A run of K > 4096 that is longer than the cap is cut as evenly as runs of that length were:
 // 1500 x 1500, K = 4100 in chains of 8, 8, 8 and 2 a run 8.7e-7 off, in chains of 8 throughout 9.3e-7, of 7 7.8e-7.
-// `joined` there: what whole chains leave of K, or one of them, goes to both ends (4089 x 1019, K = 777, 25 blocks: 3.36e-7 off
-// as shared runs, 3.39e-7 as 8 x 3 + 1, 3.27e-7 as 2 + 7 x 3 + 2; 3321 x 1275, K = 250, 8 blocks: 2.22e-7, 2.27e-7 as 4 x 2, 2.06e-7
-// as 1 + 3 x 2 + 1).
+// `joined` there: what whole chains leave of K, or one of them, goes to both ends (4089 x 1019, K = 500, 16 blocks: 2.29e-7 off
+// as shared runs, 2.30e-7 as 8 x 2, 2.21e-7 as 1 + 7 x 2 + 1; 3321 x 1275, K = 250, 8 blocks: 2.22e-7, 2.27e-7, 2.06e-7).
 //
 // Runs by CTA pairs that make five chains or more of at least three blocks take the accumulators out one after the other, and a
 // block less a chain for it: the MMAs wait less, and the second rounding weighs less than the block (4089 x 1019, K = 1001 4.47e-7
