@@ -62,7 +62,7 @@
 
 namespace {
 
-constexpr int BM = 128, BN = 128;
+constexpr int BM = 128, BN = 128, NARROW = 64;
 constexpr int PLANE_BYTES = 8192;                    // one operand slot of one stage: 128 rows of 64 bytes
 
 // Operand forms.  SPLIT: fp32 hi, bf16 of hi and lo, k-blocks of 16 (the split buffers of the C ABI).  PACKED: two fp16
@@ -77,9 +77,10 @@ template <int FORM> struct OperandMaps { CUtensorMap m[FormCfg<FORM>::MAPS]; };
 // One CTA per tile: 8 slots (A: 4, B: 4) = 64 KB per stage, 3 stages.  A pair of CTAs per 256-row tile
 // (cta_group::2): each CTA stages its own 128 rows of A (4 slots) and one of the two halves of the stacked B
 // operand (B_re rows in the first CTA, B_im rows in the second: 2 slots) = 48 KB per stage, 4 stages.
-template <bool PAIR> struct Cfg {
-    static constexpr int STAGES = PAIR ? 4 : 3;
-    static constexpr int STAGE_BYTES = (PAIR ? 6 : 8) * PLANE_BYTES;
+// A narrow tile of 128 x 64 (PACKED, one CTA): half the slots for B, as in a pair.
+template <bool PAIR, int TN> struct Cfg {
+    static constexpr int STAGES = PAIR || TN == NARROW ? 4 : 3;
+    static constexpr int STAGE_BYTES = (PAIR || TN == NARROW ? 6 : 8) * PLANE_BYTES;
     static constexpr int TILE_M = PAIR ? 2 * BM : BM;
 };
 constexpr int OPERAND_BYTES = 3 * 8 * PLANE_BYTES;   // 192 KB of operand stages in both forms
@@ -94,7 +95,8 @@ constexpr int LAUNCH_REGS = 168, ISSUE_REGS = 56, EPI_REGS = 224;
 static_assert(128 * ISSUE_REGS + EPI_THREADS * EPI_REGS <= Threads<true>::ALL * LAUNCH_REGS, "registers");
 constexpr int EPI_BYTES = EPI_GROUPS * 2 * 128 * 16 * 4;  // 32 KB: one epilogue round of both groups, re and im staging
 constexpr int SMEM_BYTES = OPERAND_BYTES + EPI_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
-static_assert(Cfg<false>::STAGES * Cfg<false>::STAGE_BYTES == OPERAND_BYTES && Cfg<true>::STAGES * Cfg<true>::STAGE_BYTES == OPERAND_BYTES, "stages");
+template <bool PAIR, int TN> constexpr bool fills = Cfg<PAIR, TN>::STAGES * Cfg<PAIR, TN>::STAGE_BYTES == OPERAND_BYTES;
+static_assert(fills<false, BN> && fills<true, BN> && fills<false, NARROW>, "stages");
 constexpr uint32_t TMEM_COLS = 512;
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 
@@ -276,8 +278,8 @@ __device__ __forceinline__ uint64_t smem_desc_mn128_h(uint32_t addr) {
     return d;
 }
 
-// kind::f16 with fp16 operands, fp32 accumulate, M = 128, N = 256
-constexpr uint32_t kInstrDescH = (1u << 4) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
+// kind::f16 with fp16 operands, fp32 accumulate, M = 128, N = both planes of a tile's TN columns
+template <int TN> constexpr uint32_t kInstrDescH = (1u << 4) | (((2u * TN) >> 3) << 17) | ((128u >> 4) << 24);
 
 // kind::f16 with bf16 operands, fp32 accumulate, M = 128, N = 256
 constexpr uint32_t kInstrDesc16 = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
@@ -389,14 +391,14 @@ __device__ __noinline__ void fma_product(const TcParams& p, void* smem) {
                       [] { asm volatile("bar.sync %0, %1;" ::"n"(1 + EPI_GROUPS), "n"(EPI_THREADS) : "memory"); });
 }
 
-// One accumulator of a chain (this thread's row, the 64 columns of its group from `tl` on) into the running sums, rounded
+// One accumulator of a chain (this thread's row, the half of the tile's columns of its group from `tl` on) into the running sums, rounded
 // to nearest: acc1 holds A_re.[B_re ; B_im], acc2 A_im.[B_re ; B_im].  The last load has completed on return.
-template <int ACC> __device__ __forceinline__ void drain_chain(uint32_t tl, float sgn, float (&sr)[64], float (&si)[64]) {
+template <int ACC, int TN> __device__ __forceinline__ void drain_chain(uint32_t tl, float sgn, float (&sr)[TN / 2], float (&si)[TN / 2]) {
 #pragma unroll
-    for (int c = 0; c < 64; c += 16) {
+    for (int c = 0; c < TN / 2; c += 16) {
         float x[16], y[16];
         tmem_ld16(tl + ACC * 256 + c, x);                // . B_re
-        tmem_ld16(tl + ACC * 256 + 128 + c, y);          // . B_im
+        tmem_ld16(tl + ACC * 256 + TN + c, y);           // . B_im
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -407,13 +409,13 @@ template <int ACC> __device__ __forceinline__ void drain_chain(uint32_t tl, floa
 }
 
 // Both accumulators together: their difference is rounded at the chain's magnitude, and only the sum at the running sums'.
-__device__ __forceinline__ void drain_exact(uint32_t tl, float sgn, float (&sr)[64], float (&si)[64]) {
+template <int TN> __device__ __forceinline__ void drain_exact(uint32_t tl, float sgn, float (&sr)[TN / 2], float (&si)[TN / 2]) {
 #pragma unroll
-    for (int c = 0; c < 64; c += 8) {
+    for (int c = 0; c < TN / 2; c += 8) {
         float a[8], f[8], b[8], e[8];
         tmem_ld8(tl + c, a);                             // A_re.B_re
-        tmem_ld8(tl + 384 + c, f);                       // A_im.B_im
-        tmem_ld8(tl + 128 + c, b);                       // A_re.B_im
+        tmem_ld8(tl + 256 + TN + c, f);                  // A_im.B_im
+        tmem_ld8(tl + TN + c, b);                        // A_re.B_im
         tmem_ld8(tl + 256 + c, e);                       // A_im.B_re
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -453,10 +455,10 @@ __device__ __forceinline__ uint32_t stage_off(int row, int chunk) {
 }
 constexpr uint32_t STAGE_PLANE = 128 * 16 * 4;
 
-// Partial tile of one CTA in cluster mode: 128 rows x 128 floats per plane over the (then idle) operand
+// Partial tile of one CTA in cluster mode: 128 rows x TN floats per plane over the (then idle) operand
 // stages, 16-byte chunks XOR-swizzled by the row like the staging tile.
-__device__ __forceinline__ int part_off(int row, int chunk) { return row * 128 + ((chunk ^ (row & 7)) << 2); }
-constexpr int PART_PLANE_BYTES = 128 * 128 * 4;
+template <int TN> __device__ __forceinline__ int part_off(int row, int chunk) { return row * TN + ((chunk ^ (row & 7)) << 2); }
+template <int TN> constexpr int PART_PLANE_BYTES = 128 * TN * 4;
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -472,10 +474,11 @@ __device__ __forceinline__ void l2_prefetch(const float* p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
+template <int TN>
 __device__ __forceinline__ void prefetch_tile_rows(const TcParams& p, const float* re, const float* im, int row,
                                                   int n0) {
     if (row >= p.M || (p.N & 3)) return;
-    const uint32_t bytes = (uint32_t) min(BN, p.N - n0) * 4u;
+    const uint32_t bytes = (uint32_t) min(TN, p.N - n0) * 4u;
     const size_t o = (size_t) row * p.N + n0;
     if (((reinterpret_cast<uintptr_t>(re + o) | reinterpret_cast<uintptr_t>(im + o)) & 15) != 0) return;
     l2_prefetch(re + o, bytes);
@@ -536,12 +539,12 @@ __device__ __forceinline__ float4 ld_peer(uint32_t local_addr, uint32_t rank) {
 // residual, old D) is issued before the first sum, so a round costs one round trip.  Fixed summation order.
 // The CL partial tiles sit in the CTAs of cluster rank peer0 + c * peer_step (one CTA per tile: 0 and 1; CTA pairs:
 // this CTA's rank in its pair and 2: the peers are the CTAs that hold the same 128 rows).
-template <int CL, bool VEC>
+template <int CL, bool VEC, int TN>
 __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_base, uint32_t crank, int m0, int n0,
                                                int et, uint32_t peer0, uint32_t peer_step) {
-    constexpr int ROWS = BM / CL;
+    constexpr int ROWS = BM / CL, LINE = TN / 4;         // chunks in a row
     constexpr int U = CL <= 4 ? 2 : 1;                   // chunks per thread and round
-    for (int base = et; base < ROWS * 32; base += EPI_THREADS * U) {
+    for (int base = et; base < ROWS * LINE; base += EPI_THREADS * U) {
         float4 xr[U][CL], xi[U][CL], vr[U], vi[U];
         size_t o[U];
         bool live[U];
@@ -549,18 +552,18 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int idx = base + EPI_THREADS * u;
-            const int r = (int) crank * ROWS + (idx >> 5), ch = idx & 31;
+            const int r = (int) crank * ROWS + idx / LINE, ch = idx % LINE;
             const int gm = m0 + r;
             gn[u] = n0 + ch * 4;
-            live[u] = idx < ROWS * 32 && gm < p.M && gn[u] < p.N;
+            live[u] = idx < ROWS * LINE && gm < p.M && gn[u] < p.N;
             o[u] = (size_t) gm * p.N + gn[u];
             vr[u] = make_float4(0.f, 0.f, 0.f, 0.f); vi[u] = vr[u];
             if (!live[u]) continue;
-            const uint32_t local = smem_base + 4u * (uint32_t) part_off(r, ch);
+            const uint32_t local = smem_base + 4u * (uint32_t) part_off<TN>(r, ch);
 #pragma unroll
             for (int c = 0; c < CL; ++c) {
                 const uint32_t peer = peer0 + (uint32_t) c * peer_step;
-                xr[u][c] = ld_peer(local, peer); xi[u][c] = ld_peer(local + PART_PLANE_BYTES, peer);
+                xr[u][c] = ld_peer(local, peer); xi[u][c] = ld_peer(local + PART_PLANE_BYTES<TN>, peer);
             }
             if (p.r_re) { vr[u] = ld_global_part<VEC>(p.r_re + o[u], p.N - gn[u]); vi[u] = ld_global_part<VEC>(p.r_im + o[u], p.N - gn[u]); }
             if (p.accumulate) {
@@ -606,14 +609,18 @@ __device__ __forceinline__ void cluster_reduce(const TcParams& p, uint32_t smem_
 // float64 and 1.19e-7 as OVERLAP.
 // Launches of one chain and one tile a CTA (NONE) leave registers of the SM to the kernels around them, and their set-up
 // runs under the tail of the kernel before (512-row training step 772 -> 743 us).
-template <bool PAIR, bool VEC, int FORM, int DRAIN>
+// TN: columns of a tile, BN or NARROW (choose_schedule).
+template <bool PAIR, bool VEC, int FORM, int DRAIN, int TN>
 __global__ void __launch_bounds__(Threads<DRAIN>::ALL, 1)
 cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__ TcParams p) {
+    static_assert(TN == BN || (TN == NARROW && !PAIR && FORM == PACKED && DRAIN != OVERLAP), "narrow tiles");
     extern __shared__ uint8_t smem_raw[];
     constexpr int BK = FormCfg<FORM>::BK;
     CNB_GSTAMP(0, threadIdx.x == 0);
     // operand stages need the alignment of their swizzle pattern; 1024 B covers every mode
-    constexpr int STAGES = Cfg<PAIR>::STAGES, STAGE_BYTES = Cfg<PAIR>::STAGE_BYTES, TILE_M = Cfg<PAIR>::TILE_M;
+    constexpr int STAGES = Cfg<PAIR, TN>::STAGES, STAGE_BYTES = Cfg<PAIR, TN>::STAGE_BYTES, TILE_M = Cfg<PAIR, TN>::TILE_M;
+    constexpr int B_LOW = STAGE_BYTES / PLANE_BYTES == 8 ? 6 : 5;          // PACKED: slot of B's low parts
+    constexpr int HALF = TN / 2;                         // columns of an epilogue group
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OPERAND_BYTES + EPI_BYTES);
     // bars[0..S) full, bars[S..2S) empty, bars[2S] accumulators ready, bars[2S+1] accumulators drained; OVERLAP: these two
@@ -622,7 +629,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tiles_n = (p.N + BN - 1) / BN;
+    const int tiles_n = (p.N + TN - 1) / TN;
     const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
     const int k_blocks = (p.K + BK - 1) / BK;
     const long total_units = (long) tiles_m * tiles_n * k_blocks;
@@ -727,7 +734,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             for (int r = 0; r <= p.whole_per_cta && live; ++r)
             for (long u = run_begin(r), ue = run_end(r); u < ue; ++u, ++it) {
                 int tile = (int) (u / k_blocks), kb = (int) (u % k_blocks);
-                int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
+                int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * TN;
                 int s = (int) (it % STAGES);
                 uint32_t phase = (uint32_t) (it / STAGES) & 1;
                 if (!mbar_wait(empty_bar(s), phase ^ 1, abort_flag, p.status, 1)) { live = false; break; }
@@ -748,7 +755,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                     load(dst, &om.m[0], p.a_mn, m0, 0);
                     load(dst + 2 * PLANE_BYTES, &om.m[1], p.a_mn, m0, 0);
                     load(dst + 4 * PLANE_BYTES, &om.m[2], p.b_mn, n0, PAIR ? (int) prank : 0);
-                    load(dst + (PAIR ? 5 : 6) * PLANE_BYTES, &om.m[3], p.b_mn, n0, PAIR ? (int) prank : 0);
+                    load(dst + B_LOW * PLANE_BYTES, &om.m[3], p.b_mn, n0, PAIR ? (int) prank : 0);
                     continue;
                 } else {
                 const CUtensorMap* maps = om.m;
@@ -807,7 +814,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             const uint32_t m_bits = PAIR ? ((256u >> 4) << 24) - ((128u >> 4) << 24) : 0u;
             const uint32_t idesc = (kInstrDesc | mn_bits) + m_bits, idesc16 = (kInstrDesc16 | mn_bits) + m_bits;
             // PACKED: one thread issues an MMA every 140 cycles; a descriptor is one addition to what is known here
-            const uint32_t idesch = (kInstrDescH | mn_bits) + m_bits;
+            const uint32_t idesch = (kInstrDescH<TN> | mn_bits) + m_bits;
             const uint64_t a_desc = p.a_mn ? smem_desc_mn128_h(0) : smem_desc_sw64(0), b_desc = p.b_mn ? smem_desc_mn128_h(0) : smem_desc_sw64(0);
             const uint32_t a_step = (p.a_mn ? 2048 : 32) >> 4, b_step = (p.b_mn ? 2048 : 32) >> 4;
             for (int r = 0; r <= p.whole_per_cta; ++r)
@@ -832,12 +839,11 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                     uint32_t st = smem_base + s * STAGE_BYTES;
                     const uint32_t first = kb == kb0 ? 0u : 1u;
                     if constexpr (FORM == PACKED) {
-                        constexpr int b_low = PAIR ? 5 : 6;
                         const uint32_t at = (st >> 4) & 0x3FFF;      // (in a cluster the CTA's rank stands above the offset)
                         // term 0: low.high, 1: high.low, 2: high.high
                         auto mma = [&](int j, int acc, int term) {
                             const uint64_t ad = a_desc + (at + (term == 0 ? 2 + acc : acc) * (PLANE_BYTES >> 4) + j * a_step);
-                            const uint64_t bd = b_desc + (at + (term == 1 ? b_low : 4) * (PLANE_BYTES >> 4) + j * b_step);
+                            const uint64_t bd = b_desc + (at + (term == 1 ? B_LOW : 4) * (PLANE_BYTES >> 4) + j * b_step);
                             const uint32_t add = j == 0 && term == 0 ? first : 1u;
                             if constexpr (PAIR) umma2_bf16(tmem_base + 256 * acc, ad, bd, idesch, add);
                             else umma_bf16(tmem_base + 256 * acc, ad, bd, idesch, add);
@@ -975,19 +981,19 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
         const uint32_t stage = smem_base + OPERAND_BYTES + (uint32_t) group * 2 * STAGE_PLANE;
         int seg = 0;
         // DRAIN: the chains of the k-blocks from `kb` to `end` of a tile into the running sums; false after a wait gave up
-        float sr[DRAIN ? 64 : 1], si[DRAIN ? 64 : 1];
+        float sr[DRAIN ? HALF : 1], si[DRAIN ? HALF : 1];
         auto sum_chains = [&](int kb, int end) {
             if constexpr (DRAIN) {
 #pragma unroll
-                for (int i = 0; i < 64; ++i) sr[i] = si[i] = 0.f;
+                for (int i = 0; i < HALF; ++i) sr[i] = si[i] = 0.f;
                 for (; kb < end; kb += kb == 0 ? p.first : p.chain, ++seg) {
                     // every warp by itself; after a wait gave up the others end at once
                     auto sum = [&](auto acc, uint32_t full, uint32_t empty) {
                         mbar_wait(full, (uint32_t) seg & 1, abort_flag, p.status, 3);
                         __syncwarp();
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        if constexpr (DRAIN == EXACT) drain_exact(tl + group * 64, sgn, sr, si);
-                        else drain_chain<decltype(acc)::value>(tl + group * 64, sgn, sr, si);
+                        if constexpr (DRAIN == EXACT) drain_exact<TN>(tl + group * HALF, sgn, sr, si);
+                        else drain_chain<decltype(acc)::value, TN>(tl + group * HALF, sgn, sr, si);
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
                         if (lane == 0) {
@@ -1006,19 +1012,19 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             // the whole k-slice is one segment; its partial sums go to shared memory for the cluster reduction
             {
                 const int tile = blockIdx.x / cluster_ctas, rows_per = BM / p.cluster;
-                const int row = (tile / tiles_n) * TILE_M + row_off + (int) crank * rows_per + et, n0 = (tile % tiles_n) * BN;
+                const int row = (tile / tiles_n) * TILE_M + row_off + (int) crank * rows_per + et, n0 = (tile % tiles_n) * TN;
                 if (group == 0 && et < rows_per) {       // the band of rows this CTA will write out
-                    if (p.r_re) prefetch_tile_rows(p, p.r_re, p.r_im, row, n0);
-                    if (p.accumulate) prefetch_tile_rows(p, p.d_re, p.d_im, row, n0);
+                    if (p.r_re) prefetch_tile_rows<TN>(p, p.r_re, p.r_im, row, n0);
+                    if (p.accumulate) prefetch_tile_rows<TN>(p, p.d_re, p.d_im, row, n0);
                 }
             }
             if constexpr (DRAIN) {
                 if (sum_chains((int) (u_begin % k_blocks), (int) (u_begin % k_blocks) + (int) (u_end - u_begin))) {           // after the last chain the stages are idle
 #pragma unroll
-                    for (int i = 0; i < 64; i += 4) {
-                        const uint32_t o = smem_base + 4u * (uint32_t) part_off(row, group * 16 + (i >> 2));
+                    for (int i = 0; i < HALF; i += 4) {
+                        const uint32_t o = smem_base + 4u * (uint32_t) part_off<TN>(row, (group * HALF + i) >> 2);
                         st_shared4(o, out(sr[i]), out(sr[i + 1]), out(sr[i + 2]), out(sr[i + 3]));
-                        st_shared4(o + PART_PLANE_BYTES, out(si[i]), out(si[i + 1]), out(si[i + 2]), out(si[i + 3]));
+                        st_shared4(o + PART_PLANE_BYTES<TN>, out(si[i]), out(si[i + 1]), out(si[i + 2]), out(si[i + 3]));
                     }
                 }
             } else {
@@ -1027,19 +1033,19 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             if (!epi_gave_up(group, abort_flag)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-                for (int c0 = group * 64; c0 < group * 64 + 64; c0 += 16) {
+                for (int c0 = group * HALF; c0 < group * HALF + HALF; c0 += 16) {
                     float a[16], f[16], b[16], e[16];
                     tmem_ld16(tl + c0, a);                   // A_re.B_re
-                    tmem_ld16(tl + 384 + c0, f);             // A_im.B_im
-                    tmem_ld16(tl + 128 + c0, b);             // A_re.B_im
+                    tmem_ld16(tl + 256 + TN + c0, f);             // A_im.B_im
+                    tmem_ld16(tl + TN + c0, b);             // A_re.B_im
                     tmem_ld16(tl + 256 + c0, e);             // A_im.B_re
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int i = 0; i < 16; i += 4) {
-                        const uint32_t o = smem_base + 4u * (uint32_t) part_off(row, (c0 + i) >> 2);
+                        const uint32_t o = smem_base + 4u * (uint32_t) part_off<TN>(row, (c0 + i) >> 2);
                         st_shared4(o, out(a[i] + sgn * f[i]), out(a[i + 1] + sgn * f[i + 1]), out(a[i + 2] + sgn * f[i + 2]),
                                    out(a[i + 3] + sgn * f[i + 3]));
-                        st_shared4(o + PART_PLANE_BYTES, out(e[i] - sgn * b[i]), out(e[i + 1] - sgn * b[i + 1]),
+                        st_shared4(o + PART_PLANE_BYTES<TN>, out(e[i] - sgn * b[i]), out(e[i + 1] - sgn * b[i + 1]),
                                    out(e[i + 2] - sgn * b[i + 2]), out(e[i + 3] - sgn * b[i + 3]));
                     }
                 }
@@ -1053,15 +1059,15 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
         for (long u = run_begin(r), ue = run_end(r); u < ue; seg += DRAIN ? 0 : 1) {
             int tile = (int) (u / k_blocks), kb0 = (int) (u % k_blocks);
             int kb1 = (int) min((long) k_blocks, kb0 + (ue - u));
-            int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
+            int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * TN;
             const bool partial = !(kb0 == 0 && kb1 == k_blocks);   // split tiles are summed with atomics
             const bool add_res = p.r_re != nullptr && kb0 == 0;
             const bool need_old = !partial && p.accumulate;
             const bool pre = VEC && (add_res || need_old);
             // one row of the tile per epilogue thread, requested before the wait for the MMAs
             if (group == 0) {
-                if (add_res) prefetch_tile_rows(p, p.r_re, p.r_im, m0 + et, n0);
-                if (need_old) prefetch_tile_rows(p, p.d_re, p.d_im, m0 + et, n0);
+                if (add_res) prefetch_tile_rows<TN>(p, p.r_re, p.r_im, m0 + et, n0);
+                if (need_old) prefetch_tile_rows<TN>(p, p.d_re, p.d_im, m0 + et, n0);
             }
             // What a round adds from global memory (the residual if there is one, else old D) is requested a round
             // ahead, the first one's under the MMAs: asked for in the round itself it doubled the round's time, and
@@ -1082,7 +1088,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                     gi[j] = ld_global_now(xi + o);
                 }
             };
-            const int c_first = group * 64, c_last = c_first + 48;
+            const int c_first = group * HALF, c_last = c_first + HALF - 16;
             if (pre) request(c_first, 0);
             if constexpr (DRAIN) {
                 if (!sum_chains(kb0, kb1)) { live = false; break; }
@@ -1092,7 +1098,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
 #pragma unroll(DRAIN ? 4 : 1)
-            for (int round = 0; round < 4; ++round) {
+            for (int round = 0; round < HALF / 16; ++round) {
                 const int c0 = c_first + 16 * round;
                 if constexpr (DRAIN) {
 #pragma unroll
@@ -1105,8 +1111,8 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                 } else {
                     float a[16], f[16], b[16], e[16];
                     tmem_ld16(tl + c0, a);                   // A_re.B_re
-                    tmem_ld16(tl + 384 + c0, f);             // A_im.B_im
-                    tmem_ld16(tl + 128 + c0, b);             // A_re.B_im
+                    tmem_ld16(tl + 256 + TN + c0, f);             // A_im.B_im
+                    tmem_ld16(tl + TN + c0, b);             // A_re.B_im
                     tmem_ld16(tl + 256 + c0, e);             // A_im.B_re
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
@@ -1209,13 +1215,13 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
             CNB_GSTAMP(6, threadIdx.x == Threads<DRAIN>::FIRST_EPI);
             if (!plain && !*abort_flag) {
                 const int tile = blockIdx.x / cluster_ctas;
-                const int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * BN;
+                const int m0 = (tile / tiles_n) * TILE_M + row_off, n0 = (tile % tiles_n) * TN;
                 const int et = (warp - EPI_WARP) * 32 + lane;
                 const uint32_t peer0 = PAIR ? prank : 0u, peer_step = PAIR ? 2u : 1u;
                 switch (p.cluster) {
-                    case 2: cluster_reduce<2, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
-                    case 4: cluster_reduce<4, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
-                    default: cluster_reduce<8, VEC>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+                    case 2: cluster_reduce<2, VEC, TN>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+                    case 4: cluster_reduce<4, VEC, TN>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
+                    default: cluster_reduce<8, VEC, TN>(p, smem_base, crank, m0, n0, et, peer0, peer_step); break;
                 }
             }
             CNB_GSTAMP(7, threadIdx.x == Threads<DRAIN>::FIRST_EPI);
@@ -1521,15 +1527,16 @@ int make_map_mn(CUtensorMap* m, const float* base, int K, int pitch) {
 }
 
 // A pair of 16-bit planes (real, imaginary; np elements apart), each [rows, K] row-major, seen as [2][rows][K]: one
-// box {BK, 128, 2} brings the 128 rows of both planes, real then imaginary (planes_per_box = 1: of one plane);
+// box {BK, 128, 2} brings the 128 rows of both planes, real then imaginary (planes_per_box = 1: of one plane; box_rows: of
+// 64 rows for narrow tiles);
 // the swizzle is the box's row of 2 BK bytes.
-int make_map16(CUtensorMap* m, const void* base, int rows, int K, int pitch, size_t np, unsigned planes_per_box, int BK,
-               CUtensorMapDataType type) {
+int make_map16(CUtensorMap* m, const void* base, int rows, int K, int pitch, size_t np, unsigned planes_per_box, unsigned box_rows,
+               int BK, CUtensorMapDataType type) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[3] = {(cuuint64_t) K, (cuuint64_t) rows, 2u};
     cuuint64_t strides[2] = {(cuuint64_t) pitch * 2u, (cuuint64_t) np * 2u};
-    cuuint32_t box[3] = {(cuuint32_t) BK, 128u, planes_per_box};
+    cuuint32_t box[3] = {(cuuint32_t) BK, box_rows, planes_per_box};
     cuuint32_t estr[3] = {1u, 1u, 1u};
     CUresult r = fn(m, type, 3, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, BK == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1540,13 +1547,13 @@ int make_map16(CUtensorMap* m, const void* base, int rows, int K, int pitch, siz
 
 // The same pair stored [K, rows] (rows contiguous, pitch % 64 == 0), seen as [2][pitch/64][K][64]: one box
 // {64, BK, 2, 2} brings two 64-row slabs of 16 k-lines of both planes, slab after slab (128-byte swizzle).
-int make_map16_mn(CUtensorMap* m, const void* base, int K, int pitch, size_t np, unsigned planes_per_box, int BK,
-                  CUtensorMapDataType type) {
+int make_map16_mn(CUtensorMap* m, const void* base, int K, int pitch, size_t np, unsigned planes_per_box, unsigned box_rows,
+                  int BK, CUtensorMapDataType type) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return cnb::set_error(CNB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     cuuint64_t dims[4] = {64u, (cuuint64_t) K, (cuuint64_t) (pitch / 64), 2u};
     cuuint64_t strides[3] = {(cuuint64_t) pitch * 2u, 128u, (cuuint64_t) np * 2u};
-    cuuint32_t box[4] = {64u, (cuuint32_t) BK, 2u, planes_per_box};
+    cuuint32_t box[4] = {64u, (cuuint32_t) BK, box_rows / 64, planes_per_box};
     cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
     CUresult r = fn(m, type, 4, const_cast<void*>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1575,12 +1582,157 @@ __global__ void zero_pair_k(float* __restrict__ a, float* __restrict__ b, size_t
 
 // The schedule of one product: which form (one CTA per tile or CTA pairs), how many CTAs, how the (tile, k-block)
 // units are dealt.  Host arithmetic only (also reachable as cnb_gemm_schedule, for tests that need no GPU).
-struct Schedule { bool pair; long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles, joined; };
+struct Schedule { bool pair; long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles, joined; int tile_n, first, rest; };
+
+// Sizes whose products have always been split ones here, at 19 bits an operand: packed ones are nearer to float64 there
+// whatever the length of the chain (512 x 1024 x 1024: 1.9e-6 -> 0.9e-6, 4096 x 1024 x 1024: 4.5e-6 -> 3.1e-6).
+bool split_sizes(int M, int N, int K) { return K % 8 == 0 && K >= 32 && M >= 64 && N >= 64; }
 
 // The longest chain of a product with K > 4096, in k-blocks of 16 (see choose_schedule).
 constexpr int kMaxChain16 = 64;
 
-// Depths below are counted in blocks of 16 and scaled to the form's own (bk = 16 or 32).
+// Every other size could run as fp32 FMAs (cgemm_simt.cu), and the tiles must not be less exact than those.  The tensor
+// core truncates as it accumulates: measured on balanced data one chain of C products is off by 4.2e-9 C of the result,
+// rounded FMAs over K products by 1.8e-8 sqrt(K), and a sum of chains rounded to nearest by what one chain is.  So a chain
+// may be 4.28 sqrt(K) long, in blocks of 32.
+int max_chain(int K) { return std::max(1, (int) (4.28 * std::sqrt((double) K) / FormCfg<PACKED>::BK)); }
+
+// The longest run of k-blocks that one CTA sums for a tile.
+int longest_run(const Schedule& q, int k_blocks) {
+    return q.cluster > 1 ? (k_blocks + q.cluster - 1) / q.cluster : q.whole_per_cta > 0 ? k_blocks : (int) std::min<long>(q.upc, k_blocks);
+}
+
+// The chains of a packed product in k-blocks of 32: a tile's first ones, and those of all others.
+//
+// At sizes that were split products, whole tiles of K <= 4096 are one chain, and a longer K is cut at choose_schedule's cap.  Whole
+// tiles that used to be shared runs (`joined`) take two chains at least, of 24 at most: what was shared had shorter chains than a
+// whole tile (4096 x 1024, K = 512: 1.57e-6 off float64, 1.83e-6 as one chain, 0.93e-6 as two; K = 1024 3.11e-6, and 1.83e-6 as
+// two).  A second chain takes up to 2.5 us (K = 256: 34.8 us as shared runs, 23.7 as one chain, 26.2 as two; K = 512 47.1,
+// 37.8, 38.0).
+//
+// At others max_chain is the line.  A run of K > 4096 that is longer than the cap is cut as evenly as runs of that length were:
+// 1500 x 1500, K = 4100 in chains of 8, 8, 8 and 2 a run 8.7e-7 off, in chains of 8 throughout 9.3e-7, of 7 7.8e-7.
+// `joined` there: what whole chains leave of K, or one of them, goes to both ends (4089 x 1019, K = 500, 16 blocks: 2.29e-7 off
+// as shared runs, 2.30e-7 as 8 x 2, 2.21e-7 as 1 + 7 x 2 + 1; 3321 x 1275, K = 250, 8 blocks: 2.22e-7, 2.27e-7, 2.06e-7).
+//
+// Runs by CTA pairs that make five chains or more of at least three blocks take the accumulators out one after the other, and a
+// block less a chain for it: the MMAs wait less, and the second rounding weighs less than the block (4089 x 1019, K = 1001 4.47e-7
+// off as shared runs, 91 us as EXACT, 81 and 3.72e-7 so; 777 x 1001, K = 1333 47.6 -> 45.0 us, 4.44e-7 -> 3.75e-7; a mean of
+// 0.95 over 28 sizes).  In fewer chains, or by single CTAs, that is no gain (1.00 to 1.04 over 85).
+struct Chains { int first, rest; bool exact; };
+Chains chain_blocks(int M, int N, int K, const Schedule& q) {
+    const int n = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK, cap = kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK;
+    auto evenly = [](int blocks, int most) { const int chains = (blocks + most - 1) / most; return (blocks + chains - 1) / chains; };
+    if (q.rest > 0) return {q.first, q.rest, true};      // (narrow_tiles)
+    if (split_sizes(M, N, K)) {
+        const int c = evenly(n, K > 4096 ? cap : q.joined ? std::max(2, std::min(24, (n + 1) / 2)) : n);
+        return {c, c, false};
+    }
+    const int run = longest_run(q, n), c = K > 4096 && run > cap ? evenly(evenly(n, cap), max_chain(K)) : max_chain(K);
+    if (q.pair && max_chain(K) >= 3 && run > 4 * c) return {c - 1, c - 1, false};
+    return {q.joined && n > c ? (n % c + c + 1) / 2 : c, c, true};
+}
+
+// Narrow tiles (128 x 64) for products of few tiles, one CTA to a tile's slice of K.  Past the MMAs such a launch takes as long as
+// half a tile of 128 x 128 needs three times: out of tensor memory (1.1 us), between the CTAs of a cluster (2.5 to 3.5 us, 38 bytes
+// a ns into an SM, and a barrier), into memory (1.2); and it leaves most SMs without a tile.
+//
+// Where twice the tiles still are one wave in the clusters of the wide ones, every element's sum is what it was, in order too
+// (product and packs, us: 300 x 300, K = 300 18.1 -> 14.6, 64 x 784, K = 784 18.4 -> 16.1, 128 x 128, K = 4096 29.6 -> 23.3).
+//
+// Where they are not, smaller clusters may be faster; clusters that are not all resident at once (15 of eight CTAs and 33 of four
+// are, on 148 SMs) never are, and neither are short runs summed with atomics.  The estimate below, fitted to 20 sizes at every
+// width and cluster that has room and to 40 that ran as such sums, has to promise a microsecond (300 x 500, K = 500 19.2 -> 17.3,
+// 256 x 512, K = 512 17.1 -> 15.2, 128 x 2048, K = 512 30.4 -> 18.7, 350 x 401, K = 1081 35.6 -> 22.7; 512 x 1024, K = 1024 stays
+// as it is).  Over 660 products of 24 to 2500 rows and columns 1.07 times as fast as without narrow tiles, none slower by more
+// than runs of one program differ, and none further off float64: chains are as short as that takes.
+//
+// Products with an N of up to 128, and gradients with an M of up to 128, are those of a head.  The gradient of a loss divides by
+// what they give, which magnifies a sum in another order, so they keep theirs where it is fixed.
+void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate, int sms) {
+    auto fit = [&](int c) { return c == 8 ? sms * 15 / 148 : c == 4 ? sms * 33 / 148 : sms / c; };
+    const long rows = (M + BM - 1) / BM, wide = rows * ((N + BN - 1) / BN), narrow = rows * ((N + NARROW - 1) / NARROW);
+    auto take = [&](int tile_n, int c) {
+        r.pair = false;
+        r.tile_n = tile_n;
+        r.cluster = c;
+        r.ctas = (tile_n == NARROW ? narrow : wide) * c;
+        r.upc = c > 1 ? 0 : k_blocks;
+        r.splits_tiles = false;
+    };
+    if (r.whole_per_cta > 0 || r.segments > 0 || (r.pair && !r.splits_tiles)) return;
+    const int c0 = r.cluster;
+    if (c0 == 1 && !r.splits_tiles) {                    // a CTA to a tile
+        if (r.ctas == wide && narrow <= sms) take(NARROW, 1);
+        return;
+    }
+    if (c0 > 1 && (k_blocks + c0 - 1) / c0 > kMaxChain16 / 2) return;        // (chains that are taken out one after the other)
+    if (c0 > 1 && narrow <= fit(c0)) return take(NARROW, c0);
+    if ((c0 > 1 && (N <= BN || (accumulate && M <= BM))) || K > 4096) return;
+
+    // The chains of the runs from k-block `from` to `to`: how many, and the sum of the cubes of their lengths, which is what the square of
+    // the error goes with: what is truncated in a chain of C, C at the magnitude of sqrt(C).
+    struct Sum { long chains, cubes; };
+    auto chains_of = [&](int from, int to, int first, int rest) {
+        Sum v = {0, 0};
+        for (int kb = from; kb < to;) {
+            const long c = std::min(kb == 0 ? first : rest, to - kb);
+            ++v.chains; v.cubes += c * c * c;
+            kb += (int) c;
+        }
+        return v;
+    };
+    auto cluster_of = [&](int c, int first, int rest) {                      // most chains of a CTA, and all cubes of a tile
+        Sum v = {0, 0};
+        for (int k = 0; k < c; ++k) {
+            const Sum w = chains_of(k_blocks * k / c, k_blocks * (k + 1) / c, first, rest);
+            v = {std::max(v.chains, w.chains), v.cubes + w.cubes};
+        }
+        return v;
+    };
+    const Chains now = chain_blocks(M, N, K, r);
+    long cubes = 0, tiles = 1;                           // of `tiles` tiles
+    if (c0 > 1) {
+        cubes = cluster_of(c0, now.first, now.rest).cubes;
+    } else {
+        tiles = r.pair ? (long) ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) : wide;
+        for (long u = 0; u < tiles * k_blocks;) {
+            const long end = std::min({(u / r.upc + 1) * r.upc, (u / k_blocks + 1) * k_blocks});
+            const int kb = (int) (u % k_blocks);
+            cubes += chains_of(kb, kb + (int) (end - u), now.first, now.rest).cubes;
+            u = end;
+        }
+    }
+    if (now.rest < (c0 > 1 ? (k_blocks + c0 - 1) / c0 : r.upc)) cubes -= cubes / 20;       // (1010 x 1595, K = 323: as many, 1.03 as far off)
+    // Costs in hundredths of a microsecond: blocks, what a cluster adds, taking a chain out of tensor memory before the next.
+    struct { int tile_n, c, first, rest; long cost; } best = {0, 0, 0, 0, 0};
+    auto consider = [&](int tile_n, int c, bool as_it_is) {
+        if ((tile_n == NARROW ? narrow : wide) > fit(c)) return;
+        static const int wide_add[4] = {140, 430, 590, 690}, narrow_add[4] = {0, 235, 345, 470};
+        const bool thin = tile_n == NARROW, crowd = (thin ? narrow : wide) * c > 100 * sms / 148;
+        const int log_c = c == 8 ? 3 : c == 4 ? 2 : c - 1, run = (k_blocks + c - 1) / c;
+        const long fixed = (thin ? (crowd ? 85 : 70) * run + narrow_add[log_c] : 90 * run + wide_add[log_c]) + (crowd && c == 8 ? 200 : 0);
+        // the longest chains that are no less exact than those of the form before; a shorter first one where that does
+        for (int rest = std::min(run, now.rest); rest >= 1; --rest)
+            for (int first = rest; first >= std::max(1, rest - 1); --first) {
+                const Sum v = cluster_of(c, first, rest);
+                if (!as_it_is && v.cubes * tiles > cubes) continue;
+                const long cost = fixed + (thin ? 50 : 100) * (v.chains - 1);
+                if (best.c == 0 || cost < best.cost) best = {tile_n, c, first, rest, cost};
+                return;
+            }
+    };
+    if (c0 > 1) consider(BN, c0, true);
+    const long before = c0 == 1 ? (N % 4 == 0 ? 800 : 1500) + (split_sizes(M, N, K) ? 0 : 300) - (accumulate ? 300 : 0) + 80 * r.upc
+                                : best.c ? best.cost : 1 << 30;
+    best.c = 0;
+    for (int c = c0 == 1 ? 8 : c0 / 2; c >= 1; c /= 2) { consider(BN, c, false); consider(NARROW, c, false); }
+    if (best.c == 0 || best.cost > before - 100) return;
+    r.first = best.first;
+    r.rest = best.rest;
+    take(best.tile_n, best.c);
+}
+
 Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int bk) {
     // Schedule, by tile count ("CTA" = one CTA, or the CTA pair of a 256-row tile; sms = how many of them this launch
     // may fill: leaving a few SMs free (gemm_cta_limit) lets a concurrent collective's kernels run beside the GEMM):
@@ -1714,57 +1866,15 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
     Schedule r;
     r.pair = pair; r.ctas = q.ctas; r.upc = q.upc; r.whole_per_cta = q.whole_per_cta; r.clear_from_row = q.clear_from_row;
     r.cluster = q.cluster; r.segments = q.segments; r.splits_tiles = q.splits_tiles; r.joined = q.joined;
+    r.tile_n = BN;
+    r.first = r.rest = 0;
+    if (packed) narrow_tiles(r, M, N, K, k_blocks, accumulate, sm_limit > 0 ? std::min(sm_limit, sm_count) : sm_count);
     return r;
 }
 
 }  // namespace
 
 namespace cnb {
-
-// Sizes whose products have always been split ones here, at 19 bits an operand: packed ones are nearer to float64 there
-// whatever the length of the chain (512 x 1024 x 1024: 1.9e-6 -> 0.9e-6, 4096 x 1024 x 1024: 4.5e-6 -> 3.1e-6).
-static bool split_sizes(int M, int N, int K) { return K % 8 == 0 && K >= 32 && M >= 64 && N >= 64; }
-
-// Every other size could run as fp32 FMAs (cgemm_simt.cu), and the tiles must not be less exact than those.  The tensor
-// core truncates as it accumulates: measured on balanced data one chain of C products is off by 4.2e-9 C of the result,
-// rounded FMAs over K products by 1.8e-8 sqrt(K), and a sum of chains rounded to nearest by what one chain is.  So a chain
-// may be 4.28 sqrt(K) long, in blocks of 32.
-static int max_chain(int K) { return std::max(1, (int) (4.28 * std::sqrt((double) K) / FormCfg<PACKED>::BK)); }
-
-// The longest run of k-blocks that one CTA sums for a tile.
-static int longest_run(const Schedule& q, int k_blocks) {
-    return q.cluster > 1 ? (k_blocks + q.cluster - 1) / q.cluster : q.whole_per_cta > 0 ? k_blocks : (int) std::min<long>(q.upc, k_blocks);
-}
-
-// The chains of a packed product in k-blocks of 32: a tile's first ones, and those of all others.
-//
-// At sizes that were split products, whole tiles of K <= 4096 are one chain, and a longer K is cut at choose_schedule's cap.  Whole
-// tiles that used to be shared runs (`joined`) take two chains at least, of 24 at most: what was shared had shorter chains than a
-// whole tile (4096 x 1024, K = 512: 1.57e-6 off float64, 1.83e-6 as one chain, 0.93e-6 as two; K = 1024 3.11e-6, and 1.83e-6 as
-// two).  A second chain takes up to 2.5 us (K = 256: 34.8 us as shared runs, 23.7 as one chain, 26.2 as two; K = 512 47.1,
-// 37.8, 38.0).
-//
-// At others max_chain is the line.  A run of K > 4096 that is longer than the cap is cut as evenly as runs of that length were:
-// 1500 x 1500, K = 4100 in chains of 8, 8, 8 and 2 a run 8.7e-7 off, in chains of 8 throughout 9.3e-7, of 7 7.8e-7.
-// `joined` there: what whole chains leave of K, or one of them, goes to both ends (4089 x 1019, K = 500, 16 blocks: 2.29e-7 off
-// as shared runs, 2.30e-7 as 8 x 2, 2.21e-7 as 1 + 7 x 2 + 1; 3321 x 1275, K = 250, 8 blocks: 2.22e-7, 2.27e-7, 2.06e-7).
-//
-// Runs by CTA pairs that make five chains or more of at least three blocks take the accumulators out one after the other, and a
-// block less a chain for it: the MMAs wait less, and the second rounding weighs less than the block (4089 x 1019, K = 1001 4.47e-7
-// off as shared runs, 91 us as EXACT, 81 and 3.72e-7 so; 777 x 1001, K = 1333 47.6 -> 45.0 us, 4.44e-7 -> 3.75e-7; a mean of
-// 0.95 over 28 sizes).  In fewer chains, or by single CTAs, that is no gain (1.00 to 1.04 over 85).
-struct Chains { int first, rest; bool exact; };
-static Chains chain_blocks(int M, int N, int K, const Schedule& q) {
-    const int n = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK, cap = kMaxChain16 * FormCfg<SPLIT>::BK / FormCfg<PACKED>::BK;
-    auto evenly = [](int blocks, int most) { const int chains = (blocks + most - 1) / most; return (blocks + chains - 1) / chains; };
-    if (split_sizes(M, N, K)) {
-        const int c = evenly(n, K > 4096 ? cap : q.joined ? std::max(2, std::min(24, (n + 1) / 2)) : n);
-        return {c, c, false};
-    }
-    const int run = longest_run(q, n), c = K > 4096 && run > cap ? evenly(evenly(n, cap), max_chain(K)) : max_chain(K);
-    if (q.pair && max_chain(K) >= 3 && run > 4 * c) return {c - 1, c - 1, false};
-    return {q.joined && n > c ? (n % c + c + 1) / 2 : c, c, true};
-}
 
 bool cgemm_tc_fits(int M, int N, int K) {
     if (split_sizes(M, N, K)) return true;
@@ -1813,22 +1923,27 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     if (!attr_set[ctx->device & 63]) {
 #define CNB_TC_ATTR(F, D)                                                                                                   \
     do {                                                                                                                    \
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, false, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES)); \
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, true, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));  \
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, false, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));  \
-        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, true, F, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));   \
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, false, F, D, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES)); \
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, true, F, D, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));  \
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, false, F, D, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));  \
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<true, true, F, D, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));   \
     } while (0)
         CNB_TC_ATTR(SPLIT, NONE); CNB_TC_ATTR(PACKED, NONE); CNB_TC_ATTR(PACKED, OVERLAP); CNB_TC_ATTR(PACKED, EXACT);
 #undef CNB_TC_ATTR
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, false, PACKED, NONE, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, true, PACKED, NONE, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, false, PACKED, EXACT, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        CNB_CUDA(cudaFuncSetAttribute(cgemm_tc_k<false, true, PACKED, EXACT, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         // the shares of a launch with running sums must add up to what it starts with
-#define CNB_TC_REGS(P, V, D)                                                                                                \
+#define CNB_TC_REGS(P, V, D, T)                                                                                              \
     do {                                                                                                                    \
         cudaFuncAttributes f;                                                                                               \
-        CNB_CUDA(cudaFuncGetAttributes(&f, cgemm_tc_k<P, V, PACKED, D>));                                                   \
+        CNB_CUDA(cudaFuncGetAttributes(&f, cgemm_tc_k<P, V, PACKED, D, T>));                                                   \
         if (f.numRegs < LAUNCH_REGS) return set_error(CNB_ERR_CUDA, "cgemm_tc: built with %d registers a thread, not %d", f.numRegs, LAUNCH_REGS); \
     } while (0)
-        CNB_TC_REGS(false, false, OVERLAP); CNB_TC_REGS(false, true, OVERLAP); CNB_TC_REGS(true, false, OVERLAP); CNB_TC_REGS(true, true, OVERLAP);
-        CNB_TC_REGS(false, false, EXACT); CNB_TC_REGS(false, true, EXACT); CNB_TC_REGS(true, false, EXACT); CNB_TC_REGS(true, true, EXACT);
+        CNB_TC_REGS(false, false, OVERLAP, BN); CNB_TC_REGS(false, true, OVERLAP, BN); CNB_TC_REGS(true, false, OVERLAP, BN); CNB_TC_REGS(true, true, OVERLAP, BN);
+        CNB_TC_REGS(false, false, EXACT, BN); CNB_TC_REGS(false, true, EXACT, BN); CNB_TC_REGS(true, false, EXACT, BN); CNB_TC_REGS(true, true, EXACT, BN);
+        CNB_TC_REGS(false, false, EXACT, NARROW); CNB_TC_REGS(false, true, EXACT, NARROW);
 #undef CNB_TC_REGS
         attr_set[ctx->device & 63] = true;
     }
@@ -1850,13 +1965,13 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     for (int side = 0; side < 2; ++side) {
         const SplitOperand& o = side ? b : a;
         const int rows = side ? N : M;
-        const unsigned planes = side ? b_planes : 2u;
+        const unsigned planes = side ? b_planes : 2u, box_rows = side ? (unsigned) q.tile_n : 128u;
         if (packed) {
             for (int k = 0; k < 2; ++k) {                // high parts, low parts
                 CUtensorMap* m = &maps_p.m[2 * side + k];
                 const __half* base = reinterpret_cast<const __half*>(o.base) + 2 * k * o.plane_pitch;
-                rc = o.mn ? make_map16_mn(m, base, K, o.pitch, o.plane_pitch, planes, bk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16)
-                          : make_map16(m, base, rows, K, o.pitch, o.plane_pitch, planes, bk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
+                rc = o.mn ? make_map16_mn(m, base, K, o.pitch, o.plane_pitch, planes, box_rows, bk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16)
+                          : make_map16(m, base, rows, K, o.pitch, o.plane_pitch, planes, box_rows, bk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
                 if (rc != CNB_OK) return rc;
             }
             continue;
@@ -1865,8 +1980,8 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
             CUtensorMap* m = &maps_s.m[4 * side + k];
             const float* base = o.base + k * o.plane_pitch;
             if (k < 2) rc = o.mn ? make_map_mn(m, base, K, o.pitch) : make_map(m, base, rows, K, o.pitch);
-            else rc = o.mn ? make_map16_mn(m, base, K, o.pitch, o.plane_pitch, planes, bk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)
-                           : make_map16(m, base, rows, K, o.pitch, o.plane_pitch, planes, bk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
+            else rc = o.mn ? make_map16_mn(m, base, K, o.pitch, o.plane_pitch, planes, 128u, bk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)
+                           : make_map16(m, base, rows, K, o.pitch, o.plane_pitch, planes, 128u, bk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
             if (rc != CNB_OK) return rc;
         }
     }
@@ -1908,13 +2023,16 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     };
     cudaError_t e;
 #define CNB_TC_GO(F, D, maps)                                                                                              \
-    (pair ? (vec ? go(cgemm_tc_k<true, true, F, D>, maps) : go(cgemm_tc_k<true, false, F, D>, maps))                       \
-          : (vec ? go(cgemm_tc_k<false, true, F, D>, maps) : go(cgemm_tc_k<false, false, F, D>, maps)))
-    if (!packed) e = CNB_TC_GO(SPLIT, NONE, maps_s);
+    (pair ? (vec ? go(cgemm_tc_k<true, true, F, D, BN>, maps) : go(cgemm_tc_k<true, false, F, D, BN>, maps))               \
+          : (vec ? go(cgemm_tc_k<false, true, F, D, BN>, maps) : go(cgemm_tc_k<false, false, F, D, BN>, maps)))
+#define CNB_TC_GO_NARROW(D) (vec ? go(cgemm_tc_k<false, true, PACKED, D, NARROW>, maps_p) : go(cgemm_tc_k<false, false, PACKED, D, NARROW>, maps_p))
+    if (q.tile_n == NARROW) e = drain == EXACT ? CNB_TC_GO_NARROW(EXACT) : CNB_TC_GO_NARROW(NONE);
+    else if (!packed) e = CNB_TC_GO(SPLIT, NONE, maps_s);
     else if (drain == EXACT) e = CNB_TC_GO(PACKED, EXACT, maps_p);
     else if (drain == OVERLAP) e = CNB_TC_GO(PACKED, OVERLAP, maps_p);
     else e = CNB_TC_GO(PACKED, NONE, maps_p);
 #undef CNB_TC_GO
+#undef CNB_TC_GO_NARROW
     CNB_CUDA(e);
     CNB_LAUNCH_CHECK("cgemm_tc");
     return CNB_OK;
@@ -2027,5 +2145,5 @@ extern "C" int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm
     if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0)
         return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_chain_packed: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
     const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK);
-    return cnb::chain_blocks(M, N, K, q).rest;
+    return chain_blocks(M, N, K, q).rest;
 }

@@ -1,0 +1,32 @@
+"""The schedule of products of few tiles (cnb_gemm_schedule_packed: host arithmetic, no GPU)."""
+import random
+
+import pytest
+
+from cnet_b200 import lib as L
+from test_gemm_schedule import SMS
+from test_gemm_schedule_packed import _schedule
+
+
+@pytest.mark.parametrize("limit", [0, 74])
+def test_narrow_tiles_fit_the_device(limit):
+    """Products of few tiles: as many CTAs as one of the two tile widths asks for, in no more clusters than are resident at once
+    (15 of eight CTAs and 33 of four on 148 SMs) where the order of the sums is free; a chain is no longer than in a run of wide tiles."""
+    rng = random.Random(3)
+    narrow = 0
+    for _ in range(400):
+        M, N, K = rng.randint(1, 700), rng.randint(1, 700), rng.randint(96, 4000)
+        s = _schedule(M, N, K, 0, limit)
+        if s["pair"] or s["atomics"] or s["segments"] or s["whole_per_cta"]:
+            continue
+        c, rows = s["cluster_ctas"], -(-M // 128)
+        assert s["ctas"] in (rows * -(-N // 64) * c, rows * -(-N // 128) * c), (M, N, K, s)
+        narrow += s["ctas"] == rows * -(-N // 64) * c and N > 64
+        sms = limit or SMS
+        fit = {1: sms, 2: sms // 2, 4: sms * 33 // 148, 8: sms * 15 // 148}[c]
+        if s["ctas"] // c > fit:
+            assert N <= 128 and s["ctas"] == rows * c, (M, N, K, s)
+        chain = L.load().cnb_gemm_chain_packed(M, N, K, 0, SMS, limit)
+        if K % 8 or M < 64 or N < 64:
+            assert chain <= max(1, int(4.28 * K ** 0.5 / 32)), (M, N, K, chain)
+    assert narrow > 100
