@@ -43,6 +43,7 @@ struct MixedPlan {
     int buffers, shift;               // shift: spread of the buffers' rows, 4 or NO_SPREAD
     Pass p[MAX_PASSES];
     float scale;
+    unsigned mag_n;                   // reciprocal of n
 };
 
 // Where element i of a row lies in a buffer: every 16th set one further (shift 4), or as it is.  Constants of the kernel: a
@@ -63,8 +64,23 @@ struct Io {
     size_t row0;
 };
 
-// What becomes of a finished row: stored, stored and taken through the tail, or added to what is there.
-enum Finish { STORE = 0, TAIL = 1, ADD = 2 };
+// What becomes of a finished row: stored, stored and taken through the tail (by the threads that hold its last butterflies, or from
+// shared memory by all in turn), or added to what is there.
+enum Finish { STORE = 0, TAIL = 1, ADD = 2, TAIL_LOOP = 3 };
+
+// The tail of an element whose transform is u: u, u o h where it is kept, CGelu of that.
+__device__ __forceinline__ void tail_store(const Io& io, const FftEpilogue& ep, size_t g, size_t at, float2 u, float hr, float hi) {
+    io.yr[g] = u.x;
+    io.yi[g] = u.y;
+    const float ar = u.x * hr - u.y * hi, ai = u.x * hi + u.y * hr;
+    const float gr = cnb_gelu(ar), gi = cnb_gelu(ai);
+    if (ep.ar) { ep.ar[at] = ar; ep.ai[at] = ai; }
+    if (ep.gr) { ep.gr[at] = gr; ep.gi[at] = gi; }
+    if (ep.sp) {
+        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 0), at, gr);
+        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 1), at, gi);
+    }
+}
 
 template <int R, int FINISH, bool CHIRP, int SHIFT>
 __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io& io, const FftEpilogue& ep) {
@@ -132,23 +148,39 @@ __device__ __forceinline__ void run_pass(const MixedPlan& pl, const Pass& d, Io&
                 if (CHIRP) u = cmul(make_float2(u.y, u.x), __ldg(io.chirp + e));
                 u.x *= pl.scale; u.y *= pl.scale;
                 if (FINISH == ADD) { u.x += old[FINISH == ADD ? q : 0].x; u.y += old[FINISH == ADD ? q : 0].y; }
-                io.yr[g] = u.x;
-                io.yi[g] = u.y;
                 if (FINISH == TAIL) {
                     // the kernels before may have written h: the read-only path only behind a barrier of this one
                     const bool lone = pl.passes == 1;
                     const float hr = lone ? cnb_ld_behind_wait(ep.hr + e) : __ldg(ep.hr + e), hi = lone ? cnb_ld_behind_wait(ep.hi + e) : __ldg(ep.hi + e);
-                    const float ar = u.x * hr - u.y * hi, ai = u.x * hi + u.y * hr;
-                    const float gr = cnb_gelu(ar), gi = cnb_gelu(ai);
-                    const size_t at = (io.row0 + row) * (size_t) pl.n + e;
-                    if (ep.ar) { ep.ar[at] = ar; ep.ai[at] = ai; }
-                    if (ep.gr) { ep.gr[at] = gr; ep.gi[at] = gi; }
-                    if (ep.sp) {
-                        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 0), at, gr);
-                        cnb_split_store1(cnb_split_component(ep.sp, ep.np, 1), at, gi);
-                    }
+                    tail_store(io, ep, g, (io.row0 + row) * (size_t) pl.n + e, u, hr, hi);
+                } else {
+                    io.yr[g] = u.x;
+                    io.yi[g] = u.y;
                 }
             }
+        }
+    }
+}
+
+// TAIL_LOOP: the rows lie finished, but for their scale (and chirp), at `s`.
+template <bool CHIRP, int SHIFT>
+__device__ __forceinline__ void tail_loop(const MixedPlan& pl, const Io& io, const FftEpilogue& ep, const float2* s) {
+    const int total = io.rows * pl.n, step = blockDim.x;
+    for (int i0 = threadIdx.x; i0 < total; i0 += 2 * step) {
+        float2 u[2], h[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int i = i0 + k * step, row = div_by(i, pl.mag_n), e = i - row * pl.n;
+            if (i >= total) break;
+            h[k] = make_float2(__ldg(ep.hr + e), __ldg(ep.hi + e));
+            u[k] = s[row * pl.stride + pad_of<SHIFT>(e)];
+            if (CHIRP) u[k] = cmul(make_float2(u[k].y, u[k].x), __ldg(io.chirp + e));
+            u[k].x *= pl.scale; u[k].y *= pl.scale;
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int i = i0 + k * step;
+            if (i < total) tail_store(io, ep, i, io.row0 * (size_t) pl.n + i, u[k], h[k].x, h[k].y);
         }
     }
 }
@@ -170,7 +202,7 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
     for (int s = 0; s < total; ++s) {
         const Pass& d = pl.p[CHIRP && s >= pl.passes ? s - pl.passes : s];
         io.src = s == 0 ? nullptr : bufs + (s & 1 ? 0 : pl.rows * pl.stride);
-        io.dst = s == total - 1 ? nullptr : bufs + (s & 1 ? pl.rows * pl.stride : 0);
+        io.dst = s == total - 1 && FINISH != TAIL_LOOP ? nullptr : bufs + (s & 1 ? pl.rows * pl.stride : 0);
         io.spectral = CHIRP && s == pl.passes;
         switch (d.radix) {
 #define CNB_RADIX(R) case R: run_pass<R, FINISH, CHIRP, SHIFT>(pl, d, io, ep); break
@@ -178,8 +210,9 @@ fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* y
             CNB_RADIX(10); CNB_RADIX(11); CNB_RADIX(12); CNB_RADIX(13); CNB_RADIX(14); CNB_RADIX(15); CNB_RADIX(16);
 #undef CNB_RADIX
         }
-        if (s < total - 1) __syncthreads();
+        if (s < total - 1 || FINISH == TAIL_LOOP) __syncthreads();
     }
+    if (FINISH == TAIL_LOOP) tail_loop<CHIRP, SHIFT>(pl, io, ep, bufs + ((total - 1) & 1 ? pl.rows * pl.stride : 0));
 }
 
 // twiddles of every pass, packed as Pass::tw says, in double
@@ -337,6 +370,7 @@ bool plan_length(int N, MixedPlan* out) {
     }
     pl.shift = m > N ? SPREAD : choose_spread(pl);
     pl.scale = (float) (1.0 / std::sqrt((double) N));
+    pl.mag_n = reciprocal(N);
     *out = pl;
     return true;
 }
@@ -376,6 +410,23 @@ void plan_batch(MixedPlan* pl, int B, int sms) {
         if (c < best * 0.999) { best = c; pl->threads = t; }
     }
     pl->rows = rows;
+}
+
+// The tail in a loop through shared memory, by all threads: written out behind a butterfly of 16 points it is 30 KB of
+// instructions, which a small batch runs through once, at the pace of their first fetch, on the few threads that have a last
+// butterfly (16 x 256 5.7 -> 3.0 us, 296 x 100 4.3 -> 2.9, 296 x 500 5.6 -> 4.2, 512 x 784 8.2 -> 6.4; in a training step, where other kernels'
+// instructions lie between, more).  Not where the trip through shared memory counts, whose row one CTA then has on its way twice: from
+// half a million elements (1024 x 512 6.2 and 6.3, 1024 x 900 11.2 and 16.3; half of that in the chirp form, 1024 x 137 7.6 and 7.4, 4096 x 137 16.8
+// and 19.5) and beyond 1024 points (86 x 2000 7.3 and 7.5).  Two elements a thread, in one round: as many threads as that takes (16 x 256
+// 3.0 us, with four 3.5).
+bool loop_tail(MixedPlan* pl, int B) {
+    const bool chirp = pl->m > pl->n;
+    if (pl->n > 1024 || (long) B * pl->n >= (chirp ? 1 << 18 : 1 << 19)) return false;
+    const int buffers = (chirp ? 2 : 1) * pl->passes > 1 ? 2 : 1;
+    if (smem_bytes(pl->m, pl->rows, buffers) > MAX_SMEM) return false;
+    pl->buffers = buffers;
+    pl->threads = std::max(pl->threads, std::min(MAX_THREADS, (pl->rows * pl->n / 2 + 31) / 32 * 32));
+    return true;
 }
 
 size_t twiddle_entries(const MixedPlan& pl) {
@@ -428,8 +479,9 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
     const float2* ch = tw + tw_entries;
     const float2* spec = ch + pl.n;
     if (inverse) { std::swap(xr, xi); std::swap(yr, yi); }
+    Finish finish = ep.hr ? TAIL : accumulate ? ADD : STORE;
+    if (finish == TAIL && loop_tail(&pl, B)) finish = TAIL_LOOP;
     const size_t smem = smem_bytes(pl.m, pl.rows, pl.buffers);
-    const Finish finish = ep.hr ? TAIL : accumulate ? ADD : STORE;
     static bool attr_done[64] = {};                         // the attribute is per device
     if (!attr_done[ctx->device & 63]) {
 #define CNB_MIXED_ATTR(F)                                                                                                          \
@@ -438,7 +490,7 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
         CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, false, NO_SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM)); \
         CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, true, SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));  \
     } while (0)
-        CNB_MIXED_ATTR(STORE); CNB_MIXED_ATTR(TAIL); CNB_MIXED_ATTR(ADD);
+        CNB_MIXED_ATTR(STORE); CNB_MIXED_ATTR(TAIL); CNB_MIXED_ATTR(ADD); CNB_MIXED_ATTR(TAIL_LOOP);
 #undef CNB_MIXED_ATTR
         attr_done[ctx->device & 63] = true;
     }
@@ -447,6 +499,7 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
 #define CNB_MIXED(F) \
     CNB_CUDA(chirp ? go(fft_mixed_k<F, true, SPREAD>) : pl.shift == SPREAD ? go(fft_mixed_k<F, false, SPREAD>) : go(fft_mixed_k<F, false, NO_SPREAD>))
     if (finish == TAIL) CNB_MIXED(TAIL);
+    else if (finish == TAIL_LOOP) CNB_MIXED(TAIL_LOOP);
     else if (finish == ADD) CNB_MIXED(ADD);
     else CNB_MIXED(STORE);
 #undef CNB_MIXED
