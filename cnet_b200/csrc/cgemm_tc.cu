@@ -1660,10 +1660,12 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         r.upc = c > 1 ? 0 : k_blocks;
         r.splits_tiles = false;
     };
-    if (r.whole_per_cta > 0 || r.segments > 0 || (r.pair && !r.splits_tiles)) return;
     const int c0 = r.cluster;
-    if (c0 == 1 && !r.splits_tiles) {                    // a CTA to a tile
-        if (r.ctas == wide && narrow <= sms) take(NARROW, 1);
+    if (r.whole_per_cta > 0 || r.segments > 0 || (r.pair && c0 > 1)) return;
+    if (c0 == 1 && !r.splits_tiles) {                    // a CTA or a pair to a tile
+        const Chains now = chain_blocks(M, N, K, r);
+        const bool whole = r.pair ? now.rest >= k_blocks || now.exact : r.ctas == wide;
+        if (whole && narrow <= sms) take(NARROW, 1);
         return;
     }
     if (c0 > 1 && (k_blocks + c0 - 1) / c0 > kMaxChain16 / 2) return;        // (chains that are taken out one after the other)
