@@ -272,30 +272,49 @@ void Linear::forward() {
 			out_size_, stream()));
 }
 
+// Whether dX* and dW* of this batch, each as it would run alone, are not much more than the device holds at once: clusters of
+// eight and four CTAs leave some SMs of 148 without.
+bool Linear::fitTogether() {
+	if (fit_batch_ != batch()) {
+		const int sms = net_->sm_count_;
+		int x[8], w[8];
+		auto share = [&](const int* v) { return (double) v[1] / (v[2] == 8 ? sms * 120 / 148 : v[2] == 4 ? sms * 132 / 148 : sms); };
+		fit_batch_ = batch();
+		fit_ = cnb_gemm_schedule_packed(batch(), in1_len, out_size_, 0, sms, 0, x) == CNB_OK &&
+				cnb_gemm_schedule_packed(out_size_, in1_len, batch(), 1, sms, 0, w) == CNB_OK && share(x) + share(w) <= 1.5;
+	}
+	return fit_;
+}
+
 void Linear::backward() {
 	CFunc* px = prev_func_[0];
 	CFunc* pw = prev_func_[1];
 	int acc_x = accumulate_into(px), acc_w = accumulate_into(pw);
+	net_->joinSide();
 	if (packs()) {
 		void* gp = net_->g_pack_;
 		check(cnb_pack_matrix(ctx(), out_.dz_star_real_, out_.dz_star_imag_, batch(), out_size_, gp, 0, stream()));
-		// Small problems give each of the 148 persistent CTAs only a few k-blocks, so prologue and
-		// epilogue dominate: run the two independent products side by side on half the SMs each.
-		const bool side_by_side = net_->side_stream_ != nullptr &&
-				(size_t) batch() * in1_len * out_size_ <= (size_t) 1536 * 1024 * 1024;
-		if (side_by_side) {
+		// Small problems give each of the 148 persistent CTAs only a few k-blocks, so prologue and epilogue dominate: the two
+		// independent products run side by side, and what follows dX* on the main stream does not wait for dW*, only the next
+		// use of the packed gradient does (joinSide).  In a captured step they take half the SMs each unless they nearly fit
+		// beside each other (us a step: 8 blocks of 1024 at 512 rows 701, each as alone 772; a language model of 43 x 1682 -> 284
+		// 124, 107).  Launched one by one the second is a few us behind the first anyway, and each goes as it would alone (4 blocks
+		// of 500 at 300 rows 289 one after the other, 311 in halves, 272; of 1024 at 512 423, 439, 408; of 300 at 2500 476, 447, 438).
+		if (net_->side_stream_ != nullptr && (size_t) batch() * in1_len * out_size_ <= (size_t) 1536 * 1024 * 1024) {
 			cudaStream_t ms = (cudaStream_t) stream(), ss = (cudaStream_t) net_->side_stream_;
-			int limit = net_->dp_gemm_ctas_ > 0 ? net_->dp_gemm_ctas_ : net_->sm_count_;
+			const int limit = net_->dp_gemm_ctas_;               // > 0: beside a collective
+			const bool halves = limit > 0 || (net_->capturing_ && !fitTogether());
 			cudaEventRecord((cudaEvent_t) net_->ev_side_fork_, ms);
 			cudaStreamWaitEvent(ss, (cudaEvent_t) net_->ev_side_fork_, 0);
-			cnb_set_gemm_sm_limit(ctx(), limit / 2);
-			check(cnb_linear_bwd_w_packed(ctx(), gp, x_pack_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
-					in1_len, out_size_, acc_w, ss));
+			cnb_set_gemm_sm_limit(ctx(), halves ? (limit > 0 ? limit : net_->sm_count_) / 2 : 0);
 			check(cnb_linear_bwd_x_packed(ctx(), gp, w_pack_, px->out_.dz_star_real_, px->out_.dz_star_imag_, batch(),
 					in1_len, out_size_, acc_x, ms));
-			cnb_set_gemm_sm_limit(ctx(), net_->dp_gemm_ctas_ > 0 ? net_->dp_gemm_ctas_ : 0);
+			check(cnb_linear_bwd_w_packed(ctx(), gp, x_pack_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
+					in1_len, out_size_, acc_w, ss));
+			cnb_set_gemm_sm_limit(ctx(), limit > 0 ? limit : 0);
 			cudaEventRecord((cudaEvent_t) net_->ev_side_join_, ss);
-			cudaStreamWaitEvent(ms, (cudaEvent_t) net_->ev_side_join_, 0);
+			net_->side_weight_ = pw;
+			if (limit > 0) net_->joinSide();
 			return;
 		}
 		check(cnb_linear_bwd_w_packed(ctx(), gp, x_pack_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
@@ -687,7 +706,7 @@ bool CNet::allocateOnGpu(int B) {
 	batch_ = cur_batch_ = B;
 	cnb_device_info(device_, &sm_count_, nullptr, nullptr, nullptr);
 	if (!bounce_ && cudaMallocHost(&bounce_, kBounceBytes) != cudaSuccess) { bounce_ = nullptr; cudaGetLastError(); }
-	if (stream_ && !side_stream_) {             // a second stream only makes sense beside a real (non-default) stream
+	if (!side_stream_) {
 		cudaStream_t st;
 		cudaEvent_t e0, e1;
 		if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess &&
@@ -1026,14 +1045,22 @@ void CNet::forward() {
 	}
 }
 
+void CNet::joinSide() {
+	if (!side_weight_) return;
+	cudaStreamWaitEvent((cudaStream_t) stream_, (cudaEvent_t) ev_side_join_, 0);
+	side_weight_ = nullptr;
+}
+
 void CNet::backward() {
 	if (!ctx_) { fail(CNB_ERR_ARG, "backward: allocateOnGpu first (there is no CPU path)"); return; }
+	struct Join { CNet* net; ~Join() { net->joinSide(); } } join = {this};       // however this pass ends
 	for (auto f : func_list_) f->grad_written_ = false;
 	main_out_->prev_func_[0]->grad_written_ = true;        // seeded by CrossEntropy::forward
 	if (dp_gemm_ctas_ > 0) cnb_set_gemm_sm_limit(ctx_, dp_gemm_ctas_);
 	size_t next_bucket = 0;
 	for (auto it = func_list_.rbegin(); it != func_list_.rend(); ++it) {
 		CFunc* f = *it;
+		if (side_weight_ && std::find(f->prev_func_.begin(), f->prev_func_.end(), side_weight_) != f->prev_func_.end()) joinSide();
 		if (!f->fused_away_ || dynamic_cast<Residual*>(f)) f->backward();
 		if (!ok_) return;
 		while (next_bucket < buckets_.size() && buckets_[next_bucket].last_writer == f) {
@@ -1049,6 +1076,7 @@ void CNet::backward() {
 
 bool CNet::reduceBucket(size_t k) {
 	const Bucket& b = buckets_[k];
+	if (nccl_.active() || sym_active_ || hook_) joinSide();          // a product of the bucket may still be on the second stream
 	if ((nccl_.active() || sym_active_ || hook_) && k == 0) {
 		// The arena accumulates until the update and is summed over the ranks in place: a second backward()
 		// before the update would reduce the already reduced part again (earlier micro-batches x ranks).

@@ -272,6 +272,9 @@ class Linear : public CFunc {                       // impl/linear.h:11-156
 	void* w_pack_ = nullptr;
 	bool x_is_packed_ = false;                      // the producer of x has written x_pack_ itself
 	unsigned long long w_pack_version_ = ~0ull;
+	int fit_batch_ = 0;                             // what fit_ holds for
+	bool fit_ = false;
+	bool fitTogether();
 	bool packs() const;                             // the batch in flight runs on packed operands
 	size_t extraBytes(int batch) const override;
 	void bindExtra(char* mem, int batch) override;
@@ -412,6 +415,8 @@ class CNet {
 	void* side_stream_ = nullptr;                   // second compute stream: dW* runs beside dX* at small batches
 	void* ev_side_fork_ = nullptr;
 	void* ev_side_join_ = nullptr;
+	CFunc* side_weight_ = nullptr;                  // whose gradient is written there; the main stream has yet to wait for ev_side_join_
+	void joinSide();
 	int sm_count_ = 0;
 	NcclGroup nccl_;                                // native data parallelism (setDataParallel)
 	// data parallelism over symmetric memory with the library's own all-reduce kernel (setSymmetricPeers)

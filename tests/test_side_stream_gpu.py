@@ -1,0 +1,94 @@
+"""dW* on a stream of its own: gradients are complete for whatever follows backward() on the net's stream, the default one
+included, and the products of a weight that two layers share add up."""
+import numpy as np
+import pytest
+
+from cnet_b200 import configs
+from cnet_b200.configs import CROSSENT, FOURIER, GELU, INPUT, LINEAR
+from cnet_b200.net import Net
+
+pytestmark = pytest.mark.gpu
+
+
+def _train(build, batch, n_in, m, own_stream, captured=False):
+    import torch
+    net = Net()
+    weights = build(net)
+    rng = np.random.default_rng(5)
+    stream = torch.cuda.Stream() if own_stream else torch.cuda.default_stream()
+    net.allocate(batch, stream=stream.cuda_stream if own_stream else None)
+    for uid, n, std in weights:
+        net.set_values(uid, *[(rng.standard_normal(n) * std).astype(np.float32) for _ in range(2)])
+    x = tuple(torch.from_numpy(rng.standard_normal((batch, n_in)).astype(np.float32)).pin_memory() for _ in range(2))
+    labels = torch.from_numpy(rng.integers(0, m, batch).astype(np.int32)).pin_memory()
+    net.upload(x=x, labels=labels)
+    got = []
+    with torch.cuda.stream(stream):
+        if captured:
+            net.sync()
+            net.capture_begin()
+            net.forward()
+            net.backward()
+            net.capture_end()
+        for _ in range(3):
+            net.update_inputs(0.0)                       # clears the gradients
+            if captured:
+                net.graph_launch()
+            else:
+                net.forward()
+                net.backward()
+            got.append(net.grad_tensor().clone())        # in stream order behind backward(), nothing else
+    torch.cuda.synchronize()
+    net.sync()
+    return [g.cpu().numpy() for g in got]
+
+
+@pytest.mark.parametrize("batch,n", [(128, 128), (300, 500), (260, 1024)])
+def test_gradients_are_complete_behind_backward(batch, n):
+    def build(net):
+        return configs.build_mixer(net, n=n, blocks=3, m=10).weights
+    runs = _train(build, batch, n, 10, False) + _train(build, batch, n, 10, True) + _train(build, batch, n, 10, True, captured=True)
+    for g in runs[1:]:
+        assert np.isfinite(g).all()
+        # the same products, perhaps in other schedules: reassociation only
+        assert np.linalg.norm(g - runs[0]) < 2e-5 * np.linalg.norm(runs[0])
+
+
+def test_a_weight_of_two_layers():
+    n, m, batch = 128, 10, 128
+
+    def build(net, shared):
+        x = net.add(INPUT, n)
+        f = net.add(FOURIER, n, prev=[x])
+        w = net.add(INPUT, n * n)
+        a = net.add(LINEAR, n, n * n, prev=[f, w])
+        g = net.add(GELU, n, prev=[a])
+        w2 = w if shared else net.add(INPUT, n * n)
+        b = net.add(LINEAR, n, n * n, prev=[g, w2])
+        wh = net.add(INPUT, n * m)
+        head = net.add(LINEAR, n, n * m, prev=[b, wh])
+        net.add(CROSSENT, m, prev=[head])
+        return [(w, n * n, n ** -0.5)] + ([] if shared else [(w2, n * n, n ** -0.5)]) + [(wh, n * m, n ** -0.5)]
+
+    def grads(shared):
+        import torch
+        net = Net()
+        weights = build(net, shared)
+        net.allocate(batch)
+        rng = np.random.default_rng(1)
+        w = [(rng.standard_normal(n * n) * n ** -0.5).astype(np.float32) for _ in range(2)]
+        wh = [(rng.standard_normal(n * m) * n ** -0.5).astype(np.float32) for _ in range(2)]
+        for uid, size, _ in weights:
+            net.set_values(uid, *(w if size == n * n else wh))
+        x = tuple(torch.from_numpy(rng.standard_normal((batch, n)).astype(np.float32)).pin_memory() for _ in range(2))
+        net.upload(x=x, labels=torch.from_numpy(rng.integers(0, m, batch).astype(np.int32)).pin_memory())
+        for _ in range(2):
+            net.update_inputs(0.0)
+            net.forward()
+            net.backward()
+        net.sync()
+        return [np.stack(net.get_wgrad(uid)) for uid, size, _ in weights if size == n * n]
+
+    one, two = grads(True), grads(False)
+    want = two[0] + two[1]
+    assert np.linalg.norm(one[0] - want) < 1e-5 * np.linalg.norm(want)
