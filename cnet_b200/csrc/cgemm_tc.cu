@@ -1582,7 +1582,7 @@ __global__ void zero_pair_k(float* __restrict__ a, float* __restrict__ b, size_t
 
 // The schedule of one product: which form (one CTA per tile or CTA pairs), how many CTAs, how the (tile, k-block)
 // units are dealt.  Host arithmetic only (also reachable as cnb_gemm_schedule, for tests that need no GPU).
-struct Schedule { bool pair; long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles, joined; int tile_n, first, rest; };
+struct Schedule { bool pair; long ctas, upc; int whole_per_cta, clear_from_row, cluster, segments; bool splits_tiles, joined; int tile_n, first, rest; bool exact; };
 
 // Sizes whose products have always been split ones here, at 19 bits an operand: packed ones are nearer to float64 there
 // whatever the length of the chain (512 x 1024 x 1024: 1.9e-6 -> 0.9e-6, 4096 x 1024 x 1024: 4.5e-6 -> 3.1e-6).
@@ -1661,7 +1661,7 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         r.splits_tiles = false;
     };
     const int c0 = r.cluster;
-    if (r.whole_per_cta > 0 || r.segments > 0 || (r.pair && c0 > 1)) return;
+    if (r.whole_per_cta > 0 || r.segments > 0) return;
     if (c0 == 1 && !r.splits_tiles) {                    // a CTA or a pair to a tile
         const Chains now = chain_blocks(M, N, K, r);
         const bool whole = r.pair ? now.rest >= k_blocks || now.exact : r.ctas == wide;
@@ -1669,7 +1669,7 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         return;
     }
     if (c0 > 1 && (k_blocks + c0 - 1) / c0 > kMaxChain16 / 2) return;        // (chains that are taken out one after the other)
-    if (c0 > 1 && narrow <= fit(c0)) return take(NARROW, c0);
+    if (c0 > 1 && !r.pair && narrow <= fit(c0)) return take(NARROW, c0);
     if ((c0 > 1 && (N <= BN || (accumulate && M <= BM))) || K > 4096) return;
 
     // The chains of the runs from k-block `from` to `to`: how many, and the sum of the cubes of their lengths, which is what the square of
@@ -1705,7 +1705,7 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
             u = end;
         }
     }
-    if (now.rest < (c0 > 1 ? (k_blocks + c0 - 1) / c0 : r.upc)) cubes -= cubes / 20;       // (1010 x 1595, K = 323: as many, 1.03 as far off)
+    const bool several = now.rest < (c0 > 1 ? (k_blocks + c0 - 1) / c0 : r.upc);
     // Costs in hundredths of a microsecond: blocks, what a cluster adds, taking a chain out of tensor memory before the next.
     struct { int tile_n, c, first, rest; long cost; } best = {0, 0, 0, 0, 0};
     auto consider = [&](int tile_n, int c, bool as_it_is) {
@@ -1718,20 +1718,28 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         for (int rest = std::min(run, now.rest); rest >= 1; --rest)
             for (int first = rest; first >= std::max(1, rest - 1); --first) {
                 const Sum v = cluster_of(c, first, rest);
-                if (!as_it_is && v.cubes * tiles > cubes) continue;
+                // (as many cubes in other runs may be 1.03 as far off: 1010 x 1595, K = 323)
+                if (!as_it_is && v.cubes * tiles * 20 > cubes * (several && c != c0 ? 19 : 20)) continue;
                 const long cost = fixed + (thin ? 50 : 100) * (v.chains - 1);
                 if (best.c == 0 || cost < best.cost) best = {tile_n, c, first, rest, cost};
                 return;
             }
     };
-    if (c0 > 1) consider(BN, c0, true);
-    const long before = c0 == 1 ? (N % 4 == 0 ? 800 : 1500) + (split_sizes(M, N, K) ? 0 : 300) - (accumulate ? 300 : 0) + 80 * r.upc
-                                : best.c ? best.cost : 1 << 30;
-    best.c = 0;
-    for (int c = c0 == 1 ? 8 : c0 / 2; c >= 1; c /= 2) { consider(BN, c, false); consider(NARROW, c, false); }
+    long before = 1 << 30;
+    if (c0 == 1) {
+        before = (N % 4 == 0 ? 800 : 1500) + (split_sizes(M, N, K) ? 0 : 300) - (accumulate ? 300 : 0) + 80 * r.upc;
+    } else if (r.pair) {                                 // two pairs to a tile of 256 x 128: as two CTAs to one of 128 x 128
+        before = 90 * ((k_blocks + 1) / 2) + 430 + 100 * (cluster_of(c0, now.first, now.rest).chains - 1);
+    } else {
+        consider(BN, c0, true);
+        if (best.c) before = best.cost;
+        best.c = 0;
+    }
+    for (int c = c0 == 1 || r.pair ? 8 : c0 / 2; c >= 1; c /= 2) { consider(BN, c, false); consider(NARROW, c, false); }
     if (best.c == 0 || best.cost > before - 100) return;
     r.first = best.first;
     r.rest = best.rest;
+    r.exact = several && now.exact;                      // runs of a single chain too
     take(best.tile_n, best.c);
 }
 
@@ -1870,6 +1878,7 @@ Schedule choose_schedule(int M, int N, int K, int accumulate, int sm_count, int 
     r.cluster = q.cluster; r.segments = q.segments; r.splits_tiles = q.splits_tiles; r.joined = q.joined;
     r.tile_n = BN;
     r.first = r.rest = 0;
+    r.exact = false;
     if (packed) narrow_tiles(r, M, N, K, k_blocks, accumulate, sm_limit > 0 ? std::min(sm_limit, sm_count) : sm_count);
     return r;
 }
@@ -2018,7 +2027,7 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     // several tiles a CTA (a single tile's runs are not: 83 x 102, K = 13688 took 1.4 us more in that form)
     const int tiles = (M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM) * ((N + BN - 1) / BN);
     const bool several = cluster == 1 && q.segments == 0 && tiles > 1 && (q.whole_per_cta > 0 || q.upc != k_blocks);
-    const Drain drain = !packed || (run <= p.chain && !several) ? NONE : run > p.chain && chains.exact ? EXACT : OVERLAP;
+    const Drain drain = q.exact ? EXACT : !packed || (run <= p.chain && !several) ? NONE : run > p.chain && chains.exact ? EXACT : OVERLAP;
     auto go = [&](auto kernel, const auto& maps) {
         return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(drain == NONE ? Threads<NONE>::ALL : Threads<OVERLAP>::ALL), SMEM_BYTES, st,
                            pair ? 2 * cluster : cluster, maps, p);
