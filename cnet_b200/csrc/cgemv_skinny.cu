@@ -15,6 +15,34 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// Sums of V values over the lanes of a warp, one of them a lane: on return v[0] is the sum of value lane_value<V>(lane), added in
+// the order of warp_sum.  Half of the values change hands at each of its steps, V - 1 shuffles in the place of 5 V.
+template <int V> __host__ __device__ constexpr int pow2_above() { return V <= 2 ? 2 : V <= 4 ? 4 : V <= 8 ? 8 : V <= 16 ? 16 : 32; }
+template <int V> __device__ __forceinline__ int lane_value(int lane) { return lane / (32 / pow2_above<V>()); }
+template <int V> __device__ __forceinline__ void warp_sums(float (&v)[V], int lane) {
+    static_assert(V <= 32, "a value a lane");
+    constexpr int P = pow2_above<V>();
+    float x[P];
+#pragma unroll
+    for (int k = 0; k < P; ++k) x[k] = k < V ? v[k < V ? k : 0] : 0.f;
+#pragma unroll
+    for (int step = 0, n = P; step < 5; ++step, n /= 2) {
+        const int o = 16 >> step;
+        if (n > 1) {
+            const bool upper = lane & o;
+#pragma unroll
+            for (int k = 0; k < P / 2; ++k) {
+                if (k >= n / 2) continue;
+                const float keep = upper ? x[k + n / 2] : x[k], send = upper ? x[k] : x[k + n / 2];
+                x[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        } else {
+            x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+        }
+    }
+    v[0] = x[0];
+}
+
 // Ordinary loads, here and below: the kernels before this one in the stream may still be writing what it reads until
 // cnb_pdl_enter returns, and a load through the read-only path (__ldg) is not held behind that.
 __device__ __forceinline__ void ldv(const float* p, float (&v)[4]) {
@@ -111,11 +139,14 @@ skinny_fwd_rows_k(const float* xr, const float* xi, const float* wr,
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long b0 = (long) blockIdx.x * RB;
     const long b1 = RB > 1 && b0 + 1 < B ? b0 + 1 : b0;
-    float a[RB][OT][2];
+    float a[RB][OT * 2];
 #pragma unroll
     for (int r = 0; r < RB; ++r)
 #pragma unroll
-        for (int o = 0; o < OT; ++o) a[r][o][0] = a[r][o][1] = 0.f;
+        for (int o = 0; o < OT * 2; ++o) a[r][o] = 0.f;
+    // Nothing here asks whether an output exists: behind such a branch each one's weights were a round trip to L2 of their own and
+    // each one's sum a chain of shuffles (86 x 256 -> 13 5.0 us, 3.1 so; 64 x 784 -> 10 4.3 and 3.5; 256 x 256 -> 16 5.9 and 3.6).
+    constexpr int G = OT <= 10 ? OT : 8;                 // outputs whose weights are in flight together
     for (int i = threadIdx.x * W; i < in; i += 256 * W) {
         float p[RB][W], q[RB][W];
 #pragma unroll
@@ -124,28 +155,31 @@ skinny_fwd_rows_k(const float* xr, const float* xi, const float* wr,
             ldv(xr + at, p[r]); ldv(xi + at, q[r]);
         }
 #pragma unroll
-        for (int o = 0; o < OT; ++o) {
-            if (o < out) {
-                float c[W], d[W];
-                ldv(wr + (size_t) o * in + i, c); ldv(wi + (size_t) o * in + i, d);
+        for (int g = 0; g < OT; g += G) {
+            float c[G][W], d[G][W];
+#pragma unroll
+            for (int o = 0; o < G; ++o) {
+                const size_t at = (size_t) min(g + o, out - 1) * in + i;
+                ldv(wr + at, c[o]); ldv(wi + at, d[o]);
+            }
+#pragma unroll
+            for (int o = 0; o < G; ++o)
 #pragma unroll
                 for (int r = 0; r < RB; ++r)
 #pragma unroll
                     for (int k = 0; k < W; ++k) {
-                        a[r][o][0] += p[r][k] * c[k] - q[r][k] * d[k];
-                        a[r][o][1] += p[r][k] * d[k] + q[r][k] * c[k];
+                        // (which product of the two is rounded is the compiler's choice in skinny_fwd_k: as there)
+                        a[r][2 * (g + o)] += fmaf(p[r][k], c[o][k], -(q[r][k] * d[o][k]));
+                        a[r][2 * (g + o) + 1] += W == 4 ? fmaf(p[r][k], d[o][k], q[r][k] * c[o][k]) : fmaf(q[r][k], c[o][k], p[r][k] * d[o][k]);
                     }
-            }
         }
     }
+    const int mine = lane_value<OT * 2>(lane);
 #pragma unroll
-    for (int r = 0; r < RB; ++r)
-#pragma unroll
-        for (int o = 0; o < OT; ++o)
-            if (o < out) {
-                const float re = warp_sum(a[r][o][0]), im = warp_sum(a[r][o][1]);
-                if (lane == 0) { part[warp][(r * OT + o) * 2] = re; part[warp][(r * OT + o) * 2 + 1] = im; }
-            }
+    for (int r = 0; r < RB; ++r) {
+        warp_sums<OT * 2>(a[r], lane);
+        if (mine < OT * 2) part[warp][r * OT * 2 + mine] = a[r][0];          // (lanes of one value write the same)
+    }
     __syncthreads();
     if (threadIdx.x < RB * OT * 2) {
         const int r = threadIdx.x / (OT * 2), o = threadIdx.x % (OT * 2) / 2;
@@ -234,7 +268,8 @@ skinny_bwd_w_stage1_k(const float* gr, const float* gi, const float* xr,
                       const float* xi, float* __restrict__ pr, float* __restrict__ pi, int B, int in,
                       int out, int rows_per_chunk) {
     cnb_pdl_enter();
-    __shared__ float sr[8][32 * W + 1], si[8][32 * W + 1];
+    constexpr int G = 4;                                 // outputs summed over the row lanes at a time
+    __shared__ __align__(16) float sr[G][8][32 * W + 4], si[G][8][32 * W + 4];
     const int col = (blockIdx.x * 32 + threadIdx.x) * W;
     const int r0 = blockIdx.y * rows_per_chunk, r1 = min(B, r0 + rows_per_chunk);
     float ar[OT][W], ai[OT][W];
@@ -243,18 +278,23 @@ skinny_bwd_w_stage1_k(const float* gr, const float* gi, const float* xr,
 #pragma unroll
         for (int k = 0; k < W; ++k) ar[o][k] = ai[o][k] = 0.f;
     if (col < in) {
-#pragma unroll 2
         for (int b = r0 + threadIdx.y; b < r1; b += 8) {
-            float x[W], y[W];
+            float x[W], y[W], a[OT], c[OT];
             ldv(xr + (size_t) b * in + col, x); ldv(xi + (size_t) b * in + col, y);
+            // all of G's row at once, whether or not the outputs exist: each behind a branch of its own they were a round trip
+            // to L2 each (200 x 333 -> 16, both stages, 6.3 -> 4.9 us)
+#pragma unroll
+            for (int o = 0; o < OT; ++o) {
+                const size_t at = (size_t) b * out + min(o, out - 1);
+                a[o] = cnb_ld_behind_wait(gr + at); c[o] = cnb_ld_behind_wait(gi + at);
+            }
 #pragma unroll
             for (int o = 0; o < OT; ++o) {
                 if (o < out) {
-                    const float a = gr[(size_t) b * out + o], c = gi[(size_t) b * out + o];
 #pragma unroll
                     for (int k = 0; k < W; ++k) {
-                        ar[o][k] += a * x[k] + c * y[k];       // (a + ic)(x - iy)
-                        ai[o][k] += c * x[k] - a * y[k];
+                        ar[o][k] += a[o] * x[k] + c[o] * y[k];   // (a + ic)(x - iy)
+                        ai[o][k] += c[o] * x[k] - a[o] * y[k];
                     }
                 }
             }
@@ -262,25 +302,29 @@ skinny_bwd_w_stage1_k(const float* gr, const float* gi, const float* xr,
     }
     const int t = threadIdx.y * 32 + threadIdx.x;
 #pragma unroll
-    for (int o = 0; o < OT; ++o) {
-        if (o < out) {
-            __syncthreads();
+    for (int g = 0; g < OT; g += G) {
+        if (g >= out) break;
+        __syncthreads();
 #pragma unroll
-            for (int k = 0; k < W; ++k) {
-                sr[threadIdx.y][threadIdx.x * W + k] = ar[o][k];
-                si[threadIdx.y][threadIdx.x * W + k] = ai[o][k];
+        for (int o = 0; o < G && g + o < OT; ++o) {
+            // (single floats, four apart from lane to lane, met in the banks: 86 x 256 -> 13 6.3 -> 4.9 us, 1000 x 700 -> 12 21.3 -> 15.3)
+            if constexpr (W == 4) {
+                *reinterpret_cast<float4*>(&sr[o][threadIdx.y][threadIdx.x * 4]) = make_float4(ar[g + o][0], ar[g + o][1], ar[g + o][2], ar[g + o][3]);
+                *reinterpret_cast<float4*>(&si[o][threadIdx.y][threadIdx.x * 4]) = make_float4(ai[g + o][0], ai[g + o][1], ai[g + o][2], ai[g + o][3]);
+            } else {
+                sr[o][threadIdx.y][threadIdx.x] = ar[g + o][0];
+                si[o][threadIdx.y][threadIdx.x] = ai[g + o][0];
             }
-            __syncthreads();
-            if (t < 32 * W) {
-                int c = blockIdx.x * 32 * W + t;
-                if (c < in) {
-                    float a = 0.f, d = 0.f;
+        }
+        __syncthreads();
+        for (int e = t; e < G * 32 * W; e += 256) {
+            const int o = e / (32 * W), u = e % (32 * W), c = blockIdx.x * 32 * W + u;
+            if (g + o >= out || c >= in) continue;
+            float a = 0.f, d = 0.f;
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) { a += sr[k][t]; d += si[k][t]; }
-                    size_t off = ((size_t) blockIdx.y * out + o) * in + c;
-                    pr[off] = a; pi[off] = d;
-                }
-            }
+            for (int k = 0; k < 8; ++k) { a += sr[o][k][u]; d += si[o][k][u]; }
+            const size_t off = ((size_t) blockIdx.y * out + g + o) * in + c;
+            pr[off] = a; pi[off] = d;
         }
     }
 }

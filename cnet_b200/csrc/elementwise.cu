@@ -103,7 +103,7 @@ colreduce_stage1_k(const float* __restrict__ gr, const float* __restrict__ gi,
                    int B, int N, int rows_per_chunk,
                    int* __restrict__ done, float* __restrict__ dvr, float* __restrict__ dvi, int accumulate_v) {
     cnb_pdl_enter();
-    __shared__ float sr[8][32 * W + 1], si[8][32 * W + 1];
+    __shared__ __align__(16) float sr[8][32 * W + 4], si[8][32 * W + 4];
     __shared__ int s_last;
     const int col = (blockIdx.x * 32 + threadIdx.x) * W;
     const int r0 = blockIdx.y * rows_per_chunk;
@@ -146,10 +146,15 @@ colreduce_stage1_k(const float* __restrict__ gr, const float* __restrict__ gi,
             }
         }
     }
+    if constexpr (W == 4) {                              // (four single floats of a lane meet those of seven others in the banks)
+        *reinterpret_cast<float4*>(&sr[threadIdx.y][threadIdx.x * 4]) = make_float4(accr[0], accr[1], accr[2], accr[3]);
+        *reinterpret_cast<float4*>(&si[threadIdx.y][threadIdx.x * 4]) = make_float4(acci[0], acci[1], acci[2], acci[3]);
+    } else {
 #pragma unroll
-    for (int k = 0; k < W; ++k) {
-        sr[threadIdx.y][threadIdx.x * W + k] = accr[k];
-        si[threadIdx.y][threadIdx.x * W + k] = acci[k];
+        for (int k = 0; k < W; ++k) {
+            sr[threadIdx.y][threadIdx.x * W + k] = accr[k];
+            si[threadIdx.y][threadIdx.x * W + k] = acci[k];
+        }
     }
     __syncthreads();
     // 32 * W columns of this block, summed over the 8 row lanes by the first 32 * W threads
