@@ -5,7 +5,10 @@
 // threads share a row and hold E elements of every plane each, so that a row of any usual length finds a form in which
 // most of them work and enough loads are in flight: 8 lanes (rows up to 32, four rows to a warp), a warp (up to 512), a
 // CTA of 128 (2048) or 512 threads (8192), a cluster of up to eight such CTAs (65536, partial sums through distributed
-// shared memory).  16-byte accesses where the row length and the planes allow them, else consecutive threads take
+// shared memory).  Elements that a row does not have still take registers, and so CTAs from an SM: with 16 a thread for all
+// rows beyond 128, forward, loss and backward one behind the other took 34.8 us at 4096 x 1000 (now, with 8, 28.9), 82.4 at
+// 2000 x 3000 (53.4), 119 at 65000 x 130 (78.9), 131 at 9000 x 777 (69.8), 109 at 1000 x 6001 (with 12, 82.1); the same
+// sums.  16-byte accesses where the row length and the planes allow them, else consecutive threads take
 // consecutive elements.  65536 x 20 through a CTA of one warp per row took 69 us a kernel, 300 x 27000 through two
 // passes over each row 60 to 82.
 #include <algorithm>
@@ -288,7 +291,7 @@ bool vec_ok(int n, std::initializer_list<const void*> planes) {
 
 }  // namespace
 
-// The form for rows of n elements (the lines are where a thread's 4 or 16 elements are used up) and its launch; NAME is
+// The form for rows of n elements (the lines are where a thread's 4, 8, 12 or 16 elements are used up) and its launch; NAME is
 // the kernel, the argument list ends with rows, n, parts and what may follow them.
 #define CNB_ROWS_GO(NAME, G, E, V, CTAS, PARTS, ...)                                                                     \
     cnb::launch(NAME<G, E, V>, dim3((unsigned) (CTAS)), dim3(cta_threads(G)), 0, st, PARTS, __VA_ARGS__)
@@ -296,8 +299,14 @@ bool vec_ok(int n, std::initializer_list<const void*> planes) {
     do {                                                                                                                 \
         if ((n) <= 32) CNB_ROWS_GO(NAME, 8, 4, V, ((size_t) (rows) + 31) / 32, 1, __VA_ARGS__);                          \
         else if ((n) <= 128) CNB_ROWS_GO(NAME, 32, 4, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                     \
+        else if ((n) <= 256) CNB_ROWS_GO(NAME, 32, 8, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                     \
+        else if ((n) <= 384) CNB_ROWS_GO(NAME, 32, 12, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                    \
         else if ((n) <= 512) CNB_ROWS_GO(NAME, 32, 16, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                    \
+        else if ((n) <= 1024) CNB_ROWS_GO(NAME, 128, 8, V, rows, 1, __VA_ARGS__);                                        \
+        else if ((n) <= 1536) CNB_ROWS_GO(NAME, 128, 12, V, rows, 1, __VA_ARGS__);                                       \
         else if ((n) <= 2048) CNB_ROWS_GO(NAME, 128, 16, V, rows, 1, __VA_ARGS__);                                       \
+        else if ((n) <= 4096) CNB_ROWS_GO(NAME, 512, 8, V, rows, 1, __VA_ARGS__);                                        \
+        else if ((n) <= 6144) CNB_ROWS_GO(NAME, 512, 12, V, rows, 1, __VA_ARGS__);                                       \
         else CNB_ROWS_GO(NAME, 512, 16, V, (size_t) (rows) * parts, parts, __VA_ARGS__);                                 \
     } while (0)
 #define CNB_ROWS(NAME, vec, rows, n, ...)                                                                                \

@@ -1,0 +1,34 @@
+"""Normalisation and loss at row lengths on both sides of every line between their forms."""
+import pytest
+
+from cnet_b200.ops import Context
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [k + d for k in (32, 128, 256, 384, 512, 1024, 1536, 2048, 4096, 6144, 8192) for d in (-1, 0, 1)])
+def test_both_sides_of_the_lines(n):
+    import torch
+    ctx = Context(arena_bytes=64 << 20)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(n)
+    rows = 37
+    z = tuple(torch.randn(rows, n, generator=gen, device="cuda") for _ in range(2))
+    g = tuple(torch.randn(rows, n, generator=gen, device="cuda") for _ in range(2))
+    labels = torch.randint(0, n, (rows,), generator=gen, device="cuda", dtype=torch.int32)
+    labels[0], labels[1] = 0, n - 1
+    full = lambda t: torch.complex(t[0].double(), t[1].double())
+    Z, G = full(z), full(g)
+    norm = Z.abs().pow(2).sum(1, keepdim=True).sqrt()
+    near = lambda got, want: float((got - want).norm() / want.norm()) < 2e-6          # sums of n terms in 32 bits, in pairs and dozens
+    y, inv = ctx.softmax_fwd(z)
+    assert near(full(y), Z / norm) and near(inv.double(), 1 / norm[:, 0])
+    want = G / norm - Z * (G * Z.conj()).real.sum(1, keepdim=True) / norm ** 3
+    assert near(full(ctx.softmax_bwd(g, z, inv)), want)
+    loss, d = ctx.crossent(z, labels)
+    power, rest = Z.abs().pow(2), torch.arange(rows, device="cuda")
+    S, m = power.sum(1), power[rest, labels.long()]
+    assert near(loss.double(), -torch.log(m / S))
+    c = (1 / S)[:, None].repeat(1, n)
+    c[rest, labels.long()] = -(S - m) / (m * S)
+    assert near(full(d), Z * c)
