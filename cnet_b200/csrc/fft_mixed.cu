@@ -185,8 +185,9 @@ __device__ __forceinline__ void tail_loop(const MixedPlan& pl, const Io& io, con
     }
 }
 
-template <int FINISH, bool CHIRP, int SHIFT>
-__global__ void __launch_bounds__(MAX_THREADS, 2)
+// CTAS: how many of 256 threads an SM's registers are to hold, two or three (fewer_waves).
+template <int FINISH, bool CHIRP, int SHIFT, int CTAS>
+__global__ void __launch_bounds__(MAX_THREADS, CTAS)
 fft_mixed_k(const float* __restrict__ xr, const float* __restrict__ xi, float* yr, float* yi,
             const float2* __restrict__ tw, const float2* __restrict__ chirp, const float2* __restrict__ spectrum, int B,
             const FftEpilogue ep, const __grid_constant__ MixedPlan pl) {
@@ -412,6 +413,19 @@ void plan_batch(MixedPlan* pl, int B, int sms) {
     pl->rows = rows;
 }
 
+// Whether 80 registers a thread instead of `regs` save a wave of CTAs.  What they cost in loads and arithmetic ahead is more than
+// what they give where they do not (us, with 96 or 112 and with 80: 1000 x 1500 with its tail 1.1 waves of three CTAs to an SM, 22.5 and
+// 16.0 by four; 4096 x 784 plain 19.0 and 17.1, with the tail 39.2 and 30.3; 2000 x 2000 32.9 and 27.3; but 500 x 900, half a wave of
+// either, 4.6 and 5.4; 4096 x 512, 1.5 and 1.2, 10.6 and 11.6; 6000 x 600 with the tail, 2.7 and 2.03, 38.1 and 40.9).
+bool fewer_waves(long ctas, int threads, size_t smem, int regs, int sms) {
+    auto waves = [&](int r) {
+        const long by_registers = 65536 / ((long) threads * r), by_memory = (long) (227 * 1024 / (smem + 1024));
+        const long fit = std::max(1L, std::min({by_registers, by_memory, 2048L / threads})) * sms;
+        return (ctas + fit - 1) / fit;
+    };
+    return waves(80) < waves(regs);
+}
+
 // The tail in a loop through shared memory, by all threads: written out behind a butterfly of 16 points it is 30 KB of
 // instructions, which a small batch runs through once, at the pace of their first fetch, on the few threads that have a last
 // butterfly (16 x 256 5.7 -> 3.0 us, 296 x 100 4.3 -> 2.9, 296 x 500 5.6 -> 4.2, 512 x 784 8.2 -> 6.4; in a training step, where other kernels'
@@ -484,24 +498,37 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
     const size_t smem = smem_bytes(pl.m, pl.rows, pl.buffers);
     static bool attr_done[64] = {};                         // the attribute is per device
     if (!attr_done[ctx->device & 63]) {
-#define CNB_MIXED_ATTR(F)                                                                                                          \
-    do {                                                                                                                           \
-        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, false, SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM)); \
-        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, false, NO_SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM)); \
-        CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, true, SPREAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM));  \
-    } while (0)
-        CNB_MIXED_ATTR(STORE); CNB_MIXED_ATTR(TAIL); CNB_MIXED_ATTR(ADD); CNB_MIXED_ATTR(TAIL_LOOP);
+#define CNB_MIXED_ATTR(F, C, S, N) \
+    CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, C, S, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM))
+#define CNB_MIXED_ATTRS(F, N) CNB_MIXED_ATTR(F, false, SPREAD, N); CNB_MIXED_ATTR(F, false, NO_SPREAD, N)
+        CNB_MIXED_ATTRS(STORE, 2); CNB_MIXED_ATTRS(TAIL, 2); CNB_MIXED_ATTRS(ADD, 2); CNB_MIXED_ATTRS(TAIL_LOOP, 2);
+        CNB_MIXED_ATTRS(STORE, 3); CNB_MIXED_ATTRS(TAIL, 3); CNB_MIXED_ATTRS(ADD, 3);
+        CNB_MIXED_ATTR(STORE, true, SPREAD, 2); CNB_MIXED_ATTR(TAIL, true, SPREAD, 2); CNB_MIXED_ATTR(ADD, true, SPREAD, 2);
+        CNB_MIXED_ATTR(TAIL_LOOP, true, SPREAD, 2);
+#undef CNB_MIXED_ATTRS
 #undef CNB_MIXED_ATTR
         attr_done[ctx->device & 63] = true;
     }
     const dim3 grid((unsigned) ((B + pl.rows - 1) / pl.rows)), block((unsigned) pl.threads);
     auto go = [&](auto kernel) { return cnb::launch(kernel, grid, block, smem, st, 1, xr, xi, yr, yi, tw, ch, spec, B, ep, pl); };
-#define CNB_MIXED(F) \
-    CNB_CUDA(chirp ? go(fft_mixed_k<F, true, SPREAD>) : pl.shift == SPREAD ? go(fft_mixed_k<F, false, SPREAD>) : go(fft_mixed_k<F, false, NO_SPREAD>))
-    if (finish == TAIL) CNB_MIXED(TAIL);
-    else if (finish == TAIL_LOOP) CNB_MIXED(TAIL_LOOP);
-    else if (finish == ADD) CNB_MIXED(ADD);
-    else CNB_MIXED(STORE);
+    const bool spread = pl.shift == SPREAD;
+#define CNB_MIXED(F, N) CNB_CUDA(spread ? go(fft_mixed_k<F, false, SPREAD, N>) : go(fft_mixed_k<F, false, NO_SPREAD, N>))
+    if (chirp) {
+        CNB_CUDA(finish == TAIL ? go(fft_mixed_k<TAIL, true, SPREAD, 2>) : finish == TAIL_LOOP ? go(fft_mixed_k<TAIL_LOOP, true, SPREAD, 2>) :
+                 finish == ADD ? go(fft_mixed_k<ADD, true, SPREAD, 2>) : go(fft_mixed_k<STORE, true, SPREAD, 2>));
+    } else if (finish == TAIL_LOOP) {
+        CNB_MIXED(TAIL_LOOP, 2);
+    } else if (fewer_waves((long) grid.x, pl.threads, smem, finish == TAIL ? 112 : 96, usable_sms(ctx))) {
+        if (finish == TAIL) CNB_MIXED(TAIL, 3);
+        else if (finish == ADD) CNB_MIXED(ADD, 3);
+        else CNB_MIXED(STORE, 3);
+    } else if (finish == TAIL) {
+        CNB_MIXED(TAIL, 2);
+    } else if (finish == ADD) {
+        CNB_MIXED(ADD, 2);
+    } else {
+        CNB_MIXED(STORE, 2);
+    }
 #undef CNB_MIXED
     CNB_LAUNCH_CHECK("fft_mixed");
     return CNB_OK;
