@@ -392,14 +392,16 @@ bool cached_plan(int N, MixedPlan* out) {
 
 // Rows per CTA and threads: about four CTAs to an SM (up to 52 KB of shared memory each), so that some load or store
 // while others transform; rows are spread over the SMs first when the batch is small; of the thread counts the one
-// that wastes the fewest lanes over the passes, or, with no more than a CTA to an SM, the one with the fewest butterflies
-// one after another (64 x 784, 128 threads instead of 64: 5.7 -> 5.1 us, with the tail 8.3 -> 6.4).
+// that wastes the fewest lanes over the passes, or, with no more than 1.75 CTAs to an SM, the one with the fewest butterflies
+// one after another (64 x 784, 128 threads instead of 64: 5.7 -> 5.1 us, with the tail 8.3 -> 6.4; at 1.5 to 1.7, 900 x 303 19.8 -> 13.6, 1000 x 300
+// 4.5 -> 3.7, 250 x 784 4.5 -> 3.9; at 2.0, 3000 x 137 16.0 and 16.6, 2662 x 77 3.2 and 3.7).
 void plan_batch(MixedPlan* pl, int B, int sms) {
     const size_t budget = 52 * 1024;
     int rows = 1;
     while (rows < 64 && smem_bytes(pl->m, rows + 1, std::max(1, pl->buffers)) <= budget && (long) (rows + 1) * pl->m <= 4096) ++rows;
     rows = std::max(1, std::min(rows, (B + 2 * sms - 1) / (2 * sms)));
-    const bool alone = (B + rows - 1) / rows <= sms;
+    const long ctas = (B + rows - 1) / rows;
+    const bool alone = 4 * ctas <= 7L * sms;
     double best = 1e30;
     for (int t = 64; t <= MAX_THREADS; t += 32) {
         double c = 0;
