@@ -1768,8 +1768,9 @@ Chains chain_blocks(int M, int N, int K, const Schedule& q) {
 // are, on 148 SMs) never are, and neither are short runs summed with atomics.  The estimate below, fitted to 20 sizes at every
 // width and cluster that has room and to 40 that ran as such sums, has to promise a microsecond (300 x 500, K = 500 19.2 -> 17.3,
 // 256 x 512, K = 512 17.1 -> 15.2, 128 x 2048, K = 512 30.4 -> 18.7, 350 x 401, K = 1081 35.6 -> 22.7; 512 x 1024, K = 1024 stays
-// as it is).  Over 660 products of 24 to 2500 rows and columns 1.07 times as fast as without narrow tiles, none slower by more
-// than runs of one program differ, and none further off float64: chains are as short as that takes.
+// as it is).  Over 600 products of 24 to 2500 rows and columns 1.09 times as fast as without narrow tiles, none slower by more than
+// runs of one program differ; of those whose sums are in another order none is more than 1.02 times as far off float64, and in the
+// mean they are nearer: chains are as short as that takes.
 //
 // Products with an N of up to 128, and gradients with an M of up to 128, are those of a head.  The gradient of a loss divides by
 // what they give, which magnifies a sum in another order, so they keep theirs where it is fixed.

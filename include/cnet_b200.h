@@ -116,7 +116,8 @@ int cnb_reserve_scratch(cnb_ctx* ctx, size_t bytes);
  * CTAs per cluster, k-blocks per run, whole tiles per CTA before the shared remainder, k-segments per tile
  * (K > 4096), tiles summed with atomics or not, first row of the output that atomics touch}. */
 int cnb_gemm_schedule(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8);
-/* The same for packed operands (k-blocks of 32), which all other tensor-core products run on. */
+/* The same for packed operands (k-blocks of 32), which all other tensor-core products run on.  Launches without pairs may have tiles
+ * of 128 x 64: their CTAs are then ceil(M / 128) ceil(N / 64) clusters. */
 int cnb_gemm_schedule_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out8);
 /* k-blocks of 32 that such a launch sums in tensor memory at most: a longer run is cut into chains of that many, which are
  * added up in registers.  (An error code, below zero, for sizes that are none.) */
