@@ -145,8 +145,9 @@ skinny_fwd_rows_k(const float* xr, const float* xi, const float* wr,
 #pragma unroll
         for (int o = 0; o < OT * 2; ++o) a[r][o] = 0.f;
     // Nothing here asks whether an output exists: behind such a branch each one's weights were a round trip to L2 of their own and
-    // each one's sum a chain of shuffles (86 x 256 -> 13 5.0 us, 3.1 so; 64 x 784 -> 10 4.3 and 3.5; 256 x 256 -> 16 5.9 and 3.6).
+    // each one's sum a chain of shuffles (86 x 256 -> 13 5.0 us, 3.1 so; 64 x 784 -> 10 4.3 and 3.5; 256 x 256 -> 16 5.9 and 3.6; 64 x 785 -> 10 5.7 and 4.0).
     constexpr int G = OT <= 10 ? OT : 8;                 // outputs whose weights are in flight together
+#pragma unroll(W == 1 ? 4 : 1)
     for (int i = threadIdx.x * W; i < in; i += 256 * W) {
         float p[RB][W], q[RB][W];
 #pragma unroll
@@ -168,9 +169,9 @@ skinny_fwd_rows_k(const float* xr, const float* xi, const float* wr,
                 for (int r = 0; r < RB; ++r)
 #pragma unroll
                     for (int k = 0; k < W; ++k) {
-                        // (which product of the two is rounded is the compiler's choice in skinny_fwd_k: as there)
+                        // (which product of the two is rounded first was the compiler's choice for each form, and is kept)
                         a[r][2 * (g + o)] += fmaf(p[r][k], c[o][k], -(q[r][k] * d[o][k]));
-                        a[r][2 * (g + o) + 1] += W == 4 ? fmaf(p[r][k], d[o][k], q[r][k] * c[o][k]) : fmaf(q[r][k], c[o][k], p[r][k] * d[o][k]);
+                        a[r][2 * (g + o) + 1] += W == 4 || RB == 2 ? fmaf(p[r][k], d[o][k], q[r][k] * c[o][k]) : fmaf(q[r][k], c[o][k], p[r][k] * d[o][k]);
                     }
         }
     }
@@ -278,25 +279,38 @@ skinny_bwd_w_stage1_k(const float* gr, const float* gi, const float* xr,
 #pragma unroll
         for (int k = 0; k < W; ++k) ar[o][k] = ai[o][k] = 0.f;
     if (col < in) {
-        for (int b = r0 + threadIdx.y; b < r1; b += 8) {
-            float x[W], y[W], a[OT], c[OT];
-            ldv(xr + (size_t) b * in + col, x); ldv(xi + (size_t) b * in + col, y);
-            // all of G's row at once, whether or not the outputs exist: each behind a branch of its own they were a round trip
-            // to L2 each (200 x 333 -> 16, both stages, 6.3 -> 4.9 us)
+        auto add = [&](int o, float a, float c, const float (&x)[W], const float (&y)[W]) {
 #pragma unroll
-            for (int o = 0; o < OT; ++o) {
-                const size_t at = (size_t) b * out + min(o, out - 1);
-                a[o] = cnb_ld_behind_wait(gr + at); c[o] = cnb_ld_behind_wait(gi + at);
+            for (int k = 0; k < W; ++k) {
+                ar[o][k] += a * x[k] + c * y[k];         // (a + ic)(x - iy)
+                ai[o][k] += c * x[k] - a * y[k];
             }
+        };
+        if constexpr (W == 4) {
+            for (int b = r0 + threadIdx.y; b < r1; b += 8) {
+                float x[W], y[W], a[OT], c[OT];
+                ldv(xr + (size_t) b * in + col, x); ldv(xi + (size_t) b * in + col, y);
+                // all of G's row at once, whether or not the outputs exist: each behind a branch of its own they were a round
+                // trip to L2 each
 #pragma unroll
-            for (int o = 0; o < OT; ++o) {
-                if (o < out) {
-#pragma unroll
-                    for (int k = 0; k < W; ++k) {
-                        ar[o][k] += a[o] * x[k] + c[o] * y[k];   // (a + ic)(x - iy)
-                        ai[o][k] += c[o] * x[k] - a[o] * y[k];
-                    }
+                for (int o = 0; o < OT; ++o) {
+                    const size_t at = (size_t) b * out + min(o, out - 1);
+                    a[o] = cnb_ld_behind_wait(gr + at); c[o] = cnb_ld_behind_wait(gi + at);
                 }
+#pragma unroll
+                for (int o = 0; o < OT; ++o)
+                    if (o < out) add(o, a[o], c[o], x, y);
+            }
+        } else {
+            // one column a lane: as many loads of G as of anything, and rows enough on their way (4096 x 1025 -> 10 31.8 us, with G
+            // requested as above 44.8)
+#pragma unroll 2
+            for (int b = r0 + threadIdx.y; b < r1; b += 8) {
+                float x[W], y[W];
+                ldv(xr + (size_t) b * in + col, x); ldv(xi + (size_t) b * in + col, y);
+#pragma unroll
+                for (int o = 0; o < OT; ++o)
+                    if (o < out) add(o, gr[(size_t) b * out + o], gi[(size_t) b * out + o], x, y);
             }
         }
     }
