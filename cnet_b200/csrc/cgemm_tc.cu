@@ -1757,6 +1757,19 @@ Chains chain_blocks(int M, int N, int K, const Schedule& q) {
     return {q.joined && n > c ? (n % c + c + 1) / 2 : c, c, true};
 }
 
+// The form of a packed launch: chains are taken out of tensor memory one after the other wherever a run is cut, also where only the
+// run of a tile's first blocks is (785 x 1218, K = 616 added to a gradient, slices of 9 and 10 blocks and a first chain of 9: launched
+// as one chain each, which the plan is not, 1.13e-6 off float64 in the place of 1.08e-6).
+Drain drain_form(int M, int N, int K, const Schedule& q, const Chains& chains) {
+    const int k_blocks = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK, run = longest_run(q, k_blocks);
+    const int first_run = q.cluster > 1 ? k_blocks / q.cluster : run;
+    // several tiles a CTA (a single tile's runs are not: 83 x 102, K = 13688 took 1.4 us more in that form)
+    const int tiles = (M + (q.pair ? 2 * BM : BM) - 1) / (q.pair ? 2 * BM : BM) * ((N + BN - 1) / BN);
+    const bool several = q.cluster == 1 && q.segments == 0 && tiles > 1 && (q.whole_per_cta > 0 || q.upc != k_blocks);
+    const bool cut = run > chains.rest || first_run > chains.first;
+    return q.exact || (cut && chains.exact) ? EXACT : cut || several ? OVERLAP : NONE;
+}
+
 // Narrow tiles (128 x 64) for products of few tiles, one CTA to a tile's slice of K.  Past the MMAs such a launch takes as long as
 // half a tile of 128 x 128 needs three times: out of tensor memory (1.1 us), between the CTAs of a cluster (2.5 to 3.5 us, 38 bytes
 // a ns into an SM, and a barrier), into memory (1.2); and it leaves most SMs without a tile.
@@ -2145,14 +2158,10 @@ int cgemm_tc_presplit(cnb_ctx* ctx, const SplitOperand& a, const SplitOperand& b
     p.status = ctx->d_status;
     const bool vec = N % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_re) | reinterpret_cast<uintptr_t>(d_im) |
                                      reinterpret_cast<uintptr_t>(r_re) | reinterpret_cast<uintptr_t>(r_im)) & 15) == 0;
-    const int k_blocks = (K + bk - 1) / bk, run = longest_run(q, k_blocks);
     const Chains chains = chain_blocks(M, N, K, q);
     p.chain = chains.rest;
     p.first = chains.first;
-    // several tiles a CTA (a single tile's runs are not: 83 x 102, K = 13688 took 1.4 us more in that form)
-    const int tiles = (M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM) * ((N + BN - 1) / BN);
-    const bool several = cluster == 1 && q.segments == 0 && tiles > 1 && (q.whole_per_cta > 0 || q.upc != k_blocks);
-    const Drain drain = q.exact ? EXACT : !packed || (run <= p.chain && !several) ? NONE : run > p.chain && chains.exact ? EXACT : OVERLAP;
+    const Drain drain = packed ? drain_form(M, N, K, q, chains) : NONE;
     auto go = [&](auto kernel, const auto& maps) {
         return cnb::launch(kernel, dim3((unsigned) (pair ? 2 * ctas : ctas)), dim3(drain == NONE ? Threads<NONE>::ALL : Threads<OVERLAP>::ALL), SMEM_BYTES, st,
                            pair ? 2 * cluster : cluster, maps, p);
@@ -2312,4 +2321,16 @@ extern "C" int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm
         return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_chain_packed: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
     const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK);
     return chain_blocks(M, N, K, q).rest;
+}
+
+extern "C" int cnb_gemm_form_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out4) {
+    if (!out4 || M <= 0 || N <= 0 || K <= 0 || sm_count <= 0)
+        return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_form_packed: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
+    const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK);
+    const Chains chains = chain_blocks(M, N, K, q);
+    out4[0] = q.tile_n;
+    out4[1] = chains.first;
+    out4[2] = chains.rest;
+    out4[3] = drain_form(M, N, K, q, chains);
+    return CNB_OK;
 }

@@ -1,4 +1,5 @@
 """The schedule of products of few tiles (cnb_gemm_schedule_packed: host arithmetic, no GPU)."""
+import ctypes as C
 import random
 
 import pytest
@@ -30,3 +31,28 @@ def test_narrow_tiles_fit_the_device(limit):
         if K % 8 or M < 64 or N < 64:
             assert chain <= max(1, int(4.28 * K ** 0.5 / 32)), (M, N, K, chain)
     assert narrow > 100
+
+
+def _form(M, N, K, acc, limit=0):
+    out = (C.c_int * 4)()
+    assert L.load().cnb_gemm_form_packed(M, N, K, acc, SMS, limit, out) == 0
+    return dict(zip(("tile_n", "first", "rest", "form"), out))
+
+
+def test_runs_that_are_cut_are_launched_so():
+    """A launch of the form that makes one chain of every run has no run that is longer than its chains: not the longest, and not the
+    one that holds a tile's first blocks, whose first chain may be shorter."""
+    rng = random.Random(4)
+    sizes = [(785, 1218, 616, 1), (282, 2355, 696, 1), (280, 2320, 640, 0), (1136, 1008, 1008, 0), (363, 2393, 640, 1)]
+    sizes += [(8 * rng.randint(8, 350), 8 * rng.randint(8, 350), 8 * rng.randint(8, 512), rng.randint(0, 1)) for _ in range(4000)]
+    shorter = 0
+    for M, N, K, acc in sizes:
+        s, f = _schedule(M, N, K, acc, 0), _form(M, N, K, acc)
+        c = s["cluster_ctas"] // (2 if s["pair"] else 1)
+        k_blocks = -(-K // 32)
+        if c == 1:
+            continue
+        shorter += f["first"] < k_blocks // c
+        if k_blocks // c > f["first"] or -(-k_blocks // c) > f["rest"]:
+            assert f["form"] != 0, (M, N, K, acc, s, f)
+    assert shorter > 3

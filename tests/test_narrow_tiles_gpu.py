@@ -60,3 +60,28 @@ def test_narrow_tiles(M, N, K, cluster):
         near(ctx.linear_bwd_w(tuple(t.T.contiguous() for t in x), tuple(t.T.contiguous() for t in w), out=tuple(t.clone() for t in r)),
              X @ W.conj().T + full(r))
     assert lib.cnb_check_device_status(ctx.h, ctx._stream()) == 0
+
+
+@pytest.mark.parametrize("M,N,K,acc,former", [
+    # a shorter first chain: cut, though the longest run is a single chain
+    (785, 1218, 616, 1, 1.0849e-06),
+    (282, 2355, 696, 1, 1.1950e-06),
+    (280, 2320, 640, 0, 1.0843e-06),
+    (1136, 1008, 1008, 0, 1.7386e-06),
+])
+def test_no_further_off_than_the_former_schedule(M, N, K, acc, former):
+    """Sums in another order than runs of pairs, summed with atomics, had: `former` is what those were off float64 by on these inputs."""
+    import torch
+    ctx = Context(arena_bytes=(64 << 20) + 24 * (M * K + N * K + 64 * (M + N + K)))
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1000003 + M * 31 + N * 17 + K)
+    planes = lambda *n: (torch.randn(*n, generator=gen, device="cuda"), torch.randn(*n, generator=gen, device="cuda"))
+    full = lambda a: torch.complex(a[0].double(), a[1].double())
+    a, b = planes(M, K), planes(K, N) if acc else planes(N, K)
+    if acc:
+        got = ctx.linear_bwd_x(a, b, out=(torch.zeros(M, N, device="cuda"), torch.zeros(M, N, device="cuda")))
+        want = full(a) @ full(b).conj()
+    else:
+        got, want = ctx.linear_fwd(a, b), full(a) @ full(b).T
+    err = float((full(got) - want).norm() / want.norm())
+    assert err <= 1.002 * former, (err, former)          # (atomics add in any order)
