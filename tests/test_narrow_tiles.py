@@ -56,3 +56,12 @@ def test_runs_that_are_cut_are_launched_so():
         if k_blocks // c > f["first"] or -(-k_blocks // c) > f["rest"]:
             assert f["form"] != 0, (M, N, K, acc, s, f)
     assert shorter > 3
+
+
+@pytest.mark.parametrize("M,N,K,acc,pair,atomics", [
+    (1820, 552, 163, 1, 1, 1),     # six chains of a block each either way: 1.16e-7 off float64 as runs of pairs, 1.18e-7 as one run
+    (2622, 482, 206, 0, 1, 1),
+])
+def test_as_many_cubes_in_another_order_are_left(M, N, K, acc, pair, atomics):
+    s = _schedule(M, N, K, acc, 0)
+    assert (s["pair"], s["atomics"]) == (pair, atomics), s

@@ -68,6 +68,10 @@ def test_narrow_tiles(M, N, K, cluster):
     (282, 2355, 696, 1, 1.1950e-06),
     (280, 2320, 640, 0, 1.0843e-06),
     (1136, 1008, 1008, 0, 1.7386e-06),
+    # as many cubes in other runs
+    (1820, 552, 163, 1, 1.1584e-07),
+    (2622, 482, 206, 0, 1.1640e-07),
+    (450, 591, 144, 0, 2.8908e-07),
 ])
 def test_no_further_off_than_the_former_schedule(M, N, K, acc, former):
     """Sums in another order than runs of pairs, summed with atomics, had: `former` is what those were off float64 by on these inputs."""
