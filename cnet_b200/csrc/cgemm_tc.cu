@@ -1781,8 +1781,9 @@ Drain drain_form(int M, int N, int K, const Schedule& q, const Chains& chains) {
 // are, on 148 SMs) never are, and neither are short runs summed with atomics.  The estimate below, fitted to 20 sizes at every
 // width and cluster that has room and to 40 that ran as such sums, has to promise a microsecond (300 x 500, K = 500 19.2 -> 17.3,
 // 256 x 512, K = 512 17.1 -> 15.2, 128 x 2048, K = 512 30.4 -> 18.7, 350 x 401, K = 1081 35.6 -> 22.7; 512 x 1024, K = 1024 stays
-// as it is).  Over 600 products of 24 to 2500 rows and columns 1.09 times as fast as without narrow tiles, none slower by more than
-// runs of one program differ.  Chains are as short as it takes that sums in another order are no further off float64: a twentieth
+// as it is).  Of 2100 products of 16 to 3000 rows and columns that run otherwise with
+// narrow tiles than without, the time is 0.82 of what it was in the mean; four take 2 to 9 % more (946 x 115, K = 2151, added, 29.7 ->
+// 32.3), the others no more than runs of one program differ.  Chains are as short as it takes that sums in another order are no further off float64: a twentieth
 // fewer cubes (below), since as many, cut elsewhere, are up to 1.02 times as far off.  Of 900 such products none is more than 1.002
 // times as far, and in the mean they are 0.89 times.
 //
@@ -1844,7 +1845,7 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
             u = end;
         }
     }
-    const bool several = now.rest < (c0 > 1 ? (k_blocks + c0 - 1) / c0 : r.upc);
+    const bool several = now.rest < (c0 > 1 ? (k_blocks + c0 - 1) / c0 : r.upc), vec = N % 4 == 0;
     // Costs in hundredths of a microsecond: blocks, what a cluster adds, taking a chain out of tensor memory before the next.
     struct { int tile_n, c, first, rest; long cost; } best = {0, 0, 0, 0, 0};
     auto consider = [&](int tile_n, int c, bool as_it_is) {
@@ -1852,7 +1853,14 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         static const int wide_add[4] = {140, 430, 590, 690}, narrow_add[4] = {0, 235, 345, 470};
         const bool thin = tile_n == NARROW, crowd = (thin ? narrow : wide) * c > 100 * sms / 148;
         const int log_c = c == 8 ? 3 : c == 4 ? 2 : c - 1, run = (k_blocks + c - 1) / c;
-        const long fixed = (thin ? (crowd ? 85 : 70) * run + narrow_add[log_c] : 90 * run + wide_add[log_c]) + (crowd && c == 8 ? 200 : 0);
+        long fixed = (thin ? (crowd ? 85 : 70) * run + narrow_add[log_c] : 90 * run + wide_add[log_c]) + (crowd && c == 8 ? 200 : 0);
+        // What is added to is read by the CTAs themselves: by one CTA for its whole tile, four bytes a lane where 16 do not fit, and
+        // by fewer CTAs of a smaller cluster (1013 x 1747, K = 366 as one run a tile 43.4 -> 55.6 us, 824 x 240, K = 680 in clusters of
+        // four 20.0 -> 21.6, 438 x 880, K = 104 as one run 16.2 -> 17.1).
+        if (accumulate && c == 1) fixed += vec ? (thin ? 300 : 100) : (thin ? 900 : 1900);
+        else if (accumulate && c0 > 1 && !r.pair && !as_it_is) fixed += 250;
+        // One row of tiles gains a microsecond less by a smaller cluster (64 x 2560, K = 336 19.1 -> 19.9).
+        else if (M <= BM && c0 > 1 && !r.pair && !as_it_is) fixed += 100;
         // the longest chains that are no less exact than those of the form before; a shorter first one where that does
         for (int rest = std::min(run, now.rest); rest >= 1; --rest)
             for (int first = rest; first >= std::max(1, rest - 1); --first) {
@@ -1866,7 +1874,7 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
     };
     long before = 1 << 30;
     if (c0 == 1) {
-        before = (N % 4 == 0 ? 800 : 1500) + (split_sizes(M, N, K) ? 0 : 300) - (accumulate ? 300 : 0) + 80 * r.upc;
+        before = (vec ? 800 : 1500) + (split_sizes(M, N, K) ? 0 : 300) - (accumulate ? 300 : 0) + 80 * r.upc;
     } else if (r.pair) {                                 // two pairs to a tile of 256 x 128: as two CTAs to one of 128 x 128
         before = 90 * ((k_blocks + 1) / 2) + 430 + 100 * (cluster_of(c0, now.first, now.rest).chains - 1);
     } else {
@@ -1875,7 +1883,11 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         best.c = 0;
     }
     for (int c = c0 == 1 || r.pair ? 8 : c0 / 2; c >= 1; c /= 2) { consider(BN, c, false); consider(NARROW, c, false); }
-    if (best.c == 0 || best.cost > before - 100) return;
+    // Runs with atomics may take less than the estimate where large clusters would replace them (257 x 112, K = 2375 21.3 -> 24.1,
+    // 1022 x 107, K = 2390 33.6 -> 35.0, 409 x 594, K = 1538 33.9 -> 37.7), which have to promise more than a microsecond then.
+    const bool eight = best.c == 8;
+    const long promise = c0 > 1 || accumulate || best.c < 4 ? 100 : !vec ? (eight ? 550 : 350) : !eight ? 100 : split_sizes(M, N, K) ? 250 : 400;
+    if (best.c == 0 || best.cost > before - promise) return;
     r.first = best.first;
     r.rest = best.rest;
     r.exact = several && now.exact;                      // runs of a single chain too

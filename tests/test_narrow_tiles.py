@@ -65,3 +65,16 @@ def test_runs_that_are_cut_are_launched_so():
 def test_as_many_cubes_in_another_order_are_left(M, N, K, acc, pair, atomics):
     s = _schedule(M, N, K, acc, 0)
     assert (s["pair"], s["atomics"]) == (pair, atomics), s
+
+
+@pytest.mark.parametrize("M,N,K,acc,ctas,cluster_ctas", [
+    (1013, 1747, 366, 1, 136, 2),      # a CTA that adds to its whole tile reads it four bytes a lane: 43.4 us as runs with atomics, 55.6
+    (2734, 478, 258, 1, 132, 2),
+    (171, 2961, 192, 1, 96, 2),
+    (824, 240, 680, 1, 112, 8),        # clusters half as wide read twice as many rows a CTA: 20.0 us, 21.6
+    (64, 2560, 336, 0, 80, 4),         # 19.1 us, 19.9
+    (1022, 107, 2390, 0, 120, 2),      # runs with atomics 33.6 us, clusters of eight 35.0
+])
+def test_products_that_smaller_clusters_slow_down(M, N, K, acc, ctas, cluster_ctas):
+    s, f = _schedule(M, N, K, acc, 0), _form(M, N, K, acc)
+    assert (s["ctas"], s["cluster_ctas"], f["tile_n"]) == (ctas, cluster_ctas, 128), (s, f)
