@@ -1816,13 +1816,9 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
     // the error goes with: what is truncated in a chain of C, C at the magnitude of sqrt(C).
     struct Sum { long chains, cubes; };
     auto chains_of = [&](int from, int to, int first, int rest) {
-        Sum v = {0, 0};
-        for (int kb = from; kb < to;) {
-            const long c = std::min(kb == 0 ? first : rest, to - kb);
-            ++v.chains; v.cubes += c * c * c;
-            kb += (int) c;
-        }
-        return v;
+        const int head = from == 0 ? std::min(first, to) : 0, whole = (to - from - head) / rest, left = (to - from - head) % rest;
+        auto cube = [](long n) { return n * n * n; };
+        return Sum{(head > 0) + whole + (left > 0), cube(head) + whole * cube(rest) + cube(left)};
     };
     auto cluster_of = [&](int c, int first, int rest) {                      // most chains of a CTA, and all cubes of a tile
         Sum v = {0, 0};
@@ -1833,21 +1829,25 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         return v;
     };
     const Chains now = chain_blocks(M, N, K, r);
-    long cubes = 0, tiles = 1;                           // of `tiles` tiles
-    if (c0 > 1) {
-        cubes = cluster_of(c0, now.first, now.rest).cubes;
-    } else {
-        tiles = r.pair ? (long) ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) : wide;
+    const long tiles = c0 > 1 ? 1 : r.pair ? (long) ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) : wide;
+    long all_cubes = 0;                                  // of `tiles` tiles, as they are; 0: not asked for yet
+    auto cubes = [&] {
+        if (all_cubes > 0) return all_cubes;
+        if (c0 > 1) return all_cubes = cluster_of(c0, now.first, now.rest).cubes;
+        long run_end = r.upc, tile = 0;                  // where the run ends; the tile's first unit
         for (long u = 0; u < tiles * k_blocks;) {
-            const long end = std::min({(u / r.upc + 1) * r.upc, (u / k_blocks + 1) * k_blocks});
-            const int kb = (int) (u % k_blocks);
-            cubes += chains_of(kb, kb + (int) (end - u), now.first, now.rest).cubes;
+            const long end = std::min(run_end, tile + k_blocks);
+            all_cubes += chains_of((int) (u - tile), (int) (end - tile), now.first, now.rest).cubes;
             u = end;
+            if (u == run_end) run_end += r.upc;
+            if (u == tile + k_blocks) tile = u;
         }
-    }
+        return all_cubes;
+    };
     const bool several = now.rest < (c0 > 1 ? (k_blocks + c0 - 1) / c0 : r.upc), vec = N % 4 == 0;
     // Costs in hundredths of a microsecond: blocks, what a cluster adds, taking a chain out of tensor memory before the next.
     struct { int tile_n, c, first, rest; long cost; } best = {0, 0, 0, 0, 0};
+    long before = 1 << 30;
     auto consider = [&](int tile_n, int c, bool as_it_is) {
         if ((tile_n == NARROW ? narrow : wide) > fit(c)) return;
         static const int wide_add[4] = {140, 430, 590, 690}, narrow_add[4] = {0, 235, 345, 470};
@@ -1861,18 +1861,20 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         else if (accumulate && c0 > 1 && !r.pair && !as_it_is) fixed += 250;
         // One row of tiles gains a microsecond less by a smaller cluster (64 x 2560, K = 336 19.1 -> 19.9).
         else if (M <= BM && c0 > 1 && !r.pair && !as_it_is) fixed += 100;
-        // the longest chains that are no less exact than those of the form before; a shorter first one where that does
-        for (int rest = std::min(run, now.rest); rest >= 1; --rest)
+        const int chain = thin ? 50 : 100;
+        // the longest chains that are no less exact than those of the form before; a shorter first one where that does.  No further
+        // than a cost that would be taken (the search through all of it took up to 14 us of the host's time a launch, 437 x 89, K = 3952).
+        const long most = best.c ? best.cost - 1 : before - 100;
+        for (int rest = std::min(run, now.rest); rest >= 1 && fixed + chain * ((run + rest - 1) / rest - 1) <= most; --rest)
             for (int first = rest; first >= std::max(1, rest - 1); --first) {
                 const Sum v = cluster_of(c, first, rest);
                 // (as many cubes in other runs may be 1.03 as far off: 1010 x 1595, K = 323; those of the same slices are not)
-                if (!as_it_is && v.cubes * tiles * 20 > cubes * (c == c0 && c0 > 1 ? 20 : 19)) continue;
-                const long cost = fixed + (thin ? 50 : 100) * (v.chains - 1);
+                if (!as_it_is && v.cubes * tiles * 20 > cubes() * (c == c0 && c0 > 1 ? 20 : 19)) continue;
+                const long cost = fixed + chain * (v.chains - 1);
                 if (best.c == 0 || cost < best.cost) best = {tile_n, c, first, rest, cost};
                 return;
             }
     };
-    long before = 1 << 30;
     if (c0 == 1) {
         before = (vec ? 800 : 1500) + (split_sizes(M, N, K) ? 0 : 300) - (accumulate ? 300 : 0) + 80 * r.upc;
     } else if (r.pair) {                                 // two pairs to a tile of 256 x 128: as two CTAs to one of 128 x 128
