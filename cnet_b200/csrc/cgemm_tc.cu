@@ -1770,6 +1770,43 @@ Drain drain_form(int M, int N, int K, const Schedule& q, const Chains& chains) {
     return q.exact || (cut && chains.exact) ? EXACT : cut || several ? OVERLAP : NONE;
 }
 
+// The chains of a run from k-block `from` to `to`: how many, and the sum of the cubes of their lengths, which is what the square of
+// the error goes with: what is truncated in a chain of C, C at the magnitude of sqrt(C).
+struct Sum { long chains, cubes; };
+Sum chains_of(int from, int to, int first, int rest) {
+    const int head = from == 0 ? std::min(first, to) : 0, whole = (to - from - head) / rest, left = (to - from - head) % rest;
+    auto cube = [](long n) { return n * n * n; };
+    return {(head > 0) + whole + (left > 0), cube(head) + whole * cube(rest) + cube(left)};
+}
+
+// The cubes of a packed launch, of a tile in the mean.
+double tile_cubes(int M, int N, int K, const Schedule& q) {
+    const int k_blocks = (K + FormCfg<PACKED>::BK - 1) / FormCfg<PACKED>::BK, tile_m = q.pair ? 2 * BM : BM;
+    const long tiles = (long) ((M + tile_m - 1) / tile_m) * ((N + q.tile_n - 1) / q.tile_n), units = tiles * k_blocks;
+    Chains chains = chain_blocks(M, N, K, q);
+    if (drain_form(M, N, K, q, chains) == NONE) chains.first = chains.rest = k_blocks;
+    double cubes = 0;
+    auto run = [&](long from, long to) { if (to > from) cubes += (double) chains_of((int) from, (int) to, chains.first, chains.rest).cubes; };
+    const long pieces = q.cluster > 1 ? q.cluster : q.segments;              // of every tile alike
+    if (pieces > 0) {
+        for (long k = 0; k < pieces; ++k)
+            if (q.cluster > 1) run(k_blocks * k / pieces, k_blocks * (k + 1) / pieces);
+            else run(k * q.upc, std::min<long>(k_blocks, (k + 1) * q.upc));
+        return cubes;
+    }
+    const long whole = std::min(tiles, q.whole_per_cta * q.ctas);
+    cubes = (double) whole * chains_of(0, k_blocks, chains.first, chains.rest).cubes;
+    long run_end = whole * k_blocks + q.upc, tile = whole * k_blocks;       // where a run ends; a tile's first unit
+    for (long u = tile; u < units && q.upc > 0;) {
+        const long end = std::min(run_end, tile + k_blocks);
+        run(u - tile, end - tile);
+        u = end;
+        if (u == run_end) run_end += q.upc;
+        if (u == tile + k_blocks) tile = u;
+    }
+    return cubes / tiles;
+}
+
 // Narrow tiles (128 x 64) for products of few tiles, one CTA to a tile's slice of K.  Past the MMAs such a launch takes as long as
 // half a tile of 128 x 128 needs three times: out of tensor memory (1.1 us), between the CTAs of a cluster (2.5 to 3.5 us, 38 bytes
 // a ns into an SM, and a barrier), into memory (1.2); and it leaves most SMs without a tile.
@@ -1812,14 +1849,6 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
     if (c0 > 1 && !r.pair && narrow <= fit(c0)) return take(NARROW, c0);
     if ((c0 > 1 && (N <= BN || (accumulate && M <= BM))) || K > 4096) return;
 
-    // The chains of the runs from k-block `from` to `to`: how many, and the sum of the cubes of their lengths, which is what the square of
-    // the error goes with: what is truncated in a chain of C, C at the magnitude of sqrt(C).
-    struct Sum { long chains, cubes; };
-    auto chains_of = [&](int from, int to, int first, int rest) {
-        const int head = from == 0 ? std::min(first, to) : 0, whole = (to - from - head) / rest, left = (to - from - head) % rest;
-        auto cube = [](long n) { return n * n * n; };
-        return Sum{(head > 0) + whole + (left > 0), cube(head) + whole * cube(rest) + cube(left)};
-    };
     auto cluster_of = [&](int c, int first, int rest) {                      // most chains of a CTA, and all cubes of a tile
         Sum v = {0, 0};
         for (int k = 0; k < c; ++k) {
@@ -2336,6 +2365,11 @@ extern "C" int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm
         return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_chain_packed: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
     const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK);
     return chain_blocks(M, N, K, q).rest;
+}
+
+extern "C" double cnb_gemm_truncation_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit) {
+    if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0) return -1.0;
+    return tile_cubes(M, N, K, choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK));
 }
 
 extern "C" int cnb_gemm_form_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out4) {

@@ -272,8 +272,9 @@ void Linear::forward() {
 			out_size_, stream()));
 }
 
-// Whether dX* and dW* of this batch, each as it would run alone, are not much more than the device holds at once: clusters of
-// eight and four CTAs leave some SMs of 148 without.
+// Whether dX* and dW* of this batch, each as it would run alone, are not much more than the device holds at once (clusters of
+// eight and four CTAs leave some SMs of 148 without), and no further off than on half of the device each: whole tiles of all SMs may
+// be one chain where those of half are two (4096 x 512 -> 512, dX* 9.3e-7 off float64 on half of the device, 1.83e-6 on all of it).
 bool Linear::fitTogether() {
 	if (fit_batch_ != batch()) {
 		const int sms = net_->sm_count_;
@@ -282,6 +283,13 @@ bool Linear::fitTogether() {
 		fit_batch_ = batch();
 		fit_ = cnb_gemm_schedule_packed(batch(), in1_len, out_size_, 0, sms, 0, x) == CNB_OK &&
 				cnb_gemm_schedule_packed(out_size_, in1_len, batch(), 1, sms, 0, w) == CNB_OK && share(x) + share(w) <= 1.5;
+		// (a twentieth fewer cubes, or the same single chain: as many in another order may be further off)
+		auto as_exact = [&](int M, int N, int K, int acc) {
+			const double alone = cnb_gemm_truncation_packed(M, N, K, acc, sms, 0), half = cnb_gemm_truncation_packed(M, N, K, acc, sms, sms / 2);
+			const double blocks = (K + 31) / 32, one = blocks * blocks * blocks;
+			return alone <= 0.95 * half || (alone == one && half == one);
+		};
+		fit_ = fit_ && as_exact(batch(), in1_len, out_size_, 0) && as_exact(out_size_, in1_len, batch(), 1);
 	}
 	return fit_;
 }
@@ -296,14 +304,15 @@ void Linear::backward() {
 		check(cnb_pack_matrix(ctx(), out_.dz_star_real_, out_.dz_star_imag_, batch(), out_size_, gp, 0, stream()));
 		// Small problems give each of the 148 persistent CTAs only a few k-blocks, so prologue and epilogue dominate: the two
 		// independent products run side by side, and what follows dX* on the main stream does not wait for dW*, only the next
-		// use of the packed gradient does (joinSide).  In a captured step they take half the SMs each unless they nearly fit
-		// beside each other (us a step: 8 blocks of 1024 at 512 rows 701, each as alone 772; a language model of 43 x 1682 -> 284
-		// 124, 107).  Launched one by one the second is a few us behind the first anyway, and each goes as it would alone (4 blocks
-		// of 500 at 300 rows 289 one after the other, 311 in halves, 272; of 1024 at 512 423, 439, 408; of 300 at 2500 476, 447, 438).
+		// use of the packed gradient does (joinSide).  On a net's own stream, captured or not (what a caller captures is not known
+		// here), they take half the SMs each unless they nearly fit beside each other (us a captured step: 8 blocks of 1024 at 512
+		// rows 701, each as alone 772; a language model of 43 x 1682 -> 284 124, 107).  On the default stream, launched one by
+		// one, the second is a few us behind the first anyway, and each goes as it would alone (4 blocks of 500 at 300 rows 289 one
+		// after the other, 311 in halves, 272; of 1024 at 512 423, 439, 408; of 300 at 2500 476, 447, 438).
 		if (net_->side_stream_ != nullptr && (size_t) batch() * in1_len * out_size_ <= (size_t) 1536 * 1024 * 1024) {
 			cudaStream_t ms = (cudaStream_t) stream(), ss = (cudaStream_t) net_->side_stream_;
 			const int limit = net_->dp_gemm_ctas_;               // > 0: beside a collective
-			const bool halves = limit > 0 || (net_->capturing_ && !fitTogether());
+			const bool halves = limit > 0 || (net_->side_halves_ && !fitTogether());
 			cudaEventRecord((cudaEvent_t) net_->ev_side_fork_, ms);
 			cudaStreamWaitEvent(ss, (cudaEvent_t) net_->ev_side_fork_, 0);
 			cnb_set_gemm_sm_limit(ctx(), halves ? (limit > 0 ? limit : net_->sm_count_) / 2 : 0);
@@ -713,6 +722,7 @@ bool CNet::allocateOnGpu(int B) {
 				cudaEventCreateWithFlags(&e0, cudaEventDisableTiming) == cudaSuccess &&
 				cudaEventCreateWithFlags(&e1, cudaEventDisableTiming) == cudaSuccess) {
 			side_stream_ = st; ev_side_fork_ = e0; ev_side_join_ = e1;
+			side_halves_ = stream_ != nullptr;
 		}
 	}
 	if ((rc = cnb_reserve_scratch(ctx_, scratchBytes(B, false))) != CNB_OK) { fail(rc, "scratch"); return false; }

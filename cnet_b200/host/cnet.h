@@ -274,7 +274,7 @@ class Linear : public CFunc {                       // impl/linear.h:11-156
 	unsigned long long w_pack_version_ = ~0ull;
 	int fit_batch_ = 0;                             // what fit_ holds for
 	bool fit_ = false;
-	bool fitTogether();
+	bool fitTogether();                             // dX* and dW* run beside each other as each would alone
 	bool packs() const;                             // the batch in flight runs on packed operands
 	size_t extraBytes(int batch) const override;
 	void bindExtra(char* mem, int batch) override;
@@ -417,6 +417,7 @@ class CNet {
 	void* ev_side_join_ = nullptr;
 	CFunc* side_weight_ = nullptr;                  // whose gradient is written there; the main stream has yet to wait for ev_side_join_
 	void joinSide();
+	bool side_halves_ = false;                      // allocated on a stream of its own: dX* and dW* on half of the device each
 	int sm_count_ = 0;
 	NcclGroup nccl_;                                // native data parallelism (setDataParallel)
 	// data parallelism over symmetric memory with the library's own all-reduce kernel (setSymmetricPeers)

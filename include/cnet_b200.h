@@ -125,6 +125,9 @@ int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm_count, int
 /* How such a launch sums: out4 = {columns of a tile, k-blocks of a tile's first chain, of its other chains, and the form: 0 every run
  * is one chain, 1 and 2 chains are taken out of tensor memory one accumulator at a time, or both together}. */
 int cnb_gemm_form_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit, int* out4);
+/* What it truncates: the sum of the cubes of its chains' k-blocks, of a tile in the mean, with which the square of that error goes.
+ * (-1 for sizes that are none.) */
+double cnb_gemm_truncation_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit);
 size_t cnb_split_floats(size_t n);
 int cnb_split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, void* stream);
 int cnb_linear_split_ok(int B, int in, int out);

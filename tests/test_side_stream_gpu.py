@@ -92,3 +92,59 @@ def test_a_weight_of_two_layers():
     one, two = grads(True), grads(False)
     want = two[0] + two[1]
     assert np.linalg.norm(one[0] - want) < 1e-5 * np.linalg.norm(want)
+
+
+def _bits(batch, n, how):
+    """Gradients of two blocks on a stream of the net's own: launched one by one, captured by the net, or captured by the caller."""
+    import torch
+    net = Net()
+    weights = configs.build_mixer(net, n=n, blocks=2, m=10).weights
+    rng = np.random.default_rng(7)
+    stream = torch.cuda.Stream()
+    net.allocate(batch, stream=stream.cuda_stream)
+    for uid, size, std in weights:
+        net.set_values(uid, *[(rng.standard_normal(size) * std).astype(np.float32) for _ in range(2)])
+    x = tuple(torch.from_numpy(rng.standard_normal((batch, n)).astype(np.float32)).pin_memory() for _ in range(2))
+    net.upload(x=x, labels=torch.from_numpy(rng.integers(0, 10, batch).astype(np.int32)).pin_memory())
+    net.forward()
+    net.backward()
+    net.sync()
+    with torch.cuda.stream(stream):
+        if how == "net":
+            net.capture_begin()
+            net.forward()
+            net.backward()
+            net.capture_end()
+        elif how == "caller":
+            graph = torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            graph.capture_begin(capture_error_mode="thread_local")
+            net.forward()
+            net.backward()
+            graph.capture_end()
+        net.update_inputs(0.0)                           # clears the gradients
+        if how == "net":
+            net.graph_launch()
+        elif how == "caller":
+            graph.replay()
+        else:
+            net.forward()
+            net.backward()
+        got = net.grad_tensor().clone()
+    torch.cuda.synchronize()
+    net.sync()
+    return got.cpu().numpy()
+
+
+@pytest.mark.parametrize("batch,n", [
+    # slices of K without atomics, others on half of the device than on all of it, which the two do not fit on together
+    (320, 640),
+    (512, 512),
+    (1024, 512),
+    # what does
+    (384, 192),
+])
+def test_a_nets_own_stream_has_one_schedule(batch, n):
+    """Steps that are launched and steps that are replayed, whoever captured them, add up in the same order."""
+    runs = [_bits(batch, n, how) for how in ("launched", "net", "caller")]
+    assert np.isfinite(runs[0]).all() and (runs[0] == runs[1]).all() and (runs[0] == runs[2]).all()
