@@ -1770,6 +1770,9 @@ Drain drain_form(int M, int N, int K, const Schedule& q, const Chains& chains) {
     return q.exact || (cut && chains.exact) ? EXACT : cut || several ? OVERLAP : NONE;
 }
 
+// Clusters of `ctas` CTAs, each with an SM to itself, that are resident at once: 15 of eight and 33 of four on 148 SMs.
+int resident_clusters(int ctas, int sms) { return ctas == 8 ? sms * 15 / 148 : ctas == 4 ? sms * 33 / 148 : sms / ctas; }
+
 // The chains of a run from k-block `from` to `to`: how many, and the sum of the cubes of their lengths, which is what the square of
 // the error goes with: what is truncated in a chain of C, C at the magnitude of sqrt(C).
 struct Sum { long chains, cubes; };
@@ -1827,7 +1830,7 @@ double tile_cubes(int M, int N, int K, const Schedule& q) {
 // Products with an N of up to 128, and gradients with an M of up to 128, are those of a head.  The gradient of a loss divides by
 // what they give, which magnifies a sum in another order, so they keep theirs where it is fixed.
 void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate, int sms) {
-    auto fit = [&](int c) { return c == 8 ? sms * 15 / 148 : c == 4 ? sms * 33 / 148 : sms / c; };
+    auto fit = [&](int c) { return resident_clusters(c, sms); };
     const long rows = (M + BM - 1) / BM, wide = rows * ((N + BN - 1) / BN), narrow = rows * ((N + NARROW - 1) / NARROW);
     auto take = [&](int tile_n, int c) {
         r.pair = false;
@@ -2365,6 +2368,13 @@ extern "C" int cnb_gemm_chain_packed(int M, int N, int K, int accumulate, int sm
         return cnb::set_error(CNB_ERR_ARG, "cnb_gemm_chain_packed: M=%d N=%d K=%d sm_count=%d", M, N, K, sm_count);
     const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, sm_limit, FormCfg<PACKED>::BK);
     return chain_blocks(M, N, K, q).rest;
+}
+
+extern "C" double cnb_gemm_share_packed(int M, int N, int K, int accumulate, int sm_count) {
+    if (M <= 0 || N <= 0 || K <= 0 || sm_count <= 0) return -1.0;
+    const Schedule q = choose_schedule(M, N, K, accumulate, sm_count, 0, FormCfg<PACKED>::BK);
+    const int ctas = q.cluster * (q.pair ? 2 : 1);
+    return (double) q.ctas / q.cluster / std::max(1, resident_clusters(ctas, sm_count));
 }
 
 extern "C" double cnb_gemm_truncation_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit) {

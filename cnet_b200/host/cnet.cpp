@@ -272,24 +272,23 @@ void Linear::forward() {
 			out_size_, stream()));
 }
 
-// Whether dX* and dW* of this batch, each as it would run alone, are not much more than the device holds at once (clusters of
-// eight and four CTAs leave some SMs of 148 without), and no further off than on half of the device each: whole tiles of all SMs may
-// be one chain where those of half are two (4096 x 512 -> 512, dX* 9.3e-7 off float64 on half of the device, 1.83e-6 on all of it).
-bool Linear::fitTogether() {
-	if (fit_batch_ != batch()) {
+// Whether dX* and dW* of this batch, each as it would run alone, are not much more than the device holds at once, and no further off
+// than on half of the device each: whole tiles of all SMs may be one chain where those of half are two (4096 x 512 -> 512, dX*
+// 9.3e-7 off float64 on half of the device, 1.83e-6 on all of it).
+bool Linear::fitTogether(int acc_x, int acc_w) {
+	const int acc = 2 * acc_x + acc_w, B = batch();
+	if (fit_batch_ != B || fit_acc_ != acc) {
 		const int sms = net_->sm_count_;
-		int x[8], w[8];
-		auto share = [&](const int* v) { return (double) v[1] / (v[2] == 8 ? sms * 120 / 148 : v[2] == 4 ? sms * 132 / 148 : sms); };
-		fit_batch_ = batch();
-		fit_ = cnb_gemm_schedule_packed(batch(), in1_len, out_size_, 0, sms, 0, x) == CNB_OK &&
-				cnb_gemm_schedule_packed(out_size_, in1_len, batch(), 1, sms, 0, w) == CNB_OK && share(x) + share(w) <= 1.5;
 		// (a twentieth fewer cubes, or the same single chain: as many in another order may be further off)
 		auto as_exact = [&](int M, int N, int K, int acc) {
 			const double alone = cnb_gemm_truncation_packed(M, N, K, acc, sms, 0), half = cnb_gemm_truncation_packed(M, N, K, acc, sms, sms / 2);
 			const double blocks = (K + 31) / 32, one = blocks * blocks * blocks;
 			return alone <= 0.95 * half || (alone == one && half == one);
 		};
-		fit_ = fit_ && as_exact(batch(), in1_len, out_size_, 0) && as_exact(out_size_, in1_len, batch(), 1);
+		fit_batch_ = B;
+		fit_acc_ = acc;
+		fit_ = cnb_gemm_share_packed(B, in1_len, out_size_, acc_x, sms) + cnb_gemm_share_packed(out_size_, in1_len, B, acc_w, sms) <= 1.5 &&
+				as_exact(B, in1_len, out_size_, acc_x) && as_exact(out_size_, in1_len, B, acc_w);
 	}
 	return fit_;
 }
@@ -312,7 +311,7 @@ void Linear::backward() {
 		if (net_->side_stream_ != nullptr && (size_t) batch() * in1_len * out_size_ <= (size_t) 1536 * 1024 * 1024) {
 			cudaStream_t ms = (cudaStream_t) stream(), ss = (cudaStream_t) net_->side_stream_;
 			const int limit = net_->dp_gemm_ctas_;               // > 0: beside a collective
-			const bool halves = limit > 0 || (net_->side_halves_ && !fitTogether());
+			const bool halves = limit > 0 || (net_->side_halves_ && !fitTogether(acc_x, acc_w));
 			cudaEventRecord((cudaEvent_t) net_->ev_side_fork_, ms);
 			cudaStreamWaitEvent(ss, (cudaEvent_t) net_->ev_side_fork_, 0);
 			cnb_set_gemm_sm_limit(ctx(), halves ? (limit > 0 ? limit : net_->sm_count_) / 2 : 0);

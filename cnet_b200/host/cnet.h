@@ -272,9 +272,9 @@ class Linear : public CFunc {                       // impl/linear.h:11-156
 	void* w_pack_ = nullptr;
 	bool x_is_packed_ = false;                      // the producer of x has written x_pack_ itself
 	unsigned long long w_pack_version_ = ~0ull;
-	int fit_batch_ = 0;                             // what fit_ holds for
+	int fit_batch_ = 0, fit_acc_ = 0;               // what fit_ holds for
 	bool fit_ = false;
-	bool fitTogether();                             // dX* and dW* run beside each other as each would alone
+	bool fitTogether(int acc_x, int acc_w);         // dX* and dW* run beside each other as each would alone
 	bool packs() const;                             // the batch in flight runs on packed operands
 	size_t extraBytes(int batch) const override;
 	void bindExtra(char* mem, int batch) override;

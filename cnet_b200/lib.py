@@ -94,6 +94,7 @@ SIGNATURES = {
     "cnb_gemm_schedule": (C.c_int, [C.c_int] * 6 + [C.POINTER(C.c_int)]),
     "cnb_gemm_schedule_packed": (C.c_int, [C.c_int] * 6 + [C.POINTER(C.c_int)]),
     "cnb_gemm_chain_packed": (C.c_int, [C.c_int] * 6),
+    "cnb_gemm_share_packed": (C.c_double, [C.c_int] * 5),
     "cnb_gemm_truncation_packed": (C.c_double, [C.c_int] * 6),
     "cnb_gemm_form_packed": (C.c_int, [C.c_int] * 6 + [C.POINTER(C.c_int)]),
     "cnb_sgd_update_split": (C.c_int, [_vp, _P, _P, _sz, C.c_float, C.c_int, _vp, C.c_int, _vp]),

@@ -128,6 +128,8 @@ int cnb_gemm_form_packed(int M, int N, int K, int accumulate, int sm_count, int 
 /* What it truncates: the sum of the cubes of its chains' k-blocks, of a tile in the mean, with which the square of that error goes.
  * (-1 for sizes that are none.) */
 double cnb_gemm_truncation_packed(int M, int N, int K, int accumulate, int sm_count, int sm_limit);
+/* How much of the device its CTAs are, 1 for as many as are resident at once.  (-1 for sizes that are none.) */
+double cnb_gemm_share_packed(int M, int N, int K, int accumulate, int sm_count);
 size_t cnb_split_floats(size_t n);
 int cnb_split_planes(cnb_ctx* ctx, const float* re, const float* im, size_t n, float* split, void* stream);
 int cnb_linear_split_ok(int B, int in, int out);

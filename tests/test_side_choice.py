@@ -26,4 +26,14 @@ def test_cubes_of_known_launches(M, N, K, acc, limit, cubes):
 
 def test_sizes_that_are_none():
     for bad in ((0, 1, 1), (1, 0, 1), (1, 1, 0)):
-        assert _cubes(*bad, 0, 0) == -1.0
+        assert _cubes(*bad, 0, 0) == -1.0 and L.load().cnb_gemm_share_packed(*bad, 0, SMS) == -1.0
+
+
+@pytest.mark.parametrize("M,N,K,acc,share", [
+    (512, 1024, 1024, 0, 32 / 33),                       # clusters of four
+    (512, 320, 512, 0, 20 / 33),
+    (512, 320, 512, 1, 12 / 15),                         # added to what is there: clusters of eight
+    (4096, 512, 512, 0, 64 / 74),                        # pairs
+])
+def test_shares_of_known_launches(M, N, K, acc, share):
+    assert L.load().cnb_gemm_share_packed(M, N, K, acc, SMS) == pytest.approx(share)

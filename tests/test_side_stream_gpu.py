@@ -148,3 +148,33 @@ def test_a_nets_own_stream_has_one_schedule(batch, n):
     """Steps that are launched and steps that are replayed, whoever captured them, add up in the same order."""
     runs = [_bits(batch, n, how) for how in ("launched", "net", "caller")]
     assert np.isfinite(runs[0]).all() and (runs[0] == runs[1]).all() and (runs[0] == runs[2]).all()
+
+
+def test_a_product_that_adds_is_asked_for_as_it_runs():
+    """Two layers of one input and one gradient, so that their dW* are the same product.  The second adds its dX* to the first's,
+    which is another schedule (512 x 320 -> 512): with it the two products do not fit together, and this dW* runs on half of the
+    device, in another order than the other."""
+    import torch
+    batch, n, m = 512, 320, 512
+    net = Net()
+    x = net.add(INPUT, n)
+    f = net.add(FOURIER, n, prev=[x])
+    wa, wb = net.add(INPUT, n * m), net.add(INPUT, n * m)
+    a, b = net.add(LINEAR, n, n * m, prev=[f, wa]), net.add(LINEAR, n, n * m, prev=[f, wb])
+    s = net.add(configs.RESIDUAL, m, prev=[a, b])
+    wh = net.add(INPUT, m * 10)
+    net.add(CROSSENT, 10, prev=[net.add(LINEAR, m, m * 10, prev=[s, wh])])
+    stream = torch.cuda.Stream()
+    net.allocate(batch, stream=stream.cuda_stream)
+    rng = np.random.default_rng(2)
+    for uid, size in ((wa, n * m), (wb, n * m), (wh, m * 10)):
+        net.set_values(uid, *[(rng.standard_normal(size) * n ** -0.5).astype(np.float32) for _ in range(2)])
+    planes = tuple(torch.from_numpy(rng.standard_normal((batch, n)).astype(np.float32)).pin_memory() for _ in range(2))
+    net.upload(x=planes, labels=torch.from_numpy(rng.integers(0, 10, batch).astype(np.int32)).pin_memory())
+    net.forward()
+    net.backward()
+    net.sync()
+    ga, gb = np.stack(net.get_wgrad(wa)), np.stack(net.get_wgrad(wb))
+    assert np.linalg.norm(ga - gb) < 1e-5 * np.linalg.norm(ga)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert (ga != gb).any()
