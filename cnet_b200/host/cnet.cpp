@@ -312,16 +312,22 @@ void Linear::backward() {
 			cudaStream_t ms = (cudaStream_t) stream(), ss = (cudaStream_t) net_->side_stream_;
 			const int limit = net_->dp_gemm_ctas_;               // > 0: beside a collective
 			const bool halves = limit > 0 || (net_->side_halves_ && !fitTogether(acc_x, acc_w));
-			cudaEventRecord((cudaEvent_t) net_->ev_side_fork_, ms);
-			cudaStreamWaitEvent(ss, (cudaEvent_t) net_->ev_side_fork_, 0);
+			cudaError_t e = cudaEventRecord((cudaEvent_t) net_->ev_side_fork_, ms);
+			if (e == cudaSuccess) e = cudaStreamWaitEvent(ss, (cudaEvent_t) net_->ev_side_fork_, 0);
+			if (e != cudaSuccess) {
+				cudaGetLastError();                              // (the next launch's check would find it again)
+				net_->fail(CNB_ERR_CUDA, std::string("backward: fork to the second stream: ") + cudaGetErrorString(e));
+				return;
+			}
 			cnb_set_gemm_sm_limit(ctx(), halves ? (limit > 0 ? limit : net_->sm_count_) / 2 : 0);
 			check(cnb_linear_bwd_x_packed(ctx(), gp, w_pack_, px->out_.dz_star_real_, px->out_.dz_star_imag_, batch(),
 					in1_len, out_size_, acc_x, ms));
 			check(cnb_linear_bwd_w_packed(ctx(), gp, x_pack_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
 					in1_len, out_size_, acc_w, ss));
 			cnb_set_gemm_sm_limit(ctx(), limit > 0 ? limit : 0);
-			cudaEventRecord((cudaEvent_t) net_->ev_side_join_, ss);
 			net_->side_weight_ = pw;
+			e = cudaEventRecord((cudaEvent_t) net_->ev_side_join_, ss);
+			if (e != cudaSuccess) net_->loseSide(e);
 			if (limit > 0) net_->joinSide();
 			return;
 		}
@@ -1056,8 +1062,17 @@ void CNet::forward() {
 
 void CNet::joinSide() {
 	if (!side_weight_) return;
-	cudaStreamWaitEvent((cudaStream_t) stream_, (cudaEvent_t) ev_side_join_, 0);
+	const cudaError_t e = cudaStreamWaitEvent((cudaStream_t) stream_, (cudaEvent_t) ev_side_join_, 0);
 	side_weight_ = nullptr;
+	if (e != cudaSuccess) loseSide(e);
+}
+
+// What follows cannot be ordered behind the second stream by an event: an error, and the host waits for it instead.
+void CNet::loseSide(int e) {
+	cudaStreamSynchronize((cudaStream_t) side_stream_);
+	cudaGetLastError();
+	side_weight_ = nullptr;
+	fail(CNB_ERR_CUDA, std::string("backward: join of the second stream: ") + cudaGetErrorString((cudaError_t) e));
 }
 
 void CNet::backward() {

@@ -417,6 +417,7 @@ class CNet {
 	void* ev_side_join_ = nullptr;
 	CFunc* side_weight_ = nullptr;                  // whose gradient is written there; the main stream has yet to wait for ev_side_join_
 	void joinSide();
+	void loseSide(int cuda_error);
 	bool side_halves_ = false;                      // allocated on a stream of its own: dX* and dW* on half of the device each
 	int sm_count_ = 0;
 	NcclGroup nccl_;                                // native data parallelism (setDataParallel)

@@ -1,10 +1,15 @@
 """dW* on a stream of its own: gradients are complete for whatever follows backward() on the net's stream, the default one
 included, and the products of a weight that two layers share add up."""
+import ctypes as C
+import os
+import subprocess
+
 import numpy as np
 import pytest
 
-from cnet_b200 import configs
+from cnet_b200 import build, configs
 from cnet_b200.configs import CROSSENT, FOURIER, GELU, INPUT, LINEAR
+from cnet_b200.lib import CnetError
 from cnet_b200.net import Net
 
 pytestmark = pytest.mark.gpu
@@ -178,3 +183,37 @@ def test_a_product_that_adds_is_asked_for_as_it_runs():
     assert np.linalg.norm(ga - gb) < 1e-5 * np.linalg.norm(ga)
     if torch.cuda.get_device_properties(0).multi_processor_count == 148:
         assert (ga != gb).any()
+
+
+@pytest.mark.parametrize("join", [0, 1])
+def test_an_event_that_fails_is_an_error(join, tmp_path):
+    """The second stream is ordered by events alone: a record or a wait that CUDA refuses (of no event) is an error of backward(), also
+    where no launch follows that would find it, and nothing is left running on that stream."""
+    import torch
+    so = str(tmp_path / "probe.so")
+    here = os.path.dirname(os.path.abspath(__file__))
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-fno-access-control", "-I/usr/local/cuda/include", os.path.join(here, "cpp", "side_event_probe.cpp"),
+                    "-o", so, "-L" + build.HERE, "-l:libcnet_b200.so", "-Wl,-rpath," + build.HERE], check=True)
+    swap = C.CDLL(so).swap_side_event
+    swap.restype, swap.argtypes = C.c_void_p, [C.c_void_p, C.c_int, C.c_void_p]
+    net = Net()
+    inp, w, wh = net.add(INPUT, 128), net.add(INPUT, 128 * 128), net.add(INPUT, 1280)
+    first = net.add(LINEAR, 128, 128 * 128, prev=[inp, w])               # the last one in backward()
+    net.add(CROSSENT, 10, prev=[net.add(LINEAR, 128, 1280, prev=[net.add(GELU, 128, prev=[first]), wh])])
+    net.allocate(128)
+    rng = np.random.default_rng(3)
+    for uid, size in ((w, 128 * 128), (wh, 1280)):
+        net.set_values(uid, *[(rng.standard_normal(size) * 0.1).astype(np.float32) for _ in range(2)])
+    x = tuple(torch.from_numpy(rng.standard_normal((128, 128)).astype(np.float32)).pin_memory() for _ in range(2))
+    net.upload(x=x, labels=torch.zeros(128, dtype=torch.int32).pin_memory())
+    net.forward()
+    event = swap(net.h, join, None)
+    with pytest.raises(CnetError):
+        net.backward()
+    swap(net.h, join, event)
+    torch.cuda.synchronize()
+    net.update_inputs(0.0)
+    net.forward()
+    net.backward()                                       # and with its event again it works
+    net.sync()
+    assert np.abs(np.stack(net.get_wgrad(w))).max() > 0
