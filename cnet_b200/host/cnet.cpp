@@ -319,12 +319,12 @@ void Linear::backward() {
 				net_->fail(CNB_ERR_CUDA, std::string("backward: fork to the second stream: ") + cudaGetErrorString(e));
 				return;
 			}
-			cnb_set_gemm_sm_limit(ctx(), halves ? (limit > 0 ? limit : net_->sm_count_) / 2 : 0);
+			if (halves) cnb_set_gemm_sm_limit(ctx(), (limit > 0 ? limit : net_->sm_count_) / 2);
 			check(cnb_linear_bwd_x_packed(ctx(), gp, w_pack_, px->out_.dz_star_real_, px->out_.dz_star_imag_, batch(),
 					in1_len, out_size_, acc_x, ms));
 			check(cnb_linear_bwd_w_packed(ctx(), gp, x_pack_, pw->out_.dz_star_real_, pw->out_.dz_star_imag_, batch(),
 					in1_len, out_size_, acc_w, ss));
-			cnb_set_gemm_sm_limit(ctx(), limit > 0 ? limit : 0);
+			if (halves) cnb_set_gemm_sm_limit(ctx(), limit > 0 ? limit : 0);
 			net_->side_weight_ = pw;
 			e = cudaEventRecord((cudaEvent_t) net_->ev_side_join_, ss);
 			if (e != cudaSuccess) net_->loseSide(e);

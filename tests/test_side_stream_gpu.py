@@ -217,3 +217,29 @@ def test_an_event_that_fails_is_an_error(join, tmp_path):
     net.backward()                                       # and with its event again it works
     net.sync()
     assert np.abs(np.stack(net.get_wgrad(w))).max() > 0
+
+
+def test_a_limit_that_a_caller_has_set_stays():
+    """cnb_set_gemm_sm_limit on a net of the default stream: backward() runs under it, and so does what follows."""
+    import torch
+    batch, n = 512, 512
+    runs = []
+    for limit in (0, 74):
+        net = Net()
+        weights = configs.build_mixer(net, n=n, blocks=2, m=10).weights
+        net.allocate(batch)
+        rng = np.random.default_rng(7)
+        for uid, size, std in weights:
+            net.set_values(uid, *[(rng.standard_normal(size) * std).astype(np.float32) for _ in range(2)])
+        x = tuple(torch.from_numpy(rng.standard_normal((batch, n)).astype(np.float32)).pin_memory() for _ in range(2))
+        net.upload(x=x, labels=torch.from_numpy(rng.integers(0, 10, batch).astype(np.int32)).pin_memory())
+        assert net.lib.cnb_set_gemm_sm_limit(net.lib.cnh_context(net.h), limit) == 0
+        for _ in range(2):                               # the second pass as the first
+            net.update_inputs(0.0)
+            net.forward()
+            net.backward()
+            net.sync()
+            runs.append(net.grad_tensor().cpu().numpy())
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert (runs[0] == runs[1]).all() and (runs[2] == runs[3]).all() and (runs[0] != runs[2]).any()
+        assert np.linalg.norm(runs[2] - runs[0]) < 2e-5 * np.linalg.norm(runs[0])
