@@ -1226,6 +1226,7 @@ cgemm_tc_k(const __grid_constant__ OperandMaps<FORM> om, const __grid_constant__
                 }
             }
             CNB_GSTAMP(7, threadIdx.x == Threads<DRAIN>::FIRST_EPI);
+            __syncwarp();                                // (lanes beyond the tile have left the loops one by one)
             cluster_sync();                              // no CTA leaves while a peer still reads its shared memory
             CNB_GSTAMP(8, threadIdx.x == Threads<DRAIN>::FIRST_EPI);
         }
@@ -1545,6 +1546,7 @@ __global__ void __launch_bounds__(256) pack_one_k(const __grid_constant__ PackJo
         low = __reduce_max_sync(0xffffffffu, warp_low[lane & 7]);
         if (lane == 0) { cta[0] = most; cta[1] = low; }
     }
+    __syncwarp();                                        // (a barrier of the aligned form takes a warp's threads together)
     cluster_sync();
     most = low = 0;
     if (lane < ctas) {
@@ -1552,6 +1554,7 @@ __global__ void __launch_bounds__(256) pack_one_k(const __grid_constant__ PackJo
         asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(most), "=r"(low) : "r"(at) : "memory");
     }
     const int e = pack_exponent(__reduce_max_sync(0xffffffffu, most), __reduce_max_sync(0xffffffffu, low));
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     if (blockIdx.x == 0 && threadIdx.x == 0) job.head->exponent = e;
     const bool plain = e == kPlain;
@@ -1591,6 +1594,7 @@ __global__ void __launch_bounds__(256) pack_one_k(const __grid_constant__ PackJo
             }
         }
     }
+    __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");      // no CTA leaves while a peer still reads its shared memory
 }
 
