@@ -415,17 +415,24 @@ void plan_batch(MixedPlan* pl, int B, int sms) {
     pl->rows = rows;
 }
 
-// Whether 80 registers a thread instead of `regs` save a wave of CTAs.  What they cost in loads and arithmetic ahead is more than
-// what they give where they do not (us, with 96 or 112 and with 80: 1000 x 1500 with its tail 1.1 waves of three CTAs to an SM, 22.5 and
-// 16.0 by four; 4096 x 784 plain 19.0 and 17.1, with the tail 39.2 and 30.3; 2000 x 2000 32.9 and 27.3; but 500 x 900, half a wave of
-// either, 4.6 and 5.4; 4096 x 512, 1.5 and 1.2, 10.6 and 11.6; 6000 x 600 with the tail, 2.7 and 2.03, 38.1 and 40.9).
-bool fewer_waves(long ctas, int threads, size_t smem, int regs, int sms) {
-    auto waves = [&](int r) {
-        const long by_registers = 65536 / ((long) threads * r), by_memory = (long) (227 * 1024 / (smem + 1024));
-        const long fit = std::max(1L, std::min({by_registers, by_memory, 2048L / threads})) * sms;
-        return (ctas + fit - 1) / fit;
+// Whether the form of fewer registers (80 a thread in the place of 96, with the tail 112) is the faster one: it has to save a wave of
+// CTAs, since what it costs in loads and arithmetic ahead is more than it gives where it does not, and to hold a third more of them
+// (us, with more registers and with 80: 4096 x 784 plain 22.3 and 19.7, 2282 x 396 8.9 and 7.1, 2000 x 2000 36.2 and 29.6; but four
+// CTAs or five to an SM 2500 x 1600 23.4 and 23.9, 12361 x 208 backward 17.4 and 17.9, 39267 x 50 11.4 and 11.5).
+//
+// With the tail, short rows store runs of a few floats into four planes, and more CTAs at once are in each other's way there: a saved
+// wave may stand for three and a half CTAs an SM, five and a half where two were resident (1000 x 1500 22.6 and 16.9, 28360 x 32 10.2
+// and 7.7; but 47095 x 50 23.0 and 25.8, 82001 x 50 34.3 and 38.6, 48007 x 72 33.4 and 36.1, 64750 x 49
+// 36.6 and 38.0; of 247 sizes that save a wave, 33 that lost by it are left out so, and 27 % of what the others gain).
+bool fewer_waves(long ctas, int threads, size_t smem, int regs, int fewer, int sms, int n, bool tail) {
+    auto fit = [&](int r) {
+        const long by_registers = 65536 / ((long) threads * ((r + 7) / 8 * 8)), by_memory = (long) (227 * 1024 / (smem + 1024));
+        return std::max(1L, std::min({by_registers, by_memory, 2048L / threads}));
     };
-    return waves(80) < waves(regs);
+    auto waves = [&](long f) { return (ctas + f * sms - 1) / (f * sms); };
+    const long before = fit(regs), after = fit(fewer), saved = waves(before) - waves(after);
+    if (saved <= 0 || 3 * after < 4 * before) return false;
+    return !tail || n > 256 || 2 * ctas <= (before == 2 ? 11 : 7) * saved * sms;
 }
 
 // The tail in a loop through shared memory, by all threads: written out behind a butterfly of 16 points it is 30 KB of
@@ -499,6 +506,7 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
     if (finish == TAIL && loop_tail(&pl, B)) finish = TAIL_LOOP;
     const size_t smem = smem_bytes(pl.m, pl.rows, pl.buffers);
     static bool attr_done[64] = {};                         // the attribute is per device
+    static int registers[3][2];                             // of a thread in each form, as the kernels were built (all devices alike)
     if (!attr_done[ctx->device & 63]) {
 #define CNB_MIXED_ATTR(F, C, S, N) \
     CNB_CUDA(cudaFuncSetAttribute(fft_mixed_k<F, C, S, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) MAX_SMEM))
@@ -509,6 +517,16 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
         CNB_MIXED_ATTR(TAIL_LOOP, true, SPREAD, 2);
 #undef CNB_MIXED_ATTRS
 #undef CNB_MIXED_ATTR
+#define CNB_MIXED_REGS(F, N)                                                                                  \
+    do {                                                                                                      \
+        cudaFuncAttributes a, b;                                                                              \
+        CNB_CUDA(cudaFuncGetAttributes(&a, fft_mixed_k<F, false, SPREAD, N>));                                \
+        CNB_CUDA(cudaFuncGetAttributes(&b, fft_mixed_k<F, false, NO_SPREAD, N>));                             \
+        registers[F][N - 2] = std::max(a.numRegs, b.numRegs);                                                 \
+    } while (0)
+        CNB_MIXED_REGS(STORE, 2); CNB_MIXED_REGS(TAIL, 2); CNB_MIXED_REGS(ADD, 2);
+        CNB_MIXED_REGS(STORE, 3); CNB_MIXED_REGS(TAIL, 3); CNB_MIXED_REGS(ADD, 3);
+#undef CNB_MIXED_REGS
         attr_done[ctx->device & 63] = true;
     }
     const dim3 grid((unsigned) ((B + pl.rows - 1) / pl.rows)), block((unsigned) pl.threads);
@@ -520,7 +538,7 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
                  finish == ADD ? go(fft_mixed_k<ADD, true, SPREAD, 2>) : go(fft_mixed_k<STORE, true, SPREAD, 2>));
     } else if (finish == TAIL_LOOP) {
         CNB_MIXED(TAIL_LOOP, 2);
-    } else if (fewer_waves((long) grid.x, pl.threads, smem, finish == TAIL ? 112 : 96, usable_sms(ctx))) {
+    } else if (fewer_waves((long) grid.x, pl.threads, smem, registers[finish][0], registers[finish][1], usable_sms(ctx), pl.n, finish == TAIL)) {
         if (finish == TAIL) CNB_MIXED(TAIL, 3);
         else if (finish == ADD) CNB_MIXED(ADD, 3);
         else CNB_MIXED(STORE, 3);
@@ -537,6 +555,20 @@ int fft_mixed(cnb_ctx* ctx, const float* xr, const float* xi, float* yr, float* 
 }
 
 }  // namespace cnb
+
+extern "C" int cnb_fft_form(int N, int B, int tail, int sm_count, int regs, int fewer_regs, int* out4) {
+    MixedPlan pl;
+    if (!out4 || B <= 0 || sm_count <= 0 || regs <= 0 || fewer_regs <= 0) return cnb::set_error(CNB_ERR_ARG, "cnb_fft_form: B=%d sm_count=%d", B, sm_count);
+    if (!cached_plan(N, &pl)) return cnb::set_error(CNB_ERR_UNSUPPORTED, "cnb_fft_form: N=%d", N);
+    plan_batch(&pl, B, sm_count);
+    const bool loop = tail && loop_tail(&pl, B);
+    const long ctas = (B + pl.rows - 1) / pl.rows;
+    out4[0] = (int) ctas;
+    out4[1] = pl.threads;
+    out4[2] = loop ? 1 : 0;
+    out4[3] = !loop && pl.m == pl.n && fewer_waves(ctas, pl.threads, smem_bytes(pl.m, pl.rows, pl.buffers), regs, fewer_regs, sm_count, N, tail != 0);
+    return CNB_OK;
+}
 
 extern "C" int cnb_fft_plan(int N, int B, int sm_count, int* out, int capacity) {
     MixedPlan pl;

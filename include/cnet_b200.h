@@ -182,6 +182,10 @@ int cnb_dft_fwd(cnb_ctx* ctx, const float* x_re, const float* x_im,
  * CPU: impl/ft.h:57-80. */
 int cnb_dft_bwd(cnb_ctx* ctx, const float* g_re, const float* g_im,
                 float* dx_re, float* dx_im, int B, int N, int accumulate, void* stream);
+/* How a transform of B rows of N (not 1024) would be launched, with the tail below or without, on a device of sm_count SMs, by kernels of
+ * `regs` registers a thread or fewer: host arithmetic only.  out4 = {CTAs, threads, the tail in a loop of its own, the form of fewer
+ * registers}. */
+int cnb_fft_form(int N, int B, int tail, int sm_count, int regs, int fewer_regs, int* out4);
 /* FourierTrans -> Hadamard(shared h) -> CGelu in one pass over the row (the N that have an FFT kernel, see
  * cnb_dft_fused_ok): u = DFT(x) is kept for the backward, y = gelu(u o h), optionally with the
  * operand split of y for the Linear that follows; y_re = y_im = NULL is allowed when y_split
