@@ -146,7 +146,8 @@ skinny_fwd_rows_k(const float* xr, const float* xi, const float* wr,
         for (int o = 0; o < OT * 2; ++o) a[r][o] = 0.f;
     // Nothing here asks whether an output exists: behind such a branch each one's weights were a round trip to L2 of their own and
     // each one's sum a chain of shuffles (86 x 256 -> 13 5.0 us, 3.1 so; 64 x 784 -> 10 4.3 and 3.5; 256 x 256 -> 16 5.9 and 3.6; 64 x 785 -> 10 5.7 and 4.0).
-    constexpr int G = OT <= 10 ? OT : 8;                 // outputs whose weights are in flight together
+    constexpr int G = OT <= 10 ? OT : OT / 2;            // outputs whose weights are in flight together
+    static_assert(OT % G == 0, "groups of outputs");
 #pragma unroll(W == 1 ? 4 : 1)
     for (int i = threadIdx.x * W; i < in; i += 256 * W) {
         float p[RB][W], q[RB][W];
@@ -286,7 +287,7 @@ skinny_bwd_w_stage1_k(const float* gr, const float* gi, const float* xr,
                 ai[o][k] += c * x[k] - a * y[k];
             }
         };
-        if constexpr (W == 4) {
+        if constexpr (W == 4 && OT > 3) {
             for (int b = r0 + threadIdx.y; b < r1; b += 8) {
                 float x[W], y[W], a[OT], c[OT];
                 ldv(xr + (size_t) b * in + col, x); ldv(xi + (size_t) b * in + col, y);
@@ -303,7 +304,8 @@ skinny_bwd_w_stage1_k(const float* gr, const float* gi, const float* xr,
             }
         } else {
             // one column a lane: as many loads of G as of anything, and rows enough on their way (4096 x 1025 -> 10 31.8 us, with G
-            // requested as above 44.8)
+            // requested as above 44.8); up to three outputs: few loads of G, and two rows on their way are worth more (2000 x 512 -> 2
+            // 6.1 -> 5.5 us)
 #pragma unroll 2
             for (int b = r0 + threadIdx.y; b < r1; b += 8) {
                 float x[W], y[W];
@@ -387,12 +389,17 @@ size_t skinny_workspace_bytes(int B, int in, int out, int sm_count) {
         else cnb::launch(KERNEL<16, W>, __VA_ARGS__);                         \
     } while (0)
 
-#define CNB_SKINNY_DISPATCH_ROWS(W, RB, ...)                                  \
+// The same for kernels that work on all of OT outputs, whether they exist or not: with few of them a bound beyond `out` is as much work
+// again for nothing (433 x 1636 -> 1 forward by the bound of 4 4.0 us, 2.4 by its own; bounds of 6 and 12 were slower than 8 and 16).
+#define CNB_SKINNY_DISPATCH_ALL(LAUNCH)                                       \
     do {                                                                      \
-        if (out <= 4) cnb::launch(skinny_fwd_rows_k<4, W, RB>, __VA_ARGS__);  \
-        else if (out <= 8) cnb::launch(skinny_fwd_rows_k<8, W, RB>, __VA_ARGS__); \
-        else if (out <= 10) cnb::launch(skinny_fwd_rows_k<10, W, RB>, __VA_ARGS__); \
-        else cnb::launch(skinny_fwd_rows_k<16, W, RB>, __VA_ARGS__);          \
+        if (out == 1) LAUNCH(1);                                              \
+        else if (out == 2) LAUNCH(2);                                         \
+        else if (out == 3) LAUNCH(3);                                         \
+        else if (out == 4) LAUNCH(4);                                         \
+        else if (out <= 8) LAUNCH(8);                                         \
+        else if (out <= 10) LAUNCH(10);                                       \
+        else LAUNCH(16);                                                      \
     } while (0)
 
 static bool aligned16(const void* a, const void* b, const void* c = nullptr, const void* d = nullptr) {
@@ -407,14 +414,13 @@ int skinny_fwd(cnb_ctx* ctx, const float* xr, const float* xi, const float* wr, 
     // with W staged, 11.1 against 9.5 at 1024, where every row or two reads W again.  Short rows leave most of a CTA's
     // threads idle: at 64 -> 4 one row per CTA is even (2.0 us at 64 rows), two are not (2.6 against 2.2 at 512).
     if (B <= 2 * usable_sms(ctx) || (B <= 512 && in >= 256)) {
-        const dim3 block(256);
-        if (B <= 2 * usable_sms(ctx)) {
-            if (vec) CNB_SKINNY_DISPATCH_ROWS(4, 1, dim3(B), block, 0, st, 1, xr, xi, wr, wi, yr, yi, B, in, out);
-            else CNB_SKINNY_DISPATCH_ROWS(1, 1, dim3(B), block, 0, st, 1, xr, xi, wr, wi, yr, yi, B, in, out);
-        } else {
-            if (vec) CNB_SKINNY_DISPATCH_ROWS(4, 2, dim3((B + 1) / 2), block, 0, st, 1, xr, xi, wr, wi, yr, yi, B, in, out);
-            else CNB_SKINNY_DISPATCH_ROWS(1, 2, dim3((B + 1) / 2), block, 0, st, 1, xr, xi, wr, wi, yr, yi, B, in, out);
-        }
+        const bool two = B > 2 * usable_sms(ctx);
+        const dim3 block(256), grid(two ? (B + 1) / 2 : B);
+#define CNB_ROWS_GO(OT, W, RB) cnb::launch(skinny_fwd_rows_k<OT, W, RB>, grid, block, 0, st, 1, xr, xi, wr, wi, yr, yi, B, in, out)
+#define CNB_ROWS(OT) (two ? vec ? CNB_ROWS_GO(OT, 4, 2) : CNB_ROWS_GO(OT, 1, 2) : vec ? CNB_ROWS_GO(OT, 4, 1) : CNB_ROWS_GO(OT, 1, 1))
+        CNB_SKINNY_DISPATCH_ALL(CNB_ROWS);
+#undef CNB_ROWS
+#undef CNB_ROWS_GO
         CNB_LAUNCH_CHECK("skinny_fwd_rows");
         return CNB_OK;
     }
@@ -473,8 +479,10 @@ int skinny_bwd_w(cnb_ctx* ctx, const float* gr, const float* gi, const float* xr
     float* pr = ws;
     float* pi = ws + (size_t) chunks * n;
     const dim3 grid(col_blocks, chunks), block(32, 8);
-    if (vec) CNB_SKINNY_DISPATCH(skinny_bwd_w_stage1_k, 4, grid, block, 0, st, 1, gr, gi, xr, xi, pr, pi, B, in, out, rows);
+#define CNB_STAGE1(OT) cnb::launch(skinny_bwd_w_stage1_k<OT, 4>, grid, block, 0, st, 1, gr, gi, xr, xi, pr, pi, B, in, out, rows)
+    if (vec) CNB_SKINNY_DISPATCH_ALL(CNB_STAGE1);
     else CNB_SKINNY_DISPATCH(skinny_bwd_w_stage1_k, 1, grid, block, 0, st, 1, gr, gi, xr, xi, pr, pi, B, in, out, rows);
+#undef CNB_STAGE1
     CNB_LAUNCH_CHECK("skinny_bwd_w_stage1");
     cnb::launch(skinny_bwd_w_stage2_k, dim3((unsigned) ((n + 31) / 32)), dim3(32, 8), 0, st, 1, pr, pi, dr, di, chunks, n, accumulate);
     CNB_LAUNCH_CHECK("skinny_bwd_w_stage2");
