@@ -215,7 +215,10 @@ cgemm_slim_k(const float* a_re, const float* a_im, long sam, long sak, const flo
 // 5.0 and 5.7; 260 x 35, K = 223, 1.1, 7.8 and 7.0).  Beyond, where A lies along k: from 1.25 tiles of 16 to an SM on, which are the second
 // round of those (177 x 285, K = 35 4.3 and 3.4; 87 x 794, K = 89 8.9 and 6.4; but 108 x 403, K = 107, 1.23, 5.8 and 6.6), up to eight of
 // these (91 x 899, K = 36, 9.2, 4.3 and 4.8), and where a tile of 16 would be a quarter empty at a K that counts (1241 x 20, K = 204 14.4 and 10.5).
+// Below a K of 16 five slabs on their way are none, and their set-up is what counts (16 x 31, K = 3 1.15 and 1.43, 123 x 381, K = 2 2.0 and
+// 2.2; 60 sizes of K from 16 to 23 0.95 of the time in the mean).
 bool slim_tiles(int M, int N, int K, bool ak, bool bk, int sms) {
+    if (K < 16) return false;
     const long slim = (long) ((M + SLIM - 1) / SLIM) * ((N + SLIM - 1) / SLIM), small = (long) ((M + 15) / 16) * ((N + 15) / 16);
     if (4 * slim <= (ak && bk ? 8 : ak || bk ? 6 : 5) * sms) return true;
     if (!ak) return false;

@@ -42,3 +42,30 @@ def test_few_outputs(B, n_in, n_out):
     near(ctx.linear_bwd_x(g, w, out=tuple(t.clone() for t in old)), G @ W.conj() + full(old), n_out)
     old = pair(n_out, n_in)
     near(ctx.linear_bwd_w(g, x, out=tuple(t.clone() for t in old)), G.T @ X.conj() + full(old), B)
+
+
+def test_a_short_k_takes_no_longer_than_a_longer_one():
+    """16 x 31, K = 3, is not the tiles of 8 x 8, whose set-up is for several slabs of K: 1.2 us, by those 1.4, as K = 20 takes."""
+    import torch
+    ctx = Context(arena_bytes=64 << 20)
+
+    def least(k):
+        g, x = [tuple(torch.randn(k, n, device="cuda") for _ in range(2)) for n in (16, 31)]
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            ctx.linear_bwd_w(g, x)
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(50):
+                ctx.linear_bwd_w(g, x)
+        times = []
+        for _ in range(30):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    assert least(3) < 0.95 * least(20)
