@@ -111,6 +111,17 @@ template <int G, int E, int VEC> struct Tile {
     }
 };
 
+// Whether rows that twelve elements a thread would hold take that form and not the one of sixteen: with fewer registers more CTAs
+// are resident, which is no gain where few are launched, and twelve scattered loads are slower than sixteen then (us, with 16 and with
+// 12: loss of 95 x 4903 3.5 and 4.6, forward of 185 x 5452 3.8 and 4.5, of 417 x 1296 2.8 and 2.9; 164 x 4394 5.7 and 4.4, 567 x 1025 4.0
+// and 2.9, 4607 x 1116 9.7 and 9.2; backward, of four planes, 95 x 4903 6.1 and 4.6, 185 x 5452 5.5 and 4.6, but 523 x 1436 3.3 and 3.8; eight
+// rows to a CTA 2276 x 378 forward 3.1 and 4.0, backward 2.9 and 3.5).
+bool twelve(int g, int vec, int planes, size_t ctas, int sms) {
+    if (g == 32) return ctas >= 5 * (size_t) sms;
+    if (planes == 4) return g != 128 || vec == 1 || ctas >= 5 * (size_t) sms;
+    return ctas >= (vec == 1 ? 1 : 5) * (size_t) sms;
+}
+
 constexpr int cta_threads(int g) { return g < 128 ? 256 : g; }
 
 template <int G, int E, int VEC>
@@ -295,24 +306,25 @@ bool vec_ok(int n, std::initializer_list<const void*> planes) {
 // the kernel, the argument list ends with rows, n, parts and what may follow them.
 #define CNB_ROWS_GO(NAME, G, E, V, CTAS, PARTS, ...)                                                                     \
     cnb::launch(NAME<G, E, V>, dim3((unsigned) (CTAS)), dim3(cta_threads(G)), 0, st, PARTS, __VA_ARGS__)
-#define CNB_ROWS_V(NAME, V, rows, n, ...)                                                                                \
+#define CNB_ROWS_V(NAME, PLANES, V, rows, n, ...)                                                                                \
     do {                                                                                                                 \
         if ((n) <= 32) CNB_ROWS_GO(NAME, 8, 4, V, ((size_t) (rows) + 31) / 32, 1, __VA_ARGS__);                          \
         else if ((n) <= 128) CNB_ROWS_GO(NAME, 32, 4, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                     \
         else if ((n) <= 256) CNB_ROWS_GO(NAME, 32, 8, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                     \
-        else if ((n) <= 384) CNB_ROWS_GO(NAME, 32, 12, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                    \
+        else if ((n) <= 384 && twelve(32, V, PLANES, ((size_t) (rows) + 7) / 8, ctx->sm_count))                          \
+            CNB_ROWS_GO(NAME, 32, 12, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                                     \
         else if ((n) <= 512) CNB_ROWS_GO(NAME, 32, 16, V, ((size_t) (rows) + 7) / 8, 1, __VA_ARGS__);                    \
         else if ((n) <= 1024) CNB_ROWS_GO(NAME, 128, 8, V, rows, 1, __VA_ARGS__);                                        \
-        else if ((n) <= 1536) CNB_ROWS_GO(NAME, 128, 12, V, rows, 1, __VA_ARGS__);                                       \
+        else if ((n) <= 1536 && twelve(128, V, PLANES, rows, ctx->sm_count)) CNB_ROWS_GO(NAME, 128, 12, V, rows, 1, __VA_ARGS__); \
         else if ((n) <= 2048) CNB_ROWS_GO(NAME, 128, 16, V, rows, 1, __VA_ARGS__);                                       \
         else if ((n) <= 4096) CNB_ROWS_GO(NAME, 512, 8, V, rows, 1, __VA_ARGS__);                                        \
-        else if ((n) <= 6144) CNB_ROWS_GO(NAME, 512, 12, V, rows, 1, __VA_ARGS__);                                       \
+        else if ((n) <= 6144 && twelve(512, V, PLANES, rows, ctx->sm_count)) CNB_ROWS_GO(NAME, 512, 12, V, rows, 1, __VA_ARGS__); \
         else CNB_ROWS_GO(NAME, 512, 16, V, (size_t) (rows) * parts, parts, __VA_ARGS__);                                 \
     } while (0)
-#define CNB_ROWS(NAME, vec, rows, n, ...)                                                                                \
+#define CNB_ROWS(NAME, PLANES, vec, rows, n, ...)                                                                                \
     do {                                                                                                                 \
-        if (vec) CNB_ROWS_V(NAME, 4, rows, n, __VA_ARGS__);                                                              \
-        else CNB_ROWS_V(NAME, 1, rows, n, __VA_ARGS__);                                                                  \
+        if (vec) CNB_ROWS_V(NAME, PLANES, 4, rows, n, __VA_ARGS__);                                                              \
+        else CNB_ROWS_V(NAME, PLANES, 1, rows, n, __VA_ARGS__);                                                                  \
         CNB_LAUNCH_CHECK(#NAME);                                                                                         \
     } while (0)
 
@@ -333,7 +345,7 @@ int cnb_softmax_fwd(cnb_ctx* ctx, const float* z_re, const float* z_im, float* y
         cnb::launch(softmax_fwd_long_k, dim3(B), dim3(512), 0, st, 1, z_re, z_im, y_re, y_im, inv_norm, N);
         CNB_LAUNCH_CHECK("softmax_fwd");
     } else {
-        CNB_ROWS(softmax_fwd_k, vec_ok(N, {z_re, z_im, y_re, y_im}), B, N, z_re, z_im, y_re, y_im, inv_norm, B, N, parts);
+        CNB_ROWS(softmax_fwd_k, 2, vec_ok(N, {z_re, z_im, y_re, y_im}), B, N, z_re, z_im, y_re, y_im, inv_norm, B, N, parts);
     }
     return CNB_OK;
 }
@@ -350,7 +362,7 @@ int cnb_softmax_bwd(cnb_ctx* ctx, const float* g_re, const float* g_im, const fl
         cnb::launch(softmax_bwd_long_k, dim3(B), dim3(512), 0, st, 1, g_re, g_im, z_re, z_im, inv_norm, dz_re, dz_im, N, accumulate);
         CNB_LAUNCH_CHECK("softmax_bwd");
     } else {
-        CNB_ROWS(softmax_bwd_k, vec_ok(N, {g_re, g_im, z_re, z_im, dz_re, dz_im}), B, N, g_re, g_im, z_re, z_im, inv_norm, dz_re,
+        CNB_ROWS(softmax_bwd_k, 4, vec_ok(N, {g_re, g_im, z_re, z_im, dz_re, dz_im}), B, N, g_re, g_im, z_re, z_im, inv_norm, dz_re,
                  dz_im, B, N, parts, accumulate);
     }
     return CNB_OK;
@@ -367,7 +379,7 @@ int cnb_crossent_fwd_bwd(cnb_ctx* ctx, const float* z_re, const float* z_im, con
         cnb::launch(crossent_long_k, dim3(B), dim3(512), 0, st, 1, z_re, z_im, labels, loss, dz_re, dz_im, M);
         CNB_LAUNCH_CHECK("crossent");
     } else {
-        CNB_ROWS(crossent_k, vec_ok(M, {z_re, z_im, dz_re, dz_im}), B, M, z_re, z_im, labels, loss, dz_re, dz_im, B, M, parts);
+        CNB_ROWS(crossent_k, 2, vec_ok(M, {z_re, z_im, dz_re, dz_im}), B, M, z_re, z_im, labels, loss, dz_re, dz_im, B, M, parts);
     }
     return CNB_OK;
 }
@@ -383,7 +395,7 @@ int cnb_l2out_fwd_bwd(cnb_ctx* ctx, const float* z_re, const float* z_im, float*
         cnb::launch(l2out_long_k, dim3(B), dim3(512), 0, st, 1, z_re, z_im, loss, dz_re, dz_im, N);
         CNB_LAUNCH_CHECK("l2out");
     } else {
-        CNB_ROWS(l2out_k, vec_ok(N, {z_re, z_im, dz_re, dz_im}), B, N, z_re, z_im, loss, dz_re, dz_im, B, N, parts);
+        CNB_ROWS(l2out_k, 2, vec_ok(N, {z_re, z_im, dz_re, dz_im}), B, N, z_re, z_im, loss, dz_re, dz_im, B, N, parts);
     }
     return CNB_OK;
 }
