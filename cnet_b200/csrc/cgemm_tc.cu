@@ -54,6 +54,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <bitset>
 #include <cmath>
 #include <cstdlib>
 #include <type_traits>
@@ -1880,6 +1881,22 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         }
         return all_cubes;
     };
+    // Where chains begin (K <= 4096), and how many of them the sums hold, over all additions of a tile: each is rounded at its magnitude.
+    struct Sums { std::bitset<128> at; int adds; };
+    auto sums = [&](int c, int first, int rest) {
+        Sums v = {{}, 0};
+        for (int k = 0, all = 0; k < c; ++k) {
+            int n = 0;
+            for (int kb = k_blocks * k / c, end = k_blocks * (k + 1) / c; kb < end; kb += kb == 0 ? first : rest) {
+                v.at.set(kb);
+                v.adds += n > 0 ? n + 1 : 0;
+                ++n;
+            }
+            v.adds += all > 0 ? all + n : 0;
+            all += n;
+        }
+        return v;
+    };
     const bool several = now.rest < (c0 > 1 ? (k_blocks + c0 - 1) / c0 : r.upc), vec = N % 4 == 0;
     // Costs in hundredths of a microsecond: blocks, what a cluster adds, taking a chain out of tensor memory before the next.
     struct { int tile_n, c, first, rest; long cost; } best = {0, 0, 0, 0, 0};
@@ -1904,8 +1921,13 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         for (int rest = std::min(run, now.rest); rest >= 1 && fixed + chain * ((run + rest - 1) / rest - 1) <= most; --rest)
             for (int first = rest; first >= std::max(1, rest - 1); --first) {
                 const Sum v = cluster_of(c, first, rest);
-                // (as many cubes in other runs may be 1.03 as far off: 1010 x 1595, K = 323; those of the same slices are not)
-                if (!as_it_is && v.cubes * tiles * 20 > cubes() * (c == c0 && c0 > 1 ? 20 : 19)) continue;
+                // As many cubes in other runs may be 1.03 as far off (1010 x 1595, K = 323), and so may the same chains added up one after
+                // the other (346 x 1698, K = 199: four in a row 1.027 as far as two by two).
+                if (!as_it_is && v.cubes * tiles * 20 > cubes() * 19) {
+                    if (c0 == 1 || c == 1 || v.cubes != cubes()) continue;
+                    const Sums before_it = sums(c0, now.first, now.rest), it = sums(c, first, rest);
+                    if (it.at != before_it.at || it.adds > before_it.adds) continue;
+                }
                 const long cost = fixed + chain * (v.chains - 1);
                 if (best.c == 0 || cost < best.cost) best = {tile_n, c, first, rest, cost};
                 return;

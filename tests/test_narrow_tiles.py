@@ -96,3 +96,9 @@ def test_the_choice_takes_little_of_the_host():
 
     for M, N, K in [(437, 89, 3952), (411, 110, 3952), (506, 124, 3888), (281, 203, 2560), (159, 4070, 3377)]:
         assert least(M, N, K) - least(4096, 4096, 64) < 6e-6, (M, N, K)
+
+
+def test_the_same_chains_in_fewer_slices_are_as_exact():
+    """Eight slices of two blocks as four of two chains each: the same cuts and no more in any sum, so no chain need be shorter."""
+    s, f = _schedule(300, 500, 500, 0, 0), _form(300, 500, 500, 0)
+    assert (s["cluster_ctas"], f["tile_n"], f["first"], f["rest"]) == (4, 64, 2, 2), (s, f)
