@@ -437,20 +437,14 @@ bool fewer_waves(long ctas, int threads, size_t smem, int regs, int fewer, int s
 
 // The tail in a loop through shared memory, by all threads: written out behind a butterfly of 16 points it is 30 KB of
 // instructions, which a small batch runs through once, at the pace of their first fetch, on the few threads that have a last
-// butterfly (16 x 256 5.7 -> 3.0 us, 296 x 100 4.3 -> 2.9, 296 x 500 5.6 -> 4.2; in a training step, where other kernels'
+// butterfly (16 x 256 5.7 -> 3.0 us, 296 x 100 4.3 -> 2.9, 296 x 500 5.6 -> 4.2, 512 x 784 8.2 -> 6.4; in a training step, where other kernels'
 // instructions lie between, more).  Not where the trip through shared memory counts, whose row one CTA then has on its way twice: from
 // half a million elements (1024 x 512 6.2 and 6.3, 1024 x 900 11.2 and 16.3; half of that in the chirp form, 1024 x 137 7.6 and 7.4, 4096 x 137 16.8
-// and 19.5) and beyond 1024 points (86 x 2000 7.3 and 7.5).  And not where a nearly full CTA has few elements a thread in the last pass anyway and that pass is
-// light, behind a first one of radix 8 or in three passes (us, written out and in a loop: 9462 x 48 5.0 and 5.4, 8310 x 56 5.0 and 5.6,
-// 512 x 784 5.8 and 6.2, 359 x 273 4.1 and 4.5, 18783 x 27 5.5 and 6.3; but 2309 x 182, 13 elements for each of 128 threads, 6.8 and 5.4,
-// 11215 x 25 4.5 and 3.8, 8148 x 42 4.8 and 4.4).  Two elements a thread, in one round: as many threads as that takes (16 x 256
+// and 19.5) and beyond 1024 points (86 x 2000 7.3 and 7.5).  Two elements a thread, in one round: as many threads as that takes (16 x 256
 // 3.0 us, with four 3.5).
 bool loop_tail(MixedPlan* pl, int B) {
     const bool chirp = pl->m > pl->n;
     if (pl->n > 1024 || (long) B * pl->n >= (chirp ? 1 << 18 : 1 << 19)) return false;
-    const Pass& last = pl->p[pl->passes - 1];
-    if (!chirp && (pl->passes > 2 || pl->p[0].radix == 8 || last.radix <= 3) && pl->threads >= 192 &&
-        (pl->rows * last.nb + pl->threads - 1) / pl->threads * last.radix <= 9) return false;
     const int buffers = (chirp ? 2 : 1) * pl->passes > 1 ? 2 : 1;
     if (smem_bytes(pl->m, pl->rows, buffers) > MAX_SMEM) return false;
     pl->buffers = buffers;

@@ -28,13 +28,3 @@ def test_no_form_for_what_has_no_kernel():
     out = (C.c_int * 4)()
     assert L.load().cnb_fft_form(1, 16, 0, SMS, 96, 80, out) < 0
     assert L.load().cnb_fft_form(100, 0, 0, SMS, 96, 80, out) < 0
-
-
-@pytest.mark.parametrize("B,N,loop", [
-    (16, 256, 1), (296, 100, 1), (296, 500, 1),         # few rows, many elements a thread
-    (2309, 182, 1), (16779, 25, 1), (15929, 30, 1), (11215, 25, 1), (8148, 42, 1),
-    (9462, 48, 0), (18783, 27, 0), (786, 448, 0), (85, 676, 0), (13480, 32, 0), (8310, 56, 0), (512, 784, 0), (359, 273, 0),
-    (4096, 512, 0), (86, 2000, 0),                                       # many elements, long rows
-])
-def test_the_tail_in_a_loop_where_it_is_faster(B, N, loop):
-    assert _form(B, N, 1)["loop"] == loop
