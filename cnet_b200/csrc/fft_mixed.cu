@@ -437,8 +437,9 @@ bool fewer_waves(long ctas, int threads, size_t smem, int regs, int fewer, int s
 
 // The tail in a loop through shared memory, by all threads: written out behind a butterfly of 16 points it is 30 KB of
 // instructions, which a small batch runs through once, at the pace of their first fetch, on the few threads that have a last
-// butterfly (16 x 256 5.7 -> 3.0 us, 296 x 100 4.3 -> 2.9, 296 x 500 5.6 -> 4.2, 512 x 784 8.2 -> 6.4; in a training step, where other kernels'
-// instructions lie between, more).  Not where the trip through shared memory counts, whose row one CTA then has on its way twice: from
+// butterfly (16 x 256 5.7 -> 3.0 us, 296 x 100 4.3 -> 2.9, 296 x 500 5.6 -> 4.2; in a training step, where other
+// kernels' instructions lie between, more: calls back to back of rows whose last pass is light are slower by the loop, 9462 x 48 5.0 and 5.3,
+// 8310 x 56 5.0 and 5.6, 512 x 784 5.8 and 6.2, and steps are not, 512 x 784 in 4 blocks 349 and 339, 359 x 273 30.9 and 29.0).  Not where the trip through shared memory counts, whose row one CTA then has on its way twice: from
 // half a million elements (1024 x 512 6.2 and 6.3, 1024 x 900 11.2 and 16.3; half of that in the chirp form, 1024 x 137 7.6 and 7.4, 4096 x 137 16.8
 // and 19.5) and beyond 1024 points (86 x 2000 7.3 and 7.5).  Two elements a thread, in one round: as many threads as that takes (16 x 256
 // 3.0 us, with four 3.5).

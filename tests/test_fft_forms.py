@@ -28,3 +28,11 @@ def test_no_form_for_what_has_no_kernel():
     out = (C.c_int * 4)()
     assert L.load().cnb_fft_form(1, 16, 0, SMS, 96, 80, out) < 0
     assert L.load().cnb_fft_form(100, 0, 0, SMS, 96, 80, out) < 0
+
+
+@pytest.mark.parametrize("B,N,loop", [
+    (16, 256, 1), (296, 500, 1), (512, 784, 1), (359, 273, 1),
+    (4096, 512, 0), (86, 2000, 0),                       # half a million elements, more than 1024 points
+])
+def test_the_tail_in_a_loop(B, N, loop):
+    assert _form(B, N, 1)["loop"] == loop
