@@ -1826,11 +1826,11 @@ double tile_cubes(int M, int N, int K, const Schedule& q) {
 // are, on 148 SMs) never are, and neither are short runs summed with atomics.  The estimate below, fitted to 20 sizes at every
 // width and cluster that has room and to 40 that ran as such sums, has to promise a microsecond (300 x 500, K = 500 19.2 -> 17.3,
 // 256 x 512, K = 512 17.1 -> 15.2, 128 x 2048, K = 512 30.4 -> 18.7, 350 x 401, K = 1081 35.6 -> 22.7; 512 x 1024, K = 1024 stays
-// as it is).  Of 2100 products of 16 to 3000 rows and columns that run otherwise with
-// narrow tiles than without, the time is 0.82 of what it was in the mean; four take 2 to 9 % more (946 x 115, K = 2151, added, 29.7 ->
-// 32.3), the others no more than runs of one program differ.  Chains are as short as it takes that sums in another order are no further off float64: a twentieth
-// fewer cubes (below), since as many, cut elsewhere, are up to 1.02 times as far off.  Of 900 such products none is more than 1.002
-// times as far, and in the mean they are 0.89 times.
+// as it is).  Of 2100 products of 16 to 3000 rows and columns that run otherwise with narrow tiles than without, the time is 0.83 of
+// what it was in the mean; seven take 2 to 6 % more (390 x 108, K = 1639 20.9 -> 22.1, 1048 x 928, K = 3432 104 -> 108), the others no
+// more than runs of one program differ.  Chains are as short as it takes that sums in another order are no further off float64: a
+// twentieth fewer cubes (below), since as many, cut elsewhere, are up to 1.02 times as far off.  None of the 2100 is more than 1.002
+// times as far, and in the mean they are 0.92 times.
 //
 // Products with an N of up to 128, and gradients with an M of up to 128, are those of a head.  The gradient of a loss divides by
 // what they give, which magnifies a sum in another order, so they keep theirs where it is fixed.
@@ -1912,8 +1912,6 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         // four 20.0 -> 21.6, 438 x 880, K = 104 as one run 16.2 -> 17.1).
         if (accumulate && c == 1) fixed += vec ? (thin ? 300 : 100) : (thin ? 900 : 1900);
         else if (accumulate && c0 > 1 && !r.pair && !as_it_is) fixed += 250;
-        // One row of tiles gains a microsecond less by a smaller cluster (64 x 2560, K = 336 19.1 -> 19.9).
-        else if (M <= BM && c0 > 1 && !r.pair && !as_it_is) fixed += 100;
         const int chain = thin ? 50 : 100;
         // the longest chains that are no less exact than those of the form before; a shorter first one where that does.  No further
         // than a cost that would be taken (the search through all of it took up to 14 us of the host's time a launch, 437 x 89, K = 3952).
@@ -1943,10 +1941,12 @@ void narrow_tiles(Schedule& r, int M, int N, int K, int k_blocks, int accumulate
         best.c = 0;
     }
     for (int c = c0 == 1 || r.pair ? 8 : c0 / 2; c >= 1; c /= 2) { consider(BN, c, false); consider(NARROW, c, false); }
-    // Runs with atomics may take less than the estimate where large clusters would replace them (257 x 112, K = 2375 21.3 -> 24.1,
-    // 1022 x 107, K = 2390 33.6 -> 35.0, 409 x 594, K = 1538 33.9 -> 37.7), which have to promise more than a microsecond then.
-    const bool eight = best.c == 8;
-    const long promise = c0 > 1 || accumulate || best.c < 4 ? 100 : !vec ? (eight ? 550 : 350) : !eight ? 100 : split_sizes(M, N, K) ? 250 : 400;
+    // Runs with atomics may take less than the estimate where large clusters would replace them, of eight for a single column of tiles (257 x
+    // 112, K = 2375 21.3 -> 24.1, 1022 x 107, K = 2390 33.6 -> 35.0) or of four for rows of 4-byte alignment (409 x 594, K = 1538 33.9 -> 37.7):
+    // those have to promise more than a microsecond.  One row of tiles gains a little less by a smaller cluster.
+    const bool column = best.c == 8 && N <= BN;
+    const long promise = c0 > 1 ? (M <= BM && !r.pair ? 120 : 100) : accumulate || best.c < 4 ? 100 :
+                         column ? (!vec ? 550 : split_sizes(M, N, K) ? 250 : 400) : best.c == 4 && !vec ? 350 : 100;
     if (best.c == 0 || best.cost > before - promise) return;
     r.first = best.first;
     r.rest = best.rest;

@@ -72,7 +72,6 @@ def test_as_many_cubes_in_another_order_are_left(M, N, K, acc, pair, atomics):
     (2734, 478, 258, 1, 132, 2),
     (171, 2961, 192, 1, 96, 2),
     (824, 240, 680, 1, 112, 8),        # clusters half as wide read twice as many rows a CTA: 20.0 us, 21.6
-    (64, 2560, 336, 0, 80, 4),         # 19.1 us, 19.9
     (1022, 107, 2390, 0, 120, 2),      # runs with atomics 33.6 us, clusters of eight 35.0
 ])
 def test_products_that_smaller_clusters_slow_down(M, N, K, acc, ctas, cluster_ctas):
